@@ -87,6 +87,12 @@ kernels::Ctx ctx_of(const at::Tensor& t, uint64_t stream) {
   return kernels::Ctx{t.is_cuda() ? (int)t.device().index() : -1, (cudaStream_t)stream};
 }
 
+void check_bias(const at::Tensor& bias, const at::Tensor& act, int C) {
+  BAGUA_CHECK(bias.device() == act.device() && bias.scalar_type() == at::kBFloat16 && bias.is_contiguous() &&
+                  bias.numel() == C,
+              Tensor, "bias must be a contiguous bf16 vector with one entry per channel, on the activation's device");
+}
+
 void check_pair(const at::Tensor& a, const at::Tensor& b) {
   BAGUA_CHECK(a.scalar_type() == b.scalar_type() && a.numel() == b.numel() && a.device() == b.device() &&
                   a.is_contiguous() && b.is_contiguous(),
@@ -682,9 +688,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         int64_t rows;
         int C;
         rows_and_channels(z, &rows, &C);
-        BAGUA_CHECK(bias.device() == z.device() && bias.scalar_type() == at::kBFloat16 && bias.is_contiguous() &&
-                        bias.numel() == C,
-                    Tensor, "bias must be a contiguous bf16 vector with one entry per channel, on the activation's device");
+        check_bias(bias, z, C);
         if (z.is_cuda())
           model_ops::bias_relu_inplace_bf16(z.data_ptr(), bias.data_ptr(), rows, C, (cudaStream_t)stream);
         else
@@ -771,9 +775,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         nhwc_dims(p, &N2, &H2, &W2, &C2);
         BAGUA_CHECK(N2 == N && C2 == C && H2 * 2 == H && W2 * 2 == W && p.device() == y.device(), Tensor,
                     "the pooled output must be [N, C, H/2, W/2] on the activation's device");
-        BAGUA_CHECK(bias.device() == y.device() && bias.scalar_type() == at::kBFloat16 && bias.is_contiguous() &&
-                        bias.numel() == C,
-                    Tensor, "bias must be a contiguous bf16 vector with one entry per channel, on the activation's device");
+        check_bias(bias, y, C);
         if (y.is_cuda())
           model_ops::bias_relu_pool_bf16(y.data_ptr(), p.data_ptr(), bias.data_ptr(), N, H, W, C, (cudaStream_t)stream);
         else
@@ -782,8 +784,26 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       py::arg("activation"), py::arg("pooled"), py::arg("bias"), py::arg("stream"),
       "activation = max(activation + bias, 0) in place; pooled = its 2x2 / stride-2 maximum.");
   m.def(
+      "k_bias_relu_pool",
+      [nhwc_dims](at::Tensor z, at::Tensor p, at::Tensor bias, uint64_t stream) {
+        int64_t N, H, W, N2, H2, W2;
+        int C, C2;
+        nhwc_dims(z, &N, &H, &W, &C);
+        nhwc_dims(p, &N2, &H2, &W2, &C2);
+        BAGUA_CHECK(N2 == N && C2 == C && H2 * 2 == H && W2 * 2 == W && p.device() == z.device(), Tensor,
+                    "the pooled output must be [N, C, H/2, W/2] on the convolution output's device");
+        check_bias(bias, z, C);
+        if (z.is_cuda())
+          model_ops::bias_relu_pool_only_bf16(z.data_ptr(), p.data_ptr(), bias.data_ptr(), N, H, W, C, (cudaStream_t)stream);
+        else
+          model_ops::bias_relu_pool_only_bf16_host(z.data_ptr(), p.data_ptr(), bias.data_ptr(), N, H, W, C);
+      },
+      py::arg("conv_output"), py::arg("pooled"), py::arg("bias"), py::arg("stream"),
+      "pooled = 2x2 / stride-2 maximum of max(conv_output + bias, 0); conv_output is only read.");
+  m.def(
       "k_bias_relu_pool_backward",
-      [nhwc_dims](at::Tensor dp, at::Tensor y, at::Tensor dz, at::Tensor db, uint64_t stream) {
+      [nhwc_dims](at::Tensor dp, at::Tensor y, at::Tensor dz, at::Tensor db, uint64_t stream,
+                  const std::optional<at::Tensor>& bias) {
         int64_t N, H, W, N2, H2, W2, N3, H3, W3;
         int C, C2, C3;
         nhwc_dims(y, &N, &H, &W, &C);
@@ -794,19 +814,24 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         BAGUA_CHECK(dp.device() == y.device() && dz.device() == y.device() && db.device() == y.device() &&
                         db.scalar_type() == at::kFloat && db.is_contiguous() && db.numel() == C,
                     Tensor, "db must be a contiguous fp32 vector with one entry per channel; all tensors on one device");
+        if (bias) check_bias(*bias, y, C);
         if (!y.is_cuda()) {
-          model_ops::bias_relu_pool_backward_bf16_host(dp.data_ptr(), y.data_ptr(), dz.data_ptr(), (float*)db.data_ptr(), N, H,
-                                                       W, C);
+          at::Tensor act = bias ? y.clone() : y;
+          if (bias) model_ops::bias_relu_inplace_bf16_host(act.data_ptr(), bias->data_ptr(), N * H * W, C);
+          model_ops::bias_relu_pool_backward_bf16_host(dp.data_ptr(), act.data_ptr(), dz.data_ptr(), (float*)db.data_ptr(), N,
+                                                       H, W, C);
           return;
         }
         const size_t need = model_ops::bias_relu_backward_scratch_bytes(N * (H / 2) * (W / 2), C);
         BAGUA_CHECK(need > 0, Tensor, "fused bias+ReLU+pool backward: unsupported shape");
         auto scratch = PoolRawTensor::allocate((int)y.device().index(), DType::U8, (int64_t)need, stream);
-        model_ops::bias_relu_pool_backward_bf16(dp.data_ptr(), y.data_ptr(), dz.data_ptr(), (float*)db.data_ptr(), N, H, W, C,
-                                                scratch->data_ptr(), (cudaStream_t)stream);
+        model_ops::bias_relu_pool_backward_bf16(dp.data_ptr(), y.data_ptr(), bias ? bias->data_ptr() : nullptr, dz.data_ptr(),
+                                                (float*)db.data_ptr(), N, H, W, C, scratch->data_ptr(), (cudaStream_t)stream);
       },
       py::arg("grad_pooled"), py::arg("output"), py::arg("grad_pre_activation"), py::arg("grad_bias"), py::arg("stream"),
-      "Backward of k_bias_relu_pool_: routes grad_pooled to each window's first maximum where it is positive.");
+      py::arg("bias") = py::none(),
+      "Backward of k_bias_relu_pool_ (`output` is the activation) or, with `bias`, of k_bias_relu_pool (`output` is the "
+      "convolution output): routes grad_pooled to each window's first maximum where it is positive.");
 
   // ---- single-GPU emulation of the fused kernels (all ranks in one cooperative launch) ----
   py::class_<fused::EmulatedArena>(m, "EmulatedArena")

@@ -31,8 +31,11 @@ __global__ void __launch_bounds__(kThreads)
   __shared__ float s_acc[kThreads * 8];
   bias_relu_backward_body(dy, y, dz, partial, rows, cgroups, s_acc);
 }
-__global__ void bias_grad_finish_kernel(const float* __restrict__ partial, float* __restrict__ db, int blocks, int C) {
-  bias_grad_finish_body(partial, db, blocks, C);
+constexpr int kFoldCols = 32, kFoldRows = 32;
+__global__ void __launch_bounds__(kFoldCols * kFoldRows)
+    bias_grad_finish_kernel(const float* __restrict__ partial, float* __restrict__ db, int blocks, int C) {
+  __shared__ float s_acc[kFoldCols * kFoldRows];
+  bias_grad_finish_body(partial, db, blocks, C, s_acc);
 }
 __global__ void __launch_bounds__(kThreads)
     maxpool2x2_forward_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, int64_t nvec_out, int64_t Wo,
@@ -51,10 +54,22 @@ __global__ void __launch_bounds__(kThreads)
   bias_relu_pool_body(y, p, bias, pooled_pixels, Wo, W, cgroups);
 }
 __global__ void __launch_bounds__(kThreads)
+    bias_relu_pool_only_kernel(const uint4* __restrict__ z, uint4* __restrict__ p, const __nv_bfloat16* __restrict__ bias,
+                               int64_t pooled_pixels, int64_t Wo, int64_t W, int cgroups) {
+  bias_relu_pool_only_body(z, p, bias, pooled_pixels, Wo, W, cgroups);
+}
+template <bool kFromZ>
+__global__ void __launch_bounds__(kThreads)
     bias_relu_pool_backward_kernel(const uint4* __restrict__ dp, const uint4* __restrict__ y, uint4* __restrict__ dz,
-                                   float* __restrict__ partial, int64_t pooled_rows, int64_t Wo, int64_t W, int cgroups) {
+                                   float* __restrict__ partial, int64_t pooled_rows, int64_t Wo, int64_t W, int cgroups,
+                                   const __nv_bfloat16* __restrict__ bias) {
   __shared__ float s_acc[kThreads * 8];
-  bias_relu_pool_backward_body(dp, y, dz, partial, pooled_rows, Wo, W, cgroups, s_acc);
+  bias_relu_pool_backward_body<kFromZ>(dp, y, dz, partial, pooled_rows, Wo, W, cgroups, s_acc, bias);
+}
+
+void fold_partials(const float* partial, float* db, int blocks, int C, cudaStream_t stream) {
+  bias_grad_finish_kernel<<<(C + kFoldCols - 1) / kFoldCols, dim3(kFoldCols, kFoldRows), 0, stream>>>(partial, db, blocks, C);
+  BAGUA_CUDA_CHECK(cudaGetLastError());
 }
 
 int pool_grid(int64_t nvec_out) {
@@ -96,8 +111,7 @@ void bias_relu_backward_bf16(const void* dy, const void* y, void* dz, float* db,
   bias_relu_backward_kernel<<<blocks, kThreads, 0, stream>>>((const uint4*)dy, (const uint4*)y, (uint4*)dz,
                                                              (float*)scratch, rows, C / 8);
   BAGUA_CUDA_CHECK(cudaGetLastError());
-  bias_grad_finish_kernel<<<(C + 127) / 128, 128, 0, stream>>>((const float*)scratch, db, blocks, C);
-  BAGUA_CUDA_CHECK(cudaGetLastError());
+  fold_partials((const float*)scratch, db, blocks, C, stream);
 }
 
 void maxpool2x2_forward_bf16(const void* x, void* y, int64_t N, int64_t H, int64_t W, int C, cudaStream_t stream) {
@@ -134,8 +148,21 @@ void bias_relu_pool_bf16(void* y, void* p, const void* bias, int64_t N, int64_t 
   BAGUA_CUDA_CHECK(cudaGetLastError());
 }
 
-void bias_relu_pool_backward_bf16(const void* dp, const void* y, void* dz, float* db, int64_t N, int64_t H, int64_t W,
-                                  int C, void* scratch, cudaStream_t stream) {
+void bias_relu_pool_only_bf16(const void* z, void* p, const void* bias, int64_t N, int64_t H, int64_t W, int C,
+                              cudaStream_t stream) {
+  BAGUA_CHECK(bias_relu_supported(N * H * W, C) && maxpool2x2_supported(N, H, W, C) && (uintptr_t)z % 16 == 0 &&
+                  (uintptr_t)p % 16 == 0,
+              Tensor,
+              "fused bias+ReLU+pool: unsupported shape [" << N << ", " << H << ", " << W << ", " << C
+                                                          << "] or unaligned buffers");
+  const int64_t pooled_pixels = N * (H / 2) * (W / 2);
+  bias_relu_pool_only_kernel<<<pool_grid(pooled_pixels * (C / 8)), kThreads, 0, stream>>>(
+      (const uint4*)z, (uint4*)p, (const __nv_bfloat16*)bias, pooled_pixels, W / 2, W, C / 8);
+  BAGUA_CUDA_CHECK(cudaGetLastError());
+}
+
+void bias_relu_pool_backward_bf16(const void* dp, const void* y, const void* bias, void* dz, float* db, int64_t N,
+                                  int64_t H, int64_t W, int C, void* scratch, cudaStream_t stream) {
   BAGUA_CHECK(bias_relu_supported(N * H * W, C) && maxpool2x2_supported(N, H, W, C) && (uintptr_t)dp % 16 == 0 &&
                   (uintptr_t)y % 16 == 0 && (uintptr_t)dz % 16 == 0 && scratch != nullptr,
               Tensor,
@@ -143,11 +170,11 @@ void bias_relu_pool_backward_bf16(const void* dp, const void* y, void* dz, float
                                                                    << "] or unaligned buffers");
   const int64_t pooled_rows = N * (H / 2) * (W / 2);
   const int blocks = backward_blocks(pooled_rows, C);
-  bias_relu_pool_backward_kernel<<<blocks, kThreads, 0, stream>>>((const uint4*)dp, (const uint4*)y, (uint4*)dz,
-                                                                  (float*)scratch, pooled_rows, W / 2, W, C / 8);
+  auto* kernel = bias ? bias_relu_pool_backward_kernel<true> : bias_relu_pool_backward_kernel<false>;
+  kernel<<<blocks, kThreads, 0, stream>>>((const uint4*)dp, (const uint4*)y, (uint4*)dz, (float*)scratch, pooled_rows,
+                                          W / 2, W, C / 8, (const __nv_bfloat16*)bias);
   BAGUA_CUDA_CHECK(cudaGetLastError());
-  bias_grad_finish_kernel<<<(C + 127) / 128, 128, 0, stream>>>((const float*)scratch, db, blocks, C);
-  BAGUA_CUDA_CHECK(cudaGetLastError());
+  fold_partials((const float*)scratch, db, blocks, C, stream);
 }
 
 }  // namespace model_ops

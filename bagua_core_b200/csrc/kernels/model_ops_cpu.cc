@@ -110,6 +110,12 @@ void bias_relu_pool_bf16_host(void* y, void* p, const void* bias, int64_t N, int
   maxpool2x2_forward_bf16_host(y, p, N, H, W, C);
 }
 
+void bias_relu_pool_only_bf16_host(const void* z, void* p, const void* bias, int64_t N, int64_t H, int64_t W, int C) {
+  const uint16_t* in = static_cast<const uint16_t*>(z);
+  std::vector<uint16_t> y(in, in + (size_t)(N * H * W * C));
+  bias_relu_pool_bf16_host(y.data(), p, bias, N, H, W, C);
+}
+
 void bias_relu_pool_backward_bf16_host(const void* dp, const void* y, void* dz, float* db, int64_t N, int64_t H,
                                        int64_t W, int C) {
   std::vector<uint16_t> dy((size_t)(N * H * W * C));

@@ -87,8 +87,9 @@ class _ConvBiasReLUFn(torch.autograd.Function):
 
 
 class _ConvBiasReLUPoolFn(torch.autograd.Function):
-    """conv → bias + ReLU → 2x2 max pooling; the full-resolution activation is kept only for the
-    backward, which produces the convolution's output gradient and the bias gradient in one pass."""
+    """conv → bias + ReLU → 2x2 max pooling.  The full-resolution activation is never written: the
+    backward, which produces the convolution's output gradient and the bias gradient in one pass,
+    makes it again from the convolution's output and the bias."""
 
     @staticmethod
     def forward(ctx, x, weight, bias, stride, padding, dilation, groups):
@@ -101,19 +102,20 @@ class _ConvBiasReLUPoolFn(torch.autograd.Function):
             y = y.contiguous(memory_format=torch.channels_last)
         n, c, h, w = y.shape
         p = torch.empty((n, c, h // 2, w // 2), dtype=y.dtype, device=y.device, memory_format=torch.channels_last)
-        _C.k_bias_relu_pool_(y, p, bias.contiguous(), _stream(y))
+        bias = bias.contiguous()
+        _C.k_bias_relu_pool(y, p, bias, _stream(y))
         _count(1)
-        ctx.save_for_backward(x, weight, y)
+        ctx.save_for_backward(x, weight, y, bias)
         return p
 
     @staticmethod
     def backward(ctx, dp):
         stride, padding, dilation, groups = ctx.conf
-        x, weight, y = ctx.saved_tensors
+        x, weight, y, bias = ctx.saved_tensors
         dp = dp.contiguous(memory_format=torch.channels_last)
         dz = torch.empty_like(y)
         db = torch.empty(weight.shape[0], dtype=torch.float32, device=y.device)
-        _C.k_bias_relu_pool_backward(dp, y, dz, db, _stream(y))
+        _C.k_bias_relu_pool_backward(dp, y, dz, db, _stream(y), bias)
         _count(2)
         with torch.autocast(y.device.type, enabled=False):
             dx, dw, _ = torch.ops.aten.convolution_backward(

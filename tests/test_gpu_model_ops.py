@@ -344,3 +344,28 @@ def test_vgg_training_with_in_place_weight_gradients_agrees_with_the_ordinary_pa
     assert results[0][2] == 0 and results[1][2] == 4 * 3  # three linear layers, four steps
     assert all(abs(a - b) < 5e-2 for a, b in zip(results[0][0], results[1][0])), (results[0][0], results[1][0])
     assert (results[0][1] - results[1][1]).abs().max().item() < 2e-2
+
+
+@pytest.mark.parametrize("shape", [(1, 8, 2, 2), (3, 2048, 4, 6), (2, 64, 6, 10), (5, 16, 14, 2), (8, 64, 56, 56)])
+def test_pooling_without_the_activation_equals_the_in_place_pair(shape):
+    """Values on a coarse grid (ties in most windows), negative biases (windows without a positive value), -0."""
+    import bagua_core_b200 as bb
+
+    n, c, h, w = shape
+    g = torch.Generator().manual_seed(sum(shape))
+
+    def rnd(*s):
+        t = ((torch.randn(*s, generator=g) * 4).round() / 4).to(torch.bfloat16).cuda()
+        return t.contiguous(memory_format=torch.channels_last) if len(s) == 4 else t
+
+    z, bias, dp = rnd(*shape), rnd(c) - 0.25, rnd(n, c, h // 2, w // 2)
+    z[:, :, 0, 0] = -0.0
+    bias[0] = -0.0
+    y, z0 = z.clone(), z.clone()
+    p, dz, db = torch.empty_like(dp), torch.empty_like(z), torch.empty(c, device="cuda")
+    bb._C.k_bias_relu_pool_(y, p, bias, _stream())
+    bb._C.k_bias_relu_pool_backward(dp, y, dz, db, _stream())
+    p2, dz2, db2 = torch.full_like(p, 9), torch.full_like(z, 9), torch.empty_like(db)
+    bb._C.k_bias_relu_pool(z, p2, bias, _stream())
+    bb._C.k_bias_relu_pool_backward(dp, z, dz2, db2, _stream(), bias)
+    assert torch.equal(z, z0) and torch.equal(p, p2) and torch.equal(dz, dz2) and torch.equal(db, db2)
