@@ -275,7 +275,9 @@ void reduce_chunk_inplace(void* x, DType dt, int64_t chunk, int n_chunks, int ta
   c.is_cuda() ? cuda::reduce_chunk_inplace(x, dt, chunk, n_chunks, target, average, c.stream)
               : cpu::reduce_chunk_inplace(x, dt, chunk, n_chunks, target, average);
 }
-size_t compress_scratch_bytes(int n_chunks, int64_t chunk_size) { return cuda::compress_scratch_bytes(n_chunks, chunk_size); }
+size_t compress_scratch_bytes(int n_chunks, int64_t chunk_size, DType dt) {
+  return cuda::compress_scratch_bytes(n_chunks, chunk_size, dt);
+}
 
 void compress_minmax_u8(const void* in, DType dt, int64_t num_real, int64_t chunk, int n_chunks, uint8_t* out,
                         size_t out_bytes, int target, void* scratch, size_t scratch_bytes, const Ctx& c) {

@@ -60,8 +60,10 @@ void reduce_chunk_inplace(void* x, DType dt, int64_t chunk_size, int num_chunks,
 constexpr int kCompressHeaderBytes = 32;
 size_t compressed_buffer_size(int n_chunks, int64_t chunk_size, DType dt);
 
-// Scratch needed by the CUDA path of compress (per-block partial min/max); 0 on the host.
-size_t compress_scratch_bytes(int n_chunks, int64_t chunk_size);
+// Scratch needed by the CUDA path of compress (slots through which the blocks of a chunk agree on its min
+// and max): memory that was zero once and that only this path has written since.  0 for chunks that
+// one block handles alone.
+size_t compress_scratch_bytes(int n_chunks, int64_t chunk_size, DType dt);
 
 // Quantise `in` (n_chunks*chunk_size allocated elements, of which `num_real` are real
 // data; min/max of a chunk are taken over its real elements only, an all-padding chunk

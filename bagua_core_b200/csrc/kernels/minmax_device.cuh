@@ -41,12 +41,17 @@ __device__ __forceinline__ Grid make_grid(float mn, float mx) {
   return g;
 }
 
-__device__ __forceinline__ uint8_t quantise(float x, const Grid& g) {
+__device__ __forceinline__ float quantise_level(float x, const Grid& g) {
   float level = rintf(x * g.scale);
   level = fminf(level, g.upper);
   float r = level - g.lower;
-  r = fminf(fmaxf(r, 0.f), 255.f);
-  return (uint8_t)r;
+  return fminf(fmaxf(r, 0.f), 255.f);
+}
+__device__ __forceinline__ uint8_t quantise(float x, const Grid& g) { return (uint8_t)quantise_level(x, g); }
+// The same byte in bits 0-7 of 0x4b0000xx: a whole number below 2^23 added to 2^23 is the low bits of the
+// sum, one addition where the conversion to an integer runs at a quarter of its rate.
+__device__ __forceinline__ uint32_t quantise_bits(float x, const Grid& g) {
+  return __float_as_uint(quantise_level(x, g) + 8388608.f);
 }
 __device__ __forceinline__ float dequantise(uint8_t q, const Grid& g) { return ((float)q + g.lower) / g.scale; }
 
@@ -227,8 +232,9 @@ __device__ __forceinline__ void store_vec(__nv_bfloat16* base, int64_t vec, cons
 }
 // quantised bytes of vector `vec` (payload pointer q must be 8-byte aligned)
 __device__ __forceinline__ uint32_t pack_q4(const float* f, const Grid& g) {
-  return (uint32_t)quantise(f[0], g) | ((uint32_t)quantise(f[1], g) << 8) | ((uint32_t)quantise(f[2], g) << 16) |
-         ((uint32_t)quantise(f[3], g) << 24);
+  const uint32_t b0 = quantise_bits(f[0], g), b1 = quantise_bits(f[1], g), b2 = quantise_bits(f[2], g),
+                 b3 = quantise_bits(f[3], g);
+  return (b0 & 0xffu) | (b1 << 8) | (b2 << 16) | (b3 << 24);
 }
 __device__ __forceinline__ uint32_t pack_qvec(const float (&f)[4], const Grid& g) { return pack_q4(f, g); }
 __device__ __forceinline__ uint2 pack_qvec(const float (&f)[8], const Grid& g) {

@@ -1,23 +1,34 @@
 // MinMaxUInt8 compression for sm_100a: per-chunk min/max, quantise, dequantise.
 //
-// Two launches per compress call regardless of the number of chunks: (1) every block
-// reduces a slice of one chunk to a partial {min,max} in scratch; (2) every block first
-// folds the partials of its chunk (they sit in L2), derives the grid, and quantises its
-// slice with 16-byte loads and stores.  No atomics, no initialisation of scratch, and
-// deterministic.  The reference issues two CUB DeviceReduce calls per chunk from a host
-// loop (bagua-core-internal/kernels/bagua_kernels.cu:312-371,533-560) and quantises one
-// byte per thread (455-479).
+// One launch per compress call, whatever the number of chunks.  A chunk belongs to a set of blocks that
+// are resident together: each reads its slice once, the set agrees on the chunk's min and max through
+// slots in global memory, and each quantises its slice.  The last 64 KiB that a block has read stay in its
+// registers between the two passes, so up to 19 MB (two blocks of 512 threads on each of 148 SMs) the
+// input is read once; beyond that chunks are taken a group at a time, a group being what fits L2, and the
+// second pass runs backwards over what L2 still holds.
 //
-// Numerics are the reference's anchored grid (see MinMaxGrid in kernels.h); the header
-// is stored in the tensor dtype and the grid is derived from the stored (rounded) values
-// on both sides.
+// Measured (kernel time; before: two launches with two full reads of the input): 16 KB of fp32 3.5 us (5.0),
+// 10 MB in 8 chunks 6.9 us (8.2), 134 MB in 8 chunks 41 us (54), 411 MB in 8 chunks 114 us (159; 78 at the
+// copy bandwidth), 206 MB of fp16 in 8 chunks 77 us (123), 1 M fp16 in 3 odd chunks 7.5 us (7.5, with
+// dequantising 3.4 us instead of 6.7).  Small calls are bound by latency (launch, one read, the exchange);
+// large ones by instructions and L2, a group's second read being served by L2 only in part.
+//
+// The reference issues two CUB DeviceReduce calls per chunk from a host loop
+// (bagua-core-internal/kernels/bagua_kernels.cu:312-371,533-560) and quantises one byte per thread
+// (455-479).
+//
+// Numerics are the reference's anchored grid (see MinMaxGrid in kernels.h); the header is stored in
+// the tensor dtype and the grid is derived from the stored (rounded) values on both sides.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <atomic>
 #include <cfloat>
 
 #include "kernels_impl.h"
+#include "launch.cuh"
 #include "minmax_device.cuh"
 
 namespace bagua {
@@ -26,137 +37,446 @@ namespace cuda {
 
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int kMaxBlocksPerChunk = 1024;
+using mmdev::from_f;
+using mmdev::to_f;
 
-inline int blocks_per_chunk(int n_chunks, int64_t chunk) {
-  // ~16 KiB of elements per block, at most ~8 blocks per SM over the whole launch
-  int64_t want = (chunk + 4095) / 4096;
-  int64_t cap = std::max<int64_t>(1, (148 * 8) / std::max(1, n_chunks));
-  int64_t b = std::min<int64_t>(std::min<int64_t>(want, cap), kMaxBlocksPerChunk);
-  return (int)std::max<int64_t>(b, 1);
+// ---- vectors at any alignment --------------------------------------------------------------
+// A vector is VE elements (16 bytes of T) and their VE quantised bytes.  Both sides are aligned in
+// buffers that were padded for it; elsewhere a chunk's payload and its elements start anywhere.
+
+// VE elements of T from a pointer that is only element-aligned: whole words where it is word-aligned,
+// else the words around it shifted by two bytes.
+template <bool kAligned, typename T>
+__device__ __forceinline__ uint4 load_elems(const T* p) {
+  if constexpr (kAligned) return *reinterpret_cast<const uint4*>(p);
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+  if ((a & 15u) == 0) return *reinterpret_cast<const uint4*>(p);
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(a & ~(uintptr_t)3);
+  if ((a & 3u) == 0) return make_uint4(w[0], w[1], w[2], w[3]);
+  // 16-bit elements at an odd element: five words cover the eight elements
+  const uint32_t w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3], w4 = w[4];
+  return make_uint4(__funnelshift_r(w0, w1, 16), __funnelshift_r(w1, w2, 16), __funnelshift_r(w2, w3, 16),
+                    __funnelshift_r(w3, w4, 16));
 }
 
-// Slice [lo, hi) of a chunk owned by block bx of nb, rounded to 16-element groups.
-__device__ __forceinline__ void block_slice(int64_t chunk, int bx, int nb, int64_t& lo, int64_t& hi) {
-  int64_t groups = (chunk + 15) / 16;
-  int64_t per = (groups + nb - 1) / nb;
-  lo = min((int64_t)bx * per * 16, chunk);
-  hi = min(lo + per * 16, chunk);
+// What is used for the last time, or not soon again, leaves L2 first: a second read of the input, and outputs
+// larger than L2.
+__device__ __forceinline__ uint64_t evict_first_policy() {
+  uint64_t policy;
+  asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+  return policy;
+}
+template <bool kAligned, typename T>
+__device__ __forceinline__ uint4 load_elems_last(const T* p, uint64_t policy) {
+  if constexpr (!kAligned) return load_elems<kAligned>(p);
+  uint4 r;
+  asm volatile("ld.global.L1::no_allocate.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
+               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+               : "l"(p), "l"(policy));
+  return r;
+}
+__device__ __forceinline__ void store_first(uint32_t* p, uint32_t w, uint64_t policy) {
+  asm volatile("st.global.L2::cache_hint.u32 [%0], %1, %2;" ::"l"(p), "r"(w), "l"(policy) : "memory");
+}
+__device__ __forceinline__ void store_first(uint2* p, uint2 w, uint64_t policy) {
+  asm volatile("st.global.L2::cache_hint.v2.u32 [%0], {%1, %2}, %3;" ::"l"(p), "r"(w.x), "r"(w.y), "l"(policy) : "memory");
+}
+__device__ __forceinline__ void store_first(uint4* p, uint4 w, uint64_t policy) {
+  asm volatile("st.global.L2::cache_hint.v4.u32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(p), "r"(w.x), "r"(w.y), "r"(w.z),
+               "r"(w.w), "l"(policy)
+               : "memory");
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads)
-    minmax_partial_kernel(const T* __restrict__ in, int64_t num_real, int64_t chunk, int first_chunk,
-                          float2* __restrict__ partial, bool vec) {
-  const int c = first_chunk + blockIdx.y;
-  int64_t real = num_real - (int64_t)c * chunk;
-  real = real < 0 ? 0 : (real > chunk ? chunk : real);
-  int64_t lo, hi;
-  block_slice(chunk, blockIdx.x, gridDim.x, lo, hi);
-  hi = min(hi, real);
-  const T* p = in + (int64_t)c * chunk;
-  float mn = FLT_MAX, mx = -FLT_MAX;
-  if (vec) {
-    // whole 16-byte vectors (consecutive lanes on consecutive vectors), then a scalar tail
-    // when `real` cuts a vector
-    constexpr int VE = mmdev::Vec16<T>::VE;
-    const int64_t full_hi = lo + ((hi > lo ? hi - lo : 0) / VE) * VE;
-#pragma unroll 4
-    for (int64_t i = lo / VE + threadIdx.x; i < full_hi / VE; i += kThreads) {
-      float v[VE];
-      mmdev::load_vec(p, i, v);
+__device__ __forceinline__ void widen(const uint4& r, float (&f)[4], const float*) {
+  f[0] = __uint_as_float(r.x);
+  f[1] = __uint_as_float(r.y);
+  f[2] = __uint_as_float(r.z);
+  f[3] = __uint_as_float(r.w);
+}
+__device__ __forceinline__ void widen(const uint4& r, float (&f)[8], const __half*) {
+  const __half2* h = reinterpret_cast<const __half2*>(&r);
 #pragma unroll
-      for (int k = 0; k < VE; ++k) {
-        mn = fminf(mn, v[k]);
-        mx = fmaxf(mx, v[k]);
+  for (int k = 0; k < 4; ++k) {
+    const float2 v = __half22float2(h[k]);
+    f[2 * k] = v.x;
+    f[2 * k + 1] = v.y;
+  }
+}
+__device__ __forceinline__ void widen(const uint4& r, float (&f)[8], const __nv_bfloat16*) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&r);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float2 v = __bfloat1622float2(h[k]);
+    f[2 * k] = v.x;
+    f[2 * k + 1] = v.y;
+  }
+}
+
+// The VE bytes at q + VE * vec, q at any address: aligned words and a byte shift.
+template <bool kAligned, int VE>
+__device__ __forceinline__ typename mmdev::QWord<VE>::type load_bytes(const uint8_t* q, int64_t vec) {
+  if constexpr (kAligned) return mmdev::load_qword<VE>(q, vec);
+  const uintptr_t a = reinterpret_cast<uintptr_t>(q) + (uintptr_t)(vec * VE);
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(a & ~(uintptr_t)3);
+  const uint32_t sh = (uint32_t)(a & 3u) * 8;
+  // the word behind the last byte is touched only when the bytes reach into it
+  if constexpr (VE == 4) {
+    const uint32_t w0 = w[0], w1 = sh ? w[1] : 0u;
+    return __funnelshift_r(w0, w1, sh);
+  } else {
+    const uint32_t w0 = w[0], w1 = w[1], w2 = sh ? w[2] : 0u;
+    return make_uint2(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh));
+  }
+}
+
+// ---- compress ------------------------------------------------------------------------------
+constexpr int kThreads = 512;
+constexpr int kVecs = 8;                       // vectors a thread keeps between the passes (32 registers)
+constexpr int kTile = kThreads * kVecs;        // vectors of a tile: 64 KiB
+constexpr int kBlocksPerSM = 2;                // 64 registers per thread
+constexpr int64_t kTileBytes = (int64_t)kTile * 16;
+// Smallest slice of a block: more blocks read a chunk faster but wait longer for each other (10 MB of fp32 in
+// 8 chunks: 8.1 us with 16 KiB, 6.9 with 64; unaligned elements, which take more instructions to load, 1 M of
+// fp16 in 3 chunks: 9.4 us with 64 KiB, 7.5 with 32).
+constexpr int64_t kSliceBytes = 64 << 10, kSliceBytesUnaligned = 32 << 10;
+constexpr int64_t kGroupBytes = 32ll << 20;    // two groups and their output are in L2 (126 MB) at a time
+
+// How the chunks of a call are dealt to blocks.  Calls of several groups have two sets of blocks, one of each
+// set on every SM, which take the groups in turn: while one set quantises its group, which is bound by
+// instructions (8 per element), the other reads the next from memory.
+struct Split {
+  int sets;
+  int per_group;  // chunks in flight together in a set
+  int per_chunk;  // blocks of one chunk
+  int grid() const { return sets * per_group * per_chunk; }
+};
+Split split_chunks(int count, int64_t chunk_bytes, bool aligned, int sms) {
+  Split s;
+  const int64_t all = (int64_t)sms * kBlocksPerSM;
+  s.per_group = (int)std::max<int64_t>(1, std::min({kGroupBytes / chunk_bytes, (int64_t)count, all}));
+  s.sets = s.per_group < count && chunk_bytes > kTileBytes ? 2 : 1;
+  if (s.sets == 2) s.per_group = std::min(s.per_group, sms);
+  // a chunk of one tile stays with one block, which then waits for nobody
+  s.per_chunk = chunk_bytes <= kTileBytes
+                    ? 1
+                    : (int)std::max<int64_t>(1, std::min<int64_t>(all / s.sets / s.per_group, chunk_bytes / (aligned ? kSliceBytes : kSliceBytesUnaligned)));
+  return s;
+}
+
+// How the blocks of a chunk agree: every block leaves {min, tag} and {max, tag} in a slot of its own, two
+// 8-byte words each of which says by its tag that it belongs to this launch, and thread t of every block
+// waits for slot t.  No atomics, no fences, nothing to reset: one store and one load across L2, where
+// maxima by atomics with an arrival counter took 4 us more with 296 blocks.
+// With 148 blocks that is 22 thousand waiting threads on 19 lines of L2 (4.6 us): above kDirect blocks the first
+// block collects, and the others wait for its answer (2.3 us; 16 blocks among themselves: 1.5 us).
+constexpr int kSlotBytes = 16;
+constexpr int kDirect = 24;
+inline size_t slot_bytes(int count, int per_chunk) { return (size_t)count * (per_chunk + 1) * kSlotBytes; }
+
+__device__ __forceinline__ void leave_minmax(unsigned long long* slot, float mn, float mx, uint32_t tag) {
+  const unsigned long long hi = (unsigned long long)tag << 32;
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(slot), "l"(hi | __float_as_uint(mn)),
+               "l"(hi | __float_as_uint(mx))
+               : "memory");
+}
+// False when the slot's block did not come in time (it cannot fail to under a cooperative launch).
+__device__ __forceinline__ bool wait_minmax(const unsigned long long* slot, float& mn, float& mx, uint32_t tag) {
+  for (int spins = 0; spins < (1 << 22); ++spins) {
+    unsigned long long a, b;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(slot) : "memory");
+    if ((uint32_t)(a >> 32) == tag && (uint32_t)(b >> 32) == tag) {
+      mn = __uint_as_float((uint32_t)a);
+      mx = __uint_as_float((uint32_t)b);
+      return true;
+    }
+  }
+  return false;
+}
+
+// Running min and max of whole vectors: 16-bit types two values at a time, without widening them.
+template <typename T>
+struct RunningMinMax;
+template <>
+struct RunningMinMax<float> {
+  float mn = FLT_MAX, mx = -FLT_MAX;
+  __device__ __forceinline__ void add(const uint4& r) {
+    const float f[4] = {__uint_as_float(r.x), __uint_as_float(r.y), __uint_as_float(r.z), __uint_as_float(r.w)};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      mn = fminf(mn, f[k]);
+      mx = fmaxf(mx, f[k]);
+    }
+  }
+  __device__ __forceinline__ void result(float& a, float& b) const {
+    a = mn;
+    b = mx;
+  }
+};
+template <typename T2>
+struct RunningMinMax2 {
+  T2 mn, mx;
+  __device__ __forceinline__ void add(const uint4& r) {
+    const T2* h = reinterpret_cast<const T2*>(&r);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      mn = __hmin2(mn, h[k]);
+      mx = __hmax2(mx, h[k]);
+    }
+  }
+  __device__ __forceinline__ void result(float& a, float& b) const {
+    a = fminf(to_f(mn.x), to_f(mn.y));
+    b = fmaxf(to_f(mx.x), to_f(mx.y));
+  }
+};
+template <>
+struct RunningMinMax<__half> : RunningMinMax2<__half2> {
+  __device__ RunningMinMax() {
+    mn = __floats2half2_rn(INFINITY, INFINITY);
+    mx = __floats2half2_rn(-INFINITY, -INFINITY);
+  }
+};
+template <>
+struct RunningMinMax<__nv_bfloat16> : RunningMinMax2<__nv_bfloat162> {
+  __device__ RunningMinMax() {
+    mn = __floats2bfloat162_rn(INFINITY, INFINITY);
+    mx = __floats2bfloat162_rn(-INFINITY, -INFINITY);
+  }
+};
+
+// The quantiser of one chunk.  Where every level lies well inside 2^22 (|upper| does, unless the values are
+// large against their range), x * scale is rounded to a whole number, to even at ties as rintf does, by
+// adding 1.5 * 2^23, and the byte is the difference of two bit patterns: two additions in place of a
+// rounding and a conversion that both run at a quarter of the rate.
+struct Quantiser {
+  static constexpr float kShift = 12582912.f;
+  mmdev::Grid g;
+  float lo, hi;  // lower and upper, shifted
+  bool shifted;
+  __device__ __forceinline__ explicit Quantiser(const mmdev::Grid& grid) : g(grid) {
+    shifted = fabsf(g.upper) < 4194304.f - 1024.f;
+    lo = g.lower + kShift;
+    hi = g.upper + kShift;
+  }
+  __device__ __forceinline__ uint32_t bits(float x) const {
+    const float t = fmaxf(fminf(__fadd_rn(__fmul_rn(x, g.scale), kShift), hi), lo);
+    return __float_as_uint(t) - __float_as_uint(lo);  // 0..255
+  }
+  __device__ __forceinline__ uint32_t pack4(const float* f) const {
+    if (shifted) return bits(f[0]) | (bits(f[1]) << 8) | (bits(f[2]) << 16) | (bits(f[3]) << 24);
+    return mmdev::pack_q4(f, g);
+  }
+  __device__ __forceinline__ uint32_t pack(const float (&f)[4]) const { return pack4(f); }
+  __device__ __forceinline__ uint2 pack(const float (&f)[8]) const { return make_uint2(pack4(f), pack4(f + 4)); }
+};
+
+// One tile of vectors in the registers of the block: kVecs per thread, kThreads apart.
+template <typename T, bool kAligned>
+struct Tile {
+  static constexpr int VE = mmdev::Vec16<T>::VE;
+  uint4 raw[kVecs];
+
+  // [p, p + n * VE), n <= kTile
+  __device__ __forceinline__ void load(const T* p, int n) {
+    const int tid = (int)threadIdx.x;
+    if (n == kTile) {
+#pragma unroll
+      for (int u = 0; u < kVecs; ++u) raw[u] = load_elems<kAligned>(p + (tid + u * kThreads) * VE);
+    } else {
+#pragma unroll
+      for (int u = 0; u < kVecs; ++u)
+        if (tid + u * kThreads < n) raw[u] = load_elems<kAligned>(p + (tid + u * kThreads) * VE);
+    }
+  }
+  // `real`: elements from the tile's first on that count (padding does not)
+  __device__ __forceinline__ void minmax_all(int n, int64_t real, RunningMinMax<T>& run, float& mn, float& mx) const {
+    const int tid = (int)threadIdx.x;
+#pragma unroll
+    for (int u = 0; u < kVecs; ++u) {
+      const int v = tid + u * kThreads;
+      if (v >= n) continue;
+      if (real >= (int64_t)n * VE) {
+        run.add(raw[u]);
+      } else {
+        float f[VE];
+        widen(raw[u], f, (const T*)nullptr);
+#pragma unroll
+        for (int k = 0; k < VE; ++k) {
+          if ((int64_t)v * VE + k < real) {
+            mn = fminf(mn, f[k]);
+            mx = fmaxf(mx, f[k]);
+          }
+        }
       }
     }
-    for (int64_t i = full_hi + threadIdx.x; i < hi; i += kThreads) {
-      float v = mmdev::to_f(p[i]);
-      mn = fminf(mn, v);
-      mx = fmaxf(mx, v);
+  }
+  __device__ __forceinline__ void quantise(int u, uint8_t* q, const Quantiser& g) const {
+    float f[VE];
+    widen(raw[u], f, (const T*)nullptr);
+    mmdev::store_qword(q, (int)threadIdx.x + u * kThreads, g.pack(f));
+  }
+  __device__ __forceinline__ void quantise_out(int u, uint8_t* q, const Quantiser& g, uint64_t policy) const {
+    float f[VE];
+    widen(raw[u], f, (const T*)nullptr);
+    store_first(reinterpret_cast<typename mmdev::QWord<VE>::type*>(q) + (int)threadIdx.x + u * kThreads, g.pack(f), policy);
+  }
+  __device__ __forceinline__ void quantise_all(uint8_t* q, int n, const Quantiser& g) const {
+#pragma unroll
+    for (int u = 0; u < kVecs; ++u)
+      if ((int)threadIdx.x + u * kThreads < n) quantise(u, q, g);
+  }
+};
+
+template <typename T, bool kAligned>
+__global__ void __launch_bounds__(kThreads, kBlocksPerSM)
+    compress_kernel(const T* __restrict__ in, int64_t num_real, int64_t chunk, int first_chunk, int count, int sets,
+                    int per_group, int per_chunk, uint8_t* __restrict__ out, size_t chunk_offset, unsigned long long* slots, uint32_t tag) {
+  constexpr int VE = mmdev::Vec16<T>::VE;
+  const int tid = (int)threadIdx.x;
+  const int slot = (int)blockIdx.x / per_chunk, part = (int)blockIdx.x % per_chunk;
+  wait_for_predecessor();
+  for (int ci = slot; ci < count; ci += sets * per_group) {
+    if (sets > 1 && ci >= per_group) {
+      // after the same block of the other set has read its slice of the group in front: the sets stay out of step
+      if (tid == 0) {
+        float unused_mn, unused_mx;
+        wait_minmax(slots + ((size_t)(ci - per_group) * (per_chunk + 1) + part) * 2, unused_mn, unused_mx, tag);
+      }
+      __syncthreads();
     }
-  } else {
-    for (int64_t i = lo + threadIdx.x; i < hi; i += kThreads) {
-      float v = mmdev::to_f(p[i]);
-      mn = fminf(mn, v);
-      mx = fmaxf(mx, v);
+    const int c = first_chunk + ci;
+    const T* p = in + (int64_t)c * chunk;
+    uint8_t* base = out + (size_t)c * chunk_offset;
+    uint8_t* q = base + kCompressHeaderBytes;
+    int64_t real = num_real - (int64_t)c * chunk;
+    real = real < 0 ? 0 : (real > chunk ? chunk : real);
+    // elements in front of the first vector (whose bytes start a word), whole vectors, elements behind the last
+    const int64_t head = kAligned ? 0 : min(chunk, (int64_t)((0 - reinterpret_cast<uintptr_t>(q)) & (uintptr_t)(VE - 1)));
+    const int64_t nvec = (chunk - head) / VE;
+    const int64_t tail = head + nvec * VE;
+    const int64_t per = ((nvec + per_chunk - 1) / per_chunk + 31) & ~(int64_t)31;  // slices start on 512 bytes
+    const int64_t lo = min((int64_t)part * per, nvec), n = min(lo + per, nvec) - lo;
+    const T* pv = p + head + lo * VE;
+    uint8_t* qv = q + head + lo * VE;
+    // first what is not a whole tile of real elements, then `full` whole tiles; the last tile stays in registers
+    const int64_t full = real == chunk ? n / kTile : 0;
+    const int64_t rest = n - full * kTile;
+    const T* pf = pv + rest * VE;
+    uint8_t* qf = qv + rest * VE;
+
+    // pass 1
+    float mn = FLT_MAX, mx = -FLT_MAX;
+    RunningMinMax<T> run;
+    Tile<T, kAligned> tile;
+    for (int64_t v = 0; v < rest; v += kTile) {
+      const int m = (int)min((int64_t)kTile, rest - v);
+      tile.load(pv + v * VE, m);
+      tile.minmax_all(m, real - head - (lo + v) * VE, run, mn, mx);
+    }
+    if (full > 0) {
+      tile.load(pf, kTile);
+      const T* next = pf + (int64_t)kTile * VE;
+      for (int64_t t = 1; t < full; ++t, next += (int64_t)kTile * VE) {
+        // a vector's successor is requested as soon as its registers are free: seven stay in flight
+#pragma unroll
+        for (int u = 0; u < kVecs; ++u) {
+          run.add(tile.raw[u]);
+          tile.raw[u] = load_elems<kAligned>(next + (tid + u * kThreads) * VE);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kVecs; ++u) run.add(tile.raw[u]);
+    }
+    {
+      float a, b;
+      run.result(a, b);
+      mn = fminf(mn, a);
+      mx = fmaxf(mx, b);
+    }
+    if constexpr (!kAligned) {
+      if (part == 0 && tid < head && tid < real) {
+        const float f = to_f(p[tid]);
+        mn = fminf(mn, f);
+        mx = fmaxf(mx, f);
+      }
+      if (part == per_chunk - 1 && tail + tid < chunk && tail + tid < real) {
+        const float f = to_f(p[tail + tid]);
+        mn = fminf(mn, f);
+        mx = fmaxf(mx, f);
+      }
+    }
+    mmdev::block_minmax<kThreads>(mn, mx);
+    if (per_chunk > 1 || sets > 1) {
+      unsigned long long* mine = slots + (size_t)ci * (per_chunk + 1) * 2;
+      if (tid == 0) leave_minmax(mine + 2 * part, mn, mx, tag);
+      bool all = true;
+      if (per_chunk <= kDirect) {
+        if (tid < per_chunk) all = wait_minmax(mine + 2 * tid, mn, mx, tag);
+      } else {
+        // many blocks: the first one collects and passes the result on
+        unsigned long long* result = mine + 2 * per_chunk;
+        if (part == 0) {
+          if (tid < per_chunk) all = wait_minmax(mine + 2 * tid, mn, mx, tag);
+          if (__syncthreads_and(all)) {
+            mmdev::block_minmax<kThreads>(mn, mx);
+            if (tid == 0) leave_minmax(result, mn, mx, tag);
+          }
+        } else if (tid == 0) {
+          all = wait_minmax(result, mn, mx, tag);
+        }
+      }
+      if (!__syncthreads_and(all)) {  // the answer is the same, only late
+        for (int64_t i = tid; i < real; i += kThreads) {
+          const float f = to_f(p[i]);
+          mn = fminf(mn, f);
+          mx = fmaxf(mx, f);
+        }
+      }
+      mmdev::block_minmax<kThreads>(mn, mx);
+    }
+    if (mn > mx) mn = mx = 0.f;  // chunk without real elements
+    if (part == 0 && tid == 0) mmdev::store_header<T>(base, mn, mx);
+    // round through the storage dtype so both sides build the same grid
+    const Quantiser g(mmdev::make_grid(to_f(from_f<T>(mn)), to_f(from_f<T>(mx))));
+
+    // pass 2: the tile in registers first, then backwards over what L2 still holds
+    if (full > 0) {
+      const uint64_t policy = evict_first_policy();
+      for (int64_t t = full - 1; t > 0; --t) {
+        const T* prev = pf + (t - 1) * (int64_t)kTile * VE;
+#pragma unroll
+        for (int u = 0; u < kVecs; ++u) {
+          if (sets > 1) {
+            tile.quantise_out(u, qf + t * (int64_t)kTile * VE, g, policy);
+            tile.raw[u] = load_elems_last<kAligned>(prev + (tid + u * kThreads) * VE, policy);
+          } else {
+            tile.quantise(u, qf + t * (int64_t)kTile * VE, g);
+            tile.raw[u] = load_elems<kAligned>(prev + (tid + u * kThreads) * VE);
+          }
+        }
+      }
+      tile.quantise_all(qf, kTile, g);
+    }
+    for (int64_t v = (rest - 1) / kTile * kTile; v >= 0 && rest > 0; v -= kTile) {
+      const int m = (int)min((int64_t)kTile, rest - v);
+      if (full > 0 || v + kTile < rest) tile.load(pv + v * VE, m);
+      tile.quantise_all(qv + v * VE, m, g);
+    }
+    if constexpr (!kAligned) {
+      if (part == 0 && tid < head) q[tid] = mmdev::quantise(to_f(p[tid]), g.g);
+      if (part == per_chunk - 1 && tail + tid < chunk) q[tail + tid] = mmdev::quantise(to_f(p[tail + tid]), g.g);
     }
   }
-  mmdev::block_minmax<kThreads>(mn, mx);
-  if (threadIdx.x == 0) partial[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = make_float2(mn, mx);
+  let_successor_start();
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads)
-    quantise_kernel(const T* __restrict__ in, int64_t chunk, int first_chunk, const float2* __restrict__ partial,
-                    int n_partial, uint8_t* __restrict__ out, size_t chunk_offset, bool vec) {
-  const int c = first_chunk + blockIdx.y;
-  // fold the partials of this chunk
-  float mn = FLT_MAX, mx = -FLT_MAX;
-  for (int i = threadIdx.x; i < n_partial; i += kThreads) {
-    float2 pm = partial[(int64_t)blockIdx.y * n_partial + i];
-    mn = fminf(mn, pm.x);
-    mx = fmaxf(mx, pm.y);
-  }
-  mmdev::block_minmax<kThreads>(mn, mx);
-  if (mn > mx) mn = mx = 0.f;  // chunk without real elements
-  uint8_t* base = out + (size_t)c * chunk_offset;
-  // round through the storage dtype so both sides build the same grid
-  const float mn_r = mmdev::to_f(mmdev::from_f<T>(mn));
-  const float mx_r = mmdev::to_f(mmdev::from_f<T>(mx));
-  if (blockIdx.x == 0 && threadIdx.x == 0) mmdev::store_header<T>(base, mn, mx);
-  const mmdev::Grid g = mmdev::make_grid(mn_r, mx_r);
-  int64_t lo, hi;
-  block_slice(chunk, blockIdx.x, gridDim.x, lo, hi);
-  const T* p = in + (int64_t)c * chunk;
-  uint8_t* q = base + kCompressHeaderBytes;
-  if (vec) {
-    constexpr int VE = mmdev::Vec16<T>::VE;
-    constexpr int U = 4;
-    const int64_t vhi = hi / VE;
-    for (int64_t i0 = lo / VE + threadIdx.x; i0 < vhi; i0 += (int64_t)U * kThreads) {
-      float v[U][VE];
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (i0 + u * kThreads < vhi) mmdev::load_vec(p, i0 + u * kThreads, v[u]);
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (i0 + u * kThreads < vhi) mmdev::store_qword(q, i0 + u * kThreads, mmdev::pack_qvec(v[u], g));
-    }
-  } else {
-    for (int64_t i = lo + threadIdx.x; i < hi; i += kThreads) q[i] = mmdev::quantise(mmdev::to_f(p[i]), g);
-  }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kThreads)
-    dequantise_kernel(const uint8_t* __restrict__ in, size_t chunk_offset, int64_t chunk, T* __restrict__ out,
-                      bool vec) {
-  const int c = blockIdx.y;
-  const uint8_t* base = in + (size_t)c * chunk_offset;
-  float mn, mx;
-  mmdev::load_header<T>(base, mn, mx);
-  const mmdev::Grid g = mmdev::make_grid(mn, mx);
-  int64_t lo, hi;
-  block_slice(chunk, blockIdx.x, gridDim.x, lo, hi);
-  const uint8_t* q = base + kCompressHeaderBytes;
-  T* o = out + (int64_t)c * chunk;
-  if (vec) {
-    constexpr int VE = mmdev::Vec16<T>::VE;
-    __shared__ float s_lut[256];
-    mmdev::build_dequant_lut<T>(s_lut, g);
-    __syncthreads();
-#pragma unroll 4
-    for (int64_t i = lo / VE + threadIdx.x; i < hi / VE; i += kThreads) {
-      float v[VE];
-      mmdev::lut_dqvec(q, i, v, s_lut);
-      mmdev::store_vec(o, i, v);
-    }
-  } else {
-    for (int64_t i = lo + threadIdx.x; i < hi; i += kThreads) o[i] = mmdev::from_f<T>(mmdev::dequantise(q[i], g));
-  }
+// A launch's tag: not that of any of the last 2^32 - 2 launches of this process, of whatever type (they share
+// slots), and not what a fresh slot holds.
+uint32_t next_tag() {
+  static std::atomic<uint32_t> launches{0};
+  uint32_t t;
+  do t = ++launches;
+  while (t == 0);
+  return t;
 }
 
 template <typename T>
@@ -165,30 +485,91 @@ void compress_t(const void* in, int64_t num_real, int64_t chunk, int n_chunks, u
   const size_t off = out_bytes / (size_t)n_chunks;
   const int first = target >= 0 ? target : 0;
   const int count = target >= 0 ? 1 : n_chunks;
-  const int bpc = blocks_per_chunk(count, chunk);
-  BAGUA_CHECK(scratch != nullptr && scratch_bytes >= (size_t)count * bpc * sizeof(float2), MemPool,
+  const bool aligned = ((uintptr_t)in % 16 == 0) && ((uintptr_t)out % 16 == 0) && (chunk % 16 == 0) && (off % 16 == 0);
+  const Split d = split_chunks(count, chunk * (int64_t)sizeof(T), aligned, sm_count());
+  auto* kernel = aligned ? compress_kernel<T, true> : compress_kernel<T, false>;
+  if (d.sets == 1 && d.per_chunk == 1) {
+    launch_overlapped(kernel, dim3(d.grid()), dim3(kThreads), s, (const T*)in, num_real, chunk, first, count, 1, d.per_group, 1,
+                      out, off, (unsigned long long*)nullptr, 0u);
+    return;
+  }
+  BAGUA_CHECK(scratch != nullptr && scratch_bytes >= slot_bytes(count, d.per_chunk), MemPool,
               "compress: scratch buffer too small");
-  const bool vec = ((uintptr_t)in % 16 == 0) && ((uintptr_t)out % 16 == 0) && (chunk % 16 == 0) && (off % 16 == 0);
-  dim3 grid(bpc, count);
-  minmax_partial_kernel<T><<<grid, kThreads, 0, s>>>((const T*)in, num_real, chunk, first, (float2*)scratch, vec);
-  BAGUA_CUDA_CHECK(cudaGetLastError());
-  quantise_kernel<T><<<grid, kThreads, 0, s>>>((const T*)in, chunk, first, (const float2*)scratch, bpc, out, off, vec);
-  BAGUA_CUDA_CHECK(cudaGetLastError());
+  const uint32_t tag = next_tag();
+  launch_cooperative(kernel, dim3(d.grid()), dim3(kThreads), s, (const T*)in, num_real, chunk, first, count, d.sets,
+                     d.per_group, d.per_chunk, out, off, (unsigned long long*)scratch, tag);
+}
+
+// ---- decompress ----------------------------------------------------------------------------
+constexpr int kDqThreads = 256;
+constexpr int kDqVecs = 8;  // quantised words in flight per thread
+
+template <typename T, bool kAligned>
+__global__ void __launch_bounds__(kDqThreads)
+    dequantise_kernel(const uint8_t* __restrict__ in, size_t chunk_offset, int64_t chunk, T* __restrict__ out) {
+  constexpr int VE = mmdev::Vec16<T>::VE;
+  __shared__ float s_lut[256];
+  const int tid = (int)threadIdx.x;
+  const int64_t c = blockIdx.y;
+  const uint8_t* base = in + (size_t)c * chunk_offset;
+  const uint8_t* q = base + kCompressHeaderBytes;
+  T* o = out + c * chunk;
+  const int64_t head =
+      kAligned ? 0 : min(chunk, (int64_t)(((0 - reinterpret_cast<uintptr_t>(o)) & (uintptr_t)15) / sizeof(T)));
+  const int64_t nvec = (chunk - head) / VE;
+  const int64_t tail = head + nvec * VE;
+  const int64_t per = ((nvec + gridDim.x - 1) / gridDim.x + 31) & ~(int64_t)31;
+  const int64_t lo = min((int64_t)blockIdx.x * per, nvec), hi = min(lo + per, nvec);
+  wait_for_predecessor();
+  float mn, mx;
+  mmdev::load_header<T>(base, mn, mx);
+  const mmdev::Grid g = mmdev::make_grid(mn, mx);
+  mmdev::build_dequant_lut<T>(s_lut, g);
+  __syncthreads();
+  const uint64_t policy = evict_first_policy();
+  typename mmdev::QWord<VE>::type w[kDqVecs];
+  for (int64_t v0 = lo + tid; v0 < hi; v0 += (int64_t)kDqVecs * kDqThreads) {
+    // all words before the first store: the compiler may not move a load over a store
+#pragma unroll
+    for (int u = 0; u < kDqVecs; ++u)
+      if (v0 + u * kDqThreads < hi) w[u] = load_bytes<kAligned, VE>(q + head, v0 + u * kDqThreads);
+#pragma unroll
+    for (int u = 0; u < kDqVecs; ++u) {
+      if (v0 + u * kDqThreads >= hi) continue;
+      float f[VE];
+      mmdev::lut_word(w[u], f, s_lut);
+      uint4 r;
+      mmdev::store_vec(reinterpret_cast<T*>(&r), 0, f);
+      store_first(reinterpret_cast<uint4*>(o + head) + v0 + u * kDqThreads, r, policy);
+    }
+  }
+  if constexpr (!kAligned) {
+    if (blockIdx.x == 0 && tid < head) o[tid] = from_f<T>(s_lut[q[tid]]);
+    if (blockIdx.x == gridDim.x - 1 && tail + tid < chunk) o[tail + tid] = from_f<T>(s_lut[q[tail + tid]]);
+  }
+  let_successor_start();
 }
 
 template <typename T>
 void decompress_t(const uint8_t* in, size_t in_bytes, int64_t chunk, int n_chunks, void* out, cudaStream_t s) {
   const size_t off = in_bytes / (size_t)n_chunks;
-  const bool vec = ((uintptr_t)in % 16 == 0) && ((uintptr_t)out % 16 == 0) && (chunk % 16 == 0) && (off % 16 == 0);
-  dim3 grid(blocks_per_chunk(n_chunks, chunk), n_chunks);
-  dequantise_kernel<T><<<grid, kThreads, 0, s>>>(in, off, chunk, (T*)out, vec);
-  BAGUA_CUDA_CHECK(cudaGetLastError());
+  const bool aligned = ((uintptr_t)in % 16 == 0) && ((uintptr_t)out % 16 == 0) && (chunk % 16 == 0) && (off % 16 == 0);
+  // a block takes at least two words per thread, and the launch at most 8 blocks per SM
+  constexpr int VE = mmdev::Vec16<T>::VE;
+  const int64_t want = (chunk / VE + kDqThreads * 2 - 1) / (kDqThreads * 2);
+  const int64_t cap = std::max<int64_t>(1, (int64_t)sm_count() * 8 / n_chunks);
+  dim3 grid((unsigned)std::max<int64_t>(1, std::min(want, cap)), (unsigned)n_chunks);
+  auto* kernel = aligned ? dequantise_kernel<T, true> : dequantise_kernel<T, false>;
+  launch_overlapped(kernel, grid, dim3(kDqThreads), s, in, off, chunk, (T*)out);
 }
 
 }  // namespace
 
-size_t compress_scratch_bytes(int n_chunks, int64_t chunk_size) {
-  return (size_t)n_chunks * (size_t)blocks_per_chunk(n_chunks, chunk_size) * sizeof(float2);
+size_t compress_scratch_bytes(int n_chunks, int64_t chunk_size, DType dt) {
+  // a call for one chunk of the buffer may give that chunk more blocks than a call for all of them
+  const int64_t bytes = chunk_size * (int64_t)dtype_bytes(dt);
+  const Split all = split_chunks(n_chunks, bytes, false, sm_count()), one = split_chunks(1, bytes, false, sm_count());
+  return bytes <= kTileBytes ? 0 : std::max(slot_bytes(n_chunks, all.per_chunk), slot_bytes(1, one.per_chunk));
 }
 
 void compress_minmax_u8(const void* in, DType dt, int64_t num_real, int64_t chunk, int n_chunks, uint8_t* out,

@@ -38,7 +38,7 @@ void log_write(LogLevel l, const char* file, int line, const std::string& msg) {
 }
 
 PoolBlock::~PoolBlock() {
-  if (pool_ && ptr_) pool_->give_back(ptr_, cls_, tag_);
+  if (pool_ && ptr_) pool_->give_back(ptr_, cls_, tag_, cleared_);
 }
 
 size_t MemoryPool::size_class(size_t bytes) {
@@ -57,14 +57,15 @@ MemoryPool& MemoryPool::for_device(int device) {
   return *p;
 }
 
-std::shared_ptr<PoolBlock> MemoryPool::pull(size_t bytes, uint64_t tag) {
+std::shared_ptr<PoolBlock> MemoryPool::pull_from(size_t bytes, uint64_t tag, bool cleared) {
   const size_t cls = size_class(bytes == 0 ? 1 : bytes);
   void* ptr = nullptr;
   {
     std::lock_guard<std::mutex> g(mu_);
     stats_.pulls++;
-    auto it = free_.find({cls, tag});
-    if (it != free_.end() && !it->second.empty()) {
+    FreeLists& lists = cleared ? free_cleared_ : free_;
+    auto it = lists.find({cls, tag});
+    if (it != lists.end() && !it->second.empty()) {
       ptr = it->second.back();
       it->second.pop_back();
     }
@@ -107,15 +108,21 @@ std::shared_ptr<PoolBlock> MemoryPool::pull(size_t bytes, uint64_t tag) {
     }
     stats_.device_allocs++;
     stats_.bytes_reserved += cls;
+    if (cleared) {
+      if (device_ >= 0)
+        BAGUA_CUDA_CHECK(cudaMemsetAsync(ptr, 0, cls, (cudaStream_t)tag));
+      else
+        std::memset(ptr, 0, cls);
+    }
   }
   {
     std::lock_guard<std::mutex> g(mu_);
     stats_.bytes_in_use += cls;
   }
-  return std::make_shared<PoolBlock>(this, ptr, bytes, cls, tag);
+  return std::make_shared<PoolBlock>(this, ptr, bytes, cls, tag, cleared);
 }
 
-void MemoryPool::give_back(void* ptr, size_t cls, uint64_t tag) {
+void MemoryPool::give_back(void* ptr, size_t cls, uint64_t tag, bool cleared) {
   std::lock_guard<std::mutex> g(mu_);
   if (device_ < 0 && guarded_.count(ptr)) {
     // host memory can be looked at right away: a block is checked every time it comes back
@@ -126,15 +133,20 @@ void MemoryPool::give_back(void* ptr, size_t cls, uint64_t tag) {
       BAGUA_LOG(Error, "host pool block of " << cls << " bytes came back with an overwritten guard region");
     }
   }
-  free_[{cls, tag}].push_back(ptr);
+  (cleared ? free_cleared_ : free_)[{cls, tag}].push_back(ptr);
   stats_.bytes_in_use -= cls;
 }
 
 void MemoryPool::release_cached() {
-  std::map<std::pair<size_t, uint64_t>, std::vector<void*>> taken;
+  FreeLists taken;
   {
     std::lock_guard<std::mutex> g(mu_);
     taken.swap(free_);
+    for (auto& kv : free_cleared_) {
+      auto& v = taken[kv.first];
+      v.insert(v.end(), kv.second.begin(), kv.second.end());
+    }
+    free_cleared_.clear();
     for (auto& kv : taken) {
       stats_.bytes_reserved -= kv.first.first * kv.second.size();
       for (void*& p : kv.second)

@@ -30,8 +30,8 @@ class MemoryPool;
 // RAII lease of a pooled block.
 class PoolBlock {
  public:
-  PoolBlock(MemoryPool* pool, void* ptr, size_t bytes, size_t cls, uint64_t tag)
-      : pool_(pool), ptr_(ptr), bytes_(bytes), cls_(cls), tag_(tag) {}
+  PoolBlock(MemoryPool* pool, void* ptr, size_t bytes, size_t cls, uint64_t tag, bool cleared)
+      : pool_(pool), ptr_(ptr), bytes_(bytes), cls_(cls), tag_(tag), cleared_(cleared) {}
   ~PoolBlock();
   PoolBlock(const PoolBlock&) = delete;
   PoolBlock& operator=(const PoolBlock&) = delete;
@@ -44,6 +44,7 @@ class PoolBlock {
   void* ptr_;
   size_t bytes_, cls_;
   uint64_t tag_;
+  bool cleared_;
 };
 
 struct PoolStats {
@@ -66,7 +67,10 @@ class MemoryPool {
   // stream the block will be used on: a freed block is only handed to a later pull with
   // the same tag, so reuse is always ordered by that stream (no host synchronisation
   // is needed before a lease is dropped).
-  std::shared_ptr<PoolBlock> pull(size_t bytes, uint64_t stream_tag = 0);
+  std::shared_ptr<PoolBlock> pull(size_t bytes, uint64_t stream_tag = 0) { return pull_from(bytes, stream_tag, false); }
+  // A block that is cleared once, when it is allocated, in the order of the stream `stream_tag`, and never
+  // handed out by `pull`: for kernels that recognise their own words in it by a tag, or put the zeros back.
+  std::shared_ptr<PoolBlock> pull_cleared(size_t bytes, uint64_t stream_tag = 0) { return pull_from(bytes, stream_tag, true); }
   void release_cached();  // returns free blocks to the device
   PoolStats stats() const;
   int device() const { return device_; }
@@ -88,11 +92,14 @@ class MemoryPool {
 
  private:
   friend class PoolBlock;
-  void give_back(void* ptr, size_t cls, uint64_t tag);
+  std::shared_ptr<PoolBlock> pull_from(size_t bytes, uint64_t tag, bool cleared);
+  void give_back(void* ptr, size_t cls, uint64_t tag, bool cleared);
+
+  using FreeLists = std::map<std::pair<size_t, uint64_t>, std::vector<void*>>;
 
   const int device_;
   mutable std::mutex mu_;
-  std::map<std::pair<size_t, uint64_t>, std::vector<void*>> free_;
+  FreeLists free_, free_cleared_;
   std::map<void*, size_t> guarded_;  // block -> capacity, for blocks that have guard regions
   std::set<void*> reported_;         // guarded blocks already reported as damaged
   PoolStats stats_;

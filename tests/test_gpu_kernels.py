@@ -349,3 +349,46 @@ def test_bucket_time_line_records_one_span_per_bucket_and_the_marks():
     assert spans[1]["end_ms"] <= spans[2]["start_ms"] + 1e-3 and spans[2]["end_ms"] <= spans[3]["start_ms"] + 1e-3
     assert bb._C.timeline_collect() == []
     backend.close()
+
+
+@pytest.mark.parametrize("n_chunks,chunk,jump", [
+    (1, 1, 1), (1, 7, 7), (5, 33, 165), (2, 16384, 32768), (3, 16385, 49155), (1, 262147, 262147), (4, 65536, 200001),
+    (8, 327680, 2621440), (3, 349527, 1048581), (2, 1 << 20, 1 << 20), (12, 1 << 20, (12 << 20) - 5), (2, 9000001, 18000002)])
+@pytest.mark.parametrize("dt", DTYPES)
+def test_minmax_uint8_splits_of_a_chunk_match_the_host(n_chunks, chunk, jump, dt):
+    """Chunks of one block and of many, of one group and of several (two sets of blocks), odd sizes and offsets;
+    from element `jump` on the values are far from the rest, so that a block with the wrong range shows."""
+    import bagua_core as bc
+
+    x = _rand(n_chunks * chunk, dt, 31) * 0.1
+    x[jump:] = 1e3
+    g = bc.BaguaTensorPy(x, "x").compress("MinMaxUInt8", n_chunks, -1)
+    c = bc.BaguaTensorPy(x.cpu(), "x").compress("MinMaxUInt8", n_chunks, -1)
+    back, back_cpu = torch.empty_like(x), torch.empty_like(x, device="cpu")
+    bc.BaguaTensorPy(back, "o").decompress_from("MinMaxUInt8", n_chunks, g)
+    bc.BaguaTensorPy(back_cpu, "o").decompress_from("MinMaxUInt8", n_chunks, c)
+    a, b = g.to_numpy_u8(), c.to_numpy_u8()
+    off = a.shape[0] // n_chunks
+    for i in range(n_chunks):
+        esz = x.element_size()
+        assert (a[i * off:i * off + 2 * esz] == b[i * off:i * off + 2 * esz]).all(), i
+        pa, pb = a[i * off + 32:i * off + 32 + chunk].astype(int), b[i * off + 32:i * off + 32 + chunk].astype(int)
+        assert abs(pa - pb).max() <= 1 and (pa != pb).mean() < 0.01, i
+    step = (x.float().view(n_chunks, chunk).amax(1) - x.float().view(n_chunks, chunk).amin(1)) / 255
+    err = (back.cpu().float() - back_cpu.float()).view(n_chunks, chunk).abs().amax(1)
+    assert (err <= step.cpu() * 1.01 + _tol(dt) * x.float().abs().max().item()).all()
+
+
+def test_minmax_uint8_values_large_against_their_range_and_not_finite():
+    """Levels beyond 2^22 (a narrow range far from zero), NaN and infinities: the same bytes as the host."""
+    import bagua_core as bc
+
+    g = torch.Generator().manual_seed(3)
+    for x in (1000.0 + 1e-3 * torch.rand(200000, generator=g), -50.0 + 1e-6 * torch.rand(70001, generator=g)):
+        a = bc.BaguaTensorPy(x.cuda(), "x").compress("MinMaxUInt8", 1, -1).to_numpy_u8().astype(int)
+        b = bc.BaguaTensorPy(x, "x").compress("MinMaxUInt8", 1, -1).to_numpy_u8().astype(int)
+        assert abs(a[:32 + x.numel()] - b[:32 + x.numel()])[list(range(8)) + list(range(32, 32 + x.numel()))].max() <= 1
+    x = torch.randn(100000, generator=g)
+    x[[5, 70000]] = float("nan")
+    a = bc.BaguaTensorPy(x.cuda(), "x").compress("MinMaxUInt8", 1, -1).to_numpy_u8()
+    assert a[32 + 5] == 255 and a[32 + 70000] == 255  # NaN takes the highest level
