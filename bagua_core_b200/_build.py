@@ -36,6 +36,8 @@ SOURCES = [
     "comm/solo_transport.cc",
     "ops/ops.cc",
     "telemetry/telemetry.cc",
+    "trainer/autograd_ops.cc",
+    "trainer/grad_hooks.cc",
     "capi/capi.cc",
     "kernels/cpu_kernels.cc",
     "kernels/elementwise.cu",

@@ -25,6 +25,8 @@
 #include "runtime/timeline.h"
 #include "telemetry/telemetry.h"
 #include "tensor/tensor.h"
+#include "trainer/autograd_ops.h"
+#include "trainer/grad_hooks.h"
 
 namespace py = pybind11;
 using namespace bagua;
@@ -78,7 +80,7 @@ struct PyComm {
   SingleCommPtr inner;
 };
 struct PyBackend {
-  std::unique_ptr<CommBackend> inner;
+  std::shared_ptr<CommBackend> inner;
 };
 
 SingleCommPtr opt_comm(const py::object& o) { return o.is_none() ? nullptr : o.cast<PyComm&>().inner; }
@@ -432,7 +434,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   // -------------------------------------------------------------------------------
   py::class_<PyBackend>(m, "BaguaCommBackendPy", py::dynamic_attr())
       .def(py::init([](size_t cap, int device_id) {
-             return PyBackend{std::make_unique<CommBackend>(cap, device_id)};
+             return PyBackend{std::make_shared<CommBackend>(cap, device_id)};
            }),
            py::arg("schedule_channel_cap"), py::arg("device_id"))
       .def("register_ordered_buckets",
@@ -832,6 +834,38 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       py::arg("bias") = py::none(),
       "Backward of k_bias_relu_pool_ (`output` is the activation) or, with `bias`, of k_bias_relu_pool (`output` is the "
       "convolution output): routes grad_pooled to each window's first maximum where it is positive.");
+
+  // ---- trainer: autograd functions and gradient hooks ---------------------------------
+  m.def("linear", &trainer::linear, py::arg("x"), py::arg("weight"), py::arg("bias"), py::arg("weight_bf16"),
+        py::arg("accumulate"),
+        "x @ weight.T + bias in bf16; with `accumulate`, the backward adds the parameters' gradients to their fp32 .grad "
+        "itself where that changes nothing a user sees.");
+  m.def("conv_bias_relu", &trainer::conv_bias_relu, py::arg("x"), py::arg("weight"), py::arg("bias"), py::arg("stride"),
+        py::arg("padding"), py::arg("dilation"), py::arg("groups"), py::arg("pool"), py::arg("weight_bf16"),
+        py::arg("accumulate"), "max(conv(x, weight) + bias, 0), followed by 2x2 pooling with `pool`.");
+  m.def("op_stats", []() {
+    auto& s = trainer::OpStats::global();
+    py::dict d;
+    d["accumulated"] = s.accumulated.load();
+    d["declined"] = s.declined.load();
+    d["launches"] = s.launches.load();
+    static const char* modes[] = {"", "addmm", "mm_add", "off"};
+    d["gemm_mode"] = modes[s.gemm_mode.load()];
+    return d;
+  });
+  py::class_<trainer::GradHooks, std::shared_ptr<trainer::GradHooks>>(m, "GradHooks")
+      .def(py::init([](PyBackend& be, int device) { return std::make_shared<trainer::GradHooks>(be.inner, device); }),
+           py::arg("backend"), py::arg("device"))
+      .def("add",
+           [](trainer::GradHooks& h, const at::Tensor& param, const at::Tensor& grad, PyTensor& t, int bucket) {
+             h.add(param, grad, t.inner, bucket);
+           },
+           py::arg("param"), py::arg("grad"), py::arg("tensor"), py::arg("bucket"))
+      .def("install", &trainer::GradHooks::install)
+      .def("remove", &trainer::GradHooks::remove)
+      .def("arm", &trainer::GradHooks::arm)
+      .def("flush", &trainer::GradHooks::flush, py::call_guard<py::gil_scoped_release>())
+      .def("set_enabled", &trainer::GradHooks::set_enabled, py::arg("on"));
 
   // ---- single-GPU emulation of the fused kernels (all ranks in one cooperative launch) ----
   py::class_<fused::EmulatedArena>(m, "EmulatedArena")

@@ -248,6 +248,14 @@ void async_model_average(float* t, const float* r, const float* cp, float nranks
   c.is_cuda() ? cuda::async_model_average(t, r, cp, nranks, n, c.stream)
               : cpu::async_model_average(t, r, cp, nranks, n);
 }
+void accumulate_bf16(float* x, const void* y, int64_t n, const Ctx& c) {
+  if (n <= 0) return;
+  if (c.is_cuda()) {
+    cuda::accumulate_bf16(x, y, n, c.stream);
+    return;
+  }
+  for (int64_t i = 0; i < n; ++i) x[i] += bf16_to_float(static_cast<const uint16_t*>(y)[i]);
+}
 void copy_bytes(void* dst, const void* src, size_t bytes, const Ctx& c) {
   if (bytes == 0 || dst == src) return;
   if (c.is_cuda())

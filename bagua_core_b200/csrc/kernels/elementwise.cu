@@ -146,6 +146,30 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
+// x += y, y in bf16: 10 bytes per element where a cast to fp32 and an addition move 18.
+__global__ void __launch_bounds__(kThreads)
+    accumulate_bf16_kernel(float* __restrict__ x, const __nv_bfloat16* __restrict__ y, int64_t n, bool vec) {
+  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  int64_t done = 0;
+  if (vec) {
+    const int64_t nv = n / 4;
+    for (int64_t i = tid; i < nv; i += stride) {
+      float4 a = reinterpret_cast<float4*>(x)[i];
+      const uint2 b = reinterpret_cast<const uint2*>(y)[i];
+      const float2 lo = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162&>(b.x));
+      const float2 hi = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162&>(b.y));
+      a.x += lo.x;
+      a.y += lo.y;
+      a.z += hi.x;
+      a.w += hi.y;
+      reinterpret_cast<float4*>(x)[i] = a;
+    }
+    done = nv * 4;
+  }
+  for (int64_t i = done + tid; i < n; i += stride) x[i] += __bfloat162float(y[i]);
+}
+
 // x as [n_chunks][chunk]; each thread owns V adjacent columns and walks the chunks.
 template <typename T, bool kVec>
 __global__ void __launch_bounds__(kThreads)
@@ -299,6 +323,11 @@ void average_inplace(void* x, const void* y, DType dt, int64_t n, cudaStream_t s
 void async_model_average(float* t, const float* r, const float* cp, float nranks, int64_t n, cudaStream_t s) {
   const bool vec = ((uintptr_t)t % 16 == 0) && ((uintptr_t)r % 16 == 0) && ((uintptr_t)cp % 16 == 0);
   async_avg_kernel<<<grid_for(vec ? n / 4 + 1 : n), kThreads, 0, s>>>(t, r, cp, nranks, n, vec);
+  BAGUA_CUDA_CHECK(cudaGetLastError());
+}
+void accumulate_bf16(float* x, const void* y, int64_t n, cudaStream_t s) {
+  const bool vec = ((uintptr_t)x % 16 == 0) && ((uintptr_t)y % 8 == 0);
+  accumulate_bf16_kernel<<<grid_for(vec ? n / 4 + 1 : n), kThreads, 0, s>>>(x, (const __nv_bfloat16*)y, n, vec);
   BAGUA_CUDA_CHECK(cudaGetLastError());
 }
 void copy_bytes(void* dst, const void* src, size_t bytes, cudaStream_t s) {

@@ -37,6 +37,8 @@ void average_inplace(void* x, const void* y, DType dt, int64_t n, const Ctx& c);
 void async_model_average(float* t, const float* reduced, const float* copy, float nranks, int64_t n,
                          const Ctx& c);
 void copy_bytes(void* dst, const void* src, size_t bytes, const Ctx& c);
+// x[i] += y[i] with x in fp32 and y in bf16: a low-precision gradient into its fp32 accumulator, in one pass.
+void accumulate_bf16(float* x, const void* y, int64_t n, const Ctx& c);
 
 // Flatten (gather = true: tensors -> flat) or unflatten (flat -> tensors) a list of tensors in
 // one launch.  Segments are sorted by `offset` and do not overlap; `segs` is a device array on

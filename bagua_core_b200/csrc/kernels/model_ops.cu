@@ -33,9 +33,14 @@ __global__ void __launch_bounds__(kThreads)
 }
 constexpr int kFoldCols = 32, kFoldRows = 32;
 __global__ void __launch_bounds__(kFoldCols * kFoldRows)
-    bias_grad_finish_kernel(const float* __restrict__ partial, float* __restrict__ db, int blocks, int C) {
+    bias_grad_finish_kernel(const float* __restrict__ partial, float* __restrict__ db, int blocks, int C, bool accumulate) {
   __shared__ float s_acc[kFoldCols * kFoldRows];
-  bias_grad_finish_body(partial, db, blocks, C, s_acc);
+  bias_grad_finish_body(partial, db, blocks, C, s_acc, accumulate);
+}
+__global__ void __launch_bounds__(kThreads)
+    column_sum_kernel(const uint4* __restrict__ x, float* __restrict__ partial, int64_t rows, int cgroups) {
+  __shared__ float s_acc[kThreads * 8];
+  column_sum_body(x, partial, rows, cgroups, s_acc);
 }
 __global__ void __launch_bounds__(kThreads)
     maxpool2x2_forward_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, int64_t nvec_out, int64_t Wo,
@@ -67,8 +72,11 @@ __global__ void __launch_bounds__(kThreads)
   bias_relu_pool_backward_body<kFromZ>(dp, y, dz, partial, pooled_rows, Wo, W, cgroups, s_acc, bias);
 }
 
-void fold_partials(const float* partial, float* db, int blocks, int C, cudaStream_t stream) {
-  bias_grad_finish_kernel<<<(C + kFoldCols - 1) / kFoldCols, dim3(kFoldCols, kFoldRows), 0, stream>>>(partial, db, blocks, C);
+void fold_partials(const float* partial, float* db, int blocks, int C, bool accumulate, cudaStream_t stream) {
+  // few partial rows need few threads
+  const int rows = blocks >= kFoldRows ? kFoldRows : blocks > 4 ? 8 : 4;
+  bias_grad_finish_kernel<<<(C + kFoldCols - 1) / kFoldCols, dim3(kFoldCols, rows), 0, stream>>>(partial, db, blocks, C,
+                                                                                                accumulate);
   BAGUA_CUDA_CHECK(cudaGetLastError());
 }
 
@@ -103,7 +111,7 @@ size_t bias_relu_backward_scratch_bytes(int64_t rows, int C) {
 }
 
 void bias_relu_backward_bf16(const void* dy, const void* y, void* dz, float* db, int64_t rows, int C, void* scratch,
-                             cudaStream_t stream) {
+                             cudaStream_t stream, bool accumulate) {
   BAGUA_CHECK(bias_relu_supported(rows, C) && (uintptr_t)dy % 16 == 0 && (uintptr_t)y % 16 == 0 &&
                   (uintptr_t)dz % 16 == 0 && scratch != nullptr,
               Tensor, "fused bias+ReLU backward: unsupported shape [" << rows << ", " << C << "] or unaligned buffers");
@@ -111,7 +119,28 @@ void bias_relu_backward_bf16(const void* dy, const void* y, void* dz, float* db,
   bias_relu_backward_kernel<<<blocks, kThreads, 0, stream>>>((const uint4*)dy, (const uint4*)y, (uint4*)dz,
                                                              (float*)scratch, rows, C / 8);
   BAGUA_CUDA_CHECK(cudaGetLastError());
-  fold_partials((const float*)scratch, db, blocks, C, stream);
+  fold_partials((const float*)scratch, db, blocks, C, accumulate, stream);
+}
+
+namespace {
+// Row slices of a column sum: enough blocks for every SM, at least 32 rows each.
+int column_sum_splits(int64_t rows, int C) {
+  const int col_blocks = (C / 8 + 31) / 32;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(rows / 32, 2 * 148 / col_blocks));
+}
+}  // namespace
+
+size_t column_sum_scratch_bytes(int64_t rows, int C) {
+  return (size_t)column_sum_splits(rows, C) * (size_t)C * sizeof(float);
+}
+
+void column_sum_bf16(const void* x, float* out, int64_t rows, int C, void* scratch, cudaStream_t stream, bool accumulate) {
+  BAGUA_CHECK(column_sum_supported(rows, C) && (uintptr_t)x % 16 == 0 && scratch != nullptr, Tensor,
+              "column sum: unsupported shape [" << rows << ", " << C << "] or unaligned buffer");
+  const int splits = column_sum_splits(rows, C);
+  column_sum_kernel<<<dim3((C / 8 + 31) / 32, splits), kThreads, 0, stream>>>((const uint4*)x, (float*)scratch, rows, C / 8);
+  BAGUA_CUDA_CHECK(cudaGetLastError());
+  fold_partials((const float*)scratch, out, splits, C, accumulate, stream);
 }
 
 void maxpool2x2_forward_bf16(const void* x, void* y, int64_t N, int64_t H, int64_t W, int C, cudaStream_t stream) {
@@ -162,7 +191,7 @@ void bias_relu_pool_only_bf16(const void* z, void* p, const void* bias, int64_t 
 }
 
 void bias_relu_pool_backward_bf16(const void* dp, const void* y, const void* bias, void* dz, float* db, int64_t N,
-                                  int64_t H, int64_t W, int C, void* scratch, cudaStream_t stream) {
+                                  int64_t H, int64_t W, int C, void* scratch, cudaStream_t stream, bool accumulate) {
   BAGUA_CHECK(bias_relu_supported(N * H * W, C) && maxpool2x2_supported(N, H, W, C) && (uintptr_t)dp % 16 == 0 &&
                   (uintptr_t)y % 16 == 0 && (uintptr_t)dz % 16 == 0 && scratch != nullptr,
               Tensor,
@@ -174,7 +203,7 @@ void bias_relu_pool_backward_bf16(const void* dp, const void* y, const void* bia
   kernel<<<blocks, kThreads, 0, stream>>>((const uint4*)dp, (const uint4*)y, (uint4*)dz, (float*)scratch, pooled_rows,
                                           W / 2, W, C / 8, (const __nv_bfloat16*)bias);
   BAGUA_CUDA_CHECK(cudaGetLastError());
-  fold_partials((const float*)scratch, db, blocks, C, stream);
+  fold_partials((const float*)scratch, db, blocks, C, accumulate, stream);
 }
 
 }  // namespace model_ops

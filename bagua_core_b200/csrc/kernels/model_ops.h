@@ -32,9 +32,15 @@ void bias_relu_inplace_bf16(void* z, const void* bias, int64_t rows, int C, cuda
 // Bytes of scratch (per-block partial sums) the backward needs for this shape.
 size_t bias_relu_backward_scratch_bytes(int64_t rows, int C);
 
-// dy, y, dz: [rows, C] bf16 (dz may alias dy); db: [C] fp32; scratch as sized above.
+// dy, y, dz: [rows, C] bf16 (dz may alias dy); db: [C] fp32, written or added to; scratch as sized above.
 void bias_relu_backward_bf16(const void* dy, const void* y, void* dz, float* db, int64_t rows, int C, void* scratch,
-                             cudaStream_t stream);
+                             cudaStream_t stream, bool accumulate = false);
+
+// out[c] (+)= sum over rows of x [rows, C] in bf16, accumulated in fp32 in a fixed order: the bias gradient of a
+// linear layer.  C a multiple of 8, x 16-byte aligned.  (3072 x 1024: 8 us; the library's reduction 13 us.)
+inline bool column_sum_supported(int64_t rows, int C) { return rows > 0 && C >= 8 && C % 8 == 0; }
+size_t column_sum_scratch_bytes(int64_t rows, int C);
+void column_sum_bf16(const void* x, float* out, int64_t rows, int C, void* scratch, cudaStream_t stream, bool accumulate);
 
 // ---- 2x2 / stride-2 max pooling on channels-last bf16 activations ---------------------
 // x: [N, H, W, C] (H, W even, C a multiple of 8), y: [N, H/2, W/2, C].  The forward stores no
@@ -57,7 +63,8 @@ void bias_relu_pool_only_bf16(const void* z, void* p, const void* bias, int64_t 
 // dz: [N, H, W, C] (every element written); db: [C] fp32; scratch of
 // bias_relu_backward_scratch_bytes(N*(H/2)*(W/2), C) bytes.
 void bias_relu_pool_backward_bf16(const void* dp, const void* y, const void* bias, void* dz, float* db, int64_t N,
-                                  int64_t H, int64_t W, int C, void* scratch, cudaStream_t stream);
+                                  int64_t H, int64_t W, int C, void* scratch, cudaStream_t stream,
+                                  bool accumulate = false);
 
 // ---- host restatements (model_ops_cpu.cc): same arguments, host pointers, any C ----------
 void bias_relu_inplace_bf16_host(void* z, const void* bias, int64_t rows, int C);

@@ -124,7 +124,8 @@ __device__ __forceinline__ void bias_relu_backward_body(const uint4* dy, const u
 // what counts is the length of a thread's chain of loads.  One thread per column walked all 592 rows in 17.7 us;
 // 32 x 32 threads per block walk 19 rows each.
 __device__ __forceinline__ void bias_grad_finish_body(const float* __restrict__ partial, float* __restrict__ db,
-                                                      int blocks, int C, float* s_acc = nullptr) {
+                                                      int blocks, int C, float* s_acc = nullptr,
+                                                      bool accumulate = false) {
   const int c = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int rows_at_once = blockDim.y > 1 ? (int)blockDim.y : 1;
   float s = 0.f;
@@ -139,7 +140,40 @@ __device__ __forceinline__ void bias_grad_finish_body(const float* __restrict__ 
     s = 0.f;
     for (int r = 0; r < rows_at_once; ++r) s += s_acc[r * blockDim.x + threadIdx.x];
   }
-  if (c < C) db[c] = s;
+  if (c < C) db[c] = accumulate ? db[c] + s : s;
+}
+
+// Column sums of x [rows, 8 * cgroups] in bf16, for any number of channel groups: warp (threadIdx.x / 32) of a
+// block takes every (blockDim.x / 32)-th row of its slice and 32 channel groups (512 contiguous bytes); the
+// warps' sums meet in s_acc (8 floats per thread) and the block leaves one partial row.
+__device__ __forceinline__ void column_sum_body(const uint4* __restrict__ x, float* __restrict__ partial, int64_t rows,
+                                                int cgroups, float* s_acc) {
+  const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5, warps = (int)blockDim.x >> 5;
+  const int cg = (int)blockIdx.x * 32 + lane;
+  const int64_t per = (rows + gridDim.y - 1) / gridDim.y;
+  const int64_t lo = (int64_t)blockIdx.y * per, hi = lo + per < rows ? lo + per : rows;
+  float acc[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) acc[k] = 0.f;
+  if (cg < cgroups) {
+#pragma unroll 4
+    for (int64_t r = lo + warp; r < hi; r += warps) {
+      float f[8];
+      unpack8(x[r * cgroups + cg], f);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) acc[k] += f[k];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) s_acc[threadIdx.x * 8 + k] = acc[k];
+  __syncthreads();
+  // thread t adds the warps' sums of column t of the block's 256
+  const int c = (int)blockIdx.x * 256 + (int)threadIdx.x;
+  if ((int)threadIdx.x < 256 && c < cgroups * 8) {
+    float s = 0.f;
+    for (int w = 0; w < warps; ++w) s += s_acc[w * 256 + threadIdx.x];
+    partial[(size_t)blockIdx.y * cgroups * 8 + c] = s;
+  }
 }
 
 // ---- 2x2 / stride-2 max pooling -------------------------------------------------------

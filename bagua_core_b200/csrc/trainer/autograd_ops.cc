@@ -1,0 +1,363 @@
+#include "autograd_ops.h"
+
+#include <ATen/autocast_mode.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/autograd/variable.h>
+
+#include <memory>
+#include <mutex>
+#include <unordered_map>
+
+#include "../common.h"
+#include "../kernels/kernels.h"
+#include "../kernels/model_ops.h"
+#include "../tensor/tensor.h"
+
+namespace bagua {
+namespace trainer {
+
+using torch::autograd::Node;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+OpStats& OpStats::global() {
+  static OpStats s;
+  return s;
+}
+
+namespace {
+
+cudaStream_t stream_of(const at::Tensor& t) {
+  return t.is_cuda() ? c10::cuda::getCurrentCUDAStream(t.device().index()).stream() : nullptr;
+}
+kernels::Ctx ctx_of(const at::Tensor& t) {
+  return kernels::Ctx{t.is_cuda() ? (int)t.device().index() : -1, stream_of(t)};
+}
+void count_launches(int n) { OpStats::global().launches += n; }
+
+// ---- uses of a weight in a graph ---------------------------------------------------------------
+// Where a weight takes part in a graph more than once, autograd adds the uses' gradients first and
+// accumulates once; accumulating each use by itself would round differently, so both uses of such a
+// pair are marked and take autograd's path.  A use lives as long as its node.
+struct Use {
+  explicit Use(const c10::TensorImpl* key) : key(key) {}
+  ~Use();
+  const c10::TensorImpl* key;
+  std::atomic<bool> shared{false}, done{false};
+};
+struct UseTable {
+  std::mutex mu;
+  std::unordered_map<const c10::TensorImpl*, std::weak_ptr<Use>> last;
+  static UseTable& global() {
+    static UseTable* t = new UseTable();  // nodes may outlive static destruction
+    return *t;
+  }
+};
+Use::~Use() {
+  auto& t = UseTable::global();
+  std::lock_guard<std::mutex> g(t.mu);
+  auto it = t.last.find(key);
+  if (it != t.last.end() && it->second.expired()) t.last.erase(it);
+}
+std::shared_ptr<Use> begin_use(const at::Tensor& param) {
+  auto use = std::make_shared<Use>(param.unsafeGetTensorImpl());
+  std::shared_ptr<Use> prev;  // released after the lock
+  auto& t = UseTable::global();
+  std::lock_guard<std::mutex> g(t.mu);
+  auto& slot = t.last[use->key];
+  prev = slot.lock();
+  if (prev && !prev->done) {
+    prev->shared = true;
+    use->shared = true;
+  }
+  slot = use;
+  return use;
+}
+
+// Whether a gradient for `param` may be added to `param.grad` here: an fp32 gradient of the parameter's shape
+// and memory layout is there, no graph of the backward is being built, and no tensor hook wants to see it.
+bool accumulates(const at::Tensor& param, const at::Tensor& like) {
+  if (!param.defined() || c10::GradMode::is_enabled() || !param.is_leaf()) return false;
+  const at::Tensor& grad = param.grad();
+  return grad.defined() && grad.scalar_type() == at::kFloat && grad.sizes() == param.sizes() &&
+         grad.strides() == param.strides() && grad.is_non_overlapping_and_dense() && grad.device() == like.device() &&
+         torch::autograd::impl::hooks(param).empty();
+}
+
+// grad += aᵀ-shaped product a b of bf16 operands, accumulated in fp32.  False: not available, nothing changed.
+bool gemm_into(at::Tensor grad, const at::Tensor& a, const at::Tensor& b) {
+  if (!grad.is_cuda()) {  // host: no mixed-precision GEMM; widen the operands
+    grad.addmm_(a.to(grad.scalar_type()), b.to(grad.scalar_type()));
+    return true;
+  }
+  auto& mode = OpStats::global().gemm_mode;
+  // A gradient that does not start on 16 bytes (it follows a tensor of odd size in its bucket) costs the library
+  // its fast kernels: 82 us instead of 22 for 3072 x 1024 x 3072.  The product then goes to a buffer of its own and
+  // is added from there.
+  const bool aligned = (uintptr_t)grad.data_ptr() % 16 == 0;
+  if (mode <= 1 && (aligned || mode == 0)) {
+    try {
+      at::addmm_out(grad, grad, a, b, at::kFloat);
+      mode = 1;
+      return true;
+    } catch (const c10::Error&) {
+      if (mode == 1) throw;  // it worked before: a real error, not a missing overload
+      mode = 2;
+    }
+  }
+  if (mode == 3) return false;
+  at::Tensor product;
+  try {
+    product = at::mm(a, b, at::kFloat);
+  } catch (const c10::Error&) {
+    mode = 3;
+    return false;
+  }
+  kernels::add_inplace(grad.data_ptr(), product.data_ptr(), DType::F32, grad.numel(), ctx_of(grad));
+  return true;
+}
+
+bool autocast_on(const at::Tensor& t) { return at::autocast::is_autocast_enabled(t.device().type()); }
+
+// No autograd below this point, and no autocast.
+struct PlainDispatch {
+  at::AutoDispatchBelowADInplaceOrView below;
+  c10::impl::ExcludeDispatchKeyGuard no_autocast{c10::autocast_dispatch_keyset};
+};
+
+template <typename N>
+std::shared_ptr<N> make_node(const at::Tensor& x, const at::Tensor& weight, const at::Tensor& bias) {
+  auto node = std::shared_ptr<N>(new N(), torch::autograd::deleteNode);
+  node->set_next_edges(torch::autograd::collect_next_edges(x, weight, bias));
+  return node;
+}
+
+std::shared_ptr<PoolRawTensor> scratch_for(const at::Tensor& t, size_t bytes) {
+  return PoolRawTensor::allocate((int)t.device().index(), DType::U8, (int64_t)bytes, (uint64_t)(uintptr_t)stream_of(t));
+}
+
+// ---- linear ------------------------------------------------------------------------------------
+struct LinearNode : public Node {
+  SavedVariable x, w;
+  at::Tensor weight, bias;  // the parameters (bias may be undefined)
+  std::shared_ptr<Use> use;  // set when gradients are to be accumulated here
+  bool accumulate = false;
+
+  std::string name() const override { return "BaguaLinearBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    x.reset_data();
+    w.reset_data();
+  }
+
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    variable_list out(3);
+    if (use) use->done = true;
+    if (!grads[0].defined()) return out;
+    c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
+    const at::Tensor dy = grads[0], xs = x.unpack(), ws = w.unpack();
+    at::Tensor dy2 = dy.dim() == 2 ? dy : dy.reshape({-1, dy.size(-1)});
+    if (task_should_compute_output(0)) {
+      at::Tensor dx = at::mm(dy2, ws);
+      out[0] = dy.dim() == 2 ? dx : dx.view(xs.sizes());
+    }
+    if (task_should_compute_output(1)) {
+      const at::Tensor x2 = xs.dim() == 2 ? xs : xs.reshape({-1, xs.size(-1)});
+      bool done = false;
+      if (accumulate) {
+        if (use && !use->shared && accumulates(weight, dy2) && weight.grad().is_contiguous()) {
+          c10::NoGradGuard no_grad;
+          done = gemm_into(weight.grad(), dy2.t(), x2);
+        }
+        auto& stats = OpStats::global();
+        done ? ++stats.accumulated : ++stats.declined;
+      }
+      if (!done) out[1] = at::mm(dy2.t(), x2);  // autograd casts it to the parameter's type
+    }
+    if (bias.defined() && task_should_compute_output(2)) out[2] = bias_grad(dy2);
+    return out;
+  }
+
+  at::Tensor bias_grad(const at::Tensor& dy2) {
+    const int64_t rows = dy2.size(0), C = dy2.size(1);
+    if (!dy2.is_cuda() || c10::GradMode::is_enabled() || dy2.scalar_type() != at::kBFloat16 || C > (1 << 24) ||
+        !model_ops::column_sum_supported(rows, (int)C) || !dy2.is_contiguous() || (uintptr_t)dy2.data_ptr() % 16 != 0)
+      return dy2.sum(at::IntArrayRef{0}, /*keepdim=*/false, at::kFloat);
+    const bool add = accumulate && use && !use->shared && accumulates(bias, dy2);
+    at::Tensor db = add ? bias.grad() : at::empty({C}, dy2.options().dtype(at::kFloat));
+    auto scratch = scratch_for(dy2, model_ops::column_sum_scratch_bytes(rows, (int)C));
+    model_ops::column_sum_bf16(dy2.data_ptr(), db.data_ptr<float>(), rows, (int)C, scratch->data_ptr(), stream_of(dy2), add);
+    count_launches(2);
+    return add ? at::Tensor() : db;
+  }
+};
+
+// ---- convolution + bias + ReLU (+ pooling) -------------------------------------------------------
+struct ConvNode : public Node {
+  SavedVariable x, w, b, act;  // act: the activation, or with pooling the convolution's output
+  at::Tensor weight, bias;
+  std::vector<int64_t> stride, padding, dilation;
+  int64_t groups = 1;
+  bool pool = false, accumulate = false;
+  std::shared_ptr<Use> use;
+
+  std::string name() const override { return pool ? "BaguaConvBiasReLUPoolBackward" : "BaguaConvBiasReLUBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    x.reset_data();
+    w.reset_data();
+    b.reset_data();
+    act.reset_data();
+  }
+
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    variable_list out(3);
+    if (use) use->done = true;
+    if (!grads[0].defined()) return out;
+    c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
+    const at::Tensor xs = x.unpack(), ws = w.unpack(), a = act.unpack(pool ? std::shared_ptr<Node>() : shared_from_this());
+    const at::Tensor dy = grads[0].contiguous(at::MemoryFormat::ChannelsLast);
+    const bool alone = accumulate && use && !use->shared;
+    const int C = (int)ws.size(0);
+    at::Tensor dz = at::empty_like(a);
+    // the bias gradient is added to `.grad` by the fold of its partial sums
+    const bool add_bias = alone && dy.is_cuda() && task_should_compute_output(2) && accumulates(bias, dy);
+    at::Tensor db = add_bias ? bias.grad() : at::empty({C}, a.options().dtype(at::kFloat));
+    backward_tail(dy, a, dz, db, add_bias);
+    if (task_should_compute_output(2) && !add_bias) out[2] = db;
+    const bool need_x = task_should_compute_output(0), need_w = task_should_compute_output(1);
+    if (need_x || need_w) {
+      const std::vector<int64_t> zero{0, 0};
+      auto g = at::convolution_backward(dz, xs, ws, c10::nullopt, stride, padding, dilation, false, zero, groups,
+                                        {need_x, need_w, false});
+      out[0] = std::get<0>(g);
+      at::Tensor dw = std::get<1>(g);
+      if (need_w && alone && dw.scalar_type() == at::kBFloat16 && accumulates(weight, dw) &&
+          dw.strides() == weight.grad().strides()) {
+        // the cast to fp32 and the addition in one pass; the same bits
+        kernels::accumulate_bf16((float*)weight.grad().data_ptr(), dw.data_ptr(), dw.numel(), ctx_of(dw));
+        if (dw.is_cuda()) count_launches(1);
+      } else {
+        out[1] = dw;
+      }
+    }
+    return out;
+  }
+
+  void backward_tail(const at::Tensor& dy, const at::Tensor& a, at::Tensor& dz, at::Tensor& db, bool add) {
+    const int64_t N = a.size(0), H = a.size(2), W = a.size(3), rows = N * H * W;
+    const int C = (int)a.size(1);
+    float* dbp = db.data_ptr<float>();
+    if (!a.is_cuda()) {
+      if (pool) {
+        at::Tensor y = a.clone();
+        model_ops::bias_relu_inplace_bf16_host(y.data_ptr(), b.unpack().data_ptr(), rows, C);
+        model_ops::bias_relu_pool_backward_bf16_host(dy.data_ptr(), y.data_ptr(), dz.data_ptr(), dbp, N, H, W, C);
+      } else {
+        model_ops::bias_relu_backward_bf16_host(dy.data_ptr(), a.data_ptr(), dz.data_ptr(), dbp, rows, C);
+      }
+      return;
+    }
+    auto scratch = scratch_for(a, model_ops::bias_relu_backward_scratch_bytes(pool ? N * (H / 2) * (W / 2) : rows, C));
+    if (pool)
+      model_ops::bias_relu_pool_backward_bf16(dy.data_ptr(), a.data_ptr(), b.unpack().data_ptr(), dz.data_ptr(), dbp, N, H,
+                                              W, C, scratch->data_ptr(), stream_of(a), add);
+    else
+      model_ops::bias_relu_backward_bf16(dy.data_ptr(), a.data_ptr(), dz.data_ptr(), dbp, rows, C, scratch->data_ptr(),
+                                         stream_of(a), add);
+    count_launches(2);  // mask and partial sums, then their fold
+  }
+};
+
+}  // namespace
+
+at::Tensor linear(const at::Tensor& x, const at::Tensor& weight, const std::optional<at::Tensor>& bias,
+                  const std::optional<at::Tensor>& w_low, bool accumulate) {
+  const at::Tensor b = bias.value_or(at::Tensor());
+  std::shared_ptr<LinearNode> node;
+  if (torch::autograd::compute_requires_grad(x, weight, b)) node = make_node<LinearNode>(x, weight, b);
+  at::Tensor xs, ws, y;
+  {
+    PlainDispatch plain;
+    xs = x.to(at::kBFloat16);
+    ws = w_low ? *w_low : weight.to(at::kBFloat16);
+    y = at::linear(xs, ws, b.defined() ? std::optional<at::Tensor>(b.to(at::kBFloat16)) : std::nullopt);
+  }
+  if (node) {
+    node->x = SavedVariable(xs, false);
+    node->w = SavedVariable(ws, false);
+    node->weight = weight;
+    node->bias = b;
+    node->accumulate = accumulate;
+    if (accumulate && weight.requires_grad()) node->use = begin_use(weight);
+    torch::autograd::set_history(y, node);
+  }
+  return y;
+}
+
+at::Tensor conv_bias_relu(const at::Tensor& x, const at::Tensor& weight, const at::Tensor& bias,
+                          const std::vector<int64_t>& stride, const std::vector<int64_t>& padding,
+                          const std::vector<int64_t>& dilation, int64_t groups, bool pool,
+                          const std::optional<at::Tensor>& w_low, bool accumulate) {
+  std::shared_ptr<ConvNode> node;
+  if (torch::autograd::compute_requires_grad(x, weight, bias)) node = make_node<ConvNode>(x, weight, bias);
+  const bool cast = autocast_on(x);
+  const at::ScalarType low = cast ? at::autocast::get_autocast_dtype(x.device().type()) : at::kBFloat16;
+  at::Tensor xs, ws, bs, z, out;
+  {
+    PlainDispatch plain;
+    xs = (cast ? x.to(low) : x).contiguous(at::MemoryFormat::ChannelsLast);
+    ws = cast ? (w_low ? *w_low : weight.to(low)) : weight;
+    bs = (cast ? bias.to(low) : bias).contiguous();
+    const std::vector<int64_t> zero{0, 0};
+    z = at::convolution(xs, ws, c10::nullopt, stride, padding, dilation, false, zero, groups)
+            .contiguous(at::MemoryFormat::ChannelsLast);
+    const int64_t N = z.size(0), H = z.size(2), W = z.size(3), rows = N * H * W;
+    const int C = (int)z.size(1);
+    BAGUA_CHECK(z.scalar_type() == at::kBFloat16 && bs.scalar_type() == at::kBFloat16, Tensor,
+                "fused convolution blocks compute in bf16");
+    if (pool) {
+      out = at::empty({N, C, H / 2, W / 2}, z.options().memory_format(at::MemoryFormat::ChannelsLast));
+      if (z.is_cuda())
+        model_ops::bias_relu_pool_only_bf16(z.data_ptr(), out.data_ptr(), bs.data_ptr(), N, H, W, C, stream_of(z));
+      else
+        model_ops::bias_relu_pool_only_bf16_host(z.data_ptr(), out.data_ptr(), bs.data_ptr(), N, H, W, C);
+    } else {
+      out = z;
+      if (z.is_cuda())
+        model_ops::bias_relu_inplace_bf16(z.data_ptr(), bs.data_ptr(), rows, C, stream_of(z));
+      else
+        model_ops::bias_relu_inplace_bf16_host(z.data_ptr(), bs.data_ptr(), rows, C);
+    }
+    if (z.is_cuda()) count_launches(1);
+  }
+  if (node) {
+    node->x = SavedVariable(xs, false);
+    node->w = SavedVariable(ws, false);
+    node->weight = weight;
+    node->bias = bias;
+    node->stride = stride;
+    node->padding = padding;
+    node->dilation = dilation;
+    node->groups = groups;
+    node->pool = pool;
+    node->accumulate = accumulate;
+    if (accumulate && weight.requires_grad()) node->use = begin_use(weight);
+    torch::autograd::set_history(out, node);
+    if (pool) {
+      node->act = SavedVariable(z, false);
+      node->b = SavedVariable(bs, false);
+    } else {
+      node->act = SavedVariable(out, /*is_output=*/true);
+    }
+  }
+  return out;
+}
+
+}  // namespace trainer
+}  // namespace bagua

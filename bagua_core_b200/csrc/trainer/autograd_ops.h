@@ -1,0 +1,39 @@
+// Autograd functions of the trainer's layers, without a Python frame in either direction.
+//
+// A training step of the benchmark models was paced by the launching threads: a Python autograd
+// function costs 40-60 us per direction (argument packing, the GIL handed to the autograd thread and
+// back, one Python call per tensor operation), against 10-15 us for the same operations from here.
+#pragma once
+
+#include <ATen/ATen.h>
+
+#include <atomic>
+#include <optional>
+#include <vector>
+
+namespace bagua {
+namespace trainer {
+
+// Weight gradients of linear layers that were added to an fp32 `.grad` by their GEMM / that took autograd's
+// path although accumulation was asked for; kernels of this package launched by these functions.
+struct OpStats {
+  std::atomic<int64_t> accumulated{0}, declined{0}, launches{0};
+  std::atomic<int> gemm_mode{0};  // 0 not decided, 1 one GEMM, 2 GEMM and an addition, 3 not available
+  static OpStats& global();
+};
+
+// y = x Wᵀ + b in bf16.  `w_low`: W in bf16 when the caller has it, else it is cast here.  With `accumulate`, the
+// backward adds the gradients of W and b to their fp32 `.grad` itself where nobody can tell the difference
+// (autograd_ops.cc, `accumulates`), and hands autograd nothing for them.
+at::Tensor linear(const at::Tensor& x, const at::Tensor& weight, const std::optional<at::Tensor>& bias,
+                  const std::optional<at::Tensor>& w_low, bool accumulate);
+
+// max(conv(x, weight) + bias, 0), channels-last, followed by 2x2 pooling with `pool`.  Inside an autocast region
+// x, weight and bias are taken in its type (the weight from `w_low` when given).
+at::Tensor conv_bias_relu(const at::Tensor& x, const at::Tensor& weight, const at::Tensor& bias,
+                          const std::vector<int64_t>& stride, const std::vector<int64_t>& padding,
+                          const std::vector<int64_t>& dilation, int64_t groups, bool pool,
+                          const std::optional<at::Tensor>& w_low, bool accumulate);
+
+}  // namespace trainer
+}  // namespace bagua

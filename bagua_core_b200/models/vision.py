@@ -120,14 +120,16 @@ class ResNet50(nn.Module):
 
 
 class MLP(nn.Module):
-    """Small model for tests and smoke runs."""
+    """Small model for tests and smoke runs.  Its layers are `ShadowLinear`, as in the other models."""
 
     def __init__(self, d_in=64, d_hidden=128, d_out=10, depth=3):
         super().__init__()
+        from ..ops.fused_linear import ShadowLinear
+
         dims = [d_in] + [d_hidden] * (depth - 1) + [d_out]
         layers = []
         for i in range(depth):
-            layers.append(nn.Linear(dims[i], dims[i + 1]))
+            layers.append(ShadowLinear(dims[i], dims[i + 1]))
             if i < depth - 1:
                 layers.append(nn.ReLU())
         self.net = nn.Sequential(*layers)

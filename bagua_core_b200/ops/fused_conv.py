@@ -1,13 +1,14 @@
 """Convolution block with the element-wise tail fused: conv → (bias + ReLU) in one in-place pass,
 and in the backward one pass that applies the ReLU mask and reduces the bias gradient.
 
-The convolution itself stays a library call (cuDNN through `aten.convolution` /
-`aten.convolution_backward`).  What the framework would run around it — a bias add, a clamp, a
-ReLU-mask kernel and a separate column reduction for the bias gradient — is replaced by the two
-sm_100a kernels of `csrc/kernels/model_ops.cu`.  The fused path needs a block computed in bf16
+The convolution itself stays a library call (cuDNN through `at::convolution` /
+`at::convolution_backward`).  What the framework would run around it — a bias add, a clamp, a
+ReLU-mask kernel and a separate column reduction for the bias gradient — is replaced by the
+sm_100a kernels of `csrc/kernels/model_ops.cu`; the autograd functions are native
+(`csrc/trainer/autograd_ops.cc`).  The fused path needs a block computed in bf16
 (bf16 autocast on CUDA, or bf16 parameters and inputs); anything else takes the plain PyTorch
 composition, so `ConvBiasReLU` is a drop-in for `Conv2d` followed by `ReLU`.  bf16 tensors on the
-CPU run the same Python path against a host restatement of the kernels
+CPU run the same path against a host restatement of the kernels
 (`csrc/kernels/model_ops_cpu.cc`), which is how the glue is tested without a GPU.
 """
 from __future__ import annotations
@@ -18,10 +19,18 @@ import torch.nn.functional as F
 
 from .._native import C as _C
 from . import shadow as _shadow
+from . import wgrad as _wgrad
 
 
-# Kernels of this module launched so far in this process (benchmarks report it).
-launches = 0
+# Kernels launched so far in this process by the functions of this file and of `fused_linear`
+# (benchmarks report it as `launches`).
+_pool_launches = 0
+
+
+def __getattr__(name):
+    if name == "launches":
+        return _pool_launches + _C.op_stats()["launches"]
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 def _stream(t: torch.Tensor) -> int:
@@ -29,99 +38,30 @@ def _stream(t: torch.Tensor) -> int:
 
 
 def _count(n: int) -> None:
-    global launches
-    launches += n
+    global _pool_launches
+    _pool_launches += n
 
 
-def _autocast_inputs(*tensors):
-    """What an autocast-aware op does with its inputs: inside an autocast region of the tensors'
-    device, floating-point inputs are cast to the region's dtype; elsewhere they pass through."""
-    dev = tensors[0].device.type
-    if not torch.is_autocast_enabled(dev):
-        return tensors
-    dtype = torch.get_autocast_dtype(dev)
-    return tuple(t.to(dtype) if t.is_floating_point() else t for t in tensors)
-
-
-def _autocast_weight(weight: torch.Tensor) -> torch.Tensor:
-    """The weight in the autocast dtype; taken from the optimizer's bf16 copy when that is current
-    (`bagua_core_b200.ops.shadow`), so that the forward pass does not cast it again."""
-    dev = weight.device.type
-    if not torch.is_autocast_enabled(dev):
-        return weight
-    return _shadow.cast_weight(weight, torch.get_autocast_dtype(dev))
-
-
-class _ConvBiasReLUFn(torch.autograd.Function):
+class _ConvBiasReLUFn:
     """Runs in the autocast dtype where autocast is on (parameters stay fp32 outside; autograd
-    casts the gradients returned here back to the parameters' dtype)."""
+    casts the gradients back to the parameters' dtype).  With `wgrad.enabled` the backward adds the
+    gradients of weight and bias to an fp32 `.grad` itself, with the bits autograd would produce."""
 
     @staticmethod
-    def forward(ctx, x, weight, bias, stride, padding, dilation, groups):
-        ctx.conf = (stride, padding, dilation, groups)
-        x, bias = _autocast_inputs(x, bias)
-        weight = _autocast_weight(weight)
-        with torch.autocast(x.device.type, enabled=False):
-            x = x.contiguous(memory_format=torch.channels_last)
-            z = torch.ops.aten.convolution(x, weight, None, stride, padding, dilation, False, [0, 0], groups)
-            z = z.contiguous(memory_format=torch.channels_last)
-        _C.k_bias_relu_(z, bias.contiguous(), _stream(z))
-        _count(1)
-        ctx.save_for_backward(x, weight, z)
-        return z
-
-    @staticmethod
-    def backward(ctx, dy):
-        stride, padding, dilation, groups = ctx.conf
-        x, weight, y = ctx.saved_tensors
-        dy = dy.contiguous(memory_format=torch.channels_last)
-        dz = torch.empty_like(y)
-        db = torch.empty(weight.shape[0], dtype=torch.float32, device=y.device)
-        _C.k_bias_relu_backward(dy, y, dz, db, _stream(y))
-        _count(2)  # mask + partial sums, then the fold of the partial sums
-        with torch.autocast(y.device.type, enabled=False):
-            dx, dw, _ = torch.ops.aten.convolution_backward(
-                dz, x, weight, None, stride, padding, dilation, False, [0, 0], groups,
-                [ctx.needs_input_grad[0], ctx.needs_input_grad[1], False])
-        return dx, dw, db, None, None, None, None  # fp32; autograd casts it to the bias parameter's dtype
+    def apply(x, weight, bias, stride, padding, dilation, groups):
+        return _C.conv_bias_relu(x, weight, bias, stride, padding, dilation, groups, False,
+                                 _shadow.autocast_copy(weight), _wgrad.enabled)
 
 
-class _ConvBiasReLUPoolFn(torch.autograd.Function):
+class _ConvBiasReLUPoolFn:
     """conv → bias + ReLU → 2x2 max pooling.  The full-resolution activation is never written: the
     backward, which produces the convolution's output gradient and the bias gradient in one pass,
     makes it again from the convolution's output and the bias."""
 
     @staticmethod
-    def forward(ctx, x, weight, bias, stride, padding, dilation, groups):
-        ctx.conf = (stride, padding, dilation, groups)
-        x, bias = _autocast_inputs(x, bias)
-        weight = _autocast_weight(weight)
-        with torch.autocast(x.device.type, enabled=False):
-            x = x.contiguous(memory_format=torch.channels_last)
-            y = torch.ops.aten.convolution(x, weight, None, stride, padding, dilation, False, [0, 0], groups)
-            y = y.contiguous(memory_format=torch.channels_last)
-        n, c, h, w = y.shape
-        p = torch.empty((n, c, h // 2, w // 2), dtype=y.dtype, device=y.device, memory_format=torch.channels_last)
-        bias = bias.contiguous()
-        _C.k_bias_relu_pool(y, p, bias, _stream(y))
-        _count(1)
-        ctx.save_for_backward(x, weight, y, bias)
-        return p
-
-    @staticmethod
-    def backward(ctx, dp):
-        stride, padding, dilation, groups = ctx.conf
-        x, weight, y, bias = ctx.saved_tensors
-        dp = dp.contiguous(memory_format=torch.channels_last)
-        dz = torch.empty_like(y)
-        db = torch.empty(weight.shape[0], dtype=torch.float32, device=y.device)
-        _C.k_bias_relu_pool_backward(dp, y, dz, db, _stream(y), bias)
-        _count(2)
-        with torch.autocast(y.device.type, enabled=False):
-            dx, dw, _ = torch.ops.aten.convolution_backward(
-                dz, x, weight, None, stride, padding, dilation, False, [0, 0], groups,
-                [ctx.needs_input_grad[0], ctx.needs_input_grad[1], False])
-        return dx, dw, db, None, None, None, None  # fp32; autograd casts it to the bias parameter's dtype
+    def apply(x, weight, bias, stride, padding, dilation, groups):
+        return _C.conv_bias_relu(x, weight, bias, stride, padding, dilation, groups, True,
+                                 _shadow.autocast_copy(weight), _wgrad.enabled)
 
 
 class _MaxPool2x2Fn(torch.autograd.Function):
@@ -173,8 +113,8 @@ class ConvBiasReLU(nn.Conv2d):
                    and _C.k_bias_relu_supported(1, self.out_channels))
         if not fusable:
             return F.relu(super().forward(x))
-        return _ConvBiasReLUFn.apply(x, self.weight, self.bias, list(self.stride), list(self.padding),
-                                     list(self.dilation), self.groups)
+        return _ConvBiasReLUFn.apply(x, self.weight, self.bias, self.stride, self.padding, self.dilation,
+                                     self.groups)
 
 
 class ConvBiasReLUPool(nn.Conv2d):
@@ -194,5 +134,5 @@ class ConvBiasReLUPool(nn.Conv2d):
             fusable = _C.k_maxpool2x2_supported(x.shape[0], h, w, self.out_channels)
         if not fusable:
             return F.max_pool2d(F.relu(super().forward(x)), 2, 2)
-        return _ConvBiasReLUPoolFn.apply(x, self.weight, self.bias, list(self.stride), list(self.padding),
-                                         list(self.dilation), self.groups)
+        return _ConvBiasReLUPoolFn.apply(x, self.weight, self.bias, self.stride, self.padding,
+                                         self.dilation, self.groups)

@@ -50,13 +50,17 @@ def lookup(param: torch.Tensor) -> Optional[torch.Tensor]:
     return s.view
 
 
-def cast_weight(param: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
-    """`param.to(dtype)`, without the cast when a current bf16 copy exists."""
+def autocast_copy(param: torch.Tensor) -> Optional[torch.Tensor]:
+    """The current bf16 copy of an fp32 `param` for a call inside a bf16 autocast region, else None (the
+    caller casts)."""
     global hits, misses
-    if dtype == torch.bfloat16 and param.dtype == torch.float32:
-        v = lookup(param)
-        if v is not None:
-            hits += 1
-            return v
+    dev = param.device.type
+    if (param.dtype != torch.float32 or not torch.is_autocast_enabled(dev)
+            or torch.get_autocast_dtype(dev) != torch.bfloat16):
+        return None
+    v = lookup(param)
+    if v is None:
         misses += 1
-    return param.to(dtype)
+    else:
+        hits += 1
+    return v

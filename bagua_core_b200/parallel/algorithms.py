@@ -48,28 +48,9 @@ class Algorithm:
 
     # -- when ---------------------------------------------------------------------------
     def init_backward_hooks(self, bm):
-        hooks = []
-        by_param = {id(t.owner): t for b in bm.bagua_buckets for t in b.tensors if t.owner is not None}
-
-        def make(t):
-            def hook(param):
-                if bm._in_no_sync:
-                    return
-                if param.grad is not t.tensor:
-                    # someone replaced .grad (e.g. zero_grad(set_to_none=True)): move the new
-                    # gradient into the bucket and make the bucket view the .grad again
-                    with torch.no_grad():
-                        t.tensor.copy_(param.grad)
-                    param.grad = t.tensor
-                bm.mark_ready(t)
-
-            return hook
-
-        for _, p in bm._named_params:
-            t = by_param.get(id(p))
-            if t is not None:
-                hooks.append(p.register_post_accumulate_grad_hook(make(t)))
-        return hooks
+        """One native hook per parameter (csrc/trainer/grad_hooks.h); `bm.mark_ready` is for algorithms
+        that mark tensors themselves."""
+        return [bm.install_native_hooks()]
 
     def init_forward_pre_hooks(self, bm):
         return []

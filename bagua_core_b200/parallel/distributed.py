@@ -45,6 +45,7 @@ class BaguaModule(nn.Module):
         self.bagua_train_step_counter = 0
         self._hooks = []
         self._events = {}
+        self._native_hooks = None
         self._pending_backward = False
         self._in_no_sync = False
         self._named_params = [(n, p) for n, p in module.named_parameters() if p.requires_grad]
@@ -91,6 +92,7 @@ class BaguaModule(nn.Module):
             for t in b.tensors:
                 t._bucket = b
                 t._step = -1
+        self._native_hooks = None
         self._mark_ready_native = self.pg.backend.mark_communication_ready
         self._on_cuda = bool(self.pg.is_cuda)
         self._hooks.extend(algo.init_backward_hooks(self))
@@ -134,7 +136,22 @@ class BaguaModule(nn.Module):
                 return intra
         return self.pg.global_comm
 
+    def install_native_hooks(self):
+        """Hooks every bucket tensor's parameter; they mark its gradient ready without entering Python."""
+        hooks = _C.GradHooks(self.pg.backend, self.pg.device.index if self._on_cuda else -1)
+        for i, b in enumerate(self.bagua_buckets):
+            for t in b.tensors:
+                if t.owner is not None:
+                    hooks.add(t.owner, t.tensor, t.backend_tensor, i)
+        hooks.install()
+        hooks.set_enabled(not self._in_no_sync)
+        self._native_hooks = hooks
+        return hooks
+
     def _arm(self):
+        if self._native_hooks is not None:
+            self._native_hooks.arm()
+            return
         for b in self.bagua_buckets:
             b._pending = len(b.tensors)
 
@@ -178,6 +195,9 @@ class BaguaModule(nn.Module):
         communicated: a parameter that took no part in this step's loss gets no gradient hook, and
         its bucket would otherwise wait for it forever (and hold back every bucket behind it).
         Its gradient goes into the reduction as it is (zero after `zero_grad`)."""
+        if self._native_hooks is not None:
+            self._native_hooks.flush()
+            return
         step = self.bagua_train_step_counter
         for b in self.bagua_buckets:
             if b._pending > 0:
@@ -230,12 +250,17 @@ class BaguaModule(nn.Module):
 
         class _Ctx:
             def __enter__(self_inner):
-                outer._in_no_sync = True
+                outer._set_no_sync(True)
 
             def __exit__(self_inner, *exc):
-                outer._in_no_sync = False
+                outer._set_no_sync(False)
 
         return _Ctx()
+
+    def _set_no_sync(self, on):
+        self._in_no_sync = on
+        if self._native_hooks is not None:
+            self._native_hooks.set_enabled(not on)
 
     # ---- checkpointing ---------------------------------------------------------------
     def bagua_state_dict(self):

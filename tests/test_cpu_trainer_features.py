@@ -186,3 +186,46 @@ def test_qadam_multi_tensor_step_equals_the_per_tensor_formulas():
         for i, p in enumerate(params):
             assert torch.equal(p.detach(), ref_p[i]), (step, i)
             assert torch.equal(opt.state[p]["exp_avg"], ref_m[i]) and torch.equal(opt.state[p]["exp_avg_sq"], ref_v[i])
+
+
+def _dropped_gradient(rank, world):
+    """A gradient dropped with set_to_none and not produced again counts as zero, and a replaced one moves back."""
+    import bagua_core_b200.parallel as P
+
+    torch.manual_seed(3)
+    model = torch.nn.ModuleDict({"a": torch.nn.Linear(4, 4), "b": torch.nn.Linear(4, 4)})
+    P.init_process_group(torch.device("cpu"))
+    opt = P.FlatSGD(model.parameters(), lr=0.1)
+
+    class Net(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.m = model
+
+        def forward(self, x, both):
+            y = self.m["a"](x)
+            return y + self.m["b"](x) if both else y
+
+    bm = P.with_bagua(Net(), [opt], P.GradientAllReduceAlgorithm(), bucket_bytes=1 << 20)
+    flat = bm.bagua_buckets[0].flattened
+    x = torch.ones(2, 4)
+    out = []
+    for both in (True, False, True):
+        for p in model.parameters():
+            p.grad = None if both else p.grad
+        if not both:
+            opt.zero_grad()
+        bm(x, both).sum().backward()
+        out.append(flat.clone())
+        inside = all(p.grad.data_ptr() >= flat.data_ptr() and p.grad.data_ptr() < flat.data_ptr() + flat.nbytes
+                     for p in model.parameters())
+        out.append(inside)
+    P.destroy_process_group()
+    return out
+
+
+def test_replaced_and_missing_gradients_end_up_in_the_bucket():
+    for first, in1, second, in2, third, in3 in run_ranks(_dropped_gradient, 2):
+        assert in1 and in2 and in3
+        assert torch.equal(first, third) and not torch.equal(first, second)
+        assert int((second == 0).sum()) >= 20  # layer b took no part

@@ -369,3 +369,58 @@ def test_pooling_without_the_activation_equals_the_in_place_pair(shape):
     bb._C.k_bias_relu_pool(z, p2, bias, _stream())
     bb._C.k_bias_relu_pool_backward(dp, z, dz2, db2, _stream(), bias)
     assert torch.equal(z, z0) and torch.equal(p, p2) and torch.equal(dz, dz2) and torch.equal(db, db2)
+
+
+@pytest.mark.parametrize("rows,n_in,n_out", [(1, 8, 8), (31, 16, 264), (3072, 64, 1024), (33, 40, 1000), (5, 72, 10), (70, 8, 4096)])
+@pytest.mark.parametrize("offset", [0, 1, 2])
+def test_linear_gradients_land_in_an_fp32_bucket_at_any_alignment(rows, n_in, n_out, offset):
+    """Weight and bias gradients are views of one buffer, back to back from element `offset` on: added in place,
+    twice, and equal to the same bf16 operands multiplied and summed in fp32."""
+    from bagua_core_b200.ops import wgrad as W
+    from bagua_core_b200.ops.fused_linear import ShadowLinear
+
+    saved, W.enabled = W.enabled, True
+    try:
+        torch.manual_seed(rows + n_out)
+        m = ShadowLinear(n_in, n_out).cuda()
+        flat = torch.zeros(offset + n_out + n_out * n_in + 8, device="cuda")
+        m.bias.grad = flat[offset:offset + n_out]
+        m.weight.grad = flat[offset + n_out:offset + n_out + n_out * n_in].view(n_out, n_in)
+        x = torch.randn(rows, n_in, device="cuda", requires_grad=True)
+        want_w, want_b = torch.zeros_like(m.weight), torch.zeros_like(m.bias)
+        for _ in range(2):
+            with torch.autocast("cuda", dtype=torch.bfloat16):
+                y = m(x)
+            dy = torch.randn_like(y)
+            y.backward(dy)
+            want_w += dy.float().t() @ x.detach().bfloat16().float()
+            want_b += dy.float().sum(0)
+        assert m.weight.grad.data_ptr() == flat[offset + n_out:].data_ptr()
+        assert (m.weight.grad - want_w).abs().max() <= 2e-3 * want_w.abs().max() + 1e-5
+        assert torch.allclose(m.bias.grad, want_b, rtol=1e-4, atol=1e-3 * rows ** 0.5)
+        assert bool((flat[:offset] == 0).all() and (flat[-8:] == 0).all())
+    finally:
+        W.enabled = saved
+
+
+def test_block_gradients_added_in_place_have_the_bits_of_the_ordinary_path():
+    from bagua_core_b200.ops import wgrad as W
+    from bagua_core_b200.ops.fused_conv import ConvBiasReLU, ConvBiasReLUPool
+
+    saved, grads = W.enabled, []
+    try:
+        for W.enabled in (False, True):
+            torch.manual_seed(5)
+            net = torch.nn.Sequential(ConvBiasReLU(3, 24, 3, padding=1), ConvBiasReLUPool(24, 64, 3, padding=1)).cuda()
+            net = net.to(memory_format=torch.channels_last)
+            for p in net.parameters():
+                p.grad = torch.zeros_like(p, memory_format=torch.preserve_format)
+            x = torch.randn(3, 3, 12, 20, device="cuda").contiguous(memory_format=torch.channels_last)
+            for _ in range(2):
+                with torch.autocast("cuda", dtype=torch.bfloat16):
+                    net(x).float().square().sum().backward()
+            grads.append([p.grad.clone() for p in net.parameters()])
+    finally:
+        W.enabled = saved
+    for a, b in zip(*grads):
+        assert torch.equal(a, b)
