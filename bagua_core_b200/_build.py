@@ -38,6 +38,7 @@ SOURCES = [
     "telemetry/telemetry.cc",
     "trainer/autograd_ops.cc",
     "trainer/grad_hooks.cc",
+    "trainer/sgd_plan.cc",
     "capi/capi.cc",
     "kernels/cpu_kernels.cc",
     "kernels/elementwise.cu",

@@ -27,6 +27,7 @@
 #include "tensor/tensor.h"
 #include "trainer/autograd_ops.h"
 #include "trainer/grad_hooks.h"
+#include "trainer/sgd_plan.h"
 
 namespace py = pybind11;
 using namespace bagua;
@@ -853,6 +854,20 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     d["gemm_mode"] = modes[s.gemm_mode.load()];
     return d;
   });
+  py::class_<trainer::SgdPlan>(m, "SgdPlan")
+      .def(py::init<>())
+      .def("add", &trainer::SgdPlan::add, py::arg("param"), py::arg("grad"), py::arg("momentum_buffer"),
+           py::arg("bf16_shadow"), py::arg("group"))
+      .def("step",
+           [](trainer::SgdPlan& p, const std::vector<std::tuple<float, float, float, float, bool>>& groups, uint64_t stream) {
+             std::vector<trainer::SgdGroup> gs;
+             gs.reserve(groups.size());
+             for (auto& [lr, momentum, dampening, wd, nesterov] : groups)
+               gs.push_back(trainer::SgdGroup{lr, momentum, dampening, wd, nesterov});
+             return p.step(gs, stream);
+           },
+           py::arg("groups"), py::arg("stream"))
+      .def("zero_grad", &trainer::SgdPlan::zero_grad, py::arg("stream"));
   py::class_<trainer::GradHooks, std::shared_ptr<trainer::GradHooks>>(m, "GradHooks")
       .def(py::init([](PyBackend& be, int device) { return std::make_shared<trainer::GradHooks>(be.inner, device); }),
            py::arg("backend"), py::arg("device"))

@@ -305,19 +305,27 @@ void decompress_minmax_u8(const uint8_t* in, size_t in_bytes, int64_t chunk, int
   c.is_cuda() ? cuda::decompress_minmax_u8(in, in_bytes, chunk, n_chunks, out, dt, c.stream)
               : cpu::decompress_minmax_u8(in, in_bytes, chunk, n_chunks, out, dt);
 }
+int sgd_steps(const SgdSegment* segs, int n, const Ctx& c) {
+  if (c.is_cuda()) return cuda::sgd_steps(segs, n, c.stream);
+  for (int k = 0; k < n; ++k) {
+    const SgdSegment& a = segs[k];
+    if (a.shadow)
+      cpu::sgd_momentum_flat_shadow(a.p, a.g, a.m, a.shadow, a.n, a.lr, a.momentum, a.dampening, a.weight_decay, a.nesterov,
+                                    a.first);
+    else
+      cpu::sgd_momentum_flat(a.p, a.g, a.m, a.n, a.lr, a.momentum, a.dampening, a.weight_decay, a.nesterov, a.first);
+  }
+  return 0;
+}
 void sgd_momentum_flat(float* p, const float* g, float* buf, int64_t n, float lr, float momentum, float dampening,
                        float wd, bool nesterov, bool first_step, const Ctx& c) {
-  if (n <= 0) return;
-  c.is_cuda() ? cuda::sgd_momentum_flat(p, g, buf, n, lr, momentum, dampening, wd, nesterov, first_step, c.stream)
-              : cpu::sgd_momentum_flat(p, g, buf, n, lr, momentum, dampening, wd, nesterov, first_step);
+  sgd_momentum_flat_shadow(p, g, buf, nullptr, n, lr, momentum, dampening, wd, nesterov, first_step, c);
 }
-
 void sgd_momentum_flat_shadow(float* p, const float* g, float* buf, void* shadow, int64_t n, float lr, float momentum,
                               float dampening, float wd, bool nesterov, bool first_step, const Ctx& c) {
   if (n <= 0) return;
-  c.is_cuda()
-      ? cuda::sgd_momentum_flat_shadow(p, g, buf, shadow, n, lr, momentum, dampening, wd, nesterov, first_step, c.stream)
-      : cpu::sgd_momentum_flat_shadow(p, g, buf, shadow, n, lr, momentum, dampening, wd, nesterov, first_step);
+  const SgdSegment a{p, g, buf, shadow, n, lr, momentum, dampening, wd, nesterov, first_step, false};
+  sgd_steps(&a, 1, c);
 }
 
 }  // namespace kernels

@@ -38,6 +38,15 @@ void async_model_average(float* t, const float* reduced, const float* copy, floa
                          const Ctx& c);
 void copy_bytes(void* dst, const void* src, size_t bytes, const Ctx& c);
 // x[i] += y[i] with x in fp32 and y in bf16: a low-precision gradient into its fp32 accumulator, in one pass.
+struct CastSegment {
+  const float* src;
+  void* dst;  // n bf16 values
+  int64_t n;
+};
+// Rounds a few fp32 buffers to bf16 in one launch (CUDA only).
+namespace cuda {
+void cast_bf16(const CastSegment* segs, int n, cudaStream_t s);
+}
 void accumulate_bf16(float* x, const void* y, int64_t n, const Ctx& c);
 
 // Flatten (gather = true: tensors -> flat) or unflatten (flat -> tensors) a list of tensors in
@@ -83,6 +92,19 @@ struct MinMaxGrid {
 MinMaxGrid minmax_grid(float mn, float mx);
 
 // ---- fused optimiser steps over flat bucket memory (no reference counterpart) -------
+// One flat buffer of an SGD step, with its hyperparameters.
+struct SgdSegment {
+  float* p;
+  const float* g;
+  float* m;
+  void* shadow;  // n bf16 values, or null
+  int64_t n;
+  float lr, momentum, dampening, weight_decay;
+  bool nesterov, first;
+  bool vec;  // set by the CUDA path
+};
+// Steps all buffers; returns how many kernels were launched.
+int sgd_steps(const SgdSegment* segs, int n, const Ctx& c);
 // p -= lr * (momentum buffer update of g (+ weight_decay * p)), torch.optim.SGD semantics.
 void sgd_momentum_flat(float* p, const float* g, float* buf, int64_t n, float lr, float momentum,
                        float dampening, float weight_decay, bool nesterov, bool first_step,

@@ -22,10 +22,7 @@ void compress_minmax_u8(const void* in, DType dt, int64_t num_real, int64_t chun
                         size_t out_bytes, int target, void* scratch, size_t scratch_bytes, cudaStream_t s);
 void decompress_minmax_u8(const uint8_t* in, size_t in_bytes, int64_t chunk, int n_chunks, void* out, DType dt,
                           cudaStream_t s);
-void sgd_momentum_flat(float* p, const float* g, float* buf, int64_t n, float lr, float momentum, float dampening,
-                       float wd, bool nesterov, bool first_step, cudaStream_t s);
-void sgd_momentum_flat_shadow(float* p, const float* g, float* buf, void* shadow, int64_t n, float lr, float momentum,
-                              float dampening, float wd, bool nesterov, bool first_step, cudaStream_t s);
+int sgd_steps(const SgdSegment* segs, int n, cudaStream_t s);
 
 }  // namespace cuda
 }  // namespace kernels

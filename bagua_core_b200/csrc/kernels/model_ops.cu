@@ -12,6 +12,7 @@
 
 #include "../common.h"
 #include "model_ops.h"
+#include "launch.cuh"
 #include "model_ops_bodies.cuh"
 
 namespace bagua {
@@ -20,47 +21,57 @@ namespace model_ops {
 namespace {
 
 using namespace bodies;
+using kernels::launch_overlapped;
+using kernels::wait_for_predecessor;
 
 __global__ void __launch_bounds__(kThreads)
     bias_relu_kernel(uint4* __restrict__ z, const __nv_bfloat16* __restrict__ bias, int64_t nvec, int cgroups) {
+  wait_for_predecessor();
   bias_relu_body(z, bias, nvec, cgroups);
 }
 __global__ void __launch_bounds__(kThreads)
     bias_relu_backward_kernel(const uint4* dy, const uint4* __restrict__ y, uint4* dz, float* __restrict__ partial,
                               int64_t rows, int cgroups) {
   __shared__ float s_acc[kThreads * 8];
+  wait_for_predecessor();
   bias_relu_backward_body(dy, y, dz, partial, rows, cgroups, s_acc);
 }
 constexpr int kFoldCols = 32, kFoldRows = 32;
 __global__ void __launch_bounds__(kFoldCols * kFoldRows)
     bias_grad_finish_kernel(const float* __restrict__ partial, float* __restrict__ db, int blocks, int C, bool accumulate) {
   __shared__ float s_acc[kFoldCols * kFoldRows];
+  wait_for_predecessor();
   bias_grad_finish_body(partial, db, blocks, C, s_acc, accumulate);
 }
 __global__ void __launch_bounds__(kThreads)
-    column_sum_kernel(const uint4* __restrict__ x, float* __restrict__ partial, int64_t rows, int cgroups) {
+    column_sum_kernel(const uint4* __restrict__ x, float* __restrict__ partial, int64_t rows, int cgroups, bool accumulate) {
   __shared__ float s_acc[kThreads * 8];
-  column_sum_body(x, partial, rows, cgroups, s_acc);
+  wait_for_predecessor();
+  column_sum_body(x, partial, rows, cgroups, s_acc, accumulate);
 }
 __global__ void __launch_bounds__(kThreads)
     maxpool2x2_forward_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, int64_t nvec_out, int64_t Wo,
                               int64_t W, int cgroups) {
+  wait_for_predecessor();
   maxpool2x2_forward_body(x, y, nvec_out, Wo, W, cgroups);
 }
 __global__ void __launch_bounds__(kThreads)
     maxpool2x2_backward_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy, uint4* __restrict__ dx,
                                int64_t nvec_out, int64_t Wo, int64_t W, int cgroups) {
+  wait_for_predecessor();
   maxpool2x2_backward_body(x, dy, dx, nvec_out, Wo, W, cgroups);
 }
 
 __global__ void __launch_bounds__(kThreads)
     bias_relu_pool_kernel(uint4* __restrict__ y, uint4* __restrict__ p, const __nv_bfloat16* __restrict__ bias,
                           int64_t pooled_pixels, int64_t Wo, int64_t W, int cgroups) {
+  wait_for_predecessor();
   bias_relu_pool_body(y, p, bias, pooled_pixels, Wo, W, cgroups);
 }
 __global__ void __launch_bounds__(kThreads)
     bias_relu_pool_only_kernel(const uint4* __restrict__ z, uint4* __restrict__ p, const __nv_bfloat16* __restrict__ bias,
                                int64_t pooled_pixels, int64_t Wo, int64_t W, int cgroups) {
+  wait_for_predecessor();
   bias_relu_pool_only_body(z, p, bias, pooled_pixels, Wo, W, cgroups);
 }
 template <bool kFromZ>
@@ -69,15 +80,14 @@ __global__ void __launch_bounds__(kThreads)
                                    float* __restrict__ partial, int64_t pooled_rows, int64_t Wo, int64_t W, int cgroups,
                                    const __nv_bfloat16* __restrict__ bias) {
   __shared__ float s_acc[kThreads * 8];
+  wait_for_predecessor();
   bias_relu_pool_backward_body<kFromZ>(dp, y, dz, partial, pooled_rows, Wo, W, cgroups, s_acc, bias);
 }
 
 void fold_partials(const float* partial, float* db, int blocks, int C, bool accumulate, cudaStream_t stream) {
   // few partial rows need few threads
   const int rows = blocks >= kFoldRows ? kFoldRows : blocks > 4 ? 8 : 4;
-  bias_grad_finish_kernel<<<(C + kFoldCols - 1) / kFoldCols, dim3(kFoldCols, rows), 0, stream>>>(partial, db, blocks, C,
-                                                                                                accumulate);
-  BAGUA_CUDA_CHECK(cudaGetLastError());
+  launch_overlapped(bias_grad_finish_kernel, dim3((C + kFoldCols - 1) / kFoldCols), dim3(kFoldCols, rows), stream, partial, db, blocks, C, accumulate);
 }
 
 int pool_grid(int64_t nvec_out) {
@@ -101,8 +111,7 @@ void bias_relu_inplace_bf16(void* z, const void* bias, int64_t rows, int C, cuda
   const int64_t nvec = rows * (C / 8);
   const int64_t want = (nvec + (int64_t)kThreads * 4 - 1) / ((int64_t)kThreads * 4);
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, 148 * 8));
-  bias_relu_kernel<<<grid, kThreads, 0, stream>>>((uint4*)z, (const __nv_bfloat16*)bias, nvec, C / 8);
-  BAGUA_CUDA_CHECK(cudaGetLastError());
+  launch_overlapped(bias_relu_kernel, dim3(grid), dim3(kThreads), stream, (uint4*)z, (const __nv_bfloat16*)bias, nvec, C / 8);
 }
 
 size_t bias_relu_backward_scratch_bytes(int64_t rows, int C) {
@@ -116,9 +125,7 @@ void bias_relu_backward_bf16(const void* dy, const void* y, void* dz, float* db,
                   (uintptr_t)dz % 16 == 0 && scratch != nullptr,
               Tensor, "fused bias+ReLU backward: unsupported shape [" << rows << ", " << C << "] or unaligned buffers");
   const int blocks = backward_blocks(rows, C);
-  bias_relu_backward_kernel<<<blocks, kThreads, 0, stream>>>((const uint4*)dy, (const uint4*)y, (uint4*)dz,
-                                                             (float*)scratch, rows, C / 8);
-  BAGUA_CUDA_CHECK(cudaGetLastError());
+  launch_overlapped(bias_relu_backward_kernel, dim3(blocks), dim3(kThreads), stream, (const uint4*)dy, (const uint4*)y, (uint4*)dz, (float*)scratch, rows, C / 8);
   fold_partials((const float*)scratch, db, blocks, C, accumulate, stream);
 }
 
@@ -131,25 +138,27 @@ int column_sum_splits(int64_t rows, int C) {
 }  // namespace
 
 size_t column_sum_scratch_bytes(int64_t rows, int C) {
-  return (size_t)column_sum_splits(rows, C) * (size_t)C * sizeof(float);
+  const int splits = column_sum_splits(rows, C);
+  return splits == 1 ? 0 : (size_t)splits * (size_t)C * sizeof(float);
 }
 
 void column_sum_bf16(const void* x, float* out, int64_t rows, int C, void* scratch, cudaStream_t stream, bool accumulate) {
-  BAGUA_CHECK(column_sum_supported(rows, C) && (uintptr_t)x % 16 == 0 && scratch != nullptr, Tensor,
+  BAGUA_CHECK(column_sum_supported(rows, C) && (uintptr_t)x % 16 == 0 &&
+                  (scratch != nullptr || column_sum_scratch_bytes(rows, C) == 0),
+              Tensor,
               "column sum: unsupported shape [" << rows << ", " << C << "] or unaligned buffer");
   const int splits = column_sum_splits(rows, C);
-  column_sum_kernel<<<dim3((C / 8 + 31) / 32, splits), kThreads, 0, stream>>>((const uint4*)x, (float*)scratch, rows, C / 8);
-  BAGUA_CUDA_CHECK(cudaGetLastError());
-  fold_partials((const float*)scratch, out, splits, C, accumulate, stream);
+  const bool direct = splits == 1;  // few rows: the one slice's sums are the result
+  launch_overlapped(column_sum_kernel, dim3((C / 8 + 31) / 32, splits), dim3(kThreads), stream, (const uint4*)x,
+                    direct ? out : (float*)scratch, rows, C / 8, direct && accumulate);
+  if (!direct) fold_partials((const float*)scratch, out, splits, C, accumulate, stream);
 }
 
 void maxpool2x2_forward_bf16(const void* x, void* y, int64_t N, int64_t H, int64_t W, int C, cudaStream_t stream) {
   BAGUA_CHECK(maxpool2x2_supported(N, H, W, C) && (uintptr_t)x % 16 == 0 && (uintptr_t)y % 16 == 0, Tensor,
               "fused max-pool: unsupported shape [" << N << ", " << H << ", " << W << ", " << C << "] or unaligned buffers");
   const int64_t nvec_out = N * (H / 2) * (W / 2) * (C / 8);
-  maxpool2x2_forward_kernel<<<pool_grid(nvec_out), kThreads, 0, stream>>>((const uint4*)x, (uint4*)y, nvec_out, W / 2, W,
-                                                                          C / 8);
-  BAGUA_CUDA_CHECK(cudaGetLastError());
+  launch_overlapped(maxpool2x2_forward_kernel, dim3(pool_grid(nvec_out)), dim3(kThreads), stream, (const uint4*)x, (uint4*)y, nvec_out, W / 2, W, C / 8);
 }
 
 void maxpool2x2_backward_bf16(const void* x, const void* dy, void* dx, int64_t N, int64_t H, int64_t W, int C,
@@ -160,9 +169,7 @@ void maxpool2x2_backward_bf16(const void* x, const void* dy, void* dx, int64_t N
               "fused max-pool backward: unsupported shape [" << N << ", " << H << ", " << W << ", " << C
                                                              << "] or unaligned buffers");
   const int64_t nvec_out = N * (H / 2) * (W / 2) * (C / 8);
-  maxpool2x2_backward_kernel<<<pool_grid(nvec_out), kThreads, 0, stream>>>((const uint4*)x, (const uint4*)dy, (uint4*)dx,
-                                                                           nvec_out, W / 2, W, C / 8);
-  BAGUA_CUDA_CHECK(cudaGetLastError());
+  launch_overlapped(maxpool2x2_backward_kernel, dim3(pool_grid(nvec_out)), dim3(kThreads), stream, (const uint4*)x, (const uint4*)dy, (uint4*)dx, nvec_out, W / 2, W, C / 8);
 }
 
 void bias_relu_pool_bf16(void* y, void* p, const void* bias, int64_t N, int64_t H, int64_t W, int C, cudaStream_t stream) {
@@ -172,9 +179,7 @@ void bias_relu_pool_bf16(void* y, void* p, const void* bias, int64_t N, int64_t 
               "fused bias+ReLU+pool: unsupported shape [" << N << ", " << H << ", " << W << ", " << C
                                                           << "] or unaligned buffers");
   const int64_t pooled_pixels = N * (H / 2) * (W / 2);
-  bias_relu_pool_kernel<<<pool_grid(pooled_pixels * (C / 8)), kThreads, 0, stream>>>(
-      (uint4*)y, (uint4*)p, (const __nv_bfloat16*)bias, pooled_pixels, W / 2, W, C / 8);
-  BAGUA_CUDA_CHECK(cudaGetLastError());
+  launch_overlapped(bias_relu_pool_kernel, dim3(pool_grid(pooled_pixels * (C / 8))), dim3(kThreads), stream, (uint4*)y, (uint4*)p, (const __nv_bfloat16*)bias, pooled_pixels, W / 2, W, C / 8);
 }
 
 void bias_relu_pool_only_bf16(const void* z, void* p, const void* bias, int64_t N, int64_t H, int64_t W, int C,
@@ -185,9 +190,7 @@ void bias_relu_pool_only_bf16(const void* z, void* p, const void* bias, int64_t 
               "fused bias+ReLU+pool: unsupported shape [" << N << ", " << H << ", " << W << ", " << C
                                                           << "] or unaligned buffers");
   const int64_t pooled_pixels = N * (H / 2) * (W / 2);
-  bias_relu_pool_only_kernel<<<pool_grid(pooled_pixels * (C / 8)), kThreads, 0, stream>>>(
-      (const uint4*)z, (uint4*)p, (const __nv_bfloat16*)bias, pooled_pixels, W / 2, W, C / 8);
-  BAGUA_CUDA_CHECK(cudaGetLastError());
+  launch_overlapped(bias_relu_pool_only_kernel, dim3(pool_grid(pooled_pixels * (C / 8))), dim3(kThreads), stream, (const uint4*)z, (uint4*)p, (const __nv_bfloat16*)bias, pooled_pixels, W / 2, W, C / 8);
 }
 
 void bias_relu_pool_backward_bf16(const void* dp, const void* y, const void* bias, void* dz, float* db, int64_t N,
@@ -200,9 +203,7 @@ void bias_relu_pool_backward_bf16(const void* dp, const void* y, const void* bia
   const int64_t pooled_rows = N * (H / 2) * (W / 2);
   const int blocks = backward_blocks(pooled_rows, C);
   auto* kernel = bias ? bias_relu_pool_backward_kernel<true> : bias_relu_pool_backward_kernel<false>;
-  kernel<<<blocks, kThreads, 0, stream>>>((const uint4*)dp, (const uint4*)y, (uint4*)dz, (float*)scratch, pooled_rows,
-                                          W / 2, W, C / 8, (const __nv_bfloat16*)bias);
-  BAGUA_CUDA_CHECK(cudaGetLastError());
+  launch_overlapped(kernel, dim3(blocks), dim3(kThreads), stream, (const uint4*)dp, (const uint4*)y, (uint4*)dz, (float*)scratch, pooled_rows, W / 2, W, C / 8, (const __nv_bfloat16*)bias);
   fold_partials((const float*)scratch, db, blocks, C, accumulate, stream);
 }
 

@@ -145,9 +145,9 @@ __device__ __forceinline__ void bias_grad_finish_body(const float* __restrict__ 
 
 // Column sums of x [rows, 8 * cgroups] in bf16, for any number of channel groups: warp (threadIdx.x / 32) of a
 // block takes every (blockDim.x / 32)-th row of its slice and 32 channel groups (512 contiguous bytes); the
-// warps' sums meet in s_acc (8 floats per thread) and the block leaves one partial row.
+// warps' sums meet in s_acc (8 floats per thread) and the block leaves one partial row (or adds to it).
 __device__ __forceinline__ void column_sum_body(const uint4* __restrict__ x, float* __restrict__ partial, int64_t rows,
-                                                int cgroups, float* s_acc) {
+                                                int cgroups, float* s_acc, bool accumulate) {
   const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5, warps = (int)blockDim.x >> 5;
   const int cg = (int)blockIdx.x * 32 + lane;
   const int64_t per = (rows + gridDim.y - 1) / gridDim.y;
@@ -172,7 +172,8 @@ __device__ __forceinline__ void column_sum_body(const uint4* __restrict__ x, flo
   if ((int)threadIdx.x < 256 && c < cgroups * 8) {
     float s = 0.f;
     for (int w = 0; w < warps; ++w) s += s_acc[w * 256 + threadIdx.x];
-    partial[(size_t)blockIdx.y * cgroups * 8 + c] = s;
+    float* out = partial + (size_t)blockIdx.y * cgroups * 8 + c;
+    *out = accumulate ? *out + s : s;
   }
 }
 

@@ -7,6 +7,7 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
 
+#include <array>
 #include <memory>
 #include <mutex>
 #include <unordered_map>
@@ -128,6 +129,32 @@ struct PlainDispatch {
   c10::impl::ExcludeDispatchKeyGuard no_autocast{c10::autocast_dispatch_keyset};
 };
 
+// Rounds tensors to bf16, those that are fp32 on a GPU in one launch together.  Undefined ones stay undefined.
+template <size_t N>
+void to_bf16(std::array<at::Tensor, N>& ts) {
+  kernels::CastSegment segs[N];
+  int n = 0;
+  for (at::Tensor& t : ts) {
+    if (!t.defined() || t.scalar_type() == at::kBFloat16) continue;
+    if (!t.is_cuda() || t.scalar_type() != at::kFloat || !t.is_non_overlapping_and_dense()) {
+      t = t.to(at::kBFloat16);
+      continue;
+    }
+    at::Tensor low = at::empty_strided(t.sizes(), t.strides(), t.options().dtype(at::kBFloat16));
+    segs[n++] = kernels::CastSegment{(const float*)t.data_ptr(), low.data_ptr(), t.numel()};
+    // the source stays alive as the caller's tensor until the launch below
+    t = low;
+  }
+  if (n) {
+    for (const at::Tensor& t : ts)
+      if (t.defined() && t.is_cuda()) {
+        kernels::cuda::cast_bf16(segs, n, stream_of(t));
+        break;
+      }
+    count_launches(1);
+  }
+}
+
 template <typename N>
 std::shared_ptr<N> make_node(const at::Tensor& x, const at::Tensor& weight, const at::Tensor& bias) {
   auto node = std::shared_ptr<N>(new N(), torch::autograd::deleteNode);
@@ -189,9 +216,11 @@ struct LinearNode : public Node {
       return dy2.sum(at::IntArrayRef{0}, /*keepdim=*/false, at::kFloat);
     const bool add = accumulate && use && !use->shared && accumulates(bias, dy2);
     at::Tensor db = add ? bias.grad() : at::empty({C}, dy2.options().dtype(at::kFloat));
-    auto scratch = scratch_for(dy2, model_ops::column_sum_scratch_bytes(rows, (int)C));
-    model_ops::column_sum_bf16(dy2.data_ptr(), db.data_ptr<float>(), rows, (int)C, scratch->data_ptr(), stream_of(dy2), add);
-    count_launches(2);
+    const size_t bytes = model_ops::column_sum_scratch_bytes(rows, (int)C);
+    std::shared_ptr<PoolRawTensor> scratch = bytes ? scratch_for(dy2, bytes) : nullptr;
+    model_ops::column_sum_bf16(dy2.data_ptr(), db.data_ptr<float>(), rows, (int)C, scratch ? scratch->data_ptr() : nullptr,
+                               stream_of(dy2), add);
+    count_launches(bytes ? 2 : 1);
     return add ? at::Tensor() : db;
   }
 };
@@ -284,9 +313,11 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& weight, const std::opti
   at::Tensor xs, ws, y;
   {
     PlainDispatch plain;
-    xs = x.to(at::kBFloat16);
-    ws = w_low ? *w_low : weight.to(at::kBFloat16);
-    y = at::linear(xs, ws, b.defined() ? std::optional<at::Tensor>(b.to(at::kBFloat16)) : std::nullopt);
+    std::array<at::Tensor, 3> low{x, w_low ? *w_low : weight, b};
+    to_bf16(low);
+    xs = low[0];
+    ws = low[1];
+    y = at::linear(xs, ws, b.defined() ? std::optional<at::Tensor>(low[2]) : std::nullopt);
   }
   if (node) {
     node->x = SavedVariable(xs, false);
@@ -311,9 +342,14 @@ at::Tensor conv_bias_relu(const at::Tensor& x, const at::Tensor& weight, const a
   at::Tensor xs, ws, bs, z, out;
   {
     PlainDispatch plain;
-    xs = (cast ? x.to(low) : x).contiguous(at::MemoryFormat::ChannelsLast);
-    ws = cast ? (w_low ? *w_low : weight.to(low)) : weight;
-    bs = (cast ? bias.to(low) : bias).contiguous();
+    std::array<at::Tensor, 3> ts{x, w_low ? *w_low : weight, bias};
+    if (cast && low == at::kBFloat16)
+      to_bf16(ts);
+    else if (cast)
+      for (at::Tensor& t : ts) t = t.to(low);
+    xs = ts[0].contiguous(at::MemoryFormat::ChannelsLast);
+    ws = ts[1];
+    bs = ts[2].contiguous();
     const std::vector<int64_t> zero{0, 0};
     z = at::convolution(xs, ws, c10::nullopt, stride, padding, dilation, false, zero, groups)
             .contiguous(at::MemoryFormat::ChannelsLast);

@@ -1,9 +1,9 @@
-"""Optimizers that work on flat bucket memory with one fused kernel per bucket.
+"""Optimizers that work on flat bucket memory with one fused kernel for all buckets.
 
 The reference contains no optimizer (it is only the communication engine); the benchmarks
 named for it train with SGD momentum 0.9, so the engine ships the obvious companion: since
 gradients already live in flat buckets, parameters and momentum are laid out the same way
-and `step()` is ONE sm_100a kernel per bucket (read p, g, m; write p, m: 20 bytes per
+and `step()` is ONE sm_100a kernel over all buckets (read p, g, m; write p, m: 20 bytes per
 parameter, the HBM minimum) instead of torch's multi-tensor loops.
 """
 from __future__ import annotations
@@ -49,6 +49,8 @@ class FlatSGD(torch.optim.Optimizer):
         super().__init__(params, defaults)
         self._flat: List[dict] = []
         self._attached_ids = set()
+        self._plan = None   # the flat buffers, laid out for the native step (`_C.SgdPlan`)
+        self._loose = None  # (parameters in the groups, those of them outside the flat buffers)
         self._steps = 0
         self.kernel_launches = 0
         # bf16 copies of the weights, written by the step kernel (see bagua_core_b200.ops.shadow)
@@ -81,6 +83,7 @@ class FlatSGD(torch.optim.Optimizer):
     def bagua_attach(self, bm):
         self._flat.clear()
         self._attached_ids.clear()
+        self._loose = None
         for p in self._shadowed:
             p._bagua_bf16 = None
         self._shadowed.clear()
@@ -97,7 +100,7 @@ class FlatSGD(torch.optim.Optimizer):
                     p.grad = flat_g[off:off + n].as_strided(tuple(p.shape), tuple(p.stride()))
                     self._attached_ids.add(id(p))
                     off += n
-                self._flat.append({"p": b.flattened, "g": flat_g, "m": torch.zeros_like(flat_g), "first": True,
+                self._flat.append({"p": b.flattened, "g": flat_g, "m": torch.zeros_like(flat_g),
                                    "runs": self._group_runs(b)})
                 continue
             if b.flattened is None or any(t.kind != "grad" for t in b.tensors):
@@ -117,8 +120,7 @@ class FlatSGD(torch.optim.Optimizer):
                     p.set_(flat_p.untyped_storage(), off, shape, stride)
                     self._attached_ids.add(id(p))
                     off += n
-            entry = {"p": flat_p, "g": b.flattened, "m": torch.zeros_like(flat_p), "first": True,
-                     "runs": self._group_runs(b)}
+            entry = {"p": flat_p, "g": b.flattened, "m": torch.zeros_like(flat_p), "runs": self._group_runs(b)}
             if self.bf16_shadow:
                 from ..ops.shadow import BF16Shadow
 
@@ -132,60 +134,63 @@ class FlatSGD(torch.optim.Optimizer):
                     off += n
                 entry["h"] = flat_h
             self._flat.append(entry)
+        # one entry per run of parameters that share a parameter group (usually one per bucket), stepped with
+        # its own group's hyperparameters as they are at the time (schedulers change them in place)
+        self._plan = _C.SgdPlan() if self._flat else None
+        for f in self._flat:
+            for lo, hi, gi in f["runs"]:
+                self._plan.add(f["p"][lo:hi], f["g"][lo:hi], f["m"][lo:hi], f["h"][lo:hi] if "h" in f else None, gi)
+
+    def _stream(self):
+        t = self._flat[0]["p"]
+        return torch.cuda.current_stream(t.device).cuda_stream if t.is_cuda else 0
+
+    def _loose_params(self):
+        """[(group, parameter)] outside the flat buffers; looked up again when a group has grown."""
+        n = sum(len(g["params"]) for g in self.param_groups)
+        if self._loose is None or self._loose[0] != n:
+            self._loose = (n, [(g, p) for g in self.param_groups for p in g["params"] if id(p) not in self._attached_ids])
+        return self._loose[1]
 
     @torch.no_grad()
     def step(self, closure=None):
         loss = closure() if closure is not None else None
-        stream = torch.cuda.current_stream().cuda_stream if (self._flat and self._flat[0]["p"].is_cuda) else 0
-        for f in self._flat:
-            # one launch per run of parameters that share a parameter group (usually one per bucket),
-            # each with its own group's hyperparameters as they are now (schedulers change them in place)
-            whole = len(f["runs"]) == 1
-            for lo, hi, gi in f["runs"]:
-                g = self.param_groups[gi]
-                p_, g_, m_ = (f["p"], f["g"], f["m"]) if whole else (f["p"][lo:hi], f["g"][lo:hi], f["m"][lo:hi])
-                if "h" in f:
-                    h_ = f["h"] if whole else f["h"][lo:hi]
-                    _C.k_sgd_momentum_flat_shadow(p_, g_, m_, h_, g["lr"], g["momentum"], g["dampening"],
-                                                  g["weight_decay"], g["nesterov"], f["first"], stream)
-                else:
-                    _C.k_sgd_momentum_flat(p_, g_, m_, g["lr"], g["momentum"], g["dampening"], g["weight_decay"],
-                                           g["nesterov"], f["first"], stream)
-                self.kernel_launches += 1
-            f["first"] = False
+        if self._plan is not None:
+            self.kernel_launches += self._plan.step(
+                [(g["lr"], g["momentum"], g["dampening"], g["weight_decay"], g["nesterov"]) for g in self.param_groups],
+                self._stream())
         if self._shadowed and not self.shadows_valid:
             self._validate_shadows()
-        for group in self.param_groups:
-            for p in group["params"]:
-                if id(p) in self._attached_ids or p.grad is None:
-                    continue
-                st = self.state[p]
-                first = "momentum_buffer" not in st
-                if first:
-                    st["momentum_buffer"] = torch.zeros_like(p, memory_format=torch.preserve_format)
-                buf = st["momentum_buffer"]
-                same_layout = (p.dtype == torch.float32 and _is_dense(p) and p.grad.dtype == torch.float32
-                               and p.grad.stride() == p.stride() and buf.stride() == p.stride())
-                if not same_layout:
-                    # layouts differ (e.g. autograd produced a contiguous gradient for a
-                    # channels_last weight): element-wise torch math is layout-agnostic
-                    d = p.grad.add(p, alpha=group["weight_decay"]) if group["weight_decay"] else p.grad
-                    if group["momentum"]:
-                        if first:
-                            buf.copy_(d)
-                        else:
-                            buf.mul_(group["momentum"]).add_(d, alpha=1 - group["dampening"])
-                        d = d.add(buf, alpha=group["momentum"]) if group["nesterov"] else buf
-                    p.add_(d, alpha=-group["lr"])
-                    continue
-                s = torch.cuda.current_stream().cuda_stream if p.is_cuda else 0
-                # dense tensors with equal strides can be updated as flat memory
-                pv = torch.as_strided(p, (p.numel(),), (1,))
-                gv = torch.as_strided(p.grad, (p.numel(),), (1,))
-                mv = torch.as_strided(st["momentum_buffer"], (p.numel(),), (1,))
-                _C.k_sgd_momentum_flat(pv, gv, mv, group["lr"], group["momentum"], group["dampening"],
-                                       group["weight_decay"], group["nesterov"], first, s)
-                self.kernel_launches += 1
+        for group, p in self._loose_params():
+            if p.grad is None:
+                continue
+            st = self.state[p]
+            first = "momentum_buffer" not in st
+            if first:
+                st["momentum_buffer"] = torch.zeros_like(p, memory_format=torch.preserve_format)
+            buf = st["momentum_buffer"]
+            same_layout = (p.dtype == torch.float32 and _is_dense(p) and p.grad.dtype == torch.float32
+                           and p.grad.stride() == p.stride() and buf.stride() == p.stride())
+            if not same_layout:
+                # layouts differ (e.g. autograd produced a contiguous gradient for a
+                # channels_last weight): element-wise torch math is layout-agnostic
+                d = p.grad.add(p, alpha=group["weight_decay"]) if group["weight_decay"] else p.grad
+                if group["momentum"]:
+                    if first:
+                        buf.copy_(d)
+                    else:
+                        buf.mul_(group["momentum"]).add_(d, alpha=1 - group["dampening"])
+                    d = d.add(buf, alpha=group["momentum"]) if group["nesterov"] else buf
+                p.add_(d, alpha=-group["lr"])
+                continue
+            s = torch.cuda.current_stream().cuda_stream if p.is_cuda else 0
+            # dense tensors with equal strides can be updated as flat memory
+            pv = torch.as_strided(p, (p.numel(),), (1,))
+            gv = torch.as_strided(p.grad, (p.numel(),), (1,))
+            mv = torch.as_strided(st["momentum_buffer"], (p.numel(),), (1,))
+            _C.k_sgd_momentum_flat(pv, gv, mv, group["lr"], group["momentum"], group["dampening"],
+                                   group["weight_decay"], group["nesterov"], first, s)
+            self.kernel_launches += 1
         self._steps += 1
         return loss
 
@@ -208,9 +213,8 @@ class FlatSGD(torch.optim.Optimizer):
     def zero_grad(self, set_to_none: bool = False):
         """Zero the flat gradient buffers with one memset per bucket; gradients stay views
         of the bucket (never set to None, which would detach them from the bucket)."""
-        for f in self._flat:
-            f["g"].zero_()
-        for group in self.param_groups:
-            for p in group["params"]:
-                if id(p) not in self._attached_ids and p.grad is not None:
-                    p.grad.zero_()
+        if self._plan is not None:
+            self._plan.zero_grad(self._stream())
+        for _, p in self._loose_params():
+            if p.grad is not None:
+                p.grad.zero_()

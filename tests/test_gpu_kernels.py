@@ -392,3 +392,35 @@ def test_minmax_uint8_values_large_against_their_range_and_not_finite():
     x[[5, 70000]] = float("nan")
     a = bc.BaguaTensorPy(x.cuda(), "x").compress("MinMaxUInt8", 1, -1).to_numpy_u8()
     assert a[32 + 5] == 255 and a[32 + 70000] == 255  # NaN takes the highest level
+
+
+def test_sgd_plan_steps_slices_of_several_buffers_with_their_groups():
+    """One launch over buffers of every alignment and size (below a tile, several tiles, none of a multiple of four),
+    more than one table of them, against the one-buffer kernel; zero_grad clears exactly the gradients."""
+    import bagua_core_b200 as bb
+
+    C, st = bb._C, torch.cuda.current_stream().cuda_stream
+    sizes = [1, 3, 4, 2047, 2048, 2049, 100001, 7, 64, 4096] * 5
+    g = torch.Generator().manual_seed(2)
+    flat = [torch.randn(sum(sizes) + 1, generator=g).cuda()[1:] for _ in range(3)]
+    ref = [t.clone() for t in flat]
+    shadow = torch.zeros(sum(sizes), dtype=torch.bfloat16, device="cuda")
+    plan, off, parts = C.SgdPlan(), 0, []
+    for i, n in enumerate(sizes):
+        sl = slice(off, off + n)
+        plan.add(flat[0][sl], flat[1][sl], flat[2][sl], shadow[sl] if i % 2 else None, i % 3)
+        parts.append((sl, i))
+        off += n
+    groups = [(0.1, 0.9, 0.0, 1e-4, False), (0.01, 0.0, 0.0, 0.0, False), (0.05, 0.8, 0.0, 1e-3, True)]
+    for step in range(2):
+        assert plan.step(groups, st) == 2  # 50 buffers, 40 to a launch
+        for sl, i in parts:
+            a = [t[sl].clone() for t in ref]  # aligned copies: the same arithmetic
+            C.k_sgd_momentum_flat(a[0], a[1], a[2], *groups[i % 3], step == 0, st)
+            ref[0][sl], ref[2][sl] = a[0], a[2]
+    torch.cuda.synchronize()
+    assert torch.equal(flat[0], ref[0]) and torch.equal(flat[2], ref[2]) and torch.equal(flat[1], ref[1])
+    for sl, i in parts:
+        assert torch.equal(shadow[sl], flat[0][sl].bfloat16() if i % 2 else torch.zeros_like(shadow[sl]))
+    plan.zero_grad(st)
+    assert not flat[1].any() and torch.equal(flat[0], ref[0])
