@@ -54,6 +54,7 @@ SOURCES = [
     "kernels/no_alloc.cu",
     "kernels/model_ops.cu",
     "kernels/model_ops_cpu.cc",
+    "kernels/encoder_ops.cu",
 ]
 
 

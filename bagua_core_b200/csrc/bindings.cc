@@ -838,12 +838,20 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
 
   // ---- trainer: autograd functions and gradient hooks ---------------------------------
   m.def("linear", &trainer::linear, py::arg("x"), py::arg("weight"), py::arg("bias"), py::arg("weight_bf16"),
-        py::arg("accumulate"),
-        "x @ weight.T + bias in bf16; with `accumulate`, the backward adds the parameters' gradients to their fp32 .grad "
+        py::arg("accumulate"), py::arg("gelu") = false,
+        "x @ weight.T + bias in bf16, through gelu if asked for; with `accumulate`, the backward adds the parameters' gradients to their fp32 .grad "
         "itself where that changes nothing a user sees.");
   m.def("conv_bias_relu", &trainer::conv_bias_relu, py::arg("x"), py::arg("weight"), py::arg("bias"), py::arg("stride"),
         py::arg("padding"), py::arg("dilation"), py::arg("groups"), py::arg("pool"), py::arg("weight_bf16"),
         py::arg("accumulate"), "max(conv(x, weight) + bias, 0), followed by 2x2 pooling with `pool`.");
+  m.def("gelu_fusable", &trainer::gelu_fusable, py::arg("x"), py::arg("out_features"));
+  m.def("add_layer_norm", &trainer::add_layer_norm, py::arg("x"), py::arg("residual"), py::arg("weight"), py::arg("bias"),
+        py::arg("eps"), py::arg("accumulate"), "layer_norm(x + residual) of bf16 activations with fp32 parameters.");
+  m.def("embed_layer_norm", &trainer::embed_layer_norm, py::arg("ids"), py::arg("tokens"), py::arg("positions"),
+        py::arg("types"), py::arg("weight"), py::arg("bias"), py::arg("eps"), py::arg("accumulate"),
+        "layer_norm(tokens[ids] + positions[:seq] + types[0]) in bf16.");
+  m.def("attention", &trainer::attention, py::arg("qkv"), py::arg("heads"), py::arg("dropout"),
+        "Multi-head attention of a packed bf16 projection (the attention kernel is the library's).");
   m.def("op_stats", []() {
     auto& s = trainer::OpStats::global();
     py::dict d;

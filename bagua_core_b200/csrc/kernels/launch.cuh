@@ -19,17 +19,23 @@ __device__ __forceinline__ void let_successor_start() { asm volatile("griddepcon
 // The kernel's blocks are scheduled, and run up to wait_for_predecessor(), while the kernel in front
 // of it ends: about 1 us less between two short kernels.
 template <typename... P, typename... A>
-inline void launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A... args) {
+inline void launch_overlapped_shared(void (*kernel)(P...), dim3 grid, dim3 block, size_t shared, cudaStream_t s, A... args) {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
+  cfg.dynamicSmemBytes = shared;
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   BAGUA_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+}
+
+template <typename... P, typename... A>
+inline void launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A... args) {
+  launch_overlapped_shared(kernel, grid, block, 0, s, args...);
 }
 
 // All blocks of the grid are resident together, or the launch fails.

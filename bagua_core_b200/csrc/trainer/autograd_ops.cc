@@ -13,6 +13,7 @@
 #include <unordered_map>
 
 #include "../common.h"
+#include "../kernels/encoder_ops.h"
 #include "../kernels/kernels.h"
 #include "../kernels/model_ops.h"
 #include "../tensor/tensor.h"
@@ -168,16 +169,17 @@ std::shared_ptr<PoolRawTensor> scratch_for(const at::Tensor& t, size_t bytes) {
 
 // ---- linear ------------------------------------------------------------------------------------
 struct LinearNode : public Node {
-  SavedVariable x, w;
+  SavedVariable x, w, z;  // z: what gelu was applied to, when it was
   at::Tensor weight, bias;  // the parameters (bias may be undefined)
   std::shared_ptr<Use> use;  // set when gradients are to be accumulated here
-  bool accumulate = false;
+  bool accumulate = false, gelu = false;
 
-  std::string name() const override { return "BaguaLinearBackward"; }
+  std::string name() const override { return gelu ? "BaguaLinearGeluBackward" : "BaguaLinearBackward"; }
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
     x.reset_data();
     w.reset_data();
+    z.reset_data();
   }
 
   variable_list apply(variable_list&& grads) override {
@@ -188,6 +190,7 @@ struct LinearNode : public Node {
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
     const at::Tensor dy = grads[0], xs = x.unpack(), ws = w.unpack();
     at::Tensor dy2 = dy.dim() == 2 ? dy : dy.reshape({-1, dy.size(-1)});
+    if (gelu) dy2 = through_gelu(dy2.contiguous(), out);
     if (task_should_compute_output(0)) {
       at::Tensor dx = at::mm(dy2, ws);
       out[0] = dy.dim() == 2 ? dx : dx.view(xs.sizes());
@@ -205,8 +208,25 @@ struct LinearNode : public Node {
       }
       if (!done) out[1] = at::mm(dy2.t(), x2);  // autograd casts it to the parameter's type
     }
-    if (bias.defined() && task_should_compute_output(2)) out[2] = bias_grad(dy2);
+    if (!gelu && bias.defined() && task_should_compute_output(2)) out[2] = bias_grad(dy2);
     return out;
+  }
+
+  // gelu' applied to the incoming gradient, and the bias gradient of the result from the same pass
+  at::Tensor through_gelu(const at::Tensor& dy2, variable_list& out) {
+    const at::Tensor zs = z.unpack();
+    const int64_t rows = dy2.size(0);
+    const int C = (int)dy2.size(1);
+    const bool want = bias.defined() && task_should_compute_output(2);
+    const bool add = want && accumulate && use && !use->shared && accumulates(bias, dy2);
+    at::Tensor db = add ? bias.grad() : at::empty({C}, dy2.options().dtype(at::kFloat));
+    at::Tensor dz = at::empty_like(dy2);
+    auto scratch = scratch_for(dy2, encoder_ops::gelu_backward_scratch_bytes(rows, C));
+    encoder_ops::gelu_backward(dy2.data_ptr(), zs.data_ptr(), dz.data_ptr(), db.data_ptr<float>(), add, scratch->data_ptr(),
+                               rows, C, stream_of(dy2));
+    count_launches(2);
+    if (want && !add) out[2] = db;
+    return dz;
   }
 
   at::Tensor bias_grad(const at::Tensor& dy2) {
@@ -303,14 +323,127 @@ struct ConvNode : public Node {
   }
 };
 
+// ---- encoder layers ------------------------------------------------------------------------------
+// An fp32 gradient for `param`: its `.grad` to be added to, or a new tensor for autograd.
+struct GradTarget {
+  at::Tensor grad;
+  bool add;
+};
+GradTarget grad_target(const at::Tensor& param, bool accumulate, bool zeroed) {
+  if (accumulate && accumulates(param, param) && param.grad().is_contiguous()) return {param.grad(), true};
+  return {zeroed ? at::zeros(param.sizes(), param.options()) : at::empty(param.sizes(), param.options()), false};
+}
+
+struct LayerNormNode : public Node {
+  SavedVariable sum, mean, rstd;
+  at::Tensor gamma, beta;
+  bool accumulate = false, residual = false;
+
+  std::string name() const override { return "BaguaAddLayerNormBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    sum.reset_data();
+    mean.reset_data();
+    rstd.reset_data();
+  }
+  variable_list apply(variable_list&& grads) override {  // x, r, gamma, beta
+    std::lock_guard<std::mutex> lock(mutex_);
+    variable_list out(4);
+    if (!grads[0].defined()) return out;
+    const at::Tensor dy = grads[0].contiguous(), s = sum.unpack(), m = mean.unpack(), rs = rstd.unpack();
+    const int H = (int)s.size(-1);
+    const int64_t rows = s.numel() / H;
+    at::Tensor ds = at::empty_like(s);
+    const GradTarget dg = grad_target(gamma, accumulate && task_should_compute_output(2), false);
+    const GradTarget db = grad_target(beta, accumulate && task_should_compute_output(3), false);
+    auto scratch = scratch_for(s, encoder_ops::layer_norm_backward_scratch_bytes(rows, H));
+    encoder_ops::layer_norm_backward(dy.data_ptr(), s.data_ptr(), gamma.data_ptr<float>(), m.data_ptr<float>(),
+                                     rs.data_ptr<float>(), ds.data_ptr(), dg.grad.data_ptr<float>(), db.grad.data_ptr<float>(),
+                                     dg.add, db.add, scratch->data_ptr(), rows, H, stream_of(s));
+    count_launches(2);
+    out[0] = ds;
+    if (residual) out[1] = ds;
+    if (!dg.add) out[2] = dg.grad;
+    if (!db.add) out[3] = db.grad;
+    return out;
+  }
+};
+
+struct EmbedNode : public Node {
+  SavedVariable ids, mean, rstd;
+  at::Tensor param[5];  // tok, pos, typ, gamma, beta
+  bool accumulate = false;
+
+  std::string name() const override { return "BaguaEmbedLayerNormBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    ids.reset_data();
+    mean.reset_data();
+    rstd.reset_data();
+  }
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    variable_list out(5);
+    if (!grads[0].defined()) return out;
+    const at::Tensor dy = grads[0].contiguous(), id = ids.unpack(), m = mean.unpack(), rs = rstd.unpack();
+    const int H = (int)param[0].size(1);
+    const int64_t batch = id.size(0), seq = id.size(1);
+    GradTarget to[5];
+    for (int k = 0; k < 5; ++k) to[k] = grad_target(param[k], accumulate && task_should_compute_output((size_t)k), true);
+    at::Tensor ds = at::empty({batch * seq, H}, dy.options().dtype(at::kFloat));
+    auto scratch = scratch_for(dy, encoder_ops::embed_backward_scratch_bytes(batch * seq, H));
+    encoder_ops::embed_layer_norm_backward(
+        dy.data_ptr(), id.data_ptr<int64_t>(), param[0].size(0), param[0].data_ptr<float>(), param[1].data_ptr<float>(),
+        param[2].data_ptr<float>(), param[3].data_ptr<float>(), m.data_ptr<float>(), rs.data_ptr<float>(), ds.data_ptr<float>(),
+        to[0].grad.data_ptr<float>(), to[1].grad.data_ptr<float>(), to[2].grad.data_ptr<float>(), to[3].grad.data_ptr<float>(),
+        to[4].grad.data_ptr<float>(), scratch->data_ptr(), batch, seq, H, stream_of(dy));
+    count_launches(3);
+    for (int k = 0; k < 5; ++k)
+      if (!to[k].add) out[(size_t)k] = to[k].grad;
+    return out;
+  }
+};
+
+// q, k, v as views of the packed projection; backward writes their gradients into one packed tensor.
+struct SplitHeadsNode : public Node {
+  int64_t batch = 0, seq = 0, heads = 0, dim = 0;
+  at::TensorOptions options;
+
+  std::string name() const override { return "BaguaSplitHeadsBackward"; }
+  variable_list apply(variable_list&& grads) override {
+    variable_list out(1);
+    at::Tensor packed = at::empty({batch, seq, 3 * heads * dim}, options);
+    const void* src[3];
+    encoder_ops::HeadStrides st[3];
+    at::Tensor keep[3];
+    for (int q = 0; q < 3; ++q) {
+      at::Tensor g = grads[(size_t)q].defined() ? grads[(size_t)q] : at::zeros({batch, heads, seq, dim}, options);
+      const bool direct = g.stride(3) == 1 && g.stride(0) % 8 == 0 && g.stride(1) % 8 == 0 && g.stride(2) % 8 == 0 &&
+                          (uintptr_t)g.data_ptr() % 16 == 0;
+      keep[q] = direct ? g : g.contiguous();
+      src[q] = keep[q].data_ptr();
+      st[q] = encoder_ops::HeadStrides{keep[q].stride(0), keep[q].stride(1), keep[q].stride(2)};
+    }
+    encoder_ops::merge_heads(src, st, packed.data_ptr(), batch, seq, (int)heads, (int)dim, stream_of(packed));
+    count_launches(1);
+    out[0] = packed;
+    return out;
+  }
+};
+
+bool fp32_param(const at::Tensor& p, int64_t H, const at::Tensor& like) {
+  return p.scalar_type() == at::kFloat && p.is_contiguous() && p.size(-1) == H && p.device() == like.device();
+}
+
 }  // namespace
 
 at::Tensor linear(const at::Tensor& x, const at::Tensor& weight, const std::optional<at::Tensor>& bias,
-                  const std::optional<at::Tensor>& w_low, bool accumulate) {
+                  const std::optional<at::Tensor>& w_low, bool accumulate, bool gelu) {
+  BAGUA_CHECK(!gelu || gelu_fusable(x, weight.size(0)), Tensor, "gelu cannot be fused with this layer");
   const at::Tensor b = bias.value_or(at::Tensor());
   std::shared_ptr<LinearNode> node;
   if (torch::autograd::compute_requires_grad(x, weight, b)) node = make_node<LinearNode>(x, weight, b);
-  at::Tensor xs, ws, y;
+  at::Tensor xs, ws, z, y;
   {
     PlainDispatch plain;
     std::array<at::Tensor, 3> low{x, w_low ? *w_low : weight, b};
@@ -318,10 +451,18 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& weight, const std::opti
     xs = low[0];
     ws = low[1];
     y = at::linear(xs, ws, b.defined() ? std::optional<at::Tensor>(low[2]) : std::nullopt);
+    if (gelu) {
+      z = y.contiguous();
+      y = at::empty_like(z);
+      encoder_ops::gelu_forward(z.data_ptr(), y.data_ptr(), z.numel(), stream_of(z));
+      count_launches(1);
+    }
   }
   if (node) {
     node->x = SavedVariable(xs, false);
     node->w = SavedVariable(ws, false);
+    if (gelu) node->z = SavedVariable(z, false);
+    node->gelu = gelu;
     node->weight = weight;
     node->bias = b;
     node->accumulate = accumulate;
@@ -393,6 +534,115 @@ at::Tensor conv_bias_relu(const at::Tensor& x, const at::Tensor& weight, const a
     }
   }
   return out;
+}
+
+at::Tensor add_layer_norm(const at::Tensor& x, const std::optional<at::Tensor>& r, const at::Tensor& gamma,
+                          const at::Tensor& beta, double eps, bool accumulate) {
+  const int64_t H = x.size(-1), rows = x.numel() / H;
+  const at::Tensor res = r.value_or(at::Tensor());
+  BAGUA_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && encoder_ops::row_supported(rows, H) &&
+                  fp32_param(gamma, H, x) && fp32_param(beta, H, x) && gamma.dim() == 1 && beta.dim() == 1 &&
+                  (!res.defined() || (res.sizes() == x.sizes() && res.scalar_type() == at::kBFloat16 && res.device() == x.device())),
+              Tensor, "add_layer_norm needs bf16 CUDA activations of one shape and fp32 parameters");
+  std::shared_ptr<LayerNormNode> node;
+  if (torch::autograd::compute_requires_grad(x, res, gamma, beta)) {
+    node = std::shared_ptr<LayerNormNode>(new LayerNormNode(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(x, res, gamma, beta));
+  }
+  at::Tensor sum, y, mean, rstd;
+  {
+    PlainDispatch plain;
+    const at::Tensor xs = x.contiguous(), rc = res.defined() ? res.contiguous() : res;
+    y = at::empty_like(xs);
+    sum = res.defined() ? at::empty_like(xs) : xs;
+    mean = at::empty({2, rows}, xs.options().dtype(at::kFloat));
+    rstd = mean.select(0, 1);
+    mean = mean.select(0, 0);
+    encoder_ops::add_layer_norm_forward(xs.data_ptr(), res.defined() ? rc.data_ptr() : nullptr, gamma.data_ptr<float>(),
+                                        beta.data_ptr<float>(), (float)eps, res.defined() ? sum.data_ptr() : nullptr, y.data_ptr(),
+                                        mean.data_ptr<float>(), rstd.data_ptr<float>(), rows, (int)H, stream_of(xs));
+    count_launches(1);
+  }
+  if (node) {
+    node->sum = SavedVariable(sum, false);
+    node->mean = SavedVariable(mean, false);
+    node->rstd = SavedVariable(rstd, false);
+    node->gamma = gamma;
+    node->beta = beta;
+    node->accumulate = accumulate;
+    node->residual = res.defined();
+    torch::autograd::set_history(y, node);
+  }
+  return y;
+}
+
+at::Tensor embed_layer_norm(const at::Tensor& ids, const at::Tensor& tok, const at::Tensor& pos, const at::Tensor& typ,
+                            const at::Tensor& gamma, const at::Tensor& beta, double eps, bool accumulate) {
+  const int64_t H = tok.size(1);
+  BAGUA_CHECK(ids.is_cuda() && ids.scalar_type() == at::kLong && ids.dim() == 2 && ids.numel() <= encoder_ops::kMaxTokens &&
+                  encoder_ops::row_supported(ids.numel(), H),
+              Tensor, "embed_layer_norm: unsupported ids");
+  for (const at::Tensor* p : {&tok, &pos, &typ, &gamma, &beta})
+    BAGUA_CHECK(fp32_param(*p, H, ids), Tensor, "embed_layer_norm needs fp32 tables on the ids' device");
+  BAGUA_CHECK(ids.size(1) <= pos.size(0), Tensor, "sequence of " << ids.size(1) << " tokens, " << pos.size(0) << " positions");
+  std::shared_ptr<EmbedNode> node;
+  if (torch::autograd::compute_requires_grad(tok, pos, typ, gamma, beta)) {
+    node = std::shared_ptr<EmbedNode>(new EmbedNode(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(tok, pos, typ, gamma, beta));
+  }
+  at::Tensor idc, y, mean, rstd;
+  {
+    PlainDispatch plain;
+    idc = ids.contiguous();
+    const int64_t batch = ids.size(0), seq = ids.size(1);
+    y = at::empty({batch, seq, H}, tok.options().dtype(at::kBFloat16));
+    mean = at::empty({2, batch * seq}, tok.options());
+    rstd = mean.select(0, 1);
+    mean = mean.select(0, 0);
+    encoder_ops::embed_layer_norm_forward(idc.data_ptr<int64_t>(), tok.size(0), tok.data_ptr<float>(), pos.data_ptr<float>(),
+                                          typ.data_ptr<float>(), gamma.data_ptr<float>(), beta.data_ptr<float>(), (float)eps,
+                                          y.data_ptr(), mean.data_ptr<float>(), rstd.data_ptr<float>(), batch, seq, (int)H,
+                                          stream_of(tok));
+    count_launches(1);
+  }
+  if (node) {
+    node->ids = SavedVariable(idc, false);
+    node->mean = SavedVariable(mean, false);
+    node->rstd = SavedVariable(rstd, false);
+    const at::Tensor* ps[5] = {&tok, &pos, &typ, &gamma, &beta};
+    for (int k = 0; k < 5; ++k) node->param[k] = *ps[k];
+    node->accumulate = accumulate;
+    torch::autograd::set_history(y, node);
+  }
+  return y;
+}
+
+at::Tensor attention(const at::Tensor& qkv, int64_t heads, double dropout) {
+  BAGUA_CHECK(qkv.is_cuda() && qkv.dim() == 3 && qkv.scalar_type() == at::kBFloat16 && qkv.size(2) % (3 * heads * 8) == 0,
+              Tensor, "attention needs a packed bf16 projection [batch, seq, 3 * heads * dim] with dim a multiple of 8");
+  const int64_t B = qkv.size(0), S = qkv.size(1), W = qkv.size(2), D = W / (3 * heads);
+  variable_list parts;
+  std::shared_ptr<SplitHeadsNode> node;
+  if (torch::autograd::compute_requires_grad(qkv)) {
+    node = std::shared_ptr<SplitHeadsNode>(new SplitHeadsNode(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(qkv));
+  }
+  {
+    PlainDispatch plain;
+    const at::Tensor c = qkv.contiguous();
+    for (int64_t q = 0; q < 3; ++q)
+      parts.push_back(c.detach().as_strided({B, heads, S, D}, {S * W, D, W, 1}, c.storage_offset() + q * heads * D));
+  }
+  if (node) {
+    node->batch = B;
+    node->seq = S;
+    node->heads = heads;
+    node->dim = D;
+    node->options = qkv.options();
+    for (at::Tensor& t : parts) torch::autograd::set_history(t, node);
+  }
+  const at::Tensor a = at::scaled_dot_product_attention(parts[0], parts[1], parts[2], c10::nullopt, dropout);
+  return a.transpose(1, 2).reshape({B, S, heads * D});
 }
 
 }  // namespace trainer

@@ -25,8 +25,23 @@ struct OpStats {
 // y = x Wᵀ + b in bf16.  `w_low`: W in bf16 when the caller has it, else it is cast here.  With `accumulate`, the
 // backward adds the gradients of W and b to their fp32 `.grad` itself where nobody can tell the difference
 // (autograd_ops.cc, `accumulates`), and hands autograd nothing for them.
+// `gelu`: y = gelu(x Wᵀ + b), whose backward makes the bias gradient in the pass that applies gelu' (needs
+// gelu_fusable()).
 at::Tensor linear(const at::Tensor& x, const at::Tensor& weight, const std::optional<at::Tensor>& bias,
-                  const std::optional<at::Tensor>& w_low, bool accumulate);
+                  const std::optional<at::Tensor>& w_low, bool accumulate, bool gelu);
+inline bool gelu_fusable(const at::Tensor& x, int64_t out_features) { return x.is_cuda() && out_features % 8 == 0 && x.numel() > 0; }
+
+// layer_norm(x + r) of bf16 activations with fp32 parameters (r may be missing); CUDA, `encoder_ops::row_supported`.
+at::Tensor add_layer_norm(const at::Tensor& x, const std::optional<at::Tensor>& r, const at::Tensor& gamma,
+                          const at::Tensor& beta, double eps, bool accumulate);
+
+// layer_norm(tok[ids] + pos[: seq] + typ[0]) in bf16 from fp32 tables; ids [batch, seq] of int64, at most
+// `encoder_ops::kMaxTokens` of them.
+at::Tensor embed_layer_norm(const at::Tensor& ids, const at::Tensor& tok, const at::Tensor& pos, const at::Tensor& typ,
+                            const at::Tensor& gamma, const at::Tensor& beta, double eps, bool accumulate);
+
+// Multi-head attention of a packed projection qkv [batch, seq, 3 * heads * dim] (bf16, CUDA): [batch, seq, heads * dim].
+at::Tensor attention(const at::Tensor& qkv, int64_t heads, double dropout);
 
 // max(conv(x, weight) + bias, 0), channels-last, followed by 2x2 pooling with `pool`.  Inside an autocast region
 // x, weight and bias are taken in its type (the weight from `w_low` when given).

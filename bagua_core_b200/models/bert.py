@@ -6,7 +6,12 @@ initialisation only.
 The encoder's projections are `ShadowLinear` modules: `nn.Linear` (same parameter names, same
 math) unless an optimizer keeps bf16 copies of the weights (`FlatSGD(bf16_shadow=True)`) or
 in-place weight-gradient accumulation is on (`bagua_core_b200.ops.wgrad.enabled`), in which case
-they skip the per-forward weight casts and the cast-and-add of every weight gradient."""
+they skip the per-forward weight casts and the cast-and-add of every weight gradient.
+
+Under bf16 autocast on a GPU what lies between the projections runs as this package's kernels
+(`csrc/kernels/encoder_ops.h`): residual sum + LayerNorm, the embedding sum + LayerNorm, GELU with the
+projection in front of it, the packing of the attention gradients.  Parameters, results (to the
+rounding of bf16) and everything else stay those of the plain composition below, which runs elsewhere."""
 from __future__ import annotations
 
 from dataclasses import dataclass
@@ -15,7 +20,12 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from .._native import C as _C
+from ..ops import wgrad
 from ..ops.fused_linear import ShadowLinear
+
+
+_EMBED_TOKENS = 4096  # encoder_ops::kMaxTokens: more tokens per batch take the framework's embedding
 
 
 @dataclass
@@ -64,6 +74,13 @@ class _LayerNorm(nn.LayerNorm):
             return F.layer_norm(x, self.normalized_shape, self.weight.to(x.dtype), self.bias.to(x.dtype), self.eps)
 
 
+def _fused(x: torch.Tensor, ln: nn.LayerNorm) -> bool:
+    """Whether the fused kernels take this activation: bf16 autocast on a GPU, fp32 parameters."""
+    return (x.is_cuda and isinstance(ln, _LayerNorm) and torch.is_autocast_enabled("cuda")
+            and torch.get_autocast_dtype("cuda") == torch.bfloat16
+            and ln.weight.dtype == torch.float32 and ln.weight.shape[0] % 8 == 0 and ln.weight.shape[0] <= 1024)
+
+
 def _layer_norm(c: "BertConfig") -> nn.LayerNorm:
     return (nn.LayerNorm if c.fp32_layernorm_io else _LayerNorm)(c.hidden, eps=c.eps)
 
@@ -83,12 +100,22 @@ class _Layer(nn.Module):
 
     def forward(self, x):
         b, s, h = x.shape
+        if x.dtype == torch.bfloat16 and _fused(x, self.ln1) and (h // self.heads) % 8 == 0 and x.numel() > 0:
+            p = self.p if self.training else 0.0
+            a = self.proj(_C.attention(self.qkv(x), self.heads, p))
+            x = self._add_norm(self.ln1, x, self.drop(a) if p else a)
+            f = self.fc2(self.fc1(x, gelu=True))
+            return self._add_norm(self.ln2, x, self.drop(f) if p else f)
         q, k, v = self.qkv(x).view(b, s, 3, self.heads, h // self.heads).permute(2, 0, 3, 1, 4)
         a = F.scaled_dot_product_attention(q, k, v, dropout_p=self.p if self.training else 0.0)
         a = a.transpose(1, 2).reshape(b, s, h)
         x = self.ln1(x + self.drop(self.proj(a)))
         f = self.fc2(F.gelu(self.fc1(x)))
         return self.ln2(x + self.drop(f))
+
+    @staticmethod
+    def _add_norm(ln, x, branch):
+        return _C.add_layer_norm(x, branch, ln.weight, ln.bias, ln.eps, wgrad.enabled)
 
 
 class BertForQuestionAnswering(nn.Module):
@@ -114,9 +141,14 @@ class BertForQuestionAnswering(nn.Module):
 
     def forward(self, input_ids, start_positions=None, end_positions=None):
         b, s = input_ids.shape
-        pos = torch.arange(s, device=input_ids.device)
-        x = self.tok(input_ids) + self.pos(pos)[None] + self.typ.weight[0][None, None]
-        x = self.drop(self.ln(x))
+        if (_fused(self.tok.weight, self.ln) and input_ids.is_cuda and input_ids.dtype == torch.int64
+                and 0 < b * s <= _EMBED_TOKENS and s <= self.pos.num_embeddings):
+            x = _C.embed_layer_norm(input_ids, self.tok.weight, self.pos.weight, self.typ.weight, self.ln.weight,
+                                    self.ln.bias, self.ln.eps, wgrad.enabled)
+        else:
+            pos = torch.arange(s, device=input_ids.device)
+            x = self.ln(self.tok(input_ids) + self.pos(pos)[None] + self.typ.weight[0][None, None])
+        x = self.drop(x)
         for layer in self.layers:
             x = layer(x)
         logits = self.qa(x).float()

@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import torch
 import torch.nn as nn
+import torch.nn.functional as F
 
 from .._native import C as _C
 from . import shadow as _shadow
@@ -22,11 +23,15 @@ from . import wgrad as _wgrad
 
 
 class ShadowLinear(nn.Linear):
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
+    def forward(self, x: torch.Tensor, gelu: bool = False) -> torch.Tensor:
+        """`gelu`: followed by GELU, in the same autograd function where the layer runs natively."""
         dev = x.device.type
         managed = getattr(self.weight, "_bagua_bf16", None) is not None  # an optimizer keeps a bf16 copy
         if ((managed or _wgrad.enabled) and torch.is_autocast_enabled(dev)
                 and torch.get_autocast_dtype(dev) == torch.bfloat16):
             # the copy when it is current, a fresh cast otherwise: the same code path either way
-            return _C.linear(x, self.weight, self.bias, _shadow.autocast_copy(self.weight), _wgrad.enabled)
-        return super().forward(x)
+            fused = gelu and _C.gelu_fusable(x, self.out_features)
+            y = _C.linear(x, self.weight, self.bias, _shadow.autocast_copy(self.weight), _wgrad.enabled, fused)
+            return F.gelu(y) if gelu and not fused else y
+        y = super().forward(x)
+        return F.gelu(y) if gelu else y

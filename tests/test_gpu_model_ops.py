@@ -424,3 +424,100 @@ def test_block_gradients_added_in_place_have_the_bits_of_the_ordinary_path():
         W.enabled = saved
     for a, b in zip(*grads):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("rows,H", [(1, 8), (3, 64), (5, 264), (37, 768), (3072, 1024), (1, 1024)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_add_layer_norm_matches_fp32_math(rows, H, offset):
+    import bagua_core_b200 as bb
+
+    g = torch.Generator().manual_seed(rows + H)
+    x, r, dy = (torch.randn(rows, H, generator=g).bfloat16().cuda().requires_grad_() for _ in range(3))
+    flat = torch.randn(2 * H + 1, generator=g).cuda()
+    gamma, beta = (flat[offset + k * H:offset + (k + 1) * H].clone() if not offset else flat[offset + k * H:offset + (k + 1) * H]
+                   for k in range(2))
+    gamma, beta = gamma.detach().requires_grad_(), beta.detach().requires_grad_()
+    for res in (r, None):
+        y = bb._C.add_layer_norm(x, res, gamma, beta, 1e-12 if H > 8 else 1e-5, False)
+        grads = torch.autograd.grad(y, [t for t in (x, res, gamma, beta) if t is not None], dy.detach())
+        s = ((x.detach().float() + res.detach().float()).bfloat16() if res is not None else x.detach()).float().requires_grad_()
+        g2, b2 = gamma.detach().clone().requires_grad_(), beta.detach().clone().requires_grad_()
+        ref = torch.nn.functional.layer_norm(s, (H,), g2, b2, 1e-12 if H > 8 else 1e-5)
+        rs, rg, rb = torch.autograd.grad(ref, (s, g2, b2), dy.detach().float())
+        assert torch.allclose(y.float(), ref, rtol=1e-2, atol=2e-2)
+        assert torch.equal(grads[0], grads[1]) if res is not None else True
+        assert torch.allclose(grads[0].float(), rs, rtol=1e-2, atol=1e-2 * rs.abs().max().item())
+        assert torch.allclose(grads[-2], rg, rtol=1e-3, atol=2e-3 * rows ** 0.5)
+        assert torch.allclose(grads[-1], rb, rtol=1e-3, atol=1e-3 * rows ** 0.5)
+
+
+@pytest.mark.parametrize("batch,seq,V,same", [(1, 1, 5, 0), (3, 7, 11, 0), (8, 384, 30522, 0), (2, 300, 9, 500), (8, 512, 1000, 3000)])
+def test_embedding_sum_and_norm_match_the_plain_composition(batch, seq, V, same):
+    """`same`: that many tokens are one id (padding): above 256 its rows are added by several blocks."""
+    import bagua_core_b200 as bb
+
+    g = torch.Generator().manual_seed(seq)
+    H = 72
+    ids = torch.randint(0, V, (batch, seq), generator=g)
+    ids.view(-1)[torch.randperm(batch * seq, generator=g)[:same]] = V - 1
+    ids = ids.cuda()
+    tabs = [torch.randn(n, H, generator=g).cuda() for n in (V, 512, 2)] + [torch.randn(H, generator=g).cuda() for _ in range(2)]
+    a, b = ([t.clone().requires_grad_() for t in tabs] for _ in range(2))
+    y = bb._C.embed_layer_norm(ids, *a, 1e-12, False)
+    s = torch.nn.functional.embedding(ids, b[0]) + b[1][:seq][None] + b[2][0][None, None]
+    ref = torch.nn.functional.layer_norm(s, (H,), b[3], b[4], 1e-12)
+    dy = torch.randn(ref.shape, generator=g).bfloat16().cuda()
+    assert torch.allclose(y.float(), ref, rtol=1e-2, atol=1e-2)
+    y.backward(dy)
+    ref.backward(dy.float())
+    for p, q in zip(a, b):
+        assert torch.allclose(p.grad, q.grad, rtol=1e-3, atol=1e-4 * max(1.0, q.grad.abs().max().item())), p.shape
+
+
+@pytest.mark.parametrize("rows,n_out", [(1, 8), (9, 264), (300, 4096)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_linear_with_gelu_matches_the_plain_composition(rows, n_out, accumulate):
+    import bagua_core_b200 as bb
+
+    torch.manual_seed(rows)
+    x = torch.randn(rows, 32, device="cuda").bfloat16().requires_grad_()
+    w, b = torch.randn(n_out, 32, device="cuda", requires_grad=True), torch.randn(n_out, device="cuda", requires_grad=True)
+    for p in (w, b):
+        p.grad = torch.zeros_like(p)
+    y = bb._C.linear(x, w, b, None, accumulate, True)
+    xr, wr, br = (t.detach().bfloat16().float().requires_grad_() for t in (x, w, b))
+    z = torch.nn.functional.linear(xr, wr, br)
+    ref = torch.nn.functional.gelu(z)
+    dy = torch.randn_like(y)
+    y.backward(dy)
+    ref.backward(dy.float())
+    assert torch.allclose(y.float(), ref, rtol=2e-2, atol=5e-2)
+    for got, want in ((x.grad, xr.grad), (w.grad, wr.grad), (b.grad, br.grad)):
+        assert (got.float() - want).abs().max() <= 2e-2 * want.abs().max() + 1e-2
+
+
+def test_bert_layers_through_the_fused_kernels_agree_with_the_plain_composition():
+    from bagua_core_b200.models import BertConfig, BertForQuestionAnswering
+    from bagua_core_b200.ops import wgrad as W
+
+    saved, out = W.enabled, []
+    try:
+        for mode in ("plain", "fused", "fused, in place"):
+            torch.manual_seed(4)
+            net = BertForQuestionAnswering(BertConfig(vocab_size=500, hidden=128, layers=2, heads=4, ffn=256, dropout=0.0,
+                                                      fp32_layernorm_io=mode == "plain")).cuda()
+            W.enabled = mode.endswith("in place")
+            for p in net.parameters():
+                p.grad = torch.zeros_like(p)
+            g = torch.Generator().manual_seed(1)
+            ids = torch.randint(0, 500, (3, 40), generator=g).cuda()
+            span = torch.randint(0, 40, (3, 2), generator=g).cuda()
+            with torch.autocast("cuda", dtype=torch.bfloat16):
+                loss = net(ids, span[:, 0], span[:, 1])
+            loss.backward()
+            out.append((loss.item(), torch.cat([p.grad.reshape(-1) for p in net.parameters()])))
+    finally:
+        W.enabled = saved
+    for loss, grad in out[1:]:
+        assert abs(loss - out[0][0]) < 2e-2
+        assert (grad - out[0][1]).norm() <= 4e-2 * out[0][1].norm()
