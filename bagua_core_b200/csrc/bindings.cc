@@ -447,8 +447,14 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
            },
            py::arg("buckets"))
       .def("mark_communication_ready",
-           [](PyBackend& be, PyTensor& t, uint64_t ev) { be.inner->mark_communication_ready(t.inner, ev); },
-           py::arg("tensor"), py::arg("ready_cuda_event_ptr"), py::call_guard<py::gil_scoped_release>())
+           [](PyBackend& be, PyTensor& t, uint64_t ev) {
+             // most marks find nothing to schedule and never block: only those that do give up the GIL (a full
+             // channel waits for the worker, and the worker may need the GIL for a Python op)
+             if (be.inner->try_mark_ready(t.inner, ev)) return;
+             py::gil_scoped_release rel;
+             be.inner->schedule_ready();
+           },
+           py::arg("tensor"), py::arg("ready_cuda_event_ptr"))
       .def("wait_pending_comm_ops", [](PyBackend& be) { return be.inner->wait_pending_comm_ops(); },
            py::call_guard<py::gil_scoped_release>())
       .def("set_watchdog_timeout", [](PyBackend& be, double s) { be.inner->set_watchdog_timeout(s); })

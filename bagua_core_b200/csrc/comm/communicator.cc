@@ -232,6 +232,7 @@ void SingleCommunicator::alltoall_inplace(RawTensor& t) {
   check_live();
   BAGUA_CHECK(t.num_elements_allocated() % nranks_ == 0, Communicator,
               "alltoall: tensor size must be divisible by the number of ranks");
+  if (nranks_ == 1) return;  // what one rank exchanges with itself stays where it is
   if (PeerArena* a = p2p_arena())
     if (fused::alltoall(*a, t.data_ptr(), t.data_ptr(), t.bytes_allocated() / (size_t)nranks_, (cudaStream_t)stream_))
       return;
@@ -273,6 +274,7 @@ void SingleCommunicator::allgather_inplace(RawTensor& t) {
   check_live();
   BAGUA_CHECK(t.num_elements_allocated() % nranks_ == 0, Communicator,
               "allgather: tensor size must be divisible by the number of ranks");
+  if (nranks_ == 1) return;
   const int64_t count = t.num_elements_allocated() / nranks_;
   const size_t es = dtype_bytes(t.dtype());
   if (PeerArena* a = p2p_arena())

@@ -214,6 +214,7 @@ void sgd_momentum_flat(float* p, const float* g, float* buf, int64_t n, float lr
 void sgd_momentum_flat_shadow(float* p, const float* g, float* buf, void* shadow, int64_t n, float lr, float momentum,
                               float dampening, float wd, bool nesterov, bool first_step) {
   sgd_momentum_flat(p, g, buf, n, lr, momentum, dampening, wd, nesterov, first_step);
+  if (!shadow) return;
   uint16_t* h = static_cast<uint16_t*>(shadow);
   for (int64_t i = 0; i < n; ++i) h[i] = float_to_bf16(p[i]);
 }
@@ -248,14 +249,6 @@ void async_model_average(float* t, const float* r, const float* cp, float nranks
   c.is_cuda() ? cuda::async_model_average(t, r, cp, nranks, n, c.stream)
               : cpu::async_model_average(t, r, cp, nranks, n);
 }
-void accumulate_bf16(float* x, const void* y, int64_t n, const Ctx& c) {
-  if (n <= 0) return;
-  if (c.is_cuda()) {
-    cuda::accumulate_bf16(x, y, n, c.stream);
-    return;
-  }
-  for (int64_t i = 0; i < n; ++i) x[i] += bf16_to_float(static_cast<const uint16_t*>(y)[i]);
-}
 void copy_bytes(void* dst, const void* src, size_t bytes, const Ctx& c) {
   if (bytes == 0 || dst == src) return;
   if (c.is_cuda())
@@ -284,7 +277,7 @@ void reduce_chunk_inplace(void* x, DType dt, int64_t chunk, int n_chunks, int ta
               : cpu::reduce_chunk_inplace(x, dt, chunk, n_chunks, target, average);
 }
 size_t compress_scratch_bytes(int n_chunks, int64_t chunk_size, DType dt) {
-  return cuda::compress_scratch_bytes(n_chunks, chunk_size, dt);
+  return cuda::compress_scratch_bytes(n_chunks, chunk_size * (int64_t)dtype_bytes(dt));
 }
 
 void compress_minmax_u8(const void* in, DType dt, int64_t num_real, int64_t chunk, int n_chunks, uint8_t* out,
@@ -305,18 +298,6 @@ void decompress_minmax_u8(const uint8_t* in, size_t in_bytes, int64_t chunk, int
   c.is_cuda() ? cuda::decompress_minmax_u8(in, in_bytes, chunk, n_chunks, out, dt, c.stream)
               : cpu::decompress_minmax_u8(in, in_bytes, chunk, n_chunks, out, dt);
 }
-int sgd_steps(const SgdSegment* segs, int n, const Ctx& c) {
-  if (c.is_cuda()) return cuda::sgd_steps(segs, n, c.stream);
-  for (int k = 0; k < n; ++k) {
-    const SgdSegment& a = segs[k];
-    if (a.shadow)
-      cpu::sgd_momentum_flat_shadow(a.p, a.g, a.m, a.shadow, a.n, a.lr, a.momentum, a.dampening, a.weight_decay, a.nesterov,
-                                    a.first);
-    else
-      cpu::sgd_momentum_flat(a.p, a.g, a.m, a.n, a.lr, a.momentum, a.dampening, a.weight_decay, a.nesterov, a.first);
-  }
-  return 0;
-}
 void sgd_momentum_flat(float* p, const float* g, float* buf, int64_t n, float lr, float momentum, float dampening,
                        float wd, bool nesterov, bool first_step, const Ctx& c) {
   sgd_momentum_flat_shadow(p, g, buf, nullptr, n, lr, momentum, dampening, wd, nesterov, first_step, c);
@@ -324,8 +305,10 @@ void sgd_momentum_flat(float* p, const float* g, float* buf, int64_t n, float lr
 void sgd_momentum_flat_shadow(float* p, const float* g, float* buf, void* shadow, int64_t n, float lr, float momentum,
                               float dampening, float wd, bool nesterov, bool first_step, const Ctx& c) {
   if (n <= 0) return;
-  const SgdSegment a{p, g, buf, shadow, n, lr, momentum, dampening, wd, nesterov, first_step, false};
-  sgd_steps(&a, 1, c);
+  if (c.is_cuda())
+    cuda::sgd_momentum_flat_shadow(p, g, buf, shadow, n, lr, momentum, dampening, wd, nesterov, first_step, c.stream);
+  else
+    cpu::sgd_momentum_flat_shadow(p, g, buf, shadow, n, lr, momentum, dampening, wd, nesterov, first_step);
 }
 
 }  // namespace kernels

@@ -398,6 +398,11 @@ int sgd_steps(const SgdSegment* segs, int n, cudaStream_t s) {
   }
   return launches;
 }
+void sgd_momentum_flat_shadow(float* p, const float* g, float* buf, void* shadow, int64_t n, float lr, float momentum,
+                              float dampening, float wd, bool nesterov, bool first_step, cudaStream_t s) {
+  const SgdSegment a{p, g, buf, shadow, n, lr, momentum, dampening, wd, nesterov, first_step, false};
+  sgd_steps(&a, 1, s);
+}
 
 }  // namespace cuda
 }  // namespace kernels

@@ -37,7 +37,6 @@ void average_inplace(void* x, const void* y, DType dt, int64_t n, const Ctx& c);
 void async_model_average(float* t, const float* reduced, const float* copy, float nranks, int64_t n,
                          const Ctx& c);
 void copy_bytes(void* dst, const void* src, size_t bytes, const Ctx& c);
-// x[i] += y[i] with x in fp32 and y in bf16: a low-precision gradient into its fp32 accumulator, in one pass.
 struct CastSegment {
   const float* src;
   void* dst;  // n bf16 values
@@ -46,8 +45,9 @@ struct CastSegment {
 // Rounds a few fp32 buffers to bf16 in one launch (CUDA only).
 namespace cuda {
 void cast_bf16(const CastSegment* segs, int n, cudaStream_t s);
-}
-void accumulate_bf16(float* x, const void* y, int64_t n, const Ctx& c);
+// x[i] += y[i] with x in fp32 and y in bf16: a low-precision gradient into its fp32 accumulator, in one pass.
+void accumulate_bf16(float* x, const void* y, int64_t n, cudaStream_t s);
+}  // namespace cuda
 
 // Flatten (gather = true: tensors -> flat) or unflatten (flat -> tensors) a list of tensors in
 // one launch.  Segments are sorted by `offset` and do not overlap; `segs` is a device array on
@@ -85,6 +85,14 @@ void compress_minmax_u8(const void* in, DType dt, int64_t num_real, int64_t chun
 void decompress_minmax_u8(const uint8_t* in, size_t in_bytes, int64_t chunk_size, int n_chunks,
                           void* out, DType dt, const Ctx& c);
 
+namespace cuda {
+// Two rounds of compress / decompress of one chunk of n elements, in place: what a low-precision exchange leaves of a
+// tensor.  Scratch as for compress with one chunk.
+// Weak: the engine's host sources are also linked without its kernels (a host-only stress program).
+void quantise_twice_minmax_u8(void* x, DType dt, int64_t n, void* scratch, size_t scratch_bytes, cudaStream_t s)
+    __attribute__((weak));
+}  // namespace cuda
+
 // Scalar definition of the quantiser, shared by host code and tests.
 struct MinMaxGrid {
   float scale, lower, upper;
@@ -103,8 +111,10 @@ struct SgdSegment {
   bool nesterov, first;
   bool vec;  // set by the CUDA path
 };
-// Steps all buffers; returns how many kernels were launched.
-int sgd_steps(const SgdSegment* segs, int n, const Ctx& c);
+// Steps all buffers; returns how many kernels were launched (CUDA only).
+namespace cuda {
+int sgd_steps(const SgdSegment* segs, int n, cudaStream_t s);
+}
 // p -= lr * (momentum buffer update of g (+ weight_decay * p)), torch.optim.SGD semantics.
 void sgd_momentum_flat(float* p, const float* g, float* buf, int64_t n, float lr, float momentum,
                        float dampening, float weight_decay, bool nesterov, bool first_step,

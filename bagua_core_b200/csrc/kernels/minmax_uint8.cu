@@ -193,6 +193,30 @@ __device__ __forceinline__ bool wait_minmax(const unsigned long long* slot, floa
   return false;
 }
 
+// The blocks of a chunk, each with its (mn, mx) in every thread, exchange them through the chunk's slots.  Afterwards
+// the chunk's min and max are those over the block's threads.  False in a thread that waited in vain.
+__device__ __forceinline__ bool agree(unsigned long long* mine, int part, int per_chunk, uint32_t tag, float& mn, float& mx) {
+  const int tid = (int)threadIdx.x;
+  if (tid == 0) leave_minmax(mine + 2 * part, mn, mx, tag);
+  bool all = true;
+  if (per_chunk <= kDirect) {
+    if (tid < per_chunk) all = wait_minmax(mine + 2 * tid, mn, mx, tag);
+    return all;
+  }
+  // many blocks: the first one collects and passes the result on
+  unsigned long long* result = mine + 2 * per_chunk;
+  if (part == 0) {
+    if (tid < per_chunk) all = wait_minmax(mine + 2 * tid, mn, mx, tag);
+    if (__syncthreads_and(all)) {
+      mmdev::block_minmax<kThreads>(mn, mx);
+      if (tid == 0) leave_minmax(result, mn, mx, tag);
+    }
+  } else if (tid == 0) {
+    all = wait_minmax(result, mn, mx, tag);
+  }
+  return all;
+}
+
 // Running min and max of whole vectors: 16-bit types two values at a time, without widening them.
 template <typename T>
 struct RunningMinMax;
@@ -250,6 +274,7 @@ struct RunningMinMax<__nv_bfloat16> : RunningMinMax2<__nv_bfloat162> {
 struct Quantiser {
   static constexpr float kShift = 12582912.f;
   mmdev::Grid g;
+  float mn, mx;  // the range it was made from, where that is needed later
   float lo, hi;  // lower and upper, shifted
   bool shifted;
   __device__ __forceinline__ explicit Quantiser(const mmdev::Grid& grid) : g(grid) {
@@ -406,24 +431,7 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSM)
     }
     mmdev::block_minmax<kThreads>(mn, mx);
     if (per_chunk > 1 || sets > 1) {
-      unsigned long long* mine = slots + (size_t)ci * (per_chunk + 1) * 2;
-      if (tid == 0) leave_minmax(mine + 2 * part, mn, mx, tag);
-      bool all = true;
-      if (per_chunk <= kDirect) {
-        if (tid < per_chunk) all = wait_minmax(mine + 2 * tid, mn, mx, tag);
-      } else {
-        // many blocks: the first one collects and passes the result on
-        unsigned long long* result = mine + 2 * per_chunk;
-        if (part == 0) {
-          if (tid < per_chunk) all = wait_minmax(mine + 2 * tid, mn, mx, tag);
-          if (__syncthreads_and(all)) {
-            mmdev::block_minmax<kThreads>(mn, mx);
-            if (tid == 0) leave_minmax(result, mn, mx, tag);
-          }
-        } else if (tid == 0) {
-          all = wait_minmax(result, mn, mx, tag);
-        }
-      }
+      const bool all = agree(slots + (size_t)ci * (per_chunk + 1) * 2, part, per_chunk, tag, mn, mx);
       if (!__syncthreads_and(all)) {  // the answer is the same, only late
         for (int64_t i = tid; i < real; i += kThreads) {
           const float f = to_f(p[i]);
@@ -467,6 +475,85 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSM)
     }
   }
   let_successor_start();
+}
+
+// ---- two rounds of quantisation in place -----------------------------------------------------
+// What ByteGrad over one rank does to a bucket: quantise, dequantise, and both again on the result.  The second
+// round's range is that of the first round's values, which is known from the first range alone (rounding is
+// monotonic), so every element goes through one table of 256 values: one read and one write where four kernels
+// and a reduction moved 36 bytes per fp32 element (10 MB: 40 us of kernels in 9 launches).
+template <typename T>
+__device__ __forceinline__ void build_twice_lut(float* lut, const Quantiser& g) {
+  const int q = (int)threadIdx.x;
+  auto once = [&](int level) { return to_f(from_f<T>(mmdev::dequantise((uint8_t)level, g.g))); };
+  const float mn = to_f(from_f<T>(g.mn)), mx = to_f(from_f<T>(g.mx));
+  const float mn2 = once((int)mmdev::quantise(mn, g.g)), mx2 = once((int)mmdev::quantise(mx, g.g));
+  const mmdev::Grid second = mmdev::make_grid(mn2, mx2);
+  if (q < 256) lut[q] = to_f(from_f<T>(mmdev::dequantise(mmdev::quantise(once(q), second), second)));
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kThreads, kBlocksPerSM)
+    quantise_twice_kernel(T* x, int64_t n, unsigned long long* slots, uint32_t tag) {
+  constexpr int VE = mmdev::Vec16<T>::VE;
+  __shared__ float s_lut[256];
+  const int tid = (int)threadIdx.x, part = (int)blockIdx.x, parts = (int)gridDim.x;
+  wait_for_predecessor();
+  const int64_t head = min(n, (int64_t)(((0 - reinterpret_cast<uintptr_t>(x)) & (uintptr_t)15) / sizeof(T)));
+  const int64_t nvec = (n - head) / VE, tail = head + nvec * VE;
+  const int64_t per = ((nvec + parts - 1) / parts + 31) & ~(int64_t)31;
+  const int64_t lo = min((int64_t)part * per, nvec), m = min(lo + per, nvec) - lo;
+  T* xv = x + head + lo * VE;
+  float mn = FLT_MAX, mx = -FLT_MAX;
+  RunningMinMax<T> run;
+  Tile<T, true> tile;
+  const int64_t tiles = (m + kTile - 1) / kTile;
+  for (int64_t t = 0; t < tiles; ++t) {  // the last tile stays in registers
+    const int k = (int)min((int64_t)kTile, m - t * kTile);
+    tile.load(xv + t * kTile * VE, k);
+    tile.minmax_all(k, (int64_t)k * VE, run, mn, mx);
+  }
+  {
+    float a, b;
+    run.result(a, b);
+    mn = fminf(mn, a);
+    mx = fmaxf(mx, b);
+  }
+  if (part == 0 && tid < head) {
+    mn = fminf(mn, to_f(x[tid]));
+    mx = fmaxf(mx, to_f(x[tid]));
+  }
+  if (part == parts - 1 && tail + tid < n) {
+    mn = fminf(mn, to_f(x[tail + tid]));
+    mx = fmaxf(mx, to_f(x[tail + tid]));
+  }
+  mmdev::block_minmax<kThreads>(mn, mx);
+  if (parts > 1) {
+    // a block that gave up could not read the chunk again, others write to it already: it passes NaN on instead
+    // (it cannot happen under a cooperative launch)
+    if (!__syncthreads_and(agree(slots, part, parts, tag, mn, mx))) mn = mx = nanf("");
+    mmdev::block_minmax<kThreads>(mn, mx);
+  }
+  if (mn > mx) mn = mx = 0.f;
+  Quantiser g(mmdev::make_grid(to_f(from_f<T>(mn)), to_f(from_f<T>(mx))));
+  g.mn = mn;
+  g.mx = mx;
+  build_twice_lut<T>(s_lut, g);
+  __syncthreads();
+  for (int64_t t = tiles - 1; t >= 0; --t) {
+    const int k = (int)min((int64_t)kTile, m - t * kTile);
+    if (t != tiles - 1) tile.load(xv + t * kTile * VE, k);
+#pragma unroll
+    for (int u = 0; u < kVecs; ++u) {
+      if (tid + u * kThreads >= k) continue;
+      float f[VE];
+      widen(tile.raw[u], f, (const T*)nullptr);
+      mmdev::lut_word(g.pack(f), f, s_lut);
+      mmdev::store_vec(xv + t * kTile * VE, tid + u * kThreads, f);
+    }
+  }
+  if (part == 0 && tid < head) x[tid] = from_f<T>(s_lut[mmdev::quantise(to_f(x[tid]), g.g)]);
+  if (part == parts - 1 && tail + tid < n) x[tail + tid] = from_f<T>(s_lut[mmdev::quantise(to_f(x[tail + tid]), g.g)]);
 }
 
 // A launch's tag: not that of any of the last 2^32 - 2 launches of this process, of whatever type (they share
@@ -551,6 +638,18 @@ __global__ void __launch_bounds__(kDqThreads)
 }
 
 template <typename T>
+void quantise_twice_t(void* x, int64_t n, void* scratch, size_t scratch_bytes, cudaStream_t s) {
+  const Split d = split_chunks(1, n * (int64_t)sizeof(T), true, sm_count());
+  if (d.per_chunk == 1) {
+    launch_overlapped(quantise_twice_kernel<T>, dim3(1), dim3(kThreads), s, (T*)x, n, (unsigned long long*)nullptr, 0u);
+    return;
+  }
+  BAGUA_CHECK(scratch != nullptr && scratch_bytes >= slot_bytes(1, d.per_chunk), MemPool, "quantise_twice: scratch too small");
+  launch_cooperative(quantise_twice_kernel<T>, dim3(d.per_chunk), dim3(kThreads), s, (T*)x, n, (unsigned long long*)scratch,
+                     next_tag());
+}
+
+template <typename T>
 void decompress_t(const uint8_t* in, size_t in_bytes, int64_t chunk, int n_chunks, void* out, cudaStream_t s) {
   const size_t off = in_bytes / (size_t)n_chunks;
   const bool aligned = ((uintptr_t)in % 16 == 0) && ((uintptr_t)out % 16 == 0) && (chunk % 16 == 0) && (off % 16 == 0);
@@ -565,9 +664,8 @@ void decompress_t(const uint8_t* in, size_t in_bytes, int64_t chunk, int n_chunk
 
 }  // namespace
 
-size_t compress_scratch_bytes(int n_chunks, int64_t chunk_size, DType dt) {
+size_t compress_scratch_bytes(int n_chunks, int64_t bytes) {
   // a call for one chunk of the buffer may give that chunk more blocks than a call for all of them
-  const int64_t bytes = chunk_size * (int64_t)dtype_bytes(dt);
   const Split all = split_chunks(n_chunks, bytes, false, sm_count()), one = split_chunks(1, bytes, false, sm_count());
   return bytes <= kTileBytes ? 0 : std::max(slot_bytes(n_chunks, all.per_chunk), slot_bytes(1, one.per_chunk));
 }
@@ -584,6 +682,15 @@ void compress_minmax_u8(const void* in, DType dt, int64_t num_real, int64_t chun
     case DType::BF16:
       compress_t<__nv_bfloat16>(in, num_real, chunk, n_chunks, out, out_bytes, target, scratch, scratch_bytes, s);
       return;
+    default: throw BaguaError(ErrorKind::Tensor, std::string("compress: unsupported dtype ") + dtype_name(dt));
+  }
+}
+
+void quantise_twice_minmax_u8(void* x, DType dt, int64_t n, void* scratch, size_t scratch_bytes, cudaStream_t s) {
+  switch (dt) {
+    case DType::F32: quantise_twice_t<float>(x, n, scratch, scratch_bytes, s); return;
+    case DType::F16: quantise_twice_t<__half>(x, n, scratch, scratch_bytes, s); return;
+    case DType::BF16: quantise_twice_t<__nv_bfloat16>(x, n, scratch, scratch_bytes, s); return;
     default: throw BaguaError(ErrorKind::Tensor, std::string("compress: unsupported dtype ") + dtype_name(dt));
   }
 }

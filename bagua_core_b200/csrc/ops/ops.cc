@@ -172,6 +172,12 @@ class CentralizedLowPrecisionSynchronous : public CommOp {
         note_fallback();
       }
       const int n = c.nranks();
+      if (n == 1 && t.device_id() >= 0) {
+        // one rank (a single GPU, or the last tier of a hierarchical job on one box): nothing travels, the values
+        // are quantised twice where they are, in one pass over them
+        tensor_ops::quantise_twice(t, method_, c.stream());
+        return;
+      }
       auto compressed = tensor_ops::compress(t, method_, n, c.stream(), -1);
       c.alltoall_inplace(*compressed);
       tensor_ops::decompress_from(t, method_, n, *compressed, c.stream());

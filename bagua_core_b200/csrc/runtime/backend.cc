@@ -1,5 +1,7 @@
 #include "backend.h"
 
+#include <algorithm>
+
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
@@ -8,7 +10,7 @@
 namespace bagua {
 
 CommBackend::CommBackend(size_t cap, int device_id)
-    : device_id_(device_id), schedule_(cap == 0 ? 1 : cap), not_waited_(0), monitor_(0),
+    : device_id_(device_id), schedule_(cap == 0 ? 1 : cap), not_waited_(0),
       watchdog_s_(env_double("BAGUA_B200_WATCHDOG_S", 300.0)) {
   if (device_id_ >= 0) BAGUA_CUDA_CHECK(cudaSetDevice(device_id_));
   Telemetry::instance().init_from_env_once();
@@ -18,7 +20,11 @@ CommBackend::CommBackend(size_t cap, int device_id)
 
 CommBackend::~CommBackend() {
   schedule_.close();
-  monitor_.close();
+  {
+    std::lock_guard<std::mutex> g(current_.mu);
+    current_.stop = true;
+  }
+  current_.stop_cv.notify_all();
   if (worker_.joinable()) worker_.join();
   if (monitor_thread_.joinable()) monitor_thread_.join();
 }
@@ -29,20 +35,23 @@ void CommBackend::worker_loop() {
     if (e != cudaSuccess) BAGUA_LOG(Error, "comm worker cannot select device " << device_id_);
   }
   for (;;) {
-    auto item = schedule_.recv();
+    auto item = schedule_.recv(kSpinUs);
     if (!item) return;
     auto& op = **item;
     BAGUA_LOG(Debug, "worker received scheduled communication operation " << op.name);
-    auto mon = std::make_shared<MonitorMsg>();
-    mon->bucket = op.bucket->name();
-    monitor_.send(mon);
+    {
+      std::lock_guard<std::mutex> g(current_.mu);
+      current_.bucket = op.bucket;
+      current_.since = std::chrono::steady_clock::now();
+      current_.reported = false;
+    }
     if (log_enabled(LogLevel::Debug)) {
       std::string names;
       for (auto& t : op.bucket->tensors()) names += (names.empty() ? "" : ",") + t->name();
       BAGUA_LOG(Debug, "executing communication op `" << op.name << "` on bucket `" << op.bucket->name()
                                                       << "`, tensors [" << names << "]");
     }
-    const uint64_t t0 = now_ms();
+    const uint64_t t0 = Telemetry::instance().now();
     std::string err;
     // Optional NVTX range per bucket (BAGUA_B200_NVTX=1) so that profiler timelines line up
     // with bucket names; a no-op when no tool is attached.
@@ -58,38 +67,35 @@ void CommBackend::worker_loop() {
       BAGUA_LOG(Error, "communication op on bucket `" << op.bucket->name() << "` failed: " << err);
     }
     if (nvtx) nvtxRangePop();
-    Telemetry::instance().record("bucket_executed", op.bucket->name(), t0, now_ms());
+    Telemetry::instance().record("bucket_executed", op.bucket->name(), t0);
+    {
+      std::lock_guard<std::mutex> g(current_.mu);
+      current_.bucket.reset();
+    }
     if (err.empty())
       op.event.finish();
     else
       op.event.fail(err);
-    mon->done.finish();
     BAGUA_LOG(Debug, "comm op executed: " << op.name);
   }
 }
 
 void CommBackend::monitor_loop() {
-  for (;;) {
-    auto msg = monitor_.recv();
-    if (!msg) return;
-    for (;;) {
-      const double limit = watchdog_s_.load();
-      if (limit <= 0) {
-        (*msg)->done.wait();
-        break;
-      }
-      if ((*msg)->done.wait_for(std::chrono::milliseconds((int64_t)(limit * 1000)))) break;
-      const std::string what =
-          "bucket `" + (*msg)->bucket + "` comm op has not finished for " + fmt_double(limit) + " s";
-      BAGUA_LOG(Error, what);
-      {
-        std::lock_guard<std::mutex> g(err_mu_);
-        if (watchdog_error_.empty()) watchdog_error_ = what;
-      }
-      // keep waiting: the op may still complete; the error is reported to the next waiter
-      (*msg)->done.wait();
-      break;
-    }
+  std::unique_lock<std::mutex> lk(current_.mu);
+  while (!current_.stop) {
+    const double limit = watchdog_s_.load();
+    // often enough to report within a tenth of the limit, at most ten times a second
+    const double look = limit <= 0 ? 0.1 : std::min(0.1, std::max(0.005, limit / 10));
+    current_.stop_cv.wait_for(lk, std::chrono::duration<double>(look), [&] { return current_.stop; });
+    if (current_.stop || !current_.bucket || current_.reported || limit <= 0) continue;
+    const std::chrono::duration<double> running = std::chrono::steady_clock::now() - current_.since;
+    if (running.count() < limit) continue;
+    // reported once; the op may still complete, the error goes to the next waiter
+    current_.reported = true;
+    const std::string what = "bucket `" + current_.bucket->name() + "` comm op has not finished for " + fmt_double(limit) + " s";
+    BAGUA_LOG(Error, what);
+    std::lock_guard<std::mutex> g(err_mu_);
+    if (watchdog_error_.empty()) watchdog_error_ = what;
   }
 }
 
@@ -123,32 +129,42 @@ bool CommBackend::should_schedule() const {
 
 void CommBackend::schedule_comm(const BucketPtr& bucket) {
   auto op = std::make_shared<ScheduledCommOp>();
-  op->name = "comm op for bucket " + bucket->name();
+  op->name = bucket->name();
   op->bucket = bucket;
   op->ops = bucket->ops_snapshot();
   EventChannel ev = op->event;
-  const uint64_t t0 = now_ms();
+  const uint64_t t0 = Telemetry::instance().now();
   if (!schedule_.send(std::move(op))) throw BaguaError(ErrorKind::InternalChannel, "schedule channel is closed");
   not_waited_.send(ev);
   EngineStats::global().buckets_scheduled++;
-  Telemetry::instance().record("bucket_scheduled", bucket->name(), t0, now_ms());
+  Telemetry::instance().record("bucket_scheduled", bucket->name(), t0);
 }
 
 void CommBackend::mark_communication_ready(const TensorPtr& tensor, uint64_t ready_cuda_event) {
-  const uint64_t t0 = now_ms();
+  const uint64_t t0 = Telemetry::instance().now();
   tensor->mark_comm_ready(ready_cuda_event);
-  {
-    std::lock_guard<std::mutex> g(mu_);
-    while (should_schedule()) {
-      BucketPtr bucket = ordered_buckets_.front();
-      ordered_buckets_.pop_front();
-      BAGUA_LOG(Debug, "bucket " << bucket->name() << " ready for communication");
-      bucket->reset_comm_ready();
-      ordered_buckets_.push_back(bucket);
-      schedule_comm(bucket);
-    }
+  schedule_ready();
+  Telemetry::instance().record("tensor_ready", tensor->name(), t0);
+}
+
+bool CommBackend::try_mark_ready(const TensorPtr& tensor, uint64_t ready_cuda_event) {
+  const uint64_t t0 = Telemetry::instance().now();
+  tensor->mark_comm_ready(ready_cuda_event);
+  Telemetry::instance().record("tensor_ready", tensor->name(), t0);
+  std::unique_lock<std::mutex> g(mu_, std::try_to_lock);
+  return g.owns_lock() && !should_schedule();
+}
+
+void CommBackend::schedule_ready() {
+  std::lock_guard<std::mutex> g(mu_);
+  while (should_schedule()) {
+    BucketPtr bucket = ordered_buckets_.front();
+    ordered_buckets_.pop_front();
+    BAGUA_LOG(Debug, "bucket " << bucket->name() << " ready for communication");
+    bucket->reset_comm_ready();
+    ordered_buckets_.push_back(bucket);
+    schedule_comm(bucket);
   }
-  Telemetry::instance().record("tensor_ready", tensor->name(), t0, now_ms());
 }
 
 size_t CommBackend::wait_pending_comm_ops() {

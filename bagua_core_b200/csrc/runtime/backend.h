@@ -46,6 +46,10 @@ class CommBackend {
 
   void register_ordered_buckets(const std::vector<BucketPtr>& buckets);
   void mark_communication_ready(const TensorPtr& tensor, uint64_t ready_cuda_event);
+  // The same without ever blocking: false when there is a bucket to schedule (or another thread holds the
+  // scheduler), and schedule_ready() is still to be called.
+  bool try_mark_ready(const TensorPtr& tensor, uint64_t ready_cuda_event);
+  void schedule_ready();
   size_t wait_pending_comm_ops();
 
   // seconds; <= 0 disables the watchdog.  Default: BAGUA_B200_WATCHDOG_S or 300.
@@ -66,11 +70,15 @@ class CommBackend {
 
   Channel<std::shared_ptr<ScheduledCommOp>> schedule_;
   Channel<EventChannel> not_waited_;
-  struct MonitorMsg {
-    std::string bucket;
-    EventChannel done{"monitor"};
-  };
-  Channel<std::shared_ptr<MonitorMsg>> monitor_;
+  // What the worker is executing, for the watchdog, which looks at it now and then: a message per bucket would
+  // wake it twice for each.
+  struct Current {
+    std::mutex mu;
+    std::condition_variable stop_cv;
+    BucketPtr bucket;  // null: nothing
+    std::chrono::steady_clock::time_point since;
+    bool reported = false, stop = false;
+  } current_;
   std::atomic<double> watchdog_s_;
   std::mutex err_mu_;
   std::string watchdog_error_;

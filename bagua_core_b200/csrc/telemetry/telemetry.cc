@@ -83,9 +83,7 @@ void Telemetry::init_from_env_once() {
   });
 }
 
-void Telemetry::record(const std::string& action, const std::string& tensor_name, uint64_t start_ms,
-                       uint64_t end_ms) {
-  if (!enabled()) return;
+void Telemetry::push(const char* action, const std::string& tensor_name, uint64_t start_ms, uint64_t end_ms) {
   {
     std::lock_guard<std::mutex> g(mu_);
     if (queue_.size() > 65536) queue_.pop_front();  // never grow without bound if the server is down

@@ -35,7 +35,11 @@ class Telemetry {
   // Reads AUTO_TUNE_SERVER_ADDR once per process.
   void init_from_env_once();
   bool enabled() const { return enabled_.load(std::memory_order_acquire); }
-  void record(const std::string& action, const std::string& tensor_name, uint64_t start_ms, uint64_t end_ms);
+  // Off (the usual case) this is one load: no strings, no clock.
+  uint64_t now() const { return enabled() ? now_ms() : 0; }
+  void record(const char* action, const std::string& tensor_name, uint64_t start_ms) {
+    if (enabled()) push(action, tensor_name, start_ms, now_ms());
+  }
   // Blocks until the queue is drained (or `timeout_ms` elapsed).  Returns spans exported so far.
   uint64_t flush(int timeout_ms = 2000);
   void shutdown();
@@ -47,6 +51,7 @@ class Telemetry {
  private:
   Telemetry() = default;
   ~Telemetry();
+  void push(const char* action, const std::string& tensor_name, uint64_t start_ms, uint64_t end_ms);
   void run();
   bool post(const std::string& body);
 

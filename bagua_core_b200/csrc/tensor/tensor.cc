@@ -56,6 +56,7 @@ void async_model_average(RawTensor& t, const RawTensor& reduced, const RawTensor
 static void reduce_chunks(RawTensor& t, int n_chunks, int target, bool avg, uint64_t stream) {
   BAGUA_CHECK(n_chunks > 0 && t.num_elements_allocated() % n_chunks == 0, Tensor,
               "reduce: tensor size " << t.num_elements_allocated() << " is not divisible by " << n_chunks);
+  if (n_chunks == 1 && target == 0) return;  // the sum, and the mean, of one chunk is that chunk
   kernels::reduce_chunk_inplace(t.data_ptr(), t.dtype(), t.num_elements_allocated() / n_chunks, n_chunks, target, avg,
                                 t.ctx(stream));
 }
@@ -100,30 +101,30 @@ void decompress_from(RawTensor& t, const std::string& method, int n_chunks, cons
                                 t.ctx(stream));
 }
 
+void quantise_twice(RawTensor& t, const std::string& method, uint64_t stream) {
+  BAGUA_CHECK(method == "MinMaxUInt8", Tensor, "unsupported compression method " << method);
+  BAGUA_CHECK(t.device_id() >= 0 && kernels::cuda::quantise_twice_minmax_u8 != nullptr, Tensor,
+              "quantise_twice works on CUDA tensors");
+  const int64_t n = t.num_elements_allocated();
+  if (n == 0) return;
+  const size_t bytes = kernels::compress_scratch_bytes(1, n, t.dtype());
+  std::shared_ptr<PoolBlock> scratch;
+  if (bytes) scratch = MemoryPool::for_device(t.device_id()).pull_cleared(bytes, stream);
+  kernels::cuda::quantise_twice_minmax_u8(t.data_ptr(), t.dtype(), n, scratch ? scratch->ptr() : nullptr, bytes,
+                                          (cudaStream_t)stream);
+}
+
 }  // namespace tensor_ops
 
 // ---------------------------------------------------------------------------------
 void BaguaTensor::mark_comm_ready(uint64_t cuda_event) {
-  std::unique_lock<std::shared_mutex> g(mu_);
   if (cuda_event == 0) BAGUA_LOG(Debug, "mark comm ready with an event 0, ignoring event");
-  ready_ = true;
-  ready_event_ = cuda_event;
+  ready_event_.store(cuda_event, std::memory_order_relaxed);
+  ready_.store(true, std::memory_order_release);
 }
-void BaguaTensor::reset_comm_ready() {
-  std::unique_lock<std::shared_mutex> g(mu_);
-  ready_ = false;
-}
-bool BaguaTensor::ready_for_comm() const {
-  if (is_padding()) return true;
-  std::shared_lock<std::shared_mutex> g(mu_);
-  return ready_;
-}
-uint64_t BaguaTensor::take_ready_event() {
-  std::unique_lock<std::shared_mutex> g(mu_);
-  uint64_t e = ready_event_;
-  ready_event_ = 0;
-  return e;
-}
+void BaguaTensor::reset_comm_ready() { ready_.store(false, std::memory_order_relaxed); }
+bool BaguaTensor::ready_for_comm() const { return padding_ || ready_.load(std::memory_order_acquire); }
+uint64_t BaguaTensor::take_ready_event() { return ready_event_.exchange(0, std::memory_order_relaxed); }
 
 std::shared_ptr<BaguaTensor> BaguaTensor::compress(const std::string& method, int n_chunks, int target_chunk) const {
   auto r = raw();
@@ -218,7 +219,6 @@ CommunicationTensor BaguaBucket::get_communication_tensor(uint64_t stream, bool 
                                                           bool force_not_copy_back) {
   CommunicationTensor ct;
   ct.stream = stream;
-  ct.bucket_tensors = tensors_;
   for (auto& t : tensors_) {
     uint64_t ev = t->take_ready_event();
     if (ev != 0 && device_ >= 0)

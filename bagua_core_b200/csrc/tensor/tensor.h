@@ -75,23 +75,23 @@ std::shared_ptr<RawTensor> compress(const RawTensor& t, const std::string& metho
                                     int target_chunk);
 void decompress_from(RawTensor& t, const std::string& method, int n_chunks, const RawTensor& compressed,
                      uint64_t stream);
+// t = decompress(compress(decompress(compress(t)))) with one chunk, in place; CUDA tensors only.
+void quantise_twice(RawTensor& t, const std::string& method, uint64_t stream);
 }  // namespace tensor_ops
 
 class BaguaTensor {
  public:
-  BaguaTensor(std::string name, std::shared_ptr<RawTensor> raw) : name_(std::move(name)), raw_(std::move(raw)) {}
+  BaguaTensor(std::string name, std::shared_ptr<RawTensor> raw)
+      : name_(std::move(name)), padding_(name_.rfind("bagua_padding_tensor", 0) == 0), raw_(std::move(raw)) {}
 
   const std::string& name() const { return name_; }
-  std::shared_ptr<RawTensor> raw() const {
-    std::shared_lock<std::shared_mutex> g(mu_);
-    return raw_;
-  }
+  const std::shared_ptr<RawTensor>& raw() const { return raw_; }
   // event == 0 means "ready, nothing to wait for on the stream"
   void mark_comm_ready(uint64_t cuda_event);
   void reset_comm_ready();
   // padding tensors (name prefix "bagua_padding_tensor") are always ready
   bool ready_for_comm() const;
-  bool is_padding() const { return name_.rfind("bagua_padding_tensor", 0) == 0; }
+  bool is_padding() const { return padding_; }
   // Returns the stored ready event and clears it.
   uint64_t take_ready_event();
 
@@ -109,10 +109,11 @@ class BaguaTensor {
 
  private:
   const std::string name_;
-  mutable std::shared_mutex mu_;
-  std::shared_ptr<RawTensor> raw_;
-  bool ready_ = false;
-  uint64_t ready_event_ = 0;
+  const bool padding_;
+  const std::shared_ptr<RawTensor> raw_;
+  // set by the thread that finished the gradient, read by the scheduler (under its lock) and the worker
+  std::atomic<bool> ready_{false};
+  std::atomic<uint64_t> ready_event_{0};
 };
 
 using TensorPtr = std::shared_ptr<BaguaTensor>;
@@ -126,7 +127,6 @@ class CommunicationTensor {
   bool need_copy_back = false;
   bool staged = false;  // `raw` is a pool buffer holding a copy of the bucket
   uint64_t stream = 0;
-  std::vector<TensorPtr> bucket_tensors;
   // staged: where every tensor sits in `raw`; on a GPU the same table also lives on the device
   std::vector<kernels::MultiCopySeg> segments;
   std::shared_ptr<RawTensor> segments_dev;

@@ -289,8 +289,13 @@ struct ConvNode : public Node {
       if (need_w && alone && dw.scalar_type() == at::kBFloat16 && accumulates(weight, dw) &&
           dw.strides() == weight.grad().strides()) {
         // the cast to fp32 and the addition in one pass; the same bits
-        kernels::accumulate_bf16((float*)weight.grad().data_ptr(), dw.data_ptr(), dw.numel(), ctx_of(dw));
-        if (dw.is_cuda()) count_launches(1);
+        if (dw.is_cuda()) {
+          kernels::cuda::accumulate_bf16((float*)weight.grad().data_ptr(), dw.data_ptr(), dw.numel(), stream_of(dw));
+          count_launches(1);
+        } else {
+          c10::NoGradGuard no_grad;
+          weight.grad().add_(dw);
+        }
       } else {
         out[1] = dw;
       }

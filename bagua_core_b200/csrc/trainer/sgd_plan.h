@@ -30,7 +30,6 @@ class SgdPlan {
   bool empty() const { return segs_.empty(); }
 
  private:
-  kernels::Ctx ctx(uint64_t stream) const { return kernels::Ctx{device_, (cudaStream_t)stream}; }
   int device_ = -1;
   std::vector<kernels::SgdSegment> segs_;
   std::vector<int> group_;

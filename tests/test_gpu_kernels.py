@@ -424,3 +424,56 @@ def test_sgd_plan_steps_slices_of_several_buffers_with_their_groups():
         assert torch.equal(shadow[sl], flat[0][sl].bfloat16() if i % 2 else torch.zeros_like(shadow[sl]))
     plan.zero_grad(st)
     assert not flat[1].any() and torch.equal(flat[0], ref[0])
+
+
+@pytest.mark.parametrize("n", [1, 5, 33, 16384, 16385, 200003, 2621440, 6000001, (1 << 23) + 7])
+@pytest.mark.parametrize("dt", DTYPES)
+@pytest.mark.parametrize("offset", [0, 1])
+def test_low_precision_op_over_one_rank_is_two_round_trips(n, dt, offset):
+    """The engine's one-rank ByteGrad (one kernel, in place) against compress / decompress called twice."""
+    import bagua_core as bc
+
+    base = _rand(n + offset, dt, n % 89) * 0.05
+    x = base[offset:]
+    want = x.clone()
+    for _ in range(2):
+        c = bc.BaguaTensorPy(want, "w").compress("MinMaxUInt8", 1, -1)
+        bc.BaguaTensorPy(want, "w").decompress_from("MinMaxUInt8", 1, c)
+    torch.cuda.synchronize()
+    comm = bc.BaguaSingleCommunicatorPy(0, 1, 0, torch.cuda.current_stream().cuda_stream, "solo")
+    t = bc.BaguaTensorPy(x, "x")
+    bucket = bc.BaguaBucketPy("b", [t])
+    bucket.append_centralized_synchronous_op(comm, None, hierarchical=False, average=True, scattergather=True,
+                                             compression="MinMaxUInt8")
+    backend = bc.BaguaCommBackendPy(10, 0)
+    backend.register_ordered_buckets([bucket])
+    first = base[:offset].clone()
+    backend.mark_communication_ready(t, 0)
+    backend.wait_pending_comm_ops()
+    torch.cuda.synchronize()
+    backend.close()
+    assert torch.equal(x, want) and torch.equal(base[:offset], first)
+
+
+@pytest.mark.parametrize("seed", range(4))
+def test_multi_copy_at_every_relative_alignment(seed):
+    """Tensors of 1 byte to several tiles at odd addresses, more of them than a block has threads."""
+    import bagua_core_b200 as bb
+
+    g = torch.Generator().manual_seed(seed)
+    pool = torch.randint(0, 256, (4 << 20,), dtype=torch.uint8, generator=g).cuda()
+    ts, off = [], seed
+    sizes = torch.randint(1, 300, (300,), generator=g).tolist() + [16384, 16383, 50001, 1, 2, 3, 15, 16, 17, 131072 + seed]
+    for n in sizes:
+        ts.append(pool[off:off + n])
+        off += n + int(torch.randint(0, 19, (1,), generator=g))
+    flat = torch.zeros(sum(sizes) + 64, dtype=torch.uint8, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    bb._C.k_multi_copy(ts, flat[:sum(sizes)], True, st)
+    want = torch.cat(ts)
+    assert torch.equal(flat[:sum(sizes)], want) and not flat[sum(sizes):].any()
+    before = pool.clone()
+    for t in ts:
+        t.zero_()
+    bb._C.k_multi_copy(ts, flat[:sum(sizes)], False, st)
+    assert torch.equal(pool, before)
