@@ -13,9 +13,9 @@ from .. import BaguaTensorPy
 
 
 def _s(t: torch.Tensor, stream=None) -> int:
-    if not t.is_cuda:
-        return 0
-    return (stream or torch.cuda.current_stream(t.device)).cuda_stream
+    if stream is None:
+        return _C.current_stream(t)
+    return stream.cuda_stream if t.is_cuda else 0
 
 
 def divide_inplace(x, divisor, stream=None):

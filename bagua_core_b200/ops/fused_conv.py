@@ -34,7 +34,7 @@ def __getattr__(name):
 
 
 def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream if t.is_cuda else 0
+    return _C.current_stream(t)
 
 
 def _count(n: int) -> None:

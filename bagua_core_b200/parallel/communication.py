@@ -18,6 +18,7 @@ import torch
 import torch.distributed as dist
 
 from .. import BaguaCommBackendPy, BaguaSingleCommunicatorPy
+from .._native import C as _C
 
 _lock = threading.Lock()
 _state: Optional["BaguaProcessGroup"] = None
@@ -91,7 +92,7 @@ class BaguaProcessGroup:
     def wait_comm_stream(self):
         """Make the current (compute) stream wait for everything queued on the comm stream."""
         if self.comm_stream is not None:
-            torch.cuda.current_stream().wait_stream(self.comm_stream)
+            _C.wait_stream(self.device.index, self.stream_ptr)
 
 
 def _bcast_str(s: Optional[str], src: int, group=None) -> str:

@@ -142,8 +142,7 @@ class FlatSGD(torch.optim.Optimizer):
                 self._plan.add(f["p"][lo:hi], f["g"][lo:hi], f["m"][lo:hi], f["h"][lo:hi] if "h" in f else None, gi)
 
     def _stream(self):
-        t = self._flat[0]["p"]
-        return torch.cuda.current_stream(t.device).cuda_stream if t.is_cuda else 0
+        return _C.current_stream(self._flat[0]["p"])
 
     def _loose_params(self):
         """[(group, parameter)] outside the flat buffers; looked up again when a group has grown."""
