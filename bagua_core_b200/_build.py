@@ -37,6 +37,7 @@ SOURCES = [
     "ops/ops.cc",
     "telemetry/telemetry.cc",
     "trainer/autograd_ops.cc",
+    "trainer/gemm.cc",
     "trainer/grad_hooks.cc",
     "trainer/sgd_plan.cc",
     "capi/capi.cc",
@@ -68,6 +69,17 @@ def _nccl_paths():
     if os.path.exists(os.path.join(inc, "nccl.h")) and os.path.exists(os.path.join(lib, "libnccl.so.2")):
         return inc, lib
     return "/usr/include", "/usr/lib/x86_64-linux-gnu"
+
+
+def _cublaslt_flags():
+    """The cuBLASLt that torch itself loads (same process, same symbols)."""
+    import torch
+
+    site = os.path.dirname(os.path.dirname(torch.__file__))
+    for d in (os.path.join(site, "nvidia", "cublas", "lib"), "/usr/local/cuda/lib64"):
+        if os.path.exists(os.path.join(d, "libcublasLt.so.12")):
+            return [f"-L{d}", "-l:libcublasLt.so.12", f"-Wl,-rpath,{d}"]
+    return ["-lcublasLt"]
 
 
 def _shared_libstdcxx_flags():
@@ -121,6 +133,7 @@ def build(verbose: bool = False, force: bool = False) -> str:
         # of libstdc++ next to the one torch uses has two sets of locale facets, and the
         # first number streamed into a std::ostream crashes.
         extra_ldflags=_shared_libstdcxx_flags()
+        + _cublaslt_flags()
         + [f"-L{nccl_lib}", "-l:libnccl.so.2", f"-Wl,-rpath,{nccl_lib}", "-lcudart"],
         build_directory=BUILD_DIR,
         with_cuda=True,

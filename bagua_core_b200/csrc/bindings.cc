@@ -13,6 +13,7 @@
 #include <pybind11/stl.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/extension.h>
 
 #include "comm/arena.h"
@@ -969,7 +970,27 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("remove", &trainer::GradHooks::remove)
       .def("arm", &trainer::GradHooks::arm)
       .def("flush", &trainer::GradHooks::flush, py::call_guard<py::gil_scoped_release>())
-      .def("set_enabled", &trainer::GradHooks::set_enabled, py::arg("on"));
+      .def("set_enabled", &trainer::GradHooks::set_enabled, py::arg("on"))
+      .def("set_callback",
+           [](trainer::GradHooks& h, py::object fn) {
+             auto holder = std::shared_ptr<py::object>(new py::object(std::move(fn)), [](py::object* o) {
+               py::gil_scoped_acquire g;
+               delete o;
+             });
+             h.set_callback([holder]() {
+               py::gil_scoped_acquire g;
+               try {
+                 (*holder)();
+               } catch (py::error_already_set& e) {
+                 e.restore();
+                 python_error err;  // reaches the caller of backward() as the Python exception it is
+                 err.persist();
+                 throw err;
+               }
+             });
+           },
+           py::arg("fn"))
+      .def("watch", &trainer::GradHooks::watch, py::arg("output"));
 
   // ---- single-GPU emulation of the fused kernels (all ranks in one cooperative launch) ----
   py::class_<fused::EmulatedArena>(m, "EmulatedArena")

@@ -17,6 +17,7 @@
 #include "../kernels/kernels.h"
 #include "../kernels/model_ops.h"
 #include "../tensor/tensor.h"
+#include "gemm.h"
 
 namespace bagua {
 namespace trainer {
@@ -100,6 +101,19 @@ bool gemm_into(at::Tensor grad, const at::Tensor& a, const at::Tensor& b) {
   // its fast kernels: 82 us instead of 22 for 3072 x 1024 x 3072.  The product then goes to a buffer of its own and
   // is added from there.
   const bool aligned = (uintptr_t)grad.data_ptr() % 16 == 0;
+  const at::Tensor dy = a.t();
+  if (aligned && gemm::weight_grad(dy, b, grad, true)) {
+    mode = 1;
+    return true;
+  }
+  if (!aligned) {
+    at::Tensor apart = at::empty(grad.sizes(), grad.options());
+    if (gemm::weight_grad(dy, b, apart, false)) {
+      mode = mode == 0 ? 1 : mode.load();
+      kernels::add_inplace(grad.data_ptr(), apart.data_ptr(), DType::F32, grad.numel(), ctx_of(grad));
+      return true;
+    }
+  }
   if (mode <= 1 && (aligned || mode == 0)) {
     try {
       at::addmm_out(grad, grad, a, b, at::kFloat);
@@ -192,7 +206,12 @@ struct LinearNode : public Node {
     at::Tensor dy2 = dy.dim() == 2 ? dy : dy.reshape({-1, dy.size(-1)});
     if (gelu) dy2 = through_gelu(dy2.contiguous(), out);
     if (task_should_compute_output(0)) {
-      at::Tensor dx = at::mm(dy2, ws);
+      at::Tensor dx;
+      if (!c10::GradMode::is_enabled()) {
+        dx = at::empty({dy2.size(0), ws.size(1)}, dy2.options());
+        if (!gemm::input_grad(dy2, ws, dx)) dx = at::Tensor();
+      }
+      if (!dx.defined()) dx = at::mm(dy2, ws);
       out[0] = dy.dim() == 2 ? dx : dx.view(xs.sizes());
     }
     if (task_should_compute_output(1)) {
@@ -455,7 +474,14 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& weight, const std::opti
     to_bf16(low);
     xs = low[0];
     ws = low[1];
-    y = at::linear(xs, ws, b.defined() ? std::optional<at::Tensor>(low[2]) : std::nullopt);
+    if (xs.is_cuda() && xs.is_contiguous() && xs.numel() > 0 && xs.dim() >= 2) {
+      std::vector<int64_t> shape(xs.sizes().begin(), xs.sizes().end());
+      shape.back() = ws.size(0);
+      y = at::empty(shape, xs.options());
+      at::Tensor y2 = y.dim() == 2 ? y : y.view({-1, ws.size(0)});
+      if (!gemm::linear(xs.dim() == 2 ? xs : xs.view({-1, xs.size(-1)}), ws, low[2], y2)) y = at::Tensor();
+    }
+    if (!y.defined()) y = at::linear(xs, ws, b.defined() ? std::optional<at::Tensor>(low[2]) : std::nullopt);
     if (gelu) {
       z = y.contiguous();
       y = at::empty_like(z);

@@ -1,6 +1,7 @@
 #include "grad_hooks.h"
 
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/engine.h>
 #include <torch/csrc/autograd/utils/lambda_post_hook.h>
 #include <torch/csrc/autograd/variable.h>
 
@@ -58,6 +59,21 @@ void GradHooks::arm() {
 void GradHooks::flush() {
   for (auto& e : entries_)
     if (!e.marked && buckets_[(size_t)e.bucket].pending > 0) mark(e);
+}
+
+void GradHooks::watch(const at::Tensor& output) {
+  std::weak_ptr<GradHooks> self = weak_from_this();
+  output.register_hook([self](const at::Tensor&) {
+    auto me = self.lock();
+    if (!me || !me->done_ || me->queued_.exchange(true)) return;
+    // whichever output fires first: the loss may depend on any of them
+    torch::autograd::Engine::get_default_engine().queue_callback([self]() {
+      auto me2 = self.lock();
+      if (!me2) return;
+      me2->queued_ = false;
+      me2->done_();
+    });
+  });
 }
 
 void GradHooks::on_gradient(size_t i) {

@@ -11,6 +11,8 @@
 #include <cuda_runtime_api.h>
 #include <torch/csrc/autograd/function.h>
 
+#include <atomic>
+#include <functional>
 #include <memory>
 #include <vector>
 
@@ -32,6 +34,9 @@ class GradHooks : public std::enable_shared_from_this<GradHooks> {
   void arm();              // before the next backward pass: nothing is marked
   void flush();            // marks what no hook has marked since arm(), in every bucket that is incomplete
   void set_enabled(bool on) { enabled_ = on; }
+  // `done` runs once, when the backward pass that reaches any of the watched outputs ends.
+  void set_callback(std::function<void()> done) { done_ = std::move(done); }
+  void watch(const at::Tensor& output);
 
  private:
   struct Entry {
@@ -52,6 +57,8 @@ class GradHooks : public std::enable_shared_from_this<GradHooks> {
   std::weak_ptr<CommBackend> backend_;
   const int device_;
   bool enabled_ = true;
+  std::function<void()> done_;
+  std::atomic<bool> queued_{false};
   std::vector<Entry> entries_;
   std::vector<Bucket> buckets_;
 };

@@ -16,6 +16,7 @@ bagua-core-py/src/lib.rs:316-349):
 """
 from __future__ import annotations
 
+import weakref
 from typing import List, Optional, Sequence
 
 import torch
@@ -145,6 +146,8 @@ class BaguaModule(nn.Module):
                     hooks.add(t.owner, t.tensor, t.backend_tensor, i)
         hooks.install()
         hooks.set_enabled(not self._in_no_sync)
+        ref = weakref.ref(self)
+        hooks.set_callback(lambda: ref()._after_backward() if ref() is not None else None)
         self._native_hooks = hooks
         return hooks
 
@@ -218,6 +221,10 @@ class BaguaModule(nn.Module):
     def _queue_post_backward(self, out):
         tensors = [t for t in _flatten_outputs(out) if isinstance(t, torch.Tensor) and t.requires_grad]
         if not tensors:
+            return
+        if self._native_hooks is not None:
+            for t in tensors:
+                self._native_hooks.watch(t)
             return
         outer = self
 
