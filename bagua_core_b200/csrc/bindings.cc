@@ -920,13 +920,15 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
 
   // ---- trainer: autograd functions and gradient hooks ---------------------------------
   m.def("linear", &trainer::linear, py::arg("x"), py::arg("weight"), py::arg("bias"), py::arg("weight_bf16"),
-        py::arg("accumulate"), py::arg("gelu") = false,
-        "x @ weight.T + bias in bf16, through gelu if asked for; with `accumulate`, the backward adds the parameters' gradients to their fp32 .grad "
+        py::arg("accumulate"), py::arg("activation") = 0,
+        "x @ weight.T + bias in bf16, through gelu (1) or ReLU (2) if asked for; with `accumulate`, the backward adds the parameters' gradients to their fp32 .grad "
         "itself where that changes nothing a user sees.");
   m.def("conv_bias_relu", &trainer::conv_bias_relu, py::arg("x"), py::arg("weight"), py::arg("bias"), py::arg("stride"),
         py::arg("padding"), py::arg("dilation"), py::arg("groups"), py::arg("pool"), py::arg("weight_bf16"),
         py::arg("accumulate"), "max(conv(x, weight) + bias, 0), followed by 2x2 pooling with `pool`.");
-  m.def("gelu_fusable", &trainer::gelu_fusable, py::arg("x"), py::arg("out_features"));
+  m.def("activation_fusable", &trainer::activation_fusable, py::arg("x"), py::arg("out_features"));
+  m.def("span_loss", &trainer::span_loss, py::arg("logits"), py::arg("start"), py::arg("end"),
+        "Mean of the cross entropies of logits[..., 0] against start and of logits[..., 1] against end.");
   m.def("add_layer_norm", &trainer::add_layer_norm, py::arg("x"), py::arg("residual"), py::arg("weight"), py::arg("bias"),
         py::arg("eps"), py::arg("accumulate"), "layer_norm(x + residual) of bf16 activations with fp32 parameters.");
   m.def("embed_layer_norm", &trainer::embed_layer_norm, py::arg("ids"), py::arg("tokens"), py::arg("positions"),

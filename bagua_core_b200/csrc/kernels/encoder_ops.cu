@@ -1,6 +1,6 @@
 // See encoder_ops.h.  All kernels are latency- and bandwidth-bound streams over activations of a few MB that
-// mostly sit in L2: 16-byte vectors, one warp per row for everything that needs row statistics (shuffles
-// instead of block barriers), column sums kept in registers over the rows a warp visits.
+// mostly sit in L2: 16-byte vectors, enough blocks for every SM, column sums kept in registers over the rows a warp
+// visits.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -24,245 +24,19 @@ using model_ops::bodies::unpack8;
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr int kMaxVecs = 4;  // H <= 32 lanes * 8 columns * kMaxVecs
-
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
-// 8 floats from an address that is 4-byte aligned; `vec`: 16-byte aligned.
-__device__ __forceinline__ void load8(const float* p, bool vec, float (&f)[8]) {
-  if (vec) {
-    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
-    f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w;
-    f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
-  } else {
-#pragma unroll
-    for (int k = 0; k < 8; ++k) f[k] = p[k];
-  }
-}
-
-template <int NV>
-struct Row {
-  float v[NV][8];
-};
-// Mean and reciprocal deviation of a row spread over a warp.
-template <int NV>
-__device__ __forceinline__ void statistics(const Row<NV>& x, int nvec, int lane, float eps, int H, float& mean, float& rstd) {
-  float s = 0.f;
-#pragma unroll
-  for (int j = 0; j < NV; ++j)
-    if (j * 32 + lane < nvec) {
-#pragma unroll
-      for (int k = 0; k < 8; ++k) s += x.v[j][k];
-    }
-  mean = warp_sum(s) / (float)H;
-  float q = 0.f;
-#pragma unroll
-  for (int j = 0; j < NV; ++j)
-    if (j * 32 + lane < nvec) {
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const float d = x.v[j][k] - mean;
-        q += d * d;
-      }
-    }
-  rstd = rsqrtf(warp_sum(q) / (float)H + eps);
-}
-
-template <int NV>
-__global__ void __launch_bounds__(kThreads)
-    add_layer_norm_kernel(const uint4* __restrict__ x, const uint4* __restrict__ r, const float* __restrict__ gamma,
-                          const float* __restrict__ beta, float eps, uint4* __restrict__ sum, uint4* __restrict__ y,
-                          float* __restrict__ mean, float* __restrict__ rstd, int64_t rows, int H, bool vec) {
-  wait_for_predecessor();
-  const int lane = (int)threadIdx.x & 31, nvec = H / 8;
-  const int64_t row = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
-  if (row >= rows) return;
-  Row<NV> a;
-#pragma unroll
-  for (int j = 0; j < NV; ++j) {
-    const int v = j * 32 + lane;
-    if (v >= nvec) continue;
-    unpack8(x[row * nvec + v], a.v[j]);
-    if (r) {
-      float b[8];
-      unpack8(r[row * nvec + v], b);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) a.v[j][k] += b[k];
-      const uint4 packed = pack8(a.v[j]);  // the sum as a bf16 residual stream holds it
-      sum[row * nvec + v] = packed;
-      unpack8(packed, a.v[j]);
-    }
-  }
-  float m, rs;
-  statistics<NV>(a, nvec, lane, eps, H, m, rs);
-  if (lane == 0) {
-    mean[row] = m;
-    rstd[row] = rs;
-  }
-#pragma unroll
-  for (int j = 0; j < NV; ++j) {
-    const int v = j * 32 + lane;
-    if (v >= nvec) continue;
-    float g[8], b[8];
-    load8(gamma + v * 8, vec, g);
-    load8(beta + v * 8, vec, b);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) a.v[j][k] = (a.v[j][k] - m) * rs * g[k] + b[k];
-    y[row * nvec + v] = pack8(a.v[j]);
-  }
-}
-
-// tok[id] + pos[p] + typ, in this order, in fp32
-template <int NV>
-__device__ __forceinline__ void gather_row(const int64_t* ids, int64_t vocab, const float* tok, const float* pos,
-                                           const float* typ, int64_t row, int64_t seq, int H, int nvec, int lane, bool vec,
-                                           Row<NV>& a) {
-  const int64_t id = ids[row];
-  const bool known = id >= 0 && id < vocab;  // an id outside the table gives a row of NaN
-  const float* t = tok + (known ? id : 0) * H;
-  const float* p = pos + (row % seq) * H;
-#pragma unroll
-  for (int j = 0; j < NV; ++j) {
-    const int v = j * 32 + lane;
-    if (v >= nvec) continue;
-    float b[8], c[8];
-    load8(t + v * 8, vec, a.v[j]);
-    load8(p + v * 8, vec, b);
-    load8(typ + v * 8, vec, c);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) a.v[j][k] = known ? a.v[j][k] + b[k] + c[k] : nanf("");
-  }
-}
-
-template <int NV>
-__global__ void __launch_bounds__(kThreads)
-    embed_layer_norm_kernel(const int64_t* __restrict__ ids, int64_t vocab, const float* __restrict__ tok,
-                            const float* __restrict__ pos,
-                            const float* __restrict__ typ, const float* __restrict__ gamma, const float* __restrict__ beta,
-                            float eps, uint4* __restrict__ y, float* __restrict__ mean, float* __restrict__ rstd, int64_t rows,
-                            int64_t seq, int H, bool vec) {
-  wait_for_predecessor();
-  const int lane = (int)threadIdx.x & 31, nvec = H / 8;
-  const int64_t row = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
-  if (row >= rows) return;
-  Row<NV> a;
-  gather_row<NV>(ids, vocab, tok, pos, typ, row, seq, H, nvec, lane, vec, a);
-  float m, rs;
-  statistics<NV>(a, nvec, lane, eps, H, m, rs);
-  if (lane == 0) {
-    mean[row] = m;
-    rstd[row] = rs;
-  }
-#pragma unroll
-  for (int j = 0; j < NV; ++j) {
-    const int v = j * 32 + lane;
-    if (v >= nvec) continue;
-    float g[8], b[8];
-    load8(gamma + v * 8, vec, g);
-    load8(beta + v * 8, vec, b);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) a.v[j][k] = (a.v[j][k] - m) * rs * g[k] + b[k];
-    y[row * nvec + v] = pack8(a.v[j]);
-  }
-}
-
-// Backward of a row: ds = rstd * (g dy - mean(g dy) - xhat * mean(g dy xhat)); column sums of dy xhat and dy, and with
-// kEmbed of ds, over the rows a warp visits, then over the block's warps, one partial row per block.
-template <int NV, bool kEmbed>
-__global__ void __launch_bounds__(kThreads)
-    layer_norm_backward_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ sum, const int64_t* __restrict__ ids,
-                               int64_t vocab, const float* __restrict__ tok, const float* __restrict__ pos, const float* __restrict__ typ,
-                               const float* __restrict__ gamma, const float* __restrict__ mean, const float* __restrict__ rstd,
-                               uint4* __restrict__ ds, float* __restrict__ ds32, float* __restrict__ partial, int64_t rows,
-                               int64_t seq, int H, bool vec) {
-  constexpr int kSums = kEmbed ? 3 : 2;
-  extern __shared__ float s_sum[];  // [kSums][H]
-  wait_for_predecessor();
-  const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5, nvec = H / 8;
-  float acc[kSums][NV][8];
-#pragma unroll
-  for (int q = 0; q < kSums; ++q)
-#pragma unroll
-    for (int j = 0; j < NV; ++j)
-#pragma unroll
-      for (int k = 0; k < 8; ++k) acc[q][j][k] = 0.f;
-  for (int64_t row = (int64_t)blockIdx.x * kWarps + warp; row < rows; row += (int64_t)gridDim.x * kWarps) {
-    const float m = mean[row], rs = rstd[row];
-    Row<NV> x, g;  // xhat, then g dy
-    if constexpr (kEmbed) gather_row<NV>(ids, vocab, tok, pos, typ, row, seq, H, nvec, lane, vec, x);
-    float c1 = 0.f, c2 = 0.f;
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-      const int v = j * 32 + lane;
-      if (v >= nvec) continue;
-      if constexpr (!kEmbed) unpack8(sum[row * nvec + v], x.v[j]);
-      float w[8];
-      unpack8(dy[row * nvec + v], g.v[j]);
-      load8(gamma + v * 8, vec, w);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        x.v[j][k] = (x.v[j][k] - m) * rs;
-        acc[0][j][k] += g.v[j][k] * x.v[j][k];
-        acc[1][j][k] += g.v[j][k];
-        g.v[j][k] *= w[k];
-        c1 += g.v[j][k];
-        c2 += g.v[j][k] * x.v[j][k];
-      }
-    }
-    c1 = warp_sum(c1) / (float)H;
-    c2 = warp_sum(c2) / (float)H;
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-      const int v = j * 32 + lane;
-      if (v >= nvec) continue;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        g.v[j][k] = rs * (g.v[j][k] - c1 - x.v[j][k] * c2);
-        if constexpr (kEmbed) acc[2][j][k] += g.v[j][k];
-      }
-      if constexpr (kEmbed) {
-        float4* o = reinterpret_cast<float4*>(ds32 + row * H + v * 8);
-        o[0] = make_float4(g.v[j][0], g.v[j][1], g.v[j][2], g.v[j][3]);
-        o[1] = make_float4(g.v[j][4], g.v[j][5], g.v[j][6], g.v[j][7]);
-      } else {
-        ds[row * nvec + v] = pack8(g.v[j]);
-      }
-    }
-  }
-  // the block's warps add up in order
-  for (int w = 0; w < kWarps; ++w) {
-    if (warp == w) {
-#pragma unroll
-      for (int q = 0; q < kSums; ++q)
-#pragma unroll
-        for (int j = 0; j < NV; ++j) {
-          const int v = j * 32 + lane;
-          if (v >= nvec) continue;
-          float* o = s_sum + q * H + v * 8;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) o[k] = w == 0 ? acc[q][j][k] : o[k] + acc[q][j][k];
-        }
-    }
-    __syncthreads();
-  }
-  for (int c = (int)threadIdx.x; c < kSums * H; c += kThreads) partial[(size_t)blockIdx.x * kSums * H + c] = s_sum[c];
-}
-
-// Column sums of `blocks` partial rows of several vectors of H columns each, to as many destinations.
+// Column sums of `blocks` partial rows.
 constexpr int kFoldCols = 32, kFoldRows = 16;
-struct FoldTargets {
-  float* out[3];
-  bool add[3];
-};
 __global__ void __launch_bounds__(kFoldCols * kFoldRows)
-    fold_kernel(const float* __restrict__ partial, FoldTargets to, int blocks, int H, int vectors) {
+    fold_kernel(const float* __restrict__ partial, float* __restrict__ out, int blocks, int C, bool accumulate) {
   __shared__ float s_acc[kFoldRows][kFoldCols];
   wait_for_predecessor();
-  const int C = H * vectors, c = (int)(blockIdx.x * kFoldCols + threadIdx.x);
+  const int c = (int)(blockIdx.x * kFoldCols + threadIdx.x);
   float s = 0.f;
   if (c < C) {
 #pragma unroll 8
@@ -274,13 +48,41 @@ __global__ void __launch_bounds__(kFoldCols * kFoldRows)
   s = 0.f;
 #pragma unroll
   for (int r = 0; r < kFoldRows; ++r) s += s_acc[r][threadIdx.x];
-  const int q = c / H;
-  float* o = to.out[q] + (c - q * H);
-  *o = to.add[q] ? *o + s : s;
+  out[c] = accumulate ? out[c] + s : s;
 }
-void fold(const float* partial, const FoldTargets& to, int blocks, int H, int vectors, cudaStream_t s) {
-  launch_overlapped(fold_kernel, dim3((H * vectors + kFoldCols - 1) / kFoldCols), dim3(kFoldCols, kFoldRows), s, partial, to,
-                    blocks, H, vectors);
+void fold(const float* partial, float* out, int blocks, int C, bool accumulate, cudaStream_t s) {
+  launch_overlapped(fold_kernel, dim3((C + kFoldCols - 1) / kFoldCols), dim3(kFoldCols, kFoldRows), s, partial, out, blocks, C,
+                    accumulate);
+}
+
+// ---- embedding ------------------------------------------------------------------------------------
+// x[row] = (tok[id] + pos[position]) + typ, in this order, in fp32; an id outside the table gives a row of NaN.
+__global__ void __launch_bounds__(kThreads)
+    embed_sum_kernel(const int64_t* __restrict__ ids, int64_t vocab, const float* __restrict__ tok, const float* __restrict__ pos,
+                     const float* __restrict__ typ, float* __restrict__ x, int64_t seq, int H) {
+  wait_for_predecessor();
+  const int64_t row = blockIdx.x, id = ids[row];
+  const bool known = id >= 0 && id < vocab;
+  const float* t = tok + (known ? id : 0) * H;
+  const float* p = pos + (row % seq) * H;
+  for (int c = (int)threadIdx.x; c < H; c += kThreads) x[row * H + c] = known ? t[c] + p[c] + typ[c] : nanf("");
+}
+
+// Column sums of x [rows, H] in fp32: threads on columns, one partial row per slice of rows.
+__global__ void __launch_bounds__(kThreads)
+    column_sum_f32_kernel(const float* __restrict__ x, float* __restrict__ partial, int64_t rows, int H) {
+  wait_for_predecessor();
+  const int c = (int)(blockIdx.x * kThreads + threadIdx.x);
+  if (c >= H) return;
+  const int64_t per = (rows + gridDim.y - 1) / gridDim.y, lo = (int64_t)blockIdx.y * per, hi = min(lo + per, rows);
+  float s = 0.f;
+#pragma unroll 8
+  for (int64_t r = lo; r < hi; ++r) s += x[r * H + c];
+  partial[(size_t)blockIdx.y * H + c] = s;
+}
+int column_slices(int64_t rows, int H) {
+  const int64_t col_blocks = (H + kThreads - 1) / kThreads;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(rows / 8, 2 * 148 / col_blocks));
 }
 
 // ---- gradients of the embedding tables ------------------------------------------------------------
@@ -371,10 +173,12 @@ __global__ void __launch_bounds__(kThreads) gelu_kernel(const uint4* __restrict_
   }
 }
 
-// Warps on rows, lanes on 8 columns each, as in the column sum of a linear layer's bias gradient.
+// Warps on rows, lanes on 8 columns each, as in the column sum of a linear layer's bias gradient.  `z`: what the
+// activation was applied to, or for ReLU its result.
+template <bool kGelu>
 __global__ void __launch_bounds__(kThreads)
-    gelu_backward_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ z, uint4* __restrict__ dz,
-                         float* __restrict__ partial, int64_t rows, int cgroups) {
+    activation_backward_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ z, uint4* __restrict__ dz,
+                               float* __restrict__ partial, int64_t rows, int cgroups, bool accumulate) {
   __shared__ float s_acc[kThreads * 8];
   wait_for_predecessor();
   const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5;
@@ -392,9 +196,13 @@ __global__ void __launch_bounds__(kThreads)
       unpack8(dy[r * cgroups + cg], g);
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const float cdf = 0.5f * (1.f + erff(f[k] * kSqrtHalf));
-        const float pdf = expf(-0.5f * f[k] * f[k]) * kInvSqrt2Pi;
-        g[k] *= cdf + f[k] * pdf;
+        if constexpr (kGelu) {
+          const float cdf = 0.5f * (1.f + erff(f[k] * kSqrtHalf));
+          const float pdf = expf(-0.5f * f[k] * f[k]) * kInvSqrt2Pi;
+          g[k] *= cdf + f[k] * pdf;
+        } else {
+          g[k] = f[k] > 0.f ? g[k] : 0.f;
+        }
       }
       const uint4 packed = pack8(g);
       dz[r * cgroups + cg] = packed;
@@ -411,12 +219,100 @@ __global__ void __launch_bounds__(kThreads)
     float s = 0.f;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) s += s_acc[w * 256 + threadIdx.x];
-    partial[(size_t)blockIdx.y * cgroups * 8 + c] = s;
+    float* out = partial + (size_t)blockIdx.y * cgroups * 8 + c;
+    *out = accumulate ? *out + s : s;
   }
 }
-int gelu_splits(int64_t rows, int C) {
+int activation_splits(int64_t rows, int C) {
   const int col_blocks = (C / 8 + 31) / 32;
+  if (rows <= 64) return 1;  // the one slice's sums are the result: one launch
   return (int)std::max<int64_t>(1, std::min<int64_t>((rows + kWarps - 1) / kWarps, 4 * 148 / col_blocks));
+}
+
+// ---- loss of a span prediction ------------------------------------------------------------------------
+// (cross_entropy(logits[..., 0], start) + cross_entropy(logits[..., 1], end)) / 2 with means over the rows whose target
+// is not -100.  A few thousand values: one block, a warp per row, both columns of a row from one read.  As framework
+// calls: 10 launches forward, 16 backward.  A target outside the sequence gives NaN.
+constexpr int kSpanThreads = 1024;
+constexpr int64_t kIgnored = -100;
+__global__ void __launch_bounds__(kSpanThreads)
+    span_loss_kernel(const __nv_bfloat162* __restrict__ logits, const int64_t* __restrict__ start,
+                     const int64_t* __restrict__ end, float* __restrict__ loss, float* __restrict__ stats, int batch, int seq) {
+  // stats: [batch][2] log-sum-exp, then the two counts
+  __shared__ float s_loss[32][2];
+  __shared__ float s_count[32][2];
+  wait_for_predecessor();
+  const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5;
+  float l[2] = {0.f, 0.f}, n[2] = {0.f, 0.f};
+  for (int b = warp; b < batch; b += kSpanThreads / 32) {
+    const __nv_bfloat162* row = logits + (size_t)b * seq;
+    float m0 = -INFINITY, m1 = -INFINITY;
+    for (int i = lane; i < seq; i += 32) {
+      const float2 v = __bfloat1622float2(row[i]);
+      m0 = fmaxf(m0, v.x);
+      m1 = fmaxf(m1, v.y);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, o));
+      m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+    }
+    float e0 = 0.f, e1 = 0.f;
+    for (int i = lane; i < seq; i += 32) {
+      const float2 v = __bfloat1622float2(row[i]);
+      e0 += expf(v.x - m0);
+      e1 += expf(v.y - m1);
+    }
+    const float lse0 = m0 + logf(warp_sum(e0)), lse1 = m1 + logf(warp_sum(e1));
+    if (lane == 0) {
+      stats[2 * b] = lse0;
+      stats[2 * b + 1] = lse1;
+      const int64_t t0 = start[b], t1 = end[b];
+      if (t0 != kIgnored) {
+        l[0] += t0 >= 0 && t0 < seq ? lse0 - __bfloat162float(row[t0].x) : nanf("");
+        n[0] += 1.f;
+      }
+      if (t1 != kIgnored) {
+        l[1] += t1 >= 0 && t1 < seq ? lse1 - __bfloat162float(row[t1].y) : nanf("");
+        n[1] += 1.f;
+      }
+    }
+  }
+  if (lane == 0) {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      s_loss[warp][k] = l[k];
+      s_count[warp][k] = n[k];
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float a[2] = {0.f, 0.f}, c[2] = {0.f, 0.f};
+    for (int w = 0; w < 32; ++w)
+      for (int k = 0; k < 2; ++k) {
+        a[k] += s_loss[w][k];
+        c[k] += s_count[w][k];
+      }
+    stats[2 * batch] = c[0];
+    stats[2 * batch + 1] = c[1];
+    *loss = (a[0] / c[0] + a[1] / c[1]) / 2.f;
+  }
+}
+__global__ void __launch_bounds__(kThreads)
+    span_loss_backward_kernel(const __nv_bfloat162* __restrict__ logits, const int64_t* __restrict__ start,
+                              const int64_t* __restrict__ end, const float* __restrict__ stats,
+                              const float* __restrict__ dloss, __nv_bfloat162* __restrict__ dlogits, int batch, int seq) {
+  wait_for_predecessor();
+  const int n = batch * seq;
+  const float g = *dloss * 0.5f, g0 = g / stats[2 * batch], g1 = g / stats[2 * batch + 1];
+  for (int v = (int)(blockIdx.x * kThreads + threadIdx.x); v < n; v += (int)gridDim.x * kThreads) {
+    const int b = v / seq, i = v - b * seq;
+    const float2 x = __bfloat1622float2(logits[v]);
+    const int64_t t0 = start[b], t1 = end[b];
+    const float d0 = t0 == kIgnored ? 0.f : (expf(x.x - stats[2 * b]) - (t0 == i ? 1.f : 0.f)) * g0;
+    const float d1 = t1 == kIgnored ? 0.f : (expf(x.y - stats[2 * b + 1]) - (t1 == i ? 1.f : 0.f)) * g1;
+    dlogits[v] = __floats2bfloat162_rn(d0, d1);
+  }
 }
 
 // ---- attention gradients ------------------------------------------------------------------------------
@@ -442,82 +338,23 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// Blocks of the row kernels whose warps each walk several rows: enough for every SM, few enough partial rows to fold.
-int walk_blocks(int64_t rows) { return (int)std::max<int64_t>(1, std::min<int64_t>((rows + kWarps - 1) / kWarps, sm_count())); }
-
-bool aligned16(const float* a, const float* b, const float* c = nullptr, const float* d = nullptr, const float* e = nullptr) {
-  return (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d | (uintptr_t)e) & 15u) == 0;
-}
-
-// The instantiation for H: 256 columns per vector of a lane.
-template <typename F>
-void with_vecs(int H, F&& f) {
-  switch ((H + 255) / 256) {
-    case 1: f(std::integral_constant<int, 1>{}); return;
-    case 2: f(std::integral_constant<int, 2>{}); return;
-    case 3: f(std::integral_constant<int, 3>{}); return;
-    default: f(std::integral_constant<int, 4>{}); return;
-  }
-}
-
 }  // namespace
 
-void add_layer_norm_forward(const void* x, const void* r, const float* gamma, const float* beta, float eps, void* sum, void* y,
-                            float* mean, float* rstd, int64_t rows, int H, cudaStream_t s) {
-  BAGUA_CHECK(row_supported(rows, H), Tensor, "layer norm: unsupported shape [" << rows << ", " << H << "]");
-  with_vecs(H, [&](auto nv) {
-    launch_overlapped(add_layer_norm_kernel<nv.value>, dim3((unsigned)((rows + kWarps - 1) / kWarps)), dim3(kThreads), s,
-                      (const uint4*)x, (const uint4*)r, gamma, beta, eps, (uint4*)sum, (uint4*)y, mean, rstd, rows, H,
-                      aligned16(gamma, beta));
-  });
+void embed_sum(const int64_t* ids, int64_t vocab, const float* tok, const float* pos, const float* typ, float* x, int64_t batch,
+               int64_t seq, int H, cudaStream_t s) {
+  launch_overlapped(embed_sum_kernel, dim3((unsigned)(batch * seq)), dim3(kThreads), s, ids, vocab, tok, pos, typ, x, seq, H);
 }
 
-size_t layer_norm_backward_scratch_bytes(int64_t rows, int H) { return (size_t)walk_blocks(rows) * 2 * H * sizeof(float); }
-void layer_norm_backward(const void* dy, const void* sum, const float* gamma, const float* mean, const float* rstd, void* ds,
-                         float* dgamma, float* dbeta, bool add_gamma, bool add_beta, void* scratch, int64_t rows, int H,
-                         cudaStream_t s) {
-  BAGUA_CHECK(row_supported(rows, H), Tensor, "layer norm: unsupported shape [" << rows << ", " << H << "]");
-  const int blocks = walk_blocks(rows);
-  with_vecs(H, [&](auto nv) {
-    kernels::launch_overlapped_shared(layer_norm_backward_kernel<nv.value, false>, dim3(blocks), dim3(kThreads),
-                                      (size_t)2 * H * sizeof(float), s, (const uint4*)dy, (const uint4*)sum,
-                                      (const int64_t*)nullptr, (int64_t)0, (const float*)nullptr, (const float*)nullptr,
-                                      (const float*)nullptr, gamma, mean, rstd, (uint4*)ds, (float*)nullptr, (float*)scratch,
-                                      rows, (int64_t)1, H, aligned16(gamma, gamma));
-  });
-  fold((const float*)scratch, FoldTargets{{dgamma, dbeta, nullptr}, {add_gamma, add_beta, false}}, blocks, H, 2, s);
-}
-
-void embed_layer_norm_forward(const int64_t* ids, int64_t vocab, const float* tok, const float* pos, const float* typ, const float* gamma,
-                              const float* beta, float eps, void* y, float* mean, float* rstd, int64_t batch, int64_t seq, int H,
-                              cudaStream_t s) {
+size_t embed_backward_scratch_bytes(int64_t rows, int H) { return (size_t)column_slices(rows, H) * H * sizeof(float); }
+void embed_backward(const float* dx, const int64_t* ids, int64_t vocab, float* dtok, float* dpos, float* dtyp, void* scratch,
+                    int64_t batch, int64_t seq, int H, cudaStream_t s) {
   const int64_t rows = batch * seq;
-  BAGUA_CHECK(row_supported(rows, H), Tensor, "embedding: unsupported shape [" << rows << ", " << H << "]");
-  with_vecs(H, [&](auto nv) {
-    launch_overlapped(embed_layer_norm_kernel<nv.value>, dim3((unsigned)((rows + kWarps - 1) / kWarps)), dim3(kThreads), s, ids,
-                      vocab, tok, pos, typ, gamma, beta, eps, (uint4*)y, mean, rstd, rows, seq, H,
-                      aligned16(gamma, beta, tok, pos, typ));
-  });
-}
-
-size_t embed_backward_scratch_bytes(int64_t rows, int H) { return (size_t)walk_blocks(rows) * 3 * H * sizeof(float); }
-void embed_layer_norm_backward(const void* dy, const int64_t* ids, int64_t vocab, const float* tok, const float* pos, const float* typ,
-                               const float* gamma, const float* mean, const float* rstd, float* ds, float* dtok, float* dpos,
-                               float* dtyp, float* dgamma, float* dbeta, void* scratch, int64_t batch, int64_t seq, int H,
-                               cudaStream_t s) {
-  const int64_t rows = batch * seq;
-  BAGUA_CHECK(row_supported(rows, H) && rows <= kMaxTokens, Tensor,
-              "embedding backward: unsupported shape [" << rows << ", " << H << "]");
-  const int blocks = walk_blocks(rows);
-  with_vecs(H, [&](auto nv) {
-    kernels::launch_overlapped_shared(layer_norm_backward_kernel<nv.value, true>, dim3(blocks), dim3(kThreads),
-                                      (size_t)3 * H * sizeof(float), s, (const uint4*)dy, (const uint4*)nullptr, ids, vocab, tok, pos,
-                                      typ, gamma, mean, rstd, (uint4*)nullptr, ds, (float*)scratch, rows, seq, H,
-                                      aligned16(gamma, gamma, tok, pos, typ));
-  });
-  fold((const float*)scratch, FoldTargets{{dgamma, dbeta, dtyp}, {true, true, true}}, blocks, H, 3, s);
-  launch_overlapped(embed_scatter_kernel, dim3((unsigned)rows), dim3(kThreads), s, ids, vocab, (const float*)ds, dtok, dpos, batch, seq,
-                    H);
+  BAGUA_CHECK(rows > 0 && rows <= kMaxTokens, Tensor, "embedding backward: " << rows << " tokens");
+  const int slices = column_slices(rows, H);
+  launch_overlapped(column_sum_f32_kernel, dim3((H + kThreads - 1) / kThreads, slices), dim3(kThreads), s, dx, (float*)scratch,
+                    rows, H);
+  fold((const float*)scratch, dtyp, slices, H, true, s);
+  launch_overlapped(embed_scatter_kernel, dim3((unsigned)rows), dim3(kThreads), s, ids, vocab, dx, dtok, dpos, batch, seq, H);
 }
 
 void gelu_forward(const void* z, void* y, int64_t n, cudaStream_t s) {
@@ -526,14 +363,33 @@ void gelu_forward(const void* z, void* y, int64_t n, cudaStream_t s) {
   launch_overlapped(gelu_kernel, dim3((unsigned)std::min<int64_t>(blocks, (int64_t)sm_count() * 8)), dim3(kThreads), s,
                     (const uint4*)z, (uint4*)y, n / 8);
 }
-size_t gelu_backward_scratch_bytes(int64_t rows, int C) { return (size_t)gelu_splits(rows, C) * C * sizeof(float); }
-void gelu_backward(const void* dy, const void* z, void* dz, float* db, bool accumulate, void* scratch, int64_t rows, int C,
-                   cudaStream_t s) {
-  BAGUA_CHECK(rows > 0 && C % 8 == 0, Tensor, "gelu backward: unsupported shape [" << rows << ", " << C << "]");
-  const int splits = gelu_splits(rows, C);
-  launch_overlapped(gelu_backward_kernel, dim3((C / 8 + 31) / 32, splits), dim3(kThreads), s, (const uint4*)dy, (const uint4*)z,
-                    (uint4*)dz, (float*)scratch, rows, C / 8);
-  fold((const float*)scratch, FoldTargets{{db, nullptr, nullptr}, {accumulate, false, false}}, splits, C, 1, s);
+size_t activation_backward_scratch_bytes(int64_t rows, int C) {
+  const int splits = activation_splits(rows, C);
+  return splits == 1 ? 0 : (size_t)splits * C * sizeof(float);
+}
+void activation_backward(bool gelu, const void* dy, const void* z, void* dz, float* db, bool accumulate, void* scratch,
+                         int64_t rows, int C, cudaStream_t s) {
+  BAGUA_CHECK(rows > 0 && C % 8 == 0, Tensor, "activation backward: unsupported shape [" << rows << ", " << C << "]");
+  const int splits = activation_splits(rows, C);
+  const bool direct = splits == 1;
+  launch_overlapped(gelu ? activation_backward_kernel<true> : activation_backward_kernel<false>,
+                    dim3((C / 8 + 31) / 32, splits), dim3(kThreads), s, (const uint4*)dy, (const uint4*)z, (uint4*)dz,
+                    direct ? db : (float*)scratch, rows, C / 8, direct && accumulate);
+  if (!direct) fold((const float*)scratch, db, splits, C, accumulate, s);
+}
+
+void span_loss_forward(const void* logits, const int64_t* start, const int64_t* end, float* loss, float* stats, int64_t batch,
+                       int64_t seq, cudaStream_t s) {
+  BAGUA_CHECK(batch > 0 && seq > 0 && batch * seq < (1ll << 30), Tensor, "span loss: unsupported shape");
+  launch_overlapped(span_loss_kernel, dim3(1), dim3(kSpanThreads), s, (const __nv_bfloat162*)logits, start, end, loss, stats,
+                    (int)batch, (int)seq);
+}
+void span_loss_backward(const void* logits, const int64_t* start, const int64_t* end, const float* stats, const float* dloss,
+                        void* dlogits, int64_t batch, int64_t seq, cudaStream_t s) {
+  const int64_t n = batch * seq;
+  launch_overlapped(span_loss_backward_kernel, dim3((unsigned)std::min<int64_t>((n + kThreads - 1) / kThreads, sm_count() * 8)),
+                    dim3(kThreads), s, (const __nv_bfloat162*)logits, start, end, stats, dloss, (__nv_bfloat162*)dlogits,
+                    (int)batch, (int)seq);
 }
 
 void merge_heads(const void* const src[3], const HeadStrides stride[3], void* out, int64_t batch, int64_t seq, int heads,

@@ -1,10 +1,11 @@
-// Fused kernels for transformer encoder layers in bf16 with fp32 parameters (sm_100a).
+// Fused kernels for transformer encoders in bf16 with fp32 parameters (sm_100a).
 //
-// Around its matrix products and attention an encoder layer is a chain of passes over [rows, H] activations
-// of a few MB: residual sum, layer normalisation, GELU, and backward their gradients with column sums over all
-// rows for the parameters.  As framework calls that is two to four launches and passes per site (sum, cast of
-// the affine parameters, normalisation; backward two kernels and an accumulation).  Here each site is one
-// kernel per direction, plus the fold of its partial column sums.
+// Around its matrix products, attention and layer normalisations (library kernels) an encoder is a chain of small
+// passes: embedding lookups and sums, GELU, the bias gradients, the packing of the attention gradients, a span loss,
+// and the dense gradient of the token table.  As framework calls that is two to sixteen launches per site; here it
+// is one per direction, plus the fold of partial column sums.  Everything on the way from the input to the loss is
+// computed with the roundings of the framework's operations: a bf16 network is chaotic enough that one rounding
+// done differently in the first layer moves gradients behind sums over all tokens by their own size.
 // No counterpart in the reference, which has no model code.
 #pragma once
 
@@ -16,38 +17,30 @@
 namespace bagua {
 namespace encoder_ops {
 
-// Hidden sizes of the row kernels: one warp per row, 8 columns per lane and step, everything in registers.
-inline bool row_supported(int64_t rows, int64_t H) { return rows > 0 && H >= 8 && H % 8 == 0 && H <= 1024; }
-
-// y = layer_norm(x + r) * gamma + beta; x, r (may be null), y in bf16, gamma and beta fp32 (at any 4-byte address).  The sum is
-// rounded to bf16 and left in `sum` (null when r is).  Statistics fp32, one per row.
-void add_layer_norm_forward(const void* x, const void* r, const float* gamma, const float* beta, float eps, void* sum, void* y,
-                            float* mean, float* rstd, int64_t rows, int H, cudaStream_t s);
-// ds (bf16) and the parameters' gradients, written or added to.  `sum`: what was normalised.
-size_t layer_norm_backward_scratch_bytes(int64_t rows, int H);
-void layer_norm_backward(const void* dy, const void* sum, const float* gamma, const float* mean, const float* rstd, void* ds,
-                         float* dgamma, float* dbeta, bool add_gamma, bool add_beta, void* scratch, int64_t rows, int H,
-                         cudaStream_t s);
-
-// Input of an encoder: y = layer_norm(tok[ids] + pos[position] + typ[0]) in bf16 from fp32 tables, ids [batch, seq].  An id
-// outside [0, vocab) gives a row of NaN and no gradient.
-void embed_layer_norm_forward(const int64_t* ids, int64_t vocab, const float* tok, const float* pos, const float* typ, const float* gamma,
-                              const float* beta, float eps, void* y, float* mean, float* rstd, int64_t batch, int64_t seq, int H,
-                              cudaStream_t s);
-// Gradients of all five tables ADDED to dtok [V, H], dpos [>= seq, H], dtyp [H], dgamma, dbeta.  ds: fp32 scratch [rows, H].  Rows of one
-// token are summed in order up to kMaxOrdered occurrences; beyond that, slices of that length are added atomically.
+// x = tok[ids] + pos[position] + typ[0] in fp32, ids [batch, seq].  An id outside [0, vocab) gives a row of NaN and no
+// gradient.
+void embed_sum(const int64_t* ids, int64_t vocab, const float* tok, const float* pos, const float* typ, float* x, int64_t batch,
+               int64_t seq, int H, cudaStream_t s);
+// The tables' gradients from dx [batch * seq, H], ADDED to dtok [vocab, H], dpos [>= seq, H] and dtyp [H].  Rows of one token
+// are summed in order up to kMaxOrdered occurrences; beyond that, slices of that length are added atomically.
 constexpr int kMaxTokens = 4096, kMaxOrdered = 256;
 size_t embed_backward_scratch_bytes(int64_t rows, int H);
-void embed_layer_norm_backward(const void* dy, const int64_t* ids, int64_t vocab, const float* tok, const float* pos, const float* typ,
-                               const float* gamma, const float* mean, const float* rstd, float* ds, float* dtok, float* dpos,
-                               float* dtyp, float* dgamma, float* dbeta, void* scratch, int64_t batch, int64_t seq, int H,
-                               cudaStream_t s);
+void embed_backward(const float* dx, const int64_t* ids, int64_t vocab, float* dtok, float* dpos, float* dtyp, void* scratch,
+                    int64_t batch, int64_t seq, int H, cudaStream_t s);
 
-// y = gelu(z) (exact); backward: dz = dy * gelu'(z) and its column sums, one pass.  [rows, C] bf16, C % 8 == 0.
+// y = gelu(z) (exact).  Backward of an activation: dz = dy * gelu'(z), or dy where the ReLU's result `z` is positive, and
+// its column sums, in one pass.  [rows, C] bf16, C % 8 == 0.
 void gelu_forward(const void* z, void* y, int64_t n, cudaStream_t s);
-size_t gelu_backward_scratch_bytes(int64_t rows, int C);
-void gelu_backward(const void* dy, const void* z, void* dz, float* db, bool accumulate, void* scratch, int64_t rows, int C,
-                   cudaStream_t s);
+size_t activation_backward_scratch_bytes(int64_t rows, int C);
+void activation_backward(bool gelu, const void* dy, const void* z, void* dz, float* db, bool accumulate, void* scratch,
+                         int64_t rows, int C, cudaStream_t s);
+
+// loss = (cross_entropy(logits[..., 0], start) + cross_entropy(logits[..., 1], end)) / 2, logits [batch, seq, 2] bf16; stats:
+// 2 * batch + 2 floats for the backward.
+void span_loss_forward(const void* logits, const int64_t* start, const int64_t* end, float* loss, float* stats, int64_t batch,
+                       int64_t seq, cudaStream_t s);
+void span_loss_backward(const void* logits, const int64_t* start, const int64_t* end, const float* stats, const float* dloss,
+                        void* dlogits, int64_t batch, int64_t seq, cudaStream_t s);
 
 // out [batch, seq, 3, heads, dim] from three gradients [batch, heads, seq, dim] whose last stride is 1; strides in
 // elements (batch, head, seq) per tensor; dim a multiple of 8, all addresses and strides of 16 bytes.

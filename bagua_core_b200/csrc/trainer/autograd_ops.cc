@@ -183,12 +183,15 @@ std::shared_ptr<PoolRawTensor> scratch_for(const at::Tensor& t, size_t bytes) {
 
 // ---- linear ------------------------------------------------------------------------------------
 struct LinearNode : public Node {
-  SavedVariable x, w, z;  // z: what gelu was applied to, when it was
+  SavedVariable x, w, z;  // z: what gelu was applied to, or the ReLU's result
   at::Tensor weight, bias;  // the parameters (bias may be undefined)
   std::shared_ptr<Use> use;  // set when gradients are to be accumulated here
-  bool accumulate = false, gelu = false;
+  bool accumulate = false;
+  int activation = kNone;
 
-  std::string name() const override { return gelu ? "BaguaLinearGeluBackward" : "BaguaLinearBackward"; }
+  std::string name() const override {
+    return activation == kGelu ? "BaguaLinearGeluBackward" : activation == kRelu ? "BaguaLinearReLUBackward" : "BaguaLinearBackward";
+  }
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
     x.reset_data();
@@ -204,7 +207,7 @@ struct LinearNode : public Node {
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
     const at::Tensor dy = grads[0], xs = x.unpack(), ws = w.unpack();
     at::Tensor dy2 = dy.dim() == 2 ? dy : dy.reshape({-1, dy.size(-1)});
-    if (gelu) dy2 = through_gelu(dy2.contiguous(), out);
+    if (activation) dy2 = through_activation(dy2.contiguous(), out);
     if (task_should_compute_output(0)) {
       at::Tensor dx;
       if (!c10::GradMode::is_enabled()) {
@@ -227,23 +230,24 @@ struct LinearNode : public Node {
       }
       if (!done) out[1] = at::mm(dy2.t(), x2);  // autograd casts it to the parameter's type
     }
-    if (!gelu && bias.defined() && task_should_compute_output(2)) out[2] = bias_grad(dy2);
+    if (!activation && bias.defined() && task_should_compute_output(2)) out[2] = bias_grad(dy2);
     return out;
   }
 
-  // gelu' applied to the incoming gradient, and the bias gradient of the result from the same pass
-  at::Tensor through_gelu(const at::Tensor& dy2, variable_list& out) {
-    const at::Tensor zs = z.unpack();
+  // the activation's derivative applied to the incoming gradient, and the bias gradient of the result from the same pass
+  at::Tensor through_activation(const at::Tensor& dy2, variable_list& out) {
+    const at::Tensor zs = z.unpack(activation == kRelu ? shared_from_this() : std::shared_ptr<Node>());
     const int64_t rows = dy2.size(0);
     const int C = (int)dy2.size(1);
     const bool want = bias.defined() && task_should_compute_output(2);
     const bool add = want && accumulate && use && !use->shared && accumulates(bias, dy2);
     at::Tensor db = add ? bias.grad() : at::empty({C}, dy2.options().dtype(at::kFloat));
     at::Tensor dz = at::empty_like(dy2);
-    auto scratch = scratch_for(dy2, encoder_ops::gelu_backward_scratch_bytes(rows, C));
-    encoder_ops::gelu_backward(dy2.data_ptr(), zs.data_ptr(), dz.data_ptr(), db.data_ptr<float>(), add, scratch->data_ptr(),
-                               rows, C, stream_of(dy2));
-    count_launches(2);
+    const size_t bytes = encoder_ops::activation_backward_scratch_bytes(rows, C);
+    std::shared_ptr<PoolRawTensor> scratch = bytes ? scratch_for(dy2, bytes) : nullptr;
+    encoder_ops::activation_backward(activation == kGelu, dy2.data_ptr(), zs.data_ptr(), dz.data_ptr(), db.data_ptr<float>(),
+                                     add, scratch ? scratch->data_ptr() : nullptr, rows, C, stream_of(dy2));
+    count_launches(bytes ? 2 : 1);
     if (want && !add) out[2] = db;
     return dz;
   }
@@ -348,82 +352,108 @@ struct ConvNode : public Node {
 };
 
 // ---- encoder layers ------------------------------------------------------------------------------
-// An fp32 gradient for `param`: its `.grad` to be added to, or a new tensor for autograd.
+// An fp32 gradient for `param`: its `.grad` to be added to, or zeros for autograd.
 struct GradTarget {
   at::Tensor grad;
   bool add;
 };
-GradTarget grad_target(const at::Tensor& param, bool accumulate, bool zeroed) {
+GradTarget grad_target(const at::Tensor& param, bool accumulate) {
   if (accumulate && accumulates(param, param) && param.grad().is_contiguous()) return {param.grad(), true};
-  return {zeroed ? at::zeros(param.sizes(), param.options()) : at::empty(param.sizes(), param.options()), false};
+  return {at::zeros(param.sizes(), param.options()), false};
+}
+
+// Adds a gradient to its place, or leaves it to autograd.
+void give(const at::Tensor& param, const at::Tensor& g, bool accumulate, at::Tensor& out) {
+  if (!g.defined()) return;
+  if (!accumulate || !accumulates(param, param) || !param.grad().is_contiguous()) {
+    out = g;  // autograd casts it to the parameter's type
+    return;
+  }
+  if (g.scalar_type() == at::kBFloat16)
+    kernels::cuda::accumulate_bf16((float*)param.grad().data_ptr(), g.data_ptr(), g.numel(), stream_of(g));
+  else
+    kernels::add_inplace(param.grad().data_ptr(), g.data_ptr(), DType::F32, g.numel(), ctx_of(g));
+  count_launches(1);
 }
 
 struct LayerNormNode : public Node {
-  SavedVariable sum, mean, rstd;
+  SavedVariable sum, mean, rstd, g, b;  // g, b: the parameters in bf16
   at::Tensor gamma, beta;
   bool accumulate = false, residual = false;
 
   std::string name() const override { return "BaguaAddLayerNormBackward"; }
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
-    sum.reset_data();
-    mean.reset_data();
-    rstd.reset_data();
+    for (SavedVariable* v : {&sum, &mean, &rstd, &g, &b}) v->reset_data();
   }
   variable_list apply(variable_list&& grads) override {  // x, r, gamma, beta
     std::lock_guard<std::mutex> lock(mutex_);
     variable_list out(4);
     if (!grads[0].defined()) return out;
-    const at::Tensor dy = grads[0].contiguous(), s = sum.unpack(), m = mean.unpack(), rs = rstd.unpack();
-    const int H = (int)s.size(-1);
-    const int64_t rows = s.numel() / H;
-    at::Tensor ds = at::empty_like(s);
-    const GradTarget dg = grad_target(gamma, accumulate && task_should_compute_output(2), false);
-    const GradTarget db = grad_target(beta, accumulate && task_should_compute_output(3), false);
-    auto scratch = scratch_for(s, encoder_ops::layer_norm_backward_scratch_bytes(rows, H));
-    encoder_ops::layer_norm_backward(dy.data_ptr(), s.data_ptr(), gamma.data_ptr<float>(), m.data_ptr<float>(),
-                                     rs.data_ptr<float>(), ds.data_ptr(), dg.grad.data_ptr<float>(), db.grad.data_ptr<float>(),
-                                     dg.add, db.add, scratch->data_ptr(), rows, H, stream_of(s));
-    count_launches(2);
-    out[0] = ds;
-    if (residual) out[1] = ds;
-    if (!dg.add) out[2] = dg.grad;
-    if (!db.add) out[3] = db.grad;
+    const at::Tensor s = sum.unpack();
+    const auto d = at::native_layer_norm_backward(grads[0].contiguous(), s, {s.size(-1)}, mean.unpack(), rstd.unpack(),
+                                                  g.unpack(), b.unpack(),
+                                                  {true, task_should_compute_output(2), task_should_compute_output(3)});
+    out[0] = std::get<0>(d);
+    if (residual) out[1] = out[0];
+    give(gamma, std::get<1>(d), accumulate, out[2]);
+    give(beta, std::get<2>(d), accumulate, out[3]);
     return out;
   }
 };
 
 struct EmbedNode : public Node {
-  SavedVariable ids, mean, rstd;
+  SavedVariable ids, sum, mean, rstd;
   at::Tensor param[5];  // tok, pos, typ, gamma, beta
   bool accumulate = false;
 
   std::string name() const override { return "BaguaEmbedLayerNormBackward"; }
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
-    ids.reset_data();
-    mean.reset_data();
-    rstd.reset_data();
+    for (SavedVariable* v : {&ids, &sum, &mean, &rstd}) v->reset_data();
   }
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
     variable_list out(5);
     if (!grads[0].defined()) return out;
-    const at::Tensor dy = grads[0].contiguous(), id = ids.unpack(), m = mean.unpack(), rs = rstd.unpack();
+    const at::Tensor id = ids.unpack(), s = sum.unpack();
     const int H = (int)param[0].size(1);
     const int64_t batch = id.size(0), seq = id.size(1);
-    GradTarget to[5];
-    for (int k = 0; k < 5; ++k) to[k] = grad_target(param[k], accumulate && task_should_compute_output((size_t)k), true);
-    at::Tensor ds = at::empty({batch * seq, H}, dy.options().dtype(at::kFloat));
-    auto scratch = scratch_for(dy, encoder_ops::embed_backward_scratch_bytes(batch * seq, H));
-    encoder_ops::embed_layer_norm_backward(
-        dy.data_ptr(), id.data_ptr<int64_t>(), param[0].size(0), param[0].data_ptr<float>(), param[1].data_ptr<float>(),
-        param[2].data_ptr<float>(), param[3].data_ptr<float>(), m.data_ptr<float>(), rs.data_ptr<float>(), ds.data_ptr<float>(),
-        to[0].grad.data_ptr<float>(), to[1].grad.data_ptr<float>(), to[2].grad.data_ptr<float>(), to[3].grad.data_ptr<float>(),
-        to[4].grad.data_ptr<float>(), scratch->data_ptr(), batch, seq, H, stream_of(dy));
+    const auto d = at::native_layer_norm_backward(grads[0].to(at::kFloat).contiguous(), s, {H}, mean.unpack(), rstd.unpack(),
+                                                  param[3], param[4], {true, true, true});
+    give(param[3], std::get<1>(d), accumulate, out[3]);
+    give(param[4], std::get<2>(d), accumulate, out[4]);
+    GradTarget to[3];
+    for (int k = 0; k < 3; ++k) to[k] = grad_target(param[k], accumulate && task_should_compute_output((size_t)k));
+    auto scratch = scratch_for(s, encoder_ops::embed_backward_scratch_bytes(batch * seq, H));
+    encoder_ops::embed_backward(std::get<0>(d).data_ptr<float>(), id.data_ptr<int64_t>(), param[0].size(0),
+                                to[0].grad.data_ptr<float>(), to[1].grad.data_ptr<float>(), to[2].grad.data_ptr<float>(),
+                                scratch->data_ptr(), batch, seq, H, stream_of(s));
     count_launches(3);
-    for (int k = 0; k < 5; ++k)
+    for (int k = 0; k < 3; ++k)
       if (!to[k].add) out[(size_t)k] = to[k].grad;
+    return out;
+  }
+};
+
+struct SpanLossNode : public Node {
+  SavedVariable logits, start, end, stats;
+
+  std::string name() const override { return "BaguaSpanLossBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (SavedVariable* v : {&logits, &start, &end, &stats}) v->reset_data();
+  }
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    variable_list out(1);
+    if (!grads[0].defined()) return out;
+    const at::Tensor x = logits.unpack(), a = start.unpack(), b = end.unpack(), st = stats.unpack();
+    at::Tensor dx = at::empty_like(x);
+    encoder_ops::span_loss_backward(x.data_ptr(), a.data_ptr<int64_t>(), b.data_ptr<int64_t>(), st.data_ptr<float>(),
+                                    grads[0].data_ptr<float>(), dx.data_ptr(), x.size(0), x.size(1), stream_of(x));
+    count_launches(1);
+    out[0] = dx;
     return out;
   }
 };
@@ -462,8 +492,9 @@ bool fp32_param(const at::Tensor& p, int64_t H, const at::Tensor& like) {
 }  // namespace
 
 at::Tensor linear(const at::Tensor& x, const at::Tensor& weight, const std::optional<at::Tensor>& bias,
-                  const std::optional<at::Tensor>& w_low, bool accumulate, bool gelu) {
-  BAGUA_CHECK(!gelu || gelu_fusable(x, weight.size(0)), Tensor, "gelu cannot be fused with this layer");
+                  const std::optional<at::Tensor>& w_low, bool accumulate, int activation) {
+  BAGUA_CHECK(activation == kNone || ((activation == kGelu || activation == kRelu) && activation_fusable(x, weight.size(0))), Tensor,
+              "the activation cannot be fused with this layer");
   const at::Tensor b = bias.value_or(at::Tensor());
   std::shared_ptr<LinearNode> node;
   if (torch::autograd::compute_requires_grad(x, weight, b)) node = make_node<LinearNode>(x, weight, b);
@@ -479,10 +510,14 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& weight, const std::opti
       shape.back() = ws.size(0);
       y = at::empty(shape, xs.options());
       at::Tensor y2 = y.dim() == 2 ? y : y.view({-1, ws.size(0)});
-      if (!gemm::linear(xs.dim() == 2 ? xs : xs.view({-1, xs.size(-1)}), ws, low[2], y2)) y = at::Tensor();
+      if (!gemm::linear(xs.dim() == 2 ? xs : xs.view({-1, xs.size(-1)}), ws, low[2], activation == kRelu, y2)) y = at::Tensor();
     }
+    const bool product_only = !y.defined();
     if (!y.defined()) y = at::linear(xs, ws, b.defined() ? std::optional<at::Tensor>(low[2]) : std::nullopt);
-    if (gelu) {
+    if (activation == kRelu) {
+      if (product_only) y.relu_();
+      y = y.contiguous();
+    } else if (activation == kGelu) {
       z = y.contiguous();
       y = at::empty_like(z);
       encoder_ops::gelu_forward(z.data_ptr(), y.data_ptr(), z.numel(), stream_of(z));
@@ -492,13 +527,14 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& weight, const std::opti
   if (node) {
     node->x = SavedVariable(xs, false);
     node->w = SavedVariable(ws, false);
-    if (gelu) node->z = SavedVariable(z, false);
-    node->gelu = gelu;
+    if (activation == kGelu) node->z = SavedVariable(z, false);
+    node->activation = activation;
     node->weight = weight;
     node->bias = b;
     node->accumulate = accumulate;
     if (accumulate && weight.requires_grad()) node->use = begin_use(weight);
     torch::autograd::set_history(y, node);
+    if (activation == kRelu) node->z = SavedVariable(y, /*is_output=*/true);
   }
   return y;
 }
@@ -569,10 +605,10 @@ at::Tensor conv_bias_relu(const at::Tensor& x, const at::Tensor& weight, const a
 
 at::Tensor add_layer_norm(const at::Tensor& x, const std::optional<at::Tensor>& r, const at::Tensor& gamma,
                           const at::Tensor& beta, double eps, bool accumulate) {
-  const int64_t H = x.size(-1), rows = x.numel() / H;
+  const int64_t H = x.size(-1);
   const at::Tensor res = r.value_or(at::Tensor());
-  BAGUA_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && encoder_ops::row_supported(rows, H) &&
-                  fp32_param(gamma, H, x) && fp32_param(beta, H, x) && gamma.dim() == 1 && beta.dim() == 1 &&
+  BAGUA_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.numel() > 0 && fp32_param(gamma, H, x) &&
+                  fp32_param(beta, H, x) && gamma.dim() == 1 && beta.dim() == 1 &&
                   (!res.defined() || (res.sizes() == x.sizes() && res.scalar_type() == at::kBFloat16 && res.device() == x.device())),
               Tensor, "add_layer_norm needs bf16 CUDA activations of one shape and fp32 parameters");
   std::shared_ptr<LayerNormNode> node;
@@ -581,23 +617,19 @@ at::Tensor add_layer_norm(const at::Tensor& x, const std::optional<at::Tensor>& 
     node->set_next_edges(torch::autograd::collect_next_edges(x, res, gamma, beta));
   }
   at::Tensor sum, y, mean, rstd;
+  std::array<at::Tensor, 2> low{gamma, beta};
   {
     PlainDispatch plain;
-    const at::Tensor xs = x.contiguous(), rc = res.defined() ? res.contiguous() : res;
-    y = at::empty_like(xs);
-    sum = res.defined() ? at::empty_like(xs) : xs;
-    mean = at::empty({2, rows}, xs.options().dtype(at::kFloat));
-    rstd = mean.select(0, 1);
-    mean = mean.select(0, 0);
-    encoder_ops::add_layer_norm_forward(xs.data_ptr(), res.defined() ? rc.data_ptr() : nullptr, gamma.data_ptr<float>(),
-                                        beta.data_ptr<float>(), (float)eps, res.defined() ? sum.data_ptr() : nullptr, y.data_ptr(),
-                                        mean.data_ptr<float>(), rstd.data_ptr<float>(), rows, (int)H, stream_of(xs));
-    count_launches(1);
+    sum = (res.defined() ? at::add(x, res) : x).contiguous();
+    to_bf16(low);
+    std::tie(y, mean, rstd) = at::native_layer_norm(sum, {H}, low[0], low[1], eps);
   }
   if (node) {
     node->sum = SavedVariable(sum, false);
     node->mean = SavedVariable(mean, false);
     node->rstd = SavedVariable(rstd, false);
+    node->g = SavedVariable(low[0], false);
+    node->b = SavedVariable(low[1], false);
     node->gamma = gamma;
     node->beta = beta;
     node->accumulate = accumulate;
@@ -610,8 +642,8 @@ at::Tensor add_layer_norm(const at::Tensor& x, const std::optional<at::Tensor>& 
 at::Tensor embed_layer_norm(const at::Tensor& ids, const at::Tensor& tok, const at::Tensor& pos, const at::Tensor& typ,
                             const at::Tensor& gamma, const at::Tensor& beta, double eps, bool accumulate) {
   const int64_t H = tok.size(1);
-  BAGUA_CHECK(ids.is_cuda() && ids.scalar_type() == at::kLong && ids.dim() == 2 && ids.numel() <= encoder_ops::kMaxTokens &&
-                  encoder_ops::row_supported(ids.numel(), H),
+  BAGUA_CHECK(ids.is_cuda() && ids.scalar_type() == at::kLong && ids.dim() == 2 && ids.numel() > 0 &&
+                  ids.numel() <= encoder_ops::kMaxTokens,
               Tensor, "embed_layer_norm: unsupported ids");
   for (const at::Tensor* p : {&tok, &pos, &typ, &gamma, &beta})
     BAGUA_CHECK(fp32_param(*p, H, ids), Tensor, "embed_layer_norm needs fp32 tables on the ids' device");
@@ -621,31 +653,67 @@ at::Tensor embed_layer_norm(const at::Tensor& ids, const at::Tensor& tok, const 
     node = std::shared_ptr<EmbedNode>(new EmbedNode(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(tok, pos, typ, gamma, beta));
   }
-  at::Tensor idc, y, mean, rstd;
+  at::Tensor idc, sum, mean, rstd;
+  std::array<at::Tensor, 1> y;
   {
     PlainDispatch plain;
     idc = ids.contiguous();
     const int64_t batch = ids.size(0), seq = ids.size(1);
-    y = at::empty({batch, seq, H}, tok.options().dtype(at::kBFloat16));
-    mean = at::empty({2, batch * seq}, tok.options());
-    rstd = mean.select(0, 1);
-    mean = mean.select(0, 0);
-    encoder_ops::embed_layer_norm_forward(idc.data_ptr<int64_t>(), tok.size(0), tok.data_ptr<float>(), pos.data_ptr<float>(),
-                                          typ.data_ptr<float>(), gamma.data_ptr<float>(), beta.data_ptr<float>(), (float)eps,
-                                          y.data_ptr(), mean.data_ptr<float>(), rstd.data_ptr<float>(), batch, seq, (int)H,
-                                          stream_of(tok));
+    sum = at::empty({batch, seq, H}, tok.options());
+    encoder_ops::embed_sum(idc.data_ptr<int64_t>(), tok.size(0), tok.data_ptr<float>(), pos.data_ptr<float>(),
+                           typ.data_ptr<float>(), sum.data_ptr<float>(), batch, seq, (int)H, stream_of(tok));
     count_launches(1);
+    std::tie(y[0], mean, rstd) = at::native_layer_norm(sum, {H}, gamma, beta, eps);
+    to_bf16(y);
   }
   if (node) {
     node->ids = SavedVariable(idc, false);
+    node->sum = SavedVariable(sum, false);
     node->mean = SavedVariable(mean, false);
     node->rstd = SavedVariable(rstd, false);
     const at::Tensor* ps[5] = {&tok, &pos, &typ, &gamma, &beta};
     for (int k = 0; k < 5; ++k) node->param[k] = *ps[k];
     node->accumulate = accumulate;
-    torch::autograd::set_history(y, node);
+    torch::autograd::set_history(y[0], node);
   }
-  return y;
+  return y[0];
+}
+
+at::Tensor span_loss(const at::Tensor& logits, const at::Tensor& start, const at::Tensor& end) {
+  const int64_t B = logits.size(0);
+  BAGUA_CHECK(logits.is_cuda() && logits.dim() == 3 && logits.size(2) == 2 && logits.scalar_type() == at::kBFloat16 &&
+                  logits.numel() > 0 && logits.numel() < (1ll << 30),
+              Tensor, "span_loss needs bf16 CUDA logits [batch, seq, 2]");
+  for (const at::Tensor* t : {&start, &end})
+    BAGUA_CHECK(t->device() == logits.device() && t->scalar_type() == at::kLong && t->dim() == 1 && t->size(0) == B, Tensor,
+                "span_loss needs int64 positions [batch] on the logits' device");
+  std::shared_ptr<SpanLossNode> node;
+  if (torch::autograd::compute_requires_grad(logits)) {
+    node = std::shared_ptr<SpanLossNode>(new SpanLossNode(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(logits));
+  }
+  at::Tensor x, a, b, loss, stats;
+  {
+    PlainDispatch plain;
+    x = logits.contiguous();
+    if ((uintptr_t)x.data_ptr() % 4 != 0) x = x.clone();
+    a = start.contiguous();
+    b = end.contiguous();
+    const auto f = x.options().dtype(at::kFloat);
+    loss = at::empty({}, f);
+    stats = at::empty({2 * B + 2}, f);
+    encoder_ops::span_loss_forward(x.data_ptr(), a.data_ptr<int64_t>(), b.data_ptr<int64_t>(), loss.data_ptr<float>(),
+                                   stats.data_ptr<float>(), B, x.size(1), stream_of(x));
+    count_launches(1);
+  }
+  if (node) {
+    node->logits = SavedVariable(x, false);
+    node->start = SavedVariable(a, false);
+    node->end = SavedVariable(b, false);
+    node->stats = SavedVariable(stats, false);
+    torch::autograd::set_history(loss, node);
+  }
+  return loss;
 }
 
 at::Tensor attention(const at::Tensor& qkv, int64_t heads, double dropout) {

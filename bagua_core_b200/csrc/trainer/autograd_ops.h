@@ -25,13 +25,17 @@ struct OpStats {
 // y = x Wᵀ + b in bf16.  `w_low`: W in bf16 when the caller has it, else it is cast here.  With `accumulate`, the
 // backward adds the gradients of W and b to their fp32 `.grad` itself where nobody can tell the difference
 // (autograd_ops.cc, `accumulates`), and hands autograd nothing for them.
-// `gelu`: y = gelu(x Wᵀ + b), whose backward makes the bias gradient in the pass that applies gelu' (needs
-// gelu_fusable()).
+// `activation`: applied to the result; its backward makes the bias gradient in the pass that applies the derivative
+// (needs activation_fusable()).
+enum Activation { kNone = 0, kGelu = 1, kRelu = 2 };
 at::Tensor linear(const at::Tensor& x, const at::Tensor& weight, const std::optional<at::Tensor>& bias,
-                  const std::optional<at::Tensor>& w_low, bool accumulate, bool gelu);
-inline bool gelu_fusable(const at::Tensor& x, int64_t out_features) { return x.is_cuda() && out_features % 8 == 0 && x.numel() > 0; }
+                  const std::optional<at::Tensor>& w_low, bool accumulate, int activation);
+inline bool activation_fusable(const at::Tensor& x, int64_t out_features) {
+  return x.is_cuda() && out_features % 8 == 0 && x.numel() > 0;
+}
 
-// layer_norm(x + r) of bf16 activations with fp32 parameters (r may be missing); CUDA, `encoder_ops::row_supported`.
+// layer_norm(x + r) of bf16 activations with fp32 parameters (r may be missing); CUDA.  The library's normalisation
+// (its kernels run at the speed of their bytes) with the casts of the parameters as one launch.
 at::Tensor add_layer_norm(const at::Tensor& x, const std::optional<at::Tensor>& r, const at::Tensor& gamma,
                           const at::Tensor& beta, double eps, bool accumulate);
 
@@ -39,6 +43,10 @@ at::Tensor add_layer_norm(const at::Tensor& x, const std::optional<at::Tensor>& 
 // `encoder_ops::kMaxTokens` of them.
 at::Tensor embed_layer_norm(const at::Tensor& ids, const at::Tensor& tok, const at::Tensor& pos, const at::Tensor& typ,
                             const at::Tensor& gamma, const at::Tensor& beta, double eps, bool accumulate);
+
+// (cross_entropy(logits[..., 0], start) + cross_entropy(logits[..., 1], end)) / 2 of bf16 logits [batch, seq, 2] with int64
+// positions [batch]; rows with position -100 do not count.
+at::Tensor span_loss(const at::Tensor& logits, const at::Tensor& start, const at::Tensor& end);
 
 // Multi-head attention of a packed projection qkv [batch, seq, 3 * heads * dim] (bf16, CUDA): [batch, seq, heads * dim].
 at::Tensor attention(const at::Tensor& qkv, int64_t heads, double dropout);

@@ -61,7 +61,7 @@ uint32_t alignment_log(const void* p) {
 struct Problem {
   cublasOperation_t opa, opb;
   int64_t a_rows, a_cols, b_rows, b_cols, d_rows, d_cols;
-  bool d_fp32, bias, forward;
+  bool d_fp32, bias, forward, relu;
 };
 
 bool build(Plan& p, cublasLtHandle_t lt, const Problem& q, const void* A, const void* B, const void* D, const void* bias) {
@@ -72,10 +72,13 @@ bool build(Plan& p, cublasLtHandle_t lt, const Problem& q, const void* A, const 
   };
   if (!set(CUBLASLT_MATMUL_DESC_TRANSA, &q.opa, sizeof(q.opa)) || !set(CUBLASLT_MATMUL_DESC_TRANSB, &q.opb, sizeof(q.opb)))
     return false;
+  if (q.bias || q.relu) {
+    const cublasLtEpilogue_t e = q.bias ? (q.relu ? CUBLASLT_EPILOGUE_RELU_BIAS : CUBLASLT_EPILOGUE_BIAS) : CUBLASLT_EPILOGUE_RELU;
+    if (!set(CUBLASLT_MATMUL_DESC_EPILOGUE, &e, sizeof(e))) return false;
+  }
   if (q.bias) {
-    const cublasLtEpilogue_t e = CUBLASLT_EPILOGUE_BIAS;
     const cudaDataType_t t = CUDA_R_16BF;
-    if (!set(CUBLASLT_MATMUL_DESC_EPILOGUE, &e, sizeof(e)) || !set(CUBLASLT_MATMUL_DESC_BIAS_DATA_TYPE, &t, sizeof(t)) ||
+    if (!set(CUBLASLT_MATMUL_DESC_BIAS_DATA_TYPE, &t, sizeof(t)) ||
         !set(CUBLASLT_MATMUL_DESC_BIAS_POINTER, &bias, sizeof(bias)))
       return false;
   }
@@ -114,7 +117,7 @@ bool run(int kind, const Problem& q, int64_t m, int64_t n, int64_t k, const at::
   key.m = m;
   key.n = n;
   key.k = k;
-  key.flags = (q.bias ? 1u : 0u) | (add ? 2u : 0u) | (alignment_log(A.data_ptr()) << 4) | (alignment_log(B.data_ptr()) << 8) |
+  key.flags = (q.bias ? 1u : 0u) | (add ? 2u : 0u) | (q.relu ? 4u : 0u) | (alignment_log(A.data_ptr()) << 4) | (alignment_log(B.data_ptr()) << 8) |
               (alignment_log(D.data_ptr()) << 12) | (q.bias ? alignment_log(bias) << 16 : 0u);
   // per thread: a plan's descriptor carries the bias pointer of the call
   using Plans = std::unordered_map<Key, std::unique_ptr<Plan>, Hash>;
@@ -149,25 +152,25 @@ bool plain(const at::Tensor& t) {
 
 }  // namespace
 
-bool linear(const at::Tensor& x, const at::Tensor& w, const at::Tensor& b, at::Tensor& y) {
+bool linear(const at::Tensor& x, const at::Tensor& w, const at::Tensor& b, bool relu, at::Tensor& y) {
   if (!plain(x) || !plain(w) || !plain(y) || (b.defined() && (b.scalar_type() != at::kBFloat16 || !b.is_contiguous())))
     return false;
   const int64_t M = x.size(0), K = x.size(1), N = w.size(0);
-  const Problem q{CUBLAS_OP_T, CUBLAS_OP_N, K, N, K, M, N, M, false, b.defined(), true};
+  const Problem q{CUBLAS_OP_T, CUBLAS_OP_N, K, N, K, M, N, M, false, b.defined(), true, relu};
   return run(0, q, M, N, K, w, x, y, b.defined() ? b.data_ptr() : nullptr, false);
 }
 
 bool input_grad(const at::Tensor& dy, const at::Tensor& w, at::Tensor& dx) {
   if (!plain(dy) || !plain(w) || !plain(dx)) return false;
   const int64_t M = dy.size(0), N = dy.size(1), K = w.size(1);
-  const Problem q{CUBLAS_OP_N, CUBLAS_OP_N, K, N, N, M, K, M, false, false, false};
+  const Problem q{CUBLAS_OP_N, CUBLAS_OP_N, K, N, N, M, K, M, false, false, false, false};
   return run(1, q, M, N, K, w, dy, dx, nullptr, false);
 }
 
 bool weight_grad(const at::Tensor& dy, const at::Tensor& x, at::Tensor& g, bool accumulate) {
   if (!plain(dy) || !plain(x) || g.scalar_type() != at::kFloat || !g.is_contiguous() || g.dim() != 2) return false;
   const int64_t M = dy.size(0), N = dy.size(1), K = x.size(1);
-  const Problem q{CUBLAS_OP_N, CUBLAS_OP_T, K, M, N, M, K, N, true, false, false};
+  const Problem q{CUBLAS_OP_N, CUBLAS_OP_T, K, M, N, M, K, N, true, false, false, false};
   return run(2, q, M, N, K, x, dy, g, nullptr, accumulate);
 }
 

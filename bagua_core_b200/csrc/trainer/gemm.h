@@ -14,8 +14,8 @@ namespace gemm {
 
 // All operands are 2-D, bf16, contiguous and on one CUDA device; false: not available for these, nothing was done.
 
-// y [M, N] = x [M, K] w [N, K]ᵀ + b [N] (b may be undefined)
-bool linear(const at::Tensor& x, const at::Tensor& w, const at::Tensor& b, at::Tensor& y);
+// y [M, N] = x [M, K] w [N, K]ᵀ + b [N] (b may be undefined), at least 0 with `relu`
+bool linear(const at::Tensor& x, const at::Tensor& w, const at::Tensor& b, bool relu, at::Tensor& y);
 // dx [M, K] = dy [M, N] w [N, K]
 bool input_grad(const at::Tensor& dy, const at::Tensor& w, at::Tensor& dx);
 // g [N, K] (fp32) = dy [M, N]ᵀ x [M, K], added to what is there with `accumulate`

@@ -9,9 +9,9 @@ in-place weight-gradient accumulation is on (`bagua_core_b200.ops.wgrad.enabled`
 they skip the per-forward weight casts and the cast-and-add of every weight gradient.
 
 Under bf16 autocast on a GPU what lies between the projections runs as this package's kernels
-(`csrc/kernels/encoder_ops.h`): residual sum + LayerNorm, the embedding sum + LayerNorm, GELU with the
-projection in front of it, the packing of the attention gradients.  Parameters, results (to the
-rounding of bf16) and everything else stay those of the plain composition below, which runs elsewhere."""
+(`csrc/kernels/encoder_ops.h`) and the library's LayerNorm in native autograd functions: the embedding
+sum and the gradients of its tables, GELU with the projection in front of it, the packing of the attention
+gradients, the span loss.  The roundings are those of the plain composition below, which runs elsewhere."""
 from __future__ import annotations
 
 from dataclasses import dataclass
@@ -104,7 +104,7 @@ class _Layer(nn.Module):
             p = self.p if self.training else 0.0
             a = self.proj(_C.attention(self.qkv(x), self.heads, p))
             x = self._add_norm(self.ln1, x, self.drop(a) if p else a)
-            f = self.fc2(self.fc1(x, gelu=True))
+            f = self.fc2(self.fc1(x, "gelu"))
             return self._add_norm(self.ln2, x, self.drop(f) if p else f)
         q, k, v = self.qkv(x).view(b, s, 3, self.heads, h // self.heads).permute(2, 0, 3, 1, 4)
         a = F.scaled_dot_product_attention(q, k, v, dropout_p=self.p if self.training else 0.0)
@@ -151,6 +151,10 @@ class BertForQuestionAnswering(nn.Module):
         x = self.drop(x)
         for layer in self.layers:
             x = layer(x)
+        if (start_positions is not None and x.dtype == torch.bfloat16 and _fused(x, self.ln) and x.numel() > 0
+                and all(t.is_cuda and t.dtype == torch.int64 and t.dim() == 1 for t in (start_positions, end_positions))):
+            logits = _C.linear(x, self.qa.weight, self.qa.bias, None, False)
+            return _C.span_loss(logits, start_positions, end_positions)
         logits = self.qa(x).float()
         start, end = logits[..., 0], logits[..., 1]
         if start_positions is None:

@@ -22,16 +22,24 @@ from . import shadow as _shadow
 from . import wgrad as _wgrad
 
 
+_ACTIVATIONS = {"gelu": (1, F.gelu), "relu": (2, F.relu)}
+
+
 class ShadowLinear(nn.Linear):
-    def forward(self, x: torch.Tensor, gelu: bool = False) -> torch.Tensor:
-        """`gelu`: followed by GELU, in the same autograd function where the layer runs natively."""
+    def forward(self, x: torch.Tensor, activation: str = "") -> torch.Tensor:
+        """`activation` ("gelu", "relu"): applied to the result, in the same autograd function where the layer runs
+        natively."""
+        code, act = _ACTIVATIONS[activation] if activation else (0, None)
         dev = x.device.type
         managed = getattr(self.weight, "_bagua_bf16", None) is not None  # an optimizer keeps a bf16 copy
         if ((managed or _wgrad.enabled) and torch.is_autocast_enabled(dev)
                 and torch.get_autocast_dtype(dev) == torch.bfloat16):
             # the copy when it is current, a fresh cast otherwise: the same code path either way
-            fused = gelu and _C.gelu_fusable(x, self.out_features)
-            y = _C.linear(x, self.weight, self.bias, _shadow.autocast_copy(self.weight), _wgrad.enabled, fused)
-            return F.gelu(y) if gelu and not fused else y
-        y = super().forward(x)
-        return F.gelu(y) if gelu else y
+            if code and _C.activation_fusable(x, self.out_features):
+                act = None
+            else:
+                code = 0
+            y = _C.linear(x, self.weight, self.bias, _shadow.autocast_copy(self.weight), _wgrad.enabled, code)
+        else:
+            y = super().forward(x)
+        return y if act is None else act(y)
