@@ -48,9 +48,11 @@ int SgdPlan::step(const std::vector<SgdGroup>& groups, uint64_t stream) {
   if (device_ >= 0)
     launches = kernels::cuda::sgd_steps(segs_.data(), (int)segs_.size(), (cudaStream_t)stream);
   else
-    for (const auto& a : segs_)
+    for (const auto& a : segs_) {
       kernels::sgd_momentum_flat_shadow(a.p, a.g, a.m, a.shadow, a.n, a.lr, a.momentum, a.dampening, a.weight_decay,
                                         a.nesterov, a.first, kernels::Ctx{});
+      ++launches;
+    }
   for (auto& a : segs_) a.first = false;
   return launches;
 }

@@ -3,7 +3,7 @@
 Under bf16 autocast every forward pass casts every fp32 weight to bf16 again (for VGG-16 that is
 33 cast kernels and 0.8 GB of traffic per step, about 5 % of the step on a B200).  An optimizer
 that already streams over all parameters can write the bf16 value of each updated parameter in the
-same pass (`FlatSGD(bf16_shadow=True)`, kernel `sgd_shadow_kernel` in `csrc/kernels/elementwise.cu`);
+same pass (`FlatSGD(bf16_shadow=True)`, kernel `sgd_kernel` in `csrc/kernels/elementwise.cu`);
 modules that compute in bf16 then take their weight from that copy (`lookup`) and skip the cast.
 
 A copy is used only while it is known to equal the parameter rounded to bf16:
