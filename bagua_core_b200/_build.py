@@ -54,6 +54,7 @@ SOURCES = [
     "kernels/fused_emu.cc",
     "kernels/no_alloc.cu",
     "kernels/model_ops.cu",
+    "kernels/first_conv.cu",
     "kernels/model_ops_cpu.cc",
     "kernels/encoder_ops.cu",
 ]

@@ -36,6 +36,18 @@ size_t bias_relu_backward_scratch_bytes(int64_t rows, int C);
 void bias_relu_backward_bf16(const void* dy, const void* y, void* dz, float* db, int64_t rows, int C, void* scratch,
                              cudaStream_t stream, bool accumulate = false);
 
+// Backward of relu(conv3x3(x) + bias), stride and padding 1, where the gradient of x is not wanted (a network's first
+// layer): with dz = dy where y > 0, dw [C, 3, 3, Ci] = sum over pixels of dz and the pixel's patch of x, db [C] = sum of
+// dz, both fp32, written or added to (db may be null); dz itself is not written.  x [N, H, W, Ci], dy and y
+// [N, H, W, C], bf16 and channels-last; dy and y 16-byte aligned.  More than 3 input channels (patches beyond 32
+// values) are the library's.
+inline bool first_conv_backward_supported(int64_t N, int64_t H, int64_t W, int64_t C, int64_t Ci) {
+  return N > 0 && H > 0 && W > 0 && N * H * W < (1ll << 30) && C >= 64 && C % 64 == 0 && C <= 4096 && Ci >= 1 && Ci <= 3;
+}
+size_t first_conv_backward_scratch_bytes(int64_t rows, int C, int Ci);
+void first_conv_backward(const void* dy, const void* y, const void* x, float* dw, bool add_w, float* db, bool add_b, int64_t N,
+                         int64_t H, int64_t W, int C, int Ci, void* scratch, cudaStream_t s);
+
 // out[c] (+)= sum over rows of x [rows, C] in bf16, accumulated in fp32 in a fixed order: the bias gradient of a
 // linear layer.  C a multiple of 8, x 16-byte aligned.  (3072 x 1024: 8 us; the library's reduction 13 us.)
 inline bool column_sum_supported(int64_t rows, int C) { return rows > 0 && C >= 8 && C % 8 == 0; }

@@ -296,6 +296,10 @@ struct ConvNode : public Node {
     const at::Tensor dy = grads[0].contiguous(at::MemoryFormat::ChannelsLast);
     const bool alone = accumulate && use && !use->shared;
     const int C = (int)ws.size(0);
+    if (!pool && first_layer(xs, dy, a)) {
+      first_layer_backward(xs, dy, a, alone, out);
+      return out;
+    }
     at::Tensor dz = at::empty_like(a);
     // the bias gradient is added to `.grad` by the fold of its partial sums
     const bool add_bias = alone && dy.is_cuda() && task_should_compute_output(2) && accumulates(bias, dy);
@@ -324,6 +328,33 @@ struct ConvNode : public Node {
       }
     }
     return out;
+  }
+
+  // A 3 x 3 convolution of few channels whose input wants no gradient: both gradients come from one kernel.
+  bool first_layer(const at::Tensor& xs, const at::Tensor& dy, const at::Tensor& a) {
+    const std::vector<int64_t> one{1, 1};
+    return a.is_cuda() && !task_should_compute_output(0) && task_should_compute_output(1) && !c10::GradMode::is_enabled() &&
+           groups == 1 && weight.size(2) == 3 && weight.size(3) == 3 && stride == one && padding == one && dilation == one &&
+           xs.scalar_type() == at::kBFloat16 && xs.is_contiguous(at::MemoryFormat::ChannelsLast) &&
+           a.is_contiguous(at::MemoryFormat::ChannelsLast) && (uintptr_t)dy.data_ptr() % 16 == 0 &&
+           (uintptr_t)a.data_ptr() % 16 == 0 &&
+           model_ops::first_conv_backward_supported(a.size(0), a.size(2), a.size(3), a.size(1), xs.size(1));
+  }
+  void first_layer_backward(const at::Tensor& xs, const at::Tensor& dy, const at::Tensor& a, bool alone, variable_list& out) {
+    const int C = (int)a.size(1), Ci = (int)xs.size(1);
+    const bool want_b = task_should_compute_output(2);
+    const bool add_b = alone && want_b && accumulates(bias, dy);
+    const bool add_w = alone && weight.is_contiguous(at::MemoryFormat::ChannelsLast) && accumulates(weight, dy);
+    const auto f = a.options().dtype(at::kFloat);
+    at::Tensor db = add_b ? bias.grad() : want_b ? at::empty({C}, f) : at::Tensor();
+    at::Tensor dw = add_w ? weight.grad() : at::empty(weight.sizes(), f, at::MemoryFormat::ChannelsLast);
+    auto scratch = scratch_for(a, model_ops::first_conv_backward_scratch_bytes(a.numel() / C, C, Ci));
+    model_ops::first_conv_backward(dy.data_ptr(), a.data_ptr(), xs.data_ptr(), dw.data_ptr<float>(), add_w,
+                                   db.defined() ? db.data_ptr<float>() : nullptr, add_b, a.size(0), a.size(2), a.size(3), C, Ci,
+                                   scratch->data_ptr(), stream_of(a));
+    count_launches(2);
+    if (!add_w) out[1] = dw;
+    if (want_b && !add_b) out[2] = db;
   }
 
   void backward_tail(const at::Tensor& dy, const at::Tensor& a, at::Tensor& dz, at::Tensor& db, bool add) {

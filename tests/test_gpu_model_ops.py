@@ -7,6 +7,12 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
+def bb_launches():
+    import bagua_core_b200 as bb
+
+    return bb._C.op_stats()["launches"]
+
+
 def _stream():
     return torch.cuda.current_stream().cuda_stream
 
@@ -424,6 +430,41 @@ def test_block_gradients_added_in_place_have_the_bits_of_the_ordinary_path():
         W.enabled = saved
     for a, b in zip(*grads):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("N,H,W,Ci,C", [(1, 1, 1, 3, 64), (1, 1, 63, 1, 64), (2, 13, 5, 2, 128), (1, 8, 8, 3, 64), (3, 65, 1, 3, 256),
+                                        (2, 61, 67, 3, 64), (8, 112, 112, 3, 64)])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_first_layer_gradients_match_fp32_math(N, H, W, Ci, C, in_place):
+    """No gradient for the input: the block's weight and bias gradients come from one kernel."""
+    from bagua_core_b200.ops import wgrad as Wg
+    from bagua_core_b200.ops.fused_conv import ConvBiasReLU
+
+    torch.manual_seed(N * H + W)
+    m = ConvBiasReLU(Ci, C, 3, padding=1).cuda().to(memory_format=torch.channels_last if in_place or N > 1 else torch.contiguous_format)
+    torch.nn.init.normal_(m.bias, 0.0, 0.1)
+    for p in m.parameters():
+        p.grad = torch.ones_like(p)
+    x = torch.randn(N, Ci, H, W, device="cuda").to(memory_format=torch.channels_last)
+    saved = Wg.enabled
+    Wg.enabled = in_place
+    try:
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = m(x)
+        dy = torch.randn(y.shape, device="cuda").to(torch.bfloat16).to(memory_format=torch.channels_last)
+        mid = bb_launches()
+        y.backward(dy)
+    finally:
+        Wg.enabled = saved
+    assert bb_launches() - mid == 2
+    dz = torch.where(y > 0, dy, torch.zeros_like(dy)).detach().double()
+    patches = torch.nn.functional.unfold(x.bfloat16().double(), 3, padding=1)  # [N, Ci * 9, H * W]
+    dw = torch.einsum("ncp,nkp->ck", dz.reshape(N, C, H * W), patches).view(C, Ci, 3, 3)
+    db = dz.sum((0, 2, 3))
+    assert (m.bias.grad.double() - (1 + db)).abs().max() <= 1e-5 * db.abs().max()
+    # rounded to bf16, and the patches' order of summation moves a few values to their neighbours
+    got, want = m.weight.grad.double() - 1, dw
+    assert ((got - want).abs() <= 4.1e-3 * want.abs() + 1e-5 * want.abs().max()).all()
 
 
 @pytest.mark.parametrize("rows,H", [(1, 8), (5, 264), (37, 768), (3072, 1024)])
