@@ -151,7 +151,10 @@ __global__ void __launch_bounds__(kThreads)
 
 // x += y, y in bf16: 10 bytes per element where a cast to fp32 and an addition move 18.
 __global__ void __launch_bounds__(kThreads)
-    accumulate_bf16_kernel(float* __restrict__ x, const __nv_bfloat16* __restrict__ y, int64_t n, bool vec) {
+    accumulate_bf16_kernel(float* __restrict__ x0, const __nv_bfloat16* __restrict__ y0, float* __restrict__ x1,
+                           const __nv_bfloat16* __restrict__ y1, int64_t n, bool vec) {
+  float* x = blockIdx.y == 0 ? x0 : x1;
+  const __nv_bfloat16* y = blockIdx.y == 0 ? y0 : y1;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   wait_for_predecessor();
@@ -351,7 +354,12 @@ void async_model_average(float* t, const float* r, const float* cp, float nranks
 void accumulate_bf16(float* x, const void* y, int64_t n, cudaStream_t s) {
   const bool vec = ((uintptr_t)x % 16 == 0) && ((uintptr_t)y % 8 == 0);
   launch_overlapped(accumulate_bf16_kernel, dim3(grid_for(vec ? n / 4 + 1 : n)), dim3(kThreads), s, x,
-                    (const __nv_bfloat16*)y, n, vec);
+                    (const __nv_bfloat16*)y, (float*)nullptr, (const __nv_bfloat16*)nullptr, n, vec);
+}
+void accumulate_bf16_pair(float* x0, const void* y0, float* x1, const void* y1, int64_t n, cudaStream_t s) {
+  const bool vec = (((uintptr_t)x0 | (uintptr_t)x1) % 16 == 0) && (((uintptr_t)y0 | (uintptr_t)y1) % 8 == 0);
+  launch_overlapped(accumulate_bf16_kernel, dim3(grid_for(vec ? n / 4 + 1 : n), 2), dim3(kThreads), s, x0,
+                    (const __nv_bfloat16*)y0, x1, (const __nv_bfloat16*)y1, n, vec);
 }
 void cast_bf16(const CastSegment* segs, int n, cudaStream_t s) {
   for (int at = 0; at < n; at += kCastSegments) {

@@ -47,6 +47,8 @@ namespace cuda {
 void cast_bf16(const CastSegment* segs, int n, cudaStream_t s);
 // x[i] += y[i] with x in fp32 and y in bf16: a low-precision gradient into its fp32 accumulator, in one pass.
 void accumulate_bf16(float* x, const void* y, int64_t n, cudaStream_t s);
+// two of one size in one launch: a normalisation's scale and shift
+void accumulate_bf16_pair(float* x0, const void* y0, float* x1, const void* y1, int64_t n, cudaStream_t s);
 }  // namespace cuda
 
 // Flatten (gather = true: tensors -> flat) or unflatten (flat -> tensors) a list of tensors in

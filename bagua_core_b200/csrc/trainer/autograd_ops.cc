@@ -1,6 +1,7 @@
 #include "autograd_ops.h"
 
 #include <ATen/autocast_mode.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
@@ -40,6 +41,17 @@ kernels::Ctx ctx_of(const at::Tensor& t) {
   return kernels::Ctx{t.is_cuda() ? (int)t.device().index() : -1, stream_of(t)};
 }
 void count_launches(int n) { OpStats::global().launches += n; }
+
+// A contiguous tensor on `like`'s device.  Straight from the allocator: a step of a medium model makes a hundred, and
+// the dispatcher costs as much as the allocation.
+at::Tensor fresh(at::IntArrayRef sizes, at::ScalarType type, const at::Tensor& like) {
+  if (like.is_cuda()) return at::detail::empty_cuda(sizes, type, like.device(), c10::nullopt);
+  return at::empty(sizes, like.options().dtype(type));
+}
+at::Tensor fresh_like(const at::Tensor& t) {
+  if (t.is_cuda() && t.is_contiguous()) return fresh(t.sizes(), t.scalar_type(), t);
+  return at::empty_like(t);
+}
 
 // ---- uses of a weight in a graph ---------------------------------------------------------------
 // Where a weight takes part in a graph more than once, autograd adds the uses' gradients first and
@@ -107,7 +119,7 @@ bool gemm_into(at::Tensor grad, const at::Tensor& a, const at::Tensor& b) {
     return true;
   }
   if (!aligned) {
-    at::Tensor apart = at::empty(grad.sizes(), grad.options());
+    at::Tensor apart = fresh(grad.sizes(), grad.scalar_type(), grad);
     if (gemm::weight_grad(dy, b, apart, false)) {
       mode = mode == 0 ? 1 : mode.load();
       kernels::add_inplace(grad.data_ptr(), apart.data_ptr(), DType::F32, grad.numel(), ctx_of(grad));
@@ -155,7 +167,7 @@ void to_bf16(std::array<at::Tensor, N>& ts) {
       t = t.to(at::kBFloat16);
       continue;
     }
-    at::Tensor low = at::empty_strided(t.sizes(), t.strides(), t.options().dtype(at::kBFloat16));
+    at::Tensor low = at::detail::empty_strided_cuda(t.sizes(), t.strides(), at::kBFloat16, t.device());
     segs[n++] = kernels::CastSegment{(const float*)t.data_ptr(), low.data_ptr(), t.numel()};
     // the source stays alive as the caller's tensor until the launch below
     t = low;
@@ -211,7 +223,7 @@ struct LinearNode : public Node {
     if (task_should_compute_output(0)) {
       at::Tensor dx;
       if (!c10::GradMode::is_enabled()) {
-        dx = at::empty({dy2.size(0), ws.size(1)}, dy2.options());
+        dx = fresh({dy2.size(0), ws.size(1)}, dy2.scalar_type(), dy2);
         if (!gemm::input_grad(dy2, ws, dx)) dx = at::Tensor();
       }
       if (!dx.defined()) dx = at::mm(dy2, ws);
@@ -241,8 +253,8 @@ struct LinearNode : public Node {
     const int C = (int)dy2.size(1);
     const bool want = bias.defined() && task_should_compute_output(2);
     const bool add = want && accumulate && use && !use->shared && accumulates(bias, dy2);
-    at::Tensor db = add ? bias.grad() : at::empty({C}, dy2.options().dtype(at::kFloat));
-    at::Tensor dz = at::empty_like(dy2);
+    at::Tensor db = add ? bias.grad() : fresh({C}, at::kFloat, dy2);
+    at::Tensor dz = fresh_like(dy2);
     const size_t bytes = encoder_ops::activation_backward_scratch_bytes(rows, C);
     std::shared_ptr<PoolRawTensor> scratch = bytes ? scratch_for(dy2, bytes) : nullptr;
     encoder_ops::activation_backward(activation == kGelu, dy2.data_ptr(), zs.data_ptr(), dz.data_ptr(), db.data_ptr<float>(),
@@ -258,7 +270,7 @@ struct LinearNode : public Node {
         !model_ops::column_sum_supported(rows, (int)C) || !dy2.is_contiguous() || (uintptr_t)dy2.data_ptr() % 16 != 0)
       return dy2.sum(at::IntArrayRef{0}, /*keepdim=*/false, at::kFloat);
     const bool add = accumulate && use && !use->shared && accumulates(bias, dy2);
-    at::Tensor db = add ? bias.grad() : at::empty({C}, dy2.options().dtype(at::kFloat));
+    at::Tensor db = add ? bias.grad() : fresh({C}, at::kFloat, dy2);
     const size_t bytes = model_ops::column_sum_scratch_bytes(rows, (int)C);
     std::shared_ptr<PoolRawTensor> scratch = bytes ? scratch_for(dy2, bytes) : nullptr;
     model_ops::column_sum_bf16(dy2.data_ptr(), db.data_ptr<float>(), rows, (int)C, scratch ? scratch->data_ptr() : nullptr,
@@ -303,7 +315,7 @@ struct ConvNode : public Node {
     at::Tensor dz = at::empty_like(a);
     // the bias gradient is added to `.grad` by the fold of its partial sums
     const bool add_bias = alone && dy.is_cuda() && task_should_compute_output(2) && accumulates(bias, dy);
-    at::Tensor db = add_bias ? bias.grad() : at::empty({C}, a.options().dtype(at::kFloat));
+    at::Tensor db = add_bias ? bias.grad() : fresh({C}, at::kFloat, a);
     backward_tail(dy, a, dz, db, add_bias);
     if (task_should_compute_output(2) && !add_bias) out[2] = db;
     const bool need_x = task_should_compute_output(0), need_w = task_should_compute_output(1);
@@ -427,8 +439,16 @@ struct LayerNormNode : public Node {
                                                   {true, task_should_compute_output(2), task_should_compute_output(3)});
     out[0] = std::get<0>(d);
     if (residual) out[1] = out[0];
-    give(gamma, std::get<1>(d), accumulate, out[2]);
-    give(beta, std::get<2>(d), accumulate, out[3]);
+    const at::Tensor &dg = std::get<1>(d), &db = std::get<2>(d);
+    if (accumulate && dg.defined() && db.defined() && accumulates(gamma, dg) && accumulates(beta, db) &&
+        gamma.grad().is_contiguous() && beta.grad().is_contiguous()) {
+      kernels::cuda::accumulate_bf16_pair(gamma.grad().data_ptr<float>(), dg.data_ptr(), beta.grad().data_ptr<float>(),
+                                          db.data_ptr(), dg.numel(), stream_of(s));
+      count_launches(1);
+      return out;
+    }
+    give(gamma, dg, accumulate, out[2]);
+    give(beta, db, accumulate, out[3]);
     return out;
   }
 };
@@ -480,7 +500,7 @@ struct SpanLossNode : public Node {
     variable_list out(1);
     if (!grads[0].defined()) return out;
     const at::Tensor x = logits.unpack(), a = start.unpack(), b = end.unpack(), st = stats.unpack();
-    at::Tensor dx = at::empty_like(x);
+    at::Tensor dx = fresh_like(x);
     encoder_ops::span_loss_backward(x.data_ptr(), a.data_ptr<int64_t>(), b.data_ptr<int64_t>(), st.data_ptr<float>(),
                                     grads[0].data_ptr<float>(), dx.data_ptr(), x.size(0), x.size(1), stream_of(x));
     count_launches(1);
@@ -539,7 +559,7 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& weight, const std::opti
     if (xs.is_cuda() && xs.is_contiguous() && xs.numel() > 0 && xs.dim() >= 2) {
       std::vector<int64_t> shape(xs.sizes().begin(), xs.sizes().end());
       shape.back() = ws.size(0);
-      y = at::empty(shape, xs.options());
+      y = fresh(shape, xs.scalar_type(), xs);
       at::Tensor y2 = y.dim() == 2 ? y : y.view({-1, ws.size(0)});
       if (!gemm::linear(xs.dim() == 2 ? xs : xs.view({-1, xs.size(-1)}), ws, low[2], activation == kRelu, y2)) y = at::Tensor();
     }
@@ -550,7 +570,7 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& weight, const std::opti
       y = y.contiguous();
     } else if (activation == kGelu) {
       z = y.contiguous();
-      y = at::empty_like(z);
+      y = fresh_like(z);
       encoder_ops::gelu_forward(z.data_ptr(), y.data_ptr(), z.numel(), stream_of(z));
       count_launches(1);
     }
@@ -690,7 +710,7 @@ at::Tensor embed_layer_norm(const at::Tensor& ids, const at::Tensor& tok, const 
     PlainDispatch plain;
     idc = ids.contiguous();
     const int64_t batch = ids.size(0), seq = ids.size(1);
-    sum = at::empty({batch, seq, H}, tok.options());
+    sum = fresh({batch, seq, H}, at::kFloat, tok);
     encoder_ops::embed_sum(idc.data_ptr<int64_t>(), tok.size(0), tok.data_ptr<float>(), pos.data_ptr<float>(),
                            typ.data_ptr<float>(), sum.data_ptr<float>(), batch, seq, (int)H, stream_of(tok));
     count_launches(1);
@@ -730,9 +750,8 @@ at::Tensor span_loss(const at::Tensor& logits, const at::Tensor& start, const at
     if ((uintptr_t)x.data_ptr() % 4 != 0) x = x.clone();
     a = start.contiguous();
     b = end.contiguous();
-    const auto f = x.options().dtype(at::kFloat);
-    loss = at::empty({}, f);
-    stats = at::empty({2 * B + 2}, f);
+    loss = fresh({}, at::kFloat, x);
+    stats = fresh({2 * B + 2}, at::kFloat, x);
     encoder_ops::span_loss_forward(x.data_ptr(), a.data_ptr<int64_t>(), b.data_ptr<int64_t>(), loss.data_ptr<float>(),
                                    stats.data_ptr<float>(), B, x.size(1), stream_of(x));
     count_launches(1);
