@@ -2,15 +2,17 @@
 // the ReLU's output; see model_ops.h.
 //
 // Nobody wants the gradient of the network's input, so the convolution's output gradient dz is needed for these two
-// sums alone, and is never written.  The weight gradient is the product [C x pixels] [pixels x 9 Ci], the bias gradient one more column of it (ones): a block walks
-// tiles of 64 pixels, masks dy with the activation into shared memory, gathers the pixels' 3 x 3 patches (at most
-// 27 values, 32 with zeros) next to it, and adds tile by tile with m16n8k16 products in fp32 registers.  The two
-// reads of [pixels, 64] are what bounds it: with 27 columns per 64 channels the product needs a hundredth of the
-// matrix rate, so mma.sync, which takes its operands from registers, is enough and leaves no accumulator to move.
-// The loads of the next tile are in flight during the products of this one.
+// sums alone, and is never written.  The weight gradient is the product [C x pixels] [pixels x 9 Ci], the bias gradient
+// one more column of it (ones): a block walks tiles of 64 pixels, masks dy with the activation into shared memory,
+// gathers the pixels' 3 x 3 patches (at most 27 values and the one, 32 with zeros) next to it, and adds tile by tile
+// with m16n8k16 products in fp32 registers.  The two reads of [pixels, C] bound it from below: with 32 columns per 64
+// channels the product needs a hundredth of the matrix rate, so mma.sync, which takes its operands from registers,
+// is enough and leaves no accumulator to move.  The loads of the next tile are in flight during the products of this
+// one; three blocks per SM, because four leave 64 registers per thread and spill.
 //
-// 32 x 224 x 224, 3 -> 64 channels (411 MB): mask and bias sums 96 us, padding of the channels and the library's
-// product 165 us, the fold, the cast and their gaps 20 us before; FIRSTNOW.
+// 32 x 224 x 224, 3 -> 64 channels (411 MB, 63 us at the copy rate): mask and bias sums 96 us, padding of the
+// channels and the library's product 165 us, fold, cast, fills and gaps 20 us before; 83 us and 5 us for the fold
+// now (98 us with a division per pixel and the bias sums in registers).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 

@@ -41,9 +41,20 @@ inline uint64_t globaltimer_ns() {
   return (uint64_t)ts.tv_sec * 1000000000ull + (uint64_t)ts.tv_nsec;
 }
 inline void st_release_sys(uint32_t* p, uint32_t v) { __atomic_store_n(p, v, __ATOMIC_RELEASE); }
-inline uint32_t ld_acquire_sys(const uint32_t* p) { return __atomic_load_n(p, __ATOMIC_ACQUIRE); }
+// Hundreds of threads share a few cores: one that polls lets the others run, or what it waits for takes time slices.
+inline void let_others_run() {
+  static thread_local unsigned polls = 0;
+  if ((++polls & 15u) == 0) sched_yield();
+}
+inline uint32_t ld_acquire_sys(const uint32_t* p) {
+  let_others_run();
+  return __atomic_load_n(p, __ATOMIC_ACQUIRE);
+}
 inline uint32_t ld_relaxed_gpu(const uint32_t* p) { return __atomic_load_n(p, __ATOMIC_RELAXED); }
-inline uint64_t ld_acquire_gpu_u64(const unsigned long long* p) { return __atomic_load_n(p, __ATOMIC_ACQUIRE); }
+inline uint64_t ld_acquire_gpu_u64(const unsigned long long* p) {
+  let_others_run();
+  return __atomic_load_n(p, __ATOMIC_ACQUIRE);
+}
 #else
 __device__ __forceinline__ uint64_t globaltimer_ns() {
   uint64_t t;
