@@ -111,10 +111,13 @@ bool gemm_into(at::Tensor grad, const at::Tensor& a, const at::Tensor& b) {
   auto& mode = OpStats::global().gemm_mode;
   // A gradient that does not start on 16 bytes (it follows a tensor of odd size in its bucket) costs the library
   // its fast kernels: 82 us instead of 22 for 3072 x 1024 x 3072.  The product then goes to a buffer of its own and
-  // is added from there.
+  // is added from there, unless so few rows are summed that the second pass over the result costs more than the
+  // slow kernel: device time apart / direct for 4096 x 4096 from 32, 128, 512 rows 76/54, 80/64, 95/118 us, for
+  // 1024 x 1024 17.5/14.4, 17.5/16.4, 18.4/20.5 us, and a launch less.
+  constexpr int64_t kFewRows = 256;
   const bool aligned = (uintptr_t)grad.data_ptr() % 16 == 0;
   const at::Tensor dy = a.t();
-  if (aligned && gemm::weight_grad(dy, b, grad, true)) {
+  if ((aligned || dy.size(0) <= kFewRows) && gemm::weight_grad(dy, b, grad, true)) {
     mode = 1;
     return true;
   }

@@ -535,6 +535,26 @@ def test_linear_with_activation_matches_the_plain_composition(rows, n_out, accum
         assert (got.float() - want).abs().max() <= 1e-2 * want.abs().max()
 
 
+@pytest.mark.parametrize("rows", [1, 256, 257])
+@pytest.mark.parametrize("n_out,n_in", [(10, 72), (136, 64)])
+def test_weight_gradient_of_any_alignment_is_accumulated(rows, n_out, n_in):
+    import bagua_core_b200 as bb
+
+    torch.manual_seed(rows)
+    x = torch.randn(rows, n_in, device="cuda").bfloat16()
+    w = torch.randn(n_out, n_in, device="cuda", requires_grad=True)
+    for offset in (0, 1, 2):
+        flat = torch.ones(n_out * n_in + 8, device="cuda")
+        w.grad = flat[offset:offset + n_out * n_in].view(n_out, n_in)
+        y = bb._C.linear(x, w, None, None, True)
+        dy = torch.randn_like(y)
+        y.backward(dy)
+        want = 1 + dy.float().t() @ x.float()
+        assert w.grad.data_ptr() == flat.data_ptr() + 4 * offset
+        assert (w.grad - want).abs().max() <= 1e-4 * want.abs().max()
+        assert (flat[:offset] == 1).all() and (flat[offset + n_out * n_in:] == 1).all()
+
+
 @pytest.mark.parametrize("batch,seq", [(1, 1), (3, 7), (8, 384), (40, 33)])
 def test_span_loss_matches_two_cross_entropies(batch, seq):
     import bagua_core_b200 as bb
