@@ -29,6 +29,7 @@ void SgdPlan::add(const at::Tensor& p, const at::Tensor& g, const at::Tensor& m,
   a.first = true;
   segs_.push_back(a);
   group_.push_back(group);
+  grad_buffer_.push_back(g.storage().data());
   keep_.insert(keep_.end(), {p, g, m});
   if (shadow) keep_.push_back(*shadow);
 }
@@ -59,10 +60,13 @@ int SgdPlan::step(const std::vector<SgdGroup>& groups, uint64_t stream) {
 
 void SgdPlan::zero_grad(uint64_t stream) {
   for (size_t k = 0; k < segs_.size();) {
-    // slices of one buffer follow each other: one memset over all of them
+    // slices of one buffer follow each other: one memset over all of them (never over two buffers, which may lie next
+    // to each other in separate allocations)
     char* from = (char*)segs_[k].g;
+    const void* buffer = grad_buffer_[k];
     size_t bytes = 0;
-    for (; k < segs_.size() && (char*)segs_[k].g == from + bytes; ++k) bytes += (size_t)segs_[k].n * sizeof(float);
+    for (; k < segs_.size() && grad_buffer_[k] == buffer && (char*)segs_[k].g == from + bytes; ++k)
+      bytes += (size_t)segs_[k].n * sizeof(float);
     if (bytes == 0) continue;
     if (device_ >= 0)
       BAGUA_CUDA_CHECK(cudaMemsetAsync(from, 0, bytes, (cudaStream_t)stream));

@@ -33,6 +33,7 @@ class SgdPlan {
   int device_ = -1;
   std::vector<kernels::SgdSegment> segs_;
   std::vector<int> group_;
+  std::vector<const void*> grad_buffer_;  // of each segment: the storage its gradient lies in
   std::vector<at::Tensor> keep_;
 };
 
