@@ -130,6 +130,8 @@ class MLP(nn.Module):
         layers = []
         for i in range(depth):
             layers.append(ShadowLinear(dims[i], dims[i + 1]))
+            # the gradients of `nn.Linear`, bit for bit: so small a network repeats its steps exactly
+            layers[-1].accumulate_in_place = False
             if i < depth - 1:
                 layers.append(nn.ReLU())
         self.net = nn.Sequential(*layers)

@@ -26,6 +26,9 @@ _ACTIVATIONS = {"gelu": (1, F.gelu), "relu": (2, F.relu)}
 
 
 class ShadowLinear(nn.Linear):
+    # False: the weight gradient goes through autograd, rounded to bf16 as `nn.Linear`'s, whatever `wgrad.enabled` says
+    accumulate_in_place = True
+
     def forward(self, x: torch.Tensor, activation: str = "") -> torch.Tensor:
         """`activation` ("gelu", "relu"): applied to the result, in the same autograd function where the layer runs
         natively."""
@@ -39,7 +42,8 @@ class ShadowLinear(nn.Linear):
                 act = None
             else:
                 code = 0
-            y = _C.linear(x, self.weight, self.bias, _shadow.autocast_copy(self.weight), _wgrad.enabled, code)
+            y = _C.linear(x, self.weight, self.bias, _shadow.autocast_copy(self.weight),
+                          _wgrad.enabled and self.accumulate_in_place, code)
         else:
             y = super().forward(x)
         return y if act is None else act(y)
