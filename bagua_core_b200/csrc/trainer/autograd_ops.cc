@@ -102,6 +102,9 @@ bool accumulates(const at::Tensor& param, const at::Tensor& like) {
          torch::autograd::impl::hooks(param).empty();
 }
 
+// A bias of C values, one per column: any other shape that broadcasts is left to autograd, which folds its gradient.
+bool per_column(const at::Tensor& bias, int64_t C) { return bias.dim() == 1 && bias.size(0) == C; }
+
 // grad += aᵀ-shaped product a b of bf16 operands, accumulated in fp32.  False: not available, nothing changed.
 bool gemm_into(at::Tensor grad, const at::Tensor& a, const at::Tensor& b) {
   if (!grad.is_cuda()) {  // host: no mixed-precision GEMM; widen the operands
@@ -159,14 +162,16 @@ struct PlainDispatch {
   c10::impl::ExcludeDispatchKeyGuard no_autocast{c10::autocast_dispatch_keyset};
 };
 
-// Rounds tensors to bf16, those that are fp32 on a GPU in one launch together.  Undefined ones stay undefined.
+// Rounds tensors to bf16, those that are fp32 on the first one's GPU in one launch together.  Undefined ones stay
+// undefined.
 template <size_t N>
 void to_bf16(std::array<at::Tensor, N>& ts) {
   kernels::CastSegment segs[N];
   int n = 0;
+  const at::Device device = ts[0].device();
   for (at::Tensor& t : ts) {
     if (!t.defined() || t.scalar_type() == at::kBFloat16) continue;
-    if (!t.is_cuda() || t.scalar_type() != at::kFloat || !t.is_non_overlapping_and_dense()) {
+    if (!t.is_cuda() || t.device() != device || t.scalar_type() != at::kFloat || !t.is_non_overlapping_and_dense()) {
       t = t.to(at::kBFloat16);
       continue;
     }
@@ -176,11 +181,7 @@ void to_bf16(std::array<at::Tensor, N>& ts) {
     t = low;
   }
   if (n) {
-    for (const at::Tensor& t : ts)
-      if (t.defined() && t.is_cuda()) {
-        kernels::cuda::cast_bf16(segs, n, stream_of(t));
-        break;
-      }
+    kernels::cuda::cast_bf16(segs, n, stream_of(ts[0]));
     count_launches(1);
   }
 }
@@ -255,7 +256,7 @@ struct LinearNode : public Node {
     const int64_t rows = dy2.size(0);
     const int C = (int)dy2.size(1);
     const bool want = bias.defined() && task_should_compute_output(2);
-    const bool add = want && accumulate && use && !use->shared && accumulates(bias, dy2);
+    const bool add = want && accumulate && use && !use->shared && per_column(bias, C) && accumulates(bias, dy2);
     at::Tensor db = add ? bias.grad() : fresh({C}, at::kFloat, dy2);
     at::Tensor dz = fresh_like(dy2);
     const size_t bytes = encoder_ops::activation_backward_scratch_bytes(rows, C);
@@ -272,7 +273,7 @@ struct LinearNode : public Node {
     if (!dy2.is_cuda() || c10::GradMode::is_enabled() || dy2.scalar_type() != at::kBFloat16 || C > (1 << 24) ||
         !model_ops::column_sum_supported(rows, (int)C) || !dy2.is_contiguous() || (uintptr_t)dy2.data_ptr() % 16 != 0)
       return dy2.sum(at::IntArrayRef{0}, /*keepdim=*/false, at::kFloat);
-    const bool add = accumulate && use && !use->shared && accumulates(bias, dy2);
+    const bool add = accumulate && use && !use->shared && per_column(bias, C) && accumulates(bias, dy2);
     at::Tensor db = add ? bias.grad() : fresh({C}, at::kFloat, dy2);
     const size_t bytes = model_ops::column_sum_scratch_bytes(rows, (int)C);
     std::shared_ptr<PoolRawTensor> scratch = bytes ? scratch_for(dy2, bytes) : nullptr;
@@ -619,6 +620,8 @@ at::Tensor conv_bias_relu(const at::Tensor& x, const at::Tensor& weight, const a
     const int C = (int)z.size(1);
     BAGUA_CHECK(z.scalar_type() == at::kBFloat16 && bs.scalar_type() == at::kBFloat16, Tensor,
                 "fused convolution blocks compute in bf16");
+    BAGUA_CHECK(bs.dim() == 1 && bs.size(0) == C && bs.device() == z.device(), Tensor,
+                "a convolution of " << C << " channels needs as many bias values on its device");
     if (pool) {
       out = at::empty({N, C, H / 2, W / 2}, z.options().memory_format(at::MemoryFormat::ChannelsLast));
       if (z.is_cuda())
@@ -701,6 +704,9 @@ at::Tensor embed_layer_norm(const at::Tensor& ids, const at::Tensor& tok, const 
               Tensor, "embed_layer_norm: unsupported ids");
   for (const at::Tensor* p : {&tok, &pos, &typ, &gamma, &beta})
     BAGUA_CHECK(fp32_param(*p, H, ids), Tensor, "embed_layer_norm needs fp32 tables on the ids' device");
+  BAGUA_CHECK(tok.dim() == 2 && pos.dim() == 2 && typ.dim() == 2 && tok.size(0) > 0 && typ.size(0) > 0 && gamma.dim() == 1 &&
+                  beta.dim() == 1,
+              Tensor, "embed_layer_norm needs tables with rows and parameters of one row");
   BAGUA_CHECK(ids.size(1) <= pos.size(0), Tensor, "sequence of " << ids.size(1) << " tokens, " << pos.size(0) << " positions");
   std::shared_ptr<EmbedNode> node;
   if (torch::autograd::compute_requires_grad(tok, pos, typ, gamma, beta)) {
@@ -770,7 +776,7 @@ at::Tensor span_loss(const at::Tensor& logits, const at::Tensor& start, const at
 }
 
 at::Tensor attention(const at::Tensor& qkv, int64_t heads, double dropout) {
-  BAGUA_CHECK(qkv.is_cuda() && qkv.dim() == 3 && qkv.scalar_type() == at::kBFloat16 && qkv.size(2) % (3 * heads * 8) == 0,
+  BAGUA_CHECK(heads > 0 && qkv.is_cuda() && qkv.dim() == 3 && qkv.scalar_type() == at::kBFloat16 && qkv.size(2) % (3 * heads * 8) == 0,
               Tensor, "attention needs a packed bf16 projection [batch, seq, 3 * heads * dim] with dim a multiple of 8");
   const int64_t B = qkv.size(0), S = qkv.size(1), W = qkv.size(2), D = W / (3 * heads);
   variable_list parts;

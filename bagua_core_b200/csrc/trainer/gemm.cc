@@ -149,13 +149,20 @@ bool run(int kind, const Problem& q, int64_t m, int64_t n, int64_t k, const at::
 bool plain(const at::Tensor& t) {
   return t.is_cuda() && t.dim() == 2 && t.scalar_type() == at::kBFloat16 && t.is_contiguous() && t.numel() > 0;
 }
+// The library is given addresses and sizes only: what does not fit together is refused here, and the framework's
+// product says why.
+bool sized(const at::Tensor& t, int64_t rows, int64_t cols, const at::Tensor& like) {
+  return t.size(0) == rows && t.size(1) == cols && t.device() == like.device();
+}
 
 }  // namespace
 
 bool linear(const at::Tensor& x, const at::Tensor& w, const at::Tensor& b, bool relu, at::Tensor& y) {
-  if (!plain(x) || !plain(w) || !plain(y) || (b.defined() && (b.scalar_type() != at::kBFloat16 || !b.is_contiguous())))
-    return false;
+  if (!plain(x) || !plain(w) || !plain(y)) return false;
   const int64_t M = x.size(0), K = x.size(1), N = w.size(0);
+  if (!sized(w, N, K, x) || !sized(y, M, N, x)) return false;
+  if (b.defined() && (b.scalar_type() != at::kBFloat16 || !b.is_contiguous() || b.dim() != 1 || b.size(0) != N || b.device() != x.device()))
+    return false;
   const Problem q{CUBLAS_OP_T, CUBLAS_OP_N, K, N, K, M, N, M, false, b.defined(), true, relu};
   return run(0, q, M, N, K, w, x, y, b.defined() ? b.data_ptr() : nullptr, false);
 }
@@ -163,6 +170,7 @@ bool linear(const at::Tensor& x, const at::Tensor& w, const at::Tensor& b, bool 
 bool input_grad(const at::Tensor& dy, const at::Tensor& w, at::Tensor& dx) {
   if (!plain(dy) || !plain(w) || !plain(dx)) return false;
   const int64_t M = dy.size(0), N = dy.size(1), K = w.size(1);
+  if (!sized(w, N, K, dy) || !sized(dx, M, K, dy)) return false;
   const Problem q{CUBLAS_OP_N, CUBLAS_OP_N, K, N, N, M, K, M, false, false, false, false};
   return run(1, q, M, N, K, w, dy, dx, nullptr, false);
 }
@@ -170,6 +178,7 @@ bool input_grad(const at::Tensor& dy, const at::Tensor& w, at::Tensor& dx) {
 bool weight_grad(const at::Tensor& dy, const at::Tensor& x, at::Tensor& g, bool accumulate) {
   if (!plain(dy) || !plain(x) || g.scalar_type() != at::kFloat || !g.is_contiguous() || g.dim() != 2) return false;
   const int64_t M = dy.size(0), N = dy.size(1), K = x.size(1);
+  if (!sized(x, M, K, dy) || !sized(g, N, K, dy)) return false;
   const Problem q{CUBLAS_OP_N, CUBLAS_OP_T, K, M, N, M, K, N, true, false, false, false};
   return run(2, q, M, N, K, x, dy, g, nullptr, accumulate);
 }

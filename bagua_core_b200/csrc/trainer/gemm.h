@@ -12,7 +12,8 @@ namespace bagua {
 namespace trainer {
 namespace gemm {
 
-// All operands are 2-D, bf16, contiguous and on one CUDA device; false: not available for these, nothing was done.
+// All operands are 2-D, bf16, contiguous, of the sizes given here and on one CUDA device; false: not available for these,
+// nothing was done.
 
 // y [M, N] = x [M, K] w [N, K]ᵀ + b [N] (b may be undefined), at least 0 with `relu`
 bool linear(const at::Tensor& x, const at::Tensor& w, const at::Tensor& b, bool relu, at::Tensor& y);

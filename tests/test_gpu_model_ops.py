@@ -597,3 +597,44 @@ def test_bert_layers_through_the_fused_kernels_agree_with_the_plain_composition(
     for loss, grad in out[1:]:
         assert abs(loss - out[0][0]) < 2e-2
         assert (grad - out[0][1]).norm() <= 4e-2 * out[0][1].norm()
+
+
+@pytest.mark.parametrize("width", [32, 128, 0])
+@pytest.mark.parametrize("activation", ["", "relu", "gelu"])
+def test_a_linear_layer_refuses_an_input_of_another_width(width, activation):
+    """The products behind the layer are given addresses and sizes only: a wrong width must be refused before them."""
+    from bagua_core_b200.ops import wgrad as W
+    from bagua_core_b200.ops.fused_linear import ShadowLinear
+
+    m, saved = ShadowLinear(64, 24).cuda(), W.enabled
+    W.enabled = True
+    try:
+        for shape in ((5, width), (2, 5, width)):
+            with torch.autocast("cuda", dtype=torch.bfloat16), pytest.raises(RuntimeError):
+                m(torch.ones(shape, device="cuda", requires_grad=True), activation)
+            with torch.autocast("cuda", dtype=torch.bfloat16), pytest.raises(RuntimeError):
+                m(torch.ones(shape[:-1] + (64,)), activation)  # on the host
+    finally:
+        W.enabled = saved
+
+
+def test_a_bias_that_is_not_one_value_per_column_takes_the_general_path():
+    import bagua_core_b200 as bb
+    from bagua_core_b200.ops.fused_conv import ConvBiasReLU
+
+    x, w = torch.randn(6, 16, device="cuda").bfloat16(), torch.randn(24, 16, device="cuda")
+    for n in (23, 25):
+        with pytest.raises(RuntimeError):
+            bb._C.linear(x, w, torch.zeros(n, device="cuda"), None, False)
+    flat = torch.zeros(64, device="cuda")  # one value for all columns, its gradient in front of others
+    b = torch.ones(1, device="cuda", requires_grad=True)
+    b.grad = flat[:1]
+    w.requires_grad_().grad = torch.zeros_like(w)
+    for activation in (0, 2):
+        y = bb._C.linear(x, w, b, None, True, activation)
+        y.sum().backward()
+    assert bool((flat[1:] == 0).all()) and flat[0] == 6 * 24 + (y > 0).sum()
+    m = ConvBiasReLU(16, 64, 3, padding=1).cuda().to(memory_format=torch.channels_last)
+    m.bias = torch.nn.Parameter(torch.zeros(32, device="cuda"))
+    with torch.autocast("cuda", dtype=torch.bfloat16), pytest.raises(RuntimeError, match="bias"):
+        m(torch.zeros(1, 16, 8, 8, device="cuda"))
