@@ -53,6 +53,10 @@ at::Tensor fresh_like(const at::Tensor& t) {
   return at::empty_like(t);
 }
 
+// A gradient comes from whoever used the result, and may be a view that starts anywhere: these kernels, and the library's
+// attention, read 16 bytes at a time without asking.
+at::Tensor vector_aligned(const at::Tensor& t) { return (uintptr_t)t.data_ptr() % 16 == 0 ? t : t.clone(); }
+
 // ---- uses of a weight in a graph ---------------------------------------------------------------
 // Where a weight takes part in a graph more than once, autograd adds the uses' gradients first and
 // accumulates once; accumulating each use by itself would round differently, so both uses of such a
@@ -222,7 +226,7 @@ struct LinearNode : public Node {
     if (!grads[0].defined()) return out;
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
     const at::Tensor dy = grads[0], xs = x.unpack(), ws = w.unpack();
-    at::Tensor dy2 = dy.dim() == 2 ? dy : dy.reshape({-1, dy.size(-1)});
+    at::Tensor dy2 = vector_aligned(dy.dim() == 2 ? dy : dy.reshape({-1, dy.size(-1)}));
     if (activation) dy2 = through_activation(dy2.contiguous(), out);
     if (task_should_compute_output(0)) {
       at::Tensor dx;
@@ -309,7 +313,7 @@ struct ConvNode : public Node {
     if (!grads[0].defined()) return out;
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
     const at::Tensor xs = x.unpack(), ws = w.unpack(), a = act.unpack(pool ? std::shared_ptr<Node>() : shared_from_this());
-    const at::Tensor dy = grads[0].contiguous(at::MemoryFormat::ChannelsLast);
+    const at::Tensor dy = vector_aligned(grads[0].contiguous(at::MemoryFormat::ChannelsLast));
     const bool alone = accumulate && use && !use->shared;
     const int C = (int)ws.size(0);
     if (!pool && first_layer(xs, dy, a)) {
@@ -529,7 +533,7 @@ struct SplitHeadsNode : public Node {
       at::Tensor g = grads[(size_t)q].defined() ? grads[(size_t)q] : at::zeros({batch, heads, seq, dim}, options);
       const bool direct = g.stride(3) == 1 && g.stride(0) % 8 == 0 && g.stride(1) % 8 == 0 && g.stride(2) % 8 == 0 &&
                           (uintptr_t)g.data_ptr() % 16 == 0;
-      keep[q] = direct ? g : g.contiguous();
+      keep[q] = direct ? g : vector_aligned(g.contiguous());
       src[q] = keep[q].data_ptr();
       st[q] = encoder_ops::HeadStrides{keep[q].stride(0), keep[q].stride(1), keep[q].stride(2)};
     }
@@ -787,7 +791,7 @@ at::Tensor attention(const at::Tensor& qkv, int64_t heads, double dropout) {
   }
   {
     PlainDispatch plain;
-    const at::Tensor c = qkv.contiguous();
+    const at::Tensor c = vector_aligned(qkv.contiguous());
     for (int64_t q = 0; q < 3; ++q)
       parts.push_back(c.detach().as_strided({B, heads, S, D}, {S * W, D, W, 1}, c.storage_offset() + q * heads * D));
   }
@@ -800,6 +804,7 @@ at::Tensor attention(const at::Tensor& qkv, int64_t heads, double dropout) {
     for (at::Tensor& t : parts) torch::autograd::set_history(t, node);
   }
   const at::Tensor a = at::scaled_dot_product_attention(parts[0], parts[1], parts[2], c10::nullopt, dropout);
+  if (node) a.register_hook([](const at::Tensor& g) { return vector_aligned(g); });
   return a.transpose(1, 2).reshape({B, S, heads * D});
 }
 

@@ -638,3 +638,30 @@ def test_a_bias_that_is_not_one_value_per_column_takes_the_general_path():
     m.bias = torch.nn.Parameter(torch.zeros(32, device="cuda"))
     with torch.autocast("cuda", dtype=torch.bfloat16), pytest.raises(RuntimeError, match="bias"):
         m(torch.zeros(1, 16, 8, 8, device="cuda"))
+
+
+@pytest.mark.parametrize("offset", [1, 4, 8])
+def test_gradients_that_start_anywhere_give_those_of_an_aligned_copy(offset):
+    import bagua_core_b200 as bb
+    from bagua_core_b200.ops.fused_conv import ConvBiasReLU, ConvBiasReLUPool
+
+    def shifted(t):  # the same values in the same strides, `offset` elements behind an aligned address
+        buf = torch.empty(t.numel() + offset, dtype=t.dtype, device=t.device)
+        return torch.as_strided(buf, t.shape, t.stride(), offset).copy_(t)
+
+    torch.manual_seed(offset)
+    layers = []
+    w = torch.randn(40, 16, device="cuda")
+    for activation in (0, 1, 2):
+        layers.append((lambda x, a=activation: bb._C.linear(x, w, None, None, False, a), torch.randn(70, 16, device="cuda").bfloat16()))
+    layers.append((lambda x: bb._C.attention(x, 2, 0.0), torch.randn(2, 16, 96, device="cuda").bfloat16()))
+    for cls in (ConvBiasReLU, ConvBiasReLUPool):
+        m = cls(16, 64, 3, padding=1).cuda().to(dtype=torch.bfloat16, memory_format=torch.channels_last)
+        layers.append((m, torch.randn(2, 16, 8, 8, device="cuda").bfloat16().contiguous(memory_format=torch.channels_last)))
+    for f, x in layers:
+        x.requires_grad_()
+        y = f(x)
+        dy = torch.randn(y.shape, device="cuda").bfloat16().as_strided(y.shape, y.stride())
+        a, b = (torch.autograd.grad(f(x), x, g)[0] for g in (dy, shifted(dy)))
+        # (the library's attention adds parts of its gradients in any order)
+        assert torch.equal(a, b) or (x.dim() == 3 and torch.allclose(a.float(), b.float(), rtol=1e-2, atol=1e-3))
