@@ -1,6 +1,7 @@
 #include "autograd_ops.h"
 
 #include <ATen/autocast_mode.h>
+#include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/function.h>
@@ -201,8 +202,26 @@ std::shared_ptr<PoolRawTensor> scratch_for(const at::Tensor& t, size_t bytes) {
   return PoolRawTensor::allocate((int)t.device().index(), DType::U8, (int64_t)bytes, (uint64_t)(uintptr_t)stream_of(t));
 }
 
+// A node that may add parameters' gradients to their `.grad` itself.
+struct AccumulatingNode : public Node {
+ protected:
+  // Has been done for input `i`.  Autograd orders the stream that a parameter's gradient is finished on (that of its
+  // accumulation node, on which its hooks run) behind the stream that made it when it hands the gradient over.  It is
+  // handed nothing here, so the order is made here; the streams differ when a model is trained on another stream than the
+  // one it was wrapped on.
+  void added(uint32_t i, const at::Tensor& on) const {
+    if (!on.is_cuda() || !next_edge(i).is_valid()) return;
+    const auto to = next_edge(i).function->stream();
+    const auto from = c10::cuda::getCurrentCUDAStream(on.device().index());
+    if (!to || *to == from.unwrap()) return;
+    at::cuda::CUDAEvent done;
+    done.record(from);
+    done.block(c10::cuda::CUDAStream(*to));
+  }
+};
+
 // ---- linear ------------------------------------------------------------------------------------
-struct LinearNode : public Node {
+struct LinearNode : public AccumulatingNode {
   SavedVariable x, w, z;  // z: what gelu was applied to, or the ReLU's result
   at::Tensor weight, bias;  // the parameters (bias may be undefined)
   std::shared_ptr<Use> use;  // set when gradients are to be accumulated here
@@ -244,6 +263,7 @@ struct LinearNode : public Node {
         if (use && !use->shared && accumulates(weight, dy2) && weight.grad().is_contiguous()) {
           c10::NoGradGuard no_grad;
           done = gemm_into(weight.grad(), dy2.t(), x2);
+          if (done) added(1, dy2);
         }
         auto& stats = OpStats::global();
         done ? ++stats.accumulated : ++stats.declined;
@@ -268,6 +288,7 @@ struct LinearNode : public Node {
     encoder_ops::activation_backward(activation == kGelu, dy2.data_ptr(), zs.data_ptr(), dz.data_ptr(), db.data_ptr<float>(),
                                      add, scratch ? scratch->data_ptr() : nullptr, rows, C, stream_of(dy2));
     count_launches(bytes ? 2 : 1);
+    if (add) added(2, dy2);
     if (want && !add) out[2] = db;
     return dz;
   }
@@ -284,12 +305,13 @@ struct LinearNode : public Node {
     model_ops::column_sum_bf16(dy2.data_ptr(), db.data_ptr<float>(), rows, (int)C, scratch ? scratch->data_ptr() : nullptr,
                                stream_of(dy2), add);
     count_launches(bytes ? 2 : 1);
+    if (add) added(2, dy2);
     return add ? at::Tensor() : db;
   }
 };
 
 // ---- convolution + bias + ReLU (+ pooling) -------------------------------------------------------
-struct ConvNode : public Node {
+struct ConvNode : public AccumulatingNode {
   SavedVariable x, w, b, act;  // act: the activation, or with pooling the convolution's output
   at::Tensor weight, bias;
   std::vector<int64_t> stride, padding, dilation;
@@ -325,6 +347,7 @@ struct ConvNode : public Node {
     const bool add_bias = alone && dy.is_cuda() && task_should_compute_output(2) && accumulates(bias, dy);
     at::Tensor db = add_bias ? bias.grad() : fresh({C}, at::kFloat, a);
     backward_tail(dy, a, dz, db, add_bias);
+    if (add_bias) added(2, dy);
     if (task_should_compute_output(2) && !add_bias) out[2] = db;
     const bool need_x = task_should_compute_output(0), need_w = task_should_compute_output(1);
     if (need_x || need_w) {
@@ -343,6 +366,7 @@ struct ConvNode : public Node {
           c10::NoGradGuard no_grad;
           weight.grad().add_(dw);
         }
+        added(1, dw);
       } else {
         out[1] = dw;
       }
@@ -373,8 +397,14 @@ struct ConvNode : public Node {
                                    db.defined() ? db.data_ptr<float>() : nullptr, add_b, a.size(0), a.size(2), a.size(3), C, Ci,
                                    scratch->data_ptr(), stream_of(a));
     count_launches(2);
-    if (!add_w) out[1] = dw;
-    if (want_b && !add_b) out[2] = db;
+    if (add_w)
+      added(1, a);
+    else
+      out[1] = dw;
+    if (add_b)
+      added(2, a);
+    else if (want_b)
+      out[2] = db;
   }
 
   void backward_tail(const at::Tensor& dy, const at::Tensor& a, at::Tensor& dz, at::Tensor& db, bool add) {
@@ -413,24 +443,30 @@ GradTarget grad_target(const at::Tensor& param, bool accumulate) {
   return {at::zeros(param.sizes(), param.options()), false};
 }
 
-// Adds a gradient to its place, or leaves it to autograd.
-void give(const at::Tensor& param, const at::Tensor& g, bool accumulate, at::Tensor& out) {
-  if (!g.defined()) return;
-  if (!accumulate || !accumulates(param, param) || !param.grad().is_contiguous()) {
-    out = g;  // autograd casts it to the parameter's type
-    return;
-  }
-  if (g.scalar_type() == at::kBFloat16)
-    kernels::cuda::accumulate_bf16((float*)param.grad().data_ptr(), g.data_ptr(), g.numel(), stream_of(g));
-  else
-    kernels::add_inplace(param.grad().data_ptr(), g.data_ptr(), DType::F32, g.numel(), ctx_of(g));
-  count_launches(1);
-}
+struct EncoderNode : public AccumulatingNode {
+  bool accumulate = false;
 
-struct LayerNormNode : public Node {
+ protected:
+  // Adds the gradient of input `i` to its place, or leaves it to autograd.
+  void give(uint32_t i, const at::Tensor& param, const at::Tensor& g, variable_list& out) const {
+    if (!g.defined()) return;
+    if (!accumulate || !accumulates(param, param) || !param.grad().is_contiguous()) {
+      out[i] = g;  // autograd casts it to the parameter's type
+      return;
+    }
+    if (g.scalar_type() == at::kBFloat16)
+      kernels::cuda::accumulate_bf16((float*)param.grad().data_ptr(), g.data_ptr(), g.numel(), stream_of(g));
+    else
+      kernels::add_inplace(param.grad().data_ptr(), g.data_ptr(), DType::F32, g.numel(), ctx_of(g));
+    count_launches(1);
+    added(i, g);
+  }
+};
+
+struct LayerNormNode : public EncoderNode {
   SavedVariable sum, mean, rstd, g, b;  // g, b: the parameters in bf16
   at::Tensor gamma, beta;
-  bool accumulate = false, residual = false;
+  bool residual = false;
 
   std::string name() const override { return "BaguaAddLayerNormBackward"; }
   void release_variables() override {
@@ -453,18 +489,19 @@ struct LayerNormNode : public Node {
       kernels::cuda::accumulate_bf16_pair(gamma.grad().data_ptr<float>(), dg.data_ptr(), beta.grad().data_ptr<float>(),
                                           db.data_ptr(), dg.numel(), stream_of(s));
       count_launches(1);
+      added(2, s);
+      added(3, s);
       return out;
     }
-    give(gamma, dg, accumulate, out[2]);
-    give(beta, db, accumulate, out[3]);
+    give(2, gamma, dg, out);
+    give(3, beta, db, out);
     return out;
   }
 };
 
-struct EmbedNode : public Node {
+struct EmbedNode : public EncoderNode {
   SavedVariable ids, sum, mean, rstd;
   at::Tensor param[5];  // tok, pos, typ, gamma, beta
-  bool accumulate = false;
 
   std::string name() const override { return "BaguaEmbedLayerNormBackward"; }
   void release_variables() override {
@@ -480,8 +517,8 @@ struct EmbedNode : public Node {
     const int64_t batch = id.size(0), seq = id.size(1);
     const auto d = at::native_layer_norm_backward(grads[0].to(at::kFloat).contiguous(), s, {H}, mean.unpack(), rstd.unpack(),
                                                   param[3], param[4], {true, true, true});
-    give(param[3], std::get<1>(d), accumulate, out[3]);
-    give(param[4], std::get<2>(d), accumulate, out[4]);
+    give(3, param[3], std::get<1>(d), out);
+    give(4, param[4], std::get<2>(d), out);
     GradTarget to[3];
     for (int k = 0; k < 3; ++k) to[k] = grad_target(param[k], accumulate && task_should_compute_output((size_t)k));
     auto scratch = scratch_for(s, encoder_ops::embed_backward_scratch_bytes(batch * seq, H));
@@ -489,8 +526,12 @@ struct EmbedNode : public Node {
                                 to[0].grad.data_ptr<float>(), to[1].grad.data_ptr<float>(), to[2].grad.data_ptr<float>(),
                                 scratch->data_ptr(), batch, seq, H, stream_of(s));
     count_launches(3);
-    for (int k = 0; k < 3; ++k)
-      if (!to[k].add) out[(size_t)k] = to[k].grad;
+    for (uint32_t k = 0; k < 3; ++k) {
+      if (to[k].add)
+        added(k, s);
+      else
+        out[k] = to[k].grad;
+    }
     return out;
   }
 };

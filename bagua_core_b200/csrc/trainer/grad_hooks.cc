@@ -5,6 +5,8 @@
 #include <torch/csrc/autograd/utils/lambda_post_hook.h>
 #include <torch/csrc/autograd/variable.h>
 
+#include <algorithm>
+
 namespace bagua {
 namespace trainer {
 
@@ -53,7 +55,10 @@ void GradHooks::remove() {
 
 void GradHooks::arm() {
   for (auto& e : entries_) e.marked = false;
-  for (auto& b : buckets_) b.pending = b.size;
+  for (auto& b : buckets_) {
+    b.pending = b.size;
+    b.streams.clear();
+  }
 }
 
 void GradHooks::flush() {
@@ -99,10 +104,21 @@ void GradHooks::mark(Entry& e) {
   Bucket& b = buckets_[(size_t)e.bucket];
   e.marked = true;
   uint64_t event = 0;
-  if (--b.pending == 0 && device_ >= 0) {
-    if (!b.event) BAGUA_CUDA_CHECK(cudaEventCreateWithFlags(&b.event, cudaEventDisableTiming));
-    BAGUA_CUDA_CHECK(cudaEventRecord(b.event, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device_).stream()));
-    event = (uint64_t)(uintptr_t)b.event;
+  --b.pending;
+  if (device_ >= 0) {
+    const cudaStream_t now = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device_).stream();
+    if (std::find(b.streams.begin(), b.streams.end(), now) == b.streams.end()) b.streams.push_back(now);
+    if (b.pending == 0) {
+      if (!b.event) BAGUA_CUDA_CHECK(cudaEventCreateWithFlags(&b.event, cudaEventDisableTiming));
+      // gradients that were finished on other streams than the last one: the event stands for them too
+      for (cudaStream_t s : b.streams)
+        if (s != now) {
+          BAGUA_CUDA_CHECK(cudaEventRecord(b.event, s));
+          BAGUA_CUDA_CHECK(cudaStreamWaitEvent(now, b.event, 0));
+        }
+      BAGUA_CUDA_CHECK(cudaEventRecord(b.event, now));
+      event = (uint64_t)(uintptr_t)b.event;
+    }
   }
   backend->mark_communication_ready(e.tensor, event);
 }

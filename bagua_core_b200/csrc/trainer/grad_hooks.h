@@ -3,7 +3,7 @@
 //
 // One hook per parameter sits behind the node that accumulates its gradient.  It keeps the bucket's
 // countdown, records the bucket's CUDA event with its last gradient (earlier ones are covered by it, being
-// on the same stream), and moves a gradient that was replaced from outside back into the bucket.  A Python
+// on the same stream or joined to it), and moves a gradient that was replaced from outside back into the bucket.  A Python
 // hook with the same duties cost 6-8 us per parameter and step, and the GIL.
 #pragma once
 
@@ -50,6 +50,7 @@ class GradHooks : public std::enable_shared_from_this<GradHooks> {
   struct Bucket {
     int size = 0, pending = 0;
     cudaEvent_t event = nullptr;
+    std::vector<cudaStream_t> streams;  // on which gradients were finished since arm(): nearly always one
   };
   void on_gradient(size_t i);
   void mark(Entry& e);

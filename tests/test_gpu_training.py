@@ -85,3 +85,57 @@ def test_bert_trains_with_a_bf16_residual_stream():
         assert all(torch.isfinite(torch.tensor(run)))
         losses.append(run)
     assert all(abs(a - b) < 5e-2 for a, b in zip(*losses)), losses
+
+
+@pytest.mark.parametrize("early_graph", [False, True])
+def test_training_on_a_side_stream_equals_training_on_the_default_stream(early_graph):
+    """A model wrapped on the default stream, trained on a stream that lags behind the host: the buckets wait for gradients
+    that were added to them there.  `early_graph`: a graph from before the wrapping keeps one layer's accumulation nodes
+    on a third stream."""
+    import os
+
+    import bagua_core_b200.parallel as P
+    from bagua_core_b200.ops import wgrad as W
+    from bagua_core_b200.ops.fused_conv import ConvBiasReLU, ConvBiasReLUPool
+    from bagua_core_b200.ops.fused_linear import ShadowLinear
+
+    os.environ.setdefault("MASTER_ADDR", "127.0.0.1")
+    os.environ.setdefault("MASTER_PORT", "29549")
+    dev = torch.device("cuda", 0)
+    saved, results = W.enabled, []
+    W.enabled = True
+    try:
+        for side in (False, True):
+            torch.manual_seed(0)
+            conv = torch.nn.Sequential(ConvBiasReLU(3, 64, 3, padding=1), ConvBiasReLUPool(64, 64, 3, padding=1), torch.nn.Flatten())
+            head = torch.nn.Sequential(ShadowLinear(64 * 16, 64), torch.nn.ReLU(), ShadowLinear(64, 16))
+            net = torch.nn.Sequential(conv, head).to(dev).to(memory_format=torch.channels_last)
+            third = torch.cuda.Stream()
+            with torch.cuda.stream(third):
+                keep = head[0](torch.zeros(1, 64 * 16, device=dev)) if early_graph else None
+            third.synchronize()
+            P.init_process_group(dev)
+            opt = P.FlatSGD(net.parameters(), lr=0.05, momentum=0.9)
+            bm = P.with_bagua(net, [opt], P.ByteGradAlgorithm(), bucket_bytes=64 << 10)
+            x = torch.randn(8, 3, 8, 8, device=dev).contiguous(memory_format=torch.channels_last)
+            stream = torch.cuda.Stream() if side else torch.cuda.current_stream()
+            stream.wait_stream(torch.cuda.current_stream())
+            grads = []
+            with torch.cuda.stream(stream):
+                for _ in range(3):
+                    opt.zero_grad()
+                    torch.cuda._sleep(20_000_000)  # about 10 ms: the host is done with the step before the GPU begins it
+                    with torch.autocast("cuda", dtype=torch.bfloat16):
+                        loss = bm(x).float().square().sum()
+                    loss.backward()
+                    grads.append([b.flattened.clone() for b in bm.bagua_buckets])
+                    opt.step()
+            torch.cuda.synchronize()
+            results.append((grads, [p.detach().clone() for p in net.parameters()]))
+            P.destroy_process_group()
+            del keep
+    finally:
+        W.enabled = saved
+    (ga, wa), (gb, wb) = results
+    for a, b in zip(sum(ga, []) + wa, sum(gb, []) + wb):
+        assert torch.equal(a, b)
