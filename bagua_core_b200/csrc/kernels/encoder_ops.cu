@@ -90,7 +90,7 @@ int column_slices(int64_t rows, int H) {
 // L2); the first of every kMaxOrdered occurrences adds up that many rows, in order.  Blocks of the first
 // sequence also add up their position over the batch.  The framework's path writes a dense gradient of the
 // whole table (zero fill, scatter, addition: about 240 us for 30522 x 1024 and 3072 tokens); this touches the
-// rows that occur.
+// rows that occur.  Either table may be missing (null): its gradient is not wanted.
 __global__ void __launch_bounds__(kThreads)
     embed_scatter_kernel(const int64_t* __restrict__ ids, int64_t vocab, const float* __restrict__ ds, float* __restrict__ dtok,
                          float* __restrict__ dpos, int64_t batch, int64_t seq, int H) {
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(kThreads)
   __shared__ int s_warp[kWarps];
   wait_for_predecessor();
   const int T = (int)(batch * seq), i = (int)blockIdx.x, tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (i < seq) {
+  if (dpos && i < seq) {
     for (int c = tid; c < H; c += kThreads) {
       float s = 0.f;
 #pragma unroll 4
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kThreads)
     }
   }
   const int64_t id = ids[i];
-  if (id < 0 || id >= vocab) return;
+  if (!dtok || id < 0 || id >= vocab) return;
   int before = 0;
   for (int j = tid; j < i; j += kThreads) before += ids[j] == id;
   // exact rank of this occurrence, when it is not the first
@@ -346,15 +346,24 @@ void embed_sum(const int64_t* ids, int64_t vocab, const float* tok, const float*
 }
 
 size_t embed_backward_scratch_bytes(int64_t rows, int H) { return (size_t)column_slices(rows, H) * H * sizeof(float); }
-void embed_backward(const float* dx, const int64_t* ids, int64_t vocab, float* dtok, float* dpos, float* dtyp, void* scratch,
-                    int64_t batch, int64_t seq, int H, cudaStream_t s) {
+int embed_backward(const float* dx, const int64_t* ids, int64_t vocab, float* dtok, float* dpos, float* dtyp, void* scratch,
+                   int64_t batch, int64_t seq, int H, cudaStream_t s) {
   const int64_t rows = batch * seq;
   BAGUA_CHECK(rows > 0 && rows <= kMaxTokens, Tensor, "embedding backward: " << rows << " tokens");
-  const int slices = column_slices(rows, H);
-  launch_overlapped(column_sum_f32_kernel, dim3((H + kThreads - 1) / kThreads, slices), dim3(kThreads), s, dx, (float*)scratch,
-                    rows, H);
-  fold((const float*)scratch, dtyp, slices, H, true, s);
-  launch_overlapped(embed_scatter_kernel, dim3((unsigned)rows), dim3(kThreads), s, ids, vocab, dx, dtok, dpos, batch, seq, H);
+  int launches = 0;
+  if (dtyp) {
+    const int slices = column_slices(rows, H);
+    launch_overlapped(column_sum_f32_kernel, dim3((H + kThreads - 1) / kThreads, slices), dim3(kThreads), s, dx, (float*)scratch,
+                      rows, H);
+    fold((const float*)scratch, dtyp, slices, H, true, s);
+    launches += 2;
+  }
+  if (dtok || dpos) {
+    launch_overlapped(embed_scatter_kernel, dim3((unsigned)(dtok ? rows : seq)), dim3(kThreads), s, ids, vocab, dx, dtok, dpos,
+                      batch, seq, H);
+    ++launches;
+  }
+  return launches;
 }
 
 void gelu_forward(const void* z, void* y, int64_t n, cudaStream_t s) {

@@ -21,12 +21,13 @@ namespace encoder_ops {
 // gradient.
 void embed_sum(const int64_t* ids, int64_t vocab, const float* tok, const float* pos, const float* typ, float* x, int64_t batch,
                int64_t seq, int H, cudaStream_t s);
-// The tables' gradients from dx [batch * seq, H], ADDED to dtok [vocab, H], dpos [>= seq, H] and dtyp [H].  Rows of one token
-// are summed in order up to kMaxOrdered occurrences; beyond that, slices of that length are added atomically.
+// The tables' gradients from dx [batch * seq, H], ADDED to dtok [vocab, H], dpos [>= seq, H] and dtyp [H], each of which
+// may be null.  Rows of one token are summed in order up to kMaxOrdered occurrences; beyond that, slices of that length are
+// added atomically.  Returns the number of kernels launched.
 constexpr int kMaxTokens = 4096, kMaxOrdered = 256;
 size_t embed_backward_scratch_bytes(int64_t rows, int H);
-void embed_backward(const float* dx, const int64_t* ids, int64_t vocab, float* dtok, float* dpos, float* dtyp, void* scratch,
-                    int64_t batch, int64_t seq, int H, cudaStream_t s);
+int embed_backward(const float* dx, const int64_t* ids, int64_t vocab, float* dtok, float* dpos, float* dtyp, void* scratch,
+                   int64_t batch, int64_t seq, int H, cudaStream_t s);
 
 // y = gelu(z) (exact).  Backward of an activation: dz = dy * gelu'(z), or dy where the ReLU's result `z` is positive, and
 // its column sums, in one pass.  [rows, C] bf16, C % 8 == 0.

@@ -436,7 +436,7 @@ struct ConvNode : public AccumulatingNode {
 // An fp32 gradient for `param`: its `.grad` to be added to, or zeros for autograd.
 struct GradTarget {
   at::Tensor grad;
-  bool add;
+  bool add = false;
 };
 GradTarget grad_target(const at::Tensor& param, bool accumulate) {
   if (accumulate && accumulates(param, param) && param.grad().is_contiguous()) return {param.grad(), true};
@@ -515,18 +515,26 @@ struct EmbedNode : public EncoderNode {
     const at::Tensor id = ids.unpack(), s = sum.unpack();
     const int H = (int)param[0].size(1);
     const int64_t batch = id.size(0), seq = id.size(1);
+    // only what is asked for: a frozen parameter has a gradient in its bucket all the same, which stays as it is
+    bool want[5];
+    for (uint32_t k = 0; k < 5; ++k) want[k] = task_should_compute_output(k);
     const auto d = at::native_layer_norm_backward(grads[0].to(at::kFloat).contiguous(), s, {H}, mean.unpack(), rstd.unpack(),
-                                                  param[3], param[4], {true, true, true});
+                                                  param[3], param[4], {want[0] || want[1] || want[2], want[3], want[4]});
     give(3, param[3], std::get<1>(d), out);
     give(4, param[4], std::get<2>(d), out);
+    if (!want[0] && !want[1] && !want[2]) return out;
     GradTarget to[3];
-    for (int k = 0; k < 3; ++k) to[k] = grad_target(param[k], accumulate && task_should_compute_output((size_t)k));
+    float* grad[3] = {nullptr, nullptr, nullptr};
+    for (int k = 0; k < 3; ++k) {
+      if (!want[k]) continue;
+      to[k] = grad_target(param[k], accumulate);
+      grad[k] = to[k].grad.data_ptr<float>();
+    }
     auto scratch = scratch_for(s, encoder_ops::embed_backward_scratch_bytes(batch * seq, H));
-    encoder_ops::embed_backward(std::get<0>(d).data_ptr<float>(), id.data_ptr<int64_t>(), param[0].size(0),
-                                to[0].grad.data_ptr<float>(), to[1].grad.data_ptr<float>(), to[2].grad.data_ptr<float>(),
-                                scratch->data_ptr(), batch, seq, H, stream_of(s));
-    count_launches(3);
+    count_launches(encoder_ops::embed_backward(std::get<0>(d).data_ptr<float>(), id.data_ptr<int64_t>(), param[0].size(0), grad[0],
+                                               grad[1], grad[2], scratch->data_ptr(), batch, seq, H, stream_of(s)));
     for (uint32_t k = 0; k < 3; ++k) {
+      if (!want[k]) continue;
       if (to[k].add)
         added(k, s);
       else

@@ -665,3 +665,27 @@ def test_gradients_that_start_anywhere_give_those_of_an_aligned_copy(offset):
         a, b = (torch.autograd.grad(f(x), x, g)[0] for g in (dy, shifted(dy)))
         # (the library's attention adds parts of its gradients in any order)
         assert torch.equal(a, b) or (x.dim() == 3 and torch.allclose(a.float(), b.float(), rtol=1e-2, atol=1e-3))
+
+
+@pytest.mark.parametrize("frozen", [(0,), (1,), (2,), (3,), (4,), (0, 1, 2), (0, 2, 3, 4), (3, 4)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_a_frozen_parameter_of_the_embedding_keeps_its_gradient(frozen, accumulate):
+    """It may be frozen after its bucket was laid out: `.grad` is there, and must not be added to."""
+    import bagua_core_b200 as bb
+
+    g = torch.Generator().manual_seed(1)
+    ids = torch.randint(0, 50, (3, 70), generator=g).cuda()
+    grads = []
+    for off in ((), frozen):
+        torch.manual_seed(0)
+        ps = [torch.randn(*s, device="cuda", requires_grad=True) for s in ((50, 72), (80, 72), (2, 72), (72,), (72,))]
+        for k, p in enumerate(ps):
+            p.grad = torch.ones_like(p)
+            p.requires_grad_(k not in off)
+        y = bb._C.embed_layer_norm(ids, *ps, 1e-12, accumulate)
+        torch.manual_seed(2)
+        y.backward(torch.randn(y.shape, device="cuda").bfloat16())
+        grads.append([p.grad for p in ps])
+    for k, (a, b) in enumerate(zip(*grads)):
+        assert not torch.equal(a, torch.ones_like(a))
+        assert torch.equal(b, torch.ones_like(a) if k in frozen else a), k
