@@ -204,7 +204,29 @@ std::shared_ptr<PoolRawTensor> scratch_for(const at::Tensor& t, size_t bytes) {
 
 // A node that may add parameters' gradients to their `.grad` itself.
 struct AccumulatingNode : public Node {
+  // For a new node: every parameter that wants a gradient is counted as used.
+  void accumulate_gradients(std::initializer_list<const at::Tensor*> params) {
+    accumulate = true;
+    size_t n = 0;
+    for (const at::Tensor* p : params)
+      if (p->defined() && p->requires_grad()) uses_[n++] = begin_use(*p);
+  }
+
  protected:
+  bool accumulate = false;
+
+  void uses_done() {
+    for (auto& u : uses_)
+      if (u) u->done = true;
+  }
+  // Whether gradients may be added here, as far as that depends on the node: it was asked to, and none of its parameters
+  // takes part in the graph elsewhere.
+  bool adds() const {
+    if (!accumulate) return false;
+    for (auto& u : uses_)
+      if (u && u->shared) return false;
+    return true;
+  }
   // Has been done for input `i`.  Autograd orders the stream that a parameter's gradient is finished on (that of its
   // accumulation node, on which its hooks run) behind the stream that made it when it hands the gradient over.  It is
   // handed nothing here, so the order is made here; the streams differ when a model is trained on another stream than the
@@ -218,14 +240,15 @@ struct AccumulatingNode : public Node {
     done.record(from);
     done.block(c10::cuda::CUDAStream(*to));
   }
+
+ private:
+  std::array<std::shared_ptr<Use>, 5> uses_;
 };
 
 // ---- linear ------------------------------------------------------------------------------------
 struct LinearNode : public AccumulatingNode {
   SavedVariable x, w, z;  // z: what gelu was applied to, or the ReLU's result
   at::Tensor weight, bias;  // the parameters (bias may be undefined)
-  std::shared_ptr<Use> use;  // set when gradients are to be accumulated here
-  bool accumulate = false;
   int activation = kNone;
 
   std::string name() const override {
@@ -241,7 +264,7 @@ struct LinearNode : public AccumulatingNode {
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
     variable_list out(3);
-    if (use) use->done = true;
+    uses_done();
     if (!grads[0].defined()) return out;
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
     const at::Tensor dy = grads[0], xs = x.unpack(), ws = w.unpack();
@@ -260,7 +283,7 @@ struct LinearNode : public AccumulatingNode {
       const at::Tensor x2 = xs.dim() == 2 ? xs : xs.reshape({-1, xs.size(-1)});
       bool done = false;
       if (accumulate) {
-        if (use && !use->shared && accumulates(weight, dy2) && weight.grad().is_contiguous()) {
+        if (adds() && accumulates(weight, dy2) && weight.grad().is_contiguous()) {
           c10::NoGradGuard no_grad;
           done = gemm_into(weight.grad(), dy2.t(), x2);
           if (done) added(1, dy2);
@@ -280,7 +303,7 @@ struct LinearNode : public AccumulatingNode {
     const int64_t rows = dy2.size(0);
     const int C = (int)dy2.size(1);
     const bool want = bias.defined() && task_should_compute_output(2);
-    const bool add = want && accumulate && use && !use->shared && per_column(bias, C) && accumulates(bias, dy2);
+    const bool add = want && adds() && per_column(bias, C) && accumulates(bias, dy2);
     at::Tensor db = add ? bias.grad() : fresh({C}, at::kFloat, dy2);
     at::Tensor dz = fresh_like(dy2);
     const size_t bytes = encoder_ops::activation_backward_scratch_bytes(rows, C);
@@ -298,7 +321,7 @@ struct LinearNode : public AccumulatingNode {
     if (!dy2.is_cuda() || c10::GradMode::is_enabled() || dy2.scalar_type() != at::kBFloat16 || C > (1 << 24) ||
         !model_ops::column_sum_supported(rows, (int)C) || !dy2.is_contiguous() || (uintptr_t)dy2.data_ptr() % 16 != 0)
       return dy2.sum(at::IntArrayRef{0}, /*keepdim=*/false, at::kFloat);
-    const bool add = accumulate && use && !use->shared && per_column(bias, C) && accumulates(bias, dy2);
+    const bool add = adds() && per_column(bias, C) && accumulates(bias, dy2);
     at::Tensor db = add ? bias.grad() : fresh({C}, at::kFloat, dy2);
     const size_t bytes = model_ops::column_sum_scratch_bytes(rows, (int)C);
     std::shared_ptr<PoolRawTensor> scratch = bytes ? scratch_for(dy2, bytes) : nullptr;
@@ -316,8 +339,7 @@ struct ConvNode : public AccumulatingNode {
   at::Tensor weight, bias;
   std::vector<int64_t> stride, padding, dilation;
   int64_t groups = 1;
-  bool pool = false, accumulate = false;
-  std::shared_ptr<Use> use;
+  bool pool = false;
 
   std::string name() const override { return pool ? "BaguaConvBiasReLUPoolBackward" : "BaguaConvBiasReLUBackward"; }
   void release_variables() override {
@@ -331,12 +353,12 @@ struct ConvNode : public AccumulatingNode {
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
     variable_list out(3);
-    if (use) use->done = true;
+    uses_done();
     if (!grads[0].defined()) return out;
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
     const at::Tensor xs = x.unpack(), ws = w.unpack(), a = act.unpack(pool ? std::shared_ptr<Node>() : shared_from_this());
     const at::Tensor dy = vector_aligned(grads[0].contiguous(at::MemoryFormat::ChannelsLast));
-    const bool alone = accumulate && use && !use->shared;
+    const bool alone = adds();
     const int C = (int)ws.size(0);
     if (!pool && first_layer(xs, dy, a)) {
       first_layer_backward(xs, dy, a, alone, out);
@@ -444,13 +466,11 @@ GradTarget grad_target(const at::Tensor& param, bool accumulate) {
 }
 
 struct EncoderNode : public AccumulatingNode {
-  bool accumulate = false;
-
  protected:
   // Adds the gradient of input `i` to its place, or leaves it to autograd.
   void give(uint32_t i, const at::Tensor& param, const at::Tensor& g, variable_list& out) const {
     if (!g.defined()) return;
-    if (!accumulate || !accumulates(param, param) || !param.grad().is_contiguous()) {
+    if (!adds() || !accumulates(param, param) || !param.grad().is_contiguous()) {
       out[i] = g;  // autograd casts it to the parameter's type
       return;
     }
@@ -476,6 +496,7 @@ struct LayerNormNode : public EncoderNode {
   variable_list apply(variable_list&& grads) override {  // x, r, gamma, beta
     std::lock_guard<std::mutex> lock(mutex_);
     variable_list out(4);
+    uses_done();
     if (!grads[0].defined()) return out;
     const at::Tensor s = sum.unpack();
     const auto d = at::native_layer_norm_backward(grads[0].contiguous(), s, {s.size(-1)}, mean.unpack(), rstd.unpack(),
@@ -484,7 +505,7 @@ struct LayerNormNode : public EncoderNode {
     out[0] = std::get<0>(d);
     if (residual) out[1] = out[0];
     const at::Tensor &dg = std::get<1>(d), &db = std::get<2>(d);
-    if (accumulate && dg.defined() && db.defined() && accumulates(gamma, dg) && accumulates(beta, db) &&
+    if (adds() && dg.defined() && db.defined() && accumulates(gamma, dg) && accumulates(beta, db) &&
         gamma.grad().is_contiguous() && beta.grad().is_contiguous()) {
       kernels::cuda::accumulate_bf16_pair(gamma.grad().data_ptr<float>(), dg.data_ptr(), beta.grad().data_ptr<float>(),
                                           db.data_ptr(), dg.numel(), stream_of(s));
@@ -511,6 +532,7 @@ struct EmbedNode : public EncoderNode {
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
     variable_list out(5);
+    uses_done();
     if (!grads[0].defined()) return out;
     const at::Tensor id = ids.unpack(), s = sum.unpack();
     const int H = (int)param[0].size(1);
@@ -527,7 +549,7 @@ struct EmbedNode : public EncoderNode {
     float* grad[3] = {nullptr, nullptr, nullptr};
     for (int k = 0; k < 3; ++k) {
       if (!want[k]) continue;
-      to[k] = grad_target(param[k], accumulate);
+      to[k] = grad_target(param[k], adds());
       grad[k] = to[k].grad.data_ptr<float>();
     }
     auto scratch = scratch_for(s, encoder_ops::embed_backward_scratch_bytes(batch * seq, H));
@@ -639,8 +661,7 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& weight, const std::opti
     node->activation = activation;
     node->weight = weight;
     node->bias = b;
-    node->accumulate = accumulate;
-    if (accumulate && weight.requires_grad()) node->use = begin_use(weight);
+    if (accumulate) node->accumulate_gradients({&weight, &b});
     torch::autograd::set_history(y, node);
     if (activation == kRelu) node->z = SavedVariable(y, /*is_output=*/true);
   }
@@ -700,8 +721,7 @@ at::Tensor conv_bias_relu(const at::Tensor& x, const at::Tensor& weight, const a
     node->dilation = dilation;
     node->groups = groups;
     node->pool = pool;
-    node->accumulate = accumulate;
-    if (accumulate && weight.requires_grad()) node->use = begin_use(weight);
+    if (accumulate) node->accumulate_gradients({&weight, &bias});
     torch::autograd::set_history(out, node);
     if (pool) {
       node->act = SavedVariable(z, false);
@@ -742,7 +762,7 @@ at::Tensor add_layer_norm(const at::Tensor& x, const std::optional<at::Tensor>& 
     node->b = SavedVariable(low[1], false);
     node->gamma = gamma;
     node->beta = beta;
-    node->accumulate = accumulate;
+    if (accumulate) node->accumulate_gradients({&gamma, &beta});
     node->residual = res.defined();
     torch::autograd::set_history(y, node);
   }
@@ -786,7 +806,7 @@ at::Tensor embed_layer_norm(const at::Tensor& ids, const at::Tensor& tok, const 
     node->rstd = SavedVariable(rstd, false);
     const at::Tensor* ps[5] = {&tok, &pos, &typ, &gamma, &beta};
     for (int k = 0; k < 5; ++k) node->param[k] = *ps[k];
-    node->accumulate = accumulate;
+    if (accumulate) node->accumulate_gradients({&tok, &pos, &typ, &gamma, &beta});
     torch::autograd::set_history(y[0], node);
   }
   return y[0];

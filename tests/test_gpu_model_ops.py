@@ -689,3 +689,27 @@ def test_a_frozen_parameter_of_the_embedding_keeps_its_gradient(frozen, accumula
     for k, (a, b) in enumerate(zip(*grads)):
         assert not torch.equal(a, torch.ones_like(a))
         assert torch.equal(b, torch.ones_like(a) if k in frozen else a), k
+
+
+def test_parameters_used_twice_in_a_graph_get_the_gradients_of_the_ordinary_path():
+    """Autograd adds the uses' gradients first and accumulates once: with a `.grad` far above them in size, adding each by
+    itself would round differently."""
+    import bagua_core_b200 as bb
+
+    g = torch.Generator().manual_seed(3)
+    ids = torch.randint(0, 40, (2, 30), generator=g).cuda()
+    x = torch.randn(60, 64, generator=g).bfloat16().cuda()
+    grads = []
+    for accumulate in (False, True):
+        torch.manual_seed(0)
+        ps = [torch.randn(*s, device="cuda", requires_grad=True) for s in ((40, 64), (30, 64), (1, 64), (64,), (64,), (64, 64), (64, 64))]
+        tok, pos, typ, gamma, beta, w1, w2 = ps
+        for p in ps:
+            p.grad = torch.full_like(p, 1e5) + torch.rand_like(p)
+        ys = [bb._C.embed_layer_norm(i, tok, pos, typ, gamma, beta, 1e-5, accumulate) for i in (ids, ids.flip(0))]
+        ys += [bb._C.add_layer_norm(x, None, gamma, beta, 1e-5, accumulate), bb._C.add_layer_norm(x * 2, None, gamma, beta, 1e-5, accumulate)]
+        ys += [bb._C.linear(x, w, beta, None, accumulate, a) for w, a in ((w1, 0), (w2, 2))]  # one bias for two layers
+        sum((k + 1) * y.float().square().sum() for k, y in enumerate(ys)).backward()
+        grads.append([p.grad for p in (tok, pos, typ, gamma, beta)])
+    for a, b in zip(*grads):
+        assert torch.equal(a, b)
