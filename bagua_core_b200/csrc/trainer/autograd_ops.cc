@@ -4,12 +4,14 @@
 #include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/autograd.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
 
 #include <array>
+#include <functional>
 #include <memory>
 #include <mutex>
 #include <unordered_map>
@@ -191,6 +193,54 @@ void to_bf16(std::array<at::Tensor, N>& ts) {
   }
 }
 
+// ---- gradients of gradients ----------------------------------------------------------------------
+// The kernels leave no history.  Where a backward pass is itself to be differentiated (create_graph=True), a node makes
+// its gradients from the plain composition of the framework's operations, evaluated again on the values that it saved.
+using Composition = std::function<at::Tensor(const std::vector<at::Tensor>&)>;
+
+// Hands its gradient to each of its edges.
+struct PassNode : public Node {
+  std::string name() const override { return "BaguaSavedValueBackward"; }
+  variable_list apply(variable_list&& grads) override { return variable_list(num_outputs(), grads[0]); }
+};
+
+// A saved value that stands for the node's inputs `inputs` (more than one: their sum), from which it may differ in type.
+struct Saved {
+  at::Tensor value;
+  std::vector<uint32_t> inputs;
+};
+
+variable_list differentiable_gradients(const Node& self, const Composition& f, const std::vector<Saved>& saved, const at::Tensor& dy) {
+  std::vector<at::Tensor> values;
+  variable_list sources;
+  std::vector<const Saved*> wanted;
+  for (const Saved& s : saved) {
+    values.push_back(s.value);
+    if (!s.value.defined()) continue;
+    torch::autograd::edge_list edges;
+    bool want = false;
+    for (uint32_t i : s.inputs) {
+      if (self.next_edge(i).is_valid()) edges.push_back(self.next_edge(i));
+      want = want || self.task_should_compute_output(i);
+    }
+    if (edges.empty()) continue;
+    auto node = std::shared_ptr<PassNode>(new PassNode(), torch::autograd::deleteNode);
+    node->set_next_edges(std::move(edges));
+    values.back() = s.value.variable_data();
+    torch::autograd::set_history(values.back(), node);
+    if (!want) continue;
+    sources.push_back(values.back());
+    wanted.push_back(&s);
+  }
+  variable_list out(self.num_outputs());
+  if (sources.empty()) return out;
+  const variable_list got = torch::autograd::grad({f(values)}, sources, {dy}, /*retain_graph=*/true, /*create_graph=*/true, /*allow_unused=*/true);
+  for (size_t k = 0; k < got.size(); ++k)
+    for (uint32_t i : wanted[k]->inputs)
+      if (self.task_should_compute_output(i)) out[i] = got[k];
+  return out;
+}
+
 template <typename N>
 std::shared_ptr<N> make_node(const at::Tensor& x, const at::Tensor& weight, const at::Tensor& bias) {
   auto node = std::shared_ptr<N>(new N(), torch::autograd::deleteNode);
@@ -246,8 +296,13 @@ struct AccumulatingNode : public Node {
 };
 
 // ---- linear ------------------------------------------------------------------------------------
+at::Tensor linear_composition(const std::vector<at::Tensor>& in, int activation) {  // x, weight, bias in one type
+  at::Tensor y = at::linear(in[0], in[1], in[2].defined() ? std::optional<at::Tensor>(in[2]) : std::nullopt);
+  return activation == kGelu ? at::gelu(y) : activation == kRelu ? at::relu(y) : y;
+}
+
 struct LinearNode : public AccumulatingNode {
-  SavedVariable x, w, z;  // z: what gelu was applied to, or the ReLU's result
+  SavedVariable x, w, b, z;  // b: in bf16; z: what gelu was applied to, or the ReLU's result
   at::Tensor weight, bias;  // the parameters (bias may be undefined)
   int activation = kNone;
 
@@ -258,6 +313,7 @@ struct LinearNode : public AccumulatingNode {
     std::lock_guard<std::mutex> lock(mutex_);
     x.reset_data();
     w.reset_data();
+    b.reset_data();
     z.reset_data();
   }
 
@@ -268,15 +324,14 @@ struct LinearNode : public AccumulatingNode {
     if (!grads[0].defined()) return out;
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
     const at::Tensor dy = grads[0], xs = x.unpack(), ws = w.unpack();
+    if (c10::GradMode::is_enabled())
+      return differentiable_gradients(*this, [this](const auto& in) { return linear_composition(in, activation); },
+                                      {{xs, {0}}, {ws, {1}}, {b.unpack(), {2}}}, dy);
     at::Tensor dy2 = vector_aligned(dy.dim() == 2 ? dy : dy.reshape({-1, dy.size(-1)}));
     if (activation) dy2 = through_activation(dy2.contiguous(), out);
     if (task_should_compute_output(0)) {
-      at::Tensor dx;
-      if (!c10::GradMode::is_enabled()) {
-        dx = fresh({dy2.size(0), ws.size(1)}, dy2.scalar_type(), dy2);
-        if (!gemm::input_grad(dy2, ws, dx)) dx = at::Tensor();
-      }
-      if (!dx.defined()) dx = at::mm(dy2, ws);
+      at::Tensor dx = fresh({dy2.size(0), ws.size(1)}, dy2.scalar_type(), dy2);
+      if (!gemm::input_grad(dy2, ws, dx)) dx = at::mm(dy2, ws);
       out[0] = dy.dim() == 2 ? dx : dx.view(xs.sizes());
     }
     if (task_should_compute_output(1)) {
@@ -318,7 +373,7 @@ struct LinearNode : public AccumulatingNode {
 
   at::Tensor bias_grad(const at::Tensor& dy2) {
     const int64_t rows = dy2.size(0), C = dy2.size(1);
-    if (!dy2.is_cuda() || c10::GradMode::is_enabled() || dy2.scalar_type() != at::kBFloat16 || C > (1 << 24) ||
+    if (!dy2.is_cuda() || dy2.scalar_type() != at::kBFloat16 || C > (1 << 24) ||
         !model_ops::column_sum_supported(rows, (int)C) || !dy2.is_contiguous() || (uintptr_t)dy2.data_ptr() % 16 != 0)
       return dy2.sum(at::IntArrayRef{0}, /*keepdim=*/false, at::kFloat);
     const bool add = adds() && per_column(bias, C) && accumulates(bias, dy2);
@@ -357,6 +412,9 @@ struct ConvNode : public AccumulatingNode {
     if (!grads[0].defined()) return out;
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
     const at::Tensor xs = x.unpack(), ws = w.unpack(), a = act.unpack(pool ? std::shared_ptr<Node>() : shared_from_this());
+    if (c10::GradMode::is_enabled())
+      return differentiable_gradients(*this, [this](const auto& in) { return composition(in); },
+                                      {{xs, {0}}, {ws, {1}}, {b.unpack(), {2}}}, grads[0]);
     const at::Tensor dy = vector_aligned(grads[0].contiguous(at::MemoryFormat::ChannelsLast));
     const bool alone = adds();
     const int C = (int)ws.size(0);
@@ -396,10 +454,17 @@ struct ConvNode : public AccumulatingNode {
     return out;
   }
 
+  at::Tensor composition(const std::vector<at::Tensor>& in) const {  // x, weight, bias in one type
+    const std::vector<int64_t> zero{0, 0};
+    const at::Tensor z = at::convolution(in[0], in[1], c10::nullopt, stride, padding, dilation, false, zero, groups);
+    const at::Tensor y = at::relu(z + in[2].view({1, -1, 1, 1}));
+    return pool ? at::max_pool2d(y, {2, 2}, {2, 2}) : y;
+  }
+
   // A 3 x 3 convolution of few channels whose input wants no gradient: both gradients come from one kernel.
   bool first_layer(const at::Tensor& xs, const at::Tensor& dy, const at::Tensor& a) {
     const std::vector<int64_t> one{1, 1};
-    return a.is_cuda() && !task_should_compute_output(0) && task_should_compute_output(1) && !c10::GradMode::is_enabled() &&
+    return a.is_cuda() && !task_should_compute_output(0) && task_should_compute_output(1) &&
            groups == 1 && weight.size(2) == 3 && weight.size(3) == 3 && stride == one && padding == one && dilation == one &&
            xs.scalar_type() == at::kBFloat16 && xs.is_contiguous(at::MemoryFormat::ChannelsLast) &&
            a.is_contiguous(at::MemoryFormat::ChannelsLast) && (uintptr_t)dy.data_ptr() % 16 == 0 &&
@@ -487,6 +552,7 @@ struct LayerNormNode : public EncoderNode {
   SavedVariable sum, mean, rstd, g, b;  // g, b: the parameters in bf16
   at::Tensor gamma, beta;
   bool residual = false;
+  double eps = 0;
 
   std::string name() const override { return "BaguaAddLayerNormBackward"; }
   void release_variables() override {
@@ -499,6 +565,10 @@ struct LayerNormNode : public EncoderNode {
     uses_done();
     if (!grads[0].defined()) return out;
     const at::Tensor s = sum.unpack();
+    if (c10::GradMode::is_enabled())
+      return differentiable_gradients(
+          *this, [this](const auto& in) { return at::layer_norm(in[0], {in[0].size(-1)}, in[1], in[2], eps); },
+          {{s, {0, 1}}, {g.unpack(), {2}}, {b.unpack(), {3}}}, grads[0]);
     const auto d = at::native_layer_norm_backward(grads[0].contiguous(), s, {s.size(-1)}, mean.unpack(), rstd.unpack(),
                                                   g.unpack(), b.unpack(),
                                                   {true, task_should_compute_output(2), task_should_compute_output(3)});
@@ -523,6 +593,8 @@ struct LayerNormNode : public EncoderNode {
 struct EmbedNode : public EncoderNode {
   SavedVariable ids, sum, mean, rstd;
   at::Tensor param[5];  // tok, pos, typ, gamma, beta
+  int64_t version[5];
+  double eps = 0;
 
   std::string name() const override { return "BaguaEmbedLayerNormBackward"; }
   void release_variables() override {
@@ -537,6 +609,21 @@ struct EmbedNode : public EncoderNode {
     const at::Tensor id = ids.unpack(), s = sum.unpack();
     const int H = (int)param[0].size(1);
     const int64_t batch = id.size(0), seq = id.size(1);
+    if (c10::GradMode::is_enabled()) {
+      std::vector<Saved> saved;
+      for (uint32_t k = 0; k < 5; ++k) {
+        BAGUA_CHECK(param[k]._version() == version[k], Tensor,
+                    "an embedding parameter needed for the gradient of a gradient was modified in place");
+        saved.push_back({param[k].detach(), {k}});
+      }
+      return differentiable_gradients(
+          *this,
+          [&](const auto& in) {
+            const at::Tensor x = at::embedding(in[0], id) + in[1].narrow(0, 0, seq).unsqueeze(0) + in[2].select(0, 0);
+            return at::layer_norm(x, {H}, in[3], in[4], eps).to(at::kBFloat16);
+          },
+          saved, grads[0]);
+    }
     // only what is asked for: a frozen parameter has a gradient in its bucket all the same, which stays as it is
     bool want[5];
     for (uint32_t k = 0; k < 5; ++k) want[k] = task_should_compute_output(k);
@@ -579,6 +666,14 @@ struct SpanLossNode : public Node {
     variable_list out(1);
     if (!grads[0].defined()) return out;
     const at::Tensor x = logits.unpack(), a = start.unpack(), b = end.unpack(), st = stats.unpack();
+    if (c10::GradMode::is_enabled())
+      return differentiable_gradients(
+          *this,
+          [&](const auto& in) {
+            const at::Tensor f = in[0].to(at::kFloat);
+            return (at::cross_entropy_loss(f.select(2, 0), a) + at::cross_entropy_loss(f.select(2, 1), b)) / 2;
+          },
+          {{x, {0}}}, grads[0]);
     at::Tensor dx = fresh_like(x);
     encoder_ops::span_loss_backward(x.data_ptr(), a.data_ptr<int64_t>(), b.data_ptr<int64_t>(), st.data_ptr<float>(),
                                     grads[0].data_ptr<float>(), dx.data_ptr(), x.size(0), x.size(1), stream_of(x));
@@ -596,6 +691,11 @@ struct SplitHeadsNode : public Node {
   std::string name() const override { return "BaguaSplitHeadsBackward"; }
   variable_list apply(variable_list&& grads) override {
     variable_list out(1);
+    if (c10::GradMode::is_enabled()) {
+      for (at::Tensor& g : grads) g = (g.defined() ? g : at::zeros({batch, heads, seq, dim}, options)).transpose(1, 2);
+      out[0] = at::stack({grads[0], grads[1], grads[2]}, 2).reshape({batch, seq, 3 * heads * dim});
+      return out;
+    }
     at::Tensor packed = at::empty({batch, seq, 3 * heads * dim}, options);
     const void* src[3];
     encoder_ops::HeadStrides st[3];
@@ -629,9 +729,9 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& weight, const std::opti
   std::shared_ptr<LinearNode> node;
   if (torch::autograd::compute_requires_grad(x, weight, b)) node = make_node<LinearNode>(x, weight, b);
   at::Tensor xs, ws, z, y;
+  std::array<at::Tensor, 3> low{x, w_low ? *w_low : weight, b};
   {
     PlainDispatch plain;
-    std::array<at::Tensor, 3> low{x, w_low ? *w_low : weight, b};
     to_bf16(low);
     xs = low[0];
     ws = low[1];
@@ -657,6 +757,7 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& weight, const std::opti
   if (node) {
     node->x = SavedVariable(xs, false);
     node->w = SavedVariable(ws, false);
+    node->b = SavedVariable(low[2], false);
     if (activation == kGelu) node->z = SavedVariable(z, false);
     node->activation = activation;
     node->weight = weight;
@@ -723,12 +824,8 @@ at::Tensor conv_bias_relu(const at::Tensor& x, const at::Tensor& weight, const a
     node->pool = pool;
     if (accumulate) node->accumulate_gradients({&weight, &bias});
     torch::autograd::set_history(out, node);
-    if (pool) {
-      node->act = SavedVariable(z, false);
-      node->b = SavedVariable(bs, false);
-    } else {
-      node->act = SavedVariable(out, /*is_output=*/true);
-    }
+    node->b = SavedVariable(bs, false);
+    node->act = pool ? SavedVariable(z, false) : SavedVariable(out, /*is_output=*/true);
   }
   return out;
 }
@@ -764,6 +861,7 @@ at::Tensor add_layer_norm(const at::Tensor& x, const std::optional<at::Tensor>& 
     node->beta = beta;
     if (accumulate) node->accumulate_gradients({&gamma, &beta});
     node->residual = res.defined();
+    node->eps = eps;
     torch::autograd::set_history(y, node);
   }
   return y;
@@ -805,7 +903,11 @@ at::Tensor embed_layer_norm(const at::Tensor& ids, const at::Tensor& tok, const 
     node->mean = SavedVariable(mean, false);
     node->rstd = SavedVariable(rstd, false);
     const at::Tensor* ps[5] = {&tok, &pos, &typ, &gamma, &beta};
-    for (int k = 0; k < 5; ++k) node->param[k] = *ps[k];
+    for (int k = 0; k < 5; ++k) {
+      node->param[k] = *ps[k];
+      node->version[k] = ps[k]->_version();
+    }
+    node->eps = eps;
     if (accumulate) node->accumulate_gradients({&tok, &pos, &typ, &gamma, &beta});
     torch::autograd::set_history(y[0], node);
   }

@@ -223,3 +223,28 @@ def test_bert_encoder_projections_take_both_options():
         # the bf16 copies hold the values the casts would produce: same training, bit for bit
         assert torch.equal(fused[r][0], both[r][0]) and fused[r][1] == both[r][1]
     assert torch.equal(both[0][0], both[1][0])
+
+
+def test_the_gradient_of_a_gradient_reaches_the_weights(wgrad):
+    """A gradient penalty, as by `torch.autograd.grad(..., create_graph=True)`."""
+    from bagua_core_b200.ops.fused_conv import ConvBiasReLU, ConvBiasReLUPool
+
+    conv = torch.nn.Conv2d(3, 8, 3, padding=1)
+    x, image = torch.randn(5, 48), torch.randn(2, 3, 6, 6)
+    m, ref = _pair(7)
+    m.weight.grad = m.bias.grad = None
+    cases = [(m, ref, x)]
+    for cls, plain in ((ConvBiasReLU, lambda t: torch.relu(conv(t))),
+                       (ConvBiasReLUPool, lambda t: torch.nn.functional.max_pool2d(torch.relu(conv(t)), 2, 2))):
+        block = cls(3, 8, 3, padding=1)
+        block.load_state_dict(conv.state_dict())
+        cases.append((block, plain, image))
+    for native, plain, value in cases:
+        got = []
+        for f, weight in ((native, native.weight), (plain, getattr(plain, "weight", conv.weight))):
+            t = value.clone().requires_grad_()
+            with torch.autocast("cpu", dtype=torch.bfloat16):
+                y = f(t)
+            (g,) = torch.autograd.grad(y.float().square().sum(), t, create_graph=True)
+            got.append(torch.autograd.grad(g.square().sum(), weight)[0])
+        assert got[1].norm() > 0 and (got[0] - got[1]).norm() <= 3e-2 * got[1].norm()

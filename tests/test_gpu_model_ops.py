@@ -713,3 +713,61 @@ def test_parameters_used_twice_in_a_graph_get_the_gradients_of_the_ordinary_path
         grads.append([p.grad for p in (tok, pos, typ, gamma, beta)])
     for a, b in zip(*grads):
         assert torch.equal(a, b)
+
+
+def _second_order(f, inputs, seed):
+    """Gradients of a sum of squared gradients, with respect to the inputs and to the first gradient's own input."""
+    y = f(*inputs)
+    g = torch.Generator().manual_seed(seed)
+    dy = torch.randn(y.shape, generator=g).to(y).requires_grad_()
+    first = torch.autograd.grad(y, inputs, dy, create_graph=True)
+    penalty = sum(t.float().square().sum() for t in first)
+    return list(first) + list(torch.autograd.grad(penalty, list(inputs) + [dy], allow_unused=True))
+
+
+def test_gradients_of_gradients_are_those_of_the_plain_composition():
+    import bagua_core_b200 as bb
+
+    C, F = bb._C, torch.nn.functional
+    torch.manual_seed(0)
+
+    def rnd(*s, bf16=False):
+        t = torch.randn(*s, device="cuda")
+        return (t.bfloat16() if bf16 else t).requires_grad_()
+
+    ids, span = torch.randint(0, 30, (2, 12)).cuda(), torch.randint(0, 12, (2, 3)).cuda()
+    b16 = lambda t: t.bfloat16()  # noqa: E731
+    acts = {0: lambda t: t, 1: F.gelu, 2: F.relu}
+    cases = []
+    for act in (0, 1, 2):
+        for bf16 in (False, True):
+            cases.append((lambda x, w, b, a=act: C.linear(x, w, b, None, True, a),
+                          lambda x, w, b, a=act: acts[a](F.linear(b16(x), b16(w), b16(b))), [rnd(2, 9, 16, bf16=bf16), rnd(24, 16), rnd(24)]))
+    for pool in (False, True):
+        cases.append((lambda x, w, b, p=pool: C.conv_bias_relu(x, w, b, [1, 1], [1, 1], [1, 1], 1, p, None, True),
+                      lambda x, w, b, p=pool: (lambda y: F.max_pool2d(y, 2, 2) if p else y)(F.relu(F.conv2d(x, w, b, padding=1))),
+                      [rnd(2, 8, 6, 6, bf16=True), rnd(16, 8, 3, 3, bf16=True), rnd(16, bf16=True)]))
+    cases.append((lambda x, r, g, b: C.add_layer_norm(x, r, g, b, 1e-5, True),
+                  lambda x, r, g, b: F.layer_norm(x + r, (64,), b16(g), b16(b), 1e-5),
+                  [rnd(5, 64, bf16=True), rnd(5, 64, bf16=True), rnd(64), rnd(64)]))
+    cases.append((lambda *t: C.embed_layer_norm(ids, *t, 1e-5, True),
+                  lambda t, p, y, g, b: b16(F.layer_norm(F.embedding(ids, t) + p[:12][None] + y[0][None, None], (64,), g, b, 1e-5)),
+                  [rnd(30, 64), rnd(20, 64), rnd(2, 64), rnd(64), rnd(64)]))
+    cases.append((lambda x: C.span_loss(x, span[0], span[1]),
+                  lambda x: (F.cross_entropy(x.float()[..., 0], span[0]) + F.cross_entropy(x.float()[..., 1], span[1])) / 2,
+                  [rnd(3, 12, 2, bf16=True)]))
+
+    def heads(x):
+        q, k, v = x.view(2, 16, 3, 2, 16).permute(2, 0, 3, 1, 4)
+        return F.scaled_dot_product_attention(q, k, v).transpose(1, 2).reshape(2, 16, 32)
+
+    cases.append((lambda x: C.attention(x, 2, 0.0), heads, [rnd(2, 16, 96, bf16=True)]))
+    with torch.nn.attention.sdpa_kernel(torch.nn.attention.SDPBackend.MATH):  # the one whose backward is differentiable
+        for n, (f, ref, inputs) in enumerate(cases):
+            for p in inputs:
+                p.grad = torch.zeros_like(p)
+            for k, (a, b) in enumerate(zip(_second_order(f, inputs, n), _second_order(ref, inputs, n))):
+                assert (a is None) == (b is None), (n, k)
+                if a is not None:  # bf16 in each of a few steps
+                    assert (a.double() - b.double()).norm() <= 3e-2 * b.double().norm() + 1e-6, (n, k)
+            assert all(bool((p.grad == 0).all()) for p in inputs)
