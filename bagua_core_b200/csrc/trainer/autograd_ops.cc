@@ -6,6 +6,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/autograd.h>
 #include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/graph_task.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
@@ -97,16 +98,6 @@ std::shared_ptr<Use> begin_use(const at::Tensor& param) {
   }
   slot = use;
   return use;
-}
-
-// Whether a gradient for `param` may be added to `param.grad` here: an fp32 gradient of the parameter's shape
-// and memory layout is there, no graph of the backward is being built, and no tensor hook wants to see it.
-bool accumulates(const at::Tensor& param, const at::Tensor& like) {
-  if (!param.defined() || c10::GradMode::is_enabled() || !param.is_leaf()) return false;
-  const at::Tensor& grad = param.grad();
-  return grad.defined() && grad.scalar_type() == at::kFloat && grad.sizes() == param.sizes() &&
-         grad.strides() == param.strides() && grad.is_non_overlapping_and_dense() && grad.device() == like.device() &&
-         torch::autograd::impl::hooks(param).empty();
 }
 
 // A bias of C values, one per column: any other shape that broadcasts is left to autograd, which folds its gradient.
@@ -256,26 +247,35 @@ std::shared_ptr<PoolRawTensor> scratch_for(const at::Tensor& t, size_t bytes) {
 struct AccumulatingNode : public Node {
   // For a new node: every parameter that wants a gradient is counted as used.
   void accumulate_gradients(std::initializer_list<const at::Tensor*> params) {
-    accumulate = true;
+    accumulate_ = true;
     size_t n = 0;
     for (const at::Tensor* p : params)
       if (p->defined() && p->requires_grad()) uses_[n++] = begin_use(*p);
   }
 
  protected:
-  bool accumulate = false;
-
+  bool accumulates() const { return accumulate_; }
   void uses_done() {
     for (auto& u : uses_)
       if (u) u->done = true;
   }
-  // Whether gradients may be added here, as far as that depends on the node: it was asked to, and none of its parameters
-  // takes part in the graph elsewhere.
-  bool adds() const {
-    if (!accumulate) return false;
+  // Whether the gradient of input `i`, the parameter `param`, may be added to `param.grad` here: the node was asked to, none
+  // of its parameters takes part in the graph elsewhere, the backward pass accumulates it (it is not one that returns the
+  // gradient, as torch.autograd.grad does), an fp32 gradient of the parameter's shape and memory layout is there, and no
+  // tensor hook wants to see it.
+  bool adds(uint32_t i, const at::Tensor& param, const at::Tensor& like) const {
+    if (!accumulate_ || !param.defined() || c10::GradMode::is_enabled() || !param.is_leaf() || !next_edge(i).is_valid()) return false;
     for (auto& u : uses_)
       if (u && u->shared) return false;
-    return true;
+    const auto* info = torch::autograd::get_current_graph_task_exec_info();
+    if (info && !info->empty()) {
+      const auto it = info->find(next_edge(i).function.get());
+      if (it == info->end() || !it->second.needed_ || it->second.captures_) return false;
+    }
+    const at::Tensor& grad = param.grad();
+    return grad.defined() && grad.scalar_type() == at::kFloat && grad.sizes() == param.sizes() &&
+           grad.strides() == param.strides() && grad.is_non_overlapping_and_dense() && grad.device() == like.device() &&
+           torch::autograd::impl::hooks(param).empty();
   }
   // Has been done for input `i`.  Autograd orders the stream that a parameter's gradient is finished on (that of its
   // accumulation node, on which its hooks run) behind the stream that made it when it hands the gradient over.  It is
@@ -292,6 +292,7 @@ struct AccumulatingNode : public Node {
   }
 
  private:
+  bool accumulate_ = false;
   std::array<std::shared_ptr<Use>, 5> uses_;
 };
 
@@ -337,8 +338,8 @@ struct LinearNode : public AccumulatingNode {
     if (task_should_compute_output(1)) {
       const at::Tensor x2 = xs.dim() == 2 ? xs : xs.reshape({-1, xs.size(-1)});
       bool done = false;
-      if (accumulate) {
-        if (adds() && accumulates(weight, dy2) && weight.grad().is_contiguous()) {
+      if (accumulates()) {
+        if (adds(1, weight, dy2) && weight.grad().is_contiguous()) {
           c10::NoGradGuard no_grad;
           done = gemm_into(weight.grad(), dy2.t(), x2);
           if (done) added(1, dy2);
@@ -358,7 +359,7 @@ struct LinearNode : public AccumulatingNode {
     const int64_t rows = dy2.size(0);
     const int C = (int)dy2.size(1);
     const bool want = bias.defined() && task_should_compute_output(2);
-    const bool add = want && adds() && per_column(bias, C) && accumulates(bias, dy2);
+    const bool add = want && per_column(bias, C) && adds(2, bias, dy2);
     at::Tensor db = add ? bias.grad() : fresh({C}, at::kFloat, dy2);
     at::Tensor dz = fresh_like(dy2);
     const size_t bytes = encoder_ops::activation_backward_scratch_bytes(rows, C);
@@ -376,7 +377,7 @@ struct LinearNode : public AccumulatingNode {
     if (!dy2.is_cuda() || dy2.scalar_type() != at::kBFloat16 || C > (1 << 24) ||
         !model_ops::column_sum_supported(rows, (int)C) || !dy2.is_contiguous() || (uintptr_t)dy2.data_ptr() % 16 != 0)
       return dy2.sum(at::IntArrayRef{0}, /*keepdim=*/false, at::kFloat);
-    const bool add = adds() && per_column(bias, C) && accumulates(bias, dy2);
+    const bool add = per_column(bias, C) && adds(2, bias, dy2);
     at::Tensor db = add ? bias.grad() : fresh({C}, at::kFloat, dy2);
     const size_t bytes = model_ops::column_sum_scratch_bytes(rows, (int)C);
     std::shared_ptr<PoolRawTensor> scratch = bytes ? scratch_for(dy2, bytes) : nullptr;
@@ -416,15 +417,14 @@ struct ConvNode : public AccumulatingNode {
       return differentiable_gradients(*this, [this](const auto& in) { return composition(in); },
                                       {{xs, {0}}, {ws, {1}}, {b.unpack(), {2}}}, grads[0]);
     const at::Tensor dy = vector_aligned(grads[0].contiguous(at::MemoryFormat::ChannelsLast));
-    const bool alone = adds();
     const int C = (int)ws.size(0);
     if (!pool && first_layer(xs, dy, a)) {
-      first_layer_backward(xs, dy, a, alone, out);
+      first_layer_backward(xs, dy, a, out);
       return out;
     }
     at::Tensor dz = at::empty_like(a);
     // the bias gradient is added to `.grad` by the fold of its partial sums
-    const bool add_bias = alone && dy.is_cuda() && task_should_compute_output(2) && accumulates(bias, dy);
+    const bool add_bias = dy.is_cuda() && task_should_compute_output(2) && adds(2, bias, dy);
     at::Tensor db = add_bias ? bias.grad() : fresh({C}, at::kFloat, a);
     backward_tail(dy, a, dz, db, add_bias);
     if (add_bias) added(2, dy);
@@ -436,7 +436,7 @@ struct ConvNode : public AccumulatingNode {
                                         {need_x, need_w, false});
       out[0] = std::get<0>(g);
       at::Tensor dw = std::get<1>(g);
-      if (need_w && alone && dw.scalar_type() == at::kBFloat16 && accumulates(weight, dw) &&
+      if (need_w && dw.scalar_type() == at::kBFloat16 && adds(1, weight, dw) &&
           dw.strides() == weight.grad().strides()) {
         // the cast to fp32 and the addition in one pass; the same bits
         if (dw.is_cuda()) {
@@ -471,11 +471,11 @@ struct ConvNode : public AccumulatingNode {
            (uintptr_t)a.data_ptr() % 16 == 0 &&
            model_ops::first_conv_backward_supported(a.size(0), a.size(2), a.size(3), a.size(1), xs.size(1));
   }
-  void first_layer_backward(const at::Tensor& xs, const at::Tensor& dy, const at::Tensor& a, bool alone, variable_list& out) {
+  void first_layer_backward(const at::Tensor& xs, const at::Tensor& dy, const at::Tensor& a, variable_list& out) {
     const int C = (int)a.size(1), Ci = (int)xs.size(1);
     const bool want_b = task_should_compute_output(2);
-    const bool add_b = alone && want_b && accumulates(bias, dy);
-    const bool add_w = alone && weight.is_contiguous(at::MemoryFormat::ChannelsLast) && accumulates(weight, dy);
+    const bool add_b = want_b && adds(2, bias, dy);
+    const bool add_w = weight.is_contiguous(at::MemoryFormat::ChannelsLast) && adds(1, weight, dy);
     const auto f = a.options().dtype(at::kFloat);
     at::Tensor db = add_b ? bias.grad() : want_b ? at::empty({C}, f) : at::Tensor();
     at::Tensor dw = add_w ? weight.grad() : at::empty(weight.sizes(), f, at::MemoryFormat::ChannelsLast);
@@ -520,22 +520,13 @@ struct ConvNode : public AccumulatingNode {
 };
 
 // ---- encoder layers ------------------------------------------------------------------------------
-// An fp32 gradient for `param`: its `.grad` to be added to, or zeros for autograd.
-struct GradTarget {
-  at::Tensor grad;
-  bool add = false;
-};
-GradTarget grad_target(const at::Tensor& param, bool accumulate) {
-  if (accumulate && accumulates(param, param) && param.grad().is_contiguous()) return {param.grad(), true};
-  return {at::zeros(param.sizes(), param.options()), false};
-}
-
 struct EncoderNode : public AccumulatingNode {
  protected:
+  bool adds_contiguous(uint32_t i, const at::Tensor& param) const { return adds(i, param, param) && param.grad().is_contiguous(); }
   // Adds the gradient of input `i` to its place, or leaves it to autograd.
   void give(uint32_t i, const at::Tensor& param, const at::Tensor& g, variable_list& out) const {
     if (!g.defined()) return;
-    if (!adds() || !accumulates(param, param) || !param.grad().is_contiguous()) {
+    if (!adds_contiguous(i, param)) {
       out[i] = g;  // autograd casts it to the parameter's type
       return;
     }
@@ -575,8 +566,7 @@ struct LayerNormNode : public EncoderNode {
     out[0] = std::get<0>(d);
     if (residual) out[1] = out[0];
     const at::Tensor &dg = std::get<1>(d), &db = std::get<2>(d);
-    if (adds() && dg.defined() && db.defined() && accumulates(gamma, dg) && accumulates(beta, db) &&
-        gamma.grad().is_contiguous() && beta.grad().is_contiguous()) {
+    if (dg.defined() && db.defined() && adds_contiguous(2, gamma) && adds_contiguous(3, beta)) {
       kernels::cuda::accumulate_bf16_pair(gamma.grad().data_ptr<float>(), dg.data_ptr(), beta.grad().data_ptr<float>(),
                                           db.data_ptr(), dg.numel(), stream_of(s));
       count_launches(1);
@@ -632,23 +622,19 @@ struct EmbedNode : public EncoderNode {
     give(3, param[3], std::get<1>(d), out);
     give(4, param[4], std::get<2>(d), out);
     if (!want[0] && !want[1] && !want[2]) return out;
-    GradTarget to[3];
+    bool add[3] = {false, false, false};
     float* grad[3] = {nullptr, nullptr, nullptr};
-    for (int k = 0; k < 3; ++k) {
+    for (uint32_t k = 0; k < 3; ++k) {
       if (!want[k]) continue;
-      to[k] = grad_target(param[k], adds());
-      grad[k] = to[k].grad.data_ptr<float>();
+      add[k] = adds_contiguous(k, param[k]);
+      if (!add[k]) out[k] = at::zeros(param[k].sizes(), param[k].options());
+      grad[k] = (add[k] ? param[k].grad() : out[k]).data_ptr<float>();
     }
     auto scratch = scratch_for(s, encoder_ops::embed_backward_scratch_bytes(batch * seq, H));
     count_launches(encoder_ops::embed_backward(std::get<0>(d).data_ptr<float>(), id.data_ptr<int64_t>(), param[0].size(0), grad[0],
                                                grad[1], grad[2], scratch->data_ptr(), batch, seq, H, stream_of(s)));
-    for (uint32_t k = 0; k < 3; ++k) {
-      if (!want[k]) continue;
-      if (to[k].add)
-        added(k, s);
-      else
-        out[k] = to[k].grad;
-    }
+    for (uint32_t k = 0; k < 3; ++k)
+      if (add[k]) added(k, s);
     return out;
   }
 };

@@ -16,9 +16,10 @@ runs them when it reaches the parameter even without a gradient.  The ordinary p
 shortcut would change what the user sees:
 
 * the feature is off (`enabled`, default False), or a higher-order graph is being built;
+* the backward pass returns the gradient instead of accumulating it (`torch.autograd.grad`);
 * `.grad` is missing, not fp32, not contiguous or of another shape;
 * the parameter has tensor hooks (`register_hook`), which autograd would apply to the gradient;
-* the same weight takes part in the graph more than once: autograd would add the uses' gradients first
+* the same parameter takes part in the graph more than once: autograd would add the uses' gradients first
   and accumulate once, so all uses take the ordinary path.
 
 Module attributes `accumulated` and `declined` count the weight gradients of linear layers that were added in

@@ -248,3 +248,25 @@ def test_the_gradient_of_a_gradient_reaches_the_weights(wgrad):
             (g,) = torch.autograd.grad(y.float().square().sum(), t, create_graph=True)
             got.append(torch.autograd.grad(g.square().sum(), weight)[0])
         assert got[1].norm() > 0 and (got[0] - got[1]).norm() <= 3e-2 * got[1].norm()
+
+
+def test_gradients_that_are_asked_for_are_returned_and_not_added(wgrad):
+    """`torch.autograd.grad` over parameters that have a `.grad`; `backward(inputs=...)` adds to those named alone."""
+    from bagua_core_b200.ops.fused_conv import ConvBiasReLU
+
+    block = ConvBiasReLU(3, 8, 3, padding=1)
+    for m, x in ((_pair(8)[0], torch.randn(5, 48)), (block, torch.randn(2, 3, 6, 6))):
+        for p in m.parameters():
+            p.grad = torch.zeros_like(p)
+
+        def loss():
+            with torch.autocast("cpu", dtype=torch.bfloat16):
+                return m(x).float().square().sum()
+
+        got = torch.autograd.grad(loss(), list(m.parameters()))
+        assert all(bool((p.grad == 0).all()) for p in m.parameters())
+        loss().backward(inputs=[m.weight])
+        assert torch.allclose(m.weight.grad, got[0], rtol=1e-2, atol=1e-2) and bool((m.bias.grad == 0).all())
+        loss().backward()
+        assert torch.allclose(m.weight.grad, 2 * got[0], rtol=1e-2, atol=2e-2)
+        assert torch.allclose(m.bias.grad, got[1], rtol=1e-2, atol=1e-2)

@@ -771,3 +771,28 @@ def test_gradients_of_gradients_are_those_of_the_plain_composition():
                 if a is not None:  # bf16 in each of a few steps
                     assert (a.double() - b.double()).norm() <= 3e-2 * b.double().norm() + 1e-6, (n, k)
             assert all(bool((p.grad == 0).all()) for p in inputs)
+
+
+def test_gradients_that_are_asked_for_are_returned_and_not_added():
+    import bagua_core_b200 as bb
+
+    g = torch.Generator().manual_seed(3)
+    ids = torch.randint(0, 40, (2, 30), generator=g).cuda()
+    x = torch.randn(60, 64, generator=g).bfloat16().cuda()
+    image = torch.randn(2, 3, 8, 8, generator=g).bfloat16().cuda().contiguous(memory_format=torch.channels_last)
+    cases = [(lambda *p: bb._C.embed_layer_norm(ids, *p, 1e-5, True), [(40, 64), (30, 64), (1, 64), (64,), (64,)]),
+             (lambda *p: bb._C.add_layer_norm(x, None, *p, 1e-5, True), [(64,), (64,)]),
+             (lambda *p: bb._C.linear(x, *p, None, True), [(24, 64), (24,)]),
+             (lambda *p: bb._C.linear(x, *p, None, True, 1), [(24, 64), (24,)]),
+             (lambda *p: bb._C.conv_bias_relu(image, p[0].bfloat16().contiguous(memory_format=torch.channels_last), p[1].bfloat16(),
+                                              [1, 1], [1, 1], [1, 1], 1, True, None, True), [(64, 3, 3, 3), (64,)])]
+    for f, shapes in cases:
+        ps = [torch.randn(*s, generator=g).cuda().requires_grad_() for s in shapes]
+        for p in ps:
+            p.grad = torch.zeros_like(p)
+        dy = torch.randn_like(f(*ps))
+        got = torch.autograd.grad(f(*ps), ps, dy)
+        assert all(bool((p.grad == 0).all()) for p in ps)
+        f(*ps).backward(dy)
+        for p, q in zip(ps, got):  # rounded to bf16 on the way where the gradient is handed over
+            assert q.norm() > 0 and (p.grad - q).norm() <= 1e-2 * q.norm()
