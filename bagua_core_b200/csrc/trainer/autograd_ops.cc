@@ -3,6 +3,7 @@
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/autograd.h>
 #include <torch/csrc/autograd/function.h>
@@ -188,6 +189,16 @@ void to_bf16(std::array<at::Tensor, N>& ts) {
 // The kernels leave no history.  Where a backward pass is itself to be differentiated (create_graph=True), a node makes
 // its gradients from the plain composition of the framework's operations, evaluated again on the values that it saved.
 using Composition = std::function<at::Tensor(const std::vector<at::Tensor>&)>;
+
+// The same composition stands in for the kernels where they would pass somebody by who looks at the operations
+// themselves: forward-mode differentiation, torch.func's transforms, tensor subclasses and dispatch modes (tracers, counters).
+bool watched(std::initializer_list<const at::Tensor*> inputs) {
+  static const c10::DispatchKeySet wrapped({c10::DispatchKey::Python, c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper});
+  if (c10::impl::TorchDispatchModeTLS::any_modes_set()) return true;
+  for (const at::Tensor* t : inputs)
+    if (t->defined() && (t->key_set().has_any(wrapped) || t->_fw_grad(/*level=*/0).defined())) return true;
+  return false;
+}
 
 // Hands its gradient to each of its edges.
 struct PassNode : public Node {
@@ -390,12 +401,20 @@ struct LinearNode : public AccumulatingNode {
 };
 
 // ---- convolution + bias + ReLU (+ pooling) -------------------------------------------------------
+at::Tensor conv_composition(const std::vector<at::Tensor>& in, const std::vector<int64_t>& stride,  // x, weight, bias in one type
+                            const std::vector<int64_t>& padding, const std::vector<int64_t>& dilation, int64_t groups, bool pool) {
+  const std::vector<int64_t> zero{0, 0};
+  const at::Tensor z = at::convolution(in[0], in[1], c10::nullopt, stride, padding, dilation, false, zero, groups);
+  const at::Tensor y = at::relu(z + in[2].view({1, -1, 1, 1}));
+  return pool ? at::max_pool2d(y, {2, 2}, {2, 2}) : y;
+}
+
 struct ConvNode : public AccumulatingNode {
   SavedVariable x, w, b, act;  // act: the activation, or with pooling the convolution's output
   at::Tensor weight, bias;
   std::vector<int64_t> stride, padding, dilation;
   int64_t groups = 1;
-  bool pool = false;
+  bool pool = false;  // 2x2, behind the ReLU
 
   std::string name() const override { return pool ? "BaguaConvBiasReLUPoolBackward" : "BaguaConvBiasReLUBackward"; }
   void release_variables() override {
@@ -414,7 +433,7 @@ struct ConvNode : public AccumulatingNode {
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
     const at::Tensor xs = x.unpack(), ws = w.unpack(), a = act.unpack(pool ? std::shared_ptr<Node>() : shared_from_this());
     if (c10::GradMode::is_enabled())
-      return differentiable_gradients(*this, [this](const auto& in) { return composition(in); },
+      return differentiable_gradients(*this, [this](const auto& in) { return conv_composition(in, stride, padding, dilation, groups, pool); },
                                       {{xs, {0}}, {ws, {1}}, {b.unpack(), {2}}}, grads[0]);
     const at::Tensor dy = vector_aligned(grads[0].contiguous(at::MemoryFormat::ChannelsLast));
     const int C = (int)ws.size(0);
@@ -452,13 +471,6 @@ struct ConvNode : public AccumulatingNode {
       }
     }
     return out;
-  }
-
-  at::Tensor composition(const std::vector<at::Tensor>& in) const {  // x, weight, bias in one type
-    const std::vector<int64_t> zero{0, 0};
-    const at::Tensor z = at::convolution(in[0], in[1], c10::nullopt, stride, padding, dilation, false, zero, groups);
-    const at::Tensor y = at::relu(z + in[2].view({1, -1, 1, 1}));
-    return pool ? at::max_pool2d(y, {2, 2}, {2, 2}) : y;
   }
 
   // A 3 x 3 convolution of few channels whose input wants no gradient: both gradients come from one kernel.
@@ -580,6 +592,11 @@ struct LayerNormNode : public EncoderNode {
   }
 };
 
+at::Tensor embed_composition(const at::Tensor& ids, const std::vector<at::Tensor>& in, double eps) {  // tok, pos, typ, gamma, beta
+  const at::Tensor x = at::embedding(in[0], ids) + in[1].narrow(0, 0, ids.size(1)).unsqueeze(0) + in[2].select(0, 0);
+  return at::layer_norm(x, {x.size(-1)}, in[3], in[4], eps).to(at::kBFloat16);
+}
+
 struct EmbedNode : public EncoderNode {
   SavedVariable ids, sum, mean, rstd;
   at::Tensor param[5];  // tok, pos, typ, gamma, beta
@@ -606,13 +623,7 @@ struct EmbedNode : public EncoderNode {
                     "an embedding parameter needed for the gradient of a gradient was modified in place");
         saved.push_back({param[k].detach(), {k}});
       }
-      return differentiable_gradients(
-          *this,
-          [&](const auto& in) {
-            const at::Tensor x = at::embedding(in[0], id) + in[1].narrow(0, 0, seq).unsqueeze(0) + in[2].select(0, 0);
-            return at::layer_norm(x, {H}, in[3], in[4], eps).to(at::kBFloat16);
-          },
-          saved, grads[0]);
+      return differentiable_gradients(*this, [&](const auto& in) { return embed_composition(id, in, eps); }, saved, grads[0]);
     }
     // only what is asked for: a frozen parameter has a gradient in its bucket all the same, which stays as it is
     bool want[5];
@@ -639,6 +650,11 @@ struct EmbedNode : public EncoderNode {
   }
 };
 
+at::Tensor span_loss_composition(const at::Tensor& logits, const at::Tensor& start, const at::Tensor& end) {
+  const at::Tensor f = logits.to(at::kFloat);
+  return (at::cross_entropy_loss(f.select(2, 0), start) + at::cross_entropy_loss(f.select(2, 1), end)) / 2;
+}
+
 struct SpanLossNode : public Node {
   SavedVariable logits, start, end, stats;
 
@@ -653,13 +669,7 @@ struct SpanLossNode : public Node {
     if (!grads[0].defined()) return out;
     const at::Tensor x = logits.unpack(), a = start.unpack(), b = end.unpack(), st = stats.unpack();
     if (c10::GradMode::is_enabled())
-      return differentiable_gradients(
-          *this,
-          [&](const auto& in) {
-            const at::Tensor f = in[0].to(at::kFloat);
-            return (at::cross_entropy_loss(f.select(2, 0), a) + at::cross_entropy_loss(f.select(2, 1), b)) / 2;
-          },
-          {{x, {0}}}, grads[0]);
+      return differentiable_gradients(*this, [&](const auto& in) { return span_loss_composition(in[0], a, b); }, {{x, {0}}}, grads[0]);
     at::Tensor dx = fresh_like(x);
     encoder_ops::span_loss_backward(x.data_ptr(), a.data_ptr<int64_t>(), b.data_ptr<int64_t>(), st.data_ptr<float>(),
                                     grads[0].data_ptr<float>(), dx.data_ptr(), x.size(0), x.size(1), stream_of(x));
@@ -712,6 +722,10 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& weight, const std::opti
   BAGUA_CHECK(activation == kNone || ((activation == kGelu || activation == kRelu) && activation_fusable(x, weight.size(0))), Tensor,
               "the activation cannot be fused with this layer");
   const at::Tensor b = bias.value_or(at::Tensor());
+  if (watched({&x, &weight, &b})) {
+    c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
+    return linear_composition({x.to(at::kBFloat16), weight.to(at::kBFloat16), b.defined() ? b.to(at::kBFloat16) : b}, activation);
+  }
   std::shared_ptr<LinearNode> node;
   if (torch::autograd::compute_requires_grad(x, weight, b)) node = make_node<LinearNode>(x, weight, b);
   at::Tensor xs, ws, z, y;
@@ -759,10 +773,15 @@ at::Tensor conv_bias_relu(const at::Tensor& x, const at::Tensor& weight, const a
                           const std::vector<int64_t>& stride, const std::vector<int64_t>& padding,
                           const std::vector<int64_t>& dilation, int64_t groups, bool pool,
                           const std::optional<at::Tensor>& w_low, bool accumulate) {
-  std::shared_ptr<ConvNode> node;
-  if (torch::autograd::compute_requires_grad(x, weight, bias)) node = make_node<ConvNode>(x, weight, bias);
   const bool cast = autocast_on(x);
   const at::ScalarType low = cast ? at::autocast::get_autocast_dtype(x.device().type()) : at::kBFloat16;
+  if (watched({&x, &weight, &bias})) {
+    c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
+    auto in = [&](const at::Tensor& t) { return cast ? t.to(low) : t; };
+    return conv_composition({in(x), in(weight), in(bias)}, stride, padding, dilation, groups, pool);
+  }
+  std::shared_ptr<ConvNode> node;
+  if (torch::autograd::compute_requires_grad(x, weight, bias)) node = make_node<ConvNode>(x, weight, bias);
   at::Tensor xs, ws, bs, z, out;
   {
     PlainDispatch plain;
@@ -824,6 +843,10 @@ at::Tensor add_layer_norm(const at::Tensor& x, const std::optional<at::Tensor>& 
                   fp32_param(beta, H, x) && gamma.dim() == 1 && beta.dim() == 1 &&
                   (!res.defined() || (res.sizes() == x.sizes() && res.scalar_type() == at::kBFloat16 && res.device() == x.device())),
               Tensor, "add_layer_norm needs bf16 CUDA activations of one shape and fp32 parameters");
+  if (watched({&x, &res, &gamma, &beta})) {
+    c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
+    return at::layer_norm(res.defined() ? x + res : x, {H}, gamma.to(x.scalar_type()), beta.to(x.scalar_type()), eps);
+  }
   std::shared_ptr<LayerNormNode> node;
   if (torch::autograd::compute_requires_grad(x, res, gamma, beta)) {
     node = std::shared_ptr<LayerNormNode>(new LayerNormNode(), torch::autograd::deleteNode);
@@ -865,6 +888,10 @@ at::Tensor embed_layer_norm(const at::Tensor& ids, const at::Tensor& tok, const 
                   beta.dim() == 1,
               Tensor, "embed_layer_norm needs tables with rows and parameters of one row");
   BAGUA_CHECK(ids.size(1) <= pos.size(0), Tensor, "sequence of " << ids.size(1) << " tokens, " << pos.size(0) << " positions");
+  if (watched({&ids, &tok, &pos, &typ, &gamma, &beta})) {
+    c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
+    return embed_composition(ids, {tok, pos, typ, gamma, beta}, eps);
+  }
   std::shared_ptr<EmbedNode> node;
   if (torch::autograd::compute_requires_grad(tok, pos, typ, gamma, beta)) {
     node = std::shared_ptr<EmbedNode>(new EmbedNode(), torch::autograd::deleteNode);
@@ -908,6 +935,10 @@ at::Tensor span_loss(const at::Tensor& logits, const at::Tensor& start, const at
   for (const at::Tensor* t : {&start, &end})
     BAGUA_CHECK(t->device() == logits.device() && t->scalar_type() == at::kLong && t->dim() == 1 && t->size(0) == B, Tensor,
                 "span_loss needs int64 positions [batch] on the logits' device");
+  if (watched({&logits, &start, &end})) {
+    c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
+    return span_loss_composition(logits, start, end);
+  }
   std::shared_ptr<SpanLossNode> node;
   if (torch::autograd::compute_requires_grad(logits)) {
     node = std::shared_ptr<SpanLossNode>(new SpanLossNode(), torch::autograd::deleteNode);
@@ -941,6 +972,11 @@ at::Tensor attention(const at::Tensor& qkv, int64_t heads, double dropout) {
               Tensor, "attention needs a packed bf16 projection [batch, seq, 3 * heads * dim] with dim a multiple of 8");
   const int64_t B = qkv.size(0), S = qkv.size(1), W = qkv.size(2), D = W / (3 * heads);
   variable_list parts;
+  if (watched({&qkv})) {
+    const at::Tensor p = qkv.view({B, S, 3, heads, D}).permute({2, 0, 3, 1, 4});
+    const at::Tensor a = at::scaled_dot_product_attention(p.select(0, 0), p.select(0, 1), p.select(0, 2), c10::nullopt, dropout);
+    return a.transpose(1, 2).reshape({B, S, heads * D});
+  }
   std::shared_ptr<SplitHeadsNode> node;
   if (torch::autograd::compute_requires_grad(qkv)) {
     node = std::shared_ptr<SplitHeadsNode>(new SplitHeadsNode(), torch::autograd::deleteNode);

@@ -270,3 +270,33 @@ def test_gradients_that_are_asked_for_are_returned_and_not_added(wgrad):
         loss().backward()
         assert torch.allclose(m.weight.grad, 2 * got[0], rtol=1e-2, atol=2e-2)
         assert torch.allclose(m.bias.grad, got[1], rtol=1e-2, atol=1e-2)
+
+
+def test_who_looks_at_the_operations_sees_the_plain_composition(wgrad):
+    """Forward-mode derivatives, `torch.func` and dispatch modes (here the FLOP counter) through the native layers."""
+    import torch.autograd.forward_ad as fwad
+    from torch.utils.flop_counter import FlopCounterMode
+
+    from bagua_core_b200.ops.fused_conv import ConvBiasReLUPool
+
+    linear, ref = _pair(9)
+    conv, block = torch.nn.Conv2d(3, 8, 3, padding=1), ConvBiasReLUPool(3, 8, 3, padding=1)
+    block.load_state_dict(conv.state_dict())
+
+    def plain_block(t):  # rounds between the product and the bias, as the block does: the same masks
+        z = torch.nn.functional.conv2d(t, conv.weight, None, padding=1)
+        return torch.nn.functional.max_pool2d(torch.relu(z + conv.bias.bfloat16().view(1, -1, 1, 1)), 2, 2)
+
+    for m, plain, x in ((linear, ref, torch.randn(5, 48)), (block, plain_block, torch.randn(2, 3, 6, 6))):
+        tangents, flops, mapped = [], [], []
+        for f in (m, plain):
+            with torch.autocast("cpu", dtype=torch.bfloat16):
+                with fwad.dual_level():
+                    tangents.append(fwad.unpack_dual(f(fwad.make_dual(x, torch.ones_like(x)))).tangent)
+                with FlopCounterMode(display=False) as counter:
+                    f(x)
+                flops.append(counter.get_total_flops())
+                mapped.append(torch.func.vmap(f)(torch.stack([x, 2 * x])))
+        assert torch.allclose(tangents[0].float(), tangents[1].float(), rtol=2e-2, atol=2e-2)
+        assert flops[0] == flops[1] > 0
+        assert torch.allclose(mapped[0].float(), mapped[1].float(), rtol=2e-2, atol=2e-2)

@@ -796,3 +796,32 @@ def test_gradients_that_are_asked_for_are_returned_and_not_added():
         f(*ps).backward(dy)
         for p, q in zip(ps, got):  # rounded to bf16 on the way where the gradient is handed over
             assert q.norm() > 0 and (p.grad - q).norm() <= 1e-2 * q.norm()
+
+
+def test_forward_mode_derivatives_are_those_of_the_plain_composition():
+    import torch.autograd.forward_ad as fwad
+
+    import bagua_core_b200 as bb
+
+    C, F = bb._C, torch.nn.functional
+    torch.manual_seed(0)
+    ids, span = torch.randint(0, 30, (2, 12)).cuda(), torch.randint(0, 12, (2, 3)).cuda()
+    b16 = lambda t: t.bfloat16()  # noqa: E731
+    cases = [(lambda x, w, b: C.linear(x, w, b, None, True, 1), lambda x, w, b: F.gelu(F.linear(b16(x), b16(w), b16(b))),
+              [torch.randn(9, 16), torch.randn(24, 16), torch.randn(24)]),
+             (lambda x, r, g, b: C.add_layer_norm(x, r, g, b, 1e-5, True), lambda x, r, g, b: F.layer_norm(x + r, (64,), b16(g), b16(b), 1e-5),
+              [b16(torch.randn(5, 64)), b16(torch.randn(5, 64)), torch.randn(64), torch.randn(64)]),
+             (lambda *t: C.embed_layer_norm(ids, *t, 1e-5, True),
+              lambda t, p, y, g, b: b16(F.layer_norm(F.embedding(ids, t) + p[:12][None] + y[0][None, None], (64,), g, b, 1e-5)),
+              [torch.randn(30, 64), torch.randn(20, 64), torch.randn(2, 64), torch.randn(64), torch.randn(64)]),
+             (lambda x: C.span_loss(x, span[0], span[1]),
+              lambda x: (F.cross_entropy(x.float()[..., 0], span[0]) + F.cross_entropy(x.float()[..., 1], span[1])) / 2,
+              [b16(torch.randn(3, 12, 2))])]
+    for n, (f, ref, inputs) in enumerate(cases):
+        inputs = [t.cuda().requires_grad_() for t in inputs]
+        got = []
+        for g in (f, ref):
+            with fwad.dual_level():
+                torch.manual_seed(n)
+                got.append(fwad.unpack_dual(g(*[fwad.make_dual(t, torch.randn_like(t)) for t in inputs])).tangent)
+        assert (got[0].double() - got[1].double()).norm() <= 2e-2 * got[1].double().norm(), n
