@@ -23,6 +23,7 @@ import torch.nn.functional as F
 from .._native import C as _C
 from ..ops import wgrad
 from ..ops.fused_linear import ShadowLinear
+from ..ops.modules import dropout, plain_embedding, untouched
 
 
 _EMBED_TOKENS = 4096  # encoder_ops::kMaxTokens: more tokens per batch take the framework's embedding
@@ -74,11 +75,14 @@ class _LayerNorm(nn.LayerNorm):
             return F.layer_norm(x, self.normalized_shape, self.weight.to(x.dtype), self.bias.to(x.dtype), self.eps)
 
 
+def _bf16_autocast(x: torch.Tensor) -> bool:
+    return x.is_cuda and torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") == torch.bfloat16
+
+
 def _fused(x: torch.Tensor, ln: nn.LayerNorm) -> bool:
-    """Whether the fused kernels take this activation: bf16 autocast on a GPU, fp32 parameters."""
-    return (x.is_cuda and isinstance(ln, _LayerNorm) and torch.is_autocast_enabled("cuda")
-            and torch.get_autocast_dtype("cuda") == torch.bfloat16
-            and ln.weight.dtype == torch.float32 and ln.weight.shape[0] % 8 == 0 and ln.weight.shape[0] <= 1024)
+    """Whether the fused kernels take this activation and the normalisation: bf16 autocast on a GPU, fp32 parameters."""
+    return (_bf16_autocast(x) and untouched(ln, _LayerNorm) and ln.weight.dtype == torch.float32
+            and ln.weight.shape[0] % 8 == 0 and ln.weight.shape[0] <= 1024)
 
 
 def _layer_norm(c: "BertConfig") -> nn.LayerNorm:
@@ -100,12 +104,12 @@ class _Layer(nn.Module):
 
     def forward(self, x):
         b, s, h = x.shape
-        if x.dtype == torch.bfloat16 and _fused(x, self.ln1) and (h // self.heads) % 8 == 0 and x.numel() > 0:
-            p = self.p if self.training else 0.0
-            a = self.proj(_C.attention(self.qkv(x), self.heads, p))
-            x = self._add_norm(self.ln1, x, self.drop(a) if p else a)
-            f = self.fc2(self.fc1(x, "gelu"))
-            return self._add_norm(self.ln2, x, self.drop(f) if p else f)
+        if (x.dtype == torch.bfloat16 and _fused(x, self.ln1) and untouched(self.ln2, _LayerNorm) and (h // self.heads) % 8 == 0
+                and x.numel() > 0):
+            a = self.proj(_C.attention(self.qkv(x), self.heads, self.p if self.training else 0.0))
+            x = self._add_norm(self.ln1, x, dropout(self.drop, a))
+            f = self.fc1(x, "gelu") if untouched(self.fc1, ShadowLinear) else F.gelu(self.fc1(x))
+            return self._add_norm(self.ln2, x, dropout(self.drop, self.fc2(f)))
         q, k, v = self.qkv(x).view(b, s, 3, self.heads, h // self.heads).permute(2, 0, 3, 1, 4)
         a = F.scaled_dot_product_attention(q, k, v, dropout_p=self.p if self.training else 0.0)
         a = a.transpose(1, 2).reshape(b, s, h)
@@ -141,8 +145,8 @@ class BertForQuestionAnswering(nn.Module):
 
     def forward(self, input_ids, start_positions=None, end_positions=None):
         b, s = input_ids.shape
-        if (_fused(self.tok.weight, self.ln) and input_ids.is_cuda and input_ids.dtype == torch.int64
-                and 0 < b * s <= _EMBED_TOKENS and s <= self.pos.num_embeddings):
+        if (plain_embedding(self.tok) and plain_embedding(self.pos) and _fused(self.tok.weight, self.ln)
+                and input_ids.is_cuda and input_ids.dtype == torch.int64 and 0 < b * s <= _EMBED_TOKENS and s <= self.pos.num_embeddings):
             x = _C.embed_layer_norm(input_ids, self.tok.weight, self.pos.weight, self.typ.weight, self.ln.weight,
                                     self.ln.bias, self.ln.eps, wgrad.enabled)
         else:
@@ -151,7 +155,8 @@ class BertForQuestionAnswering(nn.Module):
         x = self.drop(x)
         for layer in self.layers:
             x = layer(x)
-        if (start_positions is not None and x.dtype == torch.bfloat16 and _fused(x, self.ln) and x.numel() > 0
+        if (start_positions is not None and x.dtype == torch.bfloat16 and x.numel() > 0 and _bf16_autocast(x)
+                and untouched(self.qa, nn.Linear) and self.qa.out_features == 2
                 and all(t.is_cuda and t.dtype == torch.int64 and t.dim() == 1 for t in (start_positions, end_positions))):
             logits = _C.linear(x, self.qa.weight, self.qa.bias, None, False)
             return _C.span_loss(logits, start_positions, end_positions)

@@ -6,6 +6,9 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
+from ..ops.fused_linear import ShadowLinear
+from ..ops.modules import untouched
+
 _VGG16_CFG = [64, 64, "M", 128, 128, "M", 256, 256, 256, "M", 512, 512, 512, "M", 512, 512, 512, "M"]
 
 
@@ -38,7 +41,7 @@ class VGG16(nn.Module):
         self.features = nn.Sequential(*layers)
         self.avgpool = nn.AdaptiveAvgPool2d((7, 7))
         if fused_ops:
-            from ..ops.fused_linear import ShadowLinear as Linear  # nn.Linear unless the optimizer keeps bf16 weights
+            Linear = ShadowLinear  # nn.Linear unless the optimizer keeps bf16 weights
         else:
             Linear = nn.Linear
         self.classifier = nn.Sequential(
@@ -124,8 +127,6 @@ class MLP(nn.Module):
 
     def __init__(self, d_in=64, d_hidden=128, d_out=10, depth=3):
         super().__init__()
-        from ..ops.fused_linear import ShadowLinear
-
         dims = [d_in] + [d_hidden] * (depth - 1) + [d_out]
         layers = []
         for i in range(depth):
@@ -137,14 +138,16 @@ class MLP(nn.Module):
         self.net = nn.Sequential(*layers)
 
     def forward(self, x):
-        skip = False
+        if not untouched(self.net, nn.Sequential):
+            return self.net(x)
         layers = list(self.net)
-        for layer, after in zip(layers, layers[1:] + [None]):
-            if skip:
-                skip = False
-            elif type(after) is nn.ReLU and not after._forward_hooks and not after._forward_pre_hooks:
-                x = layer(x, "relu")
-                skip = True
+        k = 0
+        while k < len(layers):
+            # a ReLU is applied by the layer in front of it, where nobody waits for what is between the two
+            if k + 1 < len(layers) and untouched(layers[k], ShadowLinear) and untouched(layers[k + 1], nn.ReLU):
+                x = layers[k](x, "relu")
+                k += 2
             else:
-                x = layer(x)
+                x = layers[k](x)
+                k += 1
         return x

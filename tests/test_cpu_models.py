@@ -51,3 +51,34 @@ def test_bert_residual_stream_stays_in_bf16_under_autocast_and_training_agrees()
     assert all(d == (torch.bfloat16,) for d in seen["new"] if len(d) == 1)
     assert all(d == (torch.float32, torch.float32) for d in seen["old"] if len(d) == 2)
     assert all(abs(a - b) < 3e-2 for a, b in zip(*losses)), losses
+
+
+def test_hooks_of_the_mlp_and_its_modules_fire_and_see_what_their_module_sees():
+    from bagua_core_b200.models import MLP
+
+    torch.manual_seed(0)
+    m, x = MLP(8, 16, 4, depth=3), torch.randn(5, 8)
+    want, seen = m(x), {}
+    for name, module in m.named_modules():
+        if name:
+            module.register_forward_hook(lambda mod, args, out, name=name: seen.setdefault(name, []).append((args[0], out)))
+    assert torch.equal(m(x), want)
+    assert set(seen) == {"net", "net.0", "net.1", "net.2", "net.3", "net.4"} and all(len(v) == 1 for v in seen.values())
+    assert torch.equal(seen["net.0"][0][1], torch.nn.functional.linear(x, m.net[0].weight, m.net[0].bias))  # before the ReLU
+    assert seen["net.1"][0][0] is seen["net.0"][0][1]
+    # one module of a pair alone
+    m = MLP(8, 16, 4, depth=2)
+    out = []
+    m.net[0].register_forward_hook(lambda mod, args, o: out.append(o))
+    m(x)
+    assert bool((out[0] < 0).any())
+    # a global hook, and a layer that was replaced
+    calls = []
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda mod, args, o: calls.append(type(mod).__name__))
+    try:
+        m(x)
+    finally:
+        handle.remove()
+    assert calls.count("ReLU") == 1
+    m.net[0] = torch.nn.Linear(8, 16)
+    assert torch.equal(m(x), m.net(x))

@@ -825,3 +825,45 @@ def test_forward_mode_derivatives_are_those_of_the_plain_composition():
                 torch.manual_seed(n)
                 got.append(fwad.unpack_dual(g(*[fwad.make_dual(t, torch.randn_like(t)) for t in inputs])).tangent)
         assert (got[0].double() - got[1].double()).norm() <= 2e-2 * got[1].double().norm(), n
+
+
+def test_hooks_and_replaced_modules_of_the_encoder_are_respected():
+    import torch.nn as nn
+
+    from bagua_core_b200.models import BertConfig, BertForQuestionAnswering
+
+    torch.manual_seed(4)
+    net = BertForQuestionAnswering(BertConfig(vocab_size=500, hidden=128, layers=2, heads=4, ffn=256, dropout=0.0)).cuda()
+    ids, span = torch.randint(0, 500, (3, 40)).cuda(), torch.randint(0, 40, (3, 2)).cuda()
+
+    def loss():
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            return net(ids, span[:, 0], span[:, 1])
+
+    fused = loss()
+    seen, handles = {}, []
+    for name, module in net.named_modules():
+        if name and name not in ("typ", "layers"):  # its first row is read, it is not called; a list
+            handles.append(module.register_forward_hook(lambda m, a, o, name=name: seen.__setitem__(name, (a[0], o))))
+    plain = loss()
+    assert set(seen) == {n for n, _ in net.named_modules() if n and n not in ("typ", "layers")}
+    assert torch.allclose(fused, plain, rtol=1e-5)
+    assert bool((seen["layers.0.fc1"][1] < -0.2).any())  # what GELU is applied to, and GELU's values are above that
+    for h in handles:
+        h.remove()
+    assert torch.equal(loss(), fused)
+    for name in ("tok", "pos", "ln", "layers.0.ln1", "layers.1.ln2", "layers.0.fc1", "layers.1.drop", "qa"):  # one alone
+        seen.clear()
+        h = net.get_submodule(name).register_forward_hook(lambda m, a, o: seen.__setitem__("out", o))
+        assert torch.allclose(loss(), fused, rtol=1e-5) and seen, name
+        h.remove()
+    inner = net.qa
+    net.qa = nn.Sequential(inner, nn.Identity())
+    assert torch.allclose(loss(), fused, rtol=1e-5)
+    net.qa = inner
+    net.layers[0].drop.p = 0.9  # dropout switched on behind the configuration's back
+    assert not torch.allclose(loss(), fused, rtol=1e-3)
+    net.layers[0].drop.p = 0.0
+    net.tok = nn.Embedding.from_pretrained(net.tok.weight.detach(), freeze=False, padding_idx=int(ids[0, 0]))
+    loss().backward()
+    assert bool((net.tok.weight.grad[ids[0, 0]] == 0).all())
