@@ -8,6 +8,7 @@ parameter, the HBM minimum) instead of torch's multi-tensor loops.
 """
 from __future__ import annotations
 
+from operator import is_
 from typing import List
 
 import torch
@@ -32,7 +33,8 @@ class FlatSGD(torch.optim.Optimizer):
     """torch.optim.SGD semantics (momentum, dampening, weight decay, Nesterov).
 
     Before `with_bagua` attaches it (or for parameters outside any bucket) it updates
-    parameter by parameter with the same kernel.
+    parameter by parameter with the same kernel.  A parameter that was laid out in a flat buffer is stepped
+    with it, in the group that it was in then, as long as the buffer lives.
 
     `bf16_shadow=True`: for buckets of gradients (algorithms that do not communicate weights) the
     step kernel also writes every updated parameter rounded to bf16 into a second flat buffer, and
@@ -50,7 +52,7 @@ class FlatSGD(torch.optim.Optimizer):
         self._flat: List[dict] = []
         self._attached_ids = set()
         self._plan = None   # the flat buffers, laid out for the native step (`_C.SgdPlan`)
-        self._loose = None  # (parameters in the groups, those of them outside the flat buffers)
+        self._loose = None  # (the groups' parameters, [(group index, parameter outside the flat buffers)])
         self._steps = 0
         self.kernel_launches = 0
         # bf16 copies of the weights, written by the step kernel (see bagua_core_b200.ops.shadow)
@@ -145,11 +147,13 @@ class FlatSGD(torch.optim.Optimizer):
         return _C.current_stream(self._flat[0]["p"])
 
     def _loose_params(self):
-        """[(group, parameter)] outside the flat buffers; looked up again when a group has grown."""
-        n = sum(len(g["params"]) for g in self.param_groups)
-        if self._loose is None or self._loose[0] != n:
-            self._loose = (n, [(g, p) for g in self.param_groups for p in g["params"] if id(p) not in self._attached_ids])
-        return self._loose[1]
+        """[(group, parameter)] outside the flat buffers; looked up again when the groups' parameters are others than at
+        the last look (an added, replaced or moved parameter, a loaded state)."""
+        now = [g["params"] for g in self.param_groups]
+        if self._loose is None or len(now) != len(self._loose[0]) or not all(
+                len(a) == len(b) and all(map(is_, a, b)) for a, b in zip(now, self._loose[0])):
+            self._loose = ([list(ps) for ps in now], [(gi, p) for gi, ps in enumerate(now) for p in ps if id(p) not in self._attached_ids])
+        return [(self.param_groups[gi], p) for gi, p in self._loose[1]]
 
     @torch.no_grad()
     def step(self, closure=None):

@@ -229,3 +229,33 @@ def test_replaced_and_missing_gradients_end_up_in_the_bucket():
         assert in1 and in2 and in3
         assert torch.equal(first, third) and not torch.equal(first, second)
         assert int((second == 0).sum()) >= 20  # layer b took no part
+
+
+def test_flat_sgd_steps_the_parameters_that_are_in_its_groups_now():
+    import bagua_core_b200.parallel as P
+
+    def param(v):
+        p = torch.nn.Parameter(torch.full((3,), float(v)))
+        p.grad = torch.ones(3)
+        return p
+
+    a, b, c, d = (param(v) for v in range(4))
+    opt = P.FlatSGD([{"params": [a, b]}, {"params": [c], "lr": 0.5}], lr=0.25)
+    opt.step()
+    opt.param_groups[0]["params"][1] = d  # replaced: as many as before
+    opt.step()
+    assert [p[0].item() for p in (a, b, c, d)] == [-0.5, 0.75, 1.0, 2.75]
+    opt.zero_grad()
+    assert bool((d.grad == 0).all() and (b.grad == 1).all())
+    for p in (a, c, d):
+        p.grad.fill_(1.0)
+    opt.param_groups[0]["params"].pop()  # moved to the other group, in the same order
+    opt.param_groups[1]["params"].insert(0, d)
+    opt.step()
+    assert [p[0].item() for p in (a, c, d)] == [-0.75, 0.5, 2.25]
+    del opt.state[b]
+    state = opt.state_dict()  # a loaded state brings groups of its own
+    state["param_groups"][0]["lr"] = 1.0
+    opt.load_state_dict(state)
+    opt.step()
+    assert [p[0].item() for p in (a, c, d)] == [-1.75, 0.0, 1.75]
