@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstring>
+#include <mutex>
 
 #include "../common.h"
 #include "encoder_ops.h"
@@ -55,14 +57,47 @@ void fold(const float* partial, float* out, int blocks, int C, bool accumulate, 
                     accumulate);
 }
 
+// ---- indices outside their table -------------------------------------------------------------------
+// A kernel skips them and leaves the last one here, in host memory: the value first, then that there is one.
+struct IndexReport {
+  long long value[2];  // by kind: a token's id, a span's target
+  unsigned int seen[2];
+};
+enum { kTokenId = 0, kSpanTarget = 1 };
+__device__ __noinline__ void report_index(IndexReport* r, int kind, int64_t value) {
+  *(volatile long long*)&r->value[kind] = value;
+  __threadfence_system();
+  *(volatile unsigned int*)&r->seen[kind] = 1u;
+}
+// One per device, never given back: a captured graph keeps its address.
+IndexReport* index_report() {
+  static IndexReport* reports[64] = {};
+  static std::mutex mu;
+  int dev = 0;
+  BAGUA_CUDA_CHECK(cudaGetDevice(&dev));
+  BAGUA_CHECK(dev >= 0 && dev < 64, Tensor, "device index " << dev << " out of range");
+  std::lock_guard<std::mutex> g(mu);
+  if (!reports[dev]) {
+    // allowed while a stream is being captured, as nothing is enqueued
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    BAGUA_CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t e = cudaHostAlloc((void**)&reports[dev], sizeof(IndexReport), cudaHostAllocMapped);
+    BAGUA_CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&mode));
+    BAGUA_CUDA_CHECK(e);
+    std::memset(reports[dev], 0, sizeof(IndexReport));
+  }
+  return reports[dev];
+}
+
 // ---- embedding ------------------------------------------------------------------------------------
 // x[row] = (tok[id] + pos[position]) + typ, in this order, in fp32; an id outside the table gives a row of NaN.
 __global__ void __launch_bounds__(kThreads)
     embed_sum_kernel(const int64_t* __restrict__ ids, int64_t vocab, const float* __restrict__ tok, const float* __restrict__ pos,
-                     const float* __restrict__ typ, float* __restrict__ x, int64_t seq, int H) {
+                     const float* __restrict__ typ, float* __restrict__ x, int64_t seq, int H, IndexReport* report) {
   wait_for_predecessor();
   const int64_t row = blockIdx.x, id = ids[row];
   const bool known = id >= 0 && id < vocab;
+  if (!known && threadIdx.x == 0) report_index(report, kTokenId, id);
   const float* t = tok + (known ? id : 0) * H;
   const float* p = pos + (row % seq) * H;
   for (int c = (int)threadIdx.x; c < H; c += kThreads) x[row * H + c] = known ? t[c] + p[c] + typ[c] : nanf("");
@@ -237,7 +272,8 @@ constexpr int kSpanThreads = 1024;
 constexpr int64_t kIgnored = -100;
 __global__ void __launch_bounds__(kSpanThreads)
     span_loss_kernel(const __nv_bfloat162* __restrict__ logits, const int64_t* __restrict__ start,
-                     const int64_t* __restrict__ end, float* __restrict__ loss, float* __restrict__ stats, int batch, int seq) {
+                     const int64_t* __restrict__ end, float* __restrict__ loss, float* __restrict__ stats, int batch, int seq,
+                     IndexReport* report) {
   // stats: [batch][2] log-sum-exp, then the two counts
   __shared__ float s_loss[32][2];
   __shared__ float s_count[32][2];
@@ -268,13 +304,16 @@ __global__ void __launch_bounds__(kSpanThreads)
       stats[2 * b] = lse0;
       stats[2 * b + 1] = lse1;
       const int64_t t0 = start[b], t1 = end[b];
+      const bool in0 = t0 >= 0 && t0 < seq, in1 = t1 >= 0 && t1 < seq;
       if (t0 != kIgnored) {
-        l[0] += t0 >= 0 && t0 < seq ? lse0 - __bfloat162float(row[t0].x) : nanf("");
+        l[0] += in0 ? lse0 - __bfloat162float(row[t0].x) : nanf("");
         n[0] += 1.f;
+        if (!in0) report_index(report, kSpanTarget, t0);
       }
       if (t1 != kIgnored) {
-        l[1] += t1 >= 0 && t1 < seq ? lse1 - __bfloat162float(row[t1].y) : nanf("");
+        l[1] += in1 ? lse1 - __bfloat162float(row[t1].y) : nanf("");
         n[1] += 1.f;
+        if (!in1) report_index(report, kSpanTarget, t1);
       }
     }
   }
@@ -340,9 +379,22 @@ __global__ void __launch_bounds__(kThreads)
 
 }  // namespace
 
+void check_indices() {
+  IndexReport* r = index_report();
+  for (int kind : {kTokenId, kSpanTarget}) {
+    volatile unsigned int* seen = &r->seen[kind];
+    if (*seen == 0) continue;
+    const long long value = *(volatile long long*)&r->value[kind];
+    *seen = 0;
+    throw BaguaError(ErrorKind::Tensor, (kind == kTokenId ? "an earlier call was given the token id " : "an earlier call was given the span target ") +
+                                            std::to_string(value) + (kind == kTokenId ? ", which is not in the table" : ", which is not in the sequence"));
+  }
+}
+
 void embed_sum(const int64_t* ids, int64_t vocab, const float* tok, const float* pos, const float* typ, float* x, int64_t batch,
                int64_t seq, int H, cudaStream_t s) {
-  launch_overlapped(embed_sum_kernel, dim3((unsigned)(batch * seq)), dim3(kThreads), s, ids, vocab, tok, pos, typ, x, seq, H);
+  launch_overlapped(embed_sum_kernel, dim3((unsigned)(batch * seq)), dim3(kThreads), s, ids, vocab, tok, pos, typ, x, seq, H,
+                    index_report());
 }
 
 size_t embed_backward_scratch_bytes(int64_t rows, int H) { return (size_t)column_slices(rows, H) * H * sizeof(float); }
@@ -391,7 +443,7 @@ void span_loss_forward(const void* logits, const int64_t* start, const int64_t* 
                        int64_t seq, cudaStream_t s) {
   BAGUA_CHECK(batch > 0 && seq > 0 && batch * seq < (1ll << 30), Tensor, "span loss: unsupported shape");
   launch_overlapped(span_loss_kernel, dim3(1), dim3(kSpanThreads), s, (const __nv_bfloat162*)logits, start, end, loss, stats,
-                    (int)batch, (int)seq);
+                    (int)batch, (int)seq, index_report());
 }
 void span_loss_backward(const void* logits, const int64_t* start, const int64_t* end, const float* stats, const float* dloss,
                         void* dlogits, int64_t batch, int64_t seq, cudaStream_t s) {

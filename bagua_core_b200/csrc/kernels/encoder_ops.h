@@ -17,6 +17,11 @@
 namespace bagua {
 namespace encoder_ops {
 
+// Throws if a kernel on the current device has met a token id outside its table or a span target outside its sequence since
+// the last look.  Such a call goes on with NaN in the index's place; the error comes with the next one whose host side
+// looks after the kernel ran, as with any error that a device finds.
+void check_indices();
+
 // x = tok[ids] + pos[position] + typ[0] in fp32, ids [batch, seq].  An id outside [0, vocab) gives a row of NaN and no
 // gradient.
 void embed_sum(const int64_t* ids, int64_t vocab, const float* tok, const float* pos, const float* typ, float* x, int64_t batch,

@@ -613,6 +613,7 @@ struct EmbedNode : public EncoderNode {
     variable_list out(5);
     uses_done();
     if (!grads[0].defined()) return out;
+    encoder_ops::check_indices();
     const at::Tensor id = ids.unpack(), s = sum.unpack();
     const int H = (int)param[0].size(1);
     const int64_t batch = id.size(0), seq = id.size(1);
@@ -897,6 +898,7 @@ at::Tensor embed_layer_norm(const at::Tensor& ids, const at::Tensor& tok, const 
     node = std::shared_ptr<EmbedNode>(new EmbedNode(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(tok, pos, typ, gamma, beta));
   }
+  encoder_ops::check_indices();
   at::Tensor idc, sum, mean, rstd;
   std::array<at::Tensor, 1> y;
   {
@@ -944,6 +946,7 @@ at::Tensor span_loss(const at::Tensor& logits, const at::Tensor& start, const at
     node = std::shared_ptr<SpanLossNode>(new SpanLossNode(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(logits));
   }
+  encoder_ops::check_indices();
   at::Tensor x, a, b, loss, stats;
   {
     PlainDispatch plain;

@@ -867,3 +867,31 @@ def test_hooks_and_replaced_modules_of_the_encoder_are_respected():
     net.tok = nn.Embedding.from_pretrained(net.tok.weight.detach(), freeze=False, padding_idx=int(ids[0, 0]))
     loss().backward()
     assert bool((net.tok.weight.grad[ids[0, 0]] == 0).all())
+
+
+@pytest.mark.parametrize("bad", ["token", "negative token", "start", "end"])
+def test_an_index_outside_its_table_is_an_error(bad):
+    """The kernels skip it; the first look of the host behind it says so, and the call after that works again."""
+    from bagua_core_b200.models import BertConfig, BertForQuestionAnswering
+
+    net = BertForQuestionAnswering(BertConfig.tiny()).cuda().eval()
+    good, span = torch.randint(0, 1000, (2, 16)).cuda(), torch.randint(0, 16, (2, 2)).cuda()
+    ids, where = good.clone(), span.clone()
+    if bad.endswith("token"):
+        ids[1, 3] = 1000 if bad == "token" else -1
+    else:
+        where[0, int(bad == "end")] = 16
+
+    def loss(i, w):
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            return net(i, w[:, 0], w[:, 1])
+
+    want = loss(good, span)
+    with pytest.raises(RuntimeError, match="which is not in the"):
+        assert torch.isnan(loss(ids, where))  # (waits for it, unless it has been noticed already)
+        loss(good, span)
+    assert torch.equal(loss(good, span), want)
+    where[:, 0] = -100  # counts for nothing, and is no error
+    loss(good, torch.where(where == 16, 0, where))
+    torch.cuda.synchronize()
+    assert torch.equal(loss(good, span), want)
