@@ -1,5 +1,6 @@
 #include "gemm.h"
 
+#include <ATen/Context.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <cublasLt.h>
 
@@ -15,16 +16,29 @@ namespace gemm {
 
 namespace {
 
-// With this workspace (and the bias counted as an operand to be aligned) the library picks the forward product's
-// algorithm as the framework has it picked: the activations, and with them the ReLU masks and everything
-// behind, keep their bits.  Gradients have no such edges and may use more.
-constexpr size_t kForwardWorkspace = 1u << 20, kWorkspace = 32u << 20;
+// The forward product has the framework's own workspace (1 MB unless CUBLASLT_WORKSPACE_SIZE says otherwise) and counts its
+// bias as an operand to be aligned, so that the library picks the algorithm that the framework's layer has: the activations,
+// and with them the ReLU masks and everything behind, keep their bits.  (Without a bias the framework goes through another
+// of the library's interfaces and may get another algorithm.)  Gradients have no such edges and may use more.
+constexpr size_t kGradientWorkspace = 32u << 20;
+size_t workspace_bytes(bool forward) { return forward ? at::cuda::getCUDABlasLtWorkspaceSize() : kGradientWorkspace; }
+
+// How partial sums over parts of k may be added up: torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction.
+uint32_t reduction_schemes(at::CuBLASReductionOption option) {
+  switch (option) {
+    case at::CuBLASReductionOption::AllowReducedPrecisionWithSplitK: return CUBLASLT_REDUCTION_SCHEME_MASK;
+    case at::CuBLASReductionOption::DisallowReducedPrecisionAllowSplitK: return CUBLASLT_REDUCTION_SCHEME_COMPUTE_TYPE;
+    default: return CUBLASLT_REDUCTION_SCHEME_NONE;
+  }
+}
+
 constexpr size_t kMaxPlans = 512;  // per thread; a program with more shapes than that starts over
 
 struct Key {
   int kind, device;
   int64_t m, n, k;
-  // whether there is a bias or an addition, and how the operands are aligned (in powers of two up to 256)
+  // whether there is a bias or an addition, how the operands are aligned (in powers of two up to 256) and how partial sums
+  // may be added
   uint32_t flags;
   bool operator==(const Key& o) const { return std::memcmp(this, &o, sizeof(Key)) == 0; }
 };
@@ -64,7 +78,8 @@ struct Problem {
   bool d_fp32, bias, forward, relu;
 };
 
-bool build(Plan& p, cublasLtHandle_t lt, const Problem& q, const void* A, const void* B, const void* D, const void* bias) {
+bool build(Plan& p, cublasLtHandle_t lt, const Problem& q, const void* A, const void* B, const void* D, const void* bias,
+           at::CuBLASReductionOption reductions) {
   auto ok = [](cublasStatus_t s) { return s == CUBLAS_STATUS_SUCCESS; };
   if (!ok(cublasLtMatmulDescCreate(&p.desc, CUBLAS_COMPUTE_32F, CUDA_R_32F))) return false;
   auto set = [&](cublasLtMatmulDescAttributes_t at, const void* v, size_t n) {
@@ -89,7 +104,8 @@ bool build(Plan& p, cublasLtHandle_t lt, const Problem& q, const void* A, const 
     return false;
   cublasLtMatmulPreference_t pref = nullptr;
   if (!ok(cublasLtMatmulPreferenceCreate(&pref))) return false;
-  const size_t ws = q.forward ? kForwardWorkspace : kWorkspace;
+  const size_t ws = workspace_bytes(q.forward);
+  const uint32_t schemes = reduction_schemes(reductions);
   const uint32_t al[4] = {1u << alignment_log(A), 1u << alignment_log(B), 1u << alignment_log(D),
                           1u << alignment_log(q.bias ? bias : D)};
   cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_MAX_WORKSPACE_BYTES, &ws, sizeof(ws));
@@ -97,6 +113,7 @@ bool build(Plan& p, cublasLtHandle_t lt, const Problem& q, const void* A, const 
   cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_B_BYTES, &al[1], 4);
   cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_C_BYTES, &al[2], 4);
   cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_D_BYTES, &al[3], 4);
+  cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_REDUCTION_SCHEME_MASK, &schemes, sizeof(schemes));
   cublasLtMatmulHeuristicResult_t best;
   int found = 0;
   const cublasStatus_t s = cublasLtMatmulAlgoGetHeuristic(lt, p.desc, p.a, p.b, p.d, p.d, pref, 1, &best, &found);
@@ -117,7 +134,8 @@ bool run(int kind, const Problem& q, int64_t m, int64_t n, int64_t k, const at::
   key.m = m;
   key.n = n;
   key.k = k;
-  key.flags = (q.bias ? 1u : 0u) | (add ? 2u : 0u) | (q.relu ? 4u : 0u) | (alignment_log(A.data_ptr()) << 4) | (alignment_log(B.data_ptr()) << 8) |
+  const at::CuBLASReductionOption reductions = at::globalContext().allowBF16ReductionCuBLAS();
+  key.flags = ((uint32_t)reductions << 20) | (q.bias ? 1u : 0u) | (add ? 2u : 0u) | (q.relu ? 4u : 0u) | (alignment_log(A.data_ptr()) << 4) | (alignment_log(B.data_ptr()) << 8) |
               (alignment_log(D.data_ptr()) << 12) | (q.bias ? alignment_log(bias) << 16 : 0u);
   // per thread: a plan's descriptor carries the bias pointer of the call
   using Plans = std::unordered_map<Key, std::unique_ptr<Plan>, Hash>;
@@ -127,7 +145,7 @@ bool run(int kind, const Problem& q, int64_t m, int64_t n, int64_t k, const at::
   if (it == plans->end()) {
     if (plans->size() >= kMaxPlans) plans->clear();
     auto p = std::make_unique<Plan>();
-    p->usable = build(*p, lt, q, A.data_ptr(), B.data_ptr(), D.data_ptr(), bias);
+    p->usable = build(*p, lt, q, A.data_ptr(), B.data_ptr(), D.data_ptr(), bias, reductions);
     it = plans->emplace(key, std::move(p)).first;
   }
   Plan& p = *it->second;
@@ -136,7 +154,7 @@ bool run(int kind, const Problem& q, int64_t m, int64_t n, int64_t k, const at::
       cublasLtMatmulDescSetAttribute(p.desc, CUBLASLT_MATMUL_DESC_BIAS_POINTER, &bias, sizeof(bias)) != CUBLAS_STATUS_SUCCESS)
     return false;
   cudaStream_t s = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();
-  const size_t bytes = q.forward ? kForwardWorkspace : kWorkspace;
+  const size_t bytes = workspace_bytes(q.forward);
   auto ws = MemoryPool::for_device(device).pull(bytes, (uint64_t)(uintptr_t)s);
   const float one = 1.f, beta = add ? 1.f : 0.f;
   if (cublasLtMatmul(lt, p.desc, &one, A.data_ptr(), p.a, B.data_ptr(), p.b, &beta, D.data_ptr(), p.d, D.data_ptr(), p.d,

@@ -895,3 +895,26 @@ def test_an_index_outside_its_table_is_an_error(bad):
     loss(good, torch.where(where == 16, 0, where))
     torch.cuda.synchronize()
     assert torch.equal(loss(good, span), want)
+
+
+def test_linear_follows_the_frameworks_switch_for_partial_sums():
+    """The rows are few and k is long, so the library splits k: with the switch off no partial sum is rounded to bf16."""
+    import bagua_core_b200 as bb
+
+    settings, saved = torch.backends.cuda.matmul, torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction
+    try:
+        for M, K, N in ((32, 25088, 4096), (5, 30000, 128), (64, 128, 128), (384, 1024, 4096)):
+            torch.manual_seed(K)
+            x, w = torch.randn(M, K, device="cuda").bfloat16().requires_grad_(), torch.randn(N, K, device="cuda").bfloat16()
+            b = torch.randn(N, device="cuda").bfloat16()
+            for allow in (True, False, True):
+                settings.allow_bf16_reduced_precision_reduction = allow
+                y, ref = bb._C.linear(x, w, b, None, False), torch.nn.functional.linear(x, w, b)
+                assert torch.equal(y, ref), (M, K, N, allow)
+                dy = torch.randn_like(y)
+                (dx,) = torch.autograd.grad(y, x, dy)
+                exact = dy.double() @ w.double()
+                if not allow:  # one rounding of the result, and fp32 sums
+                    assert ((dx.double() - exact).abs() <= 2 ** -8 * exact.abs() + 1e-4 * exact.abs().max()).all()
+    finally:
+        settings.allow_bf16_reduced_precision_reduction = saved
