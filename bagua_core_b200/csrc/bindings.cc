@@ -21,6 +21,7 @@
 #include "kernels/fused.h"
 #include "kernels/fused_emu.h"
 #include "kernels/kernels.h"
+#include "kernels/encoder_ops.h"
 #include "kernels/model_ops.h"
 #include "ops/comm_op.h"
 #include "pool/resource_pool.h"
@@ -934,6 +935,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("embed_layer_norm", &trainer::embed_layer_norm, py::arg("ids"), py::arg("tokens"), py::arg("positions"),
         py::arg("types"), py::arg("weight"), py::arg("bias"), py::arg("eps"), py::arg("accumulate"),
         "layer_norm(tokens[ids] + positions[:seq] + types[0]) in bf16.");
+  m.attr("max_embedding_tokens") = encoder_ops::kMaxTokens;
   m.def("attention", &trainer::attention, py::arg("qkv"), py::arg("heads"), py::arg("dropout"),
         "Multi-head attention of a packed bf16 projection (the attention kernel is the library's).");
   m.def("op_stats", []() {

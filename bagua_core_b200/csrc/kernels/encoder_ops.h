@@ -29,7 +29,13 @@ void embed_sum(const int64_t* ids, int64_t vocab, const float* tok, const float*
 // The tables' gradients from dx [batch * seq, H], ADDED to dtok [vocab, H], dpos [>= seq, H] and dtyp [H], each of which
 // may be null.  Rows of one token are summed in order up to kMaxOrdered occurrences; beyond that, slices of that length are
 // added atomically.  Returns the number of kernels launched.
-constexpr int kMaxTokens = 4096, kMaxOrdered = 256;
+//
+// kMaxTokens: every block looks over all ids, so the scatter grows with the square of the tokens and the dense path, which
+// also writes the whole table, does not.  Embedding and normalisation in both directions, this / the framework's, us: 30522 rows
+// of 1024: 4096 tokens 127 / 452, 8192 281 / 627, 16384 676 / 1022, 32768 1716 / 1660; rows of 256: 104 / 358, 182 / 367,
+// 465 / 457, 1383 / 740; 1000 rows of 64: 102 / 350, 140 / 353, 217 / 353, 467 / 465.  The line is the last of these at which
+// this path is well ahead at every width.
+constexpr int kMaxTokens = 8192, kMaxOrdered = 256;
 size_t embed_backward_scratch_bytes(int64_t rows, int H);
 int embed_backward(const float* dx, const int64_t* ids, int64_t vocab, float* dtok, float* dpos, float* dtyp, void* scratch,
                    int64_t batch, int64_t seq, int H, cudaStream_t s);

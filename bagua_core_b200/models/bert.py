@@ -26,7 +26,7 @@ from ..ops.fused_linear import ShadowLinear
 from ..ops.modules import dropout, plain_embedding, untouched
 
 
-_EMBED_TOKENS = 4096  # encoder_ops::kMaxTokens: more tokens per batch take the framework's embedding
+_EMBED_TOKENS = _C.max_embedding_tokens  # more tokens per batch take the framework's embedding
 
 
 @dataclass

@@ -918,3 +918,8 @@ def test_linear_follows_the_frameworks_switch_for_partial_sums():
                     assert ((dx.double() - exact).abs() <= 2 ** -8 * exact.abs() + 1e-4 * exact.abs().max()).all()
     finally:
         settings.allow_bf16_reduced_precision_reduction = saved
+
+
+@pytest.mark.parametrize("batch,seq,V,same", [(16, 512, 30522, 0), (16, 512, 1000, 6000), (16, 384, 50, 0)])
+def test_embedding_at_the_largest_batches_of_its_range(batch, seq, V, same):
+    test_embedding_sum_and_norm_match_the_plain_composition(batch, seq, V, same)
