@@ -923,3 +923,30 @@ def test_linear_follows_the_frameworks_switch_for_partial_sums():
 @pytest.mark.parametrize("batch,seq,V,same", [(16, 512, 30522, 0), (16, 512, 1000, 6000), (16, 384, 50, 0)])
 def test_embedding_at_the_largest_batches_of_its_range(batch, seq, V, same):
     test_embedding_sum_and_norm_match_the_plain_composition(batch, seq, V, same)
+
+
+@pytest.mark.parametrize("hidden", [1032, 1536])
+def test_encoders_wider_than_1024_run_fused_and_agree_with_the_plain_composition(hidden):
+    from bagua_core_b200.models import BertConfig, BertForQuestionAnswering, bert
+
+    torch.manual_seed(4)
+    net = BertForQuestionAnswering(BertConfig(vocab_size=300, hidden=hidden, layers=1, heads=3 if hidden % 24 == 0 and hidden < 1100 else 12,
+                                              ffn=264, dropout=0.0)).cuda()
+    ids, span = torch.randint(0, 300, (2, 40)).cuda(), torch.randint(0, 40, (2, 2)).cuda()
+    out, saved = [], bert._fused
+    try:
+        for fused in (True, False):
+            if not fused:
+                bert._fused = lambda x, ln: False
+            net.zero_grad()
+            before = bb_launches()
+            with torch.autocast("cuda", dtype=torch.bfloat16):
+                loss = net(ids, span[:, 0], span[:, 1])
+            assert not fused or bb_launches() - before >= 6  # embedding, two normalisations' casts, GELU, output layer, loss
+            loss.backward()
+            out.append((loss.detach(), torch.cat([p.grad.flatten() for p in net.parameters()])))
+    finally:
+        bert._fused = saved
+    (la, ga), (lb, gb) = out
+    assert torch.allclose(la, lb, rtol=1e-5)
+    assert (ga - gb).norm() <= 1e-2 * gb.norm()
