@@ -119,7 +119,7 @@ class _Layer(nn.Module):
 
     @staticmethod
     def _add_norm(ln, x, branch):
-        return _C.add_layer_norm(x, branch, ln.weight, ln.bias, ln.eps, wgrad.enabled)
+        return _C.add_layer_norm(x, branch, ln.weight, ln.bias, ln.eps, wgrad.active())
 
 
 class BertForQuestionAnswering(nn.Module):
@@ -148,7 +148,7 @@ class BertForQuestionAnswering(nn.Module):
         if (plain_embedding(self.tok) and plain_embedding(self.pos) and _fused(self.tok.weight, self.ln)
                 and input_ids.is_cuda and input_ids.dtype == torch.int64 and 0 < b * s <= _EMBED_TOKENS and s <= self.pos.num_embeddings):
             x = _C.embed_layer_norm(input_ids, self.tok.weight, self.pos.weight, self.typ.weight, self.ln.weight,
-                                    self.ln.bias, self.ln.eps, wgrad.enabled)
+                                    self.ln.bias, self.ln.eps, wgrad.active())
         else:
             pos = torch.arange(s, device=input_ids.device)
             x = self.ln(self.tok(input_ids) + self.pos(pos)[None] + self.typ.weight[0][None, None])

@@ -50,7 +50,7 @@ class _ConvBiasReLUFn:
     @staticmethod
     def apply(x, weight, bias, stride, padding, dilation, groups):
         return _C.conv_bias_relu(x, weight, bias, stride, padding, dilation, groups, False,
-                                 _shadow.autocast_copy(weight), _wgrad.enabled)
+                                 _shadow.autocast_copy(weight), _wgrad.active())
 
 
 class _ConvBiasReLUPoolFn:
@@ -61,7 +61,7 @@ class _ConvBiasReLUPoolFn:
     @staticmethod
     def apply(x, weight, bias, stride, padding, dilation, groups):
         return _C.conv_bias_relu(x, weight, bias, stride, padding, dilation, groups, True,
-                                 _shadow.autocast_copy(weight), _wgrad.enabled)
+                                 _shadow.autocast_copy(weight), _wgrad.active())
 
 
 class _MaxPool2x2Fn(torch.autograd.Function):

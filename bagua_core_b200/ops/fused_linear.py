@@ -43,7 +43,7 @@ class ShadowLinear(nn.Linear):
             else:
                 code = 0
             y = _C.linear(x, self.weight, self.bias, _shadow.autocast_copy(self.weight),
-                          _wgrad.enabled and self.accumulate_in_place, code)
+                          self.accumulate_in_place and _wgrad.active(), code)
         else:
             y = super().forward(x)
         return y if act is None else act(y)

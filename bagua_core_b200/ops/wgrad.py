@@ -15,7 +15,8 @@ gradients with the kernel that reduces them.  The parameter's post-accumulate-gr
 runs them when it reaches the parameter even without a gradient.  The ordinary path is taken whenever the
 shortcut would change what the user sees:
 
-* the feature is off (`enabled`, default False), or a higher-order graph is being built;
+* the feature is off (`enabled`, default False), autograd turns out not to run the hooks of a parameter that got
+  no gradient (`active`), or a higher-order graph is being built;
 * the backward pass returns the gradient instead of accumulating it (`torch.autograd.grad`);
 * `.grad` is missing, not fp32, not contiguous or of another shape;
 * the parameter has tensor hooks (`register_hook`), which autograd would apply to the gradient;
@@ -40,6 +41,11 @@ from .._native import C as _C
 
 # Off by default.
 enabled = False
+
+
+def active() -> bool:
+    """Whether gradients may be added in place: `enabled`, and a bucket would still learn of them."""
+    return enabled and _autograd_runs_hooks_without_a_gradient()
 
 
 def __getattr__(name):
@@ -71,12 +77,15 @@ def _autograd_runs_hooks_without_a_gradient() -> bool:
             def backward(ctx, dy):
                 return dy, None
 
-        with torch.enable_grad():
-            w = torch.nn.Parameter(torch.ones(3))
-            w.grad = torch.zeros(3)
-            handle = w.register_post_accumulate_grad_hook(lambda p: fired.append(1))
-            x = torch.ones(3, requires_grad=True)
-            _Probe.apply(x, w).sum().backward()
-            handle.remove()
+        try:
+            with torch.inference_mode(False), torch.enable_grad():
+                w = torch.nn.Parameter(torch.ones(3, device="cpu"))
+                w.grad = torch.zeros(3, device="cpu")
+                handle = w.register_post_accumulate_grad_hook(lambda p: fired.append(1))
+                x = torch.ones(3, device="cpu", requires_grad=True)
+                _Probe.apply(x, w).sum().backward()
+                handle.remove()
+        except RuntimeError:  # a transform of torch.func is looking on: not found out yet
+            return False
         _hooks_run_anyway = bool(fired)
     return _hooks_run_anyway

@@ -300,3 +300,15 @@ def test_who_looks_at_the_operations_sees_the_plain_composition(wgrad):
         assert torch.allclose(tangents[0].float(), tangents[1].float(), rtol=2e-2, atol=2e-2)
         assert flops[0] == flops[1] > 0
         assert torch.allclose(mapped[0].float(), mapped[1].float(), rtol=2e-2, atol=2e-2)
+
+
+def test_nothing_is_added_in_place_where_autograd_would_not_run_the_hooks(wgrad, monkeypatch):
+    m, _ = _pair(10)
+    monkeypatch.setattr(wgrad, "_hooks_run_anyway", False)
+    a0 = wgrad.accumulated
+    _backward(m, torch.randn(5, 48))
+    assert not wgrad.active() and wgrad.accumulated == a0 and bool((m.weight.grad != 0).any())
+    monkeypatch.setattr(wgrad, "_hooks_run_anyway", None)
+    m.weight.grad.zero_()
+    _backward(m, torch.randn(5, 48))
+    assert wgrad.active() and wgrad.accumulated == a0 + 1
