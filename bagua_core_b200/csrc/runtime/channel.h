@@ -130,18 +130,6 @@ class Channel {
     not_full_.notify_one();
     return v;
   }
-  // 0 = got a value, 1 = timed out, 2 = closed
-  int recv_timeout(std::chrono::milliseconds d, T* out) {
-    std::unique_lock<std::mutex> lk(mu_);
-    if (!not_empty_.wait_for(lk, d, [&] { return closed_ || !q_.empty(); })) return 1;
-    if (q_.empty()) return 2;
-    *out = std::move(q_.front());
-    q_.pop_front();
-    size_.store(q_.size(), std::memory_order_release);
-    lk.unlock();
-    not_full_.notify_one();
-    return 0;
-  }
   void close() {
     {
       std::lock_guard<std::mutex> g(mu_);
