@@ -123,7 +123,8 @@ class ResNet50(nn.Module):
 
 
 class MLP(nn.Module):
-    """Small model for tests and smoke runs.  Its layers are `ShadowLinear`, as in the other models."""
+    """Small model for tests and smoke runs.  Its layers are `ShadowLinear`, as in the other models: natively under bf16
+    autocast where `ops.wgrad.enabled` is set or an optimizer keeps bf16 weights, `nn.Linear` otherwise."""
 
     def __init__(self, d_in=64, d_hidden=128, d_out=10, depth=3):
         super().__init__()
@@ -131,7 +132,9 @@ class MLP(nn.Module):
         layers = []
         for i in range(depth):
             layers.append(ShadowLinear(dims[i], dims[i + 1]))
-            # the gradients of `nn.Linear`, bit for bit: so small a network repeats its steps exactly
+            # Weight gradients rounded to bf16 on their way, as `nn.Linear`'s.  (Not all of its bits: natively the bias
+            # gradient is summed and kept in fp32, and the input gradient's product may be another of the library's.)
+            # Left in fp32 they are more precise, but the next step's ReLU masks notice.
             layers[-1].accumulate_in_place = False
             if i < depth - 1:
                 layers.append(nn.ReLU())
