@@ -637,6 +637,11 @@ __global__ void __launch_bounds__(kDqThreads)
   let_successor_start();
 }
 
+// Over one rank this runs beside a backward pass, as a cooperative launch that starts when all its blocks fit.  It takes
+// all the blocks it can use all the same: unlike the exchange between ranks (fused_bytegrad.cu, 32 blocks) it waits for no
+// peer, and is gone sooner than a smaller launch that occupies fewer SMs for longer.  Training steps with ByteGrad, us, with all
+// (160 blocks for 10 MB) / 148 / 64 / 32 / 16: VGG-16, batch 32: 4771 / 4766 / 4756 / 4844 / 5276; 8 layers of BERT-large, 8 x 384
+// tokens: 5000 / 5113-5540 / 5041 / 5162 / 5350.
 template <typename T>
 void quantise_twice_t(void* x, int64_t n, void* scratch, size_t scratch_bytes, cudaStream_t s) {
   const Split d = split_chunks(1, n * (int64_t)sizeof(T), true, sm_count());
