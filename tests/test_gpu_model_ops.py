@@ -950,3 +950,28 @@ def test_encoders_wider_than_1024_run_fused_and_agree_with_the_plain_composition
     (la, ga), (lb, gb) = out
     assert torch.allclose(la, lb, rtol=1e-5)
     assert (ga - gb).norm() <= 1e-2 * gb.norm()
+
+
+@pytest.mark.parametrize("batch,seq,hidden,heads,layers", [(2, 33, 128, 4, 2), (8, 384, 1024, 16, 2)])
+def test_the_fused_encoder_has_the_bits_of_the_plain_composition(batch, seq, hidden, heads, layers):
+    """From the ids to the logits every operation rounds where the framework's rounds; the loss, whose sums over rows and
+    positions are taken in another order, agrees to fp32 rounding."""
+    from bagua_core_b200.models import BertConfig, BertForQuestionAnswering, bert
+    from bagua_core_b200.ops import wgrad as W
+
+    torch.manual_seed(2)
+    net = BertForQuestionAnswering(BertConfig(vocab_size=3000, hidden=hidden, heads=heads, ffn=4 * hidden, layers=layers, dropout=0.0)).cuda()
+    ids, span = torch.randint(0, 3000, (batch, seq)).cuda(), torch.randint(0, seq, (batch, 2)).cuda()
+    saved, out = (bert._fused, W.enabled), []
+    try:
+        for mode in ("plain", "fused", "fused, in place"):
+            bert._fused = (lambda x, ln: False) if mode == "plain" else saved[0]
+            W.enabled = mode.endswith("in place")
+            with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+                out.append((*net(ids), net(ids, span[:, 0], span[:, 1])))
+    finally:
+        bert._fused, W.enabled = saved
+    plain_loss = (torch.nn.functional.cross_entropy(out[0][0], span[:, 0]) + torch.nn.functional.cross_entropy(out[0][1], span[:, 1])) / 2
+    for start, end, loss in out[1:]:
+        assert torch.equal(start, out[0][0]) and torch.equal(end, out[0][1])
+        assert torch.allclose(loss, plain_loss, rtol=1e-6, atol=0)
