@@ -21,7 +21,6 @@ namespace {
 // and with them the ReLU masks and everything behind, keep their bits.  (Without a bias the framework goes through another
 // of the library's interfaces and may get another algorithm.)  Gradients have no such edges and may use more.
 constexpr size_t kGradientWorkspace = 32u << 20;
-size_t workspace_bytes(bool forward) { return forward ? at::cuda::getCUDABlasLtWorkspaceSize() : kGradientWorkspace; }
 
 // How partial sums over parts of k may be added up: torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction.
 uint32_t reduction_schemes(at::CuBLASReductionOption option) {
@@ -54,6 +53,7 @@ struct Plan {
   cublasLtMatmulDesc_t desc = nullptr;
   cublasLtMatrixLayout_t a = nullptr, b = nullptr, d = nullptr;
   cublasLtMatmulAlgo_t algo;
+  size_t workspace = 0;
   bool usable = false;
   Plan() = default;
   Plan(const Plan&) = delete;
@@ -104,11 +104,12 @@ bool build(Plan& p, cublasLtHandle_t lt, const Problem& q, const void* A, const 
     return false;
   cublasLtMatmulPreference_t pref = nullptr;
   if (!ok(cublasLtMatmulPreferenceCreate(&pref))) return false;
-  const size_t ws = workspace_bytes(q.forward);
+  // (the framework's is read from the environment at each call, which takes longer than the rest of a launch)
+  p.workspace = q.forward ? at::cuda::getCUDABlasLtWorkspaceSize() : kGradientWorkspace;
   const uint32_t schemes = reduction_schemes(reductions);
   const uint32_t al[4] = {1u << alignment_log(A), 1u << alignment_log(B), 1u << alignment_log(D),
                           1u << alignment_log(q.bias ? bias : D)};
-  cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_MAX_WORKSPACE_BYTES, &ws, sizeof(ws));
+  cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_MAX_WORKSPACE_BYTES, &p.workspace, sizeof(p.workspace));
   cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_A_BYTES, &al[0], 4);
   cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_B_BYTES, &al[1], 4);
   cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_C_BYTES, &al[2], 4);
@@ -154,11 +155,10 @@ bool run(int kind, const Problem& q, int64_t m, int64_t n, int64_t k, const at::
       cublasLtMatmulDescSetAttribute(p.desc, CUBLASLT_MATMUL_DESC_BIAS_POINTER, &bias, sizeof(bias)) != CUBLAS_STATUS_SUCCESS)
     return false;
   cudaStream_t s = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();
-  const size_t bytes = workspace_bytes(q.forward);
-  auto ws = MemoryPool::for_device(device).pull(bytes, (uint64_t)(uintptr_t)s);
+  auto ws = MemoryPool::for_device(device).pull(p.workspace, (uint64_t)(uintptr_t)s);
   const float one = 1.f, beta = add ? 1.f : 0.f;
   if (cublasLtMatmul(lt, p.desc, &one, A.data_ptr(), p.a, B.data_ptr(), p.b, &beta, D.data_ptr(), p.d, D.data_ptr(), p.d,
-                     &p.algo, ws->ptr(), bytes, s) == CUBLAS_STATUS_SUCCESS)
+                     &p.algo, ws->ptr(), p.workspace, s) == CUBLAS_STATUS_SUCCESS)
     return true;
   p.usable = false;
   return false;
