@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <mutex>
 
@@ -71,22 +72,25 @@ __device__ __noinline__ void report_index(IndexReport* r, int kind, int64_t valu
 }
 // One per device, never given back: a captured graph keeps its address.
 IndexReport* index_report() {
-  static IndexReport* reports[64] = {};
+  static std::atomic<IndexReport*> reports[64] = {};
   static std::mutex mu;
   int dev = 0;
   BAGUA_CUDA_CHECK(cudaGetDevice(&dev));
   BAGUA_CHECK(dev >= 0 && dev < 64, Tensor, "device index " << dev << " out of range");
+  if (IndexReport* r = reports[dev].load(std::memory_order_acquire)) return r;
   std::lock_guard<std::mutex> g(mu);
-  if (!reports[dev]) {
+  if (!reports[dev].load()) {
     // allowed while a stream is being captured, as nothing is enqueued
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     BAGUA_CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&mode));
-    const cudaError_t e = cudaHostAlloc((void**)&reports[dev], sizeof(IndexReport), cudaHostAllocMapped);
+    IndexReport* r = nullptr;
+    const cudaError_t e = cudaHostAlloc((void**)&r, sizeof(IndexReport), cudaHostAllocMapped);
     BAGUA_CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&mode));
     BAGUA_CUDA_CHECK(e);
-    std::memset(reports[dev], 0, sizeof(IndexReport));
+    std::memset(r, 0, sizeof(IndexReport));
+    reports[dev].store(r, std::memory_order_release);
   }
-  return reports[dev];
+  return reports[dev].load();
 }
 
 // ---- embedding ------------------------------------------------------------------------------------

@@ -314,7 +314,8 @@ at::Tensor linear_composition(const std::vector<at::Tensor>& in, int activation)
 }
 
 struct LinearNode : public AccumulatingNode {
-  SavedVariable x, w, b, z;  // b: in bf16; z: what gelu was applied to, or the ReLU's result
+  SavedVariable x, w, z;  // z: what gelu was applied to, or the ReLU's result
+  at::Tensor b;  // with an activation: the bias in bf16, for a second backward pass
   at::Tensor weight, bias;  // the parameters (bias may be undefined)
   int activation = kNone;
 
@@ -325,8 +326,8 @@ struct LinearNode : public AccumulatingNode {
     std::lock_guard<std::mutex> lock(mutex_);
     x.reset_data();
     w.reset_data();
-    b.reset_data();
     z.reset_data();
+    b = at::Tensor();
   }
 
   variable_list apply(variable_list&& grads) override {
@@ -336,9 +337,12 @@ struct LinearNode : public AccumulatingNode {
     if (!grads[0].defined()) return out;
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
     const at::Tensor dy = grads[0], xs = x.unpack(), ws = w.unpack();
-    if (c10::GradMode::is_enabled())
+    if (c10::GradMode::is_enabled()) {
+      // (without an activation no gradient depends on the bias' value)
+      const at::Tensor bs = b.defined() || !bias.defined() ? b : bias.detach().to(at::kBFloat16);
       return differentiable_gradients(*this, [this](const auto& in) { return linear_composition(in, activation); },
-                                      {{xs, {0}}, {ws, {1}}, {b.unpack(), {2}}}, dy);
+                                      {{xs, {0}}, {ws, {1}}, {bs, {2}}}, dy);
+    }
     at::Tensor dy2 = vector_aligned(dy.dim() == 2 ? dy : dy.reshape({-1, dy.size(-1)}));
     if (activation) dy2 = through_activation(dy2.contiguous(), out);
     if (task_should_compute_output(0)) {
@@ -758,7 +762,7 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& weight, const std::opti
   if (node) {
     node->x = SavedVariable(xs, false);
     node->w = SavedVariable(ws, false);
-    node->b = SavedVariable(low[2], false);
+    if (activation) node->b = low[2];
     if (activation == kGelu) node->z = SavedVariable(z, false);
     node->activation = activation;
     node->weight = weight;

@@ -23,7 +23,7 @@ import torch.nn.functional as F
 from .._native import C as _C
 from ..ops import wgrad
 from ..ops.fused_linear import ShadowLinear
-from ..ops.modules import dropout, plain_embedding, untouched
+from ..ops.modules import drops_nothing, plain_embedding, untouched
 
 
 _EMBED_TOKENS = _C.max_embedding_tokens  # more tokens per batch take the framework's embedding
@@ -104,12 +104,16 @@ class _Layer(nn.Module):
 
     def forward(self, x):
         b, s, h = x.shape
-        if (x.dtype == torch.bfloat16 and _fused(x, self.ln1) and untouched(self.ln2, _LayerNorm) and (h // self.heads) % 8 == 0
+        m = self._modules
+        ln1, ln2 = m.get("ln1"), m.get("ln2")
+        if (x.dtype == torch.bfloat16 and _fused(x, ln1) and untouched(ln2, _LayerNorm) and (h // self.heads) % 8 == 0
                 and x.numel() > 0):
+            keep = drops_nothing(m.get("drop"))
             a = self.proj(_C.attention(self.qkv(x), self.heads, self.p if self.training else 0.0))
-            x = self._add_norm(self.ln1, x, dropout(self.drop, a))
-            f = self.fc1(x, "gelu") if untouched(self.fc1, ShadowLinear) else F.gelu(self.fc1(x))
-            return self._add_norm(self.ln2, x, dropout(self.drop, self.fc2(f)))
+            x = self._add_norm(ln1, x, a if keep else self.drop(a))
+            fc1 = self.fc1
+            f = self.fc2(fc1(x, "gelu") if untouched(fc1, ShadowLinear) else F.gelu(fc1(x)))
+            return self._add_norm(ln2, x, f if keep else self.drop(f))
         q, k, v = self.qkv(x).view(b, s, 3, self.heads, h // self.heads).permute(2, 0, 3, 1, 4)
         a = F.scaled_dot_product_attention(q, k, v, dropout_p=self.p if self.training else 0.0)
         a = a.transpose(1, 2).reshape(b, s, h)
@@ -145,7 +149,8 @@ class BertForQuestionAnswering(nn.Module):
 
     def forward(self, input_ids, start_positions=None, end_positions=None):
         b, s = input_ids.shape
-        if (plain_embedding(self.tok) and plain_embedding(self.pos) and _fused(self.tok.weight, self.ln)
+        m = self._modules
+        if (plain_embedding(m.get("tok")) and plain_embedding(m.get("pos")) and _fused(self.tok.weight, m.get("ln"))
                 and input_ids.is_cuda and input_ids.dtype == torch.int64 and 0 < b * s <= _EMBED_TOKENS and s <= self.pos.num_embeddings):
             x = _C.embed_layer_norm(input_ids, self.tok.weight, self.pos.weight, self.typ.weight, self.ln.weight,
                                     self.ln.bias, self.ln.eps, wgrad.active())
@@ -156,7 +161,7 @@ class BertForQuestionAnswering(nn.Module):
         for layer in self.layers:
             x = layer(x)
         if (start_positions is not None and x.dtype == torch.bfloat16 and x.numel() > 0 and _bf16_autocast(x)
-                and untouched(self.qa, nn.Linear) and self.qa.out_features == 2
+                and untouched(m.get("qa"), nn.Linear) and self.qa.out_features == 2
                 and all(t.is_cuda and t.dtype == torch.int64 and t.dim() == 1 for t in (start_positions, end_positions))):
             logits = _C.linear(x, self.qa.weight, self.qa.bias, None, False)
             return _C.span_loss(logits, start_positions, end_positions)

@@ -45,7 +45,7 @@ enabled = False
 
 def active() -> bool:
     """Whether gradients may be added in place: `enabled`, and a bucket would still learn of them."""
-    return enabled and _autograd_runs_hooks_without_a_gradient()
+    return enabled and (_hooks_run_anyway or _autograd_runs_hooks_without_a_gradient())
 
 
 def __getattr__(name):

@@ -149,11 +149,19 @@ class FlatSGD(torch.optim.Optimizer):
     def _loose_params(self):
         """[(group, parameter)] outside the flat buffers; looked up again when the groups' parameters are others than at
         the last look (an added, replaced or moved parameter, a loaded state)."""
-        now = [g["params"] for g in self.param_groups]
-        if self._loose is None or len(now) != len(self._loose[0]) or not all(
-                len(a) == len(b) and all(map(is_, a, b)) for a, b in zip(now, self._loose[0])):
-            self._loose = ([list(ps) for ps in now], [(gi, p) for gi, ps in enumerate(now) for p in ps if id(p) not in self._attached_ids])
-        return [(self.param_groups[gi], p) for gi, p in self._loose[1]]
+        groups, known = self.param_groups, self._loose
+        if known is None or len(groups) != len(known[0]):
+            known = None
+        else:
+            for g, ps in zip(groups, known[0]):
+                now = g["params"]
+                if len(now) != len(ps) or not all(map(is_, now, ps)):
+                    known = None
+                    break
+        if known is None:
+            known = self._loose = ([list(g["params"]) for g in groups],
+                                   [(gi, p) for gi, g in enumerate(groups) for p in g["params"] if id(p) not in self._attached_ids])
+        return [(groups[gi], p) for gi, p in known[1]] if known[1] else ()
 
     @torch.no_grad()
     def step(self, closure=None):
