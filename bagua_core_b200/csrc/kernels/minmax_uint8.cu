@@ -11,7 +11,8 @@
 // 10 MB in 8 chunks 6.9 us (8.2), 134 MB in 8 chunks 41 us (54), 411 MB in 8 chunks 114 us (159; 78 at the
 // copy bandwidth), 206 MB of fp16 in 8 chunks 77 us (123), 1 M fp16 in 3 odd chunks 7.5 us (7.5, with
 // dequantising 3.4 us instead of 6.7).  Small calls are bound by latency (launch, one read, the exchange);
-// large ones by instructions and L2, a group's second read being served by L2 only in part.
+// large ones by instructions and by what lies between the passes: at 268 MB memory sees the input and the output once,
+// at half its rate (profiles/kernel_roofline_1gpu.md).
 //
 // The reference issues two CUB DeviceReduce calls per chunk from a host loop
 // (bagua-core-internal/kernels/bagua_kernels.cu:312-371,533-560) and quantises one byte per thread

@@ -49,6 +49,17 @@ def main():
     out = torch.empty_like(x)
     bo = bc.BaguaTensorPy(out, "o")
 
+    # ByteGrad over one rank: the bucket's op on the communicator's stream, here the current one
+    comm = bc.BaguaSingleCommunicatorPy(0, 1, 0, torch.cuda.current_stream().cuda_stream, "solo")
+    solo = bc.BaguaBucketPy("solo", [bc.BaguaTensorPy(y, "solo_y")])
+    solo.append_centralized_synchronous_op(comm, None, hierarchical=False, average=True, scattergather=True, compression="MinMaxUInt8")
+    backend = bc.BaguaCommBackendPy(10, 0)
+    backend.register_ordered_buckets([solo])
+
+    def bytegrad_solo():
+        backend.mark_communication_ready(solo.tensors()[0], 0)
+        backend.wait_pending_comm_ops()
+
     cases = {
         # name: (callable, algorithmic bytes)
         "add": (lambda: ops.add_inplace(x, y), 3 * S),
@@ -58,9 +69,10 @@ def main():
         "reduce_chunk": (lambda: ops.reduce_chunk_inplace(x, n_chunks, 0, average=True), S + S // n_chunks),
         "async_average": (lambda: ops.async_model_average(x, y, m, 8), 4 * S),
         "sgd": (lambda: ops.sgd_momentum_flat(x, y, m, 1e-6, 0.9), 5 * S),
-        # two passes over the input (min/max, then quantise) + 1 byte per element out
-        "compress": (lambda: bx.compress("MinMaxUInt8", n_chunks, -1), 2 * S + S // 4),
+        # the input once and 1 byte per element out (a second read of what did not stay on chip is not counted)
+        "compress": (lambda: bx.compress("MinMaxUInt8", n_chunks, -1), S + S // 4),
         "decompress": (lambda: bo.decompress_from("MinMaxUInt8", n_chunks, comp), S // 4 + S),
+        "bytegrad_solo": (bytegrad_solo, 2 * S),  # quantised twice in place; the time holds the engine's hand-over
     }
     only = [s for s in args.only.split(",") if s]
     rows = []
