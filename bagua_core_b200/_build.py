@@ -55,6 +55,7 @@ SOURCES = [
     "kernels/no_alloc.cu",
     "kernels/model_ops.cu",
     "kernels/first_conv.cu",
+    "kernels/conv_wgrad.cu",
     "kernels/model_ops_cpu.cc",
     "kernels/encoder_ops.cu",
 ]

@@ -816,6 +816,27 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     *H = t.size(2);
     *W = t.size(3);
   };
+  m.def(
+      "k_conv_weight_gradient",
+      [nhwc_dims](at::Tensor dz, at::Tensor x, at::Tensor dw, uint64_t stream) {
+        int64_t N, H, W, N2, H2, W2;
+        int Co, Ci;
+        nhwc_dims(dz, &N, &H, &W, &Co);
+        nhwc_dims(x, &N2, &H2, &W2, &Ci);
+        BAGUA_CHECK(N2 == N && H2 == H && W2 == W && dz.is_cuda() && x.device() == dz.device() && dw.device() == dz.device(), Tensor,
+                    "dz and x must be of one size, and with dw on one GPU");
+        BAGUA_CHECK(dw.dim() == 4 && dw.size(0) == Co && dw.size(1) == Ci && dw.size(2) == 3 && dw.size(3) == 3 &&
+                        dw.is_non_overlapping_and_dense() && dw.scalar_type() == at::kBFloat16,
+                    Tensor, "dw must be [Co, Ci, 3, 3] in bf16");
+        BAGUA_CHECK(model_ops::conv_wgrad_supported(N, H, W, Co, Ci), Tensor, "channel counts must be multiples of 64");
+        const int64_t strides[4] = {dw.stride(0), dw.stride(2), dw.stride(3), dw.stride(1)};
+        const at::Tensor sums = at::empty({(int64_t)model_ops::conv_wgrad_scratch_bytes(N, H, W, Co, Ci)}, dz.options().dtype(at::kByte));
+        model_ops::conv_wgrad(dz.data_ptr(), x.data_ptr(), dw.data_ptr(), strides, N, H, W, Co, Ci, sums.data_ptr(), (cudaStream_t)stream);
+      },
+      py::arg("dz"), py::arg("x"), py::arg("dw"), py::arg("stream"),
+      "Weight gradient of a 3 x 3 convolution (stride, padding 1), summed in fp32 and rounded to bf16.");
+  m.def("k_conv_weight_gradient_preferred",
+        [](int64_t N, int64_t H, int64_t W, int64_t Co, int64_t Ci) { return model_ops::conv_wgrad_preferred(N, H, W, Co, Ci); });
   m.def("k_maxpool2x2_supported",
         [](int64_t N, int64_t H, int64_t W, int C) { return model_ops::maxpool2x2_supported(N, H, W, C); });
   m.def(

@@ -48,6 +48,15 @@ size_t first_conv_backward_scratch_bytes(int64_t rows, int C, int Ci);
 void first_conv_backward(const void* dy, const void* y, const void* x, float* dw, bool add_w, float* db, bool add_b, int64_t N,
                          int64_t H, int64_t W, int C, int Ci, void* scratch, cudaStream_t s);
 
+// dw[co, r, s, ci] = sum over pixels of dz and x shifted by (r - 1, s - 1): the weight gradient of a 3 x 3 convolution with stride
+// and padding 1, summed in fp32 and rounded to bf16.  dz [N, H, W, Co], x [N, H, W, Ci], bf16, channels-last, 16-byte aligned;
+// `strides` of dw by co, r, s, ci in elements.  Channel counts are multiples of 64.
+bool conv_wgrad_supported(int64_t N, int64_t H, int64_t W, int64_t Co, int64_t Ci);
+bool conv_wgrad_preferred(int64_t N, int64_t H, int64_t W, int64_t Co, int64_t Ci);  // supported, and faster than the library's
+size_t conv_wgrad_scratch_bytes(int64_t N, int64_t H, int64_t W, int64_t Co, int64_t Ci);
+void conv_wgrad(const void* dz, const void* x, void* dw, const int64_t (&strides)[4], int64_t N, int64_t H, int64_t W, int64_t Co,
+                int64_t Ci, void* scratch, cudaStream_t stream);
+
 // out[c] (+)= sum over rows of x [rows, C] in bf16, accumulated in fp32 in a fixed order: the bias gradient of a
 // linear layer.  C a multiple of 8, x 16-byte aligned.  (3072 x 1024: 8 us; the library's reduction 13 us.)
 inline bool column_sum_supported(int64_t rows, int C) { return rows > 0 && C >= 8 && C % 8 == 0; }

@@ -453,13 +453,14 @@ struct ConvNode : public AccumulatingNode {
     if (add_bias) added(2, dy);
     if (task_should_compute_output(2) && !add_bias) out[2] = db;
     const bool need_x = task_should_compute_output(0), need_w = task_should_compute_output(1);
-    if (need_x || need_w) {
+    const bool own = need_w && own_weight_gradient(xs, dz);
+    if (need_x || (need_w && !own)) {
       const std::vector<int64_t> zero{0, 0};
       auto g = at::convolution_backward(dz, xs, ws, c10::nullopt, stride, padding, dilation, false, zero, groups,
-                                        {need_x, need_w, false});
+                                        {need_x, need_w && !own, false});
       out[0] = std::get<0>(g);
       at::Tensor dw = std::get<1>(g);
-      if (need_w && dw.scalar_type() == at::kBFloat16 && adds(1, weight, dw) &&
+      if (need_w && !own && dw.scalar_type() == at::kBFloat16 && adds(1, weight, dw) &&
           dw.strides() == weight.grad().strides()) {
         // the cast to fp32 and the addition in one pass; the same bits
         if (dw.is_cuda()) {
@@ -474,14 +475,38 @@ struct ConvNode : public AccumulatingNode {
         out[1] = dw;
       }
     }
+    if (own) out[1] = weight_gradient(xs, dz);
     return out;
+  }
+
+  bool is_plain3x3() const {
+    const std::vector<int64_t> one{1, 1};
+    return groups == 1 && weight.size(2) == 3 && weight.size(3) == 3 && stride == one && padding == one && dilation == one;
+  }
+
+  // The weight gradient of a 3 x 3 convolution of many channels, where this package's kernel is the faster one.  bf16 parameters
+  // only: where they are fp32 (autocast) their gradients keep the bits of the library's.  Of this kernel's 0.1-0.3 % are rounded the
+  // other way, which as such is nothing; but VGG-16 at batch 32, which would take 4185 us a step instead of 4521, is chaotic: the few
+  // weights whose bf16 copies differ after one such step move the second step's gradients by 5 to 15 % (relative norm).
+  bool own_weight_gradient(const at::Tensor& xs, const at::Tensor& dz) const {
+    return dz.is_cuda() && is_plain3x3() && weight.scalar_type() == at::kBFloat16 && xs.scalar_type() == at::kBFloat16 &&
+           dz.scalar_type() == at::kBFloat16 && xs.is_contiguous(at::MemoryFormat::ChannelsLast) &&
+           dz.is_contiguous(at::MemoryFormat::ChannelsLast) && (uintptr_t)xs.data_ptr() % 16 == 0 && (uintptr_t)dz.data_ptr() % 16 == 0 &&
+           model_ops::conv_wgrad_preferred(dz.size(0), dz.size(2), dz.size(3), dz.size(1), xs.size(1));
+  }
+  static at::Tensor weight_gradient(const at::Tensor& xs, const at::Tensor& dz) {
+    const int64_t N = dz.size(0), H = dz.size(2), W = dz.size(3), Co = dz.size(1), Ci = xs.size(1);
+    const at::Tensor dw = at::empty({Co, Ci, 3, 3}, dz.options(), at::MemoryFormat::ChannelsLast);
+    const int64_t strides[4] = {dw.stride(0), dw.stride(2), dw.stride(3), dw.stride(1)};
+    const at::Tensor sums = fresh({(int64_t)model_ops::conv_wgrad_scratch_bytes(N, H, W, Co, Ci)}, at::kByte, dz);
+    model_ops::conv_wgrad(dz.data_ptr(), xs.data_ptr(), dw.data_ptr(), strides, N, H, W, Co, Ci, sums.data_ptr(), stream_of(dz));
+    count_launches(2);
+    return dw;
   }
 
   // A 3 x 3 convolution of few channels whose input wants no gradient: both gradients come from one kernel.
   bool first_layer(const at::Tensor& xs, const at::Tensor& dy, const at::Tensor& a) {
-    const std::vector<int64_t> one{1, 1};
-    return a.is_cuda() && !task_should_compute_output(0) && task_should_compute_output(1) &&
-           groups == 1 && weight.size(2) == 3 && weight.size(3) == 3 && stride == one && padding == one && dilation == one &&
+    return a.is_cuda() && !task_should_compute_output(0) && task_should_compute_output(1) && is_plain3x3() &&
            xs.scalar_type() == at::kBFloat16 && xs.is_contiguous(at::MemoryFormat::ChannelsLast) &&
            a.is_contiguous(at::MemoryFormat::ChannelsLast) && (uintptr_t)dy.data_ptr() % 16 == 0 &&
            (uintptr_t)a.data_ptr() % 16 == 0 &&

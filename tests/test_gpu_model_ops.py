@@ -467,6 +467,57 @@ def test_first_layer_gradients_match_fp32_math(N, H, W, Ci, C, in_place):
     assert ((got - want).abs() <= 4.1e-3 * want.abs() + 1e-5 * want.abs().max()).all()
 
 
+# rectangles that end with the image and that reach over it, one and several strips, rows in pairs, one block and many splits
+@pytest.mark.parametrize("N,H,W,Ci,Co", [(1, 1, 1, 64, 64), (2, 3, 7, 64, 128), (1, 14, 14, 128, 64), (3, 17, 23, 192, 64), (1, 5, 57, 64, 64),
+                                         (2, 65, 129, 64, 64), (1, 1, 3, 128, 128), (2, 9, 11, 128, 256), (5, 28, 28, 256, 128),
+                                         (1, 5, 300, 128, 128), (2, 56, 56, 128, 384), (2, 14, 14, 512, 512), (4, 112, 112, 128, 128)])
+def test_convolution_weight_gradient_is_the_rounded_sum(N, H, W, Ci, Co):
+    """Multiples of 1/4 up to 1/2: every sum is exact in fp32 in any order, so the bits are those of the rounded result."""
+    import bagua_core_b200 as bb
+
+    g = torch.Generator(device="cuda").manual_seed(H * W + Ci)
+
+    def draw(c):
+        t = torch.randint(-2, 3, (N, H, W, c), device="cuda", generator=g).to(torch.bfloat16) / 4
+        return t.permute(0, 3, 1, 2)
+
+    dz, x = draw(Co), draw(Ci)
+    xp = torch.nn.functional.pad(x.permute(0, 2, 3, 1).double(), (0, 0, 1, 1, 1, 1))
+    d = dz.permute(0, 2, 3, 1).double().reshape(-1, Co)
+    want = torch.stack([torch.stack([d.t() @ xp[:, r:r + H, s:s + W].reshape(-1, Ci) for s in range(3)], -1) for r in range(3)], -2)
+    want = want.to(torch.bfloat16)
+    for layout in (torch.channels_last, torch.contiguous_format):
+        low = torch.full((Co, Ci, 3, 3), 7.0, device="cuda", dtype=torch.bfloat16).to(memory_format=layout)
+        bb._C.k_conv_weight_gradient(dz, x, low, _stream())
+        assert torch.equal(low, want)
+
+
+@pytest.mark.parametrize("N,H,W,Ci,C,own", [(2, 56, 56, 64, 64, True), (1, 56, 56, 64, 64, False), (8, 56, 56, 256, 512, True),
+                                            (7, 56, 56, 256, 512, False), (2, 56, 56, 64, 32, False), (256, 7, 7, 64, 64, False)])
+@pytest.mark.parametrize("kind", [torch.bfloat16, torch.float32])
+def test_conv_blocks_on_both_sides_of_the_rule_for_their_weight_gradient(N, H, W, Ci, C, own, kind):
+    import bagua_core_b200 as bb
+    from bagua_core_b200.ops.fused_conv import ConvBiasReLU
+
+    assert bb._C.k_conv_weight_gradient_preferred(N, H, W, C, Ci) == own
+    torch.manual_seed(C)
+    m = ConvBiasReLU(Ci, C, 3, padding=1).cuda().to(dtype=kind, memory_format=torch.channels_last)
+    x = torch.randn(N, Ci, H, W, device="cuda", dtype=kind).to(memory_format=torch.channels_last).requires_grad_()
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        y = m(x)
+    dy = torch.randn(y.shape, device="cuda").to(torch.bfloat16).to(memory_format=torch.channels_last)
+    before = bb_launches()
+    y.backward(dy)
+    assert bb_launches() - before == (4 if own and kind is torch.bfloat16 else 2)
+    dz = torch.where(y > 0, dy, torch.zeros_like(dy)).detach()
+    ref = torch.ops.aten.convolution_backward(dz, x.detach().bfloat16(), m.weight.detach().bfloat16(), None, [1, 1], [1, 1], [1, 1], False,
+                                              [0, 0], 1, [False, True, False])[1].float()
+    got = m.weight.grad.float()
+    # two roundings to bf16 (2^-9 each) of sums in fp32 whose order differs
+    assert (got - ref).norm() <= 2 ** -8 * ref.norm()
+    assert ((got - ref).abs() <= 2 ** -7 * ref.abs() + 2e-5 * ref.abs().max()).all()
+
+
 @pytest.mark.parametrize("rows,H", [(1, 8), (5, 264), (37, 768), (3072, 1024)])
 @pytest.mark.parametrize("accumulate", [False, True])
 def test_add_layer_norm_has_the_bits_of_the_plain_composition(rows, H, accumulate):
