@@ -24,17 +24,20 @@ using namespace bodies;
 using kernels::launch_overlapped;
 using kernels::wait_for_predecessor;
 
+template <bool kSigns>
 __global__ void __launch_bounds__(kThreads)
-    bias_relu_kernel(uint4* __restrict__ z, const __nv_bfloat16* __restrict__ bias, int64_t nvec, int cgroups) {
+    bias_relu_kernel(uint4* __restrict__ z, const __nv_bfloat16* __restrict__ bias, int64_t nvec, int cgroups,
+                     uint8_t* __restrict__ signs) {
   wait_for_predecessor();
-  bias_relu_body(z, bias, nvec, cgroups);
+  bias_relu_body<kSigns>(z, bias, nvec, cgroups, signs);
 }
+template <bool kSigns>
 __global__ void __launch_bounds__(kThreads)
     bias_relu_backward_kernel(const uint4* dy, const uint4* __restrict__ y, uint4* dz, float* __restrict__ partial,
-                              int64_t rows, int cgroups) {
+                              int64_t rows, int cgroups, const uint8_t* __restrict__ signs) {
   __shared__ float s_acc[kThreads * 8];
   wait_for_predecessor();
-  bias_relu_backward_body(dy, y, dz, partial, rows, cgroups, s_acc);
+  bias_relu_backward_body<kSigns>(dy, y, dz, partial, rows, cgroups, s_acc, signs);
 }
 constexpr int kFoldCols = 32, kFoldRows = 32;
 __global__ void __launch_bounds__(kFoldCols * kFoldRows)
@@ -68,11 +71,19 @@ __global__ void __launch_bounds__(kThreads)
   wait_for_predecessor();
   bias_relu_pool_body(y, p, bias, pooled_pixels, Wo, W, cgroups);
 }
+template <bool kCodes>
 __global__ void __launch_bounds__(kThreads)
     bias_relu_pool_only_kernel(const uint4* __restrict__ z, uint4* __restrict__ p, const __nv_bfloat16* __restrict__ bias,
-                               int64_t pooled_pixels, int64_t Wo, int64_t W, int cgroups) {
+                               int64_t pooled_pixels, int64_t Wo, int64_t W, int cgroups, uint32_t* __restrict__ codes) {
   wait_for_predecessor();
-  bias_relu_pool_only_body(z, p, bias, pooled_pixels, Wo, W, cgroups);
+  bias_relu_pool_only_body<kCodes>(z, p, bias, pooled_pixels, Wo, W, cgroups, codes);
+}
+__global__ void __launch_bounds__(kThreads)
+    bias_relu_pool_backward_codes_kernel(const uint4* __restrict__ dp, const uint32_t* __restrict__ codes, uint4* __restrict__ dz,
+                                         float* __restrict__ partial, int64_t pooled_rows, int64_t Wo, int64_t W, int cgroups) {
+  __shared__ float s_acc[kThreads * 8];
+  wait_for_predecessor();
+  bias_relu_pool_backward_codes_body(dp, codes, dz, partial, pooled_rows, Wo, W, cgroups, s_acc);
 }
 template <bool kFromZ>
 __global__ void __launch_bounds__(kThreads)
@@ -105,13 +116,14 @@ int backward_blocks(int64_t rows, int C) {
 
 static_assert(kThreads == kBlockThreads, "bias_relu_supported() assumes the kernels' block size");
 
-void bias_relu_inplace_bf16(void* z, const void* bias, int64_t rows, int C, cudaStream_t stream) {
+void bias_relu_inplace_bf16(void* z, const void* bias, int64_t rows, int C, cudaStream_t stream, void* signs) {
   BAGUA_CHECK(bias_relu_supported(rows, C) && (uintptr_t)z % 16 == 0, Tensor,
               "fused bias+ReLU: unsupported shape [" << rows << ", " << C << "] or unaligned activation");
   const int64_t nvec = rows * (C / 8);
   const int64_t want = (nvec + (int64_t)kThreads * 4 - 1) / ((int64_t)kThreads * 4);
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, 148 * 8));
-  launch_overlapped(bias_relu_kernel, dim3(grid), dim3(kThreads), stream, (uint4*)z, (const __nv_bfloat16*)bias, nvec, C / 8);
+  launch_overlapped(signs ? bias_relu_kernel<true> : bias_relu_kernel<false>, dim3(grid), dim3(kThreads), stream, (uint4*)z,
+                    (const __nv_bfloat16*)bias, nvec, C / 8, (uint8_t*)signs);
 }
 
 size_t bias_relu_backward_scratch_bytes(int64_t rows, int C) {
@@ -120,12 +132,13 @@ size_t bias_relu_backward_scratch_bytes(int64_t rows, int C) {
 }
 
 void bias_relu_backward_bf16(const void* dy, const void* y, void* dz, float* db, int64_t rows, int C, void* scratch,
-                             cudaStream_t stream, bool accumulate) {
+                             cudaStream_t stream, bool accumulate, const void* signs) {
   BAGUA_CHECK(bias_relu_supported(rows, C) && (uintptr_t)dy % 16 == 0 && (uintptr_t)y % 16 == 0 &&
                   (uintptr_t)dz % 16 == 0 && scratch != nullptr,
               Tensor, "fused bias+ReLU backward: unsupported shape [" << rows << ", " << C << "] or unaligned buffers");
   const int blocks = backward_blocks(rows, C);
-  launch_overlapped(bias_relu_backward_kernel, dim3(blocks), dim3(kThreads), stream, (const uint4*)dy, (const uint4*)y, (uint4*)dz, (float*)scratch, rows, C / 8);
+  launch_overlapped(signs ? bias_relu_backward_kernel<true> : bias_relu_backward_kernel<false>, dim3(blocks), dim3(kThreads), stream,
+                    (const uint4*)dy, (const uint4*)y, (uint4*)dz, (float*)scratch, rows, C / 8, (const uint8_t*)signs);
   fold_partials((const float*)scratch, db, blocks, C, accumulate, stream);
 }
 
@@ -183,14 +196,16 @@ void bias_relu_pool_bf16(void* y, void* p, const void* bias, int64_t N, int64_t 
 }
 
 void bias_relu_pool_only_bf16(const void* z, void* p, const void* bias, int64_t N, int64_t H, int64_t W, int C,
-                              cudaStream_t stream) {
+                              cudaStream_t stream, void* codes) {
   BAGUA_CHECK(bias_relu_supported(N * H * W, C) && maxpool2x2_supported(N, H, W, C) && (uintptr_t)z % 16 == 0 &&
                   (uintptr_t)p % 16 == 0,
               Tensor,
               "fused bias+ReLU+pool: unsupported shape [" << N << ", " << H << ", " << W << ", " << C
                                                           << "] or unaligned buffers");
   const int64_t pooled_pixels = N * (H / 2) * (W / 2);
-  launch_overlapped(bias_relu_pool_only_kernel, dim3(pool_grid(pooled_pixels * (C / 8))), dim3(kThreads), stream, (const uint4*)z, (uint4*)p, (const __nv_bfloat16*)bias, pooled_pixels, W / 2, W, C / 8);
+  launch_overlapped(codes ? bias_relu_pool_only_kernel<true> : bias_relu_pool_only_kernel<false>, dim3(pool_grid(pooled_pixels * (C / 8))),
+                    dim3(kThreads), stream, (const uint4*)z, (uint4*)p, (const __nv_bfloat16*)bias, pooled_pixels, W / 2, W, C / 8,
+                    (uint32_t*)codes);
 }
 
 void bias_relu_pool_backward_bf16(const void* dp, const void* y, const void* bias, void* dz, float* db, int64_t N,
@@ -204,6 +219,19 @@ void bias_relu_pool_backward_bf16(const void* dp, const void* y, const void* bia
   const int blocks = backward_blocks(pooled_rows, C);
   auto* kernel = bias ? bias_relu_pool_backward_kernel<true> : bias_relu_pool_backward_kernel<false>;
   launch_overlapped(kernel, dim3(blocks), dim3(kThreads), stream, (const uint4*)dp, (const uint4*)y, (uint4*)dz, (float*)scratch, pooled_rows, W / 2, W, C / 8, (const __nv_bfloat16*)bias);
+  fold_partials((const float*)scratch, db, blocks, C, accumulate, stream);
+}
+
+void bias_relu_pool_backward_codes_bf16(const void* dp, const void* codes, void* dz, float* db, int64_t N, int64_t H, int64_t W, int C,
+                                        void* scratch, cudaStream_t stream, bool accumulate) {
+  BAGUA_CHECK(bias_relu_supported(N * H * W, C) && maxpool2x2_supported(N, H, W, C) && (uintptr_t)dp % 16 == 0 &&
+                  (uintptr_t)codes % 4 == 0 && (uintptr_t)dz % 16 == 0 && scratch != nullptr,
+              Tensor, "fused bias+ReLU+pool backward: unsupported shape [" << N << ", " << H << ", " << W << ", " << C
+                                                                           << "] or unaligned buffers");
+  const int64_t pooled_rows = N * (H / 2) * (W / 2);
+  const int blocks = backward_blocks(pooled_rows, C);
+  launch_overlapped(bias_relu_pool_backward_codes_kernel, dim3(blocks), dim3(kThreads), stream, (const uint4*)dp, (const uint32_t*)codes,
+                    (uint4*)dz, (float*)scratch, pooled_rows, W / 2, W, C / 8);
   fold_partials((const float*)scratch, db, blocks, C, accumulate, stream);
 }
 

@@ -35,6 +35,69 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
   return r;
 }
 
+// Two bf16 values of one sign per word, compared as 16-bit integers: activations behind a ReLU are
+// not negative, and their bit patterns are ordered like their values.
+#ifdef BAGUA_HOST_EMULATION
+__device__ __forceinline__ uint32_t max_u16x2(uint32_t a, uint32_t b) {
+  const uint32_t lo = (a & 0xffffu) > (b & 0xffffu) ? a : b, hi = (a >> 16) > (b >> 16) ? a : b;
+  return (lo & 0xffffu) | (hi & 0xffff0000u);
+}
+__device__ __forceinline__ uint32_t eq_u16x2(uint32_t a, uint32_t b) {
+  const uint32_t d = a ^ b;
+  return ((d & 0xffffu) ? 0u : 0xffffu) | ((d >> 16) ? 0u : 0xffff0000u);
+}
+#else
+__device__ __forceinline__ uint32_t max_u16x2(uint32_t a, uint32_t b) { return __vmaxu2(a, b); }
+__device__ __forceinline__ uint32_t eq_u16x2(uint32_t a, uint32_t b) { return __vcmpeq2(a, b); }
+#endif
+
+// max(x + b, 0) of two bf16 values, rounded once: the bits of an addition in fp32 that is rounded to bf16 afterwards (where
+// that one is inexact, the smaller operand is too small for a tie).  Comparisons are masks of 0xffff.
+#ifdef BAGUA_HOST_EMULATION
+__device__ __forceinline__ float bf16_value(uint32_t half) {
+  const uint32_t u = half << 16;
+  float f;
+  memcpy(&f, &u, 4);
+  return f;
+}
+__device__ __forceinline__ uint32_t bias_relu_x2(uint32_t x, uint32_t b) {
+  uint32_t r = 0;
+  for (int k = 0; k < 32; k += 16) {
+    const __nv_bfloat16 v = __float2bfloat16_rn(fmaxf(bf16_value(x >> k & 0xffffu) + bf16_value(b >> k & 0xffffu), 0.f));
+    uint16_t u;
+    memcpy(&u, &v, 2);
+    r |= (uint32_t)u << k;
+  }
+  return r & 0x7fff7fffu;
+}
+__device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) { return max_u16x2(a, b); }
+__device__ __forceinline__ uint32_t eq_bf16x2(uint32_t a, uint32_t b) { return eq_u16x2(a, b); }
+#else
+__device__ __forceinline__ __nv_bfloat162 as_bf162(uint32_t v) { return *reinterpret_cast<const __nv_bfloat162*>(&v); }
+__device__ __forceinline__ uint32_t bits_of(__nv_bfloat162 v) { return *reinterpret_cast<const uint32_t*>(&v); }
+__device__ __forceinline__ uint32_t bias_relu_x2(uint32_t x, uint32_t b) {
+  return bits_of(__hmax2(__hadd2(as_bf162(x), as_bf162(b)), as_bf162(0u))) & 0x7fff7fffu;
+}
+__device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) { return bits_of(__hmax2(as_bf162(a), as_bf162(b))); }
+__device__ __forceinline__ uint32_t eq_bf16x2(uint32_t a, uint32_t b) { return __heq2_mask(as_bf162(a), as_bf162(b)); }
+#endif
+
+__device__ __forceinline__ uint4 clear_signs(const uint4& a) {
+  return make_uint4(a.x & 0x7fff7fffu, a.y & 0x7fff7fffu, a.z & 0x7fff7fffu, a.w & 0x7fff7fffu);
+}
+
+// What a backward pass wants of eight 16-bit values is one bit each: bit 2 k + half of the result is set where half `half` of
+// mask k is (masks of 0xffff or 0 per half) ...
+__device__ __forceinline__ uint32_t gather_bits(uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3) {
+  const uint32_t a = (m0 & 0x00010001u) | (m1 & 0x00040004u) | (m2 & 0x00100010u) | (m3 & 0x00400040u);
+  return (a | (a >> 15)) & 0xffu;
+}
+// ... and mask k again.
+__device__ __forceinline__ uint32_t spread_bits(uint32_t bits, int k) {
+  const uint32_t b = bits >> (2 * k);
+  return ((0u - (b & 1u)) & 0x0000ffffu) | ((0u - ((b >> 1) & 1u)) & 0xffff0000u);
+}
+
 // ---- forward ----------------------------------------------------------------------
 __device__ __forceinline__ uint4 bias_relu_vec(const uint4& x, const float* b) {
   float f[8];
@@ -52,21 +115,30 @@ __device__ __forceinline__ void load_bias8(const __nv_bfloat16* __restrict__ bia
 
 // cgroups = C / 8 vectors per row.  cgroups divides kThreads, hence the grid stride too, so all
 // vectors a thread visits belong to one channel group: its bias stays in registers and the loop
-// has no division.
+// has no division.  kSigns: which values are positive is left in `signs`, a byte per vector.
+template <bool kSigns = false>
 __device__ __forceinline__ void bias_relu_body(uint4* __restrict__ z, const __nv_bfloat16* __restrict__ bias,
-                                               int64_t nvec, int cgroups) {
+                                               int64_t nvec, int cgroups, uint8_t* __restrict__ signs = nullptr) {
   float bs[8];
   load_bias8(bias, (int)(threadIdx.x % cgroups), bs);
   const int64_t stride = (int64_t)gridDim.x * kThreads;
   int64_t v = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  auto one = [&](int64_t at, const uint4& in) {
+    const uint4 r = bias_relu_vec(in, bs);
+    z[at] = r;
+    if constexpr (kSigns) {
+      const uint4 y = clear_signs(r);  // -0 is not positive
+      signs[at] = (uint8_t)gather_bits(~eq_u16x2(y.x, 0u), ~eq_u16x2(y.y, 0u), ~eq_u16x2(y.z, 0u), ~eq_u16x2(y.w, 0u));
+    }
+  };
   for (; v + 3 * stride < nvec; v += 4 * stride) {
     const uint4 a = z[v], b = z[v + stride], c = z[v + 2 * stride], d = z[v + 3 * stride];
-    z[v] = bias_relu_vec(a, bs);
-    z[v + stride] = bias_relu_vec(b, bs);
-    z[v + 2 * stride] = bias_relu_vec(c, bs);
-    z[v + 3 * stride] = bias_relu_vec(d, bs);
+    one(v, a);
+    one(v + stride, b);
+    one(v + 2 * stride, c);
+    one(v + 3 * stride, d);
   }
-  for (; v < nvec; v += stride) z[v] = bias_relu_vec(z[v], bs);
+  for (; v < nvec; v += stride) one(v, z[v]);
 }
 
 // ---- backward ---------------------------------------------------------------------
@@ -84,9 +156,11 @@ __device__ __forceinline__ uint4 relu_mask_acc(const uint4& dy, const uint4& y, 
 
 // Threads are laid out [rows_per_iter][cgroups]: thread (ro, cg) visits rows ro, ro + R, ...
 // (R = gridDim.x * rows_per_iter apart) and always the same 8 channels.  cgroups divides kThreads.
+// kSigns: `signs` as the forward left them stand in for y, a sixteenth of its bytes.
+template <bool kSigns = false>
 __device__ __forceinline__ void bias_relu_backward_body(const uint4* dy, const uint4* __restrict__ y, uint4* dz,
                                                         float* __restrict__ partial, int64_t rows, int cgroups,
-                                                        float* s_acc) {
+                                                        float* s_acc, const uint8_t* __restrict__ signs = nullptr) {
   const int rows_per_iter = kThreads / cgroups;
   const int cg = threadIdx.x % cgroups, ro = threadIdx.x / cgroups;
   const int64_t step = (int64_t)gridDim.x * rows_per_iter;
@@ -94,15 +168,39 @@ __device__ __forceinline__ void bias_relu_backward_body(const uint4* dy, const u
 #pragma unroll
   for (int k = 0; k < 8; ++k) acc[k] = 0.f;
   int64_t row = (int64_t)blockIdx.x * rows_per_iter + ro;
-  for (; row + step < rows; row += 2 * step) {
-    const int64_t v0 = row * cgroups + cg, v1 = (row + step) * cgroups + cg;
-    const uint4 a0 = dy[v0], b0 = y[v0], a1 = dy[v1], b1 = y[v1];
-    dz[v0] = relu_mask_acc(a0, b0, acc);
-    dz[v1] = relu_mask_acc(a1, b1, acc);
-  }
-  for (; row < rows; row += step) {
-    const int64_t v0 = row * cgroups + cg;
-    dz[v0] = relu_mask_acc(dy[v0], y[v0], acc);
+  if constexpr (kSigns) {
+    auto one = [&](const uint4& g, uint32_t bits) {
+      const uint4 r = make_uint4(g.x & spread_bits(bits, 0), g.y & spread_bits(bits, 1), g.z & spread_bits(bits, 2), g.w & spread_bits(bits, 3));
+      float f[8];
+      unpack8(r, f);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) acc[k] += f[k];
+      return r;
+    };
+    for (; row + 3 * step < rows; row += 4 * step) {
+      const int64_t v0 = row * cgroups + cg, dv = step * cgroups;
+      const uint4 a0 = dy[v0], a1 = dy[v0 + dv], a2 = dy[v0 + 2 * dv], a3 = dy[v0 + 3 * dv];
+      const uint32_t b0 = signs[v0], b1 = signs[v0 + dv], b2 = signs[v0 + 2 * dv], b3 = signs[v0 + 3 * dv];
+      dz[v0] = one(a0, b0);
+      dz[v0 + dv] = one(a1, b1);
+      dz[v0 + 2 * dv] = one(a2, b2);
+      dz[v0 + 3 * dv] = one(a3, b3);
+    }
+    for (; row < rows; row += step) {
+      const int64_t v0 = row * cgroups + cg;
+      dz[v0] = one(dy[v0], signs[v0]);
+    }
+  } else {
+    for (; row + step < rows; row += 2 * step) {
+      const int64_t v0 = row * cgroups + cg, v1 = (row + step) * cgroups + cg;
+      const uint4 a0 = dy[v0], b0 = y[v0], a1 = dy[v1], b1 = y[v1];
+      dz[v0] = relu_mask_acc(a0, b0, acc);
+      dz[v1] = relu_mask_acc(a1, b1, acc);
+    }
+    for (; row < rows; row += step) {
+      const int64_t v0 = row * cgroups + cg;
+      dz[v0] = relu_mask_acc(dy[v0], y[v0], acc);
+    }
   }
 #pragma unroll
   for (int k = 0; k < 8; ++k) s_acc[threadIdx.x * 8 + k] = acc[k];
@@ -303,21 +401,54 @@ __device__ __forceinline__ void bias_relu_pool_body(uint4* __restrict__ y, uint4
   }
 }
 
-// The same maximum without the activation: z is only read, and only the pooled output is written.  What the
-// backward needs of the activation (the arg-max of each window and whether it is positive) follows from z
-// and the bias again, so a block whose full-resolution activation nobody else reads moves 1.25 instead of
-// 2.25 activations forward and the same bytes back (64 channels at 224 x 224, batch 32: 73 -> 43 us forward).
+// The maximum of four positions, none of them negative; in their places, masks that are set at the first one that holds it, if
+// it is not zero.
+__device__ __forceinline__ uint32_t first_max(uint32_t& y0, uint32_t& y1, uint32_t& y2, uint32_t& y3) {
+  const uint32_t m = max_bf16x2(max_bf16x2(y0, y1), max_bf16x2(y2, y3)), none = eq_bf16x2(m, 0u);
+  const uint32_t e0 = eq_bf16x2(y0, m), e01 = e0 | eq_bf16x2(y1, m), e012 = e01 | eq_bf16x2(y2, m);
+  y0 = e0 & ~none;
+  y1 = e01 & ~e0 & ~none;
+  y2 = e012 & ~e01 & ~none;
+  y3 = ~e012 & ~none;
+  return m;
+}
+
+// The same maximum without the activation: z is only read, and only the pooled output is written.  kCodes: with what the
+// backward needs of the activation, in four bytes per pooled vector: byte `position` has a bit for every channel whose first
+// maximum, if it is positive, is at that position of the window.  (64 channels at 224 x 224, batch 32, us: forward / backward
+// 43.5 / 76.6 where the backward makes the activation again from z and the bias, 48.0 / 43.9 with codes.)
+template <bool kCodes = false>
 __device__ __forceinline__ void bias_relu_pool_only_body(const uint4* __restrict__ z, uint4* __restrict__ p,
                                                          const __nv_bfloat16* __restrict__ bias, int64_t pooled_pixels,
-                                                         int64_t Wo, int64_t W, int cgroups) {
+                                                         int64_t Wo, int64_t W, int cgroups, uint32_t* __restrict__ codes = nullptr) {
   const int cg = (int)(threadIdx.x % cgroups);
   float b[8];
   load_bias8(bias, cg, b);
+  const uint4 b2 = pack8(b);
   const int64_t pixel_step = (int64_t)gridDim.x * (kThreads / cgroups);
   for (int64_t px = (int64_t)blockIdx.x * (kThreads / cgroups) + threadIdx.x / cgroups; px < pooled_pixels;
        px += pixel_step) {
     const PoolIndex q = pool_index(px, cg, Wo, W, cgroups);
-    const uint4 a0 = z[q.x00], a1 = z[q.x00 + q.dw], a2 = z[q.x00 + q.dh], a3 = z[q.x00 + q.dh + q.dw];
+    uint4 a0 = z[q.x00], a1 = z[q.x00 + q.dw], a2 = z[q.x00 + q.dh], a3 = z[q.x00 + q.dh + q.dw];
+    if constexpr (kCodes) {
+      // two channels an instruction: one at a time, as below, the instructions took 57 us where memory takes 43
+      auto active = [&](const uint4& v) {
+        return make_uint4(bias_relu_x2(v.x, b2.x), bias_relu_x2(v.y, b2.y), bias_relu_x2(v.z, b2.z), bias_relu_x2(v.w, b2.w));
+      };
+      a0 = active(a0);
+      a1 = active(a1);
+      a2 = active(a2);
+      a3 = active(a3);
+      uint4 m;
+      m.x = first_max(a0.x, a1.x, a2.x, a3.x);
+      m.y = first_max(a0.y, a1.y, a2.y, a3.y);
+      m.z = first_max(a0.z, a1.z, a2.z, a3.z);
+      m.w = first_max(a0.w, a1.w, a2.w, a3.w);
+      p[px * cgroups + cg] = m;
+      codes[px * cgroups + cg] = gather_bits(a0.x, a0.y, a0.z, a0.w) | gather_bits(a1.x, a1.y, a1.z, a1.w) << 8 |
+                                 gather_bits(a2.x, a2.y, a2.z, a2.w) << 16 | gather_bits(a3.x, a3.y, a3.z, a3.w) << 24;
+      continue;
+    }
     float f0[8], f1[8], f2[8], f3[8];
     unpack8(a0, f0);
     unpack8(a1, f1);
@@ -330,35 +461,15 @@ __device__ __forceinline__ void bias_relu_pool_only_body(const uint4* __restrict
   }
 }
 
-// Two bf16 values of one sign per word, compared as 16-bit integers: activations behind a ReLU are
-// not negative, and their bit patterns are ordered like their values.
-#ifdef BAGUA_HOST_EMULATION
-__device__ __forceinline__ uint32_t max_u16x2(uint32_t a, uint32_t b) {
-  const uint32_t lo = (a & 0xffffu) > (b & 0xffffu) ? a : b, hi = (a >> 16) > (b >> 16) ? a : b;
-  return (lo & 0xffffu) | (hi & 0xffff0000u);
-}
-__device__ __forceinline__ uint32_t eq_u16x2(uint32_t a, uint32_t b) {
-  const uint32_t d = a ^ b;
-  return ((d & 0xffffu) ? 0u : 0xffffu) | ((d >> 16) ? 0u : 0xffff0000u);
-}
-#else
-__device__ __forceinline__ uint32_t max_u16x2(uint32_t a, uint32_t b) { return __vmaxu2(a, b); }
-__device__ __forceinline__ uint32_t eq_u16x2(uint32_t a, uint32_t b) { return __vcmpeq2(a, b); }
-#endif
-
-__device__ __forceinline__ uint4 clear_signs(const uint4& a) {
-  return make_uint4(a.x & 0x7fff7fffu, a.y & 0x7fff7fffu, a.z & 0x7fff7fffu, a.w & 0x7fff7fffu);
-}
 // g for the first of four positions that holds the maximum, zero for the others; nothing where the maximum is zero.
 __device__ __forceinline__ uint32_t route_to_first_max(uint32_t& y0, uint32_t& y1, uint32_t& y2, uint32_t& y3, uint32_t g) {
-  const uint32_t m = max_u16x2(max_u16x2(y0, y1), max_u16x2(y2, y3));
-  g &= ~eq_u16x2(m, 0u);
-  const uint32_t e0 = eq_u16x2(y0, m), e01 = e0 | eq_u16x2(y1, m), e012 = e01 | eq_u16x2(y2, m);
-  y0 = g & e0;
-  y1 = g & e01 & ~e0;
-  y2 = g & e012 & ~e01;
-  y3 = g & ~e012;
-  return g;
+  first_max(y0, y1, y2, y3);
+  const uint32_t any = y0 | y1 | y2 | y3;
+  y0 &= g;
+  y1 &= g;
+  y2 &= g;
+  y3 &= g;
+  return g & any;
 }
 
 // Backward of the pair: dz = dp routed to each window's first maximum of y, masked by y > 0,
@@ -439,6 +550,47 @@ __device__ __forceinline__ void bias_relu_pool_backward_body(const uint4* __rest
     dz[q.x00 + q.dw] = pack8(f1);
     dz[q.x00 + q.dh] = pack8(f2);
     dz[q.x00 + q.dh + q.dw] = pack8(f3);
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) s_acc[threadIdx.x * 8 + k] = acc[k];
+  __syncthreads();
+  const int C = cgroups * 8;
+  for (int c = threadIdx.x; c < C; c += kThreads) {
+    const int g = c >> 3, k = c & 7;
+    float s = 0.f;
+    for (int r = 0; r < rows_per_iter; ++r) s += s_acc[(r * cgroups + g) * 8 + k];
+    partial[(size_t)blockIdx.x * C + c] = s;
+  }
+}
+
+// The same from the forward's codes: neither z nor the activation is read.
+__device__ __forceinline__ void bias_relu_pool_backward_codes_body(const uint4* __restrict__ dp, const uint32_t* __restrict__ codes,
+                                                                   uint4* __restrict__ dz, float* __restrict__ partial, int64_t pooled_rows,
+                                                                   int64_t Wo, int64_t W, int cgroups, float* s_acc) {
+  const int rows_per_iter = kThreads / cgroups;
+  const int cg = threadIdx.x % cgroups, ro = threadIdx.x / cgroups;
+  const int64_t step = (int64_t)gridDim.x * rows_per_iter;
+  float acc[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) acc[k] = 0.f;
+#pragma unroll 2
+  for (int64_t pr = (int64_t)blockIdx.x * rows_per_iter + ro; pr < pooled_rows; pr += step) {
+    const int64_t v = pr * cgroups + cg;
+    const uint4 g = dp[v];
+    const uint32_t code = codes[v];
+    const PoolIndex q = pool_index(pr, cg, Wo, W, cgroups);
+    uint4 sum = make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int at = 0; at < 4; ++at) {
+      const uint32_t bits = code >> (8 * at);
+      const uint4 r = make_uint4(g.x & spread_bits(bits, 0), g.y & spread_bits(bits, 1), g.z & spread_bits(bits, 2), g.w & spread_bits(bits, 3));
+      dz[q.x00 + (at & 1 ? q.dw : 0) + (at & 2 ? q.dh : 0)] = r;
+      sum = make_uint4(sum.x | r.x, sum.y | r.y, sum.z | r.z, sum.w | r.w);  // a channel goes to one position at most
+    }
+    float f[8];
+    unpack8(sum, f);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) acc[k] += f[k];
   }
 #pragma unroll
   for (int k = 0; k < 8; ++k) s_acc[threadIdx.x * 8 + k] = acc[k];

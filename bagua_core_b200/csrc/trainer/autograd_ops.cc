@@ -414,7 +414,9 @@ at::Tensor conv_composition(const std::vector<at::Tensor>& in, const std::vector
 }
 
 struct ConvNode : public AccumulatingNode {
-  SavedVariable x, w, b, act;  // act: the activation, or with pooling the convolution's output
+  SavedVariable x, w, b, act;  // act: the activation, or with pooling the convolution's output (CPU)
+  // CUDA: a bit per value of the activation, whether it is positive; with pooling four per pooled value, where it came from
+  SavedVariable signs;
   at::Tensor weight, bias;
   std::vector<int64_t> stride, padding, dilation;
   int64_t groups = 1;
@@ -427,6 +429,7 @@ struct ConvNode : public AccumulatingNode {
     w.reset_data();
     b.reset_data();
     act.reset_data();
+    signs.reset_data();
   }
 
   variable_list apply(variable_list&& grads) override {
@@ -435,7 +438,8 @@ struct ConvNode : public AccumulatingNode {
     uses_done();
     if (!grads[0].defined()) return out;
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
-    const at::Tensor xs = x.unpack(), ws = w.unpack(), a = act.unpack(pool ? std::shared_ptr<Node>() : shared_from_this());
+    const at::Tensor xs = x.unpack(), ws = w.unpack(), bits = signs.unpack();
+    const at::Tensor a = pool && bits.defined() ? at::Tensor() : act.unpack(pool ? std::shared_ptr<Node>() : shared_from_this());
     if (c10::GradMode::is_enabled())
       return differentiable_gradients(*this, [this](const auto& in) { return conv_composition(in, stride, padding, dilation, groups, pool); },
                                       {{xs, {0}}, {ws, {1}}, {b.unpack(), {2}}}, grads[0]);
@@ -445,11 +449,12 @@ struct ConvNode : public AccumulatingNode {
       first_layer_backward(xs, dy, a, out);
       return out;
     }
-    at::Tensor dz = at::empty_like(a);
+    at::Tensor dz = at::empty({dy.size(0), C, dy.size(2) * (pool ? 2 : 1), dy.size(3) * (pool ? 2 : 1)}, dy.options().dtype(at::kBFloat16),
+                              at::MemoryFormat::ChannelsLast);
     // the bias gradient is added to `.grad` by the fold of its partial sums
     const bool add_bias = dy.is_cuda() && task_should_compute_output(2) && adds(2, bias, dy);
-    at::Tensor db = add_bias ? bias.grad() : fresh({C}, at::kFloat, a);
-    backward_tail(dy, a, dz, db, add_bias);
+    at::Tensor db = add_bias ? bias.grad() : fresh({C}, at::kFloat, dz);
+    backward_tail(dy, a, bits, dz, db, add_bias);
     if (add_bias) added(2, dy);
     if (task_should_compute_output(2) && !add_bias) out[2] = db;
     const bool need_x = task_should_compute_output(0), need_w = task_should_compute_output(1);
@@ -535,11 +540,11 @@ struct ConvNode : public AccumulatingNode {
       out[2] = db;
   }
 
-  void backward_tail(const at::Tensor& dy, const at::Tensor& a, at::Tensor& dz, at::Tensor& db, bool add) {
-    const int64_t N = a.size(0), H = a.size(2), W = a.size(3), rows = N * H * W;
-    const int C = (int)a.size(1);
+  void backward_tail(const at::Tensor& dy, const at::Tensor& a, const at::Tensor& bits, at::Tensor& dz, at::Tensor& db, bool add) {
+    const int64_t N = dz.size(0), H = dz.size(2), W = dz.size(3), rows = N * H * W;
+    const int C = (int)dz.size(1);
     float* dbp = db.data_ptr<float>();
-    if (!a.is_cuda()) {
+    if (!dz.is_cuda()) {
       if (pool) {
         at::Tensor y = a.clone();
         model_ops::bias_relu_inplace_bf16_host(y.data_ptr(), b.unpack().data_ptr(), rows, C);
@@ -549,13 +554,13 @@ struct ConvNode : public AccumulatingNode {
       }
       return;
     }
-    auto scratch = scratch_for(a, model_ops::bias_relu_backward_scratch_bytes(pool ? N * (H / 2) * (W / 2) : rows, C));
+    auto scratch = scratch_for(dz, model_ops::bias_relu_backward_scratch_bytes(pool ? N * (H / 2) * (W / 2) : rows, C));
     if (pool)
-      model_ops::bias_relu_pool_backward_bf16(dy.data_ptr(), a.data_ptr(), b.unpack().data_ptr(), dz.data_ptr(), dbp, N, H,
-                                              W, C, scratch->data_ptr(), stream_of(a), add);
+      model_ops::bias_relu_pool_backward_codes_bf16(dy.data_ptr(), bits.data_ptr(), dz.data_ptr(), dbp, N, H, W, C, scratch->data_ptr(),
+                                                    stream_of(dz), add);
     else
       model_ops::bias_relu_backward_bf16(dy.data_ptr(), a.data_ptr(), dz.data_ptr(), dbp, rows, C, scratch->data_ptr(),
-                                         stream_of(a), add);
+                                         stream_of(dz), add, bits.data_ptr());
     count_launches(2);  // mask and partial sums, then their fold
   }
 };
@@ -812,7 +817,7 @@ at::Tensor conv_bias_relu(const at::Tensor& x, const at::Tensor& weight, const a
   }
   std::shared_ptr<ConvNode> node;
   if (torch::autograd::compute_requires_grad(x, weight, bias)) node = make_node<ConvNode>(x, weight, bias);
-  at::Tensor xs, ws, bs, z, out;
+  at::Tensor xs, ws, bs, z, out, signs;
   {
     PlainDispatch plain;
     std::array<at::Tensor, 3> ts{x, w_low ? *w_low : weight, bias};
@@ -834,15 +839,18 @@ at::Tensor conv_bias_relu(const at::Tensor& x, const at::Tensor& weight, const a
                 "a convolution of " << C << " channels needs as many bias values on its device");
     if (pool) {
       out = at::empty({N, C, H / 2, W / 2}, z.options().memory_format(at::MemoryFormat::ChannelsLast));
-      if (z.is_cuda())
-        model_ops::bias_relu_pool_only_bf16(z.data_ptr(), out.data_ptr(), bs.data_ptr(), N, H, W, C, stream_of(z));
-      else
+      if (z.is_cuda()) {
+        if (node) signs = fresh({out.numel() / 8}, at::kInt, z);
+        model_ops::bias_relu_pool_only_bf16(z.data_ptr(), out.data_ptr(), bs.data_ptr(), N, H, W, C, stream_of(z),
+                                            node ? signs.data_ptr() : nullptr);
+      } else
         model_ops::bias_relu_pool_only_bf16_host(z.data_ptr(), out.data_ptr(), bs.data_ptr(), N, H, W, C);
     } else {
       out = z;
-      if (z.is_cuda())
-        model_ops::bias_relu_inplace_bf16(z.data_ptr(), bs.data_ptr(), rows, C, stream_of(z));
-      else
+      if (z.is_cuda()) {
+        if (node) signs = fresh({z.numel() / 8}, at::kByte, z);
+        model_ops::bias_relu_inplace_bf16(z.data_ptr(), bs.data_ptr(), rows, C, stream_of(z), node ? signs.data_ptr() : nullptr);
+      } else
         model_ops::bias_relu_inplace_bf16_host(z.data_ptr(), bs.data_ptr(), rows, C);
     }
     if (z.is_cuda()) count_launches(1);
@@ -860,7 +868,11 @@ at::Tensor conv_bias_relu(const at::Tensor& x, const at::Tensor& weight, const a
     if (accumulate) node->accumulate_gradients({&weight, &bias});
     torch::autograd::set_history(out, node);
     node->b = SavedVariable(bs, false);
-    node->act = pool ? SavedVariable(z, false) : SavedVariable(out, /*is_output=*/true);
+    node->signs = SavedVariable(signs, false);
+    if (!pool)
+      node->act = SavedVariable(out, /*is_output=*/true);
+    else if (!signs.defined())
+      node->act = SavedVariable(z, false);
   }
   return out;
 }

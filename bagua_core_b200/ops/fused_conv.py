@@ -56,7 +56,7 @@ class _ConvBiasReLUFn:
 class _ConvBiasReLUPoolFn:
     """conv → bias + ReLU → 2x2 max pooling.  The full-resolution activation is never written: the
     backward, which produces the convolution's output gradient and the bias gradient in one pass,
-    makes it again from the convolution's output and the bias."""
+    routes the gradient by four bits per pooled value that the forward leaves."""
 
     @staticmethod
     def apply(x, weight, bias, stride, padding, dilation, groups):

@@ -467,6 +467,39 @@ def test_first_layer_gradients_match_fp32_math(N, H, W, Ci, C, in_place):
     assert ((got - want).abs() <= 4.1e-3 * want.abs() + 1e-5 * want.abs().max()).all()
 
 
+@pytest.mark.parametrize("N,C,H,W", [(1, 8, 2, 2), (2, 64, 6, 10), (1, 2048, 4, 2), (3, 16, 1, 7), (5, 32, 34, 38), (2, 128, 3, 5), (8, 64, 112, 96)])
+@pytest.mark.parametrize("pool", [False, True])
+def test_blocks_keep_the_signs_and_places_that_their_backward_needs(N, C, H, W, pool):
+    """An identity as convolution, and few values, so that windows are full of ties, zeros and negative zeros."""
+    from bagua_core_b200.ops.fused_conv import ConvBiasReLU, ConvBiasReLUPool
+
+    if pool and (H % 2 or W % 2):
+        pytest.skip("windows do not tile the image: the framework's path")
+    g = torch.Generator(device="cuda").manual_seed(C + H)
+
+    def draw(*shape):
+        return (torch.randint(-2, 3, shape, device="cuda", generator=g) / 2).to(torch.bfloat16)
+
+    m = (ConvBiasReLUPool if pool else ConvBiasReLU)(C, C, 1).cuda().to(dtype=torch.bfloat16)
+    with torch.no_grad():
+        m.weight.copy_(torch.eye(C).view(C, C, 1, 1))
+        m.bias.copy_(torch.where(torch.rand(C, device="cuda", generator=g) < 0.5, -0.0, -0.5))
+    x = draw(N, H, W, C).permute(0, 3, 1, 2).requires_grad_()
+    ref = x.detach().clone(memory_format=torch.preserve_format).requires_grad_()
+    z = ref + m.bias.detach().view(1, -1, 1, 1)
+    z.retain_grad()
+    want = torch.relu(z)
+    want = torch.nn.functional.max_pool2d(want, 2, 2) if pool else want
+    y = m(x)
+    assert torch.equal(y, want)
+    dy = draw(*y.permute(0, 2, 3, 1).shape).permute(0, 3, 1, 2)
+    y.backward(dy)
+    want.backward(dy)
+    assert torch.equal(x.grad, ref.grad)
+    # sums of halves are exact in fp32
+    assert torch.equal(m.bias.grad, z.grad.float().sum((0, 2, 3)).to(torch.bfloat16))
+
+
 # rectangles that end with the image and that reach over it, one and several strips, rows in pairs, one block and many splits
 @pytest.mark.parametrize("N,H,W,Ci,Co", [(1, 1, 1, 64, 64), (2, 3, 7, 64, 128), (1, 14, 14, 128, 64), (3, 17, 23, 192, 64), (1, 5, 57, 64, 64),
                                          (2, 65, 129, 64, 64), (1, 1, 3, 128, 128), (2, 9, 11, 128, 256), (5, 28, 28, 256, 128),
