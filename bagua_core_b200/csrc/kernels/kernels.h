@@ -89,8 +89,9 @@ void decompress_minmax_u8(const uint8_t* in, size_t in_bytes, int64_t chunk_size
 
 namespace cuda {
 // Two rounds of compress / decompress of one chunk of n elements, in place: what a low-precision exchange leaves of a
-// tensor.  Scratch as for compress with one chunk.
+// tensor.  Scratch: cleared memory of the size given, as for compress.
 // Weak: the engine's host sources are also linked without its kernels (a host-only stress program).
+size_t quantise_twice_scratch_bytes(int64_t bytes) __attribute__((weak));
 void quantise_twice_minmax_u8(void* x, DType dt, int64_t n, void* scratch, size_t scratch_bytes, cudaStream_t s)
     __attribute__((weak));
 }  // namespace cuda

@@ -38,6 +38,25 @@ inline void launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, cudaS
   launch_overlapped_shared(kernel, grid, block, 0, s, args...);
 }
 
+// `clusters` clusters of `blocks` blocks each, which may start while the kernel in front of them ends.  More than 8 blocks need
+// cudaFuncAttributeNonPortableClusterSizeAllowed.
+template <typename... P, typename... A>
+inline void launch_clusters(void (*kernel)(P...), int clusters, int blocks, dim3 block, cudaStream_t s, A... args) {
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)blocks;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(clusters * blocks));
+  cfg.blockDim = block;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  BAGUA_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+}
+
 // All blocks of the grid are resident together, or the launch fails.
 template <typename... P, typename... A>
 inline void launch_cooperative(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A... args) {

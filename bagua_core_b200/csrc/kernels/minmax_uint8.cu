@@ -1,18 +1,17 @@
 // MinMaxUInt8 compression for sm_100a: per-chunk min/max, quantise, dequantise.
 //
-// One launch per compress call, whatever the number of chunks.  A chunk belongs to a set of blocks that
-// are resident together: each reads its slice once, the set agrees on the chunk's min and max through
-// slots in global memory, and each quantises its slice.  The last 64 KiB that a block has read stay in its
-// registers between the two passes, so up to 19 MB (two blocks of 512 threads on each of 148 SMs) the
+// One launch per compress call, whatever the number of chunks.  A chunk belongs to a block, to a cluster of blocks (up to
+// 2 MB), or to a set of blocks of a launch that is resident as a whole: each block reads its slice once, they agree on the
+// chunk's min and max (through shared memory, or through slots in global memory), and each quantises its slice.  The last 64 KiB that a
+// block has read stay in its registers between the two passes, so up to 19 MB (two blocks of 512 threads on each of 148 SMs) the
 // input is read once; beyond that chunks are taken a group at a time, a group being what fits L2, and the
 // second pass runs backwards over what L2 still holds.
 //
-// Measured (kernel time; before: two launches with two full reads of the input): 16 KB of fp32 3.5 us (5.0),
-// 10 MB in 8 chunks 6.9 us (8.2), 134 MB in 8 chunks 41 us (54), 411 MB in 8 chunks 114 us (159; 78 at the
-// copy bandwidth), 206 MB of fp16 in 8 chunks 77 us (123), 1 M fp16 in 3 odd chunks 7.5 us (7.5, with
-// dequantising 3.4 us instead of 6.7).  Small calls are bound by latency (launch, one read, the exchange);
-// large ones by instructions and by what lies between the passes: at 268 MB memory sees the input and the output once,
-// at half its rate (profiles/kernel_roofline_1gpu.md).
+// Measured, us, calls back to back, compress / both directions (before clusters, and with the dequantiser's loads behind its table):
+// 16 KB of fp32 2.8 / 4.9 (3.0 / 4.8), 1 MB 4.4 / 6.9 (6.2 / 8.7), 10 MB in 8 chunks 7.5 / 11.6 (8.2 / 13.3), 1 M fp16 in 3 odd
+// chunks 7.7 / 10.2 (9.9 / 12.9), 411 MB in 8 chunks 116.9 / 212 (116.3 / 216; 78 / 157 at the copy bandwidth), 206 MB of fp16
+// 77.8 / 131.8.  Small calls are bound by latency (launch, one read, the exchange); large ones by what lies between the passes: at
+// 268 MB memory sees the input and the output once, at half its rate (profiles/kernel_roofline_1gpu.md).
 //
 // The reference issues two CUB DeviceReduce calls per chunk from a host loop
 // (bagua-core-internal/kernels/bagua_kernels.cu:312-371,533-560) and quantises one byte per thread
@@ -218,6 +217,44 @@ __device__ __forceinline__ bool agree(unsigned long long* mine, int part, int pe
   return all;
 }
 
+// Smaller chunks belong to a cluster instead, whose blocks agree through each other's shared memory: nothing of the launch has
+// to be resident as a whole, it may start while its predecessor ends, and it needs no slots.  (Cooperative launches follow each
+// other in steps of 2 us.)  Up to 8 chunks have up to 16 blocks each; more chunks have 8, as clusters of 16 do not find room on all
+// SMs at once.  The last slice sizes are those beyond which the launch of all SMs is as fast or faster.  us, cooperative / cluster:
+// fp32, one chunk of 128 KB 6.2/4.3, 1 MB 6.2/4.4, 1.6 MB 8.2/6.1, 2.1 MB 8.2/6.8, 3.2 MB 8.2/9.0; 8 chunks of 0.4 MB 8.2/5.2, of 1.3 MB
+// 8.2/7.5, of 2 MB 10.3/9.0; 16 chunks of 0.4 MB 8.2/8.5 by 16 and 5.8 by 8 blocks, of 1.3 MB 10.3/10.7 by 8; unaligned fp16,
+// 3 chunks of 0.7 MB 9.4/7.8, of 1.4 MB 9.5/10.2.
+constexpr int64_t kClusterSlice = 32 << 10;  // aimed at
+// Blocks of the cluster that handles a chunk of this size; 1: a block alone, 0: no cluster.
+int cluster_blocks(int64_t chunk_bytes, int count, bool aligned) {
+  const int most = count <= 8 ? 16 : 8;
+  if (chunk_bytes <= kTileBytes) return 1;
+  if (chunk_bytes > most * (!aligned ? kTileBytes : count <= 8 ? 2 * kTileBytes : kTileBytes + kTileBytes / 2)) return 0;
+  int n = 2;
+  while (n < most && n * kClusterSlice < chunk_bytes) n *= 2;
+  return n;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// The blocks of a cluster, each with its (mn, mx) in every thread, exchange them: afterwards the chunk's are those over the block's
+// threads.  The caller waits (cluster_wait) before it leaves, as its neighbours read its memory.
+__device__ __forceinline__ void agree_in_cluster(int part, int per_chunk, float& mn, float& mx) {
+  __shared__ __align__(8) float2 s_mine;
+  const int tid = (int)threadIdx.x;
+  if (tid == 0) s_mine = make_float2(mn, mx);
+  cluster_arrive();
+  cluster_wait();
+  if (tid < per_chunk && tid != part) {
+    uint32_t there;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"((uint32_t)__cvta_generic_to_shared(&s_mine)), "r"(tid));
+    float a, b;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "r"(there) : "memory");
+    mn = fminf(mn, a);
+    mx = fmaxf(mx, b);
+  }
+  cluster_arrive();
+}
+
 // Running min and max of whole vectors: 16-bit types two values at a time, without widening them.
 template <typename T>
 struct RunningMinMax;
@@ -352,13 +389,14 @@ struct Tile {
   }
 };
 
-template <typename T, bool kAligned>
+template <typename T, bool kAligned, bool kCluster>
 __global__ void __launch_bounds__(kThreads, kBlocksPerSM)
     compress_kernel(const T* __restrict__ in, int64_t num_real, int64_t chunk, int first_chunk, int count, int sets,
                     int per_group, int per_chunk, uint8_t* __restrict__ out, size_t chunk_offset, unsigned long long* slots, uint32_t tag) {
   constexpr int VE = mmdev::Vec16<T>::VE;
   const int tid = (int)threadIdx.x;
   const int slot = (int)blockIdx.x / per_chunk, part = (int)blockIdx.x % per_chunk;
+  let_successor_start();
   wait_for_predecessor();
   for (int ci = slot; ci < count; ci += sets * per_group) {
     if (sets > 1 && ci >= per_group) {
@@ -431,7 +469,10 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSM)
       }
     }
     mmdev::block_minmax<kThreads>(mn, mx);
-    if (per_chunk > 1 || sets > 1) {
+    if constexpr (kCluster) {
+      agree_in_cluster(part, per_chunk, mn, mx);
+      mmdev::block_minmax<kThreads>(mn, mx);
+    } else if (per_chunk > 1 || sets > 1) {
       const bool all = agree(slots + (size_t)ci * (per_chunk + 1) * 2, part, per_chunk, tag, mn, mx);
       if (!__syncthreads_and(all)) {  // the answer is the same, only late
         for (int64_t i = tid; i < real; i += kThreads) {
@@ -474,8 +515,11 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSM)
       if (part == 0 && tid < head) q[tid] = mmdev::quantise(to_f(p[tid]), g.g);
       if (part == per_chunk - 1 && tail + tid < chunk) q[tail + tid] = mmdev::quantise(to_f(p[tail + tid]), g.g);
     }
+    if constexpr (kCluster) {
+      cluster_wait();
+      break;  // one chunk per cluster
+    }
   }
-  let_successor_start();
 }
 
 // ---- two rounds of quantisation in place -----------------------------------------------------
@@ -574,13 +618,27 @@ void compress_t(const void* in, int64_t num_real, int64_t chunk, int n_chunks, u
   const int first = target >= 0 ? target : 0;
   const int count = target >= 0 ? 1 : n_chunks;
   const bool aligned = ((uintptr_t)in % 16 == 0) && ((uintptr_t)out % 16 == 0) && (chunk % 16 == 0) && (off % 16 == 0);
-  const Split d = split_chunks(count, chunk * (int64_t)sizeof(T), aligned, sm_count());
-  auto* kernel = aligned ? compress_kernel<T, true> : compress_kernel<T, false>;
-  if (d.sets == 1 && d.per_chunk == 1) {
-    launch_overlapped(kernel, dim3(d.grid()), dim3(kThreads), s, (const T*)in, num_real, chunk, first, count, 1, d.per_group, 1,
-                      out, off, (unsigned long long*)nullptr, 0u);
+  const int blocks = cluster_blocks(chunk * (int64_t)sizeof(T), count, aligned);
+  if (blocks == 1) {
+    launch_overlapped(aligned ? compress_kernel<T, true, false> : compress_kernel<T, false, false>, dim3(count), dim3(kThreads), s,
+                      (const T*)in, num_real, chunk, first, count, 1, count, 1, out, off, (unsigned long long*)nullptr, 0u);
     return;
   }
+  if (blocks > 1) {
+    auto* kernel = aligned ? compress_kernel<T, true, true> : compress_kernel<T, false, true>;
+    static std::atomic<uint64_t> allowed[2] = {};  // by device; set twice does no harm
+    int dev = 0;
+    BAGUA_CUDA_CHECK(cudaGetDevice(&dev));
+    if (!(allowed[aligned].load(std::memory_order_relaxed) >> (dev & 63) & 1)) {
+      BAGUA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+      allowed[aligned] |= 1ull << (dev & 63);
+    }
+    launch_clusters(kernel, count, blocks, dim3(kThreads), s, (const T*)in, num_real, chunk, first, count, 1, count, blocks, out, off,
+                    (unsigned long long*)nullptr, 0u);
+    return;
+  }
+  const Split d = split_chunks(count, chunk * (int64_t)sizeof(T), aligned, sm_count());
+  auto* kernel = aligned ? compress_kernel<T, true, false> : compress_kernel<T, false, false>;
   BAGUA_CHECK(scratch != nullptr && scratch_bytes >= slot_bytes(count, d.per_chunk), MemPool,
               "compress: scratch buffer too small");
   const uint32_t tag = next_tag();
@@ -589,10 +647,14 @@ void compress_t(const void* in, int64_t num_real, int64_t chunk, int n_chunks, u
 }
 
 // ---- decompress ----------------------------------------------------------------------------
+// kVecs quantised words per thread are in flight.  kAhead: the first of them before the table is made and the others behind the stores
+// of those in front, for blocks that have many (411 MB of fp32: 90.4 us, 95-97 with the loads behind the table; half as much fp16:
+// 53.2, 55.5-58); where a thread has a few words, four at a time behind the table are the faster (10 MB of fp32: 3.8 us, 4.6-5.2
+// with eight, of whose places most are empty; 4 MB of fp16 3.4, 3.8-4.0).
 constexpr int kDqThreads = 256;
-constexpr int kDqVecs = 8;  // quantised words in flight per thread
+constexpr int kDqMany = 8, kDqFew = 4;
 
-template <typename T, bool kAligned>
+template <typename T, bool kAligned, int kDqVecs, bool kAhead>
 __global__ void __launch_bounds__(kDqThreads)
     dequantise_kernel(const uint8_t* __restrict__ in, size_t chunk_offset, int64_t chunk, T* __restrict__ out) {
   constexpr int VE = mmdev::Vec16<T>::VE;
@@ -608,19 +670,24 @@ __global__ void __launch_bounds__(kDqThreads)
   const int64_t tail = head + nvec * VE;
   const int64_t per = ((nvec + gridDim.x - 1) / gridDim.x + 31) & ~(int64_t)31;
   const int64_t lo = min((int64_t)blockIdx.x * per, nvec), hi = min(lo + per, nvec);
+  const uint64_t policy = evict_first_policy();
+  typename mmdev::QWord<VE>::type w[kDqVecs];
+  // all words before the first store: the compiler may not move a load over a store
+  auto load = [&](int64_t v0) {
+#pragma unroll
+    for (int u = 0; u < kDqVecs; ++u)
+      if (v0 + u * kDqThreads < hi) w[u] = load_bytes<kAligned, VE>(q + head, v0 + u * kDqThreads);
+  };
+  let_successor_start();
   wait_for_predecessor();
+  if constexpr (kAhead) load(lo + tid);
   float mn, mx;
   mmdev::load_header<T>(base, mn, mx);
   const mmdev::Grid g = mmdev::make_grid(mn, mx);
   mmdev::build_dequant_lut<T>(s_lut, g);
   __syncthreads();
-  const uint64_t policy = evict_first_policy();
-  typename mmdev::QWord<VE>::type w[kDqVecs];
-  for (int64_t v0 = lo + tid; v0 < hi; v0 += (int64_t)kDqVecs * kDqThreads) {
-    // all words before the first store: the compiler may not move a load over a store
-#pragma unroll
-    for (int u = 0; u < kDqVecs; ++u)
-      if (v0 + u * kDqThreads < hi) w[u] = load_bytes<kAligned, VE>(q + head, v0 + u * kDqThreads);
+  for (int64_t v0 = lo + tid; v0 < hi;) {
+    if constexpr (!kAhead) load(v0);
 #pragma unroll
     for (int u = 0; u < kDqVecs; ++u) {
       if (v0 + u * kDqThreads >= hi) continue;
@@ -630,12 +697,13 @@ __global__ void __launch_bounds__(kDqThreads)
       mmdev::store_vec(reinterpret_cast<T*>(&r), 0, f);
       store_first(reinterpret_cast<uint4*>(o + head) + v0 + u * kDqThreads, r, policy);
     }
+    v0 += (int64_t)kDqVecs * kDqThreads;
+    if constexpr (kAhead) load(v0);
   }
   if constexpr (!kAligned) {
     if (blockIdx.x == 0 && tid < head) o[tid] = from_f<T>(s_lut[q[tid]]);
     if (blockIdx.x == gridDim.x - 1 && tail + tid < chunk) o[tail + tid] = from_f<T>(s_lut[q[tail + tid]]);
   }
-  let_successor_start();
 }
 
 // Over one rank this runs beside a backward pass, as a cooperative launch that starts when all its blocks fit.  It takes
@@ -664,7 +732,9 @@ void decompress_t(const uint8_t* in, size_t in_bytes, int64_t chunk, int n_chunk
   const int64_t want = (chunk / VE + kDqThreads * 2 - 1) / (kDqThreads * 2);
   const int64_t cap = std::max<int64_t>(1, (int64_t)sm_count() * 8 / n_chunks);
   dim3 grid((unsigned)std::max<int64_t>(1, std::min(want, cap)), (unsigned)n_chunks);
-  auto* kernel = aligned ? dequantise_kernel<T, true> : dequantise_kernel<T, false>;
+  const bool many = chunk / VE > (int64_t)grid.x * kDqThreads * kDqMany;
+  auto* kernel = many ? (aligned ? dequantise_kernel<T, true, kDqMany, true> : dequantise_kernel<T, false, kDqMany, true>)
+                      : (aligned ? dequantise_kernel<T, true, kDqFew, false> : dequantise_kernel<T, false, kDqFew, false>);
   launch_overlapped(kernel, grid, dim3(kDqThreads), s, in, off, chunk, (T*)out);
 }
 
@@ -672,8 +742,10 @@ void decompress_t(const uint8_t* in, size_t in_bytes, int64_t chunk, int n_chunk
 
 size_t compress_scratch_bytes(int n_chunks, int64_t bytes) {
   // a call for one chunk of the buffer may give that chunk more blocks than a call for all of them
-  const Split all = split_chunks(n_chunks, bytes, false, sm_count()), one = split_chunks(1, bytes, false, sm_count());
-  return bytes <= kTileBytes ? 0 : std::max(slot_bytes(n_chunks, all.per_chunk), slot_bytes(1, one.per_chunk));
+  size_t most = 0;
+  for (int count : {n_chunks, 1})
+    if (!cluster_blocks(bytes, count, false)) most = std::max(most, slot_bytes(count, split_chunks(count, bytes, false, sm_count()).per_chunk));
+  return most;
 }
 
 void compress_minmax_u8(const void* in, DType dt, int64_t num_real, int64_t chunk, int n_chunks, uint8_t* out,
@@ -692,6 +764,9 @@ void compress_minmax_u8(const void* in, DType dt, int64_t num_real, int64_t chun
   }
 }
 
+size_t quantise_twice_scratch_bytes(int64_t bytes) {
+  return bytes <= kTileBytes ? 0 : slot_bytes(1, split_chunks(1, bytes, true, sm_count()).per_chunk);
+}
 void quantise_twice_minmax_u8(void* x, DType dt, int64_t n, void* scratch, size_t scratch_bytes, cudaStream_t s) {
   switch (dt) {
     case DType::F32: quantise_twice_t<float>(x, n, scratch, scratch_bytes, s); return;

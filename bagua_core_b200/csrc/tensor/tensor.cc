@@ -107,7 +107,7 @@ void quantise_twice(RawTensor& t, const std::string& method, uint64_t stream) {
               "quantise_twice works on CUDA tensors");
   const int64_t n = t.num_elements_allocated();
   if (n == 0) return;
-  const size_t bytes = kernels::compress_scratch_bytes(1, n, t.dtype());
+  const size_t bytes = kernels::cuda::quantise_twice_scratch_bytes(n * (int64_t)dtype_bytes(t.dtype()));
   std::shared_ptr<PoolBlock> scratch;
   if (bytes) scratch = MemoryPool::for_device(t.device_id()).pull_cleared(bytes, stream);
   kernels::cuda::quantise_twice_minmax_u8(t.data_ptr(), t.dtype(), n, scratch ? scratch->ptr() : nullptr, bytes,

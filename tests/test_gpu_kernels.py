@@ -379,6 +379,16 @@ def test_minmax_uint8_splits_of_a_chunk_match_the_host(n_chunks, chunk, jump, dt
     assert (err <= step.cpu() * 1.01 + _tol(dt) * x.float().abs().max().item()).all()
 
 
+# one block, clusters of 2 to 16, the last cluster and the first launch of all SMs; more than 8 chunks; with one element more
+@pytest.mark.parametrize("nbytes,n_chunks", [(65536, 3), (65600, 1), (131136, 2), (524352, 1), (2097152, 1), (2097216, 1), (2097152, 2),
+                                             (400064, 9), (786432, 9), (786496, 9), (1048576, 3), (1048640, 3)])
+@pytest.mark.parametrize("odd", [0, 1])
+@pytest.mark.parametrize("dt", DTYPES)
+def test_compression_on_both_sides_of_the_rule_for_clusters(nbytes, n_chunks, odd, dt):
+    chunk = nbytes // torch.empty((), dtype=dt).element_size() + odd
+    test_minmax_uint8_splits_of_a_chunk_match_the_host(n_chunks, chunk, (n_chunks - 1) * chunk + chunk * 2 // 3, dt)
+
+
 def test_minmax_uint8_values_large_against_their_range_and_not_finite():
     """Levels beyond 2^22 (a narrow range far from zero), NaN and infinities: the same bytes as the host."""
     import bagua_core as bc
