@@ -61,6 +61,19 @@ struct MultiCopySeg {
 };
 void multi_copy(const MultiCopySeg* segs, int nseg, void* flat, size_t total_bytes, bool gather, const Ctx& c);
 
+// Buckets that are handed to the GPU together, in one launch each way.
+constexpr int kMaxJoined = 16;
+struct MultiCopyItem {
+  const MultiCopySeg* segs;  // on the device
+  int nseg;
+  void* flat;
+  size_t bytes;
+};
+struct QuantiseItem {
+  void* x;
+  int64_t n;
+};
+
 // x viewed as [num_chunks][chunk_size]: column sum (fp32, chunk order 0..n-1), optional
 // division by num_chunks, written into chunk `target_chunk`.
 void reduce_chunk_inplace(void* x, DType dt, int64_t chunk_size, int num_chunks, int target_chunk,
@@ -88,12 +101,13 @@ void decompress_minmax_u8(const uint8_t* in, size_t in_bytes, int64_t chunk_size
                           void* out, DType dt, const Ctx& c);
 
 namespace cuda {
-// Two rounds of compress / decompress of one chunk of n elements, in place: what a low-precision exchange leaves of a
-// tensor.  Scratch: cleared memory of the size given, as for compress.
+// Two rounds of compress / decompress of up to kMaxJoined buffers, each as one chunk, in place: what a low-precision exchange leaves of
+// a tensor.  Scratch: cleared memory of the size given, as for compress.
 // Weak: the engine's host sources are also linked without its kernels (a host-only stress program).
-size_t quantise_twice_scratch_bytes(int64_t bytes) __attribute__((weak));
-void quantise_twice_minmax_u8(void* x, DType dt, int64_t n, void* scratch, size_t scratch_bytes, cudaStream_t s)
+size_t quantise_twice_scratch_bytes(const QuantiseItem* items, int count, DType dt) __attribute__((weak));
+void quantise_twice_minmax_u8(const QuantiseItem* items, int count, DType dt, void* scratch, size_t scratch_bytes, cudaStream_t s)
     __attribute__((weak));
+void multi_copy_joined(const MultiCopyItem* items, int count, bool gather, cudaStream_t s) __attribute__((weak));
 }  // namespace cuda
 
 // Scalar definition of the quantiser, shared by host code and tests.

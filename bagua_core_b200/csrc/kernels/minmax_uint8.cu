@@ -537,12 +537,26 @@ __device__ __forceinline__ void build_twice_lut(float* lut, const Quantiser& g) 
   if (q < 256) lut[q] = to_f(from_f<T>(mmdev::dequantise(mmdev::quantise(once(q), second), second)));
 }
 
+// The buffers of a launch, which share its blocks by their sizes: all read, agree and write at the same time, so that several buffers pay
+// for the latencies of one.
+struct QuantiseBatch {
+  QuantiseItem item[kMaxJoined];
+  int end[kMaxJoined];  // blocks up to the buffer's last; its slots, one more than blocks, lie in the same order
+  int count;
+};
+
 template <typename T>
 __global__ void __launch_bounds__(kThreads, kBlocksPerSM)
-    quantise_twice_kernel(T* x, int64_t n, unsigned long long* slots, uint32_t tag) {
+    quantise_twice_kernel(const __grid_constant__ QuantiseBatch batch, unsigned long long* all_slots, uint32_t tag) {
   constexpr int VE = mmdev::Vec16<T>::VE;
   __shared__ float s_lut[256];
-  const int tid = (int)threadIdx.x, part = (int)blockIdx.x, parts = (int)gridDim.x;
+  const int tid = (int)threadIdx.x;
+  int k = 0, first = 0;
+  while ((int)blockIdx.x >= batch.end[k]) first = batch.end[k++];
+  const int part = (int)blockIdx.x - first, parts = batch.end[k] - first;
+  unsigned long long* slots = all_slots + 2 * (first + k);
+  T* x = (T*)batch.item[k].x;
+  const int64_t n = batch.item[k].n;
   wait_for_predecessor();
   const int64_t head = min(n, (int64_t)(((0 - reinterpret_cast<uintptr_t>(x)) & (uintptr_t)15) / sizeof(T)));
   const int64_t nvec = (n - head) / VE, tail = head + nvec * VE;
@@ -554,9 +568,9 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSM)
   Tile<T, true> tile;
   const int64_t tiles = (m + kTile - 1) / kTile;
   for (int64_t t = 0; t < tiles; ++t) {  // the last tile stays in registers
-    const int k = (int)min((int64_t)kTile, m - t * kTile);
-    tile.load(xv + t * kTile * VE, k);
-    tile.minmax_all(k, (int64_t)k * VE, run, mn, mx);
+    const int many = (int)min((int64_t)kTile, m - t * kTile);
+    tile.load(xv + t * kTile * VE, many);
+    tile.minmax_all(many, (int64_t)many * VE, run, mn, mx);
   }
   {
     float a, b;
@@ -586,11 +600,11 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSM)
   build_twice_lut<T>(s_lut, g);
   __syncthreads();
   for (int64_t t = tiles - 1; t >= 0; --t) {
-    const int k = (int)min((int64_t)kTile, m - t * kTile);
-    if (t != tiles - 1) tile.load(xv + t * kTile * VE, k);
+    const int many = (int)min((int64_t)kTile, m - t * kTile);
+    if (t != tiles - 1) tile.load(xv + t * kTile * VE, many);
 #pragma unroll
     for (int u = 0; u < kVecs; ++u) {
-      if (tid + u * kThreads >= k) continue;
+      if (tid + u * kThreads >= many) continue;
       float f[VE];
       widen(tile.raw[u], f, (const T*)nullptr);
       mmdev::lut_word(g.pack(f), f, s_lut);
@@ -711,16 +725,38 @@ __global__ void __launch_bounds__(kDqThreads)
 // peer, and is gone sooner than a smaller launch that occupies fewer SMs for longer.  Training steps with ByteGrad, us, with all
 // (160 blocks for 10 MB) / 148 / 64 / 32 / 16: VGG-16, batch 32: 4771 / 4766 / 4756 / 4844 / 5276; 8 layers of BERT-large, 8 x 384
 // tokens: 5000 / 5113-5540 / 5041 / 5162 / 5350.
+QuantiseBatch quantise_batch(const QuantiseItem* items, int count, int64_t esize) {
+  QuantiseBatch b;
+  b.count = count;
+  const int64_t all = (int64_t)sm_count() * kBlocksPerSM;
+  int64_t wanted = 0, parts[kMaxJoined];
+  for (int k = 0; k < count; ++k) {
+    b.item[k] = items[k];
+    wanted += parts[k] = split_chunks(1, items[k].n * esize, true, sm_count()).per_chunk;
+  }
+  int blocks = 0;
+  for (int k = 0; k < count; ++k) {
+    // more than there is room for: each buffer's share, rounded so that the sum fits
+    if (wanted > all) parts[k] = std::max<int64_t>(1, parts[k] * (all - count) / wanted);
+    b.end[k] = blocks += (int)parts[k];
+  }
+  return b;
+}
+size_t batch_slot_bytes(const QuantiseBatch& b) {
+  const int blocks = b.end[b.count - 1];
+  return blocks == b.count ? 0 : (size_t)(blocks + b.count) * kSlotBytes;  // a block alone waits for nobody
+}
+
 template <typename T>
-void quantise_twice_t(void* x, int64_t n, void* scratch, size_t scratch_bytes, cudaStream_t s) {
-  const Split d = split_chunks(1, n * (int64_t)sizeof(T), true, sm_count());
-  if (d.per_chunk == 1) {
-    launch_overlapped(quantise_twice_kernel<T>, dim3(1), dim3(kThreads), s, (T*)x, n, (unsigned long long*)nullptr, 0u);
+void quantise_twice_t(const QuantiseItem* items, int count, void* scratch, size_t scratch_bytes, cudaStream_t s) {
+  const QuantiseBatch b = quantise_batch(items, count, (int64_t)sizeof(T));
+  const dim3 grid(b.end[b.count - 1]);
+  if (batch_slot_bytes(b) == 0) {  // nobody waits for anybody
+    launch_overlapped(quantise_twice_kernel<T>, grid, dim3(kThreads), s, b, (unsigned long long*)nullptr, 0u);
     return;
   }
-  BAGUA_CHECK(scratch != nullptr && scratch_bytes >= slot_bytes(1, d.per_chunk), MemPool, "quantise_twice: scratch too small");
-  launch_cooperative(quantise_twice_kernel<T>, dim3(d.per_chunk), dim3(kThreads), s, (T*)x, n, (unsigned long long*)scratch,
-                     next_tag());
+  BAGUA_CHECK(scratch != nullptr && scratch_bytes >= batch_slot_bytes(b), MemPool, "quantise_twice: scratch too small");
+  launch_cooperative(quantise_twice_kernel<T>, grid, dim3(kThreads), s, b, (unsigned long long*)scratch, next_tag());
 }
 
 template <typename T>
@@ -764,14 +800,15 @@ void compress_minmax_u8(const void* in, DType dt, int64_t num_real, int64_t chun
   }
 }
 
-size_t quantise_twice_scratch_bytes(int64_t bytes) {
-  return bytes <= kTileBytes ? 0 : slot_bytes(1, split_chunks(1, bytes, true, sm_count()).per_chunk);
+size_t quantise_twice_scratch_bytes(const QuantiseItem* items, int count, DType dt) {
+  return batch_slot_bytes(quantise_batch(items, count, (int64_t)dtype_bytes(dt)));
 }
-void quantise_twice_minmax_u8(void* x, DType dt, int64_t n, void* scratch, size_t scratch_bytes, cudaStream_t s) {
+void quantise_twice_minmax_u8(const QuantiseItem* items, int count, DType dt, void* scratch, size_t scratch_bytes, cudaStream_t s) {
+  BAGUA_CHECK(count > 0 && count <= kMaxJoined, Tensor, "quantise_twice: " << count << " buffers");
   switch (dt) {
-    case DType::F32: quantise_twice_t<float>(x, n, scratch, scratch_bytes, s); return;
-    case DType::F16: quantise_twice_t<__half>(x, n, scratch, scratch_bytes, s); return;
-    case DType::BF16: quantise_twice_t<__nv_bfloat16>(x, n, scratch, scratch_bytes, s); return;
+    case DType::F32: quantise_twice_t<float>(items, count, scratch, scratch_bytes, s); return;
+    case DType::F16: quantise_twice_t<__half>(items, count, scratch, scratch_bytes, s); return;
+    case DType::BF16: quantise_twice_t<__nv_bfloat16>(items, count, scratch, scratch_bytes, s); return;
     default: throw BaguaError(ErrorKind::Tensor, std::string("compress: unsupported dtype ") + dtype_name(dt));
   }
 }

@@ -1,4 +1,4 @@
-// Flatten / unflatten of a staged bucket in ONE launch.
+// Flatten / unflatten of a staged bucket, or of several, in ONE launch.
 //
 // A bucket whose tensors are not address-contiguous is communicated through a flat staging
 // buffer (reference: one cudaMemcpyAsync per tensor into the buffer and one per tensor back,
@@ -61,54 +61,100 @@ __device__ __forceinline__ void copy_range(char* __restrict__ dst, const char* _
   if (tid < n - done) dst[nv * 16 + tid] = src[nv * 16 + tid];
 }
 
-__global__ void __launch_bounds__(kMcThreads)
-    multi_copy_kernel(const MultiCopySeg* __restrict__ segs, int nseg, char* flat, unsigned long long total, int gather) {
+// Buckets that are copied in one launch; a bucket's tiles follow those of the ones in front of it.  (As few as there are: a launch with
+// 650 bytes of parameters reaches the GPU 2-3 us later than one with 50.)
+template <int kMost>
+struct Joined {
+  MultiCopyItem item[kMost];
+  unsigned long long end[kMost];  // tiles up to the bucket's last
+  int count;
+};
+
+// Bytes t0 to t1, a tile, of a bucket's flat range.
+__device__ __forceinline__ void copy_tile(const MultiCopySeg* __restrict__ segs, int nseg, char* flat, unsigned long long t0,
+                                          unsigned long long t1, int gather) {
   __shared__ MultiCopySeg s_seg[32];
   const int tid = (int)threadIdx.x;
-  const unsigned long long ntiles = (total + kTileBytes - 1) / kTileBytes;
-  wait_for_predecessor();
-  for (unsigned long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const unsigned long long t0 = tile * kTileBytes, t1 = min(t0 + kTileBytes, total);
-    // segments are sorted by offset and do not overlap: the first of the tile is the number of those that end in front
-    int first = 0;
-    for (int k0 = 0; k0 < nseg; k0 += kMcThreads) {
-      const int k = k0 + tid;
-      const int n = __syncthreads_count(k < nseg && segs[k].offset + segs[k].bytes <= t0);
-      first += n;
-      if (n < kMcThreads) break;
-    }
-    bool more = true;
-    for (int k0 = first; more && k0 < nseg; k0 += 32) {
-      if (tid < 32 && k0 + tid < nseg) s_seg[tid] = segs[k0 + tid];
-      __syncthreads();
-      for (int k = 0; k < 32 && k0 + k < nseg; ++k) {
-        const MultiCopySeg& sg = s_seg[k];
-        if (sg.offset >= t1) {
-          more = false;
-          break;
-        }
-        const unsigned long long a = max(sg.offset, t0), b = min(sg.offset + sg.bytes, t1);
-        if (b <= a) continue;
-        char* in_flat = flat + a;
-        char* in_tensor = reinterpret_cast<char*>(sg.ptr) + (a - sg.offset);
-        if (gather)
-          copy_range(in_flat, in_tensor, (int)(b - a));
-        else
-          copy_range(in_tensor, in_flat, (int)(b - a));
+  // segments are sorted by offset and do not overlap: the first of the tile is the number of those that end in front
+  int first = 0;
+  for (int k0 = 0; k0 < nseg; k0 += kMcThreads) {
+    const int k = k0 + tid;
+    const int n = __syncthreads_count(k < nseg && segs[k].offset + segs[k].bytes <= t0);
+    first += n;
+    if (n < kMcThreads) break;
+  }
+  bool more = true;
+  for (int k0 = first; more && k0 < nseg; k0 += 32) {
+    if (tid < 32 && k0 + tid < nseg) s_seg[tid] = segs[k0 + tid];
+    __syncthreads();
+    for (int k = 0; k < 32 && k0 + k < nseg; ++k) {
+      const MultiCopySeg& sg = s_seg[k];
+      if (sg.offset >= t1) {
+        more = false;
+        break;
       }
-      __syncthreads();
+      const unsigned long long a = max(sg.offset, t0), b = min(sg.offset + sg.bytes, t1);
+      if (b <= a) continue;
+      char* in_flat = flat + a;
+      char* in_tensor = reinterpret_cast<char*>(sg.ptr) + (a - sg.offset);
+      if (gather)
+        copy_range(in_flat, in_tensor, (int)(b - a));
+      else
+        copy_range(in_tensor, in_flat, (int)(b - a));
     }
+    __syncthreads();
+  }
+}
+
+template <int kMost>
+__global__ void __launch_bounds__(kMcThreads)
+    multi_copy_kernel(const __grid_constant__ Joined<kMost> joined, int gather) {
+  wait_for_predecessor();
+  int bucket = 0;
+  unsigned long long before = 0;  // tiles in front of the bucket
+  const unsigned long long tiles = joined.end[kMost == 1 ? 0 : joined.count - 1];
+  for (unsigned long long at = blockIdx.x; at < tiles; at += gridDim.x) {
+    if constexpr (kMost > 1)
+      while (at >= joined.end[bucket]) before = joined.end[bucket++];
+    const MultiCopyItem& item = joined.item[kMost == 1 ? 0 : bucket];
+    const unsigned long long t0 = (at - before) * kTileBytes;
+    copy_tile(item.segs, item.nseg, (char*)item.flat, t0, min(t0 + kTileBytes, (unsigned long long)item.bytes), gather);
   }
 }
 
 }  // namespace
 
+namespace {
+template <int kMost>
+void launch_joined(const MultiCopyItem* items, int count, bool gather, cudaStream_t s) {
+  Joined<kMost> j;
+  j.count = 0;
+  unsigned long long tiles = 0;
+  for (int k = 0; k < count; ++k) {
+    if (items[k].nseg <= 0 || items[k].bytes == 0) continue;
+    tiles += (items[k].bytes + kTileBytes - 1) / kTileBytes;
+    j.item[j.count] = items[k];
+    j.end[j.count++] = tiles;
+  }
+  if (tiles == 0) return;
+  const int grid = (int)std::min<unsigned long long>(tiles, (unsigned long long)sm_count() * 8ull);
+  launch_overlapped(multi_copy_kernel<kMost>, dim3(grid), dim3(kMcThreads), s, j, gather ? 1 : 0);
+}
+}  // namespace
+
+void multi_copy_joined(const MultiCopyItem* items, int count, bool gather, cudaStream_t s) {
+  BAGUA_CHECK(count <= kMaxJoined, Tensor, "too many buckets for one launch");
+  if (count == 1)
+    launch_joined<1>(items, count, gather, s);
+  else if (count <= 4)
+    launch_joined<4>(items, count, gather, s);
+  else
+    launch_joined<kMaxJoined>(items, count, gather, s);
+}
+
 void multi_copy(const MultiCopySeg* segs_dev, int nseg, void* flat, size_t total_bytes, bool gather, cudaStream_t s) {
-  if (nseg <= 0 || total_bytes == 0) return;
-  const unsigned long long ntiles = (total_bytes + kTileBytes - 1) / kTileBytes;
-  const int grid = (int)std::min<unsigned long long>(ntiles, (unsigned long long)sm_count() * 8ull);
-  launch_overlapped(multi_copy_kernel, dim3(grid), dim3(kMcThreads), s, segs_dev, nseg, (char*)flat,
-                    (unsigned long long)total_bytes, gather ? 1 : 0);
+  const MultiCopyItem one{segs_dev, nseg, flat, total_bytes};
+  multi_copy_joined(&one, 1, gather, s);
 }
 
 }  // namespace cuda

@@ -29,6 +29,13 @@ class CommOp {
  public:
   virtual ~CommOp() = default;
   virtual void execute_background_communication(const BucketPtr& bucket) = 0;
+  // Whether the op's part on `bucket` is one that several buckets can do in one launch, and if so with `other`, the op of another
+  // bucket, too.  Such buckets may be executed together, by one of their ops; the results are those of one after the other.
+  virtual bool joins(const BucketPtr& /*bucket*/) const { return false; }
+  virtual bool joins_with(const CommOp& /*other*/) const { return false; }
+  virtual void execute_joined(const std::vector<BucketPtr>& buckets) {
+    for (const BucketPtr& b : buckets) execute_background_communication(b);
+  }
   virtual std::string describe() const = 0;
   // State worth checkpointing (e.g. the gossip step counter); empty for stateless ops.
   virtual std::vector<std::pair<std::string, int64_t>> state() const { return {}; }

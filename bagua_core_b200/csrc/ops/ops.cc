@@ -5,6 +5,8 @@
 
 #include <cstdio>
 #include <cstdlib>
+#include <deque>
+#include <functional>
 
 #include "../comm/arena.h"
 #include "../kernels/fused.h"
@@ -63,9 +65,10 @@ void note_fallback() { EngineStats::global().library_fallbacks++; }
 
 struct OpFrame {
   // Common prologue/epilogue of an op: lock, stream, communication tensor, release.
-  OpFrame(const BucketPtr& bucket, Communicator& comm, bool force_copy, bool no_copy_back)
+  OpFrame(const BucketPtr& bucket, Communicator& comm, bool force_copy, bool no_copy_back,
+          std::vector<kernels::MultiCopyItem>* gather = nullptr)
       : lock(bucket->exec_mutex()), stream(comm.stream()) {
-    ct = bucket->get_communication_tensor(stream, force_copy, no_copy_back);
+    ct = bucket->get_communication_tensor(stream, force_copy, no_copy_back, gather);
     if (ct.staged) EngineStats::global().staged_copies++;
     EngineStats::global().bytes_communicated += ct.raw->bytes_allocated();
     gpu = ct.raw->device_id() >= 0;
@@ -85,6 +88,36 @@ struct OpFrame {
   bool gpu = false;
   uint64_t ticket = 0;
 };
+
+// Buckets of a communicator of one rank on a GPU: nothing travels, each bucket's part is local, and several that are ready at once are
+// gathered, worked on and scattered in one launch each.  Not where somebody looks at them one by one.
+bool joins_over_one_rank(const Communicator& comm, const BucketPtr& bucket) {
+  return bucket->device_id() >= 0 && comm.kind() == Communicator::Kind::Single && comm.internode() && comm.internode()->nranks() == 1 &&
+         !EngineConfig::global().sync_per_bucket && !BucketTimeline::instance().enabled() &&
+         kernels::cuda::multi_copy_joined != nullptr;
+}
+void copy_joined(std::vector<kernels::MultiCopyItem>& items, bool gather, uint64_t stream) {
+  for (size_t from = 0; from < items.size(); from += kernels::kMaxJoined)
+    kernels::cuda::multi_copy_joined(items.data() + from, (int)std::min<size_t>(kernels::kMaxJoined, items.size() - from), gather,
+                                     (cudaStream_t)stream);
+}
+void run_joined(Communicator& comm, const std::vector<BucketPtr>& buckets, const std::function<void(std::vector<RawTensor*>&)>& work) {
+  std::vector<kernels::MultiCopyItem> gather, scatter;
+  std::deque<OpFrame> frames;
+  std::vector<RawTensor*> raws;
+  for (const BucketPtr& b : buckets) {
+    frames.emplace_back(b, comm, false, false, &gather);
+    raws.push_back(frames.back().ct.raw.get());
+  }
+  copy_joined(gather, true, comm.stream());
+  work(raws);
+  for (OpFrame& f : frames) f.ct.finish(false, &scatter);
+  copy_joined(scatter, false, comm.stream());
+}
+bool occupies_for_probe() {
+  static const bool on = std::getenv("BAGUA_B200_PROBE_OCCUPY") != nullptr;
+  return on;
+}
 
 // ---------------------------------------------------------------------------------
 // O1: centralized, full precision, synchronous (gradient all-reduce)
@@ -144,6 +177,17 @@ class CentralizedFullPrecisionSynchronous : public CommOp {
     o << "CentralizedFullPrecisionSynchronous{average=" << average_ << ", scattergather=" << scattergather_ << "}";
     return o.str();
   }
+  // over one rank: a bucket that is not staged is done as it is
+  bool joins(const BucketPtr& bucket) const override {
+    return joins_over_one_rank(*comm_, bucket) && !occupies_for_probe() && !bucket->contiguous();
+  }
+  bool joins_with(const CommOp& other) const override {
+    auto* o = dynamic_cast<const CentralizedFullPrecisionSynchronous*>(&other);
+    return o && o->comm_->internode() == comm_->internode();
+  }
+  void execute_joined(const std::vector<BucketPtr>& buckets) override {
+    run_joined(*comm_, buckets, [](std::vector<RawTensor*>&) {});
+  }
 
  private:
   std::shared_ptr<Communicator> comm_;
@@ -175,7 +219,7 @@ class CentralizedLowPrecisionSynchronous : public CommOp {
       if (n == 1 && t.device_id() >= 0) {
         // one rank (a single GPU, or the last tier of a hierarchical job on one box): nothing travels, the values
         // are quantised twice where they are, in one pass over them
-        tensor_ops::quantise_twice(t, method_, c.stream());
+        tensor_ops::quantise_twice({&t}, method_, c.stream());
         return;
       }
       auto compressed = tensor_ops::compress(t, method_, n, c.stream(), -1);
@@ -195,6 +239,14 @@ class CentralizedLowPrecisionSynchronous : public CommOp {
     std::ostringstream o;
     o << "CentralizedLowPrecisionSynchronous{average=" << average_ << ", compression=" << method_ << "}";
     return o.str();
+  }
+  bool joins(const BucketPtr& bucket) const override { return joins_over_one_rank(*comm_, bucket); }
+  bool joins_with(const CommOp& other) const override {
+    auto* o = dynamic_cast<const CentralizedLowPrecisionSynchronous*>(&other);
+    return o && o->comm_->internode() == comm_->internode() && o->method_ == method_;
+  }
+  void execute_joined(const std::vector<BucketPtr>& buckets) override {
+    run_joined(*comm_, buckets, [&](std::vector<RawTensor*>& ts) { tensor_ops::quantise_twice(ts, method_, comm_->stream()); });
   }
 
  private:

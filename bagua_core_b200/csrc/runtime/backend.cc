@@ -34,49 +34,102 @@ void CommBackend::worker_loop() {
     cudaError_t e = cudaSetDevice(device_id_);
     if (e != cudaSuccess) BAGUA_LOG(Error, "comm worker cannot select device " << device_id_);
   }
+  std::vector<std::shared_ptr<ScheduledCommOp>> batch;
   for (;;) {
-    auto item = schedule_.recv(kSpinUs);
-    if (!item) return;
-    auto& op = **item;
-    BAGUA_LOG(Debug, "worker received scheduled communication operation " << op.name);
-    {
-      std::lock_guard<std::mutex> g(current_.mu);
-      current_.bucket = op.bucket;
-      current_.since = std::chrono::steady_clock::now();
-      current_.reported = false;
+    batch.clear();
+    if (next_) {
+      batch.push_back(std::move(next_));
+      next_.reset();
+    } else {
+      auto item = schedule_.recv(kSpinUs);
+      if (!item) return;
+      batch.push_back(std::move(*item));
     }
+    const bool joinable = batch[0]->ops.size() == 1 && batch[0]->ops[0]->joins(batch[0]->bucket);
+    if (joinable) join_followers(batch);
+    execute(batch);
+    if (!joinable) continue;
+    int64_t bytes = 0;
+    for (auto& item : batch) bytes += item->bucket->total_allocated() * (int64_t)dtype_bytes(item->bucket->dtype());
+    busy_until_ = std::max(busy_until_, std::chrono::steady_clock::now()) + std::chrono::microseconds(kJoinBaseUs + bytes / kJoinBytesPerUs);
+  }
+}
+
+void CommBackend::join_followers(std::vector<std::shared_ptr<ScheduledCommOp>>& batch) {
+  const auto now = std::chrono::steady_clock::now();
+  const auto until = std::min(busy_until_ - std::chrono::microseconds(kJoinAheadUs), now + std::chrono::microseconds(kJoinMostUs));
+  while (batch.size() < (size_t)kernels::kMaxJoined) {
+    std::optional<std::shared_ptr<ScheduledCommOp>> item;
+    spin_until(
+        [&] {
+          return (item = schedule_.try_recv()) || waiters_.load(std::memory_order_acquire) > 0 ||
+                 std::chrono::steady_clock::now() >= until;
+        },
+        (int)kJoinMostUs);
+    if (!item && !(item = schedule_.try_recv())) break;  // (what was sent before the waiter came)
+    const ScheduledCommOp& op = **item;
+    bool joins = op.ops.size() == 1 && op.ops[0]->joins(op.bucket) && batch[0]->ops[0]->joins_with(*op.ops[0]) &&
+                 op.bucket->dtype() == batch[0]->bucket->dtype();
+    for (auto& b : batch) joins = joins && b->bucket != op.bucket;  // twice in a row is one after the other
+    if (!joins) {
+      next_ = std::move(*item);
+      break;
+    }
+    batch.push_back(std::move(*item));
+  }
+}
+
+void CommBackend::execute(const std::vector<std::shared_ptr<ScheduledCommOp>>& batch) {
+  for (auto& item : batch) {
+    BAGUA_LOG(Debug, "worker received scheduled communication operation " << item->name);
     if (log_enabled(LogLevel::Debug)) {
       std::string names;
-      for (auto& t : op.bucket->tensors()) names += (names.empty() ? "" : ",") + t->name();
-      BAGUA_LOG(Debug, "executing communication op `" << op.name << "` on bucket `" << op.bucket->name()
+      for (auto& t : item->bucket->tensors()) names += (names.empty() ? "" : ",") + t->name();
+      BAGUA_LOG(Debug, "executing communication op `" << item->name << "` on bucket `" << item->bucket->name()
                                                       << "`, tensors [" << names << "]");
     }
-    const uint64_t t0 = Telemetry::instance().now();
-    std::string err;
-    // Optional NVTX range per bucket (BAGUA_B200_NVTX=1) so that profiler timelines line up
-    // with bucket names; a no-op when no tool is attached.
-    static const bool nvtx = env_long("BAGUA_B200_NVTX", 0) != 0;
-    if (nvtx) nvtxRangePushA(op.bucket->name().c_str());
-    try {
+  }
+  const ScheduledCommOp& op = *batch[0];
+  {
+    std::lock_guard<std::mutex> g(current_.mu);
+    current_.bucket = op.bucket;
+    current_.since = std::chrono::steady_clock::now();
+    current_.reported = false;
+  }
+  const uint64_t t0 = Telemetry::instance().now();
+  std::string err;
+  // Optional NVTX range per bucket (BAGUA_B200_NVTX=1) so that profiler timelines line up
+  // with bucket names; a no-op when no tool is attached.
+  static const bool nvtx = env_long("BAGUA_B200_NVTX", 0) != 0;
+  if (nvtx) nvtxRangePushA(op.bucket->name().c_str());
+  try {
+    if (batch.size() > 1) {
+      std::vector<BucketPtr> buckets;
+      for (auto& item : batch) buckets.push_back(item->bucket);
+      op.ops[0]->execute_joined(buckets);
+      EngineStats::global().ops_executed += batch.size();
+    } else {
       for (auto& o : op.ops) {
         o->execute_background_communication(op.bucket);
         EngineStats::global().ops_executed++;
       }
-    } catch (const std::exception& e) {
-      err = e.what();
-      BAGUA_LOG(Error, "communication op on bucket `" << op.bucket->name() << "` failed: " << err);
     }
-    if (nvtx) nvtxRangePop();
-    Telemetry::instance().record("bucket_executed", op.bucket->name(), t0);
-    {
-      std::lock_guard<std::mutex> g(current_.mu);
-      current_.bucket.reset();
-    }
+  } catch (const std::exception& e) {
+    err = e.what();
+    BAGUA_LOG(Error, "communication op on bucket `" << op.bucket->name() << "` failed: " << err);
+  }
+  if (nvtx) nvtxRangePop();
+  for (auto& item : batch) Telemetry::instance().record("bucket_executed", item->bucket->name(), t0);
+  {
+    std::lock_guard<std::mutex> g(current_.mu);
+    current_.bucket.reset();
+  }
+  for (auto& item : batch) {
     if (err.empty())
-      op.event.finish();
+      item->event.finish();
     else
-      op.event.fail(err);
-    BAGUA_LOG(Debug, "comm op executed: " << op.name);
+      item->event.fail(err);
+    BAGUA_LOG(Debug, "comm op executed: " << item->name);
   }
 }
 
@@ -170,6 +223,11 @@ void CommBackend::schedule_ready() {
 size_t CommBackend::wait_pending_comm_ops() {
   size_t n = 0;
   std::string first_error;
+  struct Waiting {
+    std::atomic<int>& n;
+    explicit Waiting(std::atomic<int>& n) : n(n) { ++n; }
+    ~Waiting() { --n; }
+  } waiting(waiters_);
   for (;;) {
     auto ev = not_waited_.try_recv();
     if (!ev) break;

@@ -121,6 +121,7 @@ class Channel {
     return v;
   }
   std::optional<T> try_recv() {
+    if (size_.load(std::memory_order_acquire) == 0) return std::nullopt;  // without the lock, for those who poll
     std::unique_lock<std::mutex> lk(mu_);
     if (q_.empty()) return std::nullopt;
     T v = std::move(q_.front());

@@ -101,17 +101,26 @@ void decompress_from(RawTensor& t, const std::string& method, int n_chunks, cons
                                 t.ctx(stream));
 }
 
-void quantise_twice(RawTensor& t, const std::string& method, uint64_t stream) {
+void quantise_twice(const std::vector<RawTensor*>& ts, const std::string& method, uint64_t stream) {
   BAGUA_CHECK(method == "MinMaxUInt8", Tensor, "unsupported compression method " << method);
-  BAGUA_CHECK(t.device_id() >= 0 && kernels::cuda::quantise_twice_minmax_u8 != nullptr, Tensor,
-              "quantise_twice works on CUDA tensors");
-  const int64_t n = t.num_elements_allocated();
-  if (n == 0) return;
-  const size_t bytes = kernels::cuda::quantise_twice_scratch_bytes(n * (int64_t)dtype_bytes(t.dtype()));
-  std::shared_ptr<PoolBlock> scratch;
-  if (bytes) scratch = MemoryPool::for_device(t.device_id()).pull_cleared(bytes, stream);
-  kernels::cuda::quantise_twice_minmax_u8(t.data_ptr(), t.dtype(), n, scratch ? scratch->ptr() : nullptr, bytes,
-                                          (cudaStream_t)stream);
+  for (size_t from = 0; from < ts.size(); from += kernels::kMaxJoined) {
+    const int count = (int)std::min<size_t>(kernels::kMaxJoined, ts.size() - from);
+    kernels::QuantiseItem items[kernels::kMaxJoined];
+    int used = 0;
+    for (int k = 0; k < count; ++k) {
+      RawTensor& t = *ts[from + k];
+      BAGUA_CHECK(t.device_id() >= 0 && t.device_id() == ts[0]->device_id() && t.dtype() == ts[0]->dtype() &&
+                      kernels::cuda::quantise_twice_minmax_u8 != nullptr,
+                  Tensor, "quantise_twice works on CUDA tensors of one type and device");
+      if (t.num_elements_allocated()) items[used++] = {t.data_ptr(), t.num_elements_allocated()};
+    }
+    if (used == 0) continue;
+    const size_t bytes = kernels::cuda::quantise_twice_scratch_bytes(items, used, ts[0]->dtype());
+    std::shared_ptr<PoolBlock> scratch;
+    if (bytes) scratch = MemoryPool::for_device(ts[0]->device_id()).pull_cleared(bytes, stream);
+    kernels::cuda::quantise_twice_minmax_u8(items, used, ts[0]->dtype(), scratch ? scratch->ptr() : nullptr, bytes,
+                                            (cudaStream_t)stream);
+  }
 }
 
 }  // namespace tensor_ops
@@ -215,8 +224,8 @@ std::string BaguaBucket::describe_ops() const {
   return oss.str();
 }
 
-CommunicationTensor BaguaBucket::get_communication_tensor(uint64_t stream, bool force_copy,
-                                                          bool force_not_copy_back) {
+CommunicationTensor BaguaBucket::get_communication_tensor(uint64_t stream, bool force_copy, bool force_not_copy_back,
+                                                          std::vector<kernels::MultiCopyItem>* gather) {
   CommunicationTensor ct;
   ct.stream = stream;
   for (auto& t : tensors_) {
@@ -261,16 +270,23 @@ CommunicationTensor BaguaBucket::get_communication_tensor(uint64_t stream, bool 
     ct.segments_dev = seg_cache_dev_;
     table = (const kernels::MultiCopySeg*)seg_cache_dev_->data_ptr();
   }
-  kernels::multi_copy(table, (int)ct.segments.size(), buf->data_ptr(), (size_t)off, /*gather=*/true, c);
   ct.raw = buf;
+  if (gather && ct.segments_dev)
+    gather->push_back(ct.copy_item());
+  else
+    kernels::multi_copy(table, (int)ct.segments.size(), buf->data_ptr(), (size_t)off, /*gather=*/true, c);
   ct.staged = true;
   ct.need_copy_back = !force_not_copy_back;
   return ct;
 }
 
-void CommunicationTensor::finish(bool sync_stream) {
+void CommunicationTensor::finish(bool sync_stream, std::vector<kernels::MultiCopyItem>* scatter) {
   if (!raw) return;
   const int device = raw->device_id();
+  if (need_copy_back && scatter && segments_dev) {
+    scatter->push_back(copy_item());
+    return;  // `raw` is wanted until that is launched
+  }
   if (need_copy_back && !segments.empty()) {
     // one launch scatters the result back (reference: one copy per tensor, datatypes/mod.rs:1048-1059)
     kernels::Ctx c{device, (cudaStream_t)stream};

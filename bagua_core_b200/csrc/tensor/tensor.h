@@ -75,8 +75,9 @@ std::shared_ptr<RawTensor> compress(const RawTensor& t, const std::string& metho
                                     int target_chunk);
 void decompress_from(RawTensor& t, const std::string& method, int n_chunks, const RawTensor& compressed,
                      uint64_t stream);
-// t = decompress(compress(decompress(compress(t)))) with one chunk, in place; CUDA tensors only.
-void quantise_twice(RawTensor& t, const std::string& method, uint64_t stream);
+// t = decompress(compress(decompress(compress(t)))) with one chunk, in place, for tensors of one type on one GPU, in one launch for
+// every kernels::kMaxJoined of them.
+void quantise_twice(const std::vector<RawTensor*>& ts, const std::string& method, uint64_t stream);
 }  // namespace tensor_ops
 
 class BaguaTensor {
@@ -130,7 +131,11 @@ class CommunicationTensor {
   // staged: where every tensor sits in `raw`; on a GPU the same table also lives on the device
   std::vector<kernels::MultiCopySeg> segments;
   std::shared_ptr<RawTensor> segments_dev;
-  void finish(bool sync_stream);
+  // `scatter`: the copy back is left to the caller, who launches it together with others'.
+  void finish(bool sync_stream, std::vector<kernels::MultiCopyItem>* scatter = nullptr);
+  kernels::MultiCopyItem copy_item() const {
+    return {(const kernels::MultiCopySeg*)segments_dev->data_ptr(), (int)segments.size(), raw->data_ptr(), raw->bytes_allocated()};
+  }
 };
 
 class BaguaBucket {
@@ -154,8 +159,10 @@ class BaguaBucket {
   std::vector<std::shared_ptr<CommOp>> ops_snapshot() const;
   std::string describe_ops() const;
 
-  // Waits (stream-side) on every tensor's ready event, then aliases or stages.
-  CommunicationTensor get_communication_tensor(uint64_t stream, bool force_copy, bool force_not_copy_back);
+  // Waits (stream-side) on every tensor's ready event, then aliases or stages.  `gather`: on a GPU the copy into the staging buffer
+  // is left to the caller, who launches it together with others'.
+  CommunicationTensor get_communication_tensor(uint64_t stream, bool force_copy, bool force_not_copy_back,
+                                               std::vector<kernels::MultiCopyItem>* gather = nullptr);
 
   std::mutex& exec_mutex() { return exec_mu_; }
 

@@ -487,3 +487,43 @@ def test_multi_copy_at_every_relative_alignment(seed):
         t.zero_()
     bb._C.k_multi_copy(ts, flat[:sum(sizes)], False, st)
     assert torch.equal(pool, before)
+
+
+@pytest.mark.parametrize("sizes", [[3], [40] * 3, [1, 7, 20000, 300007, 33, 70001, 5] * 6, [2621440, 2621440, 17, 1 << 20, 5000003], [200003] * 33])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("staged", [False, True])
+@pytest.mark.parametrize("compression", ["MinMaxUInt8", None])
+def test_buckets_that_are_handed_over_together_get_what_they_get_alone(sizes, dt, staged, compression):
+    """A burst of buckets over one rank, three times without waiting between: joined launches of any mix of sizes, never of a bucket with
+    itself."""
+    import bagua_core as bc
+
+    stream = torch.cuda.Stream()
+    comm = bc.BaguaSingleCommunicatorPy(0, 1, 0, stream.cuda_stream, "solo")
+    parts, buckets, want = [], [], []
+    for i, n in enumerate(sizes):
+        a = _rand(n + 64, dt, i)[:n] * (i + 1)
+        ts = [a] if not staged else [a[:n // 3 + 1], _rand(n + 64, dt, 100 + i)[8:8 + n]]
+        parts.append(ts)
+        tensors = [bc.BaguaTensorPy(t, "b%d_%d" % (i, k)) for k, t in enumerate(ts)]
+        bucket = bc.BaguaBucketPy("b%d" % i, tensors)
+        bucket.append_centralized_synchronous_op(comm, None, hierarchical=False, average=True, scattergather=True, compression=compression)
+        buckets.append((bucket, tensors))
+        flat = torch.cat(ts)
+        if compression:
+            for _ in range(6):
+                c = bc.BaguaTensorPy(flat, "w").compress("MinMaxUInt8", 1, -1)
+                bc.BaguaTensorPy(flat, "w").decompress_from("MinMaxUInt8", 1, c)
+        want.append(flat)
+    torch.cuda.synchronize()
+    backend = bc.BaguaCommBackendPy(100, 0)
+    backend.register_ordered_buckets([b for b, _ in buckets])
+    for _ in range(3):
+        for _, tensors in buckets:
+            for t in tensors:
+                backend.mark_communication_ready(t, 0)
+    assert backend.wait_pending_comm_ops() == 3 * len(sizes)
+    torch.cuda.synchronize()
+    backend.close()
+    for ts, w in zip(parts, want):
+        assert torch.equal(torch.cat(ts), w)
