@@ -54,12 +54,12 @@ struct alignas(16) Pack {
   T v[VecTraits<T>::N];
 };
 
+// Two items per thread, as many blocks as that takes.  (Large streams are slower through the 1184 blocks that are resident at a time, each
+// with a share of the whole: those run apart, and the memory sees all their places at once, while blocks that come and go pass over
+// it as one front.  100 M elements, resident / as here, us: average of fp32 191 / 172, of bf16 98 / 88; bf16 added to fp32 165 / 145;
+// asynchronous average 277 / 274, but 307 with one item per thread.)
 inline int grid_for(int64_t work_items) {
-  int64_t blocks = (work_items + kThreads - 1) / kThreads;
-  int64_t cap = (int64_t)kSMs * 8;
-  if (blocks > cap) blocks = cap;
-  if (blocks < 1) blocks = 1;
-  return (int)blocks;
+  return (int)std::max<int64_t>(1, std::min<int64_t>((work_items + 2 * kThreads - 1) / (2 * kThreads), 1 << 30));
 }
 
 // x[i] = op(x[i], y[i]) (y may be null for unary ops)
@@ -178,8 +178,9 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // fp32 -> bf16 of a few buffers in one launch: a layer's input, weight and bias under autocast, of which the bias
-// alone used to cost a launch.  Tiles as in the SGD kernel.
-constexpr int kCastVecs = 4;
+// alone used to cost a launch.  Tiles as in the SGD kernel, a block each (103 M elements: 87 us, 101 with 1184 resident blocks and four
+// vectors per thread).
+constexpr int kCastVecs = 2;
 constexpr int kCastTile = kThreads * 4 * kCastVecs;
 constexpr int kCastSegments = 8;
 struct CastTable {
@@ -275,8 +276,10 @@ __device__ __forceinline__ void sgd_update(const SgdSegment& a, float& pv, float
 // SGD steps of several flat buffers in one launch, each with its own hyperparameters: a stream of 20 bytes per
 // parameter (22 with the bf16 copy), bound by memory.  One launch per buffer left the chip to drain and fill again
 // between buffers of a few MB (10 buckets of 10 MB with bf16 copies: 108 us, now 97; 86 at the copy bandwidth).
-// Buffers are cut into tiles of kSgdTile elements, which the blocks take in turn; the table travels with the launch.
-constexpr int kSgdVecs = 2;
+// Buffers are cut into tiles of kSgdTile elements, a block each; the table travels with the launch.  (Blocks that stay and take the tiles
+// in turn are slower, see grid_for(): 138 M elements 485 us, 397 with a block per tile, 403 with tiles of two vectors per thread; 25.6 M with bf16
+// copies 102.6, 84.7, 88.2.)
+constexpr int kSgdVecs = 1;
 constexpr int kSgdTile = kThreads * 4 * kSgdVecs;
 constexpr int kSgdSegments = 40;
 struct SgdTable {
@@ -371,8 +374,7 @@ void cast_bf16(const CastSegment* segs, int n, cudaStream_t s) {
       t.first_tile[k + 1] = t.first_tile[k] + (segs[at + k].n + kCastTile - 1) / kCastTile;
     }
     if (t.first_tile[t.n] == 0) continue;
-    launch_overlapped(cast_bf16_kernel, dim3((unsigned)std::min<int64_t>(t.first_tile[t.n], (int64_t)kSMs * 8)), dim3(kThreads),
-                      s, t);
+    launch_overlapped(cast_bf16_kernel, dim3((unsigned)t.first_tile[t.n]), dim3(kThreads), s, t);
   }
 }
 void copy_bytes(void* dst, const void* src, size_t bytes, cudaStream_t s) {
@@ -400,8 +402,7 @@ int sgd_steps(const SgdSegment* segs, int n, cudaStream_t s) {
       t.first_tile[k + 1] = t.first_tile[k] + (a.n + kSgdTile - 1) / kSgdTile;
     }
     if (t.first_tile[t.n] == 0) continue;
-    const int grid = (int)std::min<int64_t>(t.first_tile[t.n], (int64_t)kSMs * 8);
-    launch_overlapped(sgd_kernel, dim3(grid), dim3(kThreads), s, t);
+    launch_overlapped(sgd_kernel, dim3((unsigned)t.first_tile[t.n]), dim3(kThreads), s, t);
     ++launches;
   }
   return launches;

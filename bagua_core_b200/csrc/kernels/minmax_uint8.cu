@@ -763,12 +763,14 @@ template <typename T>
 void decompress_t(const uint8_t* in, size_t in_bytes, int64_t chunk, int n_chunks, void* out, cudaStream_t s) {
   const size_t off = in_bytes / (size_t)n_chunks;
   const bool aligned = ((uintptr_t)in % 16 == 0) && ((uintptr_t)out % 16 == 0) && (chunk % 16 == 0) && (off % 16 == 0);
-  // a block takes at least two words per thread, and the launch at most 8 blocks per SM
+  // a block takes at least two words per thread; where that is more than 8 blocks per SM, as many as kDqMany words per thread take
   constexpr int VE = mmdev::Vec16<T>::VE;
-  const int64_t want = (chunk / VE + kDqThreads * 2 - 1) / (kDqThreads * 2);
+  const int64_t words = chunk / VE;
+  const int64_t want = std::max<int64_t>(1, (words + kDqThreads * 2 - 1) / (kDqThreads * 2));
   const int64_t cap = std::max<int64_t>(1, (int64_t)sm_count() * 8 / n_chunks);
-  dim3 grid((unsigned)std::max<int64_t>(1, std::min(want, cap)), (unsigned)n_chunks);
-  const bool many = chunk / VE > (int64_t)grid.x * kDqThreads * kDqMany;
+  const int64_t blocks = std::min(want, std::max(cap, (words + kDqThreads * kDqMany - 1) / (kDqThreads * kDqMany)));
+  const dim3 grid((unsigned)blocks, (unsigned)n_chunks);
+  const bool many = words > blocks * kDqThreads * kDqFew;
   auto* kernel = many ? (aligned ? dequantise_kernel<T, true, kDqMany, true> : dequantise_kernel<T, false, kDqMany, true>)
                       : (aligned ? dequantise_kernel<T, true, kDqFew, false> : dequantise_kernel<T, false, kDqFew, false>);
   launch_overlapped(kernel, grid, dim3(kDqThreads), s, in, off, chunk, (T*)out);

@@ -101,9 +101,10 @@ void fold_partials(const float* partial, float* db, int blocks, int C, bool accu
   launch_overlapped(bias_grad_finish_kernel, dim3((C + kFoldCols - 1) / kFoldCols), dim3(kFoldCols, rows), stream, partial, db, blocks, C, accumulate);
 }
 
+// A thread per vector and no more: blocks that come and go pass over the memory as one front, where those that stay walk apart
+// (forward with pooling, 64 channels at 224 x 224, batch 32: 45.0 us through 1184 blocks, 42.6 so).
 int pool_grid(int64_t nvec_out) {
-  const int64_t want = (nvec_out + kThreads - 1) / kThreads;
-  return (int)std::max<int64_t>(1, std::min<int64_t>(want, 148 * 8));
+  return (int)std::max<int64_t>(1, std::min<int64_t>((nvec_out + kThreads - 1) / kThreads, 1 << 30));
 }
 
 int backward_blocks(int64_t rows, int C) {
@@ -121,7 +122,9 @@ void bias_relu_inplace_bf16(void* z, const void* bias, int64_t rows, int C, cuda
               "fused bias+ReLU: unsupported shape [" << rows << ", " << C << "] or unaligned activation");
   const int64_t nvec = rows * (C / 8);
   const int64_t want = (nvec + (int64_t)kThreads * 4 - 1) / ((int64_t)kThreads * 4);
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, 148 * 8));
+  // four vectors per thread and no more, as in pool_grid() (64 channels at 224 x 224, batch 32: 74.5 us through 1184 blocks, 64.9 so, 86.6
+  // with two vectors per thread, to which reading the bias is more)
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, 1 << 30));
   launch_overlapped(signs ? bias_relu_kernel<true> : bias_relu_kernel<false>, dim3(grid), dim3(kThreads), stream, (uint4*)z,
                     (const __nv_bfloat16*)bias, nvec, C / 8, (uint8_t*)signs);
 }

@@ -137,7 +137,7 @@ void launch_joined(const MultiCopyItem* items, int count, bool gather, cudaStrea
     j.end[j.count++] = tiles;
   }
   if (tiles == 0) return;
-  const int grid = (int)std::min<unsigned long long>(tiles, (unsigned long long)sm_count() * 8ull);
+  const int grid = (int)std::min<unsigned long long>(tiles, 1ull << 30);
   launch_overlapped(multi_copy_kernel<kMost>, dim3(grid), dim3(kMcThreads), s, j, gather ? 1 : 0);
 }
 }  // namespace
