@@ -9,8 +9,8 @@
 //
 // Measured, us, calls back to back, compress / both directions (before clusters, and with the dequantiser's loads behind its table):
 // 16 KB of fp32 2.8 / 4.9 (3.0 / 4.8), 1 MB 4.4 / 6.9 (6.2 / 8.7), 10 MB in 8 chunks 7.5 / 11.6 (8.2 / 13.3), 1 M fp16 in 3 odd
-// chunks 7.7 / 10.2 (9.9 / 12.9), 411 MB in 8 chunks 116.9 / 212 (116.3 / 216; 78 / 157 at the copy bandwidth), 206 MB of fp16
-// 77.8 / 131.8.  Small calls are bound by latency (launch, one read, the exchange); large ones by what lies between the passes: at
+// chunks 7.7 / 10.2 (9.9 / 12.9), 411 MB in 8 chunks 112 / 200 (116.3 / 216; 78 / 157 at the copy bandwidth), 206 MB of fp16
+// 73.8 / 122.8 (76.6 / 131.6).  Small calls are bound by latency (launch, one read, the exchange); large ones by what lies between the passes: at
 // 268 MB memory sees the input and the output once, at half its rate (profiles/kernel_roofline_1gpu.md).
 //
 // The reference issues two CUB DeviceReduce calls per chunk from a host loop
@@ -418,14 +418,20 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSM)
     const int64_t nvec = (chunk - head) / VE;
     const int64_t tail = head + nvec * VE;
     const int64_t per = ((nvec + per_chunk - 1) / per_chunk + 31) & ~(int64_t)31;  // slices start on 512 bytes
-    const int64_t lo = min((int64_t)part * per, nvec), n = min(lo + per, nvec) - lo;
+    // Blocks of several tiles take every per_chunk-th of the chunk's, and the last block what is left: together they pass over memory as
+    // one front (411 MB in 8 chunks 115.7 us in slices, 112.0 so; half as much fp16 76.6, 73.8).  Blocks of fewer have a slice each.
+    const bool front = real == chunk && nvec >= 2 * (int64_t)kTile * per_chunk;
+    const int64_t whole = nvec / kTile;
+    const int64_t lo = front ? whole * kTile : min((int64_t)part * per, nvec);
+    const int64_t n = front ? (part == per_chunk - 1 ? nvec - lo : 0) : min(lo + per, nvec) - lo;
     const T* pv = p + head + lo * VE;
     uint8_t* qv = q + head + lo * VE;
     // first what is not a whole tile of real elements, then `full` whole tiles; the last tile stays in registers
-    const int64_t full = real == chunk ? n / kTile : 0;
-    const int64_t rest = n - full * kTile;
-    const T* pf = pv + rest * VE;
-    uint8_t* qf = qv + rest * VE;
+    const int64_t full = front ? (whole - part + per_chunk - 1) / per_chunk : real == chunk ? n / kTile : 0;
+    const int64_t rest = front ? n : n - full * kTile;
+    const int64_t step = (int64_t)kTile * VE * (front ? per_chunk : 1);  // from one whole tile to the next
+    const T* pf = front ? p + head + (int64_t)part * kTile * VE : pv + rest * VE;
+    uint8_t* qf = front ? q + head + (int64_t)part * kTile * VE : qv + rest * VE;
 
     // pass 1
     float mn = FLT_MAX, mx = -FLT_MAX;
@@ -438,8 +444,8 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSM)
     }
     if (full > 0) {
       tile.load(pf, kTile);
-      const T* next = pf + (int64_t)kTile * VE;
-      for (int64_t t = 1; t < full; ++t, next += (int64_t)kTile * VE) {
+      const T* next = pf + step;
+      for (int64_t t = 1; t < full; ++t, next += step) {
         // a vector's successor is requested as soon as its registers are free: seven stay in flight
 #pragma unroll
         for (int u = 0; u < kVecs; ++u) {
@@ -492,14 +498,14 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSM)
     if (full > 0) {
       const uint64_t policy = evict_first_policy();
       for (int64_t t = full - 1; t > 0; --t) {
-        const T* prev = pf + (t - 1) * (int64_t)kTile * VE;
+        const T* prev = pf + (t - 1) * step;
 #pragma unroll
         for (int u = 0; u < kVecs; ++u) {
           if (sets > 1) {
-            tile.quantise_out(u, qf + t * (int64_t)kTile * VE, g, policy);
+            tile.quantise_out(u, qf + t * step, g, policy);
             tile.raw[u] = load_elems_last<kAligned>(prev + (tid + u * kThreads) * VE, policy);
           } else {
-            tile.quantise(u, qf + t * (int64_t)kTile * VE, g);
+            tile.quantise(u, qf + t * step, g);
             tile.raw[u] = load_elems<kAligned>(prev + (tid + u * kThreads) * VE);
           }
         }
