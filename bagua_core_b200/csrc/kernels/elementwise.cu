@@ -334,8 +334,46 @@ __global__ void __launch_bounds__(kThreads) sgd_kernel(const __grid_constant__ S
   }
 }
 
+// Zeros for several buffers in one launch (13 buckets of 553 MB together: 112 us as memsets, 78 so; one buffer alone is a memset, which
+// is as fast from 40 MB on and 1 us faster below).
+constexpr int kFillVecs = 4;
+constexpr int kFillTile = kThreads * 4 * kFillVecs;
+constexpr int kFillSegments = 40;
+struct FillTable {
+  FillSegment seg[kFillSegments];
+  int64_t first_tile[kFillSegments + 1];
+};
+__global__ void __launch_bounds__(kThreads) fill_zero_kernel(const __grid_constant__ FillTable table) {
+  wait_for_predecessor();
+  int k = 0;
+  while ((int64_t)blockIdx.x >= table.first_tile[k + 1]) ++k;
+  float* p = table.seg[k].p;
+  const int64_t base = ((int64_t)blockIdx.x - table.first_tile[k]) * kFillTile, end = min(base + kFillTile, table.seg[k].n);
+  if (end - base == kFillTile && reinterpret_cast<uintptr_t>(p) % 16 == 0) {
+#pragma unroll
+    for (int u = 0; u < kFillVecs; ++u) reinterpret_cast<float4*>(p + base)[u * kThreads + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
+  } else {
+    for (int64_t i = base + threadIdx.x; i < end; i += kThreads) p[i] = 0.f;
+  }
+}
+
 }  // namespace
 
+void fill_zero(const FillSegment* segs, int n, cudaStream_t s) {
+  for (int at = 0; at < n; at += kFillSegments) {
+    FillTable t;
+    const int count = std::min(kFillSegments, n - at);
+    t.first_tile[0] = 0;
+    for (int k = 0; k < count; ++k) {
+      t.seg[k] = segs[at + k];
+      t.first_tile[k + 1] = t.first_tile[k] + (segs[at + k].n + kFillTile - 1) / kFillTile;
+    }
+    if (count == 1)
+      BAGUA_CUDA_CHECK(cudaMemsetAsync(segs[at].p, 0, (size_t)segs[at].n * sizeof(float), s));
+    else if (t.first_tile[count] > 0)
+      launch_overlapped(fill_zero_kernel, dim3((unsigned)t.first_tile[count]), dim3(kThreads), s, t);
+  }
+}
 void divide_inplace(void* x, DType dt, int64_t n, float d, cudaStream_t s) {
   dispatch_ew(x, nullptr, dt, n, OpDiv{d}, s);
 }

@@ -131,6 +131,12 @@ struct SgdSegment {
 // Steps all buffers; returns how many kernels were launched (CUDA only).
 namespace cuda {
 int sgd_steps(const SgdSegment* segs, int n, cudaStream_t s);
+// Zeroes several buffers of floats.
+struct FillSegment {
+  float* p;
+  int64_t n;
+};
+void fill_zero(const FillSegment* segs, int n, cudaStream_t s);
 }
 // p -= lr * (momentum buffer update of g (+ weight_decay * p)), torch.optim.SGD semantics.
 void sgd_momentum_flat(float* p, const float* g, float* buf, int64_t n, float lr, float momentum,

@@ -59,20 +59,20 @@ int SgdPlan::step(const std::vector<SgdGroup>& groups, uint64_t stream) {
 }
 
 void SgdPlan::zero_grad(uint64_t stream) {
+  std::vector<kernels::cuda::FillSegment> fill;
   for (size_t k = 0; k < segs_.size();) {
-    // slices of one buffer follow each other: one memset over all of them (never over two buffers, which may lie next
+    // slices of one buffer follow each other: one segment for all of them (never over two buffers, which may lie next
     // to each other in separate allocations)
-    char* from = (char*)segs_[k].g;
+    float* from = const_cast<float*>(segs_[k].g);
     const void* buffer = grad_buffer_[k];
-    size_t bytes = 0;
-    for (; k < segs_.size() && grad_buffer_[k] == buffer && (char*)segs_[k].g == from + bytes; ++k)
-      bytes += (size_t)segs_[k].n * sizeof(float);
-    if (bytes == 0) continue;
-    if (device_ >= 0)
-      BAGUA_CUDA_CHECK(cudaMemsetAsync(from, 0, bytes, (cudaStream_t)stream));
-    else
-      std::memset(from, 0, bytes);
+    int64_t n = 0;
+    for (; k < segs_.size() && grad_buffer_[k] == buffer && segs_[k].g == from + n; ++k) n += segs_[k].n;
+    if (n) fill.push_back({from, n});
   }
+  if (device_ >= 0)
+    kernels::cuda::fill_zero(fill.data(), (int)fill.size(), (cudaStream_t)stream);
+  else
+    for (const auto& f : fill) std::memset(f.p, 0, (size_t)f.n * sizeof(float));
 }
 
 }  // namespace trainer

@@ -222,7 +222,7 @@ class FlatSGD(torch.optim.Optimizer):
             self._validate_shadows()
 
     def zero_grad(self, set_to_none: bool = False):
-        """Zero the flat gradient buffers with one memset per bucket; gradients stay views
+        """Zero the flat gradient buffers in one launch; gradients stay views
         of the bucket (never set to None, which would detach them from the bucket)."""
         if self._plan is not None:
             self._plan.zero_grad(self._stream())

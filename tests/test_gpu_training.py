@@ -139,3 +139,24 @@ def test_training_on_a_side_stream_equals_training_on_the_default_stream(early_g
     (ga, wa), (gb, wb) = results
     for a, b in zip(sum(ga, []) + wa, sum(gb, []) + wb):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("sizes", [[5], [4096, 4097], [1, 70001, 3, 4095, 16384] * 9])
+def test_zero_grad_clears_every_bucket_and_nothing_else(sizes):
+    """One buffer, and more of them than a launch takes, with tiles that end in the middle."""
+    import bagua_core_b200.parallel as P
+
+    m = torch.nn.Module()
+    for i, n in enumerate(sizes):
+        m.register_parameter("w%d" % i, torch.nn.Parameter(torch.full((n,), float(i), device="cuda")))
+    opt = P.FlatSGD(m.parameters(), lr=0.5)
+    bagua = P.with_bagua(m, [opt], P.GradientAllReduceAlgorithm(), process_group=P.init_process_group(torch.device("cuda", 0)), bucket_bytes=4)
+    assert len(bagua.bagua_buckets) == len(sizes)
+    for b in bagua.bagua_buckets:
+        b.flattened.fill_(7)
+    opt.zero_grad(set_to_none=False)
+    for b in bagua.bagua_buckets:
+        assert not b.flattened.any()
+    opt.step()
+    for i, p in enumerate(m.parameters()):
+        assert (p == i).all() and not p.grad.any()
