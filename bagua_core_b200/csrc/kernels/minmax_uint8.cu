@@ -419,8 +419,9 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSM)
     const int64_t tail = head + nvec * VE;
     const int64_t per = ((nvec + per_chunk - 1) / per_chunk + 31) & ~(int64_t)31;  // slices start on 512 bytes
     // Blocks of several tiles take every per_chunk-th of the chunk's, and the last block what is left: together they pass over memory as
-    // one front (411 MB in 8 chunks 115.7 us in slices, 112.0 so; half as much fp16 76.6, 73.8).  Blocks of fewer have a slice each.
-    const bool front = real == chunk && nvec >= 2 * (int64_t)kTile * per_chunk;
+    // one front (411 MB in 8 chunks 115.7 us in slices, 112.0 so; half as much fp16 76.6, 73.8; but unaligned 103 MB in 2 chunks 60.1, 63.3).
+    // Blocks of fewer have a slice each.
+    const bool front = kAligned && real == chunk && nvec >= 2 * (int64_t)kTile * per_chunk;
     const int64_t whole = nvec / kTile;
     const int64_t lo = front ? whole * kTile : min((int64_t)part * per, nvec);
     const int64_t n = front ? (part == per_chunk - 1 ? nvec - lo : 0) : min(lo + per, nvec) - lo;
@@ -667,10 +668,10 @@ void compress_t(const void* in, int64_t num_real, int64_t chunk, int n_chunks, u
 }
 
 // ---- decompress ----------------------------------------------------------------------------
-// kVecs quantised words per thread are in flight.  kAhead: the first of them before the table is made and the others behind the stores
-// of those in front, for blocks that have many (411 MB of fp32: 90.4 us, 95-97 with the loads behind the table; half as much fp16:
-// 53.2, 55.5-58); where a thread has a few words, four at a time behind the table are the faster (10 MB of fp32: 3.8 us, 4.6-5.2
-// with eight, of whose places most are empty; 4 MB of fp16 3.4, 3.8-4.0).
+// kDqVecs quantised words per thread are in flight.  kAhead: the loads in front of the table, for blocks of many words (411 MB of
+// fp32: 79 us, 95-97 with the loads behind the table of 1184 resident blocks; half as much fp16 47.8, 55).  Where those blocks have few
+// words a thread the table comes first: up to four words four at a time (10 MB of fp32: 3.7 us, 4.2-4.6 with eight, of whose places most
+// are empty), else eight (34 MB of fp32 7.0 us, 7.4 ahead, 7.7 by four in twice the blocks; 23 MB of unaligned fp16 8.9, 9.5, 8.5).
 constexpr int kDqThreads = 256;
 constexpr int kDqMany = 8, kDqFew = 4;
 
@@ -769,16 +770,14 @@ template <typename T>
 void decompress_t(const uint8_t* in, size_t in_bytes, int64_t chunk, int n_chunks, void* out, cudaStream_t s) {
   const size_t off = in_bytes / (size_t)n_chunks;
   const bool aligned = ((uintptr_t)in % 16 == 0) && ((uintptr_t)out % 16 == 0) && (chunk % 16 == 0) && (off % 16 == 0);
-  // a block takes at least two words per thread; where that is more than 8 blocks per SM, as many as kDqMany words per thread take
+  // a block takes at least two words per thread, up to 8 blocks per SM; where those would have more than kDqMany, as many as that takes
   constexpr int VE = mmdev::Vec16<T>::VE;
-  const int64_t words = chunk / VE;
-  const int64_t want = std::max<int64_t>(1, (words + kDqThreads * 2 - 1) / (kDqThreads * 2));
-  const int64_t cap = std::max<int64_t>(1, (int64_t)sm_count() * 8 / n_chunks);
-  const int64_t blocks = std::min(want, std::max(cap, (words + kDqThreads * kDqMany - 1) / (kDqThreads * kDqMany)));
-  const dim3 grid((unsigned)blocks, (unsigned)n_chunks);
-  const bool many = words > blocks * kDqThreads * kDqFew;
-  auto* kernel = many ? (aligned ? dequantise_kernel<T, true, kDqMany, true> : dequantise_kernel<T, false, kDqMany, true>)
-                      : (aligned ? dequantise_kernel<T, true, kDqFew, false> : dequantise_kernel<T, false, kDqFew, false>);
+  const int64_t words = chunk / VE, cap = std::max<int64_t>(1, (int64_t)sm_count() * 8 / n_chunks);
+  const int64_t want = std::max<int64_t>(1, (words + kDqThreads * 2 - 1) / (kDqThreads * 2)), each = kDqThreads * kDqMany;
+  const dim3 grid((unsigned)std::min(want, std::max(cap, (words + each - 1) / each)), (unsigned)n_chunks);
+  auto* kernel = words > cap * each                     ? (aligned ? dequantise_kernel<T, true, kDqMany, true> : dequantise_kernel<T, false, kDqMany, true>)
+                 : words > cap * kDqThreads * kDqFew ? (aligned ? dequantise_kernel<T, true, kDqMany, false> : dequantise_kernel<T, false, kDqMany, false>)
+                                                        : (aligned ? dequantise_kernel<T, true, kDqFew, false> : dequantise_kernel<T, false, kDqFew, false>);
   launch_overlapped(kernel, grid, dim3(kDqThreads), s, in, off, chunk, (T*)out);
 }
 

@@ -2,7 +2,8 @@
 and in the backward one pass that applies the ReLU mask and reduces the bias gradient.
 
 The convolution itself stays a library call (cuDNN through `at::convolution` /
-`at::convolution_backward`).  What the framework would run around it — a bias add, a clamp, a
+`at::convolution_backward`), but for the weight gradient of 3 x 3 convolutions with bf16 parameters
+(`csrc/kernels/conv_wgrad.cu`, where its rule takes it).  What the framework would run around it — a bias add, a clamp, a
 ReLU-mask kernel and a separate column reduction for the bias gradient — is replaced by the
 sm_100a kernels of `csrc/kernels/model_ops.cu`; the autograd functions are native
 (`csrc/trainer/autograd_ops.cc`).  The fused path needs a block computed in bf16
