@@ -11,7 +11,7 @@
 // 16 KB of fp32 2.8 / 4.9 (3.0 / 4.8), 1 MB 4.4 / 6.9 (6.2 / 8.7), 10 MB in 8 chunks 7.5 / 11.6 (8.2 / 13.3), 1 M fp16 in 3 odd
 // chunks 7.7 / 10.2 (9.9 / 12.9), 411 MB in 8 chunks 112 / 200 (116.3 / 216; 78 / 157 at the copy bandwidth), 206 MB of fp16
 // 73.8 / 122.8 (76.6 / 131.6).  Small calls are bound by latency (launch, one read, the exchange); large ones by what lies between the passes: at
-// 268 MB memory sees the input and the output once, at half its rate (profiles/kernel_roofline_1gpu.md).
+// 268 MB memory sees the input and the output once, at half its rate.
 //
 // The reference issues two CUB DeviceReduce calls per chunk from a host loop
 // (bagua-core-internal/kernels/bagua_kernels.cu:312-371,533-560) and quantises one byte per thread
