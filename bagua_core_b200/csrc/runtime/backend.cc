@@ -45,7 +45,7 @@ void CommBackend::worker_loop() {
       if (!item) return;
       batch.push_back(std::move(*item));
     }
-    const bool joinable = batch[0]->ops.size() == 1 && batch[0]->ops[0]->joins(batch[0]->bucket);
+    const bool joinable = batch[0]->joins();
     if (joinable) join_followers(batch);
     execute(batch);
     if (!joinable) continue;
@@ -68,8 +68,7 @@ void CommBackend::join_followers(std::vector<std::shared_ptr<ScheduledCommOp>>& 
         (int)kJoinMostUs);
     if (!item && !(item = schedule_.try_recv())) break;  // (what was sent before the waiter came)
     const ScheduledCommOp& op = **item;
-    bool joins = op.ops.size() == 1 && op.ops[0]->joins(op.bucket) && batch[0]->ops[0]->joins_with(*op.ops[0]) &&
-                 op.bucket->dtype() == batch[0]->bucket->dtype();
+    bool joins = op.joins() && batch[0]->ops[0]->joins_with(*op.ops[0]) && op.bucket->dtype() == batch[0]->bucket->dtype();
     for (auto& b : batch) joins = joins && b->bucket != op.bucket;  // twice in a row is one after the other
     if (!joins) {
       next_ = std::move(*item);
@@ -152,10 +151,33 @@ void CommBackend::monitor_loop() {
   }
 }
 
+namespace {
+// Tensors may overlap without starting at one address (views).  By their starts, a tensor that overlaps any in front of it overlaps the
+// one of them that ends last.
+std::unordered_set<const BaguaBucket*> buckets_that_share_memory(const std::vector<BucketPtr>& buckets) {
+  struct Span {
+    uint64_t from, to;
+    const BaguaBucket* bucket;
+  };
+  std::vector<Span> spans;
+  for (auto& b : buckets)
+    for (auto& t : b->tensors())
+      if (const uint64_t bytes = t->raw()->bytes_allocated()) spans.push_back({t->data_ptr(), t->data_ptr() + bytes, b.get()});
+  std::sort(spans.begin(), spans.end(), [](const Span& a, const Span& b) { return a.from < b.from; });
+  std::unordered_set<const BaguaBucket*> sharing;
+  for (size_t k = 1, last = 0; k < spans.size(); ++k) {
+    if (spans[k].from < spans[last].to && spans[k].bucket != spans[last].bucket) sharing.insert({spans[k].bucket, spans[last].bucket});
+    if (spans[k].to > spans[last].to) last = k;
+  }
+  return sharing;
+}
+}  // namespace
+
 void CommBackend::register_ordered_buckets(const std::vector<BucketPtr>& buckets) {
   wait_pending_comm_ops();
   std::lock_guard<std::mutex> g(mu_);
   ordered_buckets_.clear();
+  sharing_.clear();
   std::unordered_set<std::string> names;
   std::unordered_set<uint64_t> ptrs;
   for (auto& b : buckets) {
@@ -173,6 +195,7 @@ void CommBackend::register_ordered_buckets(const std::vector<BucketPtr>& buckets
     }
     ordered_buckets_.push_back(b);
   }
+  sharing_ = buckets_that_share_memory(buckets);
 }
 
 bool CommBackend::should_schedule() const {
@@ -185,6 +208,7 @@ void CommBackend::schedule_comm(const BucketPtr& bucket) {
   op->name = bucket->name();
   op->bucket = bucket;
   op->ops = bucket->ops_snapshot();
+  op->shares_memory = sharing_.count(bucket.get()) != 0;
   EventChannel ev = op->event;
   const uint64_t t0 = Telemetry::instance().now();
   if (!schedule_.send(std::move(op))) throw BaguaError(ErrorKind::InternalChannel, "schedule channel is closed");

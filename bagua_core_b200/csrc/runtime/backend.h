@@ -35,6 +35,9 @@ struct ScheduledCommOp {
   BucketPtr bucket;
   std::vector<std::shared_ptr<CommOp>> ops;
   EventChannel event{"comm_op"};
+  bool shares_memory = false;  // with another registered bucket
+  // Whether it may be executed together with others.
+  bool joins() const { return !shares_memory && ops.size() == 1 && ops[0]->joins(bucket); }
 };
 
 class CommBackend {
@@ -70,6 +73,7 @@ class CommBackend {
 
   const int device_id_;
   std::deque<BucketPtr> ordered_buckets_;
+  std::unordered_set<const BaguaBucket*> sharing_;  // of them, those that share memory with another
   std::mutex mu_;  // guards ordered_buckets_ and registration state
 
   Channel<std::shared_ptr<ScheduledCommOp>> schedule_;

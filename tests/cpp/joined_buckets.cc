@@ -1,0 +1,206 @@
+// Buckets that the engine hands to the GPU together (a communicator of one rank), without a GPU: the engine's own sources run
+// over a stand-in for the CUDA runtime and for the kernels, in which device memory is host memory and a launch does its work
+// at once.  The first bucket of a burst is held inside its launch until the others are scheduled, so that those are joined.
+//
+//   overlap   buckets that share memory get what they get one after the other
+#include <cuda_runtime.h>
+
+#include <condition_variable>
+#include <cstdio>
+#include <cstring>
+#include <functional>
+#include <map>
+#include <string>
+#include <thread>
+
+#include "comm/arena.h"
+#include "comm/communicator.h"
+#include "kernels/kernels_impl.h"
+#include "ops/comm_op.h"
+#include "pool/resource_pool.h"
+#include "runtime/backend.h"
+
+using namespace bagua;
+
+namespace {
+int failures = 0;
+#define EXPECT(cond, ...)                             \
+  do {                                                \
+    if (!(cond)) {                                    \
+      std::fprintf(stderr, "line %d: ", __LINE__);    \
+      std::fprintf(stderr, __VA_ARGS__);              \
+      std::fprintf(stderr, "\n");                     \
+      ++failures;                                     \
+    }                                                 \
+  } while (0)
+
+// ---- a launch that is held --------------------------------------------------------------------------
+struct Gate {
+  std::mutex mu;
+  std::condition_variable cv;
+  bool closed = false, reached = false;
+  void close() {
+    std::lock_guard<std::mutex> g(mu);
+    closed = true;
+    reached = false;
+  }
+  void pass() {
+    std::unique_lock<std::mutex> lk(mu);
+    reached = true;
+    cv.notify_all();
+    cv.wait(lk, [&] { return !closed; });
+  }
+  void wait_reached() {
+    std::unique_lock<std::mutex> lk(mu);
+    cv.wait(lk, [&] { return reached; });
+  }
+  void open() {
+    std::lock_guard<std::mutex> g(mu);
+    closed = false;
+    cv.notify_all();
+  }
+} gate;
+std::mutex launches_mu;
+std::vector<int> quantise_launches;  // buffers of each
+}  // namespace
+
+// ---- the stand-in for the CUDA runtime ----------------------------------------------------------------
+extern "C" {
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGetDevice(int* d) {
+  *d = 0;
+  return cudaSuccess;
+}
+cudaError_t cudaMalloc(void** p, size_t n) {
+  *p = std::aligned_alloc(256, (n + 255) / 256 * 256);
+  return cudaSuccess;
+}
+cudaError_t cudaFree(void* p) {
+  std::free(p);
+  return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
+  std::memcpy(d, s, n);
+  return cudaSuccess;
+}
+cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) {
+  std::memset(d, v, n);
+  return cudaSuccess;
+}
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+}
+
+// ---- a communicator of one rank, and the kernels -------------------------------------------------------
+namespace bagua {
+PeerArena::~PeerArena() {}
+SingleCommunicator::SingleCommunicator(int rank, int nranks, int device_id, uint64_t stream, const std::string&)
+    : rank_(rank), nranks_(nranks), device_id_(device_id), stream_(stream) {}
+SingleCommunicator::~SingleCommunicator() {}
+void SingleCommunicator::check_all_device_status() {}
+std::shared_ptr<Communicator> Communicator::create(SingleCommPtr internode, SingleCommPtr, bool) {
+  auto c = std::make_shared<Communicator>();
+  c->internode_ = std::move(internode);
+  return c;
+}
+uint64_t Communicator::stream() const { return internode_->stream(); }
+void Communicator::execute_communication(RawTensor& t, bool, bool, bool, const std::function<void(SingleCommunicator&, RawTensor&)>& hook) {
+  hook(*internode_, t);
+}
+namespace kernels {
+namespace cuda {
+void multi_copy_joined(const MultiCopyItem* items, int count, bool gather, cudaStream_t) {
+  for (int k = 0; k < count; ++k)
+    for (int s = 0; s < items[k].nseg; ++s) {
+      const MultiCopySeg& sg = items[k].segs[s];
+      char* flat = (char*)items[k].flat + sg.offset;
+      std::memcpy(gather ? flat : (char*)sg.ptr, gather ? (char*)sg.ptr : flat, sg.bytes);
+    }
+}
+void multi_copy(const MultiCopySeg* segs, int nseg, void* flat, size_t bytes, bool gather, cudaStream_t s) {
+  const MultiCopyItem one{segs, nseg, flat, bytes};
+  multi_copy_joined(&one, 1, gather, s);
+}
+size_t quantise_twice_scratch_bytes(const QuantiseItem*, int count, DType) { return 32 * (size_t)count; }
+// x -> 2 x + 1 stands for the work: twice on the same values is not once.  All buffers of a launch are read before any is written.
+void quantise_twice_minmax_u8(const QuantiseItem* items, int count, DType, void*, size_t, cudaStream_t) {
+  gate.pass();
+  {
+    std::lock_guard<std::mutex> g(launches_mu);
+    quantise_launches.push_back(count);
+  }
+  std::vector<std::vector<float>> read;
+  for (int k = 0; k < count; ++k) read.emplace_back((float*)items[k].x, (float*)items[k].x + items[k].n);
+  for (int k = 0; k < count; ++k)
+    for (int64_t i = 0; i < items[k].n; ++i) ((float*)items[k].x)[i] = 2 * read[k][i] + 1;
+}
+}  // namespace cuda
+}  // namespace kernels
+}  // namespace bagua
+
+namespace {
+struct View : RawTensor {
+  View(float* p, int64_t n) : p(p), n(n) {}
+  void* data_ptr() const override { return p; }
+  int64_t num_elements() const override { return n; }
+  int64_t num_elements_allocated() const override { return n; }
+  int device_id() const override { return 0; }
+  DType dtype() const override { return DType::F32; }
+  float* p;
+  int64_t n;
+};
+
+std::shared_ptr<Communicator> one_rank(uint64_t stream) {
+  return Communicator::create(std::make_shared<SingleCommunicator>(0, 1, 0, stream, "solo"), nullptr, false);
+}
+
+using Spans = std::vector<std::pair<float*, int64_t>>;
+BucketPtr make_bucket(const std::string& name, const Spans& spans, const std::shared_ptr<CommOp>& op) {
+  std::vector<TensorPtr> ts;
+  for (auto& [p, n] : spans) ts.push_back(std::make_shared<BaguaTensor>(name + "_" + std::to_string(ts.size()), std::make_shared<View>(p, n)));
+  auto b = std::make_shared<BaguaBucket>(name, ts);
+  b->append_op(op);
+  return b;
+}
+void mark(CommBackend& backend, const BucketPtr& b) {
+  for (auto& t : b->tensors()) backend.mark_communication_ready(t, 0);
+}
+// The buckets in their order, the first held until the last is scheduled.
+void burst(CommBackend& backend, const std::vector<BucketPtr>& buckets, const std::function<void()>& while_held = {}) {
+  gate.close();
+  mark(backend, buckets[0]);
+  gate.wait_reached();
+  for (size_t k = 1; k < buckets.size(); ++k) mark(backend, buckets[k]);
+  if (while_held) while_held();
+  gate.open();
+}
+
+void overlap() {
+  std::vector<float> x(1000), y(1000), first(16);
+  auto op = make_centralized_low_precision_op(one_rank(1), true, "MinMaxUInt8");
+  // b shares part of a's memory behind its first element, c none; d is staged, and one of its tensors lies in c's
+  CommBackend backend(100, 0);
+  const std::vector<BucketPtr> buckets = {make_bucket("first", {{first.data(), 16}}, op), make_bucket("a", {{x.data(), 600}}, op),
+                                          make_bucket("b", {{x.data() + 400, 600}}, op), make_bucket("c", {{y.data(), 500}}, op),
+                                          make_bucket("d", {{y.data() + 600, 100}, {y.data() + 450, 20}}, op)};
+  backend.register_ordered_buckets(buckets);
+  burst(backend, buckets);
+  EXPECT(backend.wait_pending_comm_ops() == 5, "five buckets");
+  for (int i = 0; i < 1000; ++i) {
+    const float wx = i >= 400 && i < 600 ? 3 : 1, wy = i >= 450 && i < 470 ? 3 : i < 500 || (i >= 600 && i < 700) ? 1 : 0;
+    if (x[i] != wx || y[i] != wy) {
+      EXPECT(false, "value %d is %g / %g, not %g / %g", i, x[i], y[i], wx, wy);
+      break;
+    }
+  }
+}
+
+const std::map<std::string, void (*)()> kCases = {{"overlap", overlap}};
+}  // namespace
+
+int main(int argc, char** argv) {
+  if (argc != 2 || !kCases.count(argv[1])) return 2;
+  kCases.at(argv[1])();
+  std::printf("%s: %d failures\n", argv[1], failures);
+  return failures ? 1 : 0;
+}
