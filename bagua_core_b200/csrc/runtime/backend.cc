@@ -151,33 +151,11 @@ void CommBackend::monitor_loop() {
   }
 }
 
-namespace {
-// Tensors may overlap without starting at one address (views).  By their starts, a tensor that overlaps any in front of it overlaps the
-// one of them that ends last.
-std::unordered_set<const BaguaBucket*> buckets_that_share_memory(const std::vector<BucketPtr>& buckets) {
-  struct Span {
-    uint64_t from, to;
-    const BaguaBucket* bucket;
-  };
-  std::vector<Span> spans;
-  for (auto& b : buckets)
-    for (auto& t : b->tensors())
-      if (const uint64_t bytes = t->raw()->bytes_allocated()) spans.push_back({t->data_ptr(), t->data_ptr() + bytes, b.get()});
-  std::sort(spans.begin(), spans.end(), [](const Span& a, const Span& b) { return a.from < b.from; });
-  std::unordered_set<const BaguaBucket*> sharing;
-  for (size_t k = 1, last = 0; k < spans.size(); ++k) {
-    if (spans[k].from < spans[last].to && spans[k].bucket != spans[last].bucket) sharing.insert({spans[k].bucket, spans[last].bucket});
-    if (spans[k].to > spans[last].to) last = k;
-  }
-  return sharing;
-}
-}  // namespace
-
 void CommBackend::register_ordered_buckets(const std::vector<BucketPtr>& buckets) {
   wait_pending_comm_ops();
   std::lock_guard<std::mutex> g(mu_);
   ordered_buckets_.clear();
-  sharing_.clear();
+  places_.clear();
   std::unordered_set<std::string> names;
   std::unordered_set<uint64_t> ptrs;
   for (auto& b : buckets) {
@@ -195,7 +173,27 @@ void CommBackend::register_ordered_buckets(const std::vector<BucketPtr>& buckets
     }
     ordered_buckets_.push_back(b);
   }
-  sharing_ = buckets_that_share_memory(buckets);
+  // Tensors may overlap without starting at one address (views).  By their starts, one that overlaps any in front of it overlaps the
+  // one of them that ends last.
+  struct Span {
+    uint64_t from, to;
+    const BaguaBucket* bucket;
+  };
+  std::vector<Span> spans;
+  for (auto& b : buckets) {
+    auto place = std::make_shared<const MemorySpans>(b->memory_spans());
+    for (auto& [from, to] : *place)
+      if (from < to) spans.push_back({from, to, b.get()});
+    places_[b.get()] = std::move(place);
+  }
+  std::sort(spans.begin(), spans.end(), [](const Span& a, const Span& b) { return a.from < b.from; });
+  for (size_t k = 1, last = 0; k < spans.size(); ++k) {
+    if (spans[k].from < spans[last].to && spans[k].bucket != spans[last].bucket) {
+      places_.erase(spans[k].bucket);
+      places_.erase(spans[last].bucket);
+    }
+    if (spans[k].to > spans[last].to) last = k;
+  }
 }
 
 bool CommBackend::should_schedule() const {
@@ -208,7 +206,7 @@ void CommBackend::schedule_comm(const BucketPtr& bucket) {
   op->name = bucket->name();
   op->bucket = bucket;
   op->ops = bucket->ops_snapshot();
-  op->shares_memory = sharing_.count(bucket.get()) != 0;
+  if (auto it = places_.find(bucket.get()); it != places_.end()) op->place = it->second;
   EventChannel ev = op->event;
   const uint64_t t0 = Telemetry::instance().now();
   if (!schedule_.send(std::move(op))) throw BaguaError(ErrorKind::InternalChannel, "schedule channel is closed");

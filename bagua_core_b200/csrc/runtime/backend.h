@@ -35,9 +35,10 @@ struct ScheduledCommOp {
   BucketPtr bucket;
   std::vector<std::shared_ptr<CommOp>> ops;
   EventChannel event{"comm_op"};
-  bool shares_memory = false;  // with another registered bucket
+  // Where the bucket's tensors lay when it was registered; null: it shared memory with another.
+  std::shared_ptr<const MemorySpans> place;
   // Whether it may be executed together with others.
-  bool joins() const { return !shares_memory && ops.size() == 1 && ops[0]->joins(bucket); }
+  bool joins() const { return place && ops.size() == 1 && ops[0]->joins(bucket) && bucket->memory_spans() == *place; }
 };
 
 class CommBackend {
@@ -73,7 +74,7 @@ class CommBackend {
 
   const int device_id_;
   std::deque<BucketPtr> ordered_buckets_;
-  std::unordered_set<const BaguaBucket*> sharing_;  // of them, those that share memory with another
+  std::unordered_map<const BaguaBucket*, std::shared_ptr<const MemorySpans>> places_;  // of those that share no memory with others
   std::mutex mu_;  // guards ordered_buckets_ and registration state
 
   Channel<std::shared_ptr<ScheduledCommOp>> schedule_;

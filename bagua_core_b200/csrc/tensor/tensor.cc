@@ -185,6 +185,13 @@ bool BaguaBucket::contiguous() const {
   return true;
 }
 
+MemorySpans BaguaBucket::memory_spans() const {
+  MemorySpans spans;
+  spans.reserve(tensors_.size());
+  for (auto& t : tensors_) spans.emplace_back(t->data_ptr(), t->data_ptr() + t->raw()->bytes_allocated());
+  return spans;
+}
+
 bool BaguaBucket::ready_for_comm() const {
   // Asked after every tensor that becomes ready.  A trainer lists a bucket's tensors in the order
   // their gradients appear, so the ones at the back are the last to become ready: looking from the

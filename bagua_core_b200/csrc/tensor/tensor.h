@@ -138,6 +138,8 @@ class CommunicationTensor {
   }
 };
 
+using MemorySpans = std::vector<std::pair<uint64_t, uint64_t>>;  // addresses: from, to
+
 class BaguaBucket {
  public:
   // Validation: non-empty, same dtype, same device, allocated >= numel.
@@ -149,6 +151,7 @@ class BaguaBucket {
   int device_id() const { return device_; }
   int64_t total_allocated() const;
   bool contiguous() const;  // tensors address-adjacent in list order
+  MemorySpans memory_spans() const;  // of every tensor, in list order
 
   bool ready_for_comm() const;
   void reset_comm_ready();

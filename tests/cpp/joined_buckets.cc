@@ -2,7 +2,7 @@
 // over a stand-in for the CUDA runtime and for the kernels, in which device memory is host memory and a launch does its work
 // at once.  The first bucket of a burst is held inside its launch until the others are scheduled, so that those are joined.
 //
-//   overlap   buckets that share memory get what they get one after the other
+//   overlap   buckets that share memory, or whose tensors have moved to where they do, get what they get one after the other
 #include <cuda_runtime.h>
 
 #include <condition_variable>
@@ -190,6 +190,18 @@ void overlap() {
     const float wx = i >= 400 && i < 600 ? 3 : 1, wy = i >= 450 && i < 470 ? 3 : i < 500 || (i >= 600 && i < 700) ? 1 : 0;
     if (x[i] != wx || y[i] != wy) {
       EXPECT(false, "value %d is %g / %g, not %g / %g", i, x[i], y[i], wx, wy);
+      break;
+    }
+  }
+  // c's tensor moves to where a is
+  dynamic_cast<View&>(*buckets[3]->tensors()[0]->raw()).p = x.data();
+  std::fill(x.begin(), x.end(), 0.f);
+  burst(backend, buckets);
+  backend.wait_pending_comm_ops();
+  for (int i = 0; i < 1000; ++i) {
+    const float want = i < 400 ? 3 : i < 500 ? 7 : i < 600 ? 3 : 1;
+    if (x[i] != want) {
+      EXPECT(false, "moved: value %d is %g, not %g", i, x[i], want);
       break;
     }
   }
