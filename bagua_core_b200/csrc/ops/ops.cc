@@ -3,6 +3,7 @@
 // body is also the CPU backend and the measured baseline.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <deque>
@@ -65,9 +66,11 @@ void note_fallback() { EngineStats::global().library_fallbacks++; }
 
 struct OpFrame {
   // Common prologue/epilogue of an op: lock, stream, communication tensor, release.
-  OpFrame(const BucketPtr& bucket, Communicator& comm, bool force_copy, bool no_copy_back,
-          std::vector<kernels::MultiCopyItem>* gather = nullptr)
-      : lock(bucket->exec_mutex()), stream(comm.stream()) {
+  OpFrame(const BucketPtr& bucket, Communicator& comm, bool force_copy, bool no_copy_back)
+      : OpFrame(std::unique_lock<std::mutex>(bucket->exec_mutex()), bucket, comm, force_copy, no_copy_back, nullptr) {}
+  OpFrame(std::unique_lock<std::mutex> locked, const BucketPtr& bucket, Communicator& comm, bool force_copy, bool no_copy_back,
+          std::vector<kernels::MultiCopyItem>* gather)
+      : lock(std::move(locked)), stream(comm.stream()) {
     ct = bucket->get_communication_tensor(stream, force_copy, no_copy_back, gather);
     if (ct.staged) EngineStats::global().staged_copies++;
     EngineStats::global().bytes_communicated += ct.raw->bytes_allocated();
@@ -103,12 +106,23 @@ void copy_joined(std::vector<kernels::MultiCopyItem>& items, bool gather, uint64
     kernels::cuda::multi_copy_joined(items.data() + from, (int)std::min<size_t>(kernels::kMaxJoined, items.size() - from), gather,
                                      (cudaStream_t)stream);
 }
+// Held together the locks of several buckets are taken by address: two backends may hold the same buckets in different orders.
+std::vector<std::unique_lock<std::mutex>> lock_all(const std::vector<BucketPtr>& buckets) {
+  std::vector<std::unique_lock<std::mutex>> locks;
+  for (const BucketPtr& b : buckets) locks.emplace_back(b->exec_mutex(), std::defer_lock);
+  std::vector<std::unique_lock<std::mutex>*> order;
+  for (auto& l : locks) order.push_back(&l);
+  std::sort(order.begin(), order.end(), [](auto* a, auto* b) { return std::less<std::mutex*>()(a->mutex(), b->mutex()); });
+  for (auto* l : order) l->lock();
+  return locks;
+}
 void run_joined(Communicator& comm, const std::vector<BucketPtr>& buckets, const std::function<void(std::vector<RawTensor*>&)>& work) {
+  auto locks = lock_all(buckets);
   std::vector<kernels::MultiCopyItem> gather, scatter;
   std::deque<OpFrame> frames;
   std::vector<RawTensor*> raws;
-  for (const BucketPtr& b : buckets) {
-    frames.emplace_back(b, comm, false, false, &gather);
+  for (size_t k = 0; k < buckets.size(); ++k) {
+    frames.emplace_back(std::move(locks[k]), buckets[k], comm, false, false, &gather);
     raws.push_back(frames.back().ct.raw.get());
   }
   copy_joined(gather, true, comm.stream());

@@ -2,9 +2,11 @@
 // over a stand-in for the CUDA runtime and for the kernels, in which device memory is host memory and a launch does its work
 // at once.  The first bucket of a burst is held inside its launch until the others are scheduled, so that those are joined.
 //
+//   locks     backends that hold the same buckets in opposite orders do not wait for each other
 //   overlap   buckets that share memory, or whose tensors have moved to where they do, get what they get one after the other
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <condition_variable>
 #include <cstdio>
 #include <cstring>
@@ -207,7 +209,27 @@ void overlap() {
   }
 }
 
-const std::map<std::string, void (*)()> kCases = {{"overlap", overlap}};
+// Two backends, the same buckets in opposite orders: a launch that waits for several buckets' locks takes them in one order.  (A deadlock
+// shows as a test that does not end, and ThreadSanitizer reports two orders that only might have met.)
+void locks() {
+  std::vector<float> x(64), held(32);
+  auto op = make_centralized_low_precision_op(one_rank(1), true, "MinMaxUInt8");
+  std::vector<BucketPtr> buckets;
+  for (int k = 0; k < 4; ++k) buckets.push_back(make_bucket("b" + std::to_string(k), {{x.data() + 16 * k, 16}}, op));
+  for (int turn = 0; turn < 2; ++turn) {
+    CommBackend backend(100, 0);
+    std::vector<BucketPtr> order = buckets;
+    if (turn) std::reverse(order.begin(), order.end());
+    order.insert(order.begin(), make_bucket("held", {{held.data() + 16 * turn, 16}}, op));
+    backend.register_ordered_buckets(order);
+    burst(backend, order);
+    EXPECT(backend.wait_pending_comm_ops() == 5, "five buckets");
+  }
+  EXPECT(quantise_launches == (std::vector<int>{1, 4, 1, 4}), "the four were not joined");
+  for (float v : x) EXPECT(v == 3, "%g", v);
+}
+
+const std::map<std::string, void (*)()> kCases = {{"locks", locks}, {"overlap", overlap}};
 }  // namespace
 
 int main(int argc, char** argv) {

@@ -37,3 +37,7 @@ def _run(program, case):
 
 def test_buckets_that_share_memory_are_executed_one_after_the_other(program):
     _run(program, "overlap")
+
+
+def test_joined_buckets_are_locked_in_one_order(program):
+    _run(program, "locks")
