@@ -3,6 +3,7 @@ takes and returns low precision, statistics still in fp32) and is unchanged outs
 import copy
 
 import torch
+import torch.fx
 
 from bagua_core_b200.models import BertConfig, BertForQuestionAnswering
 
@@ -82,3 +83,16 @@ def test_hooks_of_the_mlp_and_its_modules_fire_and_see_what_their_module_sees():
     assert calls.count("ReLU") == 1
     m.net[0] = torch.nn.Linear(8, 16)
     assert torch.equal(m(x), m.net(x))
+
+
+def test_vgg16_is_traced_and_scripted_whatever_size_its_images_have():
+    from bagua_core_b200.models import VGG16
+
+    torch.manual_seed(0)
+    m = VGG16(num_classes=3).eval()
+    with torch.no_grad():
+        traced = torch.jit.trace(m, torch.randn(1, 3, 224, 224))
+        x = torch.randn(1, 3, 64, 96)
+        want = m(x)
+        for other in (traced, torch.jit.script(m), torch.fx.symbolic_trace(m)):
+            assert torch.equal(other(x), want)
