@@ -25,15 +25,19 @@ struct EngineConfig {
   static EngineConfig& global();
 };
 
+// Buckets that are executed together have at most this many bytes each, and as many in all of those that are staged.
+constexpr int64_t kJoinedBytes = 32 << 20;
+
 class CommOp {
  public:
   virtual ~CommOp() = default;
   virtual void execute_background_communication(const BucketPtr& bucket) = 0;
   // Whether the op's part on `bucket` is one that several buckets can do in one launch, and if so with `other`, the op of another
-  // bucket, too.  Such buckets may be executed together, by one of their ops; the results are those of one after the other.
+  // bucket, too.  Such buckets are executed together, by one of their ops; the results are those of one after the other.  Those that
+  // are staged are staged in one buffer of `staging_bytes`, which is the same from call to call.
   virtual bool joins(const BucketPtr& /*bucket*/) const { return false; }
   virtual bool joins_with(const CommOp& /*other*/) const { return false; }
-  virtual void execute_joined(const std::vector<BucketPtr>& buckets) {
+  virtual void execute_joined(const std::vector<BucketPtr>& buckets, int64_t /*staging_bytes*/) {
     for (const BucketPtr& b : buckets) execute_background_communication(b);
   }
   virtual std::string describe() const = 0;

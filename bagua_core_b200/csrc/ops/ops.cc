@@ -69,9 +69,9 @@ struct OpFrame {
   OpFrame(const BucketPtr& bucket, Communicator& comm, bool force_copy, bool no_copy_back)
       : OpFrame(std::unique_lock<std::mutex>(bucket->exec_mutex()), bucket, comm, force_copy, no_copy_back, nullptr) {}
   OpFrame(std::unique_lock<std::mutex> locked, const BucketPtr& bucket, Communicator& comm, bool force_copy, bool no_copy_back,
-          std::vector<kernels::MultiCopyItem>* gather)
+          JoinedStaging* joined)
       : lock(std::move(locked)), stream(comm.stream()) {
-    ct = bucket->get_communication_tensor(stream, force_copy, no_copy_back, gather);
+    ct = bucket->get_communication_tensor(stream, force_copy, no_copy_back, joined);
     if (ct.staged) EngineStats::global().staged_copies++;
     EngineStats::global().bytes_communicated += ct.raw->bytes_allocated();
     gpu = ct.raw->device_id() >= 0;
@@ -95,9 +95,9 @@ struct OpFrame {
 // Buckets of a communicator of one rank on a GPU: nothing travels, each bucket's part is local, and several that are ready at once are
 // gathered, worked on and scattered in one launch each.  Not where somebody looks at them one by one, nor buckets that keep the GPU busy
 // for longer than they wait for it anyway (VGG-16's bf16 buckets, one of them of 205 MB, quantised: 185 us alone, 192 all joined, 180-183 with this limit).
-constexpr int64_t kJoinedBucketBytes = 32 << 20;
 bool joins_over_one_rank(const Communicator& comm, const BucketPtr& bucket) {
-  return bucket->device_id() >= 0 && bucket->total_allocated() * (int64_t)dtype_bytes(bucket->dtype()) <= kJoinedBucketBytes && comm.kind() == Communicator::Kind::Single && comm.internode() && comm.internode()->nranks() == 1 &&
+  return bucket->device_id() >= 0 && bucket->total_allocated() * (int64_t)dtype_bytes(bucket->dtype()) <= kJoinedBytes &&
+         comm.kind() == Communicator::Kind::Single && comm.internode() && comm.internode()->nranks() == 1 &&
          !EngineConfig::global().sync_per_bucket && !BucketTimeline::instance().enabled() &&
          kernels::cuda::multi_copy_joined != nullptr;
 }
@@ -116,16 +116,20 @@ std::vector<std::unique_lock<std::mutex>> lock_all(const std::vector<BucketPtr>&
   for (auto* l : order) l->lock();
   return locks;
 }
-void run_joined(Communicator& comm, const std::vector<BucketPtr>& buckets, const std::function<void(std::vector<RawTensor*>&)>& work) {
+// All staging buffers of the batch are wanted until its scatter is launched; they are parts of one block, which every batch of these
+// buckets pulls in the same size: what the pool holds does not depend on which buckets happened to meet.
+void run_joined(Communicator& comm, const std::vector<BucketPtr>& buckets, int64_t staging_bytes,
+                const std::function<void(std::vector<RawTensor*>&)>& work) {
   auto locks = lock_all(buckets);
-  std::vector<kernels::MultiCopyItem> gather, scatter;
+  JoinedStaging staging(staging_bytes, buckets[0]->device_id(), comm.stream());
+  std::vector<kernels::MultiCopyItem> scatter;
   std::deque<OpFrame> frames;
   std::vector<RawTensor*> raws;
   for (size_t k = 0; k < buckets.size(); ++k) {
-    frames.emplace_back(std::move(locks[k]), buckets[k], comm, false, false, &gather);
+    frames.emplace_back(std::move(locks[k]), buckets[k], comm, false, false, &staging);
     raws.push_back(frames.back().ct.raw.get());
   }
-  copy_joined(gather, true, comm.stream());
+  copy_joined(staging.gather, true, comm.stream());
   work(raws);
   for (OpFrame& f : frames) f.ct.finish(false, &scatter);
   copy_joined(scatter, false, comm.stream());
@@ -201,8 +205,8 @@ class CentralizedFullPrecisionSynchronous : public CommOp {
     auto* o = dynamic_cast<const CentralizedFullPrecisionSynchronous*>(&other);
     return o && o->comm_->internode() == comm_->internode();
   }
-  void execute_joined(const std::vector<BucketPtr>& buckets) override {
-    run_joined(*comm_, buckets, [](std::vector<RawTensor*>&) {});
+  void execute_joined(const std::vector<BucketPtr>& buckets, int64_t staging_bytes) override {
+    run_joined(*comm_, buckets, staging_bytes, [](std::vector<RawTensor*>&) {});
   }
 
  private:
@@ -261,8 +265,9 @@ class CentralizedLowPrecisionSynchronous : public CommOp {
     auto* o = dynamic_cast<const CentralizedLowPrecisionSynchronous*>(&other);
     return o && o->comm_->internode() == comm_->internode() && o->method_ == method_;
   }
-  void execute_joined(const std::vector<BucketPtr>& buckets) override {
-    run_joined(*comm_, buckets, [&](std::vector<RawTensor*>& ts) { tensor_ops::quantise_twice(ts, method_, comm_->stream()); });
+  void execute_joined(const std::vector<BucketPtr>& buckets, int64_t staging_bytes) override {
+    run_joined(*comm_, buckets, staging_bytes,
+               [&](std::vector<RawTensor*>& ts) { tensor_ops::quantise_twice(ts, method_, comm_->stream()); });
   }
 
  private:

@@ -47,7 +47,7 @@ void CommBackend::worker_loop() {
     }
     const bool joinable = batch[0]->joins();
     if (joinable) join_followers(batch);
-    execute(batch);
+    execute(batch, joinable);
     if (!joinable) continue;
     int64_t bytes = 0;
     for (auto& item : batch) bytes += item->bucket->total_allocated() * (int64_t)dtype_bytes(item->bucket->dtype());
@@ -58,6 +58,7 @@ void CommBackend::worker_loop() {
 void CommBackend::join_followers(std::vector<std::shared_ptr<ScheduledCommOp>>& batch) {
   const auto now = std::chrono::steady_clock::now();
   const auto until = std::min(busy_until_ - std::chrono::microseconds(kJoinAheadUs), now + std::chrono::microseconds(kJoinMostUs));
+  int64_t staged = batch[0]->place->staged_bytes;
   while (batch.size() < (size_t)kernels::kMaxJoined) {
     std::optional<std::shared_ptr<ScheduledCommOp>> item;
     spin_until(
@@ -70,6 +71,7 @@ void CommBackend::join_followers(std::vector<std::shared_ptr<ScheduledCommOp>>& 
     const ScheduledCommOp& op = **item;
     bool joins = op.joins() && batch[0]->ops[0]->joins_with(*op.ops[0]) && op.bucket->dtype() == batch[0]->bucket->dtype();
     for (auto& b : batch) joins = joins && b->bucket != op.bucket;  // twice in a row is one after the other
+    if (joins) joins = (staged += op.place->staged_bytes) <= batch[0]->staging_bytes;
     if (!joins) {
       next_ = std::move(*item);
       break;
@@ -78,7 +80,7 @@ void CommBackend::join_followers(std::vector<std::shared_ptr<ScheduledCommOp>>& 
   }
 }
 
-void CommBackend::execute(const std::vector<std::shared_ptr<ScheduledCommOp>>& batch) {
+void CommBackend::execute(const std::vector<std::shared_ptr<ScheduledCommOp>>& batch, bool joined) {
   for (auto& item : batch) {
     BAGUA_LOG(Debug, "worker received scheduled communication operation " << item->name);
     if (log_enabled(LogLevel::Debug)) {
@@ -102,10 +104,10 @@ void CommBackend::execute(const std::vector<std::shared_ptr<ScheduledCommOp>>& b
   static const bool nvtx = env_long("BAGUA_B200_NVTX", 0) != 0;
   if (nvtx) nvtxRangePushA(op.bucket->name().c_str());
   try {
-    if (batch.size() > 1) {
+    if (joined) {
       std::vector<BucketPtr> buckets;
       for (auto& item : batch) buckets.push_back(item->bucket);
-      op.ops[0]->execute_joined(buckets);
+      op.ops[0]->execute_joined(buckets, op.staging_bytes);
       EngineStats::global().ops_executed += batch.size();
     } else {
       for (auto& o : op.ops) {
@@ -181,8 +183,8 @@ void CommBackend::register_ordered_buckets(const std::vector<BucketPtr>& buckets
   };
   std::vector<Span> spans;
   for (auto& b : buckets) {
-    auto place = std::make_shared<const MemorySpans>(b->memory_spans());
-    for (auto& [from, to] : *place)
+    auto place = std::make_shared<const ScheduledCommOp::Place>(ScheduledCommOp::Place{b->memory_spans(), b->staged_bytes()});
+    for (auto& [from, to] : place->spans)
       if (from < to) spans.push_back({from, to, b.get()});
     places_[b.get()] = std::move(place);
   }
@@ -194,6 +196,10 @@ void CommBackend::register_ordered_buckets(const std::vector<BucketPtr>& buckets
     }
     if (spans[k].to > spans[last].to) last = k;
   }
+  staging_bytes_ = 0;
+  for (auto& [bucket, place] : places_)
+    if (place->staged_bytes <= kJoinedBytes) staging_bytes_ += place->staged_bytes;
+  staging_bytes_ = std::min(staging_bytes_, kJoinedBytes);
 }
 
 bool CommBackend::should_schedule() const {
@@ -207,6 +213,7 @@ void CommBackend::schedule_comm(const BucketPtr& bucket) {
   op->bucket = bucket;
   op->ops = bucket->ops_snapshot();
   if (auto it = places_.find(bucket.get()); it != places_.end()) op->place = it->second;
+  op->staging_bytes = staging_bytes_;
   EventChannel ev = op->event;
   const uint64_t t0 = Telemetry::instance().now();
   if (!schedule_.send(std::move(op))) throw BaguaError(ErrorKind::InternalChannel, "schedule channel is closed");

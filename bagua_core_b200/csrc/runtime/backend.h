@@ -35,10 +35,15 @@ struct ScheduledCommOp {
   BucketPtr bucket;
   std::vector<std::shared_ptr<CommOp>> ops;
   EventChannel event{"comm_op"};
-  // Where the bucket's tensors lay when it was registered; null: it shared memory with another.
-  std::shared_ptr<const MemorySpans> place;
+  // Where the bucket's tensors lay when it was registered, and what staging it takes; null: it shared memory with another.
+  struct Place {
+    MemorySpans spans;
+    int64_t staged_bytes;
+  };
+  std::shared_ptr<const Place> place;
+  int64_t staging_bytes = 0;  // of a batch that it is executed in
   // Whether it may be executed together with others.
-  bool joins() const { return place && ops.size() == 1 && ops[0]->joins(bucket) && bucket->memory_spans() == *place; }
+  bool joins() const { return place && ops.size() == 1 && ops[0]->joins(bucket) && bucket->memory_spans() == place->spans; }
 };
 
 class CommBackend {
@@ -66,15 +71,16 @@ class CommBackend {
   bool should_schedule() const;
   void schedule_comm(const BucketPtr& bucket);
   void worker_loop();
-  // Runs the ops of `batch`, of one bucket or of several that are executed together.
-  void execute(const std::vector<std::shared_ptr<ScheduledCommOp>>& batch);
+  // Runs the ops of `batch`, of one bucket or of several that are executed together (`joined`: as such, also if there is one).
+  void execute(const std::vector<std::shared_ptr<ScheduledCommOp>>& batch, bool joined);
   // Adds to `batch` what is scheduled behind it and can be executed with it; what was received and cannot stays in `next_`.
   void join_followers(std::vector<std::shared_ptr<ScheduledCommOp>>& batch);
   void monitor_loop();
 
   const int device_id_;
   std::deque<BucketPtr> ordered_buckets_;
-  std::unordered_map<const BaguaBucket*, std::shared_ptr<const MemorySpans>> places_;  // of those that share no memory with others
+  std::unordered_map<const BaguaBucket*, std::shared_ptr<const ScheduledCommOp::Place>> places_;  // of those that share no memory with others
+  int64_t staging_bytes_ = 0;  // what those of them that are staged take, at most kJoinedBytes
   std::mutex mu_;  // guards ordered_buckets_ and registration state
 
   Channel<std::shared_ptr<ScheduledCommOp>> schedule_;

@@ -231,8 +231,19 @@ std::string BaguaBucket::describe_ops() const {
   return oss.str();
 }
 
+JoinedStaging::JoinedStaging(int64_t bytes, int device, uint64_t stream) : bytes_(bytes), device_(device), stream_(stream) {}
+
+std::shared_ptr<PoolRawTensor> JoinedStaging::take(DType dt, int64_t numel) {
+  const int64_t part = part_bytes(numel * (int64_t)dtype_bytes(dt));
+  if (used_ + part > bytes_) return PoolRawTensor::allocate(device_, dt, numel, stream_);
+  if (!block_) block_ = MemoryPool::for_device(device_).pull((size_t)bytes_, stream_);
+  auto t = std::make_shared<PoolRawTensor>((char*)block_->ptr() + used_, block_, numel, numel, dt, device_);
+  used_ += part;
+  return t;
+}
+
 CommunicationTensor BaguaBucket::get_communication_tensor(uint64_t stream, bool force_copy, bool force_not_copy_back,
-                                                          std::vector<kernels::MultiCopyItem>* gather) {
+                                                          JoinedStaging* joined) {
   CommunicationTensor ct;
   ct.stream = stream;
   for (auto& t : tensors_) {
@@ -251,7 +262,7 @@ CommunicationTensor BaguaBucket::get_communication_tensor(uint64_t stream, bool 
   }
   // Staged: one launch gathers every tensor into a pool buffer (the reference issues one copy
   // per tensor, datatypes/mod.rs:1012-1023).
-  auto buf = PoolRawTensor::allocate(device_, dtype_, total, stream);
+  auto buf = joined ? joined->take(dtype_, total) : PoolRawTensor::allocate(device_, dtype_, total, stream);
   const size_t es = dtype_bytes(dtype_);
   unsigned long long off = 0;
   kernels::Ctx c{device_, (cudaStream_t)stream};
@@ -278,8 +289,8 @@ CommunicationTensor BaguaBucket::get_communication_tensor(uint64_t stream, bool 
     table = (const kernels::MultiCopySeg*)seg_cache_dev_->data_ptr();
   }
   ct.raw = buf;
-  if (gather && ct.segments_dev)
-    gather->push_back(ct.copy_item());
+  if (joined && ct.segments_dev)
+    joined->gather.push_back(ct.copy_item());
   else
     kernels::multi_copy(table, (int)ct.segments.size(), buf->data_ptr(), (size_t)off, /*gather=*/true, c);
   ct.staged = true;

@@ -138,6 +138,23 @@ class CommunicationTensor {
   }
 };
 
+// Where buckets that are executed together are staged: a part of one block each.
+class JoinedStaging {
+ public:
+  JoinedStaging(int64_t bytes, int device, uint64_t stream);
+  // The next part; a block of its own where there is no room.
+  std::shared_ptr<PoolRawTensor> take(DType dt, int64_t numel);
+  static int64_t part_bytes(int64_t bytes) { return (int64_t)align_up((size_t)bytes, 256); }
+  std::vector<kernels::MultiCopyItem> gather;  // the copies into it, which the caller launches
+
+ private:
+  const int64_t bytes_;
+  const int device_;
+  const uint64_t stream_;
+  std::shared_ptr<PoolBlock> block_;  // null until the first part is taken
+  int64_t used_ = 0;
+};
+
 using MemorySpans = std::vector<std::pair<uint64_t, uint64_t>>;  // addresses: from, to
 
 class BaguaBucket {
@@ -151,6 +168,9 @@ class BaguaBucket {
   int device_id() const { return device_; }
   int64_t total_allocated() const;
   bool contiguous() const;  // tensors address-adjacent in list order
+  int64_t staged_bytes() const {  // of a JoinedStaging
+    return contiguous() ? 0 : JoinedStaging::part_bytes(total_allocated() * (int64_t)dtype_bytes(dtype_));
+  }
   MemorySpans memory_spans() const;  // of every tensor, in list order
 
   bool ready_for_comm() const;
@@ -162,10 +182,10 @@ class BaguaBucket {
   std::vector<std::shared_ptr<CommOp>> ops_snapshot() const;
   std::string describe_ops() const;
 
-  // Waits (stream-side) on every tensor's ready event, then aliases or stages.  `gather`: on a GPU the copy into the staging buffer
-  // is left to the caller, who launches it together with others'.
+  // Waits (stream-side) on every tensor's ready event, then aliases or stages, with `joined` there; on a GPU the copy is
+  // then left to the caller, who launches it together with others'.
   CommunicationTensor get_communication_tensor(uint64_t stream, bool force_copy, bool force_not_copy_back,
-                                               std::vector<kernels::MultiCopyItem>* gather = nullptr);
+                                               JoinedStaging* joined = nullptr);
 
   std::mutex& exec_mutex() { return exec_mu_; }
 

@@ -3,6 +3,7 @@
 // at once.  The first bucket of a burst is held inside its launch until the others are scheduled, so that those are joined.
 //
 //   locks     backends that hold the same buckets in opposite orders do not wait for each other
+//   staging   buckets that are staged together take one block from the pool, whichever of them meet
 //   overlap   buckets that share memory, or whose tensors have moved to where they do, get what they get one after the other
 #include <cuda_runtime.h>
 
@@ -229,7 +230,50 @@ void locks() {
   for (float v : x) EXPECT(v == 3, "%g", v);
 }
 
-const std::map<std::string, void (*)()> kCases = {{"locks", locks}, {"overlap", overlap}};
+// Twelve staged buckets of 6 MB: executed one by one, then in bursts of any length.
+void staging() {
+  constexpr int64_t kHalf = 3 << 18;  // floats
+  constexpr int kBuckets = 12;
+  std::vector<float> x((size_t)kBuckets * 2 * (kHalf + 16));
+  auto op = make_centralized_low_precision_op(one_rank(1), true, "MinMaxUInt8");
+  CommBackend backend(100, 0);
+  std::vector<BucketPtr> buckets;
+  for (int k = 0; k < kBuckets; ++k) {
+    float* at = x.data() + (size_t)k * 2 * (kHalf + 16);
+    buckets.push_back(make_bucket("b" + std::to_string(k), {{at, kHalf}, {at + kHalf + 16, kHalf}}, op));
+  }
+  backend.register_ordered_buckets(buckets);
+  const MemoryPool& pool = MemoryPool::for_device(0);
+  for (auto& b : buckets) {
+    mark(backend, b);
+    backend.wait_pending_comm_ops();
+  }
+  const PoolStats first = pool.stats();
+  EXPECT(first.bytes_reserved <= (32 << 20) + kBuckets * 4096, "%llu bytes reserved", (unsigned long long)first.bytes_reserved);
+  quantise_launches.clear();
+  burst(backend, buckets);
+  backend.wait_pending_comm_ops();
+  EXPECT(quantise_launches == (std::vector<int>{1, 5, 5, 1}), "five buckets at a time stay below 32 MB");
+  for (size_t many = 1; many <= kBuckets; ++many)
+    for (size_t from = 0; from < kBuckets; from += many) {
+      burst(backend, {buckets.begin() + from, buckets.begin() + std::min<size_t>(from + many, kBuckets)});
+      backend.wait_pending_comm_ops();
+    }
+  EXPECT(pool.stats().device_allocs == first.device_allocs, "%llu allocations, %llu before",
+         (unsigned long long)pool.stats().device_allocs, (unsigned long long)first.device_allocs);
+  const float want = (float)((1 << (kBuckets + 2)) - 1);
+  for (int k = 0; k < kBuckets; ++k)
+    for (int64_t i = 0; i < 2 * kHalf + 32; ++i) {
+      const bool mine = i < kHalf || (i >= kHalf + 16 && i < 2 * kHalf + 16);
+      const float v = x[(size_t)k * 2 * (kHalf + 16) + (size_t)i];
+      if (v != (mine ? want : 0.f)) {
+        EXPECT(false, "bucket %d, value %lld: %g", k, (long long)i, v);
+        return;
+      }
+    }
+}
+
+const std::map<std::string, void (*)()> kCases = {{"locks", locks}, {"overlap", overlap}, {"staging", staging}};
 }  // namespace
 
 int main(int argc, char** argv) {

@@ -41,3 +41,7 @@ def test_buckets_that_share_memory_are_executed_one_after_the_other(program):
 
 def test_joined_buckets_are_locked_in_one_order(program):
     _run(program, "locks")
+
+
+def test_staged_buckets_share_one_block_however_they_meet(program):
+    _run(program, "staging")
