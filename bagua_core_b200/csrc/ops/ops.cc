@@ -95,8 +95,8 @@ struct OpFrame {
 // Buckets of a communicator of one rank on a GPU: nothing travels, each bucket's part is local, and several that are ready at once are
 // gathered, worked on and scattered in one launch each.  Not where somebody looks at them one by one, nor buckets that keep the GPU busy
 // for longer than they wait for it anyway (VGG-16's bf16 buckets, one of them of 205 MB, quantised: 185 us alone, 192 all joined, 180-183 with this limit).
-bool joins_over_one_rank(const Communicator& comm, const BucketPtr& bucket) {
-  return bucket->device_id() >= 0 && bucket->total_allocated() * (int64_t)dtype_bytes(bucket->dtype()) <= kJoinedBytes &&
+bool joins_over_one_rank(const Communicator& comm, const BaguaBucket& bucket, const BucketLayout& layout) {
+  return bucket.device_id() >= 0 && layout.bytes <= kJoinedBytes &&
          comm.kind() == Communicator::Kind::Single && comm.internode() && comm.internode()->nranks() == 1 &&
          !EngineConfig::global().sync_per_bucket && !BucketTimeline::instance().enabled() &&
          kernels::cuda::multi_copy_joined != nullptr;
@@ -198,8 +198,8 @@ class CentralizedFullPrecisionSynchronous : public CommOp {
     return o.str();
   }
   // over one rank: a bucket that is not staged is done as it is
-  bool joins(const BucketPtr& bucket) const override {
-    return joins_over_one_rank(*comm_, bucket) && !occupies_for_probe() && !bucket->contiguous();
+  bool joins(const BaguaBucket& bucket, const BucketLayout& layout) const override {
+    return joins_over_one_rank(*comm_, bucket, layout) && !occupies_for_probe() && !layout.contiguous;
   }
   bool joins_with(const CommOp& other) const override {
     auto* o = dynamic_cast<const CentralizedFullPrecisionSynchronous*>(&other);
@@ -260,7 +260,7 @@ class CentralizedLowPrecisionSynchronous : public CommOp {
     o << "CentralizedLowPrecisionSynchronous{average=" << average_ << ", compression=" << method_ << "}";
     return o.str();
   }
-  bool joins(const BucketPtr& bucket) const override { return joins_over_one_rank(*comm_, bucket); }
+  bool joins(const BaguaBucket& bucket, const BucketLayout& layout) const override { return joins_over_one_rank(*comm_, bucket, layout); }
   bool joins_with(const CommOp& other) const override {
     auto* o = dynamic_cast<const CentralizedLowPrecisionSynchronous*>(&other);
     return o && o->comm_->internode() == comm_->internode() && o->method_ == method_;

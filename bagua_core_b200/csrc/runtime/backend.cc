@@ -50,7 +50,7 @@ void CommBackend::worker_loop() {
     execute(batch, joinable);
     if (!joinable) continue;
     int64_t bytes = 0;
-    for (auto& item : batch) bytes += item->bucket->total_allocated() * (int64_t)dtype_bytes(item->bucket->dtype());
+    for (auto& item : batch) bytes += item->layout->bytes;
     busy_until_ = std::max(busy_until_, std::chrono::steady_clock::now()) + std::chrono::microseconds(kJoinBaseUs + bytes / kJoinBytesPerUs);
   }
 }
@@ -58,7 +58,7 @@ void CommBackend::worker_loop() {
 void CommBackend::join_followers(std::vector<std::shared_ptr<ScheduledCommOp>>& batch) {
   const auto now = std::chrono::steady_clock::now();
   const auto until = std::min(busy_until_ - std::chrono::microseconds(kJoinAheadUs), now + std::chrono::microseconds(kJoinMostUs));
-  int64_t staged = batch[0]->place->staged_bytes;
+  int64_t staged = batch[0]->layout->staged_bytes();
   while (batch.size() < (size_t)kernels::kMaxJoined) {
     std::optional<std::shared_ptr<ScheduledCommOp>> item;
     spin_until(
@@ -71,7 +71,7 @@ void CommBackend::join_followers(std::vector<std::shared_ptr<ScheduledCommOp>>& 
     const ScheduledCommOp& op = **item;
     bool joins = op.joins() && batch[0]->ops[0]->joins_with(*op.ops[0]) && op.bucket->dtype() == batch[0]->bucket->dtype();
     for (auto& b : batch) joins = joins && b->bucket != op.bucket;  // twice in a row is one after the other
-    if (joins) joins = (staged += op.place->staged_bytes) <= batch[0]->staging_bytes;
+    if (joins) joins = (staged += op.layout->staged_bytes()) <= batch[0]->staging_bytes;
     if (!joins) {
       next_ = std::move(*item);
       break;
@@ -157,7 +157,7 @@ void CommBackend::register_ordered_buckets(const std::vector<BucketPtr>& buckets
   wait_pending_comm_ops();
   std::lock_guard<std::mutex> g(mu_);
   ordered_buckets_.clear();
-  places_.clear();
+  layouts_.clear();
   std::unordered_set<std::string> names;
   std::unordered_set<uint64_t> ptrs;
   for (auto& b : buckets) {
@@ -183,22 +183,22 @@ void CommBackend::register_ordered_buckets(const std::vector<BucketPtr>& buckets
   };
   std::vector<Span> spans;
   for (auto& b : buckets) {
-    auto place = std::make_shared<const ScheduledCommOp::Place>(ScheduledCommOp::Place{b->memory_spans(), b->staged_bytes()});
-    for (auto& [from, to] : place->spans)
+    auto layout = std::make_shared<const BucketLayout>(b->layout());
+    for (auto& [from, to] : layout->spans)
       if (from < to) spans.push_back({from, to, b.get()});
-    places_[b.get()] = std::move(place);
+    layouts_[b.get()] = std::move(layout);
   }
   std::sort(spans.begin(), spans.end(), [](const Span& a, const Span& b) { return a.from < b.from; });
   for (size_t k = 1, last = 0; k < spans.size(); ++k) {
     if (spans[k].from < spans[last].to && spans[k].bucket != spans[last].bucket) {
-      places_.erase(spans[k].bucket);
-      places_.erase(spans[last].bucket);
+      layouts_.erase(spans[k].bucket);
+      layouts_.erase(spans[last].bucket);
     }
     if (spans[k].to > spans[last].to) last = k;
   }
   staging_bytes_ = 0;
-  for (auto& [bucket, place] : places_)
-    if (place->staged_bytes <= kJoinedBytes) staging_bytes_ += place->staged_bytes;
+  for (auto& [bucket, layout] : layouts_)
+    if (layout->bytes <= kJoinedBytes) staging_bytes_ += layout->staged_bytes();
   staging_bytes_ = std::min(staging_bytes_, kJoinedBytes);
 }
 
@@ -212,7 +212,7 @@ void CommBackend::schedule_comm(const BucketPtr& bucket) {
   op->name = bucket->name();
   op->bucket = bucket;
   op->ops = bucket->ops_snapshot();
-  if (auto it = places_.find(bucket.get()); it != places_.end()) op->place = it->second;
+  if (auto it = layouts_.find(bucket.get()); it != layouts_.end()) op->layout = it->second;
   op->staging_bytes = staging_bytes_;
   EventChannel ev = op->event;
   const uint64_t t0 = Telemetry::instance().now();

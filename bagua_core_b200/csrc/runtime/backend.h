@@ -35,15 +35,12 @@ struct ScheduledCommOp {
   BucketPtr bucket;
   std::vector<std::shared_ptr<CommOp>> ops;
   EventChannel event{"comm_op"};
-  // Where the bucket's tensors lay when it was registered, and what staging it takes; null: it shared memory with another.
-  struct Place {
-    MemorySpans spans;
-    int64_t staged_bytes;
-  };
-  std::shared_ptr<const Place> place;
+  // How the bucket's tensors lay when it was registered; null: it shared memory with another.
+  std::shared_ptr<const BucketLayout> layout;
   int64_t staging_bytes = 0;  // of a batch that it is executed in
   // Whether it may be executed together with others.
-  bool joins() const { return place && ops.size() == 1 && ops[0]->joins(bucket) && bucket->memory_spans() == place->spans; }
+  // (asked for every bucket on the worker, so with one pass over its tensors)
+  bool joins() const { return layout && ops.size() == 1 && ops[0]->joins(*bucket, *layout) && bucket->lies_as(*layout); }
 };
 
 class CommBackend {
@@ -79,7 +76,7 @@ class CommBackend {
 
   const int device_id_;
   std::deque<BucketPtr> ordered_buckets_;
-  std::unordered_map<const BaguaBucket*, std::shared_ptr<const ScheduledCommOp::Place>> places_;  // of those that share no memory with others
+  std::unordered_map<const BaguaBucket*, std::shared_ptr<const BucketLayout>> layouts_;  // of those that share no memory with others
   int64_t staging_bytes_ = 0;  // what those of them that are staged take, at most kJoinedBytes
   std::mutex mu_;  // guards ordered_buckets_ and registration state
 

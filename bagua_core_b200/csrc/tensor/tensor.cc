@@ -185,11 +185,25 @@ bool BaguaBucket::contiguous() const {
   return true;
 }
 
-MemorySpans BaguaBucket::memory_spans() const {
-  MemorySpans spans;
-  spans.reserve(tensors_.size());
-  for (auto& t : tensors_) spans.emplace_back(t->data_ptr(), t->data_ptr() + t->raw()->bytes_allocated());
-  return spans;
+BucketLayout BaguaBucket::layout() const {
+  BucketLayout l;
+  l.spans.reserve(tensors_.size());
+  for (auto& t : tensors_) {
+    const uint64_t from = t->data_ptr();
+    l.spans.emplace_back(from, from + t->raw()->bytes_allocated());
+    l.bytes += (int64_t)t->raw()->bytes_allocated();
+  }
+  l.contiguous = contiguous();
+  return l;
+}
+bool BaguaBucket::lies_as(const BucketLayout& then) const {
+  const uint64_t es = dtype_bytes(dtype_);
+  for (size_t k = 0; k < tensors_.size(); ++k) {
+    const RawTensor& t = *tensors_[k]->raw();
+    const auto& [from, to] = then.spans[k];
+    if ((uint64_t)(uintptr_t)t.data_ptr() != from || from + (uint64_t)t.num_elements_allocated() * es != to) return false;
+  }
+  return true;
 }
 
 bool BaguaBucket::ready_for_comm() const {

@@ -155,7 +155,13 @@ class JoinedStaging {
   int64_t used_ = 0;
 };
 
-using MemorySpans = std::vector<std::pair<uint64_t, uint64_t>>;  // addresses: from, to
+// Where a bucket's tensors lie, in list order.
+struct BucketLayout {
+  std::vector<std::pair<uint64_t, uint64_t>> spans;  // addresses: from, to
+  int64_t bytes = 0;                                 // of all
+  bool contiguous = false;
+  int64_t staged_bytes() const { return contiguous ? 0 : JoinedStaging::part_bytes(bytes); }
+};
 
 class BaguaBucket {
  public:
@@ -168,10 +174,8 @@ class BaguaBucket {
   int device_id() const { return device_; }
   int64_t total_allocated() const;
   bool contiguous() const;  // tensors address-adjacent in list order
-  int64_t staged_bytes() const {  // of a JoinedStaging
-    return contiguous() ? 0 : JoinedStaging::part_bytes(total_allocated() * (int64_t)dtype_bytes(dtype_));
-  }
-  MemorySpans memory_spans() const;  // of every tensor, in list order
+  BucketLayout layout() const;
+  bool lies_as(const BucketLayout& then) const;
 
   bool ready_for_comm() const;
   void reset_comm_ready();
