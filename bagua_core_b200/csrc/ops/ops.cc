@@ -117,22 +117,30 @@ std::vector<std::unique_lock<std::mutex>> lock_all(const std::vector<BucketPtr>&
   return locks;
 }
 // All staging buffers of the batch are wanted until its scatter is launched; they are parts of one block, which every batch of these
-// buckets pulls in the same size: what the pool holds does not depend on which buckets happened to meet.
-void run_joined(Communicator& comm, const std::vector<BucketPtr>& buckets, int64_t staging_bytes,
-                const std::function<void(std::vector<RawTensor*>&)>& work) {
+// buckets pulls in the same size: what the pool holds does not depend on which buckets happened to meet.  A bucket that cannot be
+// prepared fails alone.
+std::vector<std::string> run_joined(Communicator& comm, const std::vector<BucketPtr>& buckets, int64_t staging_bytes,
+                                    const std::function<void(std::vector<RawTensor*>&)>& work) {
+  std::vector<std::string> errors(buckets.size());
   auto locks = lock_all(buckets);
   JoinedStaging staging(staging_bytes, buckets[0]->device_id(), comm.stream());
   std::vector<kernels::MultiCopyItem> scatter;
   std::deque<OpFrame> frames;
   std::vector<RawTensor*> raws;
   for (size_t k = 0; k < buckets.size(); ++k) {
-    frames.emplace_back(std::move(locks[k]), buckets[k], comm, false, false, &staging);
-    raws.push_back(frames.back().ct.raw.get());
+    try {
+      frames.emplace_back(std::move(locks[k]), buckets[k], comm, false, false, &staging);
+      raws.push_back(frames.back().ct.raw.get());
+    } catch (const std::exception& e) {
+      errors[k] = e.what();
+    }
   }
+  if (frames.empty()) return errors;
   copy_joined(staging.gather, true, comm.stream());
   work(raws);
   for (OpFrame& f : frames) f.ct.finish(false, &scatter);
   copy_joined(scatter, false, comm.stream());
+  return errors;
 }
 bool occupies_for_probe() {
   static const bool on = std::getenv("BAGUA_B200_PROBE_OCCUPY") != nullptr;
@@ -205,8 +213,8 @@ class CentralizedFullPrecisionSynchronous : public CommOp {
     auto* o = dynamic_cast<const CentralizedFullPrecisionSynchronous*>(&other);
     return o && o->comm_->internode() == comm_->internode();
   }
-  void execute_joined(const std::vector<BucketPtr>& buckets, int64_t staging_bytes) override {
-    run_joined(*comm_, buckets, staging_bytes, [](std::vector<RawTensor*>&) {});
+  std::vector<std::string> execute_joined(const std::vector<BucketPtr>& buckets, int64_t staging_bytes) override {
+    return run_joined(*comm_, buckets, staging_bytes, [](std::vector<RawTensor*>&) {});
   }
 
  private:
@@ -265,8 +273,8 @@ class CentralizedLowPrecisionSynchronous : public CommOp {
     auto* o = dynamic_cast<const CentralizedLowPrecisionSynchronous*>(&other);
     return o && o->comm_->internode() == comm_->internode() && o->method_ == method_;
   }
-  void execute_joined(const std::vector<BucketPtr>& buckets, int64_t staging_bytes) override {
-    run_joined(*comm_, buckets, staging_bytes,
+  std::vector<std::string> execute_joined(const std::vector<BucketPtr>& buckets, int64_t staging_bytes) override {
+    return run_joined(*comm_, buckets, staging_bytes,
                [&](std::vector<RawTensor*>& ts) { tensor_ops::quantise_twice(ts, method_, comm_->stream()); });
   }
 

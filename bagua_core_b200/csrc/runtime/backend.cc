@@ -80,6 +80,14 @@ void CommBackend::join_followers(std::vector<std::shared_ptr<ScheduledCommOp>>& 
   }
 }
 
+namespace {
+std::string names_of(const std::vector<BucketPtr>& buckets) {
+  std::string s = buckets.size() > 1 ? "buckets " : "bucket ";
+  for (size_t k = 0; k < buckets.size(); ++k) s += (k ? ", `" : "`") + buckets[k]->name() + "`";
+  return s;
+}
+}  // namespace
+
 void CommBackend::execute(const std::vector<std::shared_ptr<ScheduledCommOp>>& batch, bool joined) {
   for (auto& item : batch) {
     BAGUA_LOG(Debug, "worker received scheduled communication operation " << item->name);
@@ -91,24 +99,27 @@ void CommBackend::execute(const std::vector<std::shared_ptr<ScheduledCommOp>>& b
     }
   }
   const ScheduledCommOp& op = *batch[0];
+  std::vector<BucketPtr> buckets;
+  for (auto& item : batch) buckets.push_back(item->bucket);
   {
     std::lock_guard<std::mutex> g(current_.mu);
-    current_.bucket = op.bucket;
+    current_.buckets = buckets;
     current_.since = std::chrono::steady_clock::now();
     current_.reported = false;
   }
   const uint64_t t0 = Telemetry::instance().now();
-  std::string err;
-  // Optional NVTX range per bucket (BAGUA_B200_NVTX=1) so that profiler timelines line up
+  std::vector<std::string> errors(batch.size());
+  // Optional NVTX range per bucket or joined batch (BAGUA_B200_NVTX=1) so that profiler timelines line up
   // with bucket names; a no-op when no tool is attached.
   static const bool nvtx = env_long("BAGUA_B200_NVTX", 0) != 0;
-  if (nvtx) nvtxRangePushA(op.bucket->name().c_str());
+  if (nvtx) nvtxRangePushA(batch.size() > 1 ? names_of(buckets).c_str() : op.bucket->name().c_str());
   try {
     if (joined) {
-      std::vector<BucketPtr> buckets;
-      for (auto& item : batch) buckets.push_back(item->bucket);
-      op.ops[0]->execute_joined(buckets, op.staging_bytes);
-      EngineStats::global().ops_executed += batch.size();
+      errors = op.ops[0]->execute_joined(buckets, op.staging_bytes);
+      EngineStats::global().ops_executed += (uint64_t)std::count(errors.begin(), errors.end(), "");
+      for (size_t k = 0; k < batch.size(); ++k)
+        if (!errors[k].empty())
+          BAGUA_LOG(Error, "communication op on bucket `" << batch[k]->bucket->name() << "` failed: " << errors[k]);
     } else {
       for (auto& o : op.ops) {
         o->execute_background_communication(op.bucket);
@@ -116,21 +127,21 @@ void CommBackend::execute(const std::vector<std::shared_ptr<ScheduledCommOp>>& b
       }
     }
   } catch (const std::exception& e) {
-    err = e.what();
-    BAGUA_LOG(Error, "communication op on bucket `" << op.bucket->name() << "` failed: " << err);
+    errors.assign(batch.size(), e.what());
+    BAGUA_LOG(Error, "communication op on " << names_of(buckets) << " failed: " << e.what());
   }
   if (nvtx) nvtxRangePop();
   for (auto& item : batch) Telemetry::instance().record("bucket_executed", item->bucket->name(), t0);
   {
     std::lock_guard<std::mutex> g(current_.mu);
-    current_.bucket.reset();
+    current_.buckets.clear();
   }
-  for (auto& item : batch) {
-    if (err.empty())
-      item->event.finish();
+  for (size_t k = 0; k < batch.size(); ++k) {
+    if (errors[k].empty())
+      batch[k]->event.finish();
     else
-      item->event.fail(err);
-    BAGUA_LOG(Debug, "comm op executed: " << item->name);
+      batch[k]->event.fail(errors[k]);
+    BAGUA_LOG(Debug, "comm op executed: " << batch[k]->name);
   }
 }
 
@@ -141,12 +152,12 @@ void CommBackend::monitor_loop() {
     // often enough to report within a tenth of the limit, at most ten times a second
     const double look = limit <= 0 ? 0.1 : std::min(0.1, std::max(0.005, limit / 10));
     current_.stop_cv.wait_for(lk, std::chrono::duration<double>(look), [&] { return current_.stop; });
-    if (current_.stop || !current_.bucket || current_.reported || limit <= 0) continue;
+    if (current_.stop || current_.buckets.empty() || current_.reported || limit <= 0) continue;
     const std::chrono::duration<double> running = std::chrono::steady_clock::now() - current_.since;
     if (running.count() < limit) continue;
     // reported once; the op may still complete, the error goes to the next waiter
     current_.reported = true;
-    const std::string what = "bucket `" + current_.bucket->name() + "` comm op has not finished for " + fmt_double(limit) + " s";
+    const std::string what = names_of(current_.buckets) + " comm op has not finished for " + fmt_double(limit) + " s";
     BAGUA_LOG(Error, what);
     std::lock_guard<std::mutex> g(err_mu_);
     if (watchdog_error_.empty()) watchdog_error_ = what;

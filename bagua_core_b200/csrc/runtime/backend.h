@@ -97,7 +97,7 @@ class CommBackend {
   struct Current {
     std::mutex mu;
     std::condition_variable stop_cv;
-    BucketPtr bucket;  // null: nothing
+    std::vector<BucketPtr> buckets;  // empty: nothing
     std::chrono::steady_clock::time_point since;
     bool reported = false, stop = false;
   } current_;

@@ -249,8 +249,14 @@ JoinedStaging::JoinedStaging(int64_t bytes, int device, uint64_t stream) : bytes
 
 std::shared_ptr<PoolRawTensor> JoinedStaging::take(DType dt, int64_t numel) {
   const int64_t part = part_bytes(numel * (int64_t)dtype_bytes(dt));
+  if (!block_ && part <= bytes_) {
+    try {
+      block_ = MemoryPool::for_device(device_).pull((size_t)bytes_, stream_);
+    } catch (const BaguaError&) {
+      bytes_ = 0;
+    }
+  }
   if (used_ + part > bytes_) return PoolRawTensor::allocate(device_, dt, numel, stream_);
-  if (!block_) block_ = MemoryPool::for_device(device_).pull((size_t)bytes_, stream_);
   auto t = std::make_shared<PoolRawTensor>((char*)block_->ptr() + used_, block_, numel, numel, dt, device_);
   used_ += part;
   return t;

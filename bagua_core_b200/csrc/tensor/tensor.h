@@ -142,13 +142,13 @@ class CommunicationTensor {
 class JoinedStaging {
  public:
   JoinedStaging(int64_t bytes, int device, uint64_t stream);
-  // The next part; a block of its own where there is no room.
+  // The next part; a block of its own where there is no room, or no block of that size to be had.
   std::shared_ptr<PoolRawTensor> take(DType dt, int64_t numel);
   static int64_t part_bytes(int64_t bytes) { return (int64_t)align_up((size_t)bytes, 256); }
   std::vector<kernels::MultiCopyItem> gather;  // the copies into it, which the caller launches
 
  private:
-  const int64_t bytes_;
+  int64_t bytes_;
   const int device_;
   const uint64_t stream_;
   std::shared_ptr<PoolBlock> block_;  // null until the first part is taken

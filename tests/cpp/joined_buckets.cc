@@ -2,6 +2,8 @@
 // over a stand-in for the CUDA runtime and for the kernels, in which device memory is host memory and a launch does its work
 // at once.  The first bucket of a burst is held inside its launch until the others are scheduled, so that those are joined.
 //
+//   failing   a bucket that cannot be prepared fails alone
+//   watchdog  a launch that does not return is reported under the names of all its buckets
 //   locks     backends that hold the same buckets in opposite orders do not wait for each other
 //   staging   buckets that are staged together take one block from the pool, whichever of them meet
 //   overlap   buckets that share memory, or whose tensors have moved to where they do, get what they get one after the other
@@ -41,7 +43,7 @@ int failures = 0;
 struct Gate {
   std::mutex mu;
   std::condition_variable cv;
-  bool closed = false, reached = false;
+  bool closed = false, reached = false, let_one = false;
   void close() {
     std::lock_guard<std::mutex> g(mu);
     closed = true;
@@ -51,7 +53,14 @@ struct Gate {
     std::unique_lock<std::mutex> lk(mu);
     reached = true;
     cv.notify_all();
-    cv.wait(lk, [&] { return !closed; });
+    cv.wait(lk, [&] { return !closed || let_one; });
+    if (let_one) reached = let_one = false;
+  }
+  void pass_one() {
+    std::lock_guard<std::mutex> g(mu);
+    let_one = true;
+    reached = false;
+    cv.notify_all();
   }
   void wait_reached() {
     std::unique_lock<std::mutex> lk(mu);
@@ -90,7 +99,9 @@ cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) {
   std::memset(d, v, n);
   return cudaSuccess;
 }
-cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+const cudaEvent_t kNoEvent = (cudaEvent_t)(uintptr_t)0xbad;
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t e, unsigned) { return e == kNoEvent ? cudaErrorInvalidResourceHandle : cudaSuccess; }
+const char* cudaGetErrorString(cudaError_t) { return "no such event"; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 }
 
@@ -169,13 +180,14 @@ void mark(CommBackend& backend, const BucketPtr& b) {
   for (auto& t : b->tensors()) backend.mark_communication_ready(t, 0);
 }
 // The buckets in their order, the first held until the last is scheduled.
-void burst(CommBackend& backend, const std::vector<BucketPtr>& buckets, const std::function<void()>& while_held = {}) {
+void burst(CommBackend& backend, const std::vector<BucketPtr>& buckets, const std::function<void()>& while_held = {},
+           bool open = true) {
   gate.close();
   mark(backend, buckets[0]);
   gate.wait_reached();
   for (size_t k = 1; k < buckets.size(); ++k) mark(backend, buckets[k]);
   if (while_held) while_held();
-  gate.open();
+  if (open) gate.open();
 }
 
 void overlap() {
@@ -230,6 +242,70 @@ void locks() {
   for (float v : x) EXPECT(v == 3, "%g", v);
 }
 
+std::string error_of_wait(CommBackend& backend) {
+  try {
+    backend.wait_pending_comm_ops();
+  } catch (const std::exception& e) {
+    return e.what();
+  }
+  return "";
+}
+
+void failing() {
+  for (const bool staged : {false, true}) {
+    std::vector<float> x(6 * 16), held(16);
+    auto op = make_centralized_low_precision_op(one_rank(1), true, "MinMaxUInt8");
+    CommBackend backend(100, 0);
+    std::vector<BucketPtr> buckets = {make_bucket("held", {{held.data(), 16}}, op)};
+    for (int k = 0; k < 6; ++k) {
+      float* at = x.data() + 16 * k;
+      buckets.push_back(make_bucket("b" + std::to_string(k), staged ? Spans{{at, 4}, {at + 8, 8}} : Spans{{at, 16}}, op));
+    }
+    backend.register_ordered_buckets(buckets);
+    quantise_launches.clear();
+    gate.close();
+    mark(backend, buckets[0]);
+    gate.wait_reached();
+    for (size_t k = 1; k < buckets.size(); ++k)
+      for (auto& t : buckets[k]->tensors()) backend.mark_communication_ready(t, k == 3 ? (uint64_t)(uintptr_t)kNoEvent : 0);
+    gate.open();
+    const std::string error = error_of_wait(backend);
+    EXPECT(error.find("no such event") != std::string::npos, "the error was: %s", error.c_str());
+    EXPECT(quantise_launches == (std::vector<int>{1, 5}), "the other five were not worked on together");
+    for (int i = 0; i < 96; ++i) {
+      const float want = i / 16 == 2 || (staged && i % 16 >= 4 && i % 16 < 8) ? 0 : 1;
+      if (x[(size_t)i] != want) {
+        EXPECT(false, "value %d is %g", i, x[(size_t)i]);
+        break;
+      }
+    }
+    // and the next time it is a bucket like the others
+    burst(backend, buckets);
+    EXPECT(error_of_wait(backend).empty(), "the second burst failed");
+    EXPECT(x[32] == 1 && x[0] == 3, "%g %g", x[32], x[0]);
+  }
+}
+
+void watchdog() {
+  std::vector<float> x(64);
+  auto op = make_centralized_low_precision_op(one_rank(1), true, "MinMaxUInt8");
+  CommBackend backend(100, 0);
+  std::vector<BucketPtr> buckets;
+  for (int k = 0; k < 4; ++k) buckets.push_back(make_bucket("b" + std::to_string(k), {{x.data() + 16 * k, 16}}, op));
+  backend.register_ordered_buckets(buckets);
+  burst(backend, buckets, [] {
+    gate.pass_one();
+    gate.wait_reached();
+  }, /*open=*/false);
+  backend.set_watchdog_timeout(0.05);
+  const std::string error = error_of_wait(backend);
+  EXPECT(error.find("buckets `b1`, `b2`, `b3` comm op has not finished") != std::string::npos, "the report was: %s", error.c_str());
+  backend.set_watchdog_timeout(0);
+  gate.open();
+  error_of_wait(backend);
+  for (float v : x) EXPECT(v == 1, "%g", v);
+}
+
 // Twelve staged buckets of 6 MB: executed one by one, then in bursts of any length.
 void staging() {
   constexpr int64_t kHalf = 3 << 18;  // floats
@@ -273,7 +349,8 @@ void staging() {
     }
 }
 
-const std::map<std::string, void (*)()> kCases = {{"locks", locks}, {"overlap", overlap}, {"staging", staging}};
+const std::map<std::string, void (*)()> kCases = {
+    {"failing", failing}, {"locks", locks}, {"overlap", overlap}, {"staging", staging}, {"watchdog", watchdog}};
 }  // namespace
 
 int main(int argc, char** argv) {

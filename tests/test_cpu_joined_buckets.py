@@ -45,3 +45,11 @@ def test_joined_buckets_are_locked_in_one_order(program):
 
 def test_staged_buckets_share_one_block_however_they_meet(program):
     _run(program, "staging")
+
+
+def test_a_bucket_that_cannot_be_prepared_fails_alone(program):
+    _run(program, "failing")
+
+
+def test_the_watchdog_names_all_buckets_of_a_launch(program):
+    _run(program, "watchdog")
