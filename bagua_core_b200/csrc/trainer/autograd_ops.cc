@@ -415,7 +415,8 @@ at::Tensor conv_composition(const std::vector<at::Tensor>& in, const std::vector
 
 struct ConvNode : public AccumulatingNode {
   SavedVariable x, w, b, act;  // act: the activation, or with pooling the convolution's output (CPU)
-  // CUDA: a bit per value of the activation, whether it is positive; with pooling four per pooled value, where it came from
+  // CUDA: a bit per value of the activation, whether it is positive; with pooling four per pooled value, where it came from.
+  // Not where first_layer() is expected to serve: that reads the activation.
   SavedVariable signs;
   at::Tensor weight, bias;
   std::vector<int64_t> stride, padding, dilation;
@@ -510,12 +511,13 @@ struct ConvNode : public AccumulatingNode {
   }
 
   // A 3 x 3 convolution of few channels whose input wants no gradient: both gradients come from one kernel.
-  bool first_layer(const at::Tensor& xs, const at::Tensor& dy, const at::Tensor& a) {
-    return a.is_cuda() && !task_should_compute_output(0) && task_should_compute_output(1) && is_plain3x3() &&
-           xs.scalar_type() == at::kBFloat16 && xs.is_contiguous(at::MemoryFormat::ChannelsLast) &&
-           a.is_contiguous(at::MemoryFormat::ChannelsLast) && (uintptr_t)dy.data_ptr() % 16 == 0 &&
-           (uintptr_t)a.data_ptr() % 16 == 0 &&
+  bool first_layer_shape(const at::Tensor& xs, const at::Tensor& a) const {
+    return a.is_cuda() && is_plain3x3() && xs.scalar_type() == at::kBFloat16 && xs.is_contiguous(at::MemoryFormat::ChannelsLast) &&
+           a.is_contiguous(at::MemoryFormat::ChannelsLast) && (uintptr_t)a.data_ptr() % 16 == 0 &&
            model_ops::first_conv_backward_supported(a.size(0), a.size(2), a.size(3), a.size(1), xs.size(1));
+  }
+  bool first_layer(const at::Tensor& xs, const at::Tensor& dy, const at::Tensor& a) {
+    return !task_should_compute_output(0) && task_should_compute_output(1) && (uintptr_t)dy.data_ptr() % 16 == 0 && first_layer_shape(xs, a);
   }
   void first_layer_backward(const at::Tensor& xs, const at::Tensor& dy, const at::Tensor& a, variable_list& out) {
     const int C = (int)a.size(1), Ci = (int)xs.size(1);
@@ -560,7 +562,7 @@ struct ConvNode : public AccumulatingNode {
                                                     stream_of(dz), add);
     else
       model_ops::bias_relu_backward_bf16(dy.data_ptr(), a.data_ptr(), dz.data_ptr(), dbp, rows, C, scratch->data_ptr(),
-                                         stream_of(dz), add, bits.data_ptr());
+                                         stream_of(dz), add, bits.defined() ? bits.data_ptr() : nullptr);
     count_launches(2);  // mask and partial sums, then their fold
   }
 };
@@ -816,7 +818,16 @@ at::Tensor conv_bias_relu(const at::Tensor& x, const at::Tensor& weight, const a
     return conv_composition({in(x), in(weight), in(bias)}, stride, padding, dilation, groups, pool);
   }
   std::shared_ptr<ConvNode> node;
-  if (torch::autograd::compute_requires_grad(x, weight, bias)) node = make_node<ConvNode>(x, weight, bias);
+  if (torch::autograd::compute_requires_grad(x, weight, bias)) {
+    node = make_node<ConvNode>(x, weight, bias);
+    node->weight = weight;
+    node->bias = bias;
+    node->stride = stride;
+    node->padding = padding;
+    node->dilation = dilation;
+    node->groups = groups;
+    node->pool = pool;
+  }
   at::Tensor xs, ws, bs, z, out, signs;
   {
     PlainDispatch plain;
@@ -848,8 +859,9 @@ at::Tensor conv_bias_relu(const at::Tensor& x, const at::Tensor& weight, const a
     } else {
       out = z;
       if (z.is_cuda()) {
-        if (node) signs = fresh({z.numel() / 8}, at::kByte, z);
-        model_ops::bias_relu_inplace_bf16(z.data_ptr(), bs.data_ptr(), rows, C, stream_of(z), node ? signs.data_ptr() : nullptr);
+        if (node && (x.requires_grad() || !weight.requires_grad() || !node->first_layer_shape(xs, z)))
+          signs = fresh({z.numel() / 8}, at::kByte, z);
+        model_ops::bias_relu_inplace_bf16(z.data_ptr(), bs.data_ptr(), rows, C, stream_of(z), signs.defined() ? signs.data_ptr() : nullptr);
       } else
         model_ops::bias_relu_inplace_bf16_host(z.data_ptr(), bs.data_ptr(), rows, C);
     }
@@ -858,13 +870,6 @@ at::Tensor conv_bias_relu(const at::Tensor& x, const at::Tensor& weight, const a
   if (node) {
     node->x = SavedVariable(xs, false);
     node->w = SavedVariable(ws, false);
-    node->weight = weight;
-    node->bias = bias;
-    node->stride = stride;
-    node->padding = padding;
-    node->dilation = dilation;
-    node->groups = groups;
-    node->pool = pool;
     if (accumulate) node->accumulate_gradients({&weight, &bias});
     torch::autograd::set_history(out, node);
     node->b = SavedVariable(bs, false);

@@ -467,6 +467,24 @@ def test_first_layer_gradients_match_fp32_math(N, H, W, Ci, C, in_place):
     assert ((got - want).abs() <= 4.1e-3 * want.abs() + 1e-5 * want.abs().max()).all()
 
 
+@pytest.mark.parametrize("image_grad,c_in,kept", [(False, 3, False), (True, 3, True), (False, 64, True)])
+def test_a_block_whose_backward_reads_the_activation_keeps_no_signs(image_grad, c_in, kept):
+    from bagua_core_b200.ops.fused_conv import ConvBiasReLU
+
+    torch.manual_seed(c_in)
+    m = ConvBiasReLU(c_in, 64, 3, padding=1).cuda().to(memory_format=torch.channels_last)
+    x = torch.randn(2, c_in, 14, 10, device="cuda").to(memory_format=torch.channels_last).requires_grad_(image_grad)
+    seen = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: seen.append(t) or t, lambda t: t), torch.autocast("cuda", dtype=torch.bfloat16):
+        y = m(x)
+    assert [t.numel() for t in seen if t.dtype == torch.uint8] == ([y.numel() // 8] if kept else [])
+    dy = torch.randn(y.shape, device="cuda").to(torch.bfloat16).to(memory_format=torch.channels_last)
+    # the bias gradient alone takes the general path, with or without them
+    db, = torch.autograd.grad(y, [m.bias], dy)
+    want = torch.where(y > 0, dy, torch.zeros_like(dy)).double().sum((0, 2, 3))
+    assert (db.double() - want).abs().max() <= 1e-5 * want.abs().max()
+
+
 @pytest.mark.parametrize("N,C,H,W", [(1, 8, 2, 2), (2, 64, 6, 10), (1, 2048, 4, 2), (3, 16, 1, 7), (5, 32, 34, 38), (2, 128, 3, 5), (8, 64, 112, 96)])
 @pytest.mark.parametrize("pool", [False, True])
 def test_blocks_keep_the_signs_and_places_that_their_backward_needs(N, C, H, W, pool):
