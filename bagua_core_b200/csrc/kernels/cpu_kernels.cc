@@ -276,8 +276,8 @@ void reduce_chunk_inplace(void* x, DType dt, int64_t chunk, int n_chunks, int ta
   c.is_cuda() ? cuda::reduce_chunk_inplace(x, dt, chunk, n_chunks, target, average, c.stream)
               : cpu::reduce_chunk_inplace(x, dt, chunk, n_chunks, target, average);
 }
-size_t compress_scratch_bytes(int n_chunks, int64_t chunk_size, DType dt) {
-  return cuda::compress_scratch_bytes(n_chunks, chunk_size * (int64_t)dtype_bytes(dt));
+size_t compress_scratch_bytes(int n_chunks, int64_t chunk_size, DType dt, const Ctx& c) {
+  return c.is_cuda() ? cuda::compress_scratch_bytes(n_chunks, chunk_size * (int64_t)dtype_bytes(dt), c.stream) : 0;
 }
 
 void compress_minmax_u8(const void* in, DType dt, int64_t num_real, int64_t chunk, int n_chunks, uint8_t* out,

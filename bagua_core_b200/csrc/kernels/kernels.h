@@ -88,8 +88,8 @@ size_t compressed_buffer_size(int n_chunks, int64_t chunk_size, DType dt);
 
 // Scratch needed by the CUDA path of compress (slots through which the blocks of a chunk agree on its min
 // and max): memory that was zero once and that only this path has written since.  0 for chunks that
-// one block handles alone.
-size_t compress_scratch_bytes(int n_chunks, int64_t chunk_size, DType dt);
+// one block or one cluster handles alone.
+size_t compress_scratch_bytes(int n_chunks, int64_t chunk_size, DType dt, const Ctx& c);
 
 // Quantise `in` (n_chunks*chunk_size allocated elements, of which `num_real` are real
 // data; min/max of a chunk are taken over its real elements only, an all-padding chunk

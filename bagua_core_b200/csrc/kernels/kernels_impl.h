@@ -16,7 +16,8 @@ void async_model_average(float* t, const float* r, const float* cp, float nranks
 void copy_bytes(void* dst, const void* src, size_t bytes, cudaStream_t s);
 void multi_copy(const MultiCopySeg* segs_dev, int nseg, void* flat, size_t total_bytes, bool gather, cudaStream_t s);
 void reduce_chunk_inplace(void* x, DType dt, int64_t chunk, int n_chunks, int target, bool average, cudaStream_t s);
-size_t compress_scratch_bytes(int n_chunks, int64_t chunk_bytes);
+// (weak, like those of kernels.h)
+size_t compress_scratch_bytes(int n_chunks, int64_t chunk_bytes, cudaStream_t s) __attribute__((weak));
 void compress_minmax_u8(const void* in, DType dt, int64_t num_real, int64_t chunk, int n_chunks, uint8_t* out,
                         size_t out_bytes, int target, void* scratch, size_t scratch_bytes, cudaStream_t s);
 void decompress_minmax_u8(const uint8_t* in, size_t in_bytes, int64_t chunk, int n_chunks, void* out, DType dt,

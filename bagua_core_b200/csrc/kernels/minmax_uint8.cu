@@ -26,10 +26,13 @@
 #include <algorithm>
 #include <atomic>
 #include <cfloat>
+#include <map>
+#include <mutex>
 
 #include "kernels_impl.h"
 #include "launch.cuh"
 #include "minmax_device.cuh"
+#include "minmax_split.h"
 
 namespace bagua {
 namespace kernels {
@@ -39,6 +42,7 @@ namespace {
 
 using mmdev::from_f;
 using mmdev::to_f;
+using namespace minmax_split;
 
 // ---- vectors at any alignment --------------------------------------------------------------
 // A vector is VE elements (16 bytes of T) and their VE quantised bytes.  Both sides are aligned in
@@ -133,35 +137,7 @@ __device__ __forceinline__ typename mmdev::QWord<VE>::type load_bytes(const uint
 constexpr int kThreads = 512;
 constexpr int kVecs = 8;                       // vectors a thread keeps between the passes (32 registers)
 constexpr int kTile = kThreads * kVecs;        // vectors of a tile: 64 KiB
-constexpr int kBlocksPerSM = 2;                // 64 registers per thread
-constexpr int64_t kTileBytes = (int64_t)kTile * 16;
-// Smallest slice of a block: more blocks read a chunk faster but wait longer for each other (10 MB of fp32 in
-// 8 chunks: 8.1 us with 16 KiB, 6.9 with 64; unaligned elements, which take more instructions to load, 1 M of
-// fp16 in 3 chunks: 9.4 us with 64 KiB, 7.5 with 32).
-constexpr int64_t kSliceBytes = 64 << 10, kSliceBytesUnaligned = 32 << 10;
-constexpr int64_t kGroupBytes = 32ll << 20;    // two groups and their output are in L2 (126 MB) at a time
-
-// How the chunks of a call are dealt to blocks.  Calls of several groups have two sets of blocks, one of each
-// set on every SM, which take the groups in turn: while one set quantises its group, which is bound by
-// instructions (8 per element), the other reads the next from memory.
-struct Split {
-  int sets;
-  int per_group;  // chunks in flight together in a set
-  int per_chunk;  // blocks of one chunk
-  int grid() const { return sets * per_group * per_chunk; }
-};
-Split split_chunks(int count, int64_t chunk_bytes, bool aligned, int sms) {
-  Split s;
-  const int64_t all = (int64_t)sms * kBlocksPerSM;
-  s.per_group = (int)std::max<int64_t>(1, std::min({kGroupBytes / chunk_bytes, (int64_t)count, all}));
-  s.sets = s.per_group < count && chunk_bytes > kTileBytes ? 2 : 1;
-  if (s.sets == 2) s.per_group = std::min(s.per_group, sms);
-  // a chunk of one tile stays with one block, which then waits for nobody
-  s.per_chunk = chunk_bytes <= kTileBytes
-                    ? 1
-                    : (int)std::max<int64_t>(1, std::min<int64_t>(all / s.sets / s.per_group, chunk_bytes / (aligned ? kSliceBytes : kSliceBytesUnaligned)));
-  return s;
-}
+static_assert(kTileBytes == (int64_t)kTile * 16, "the rules of minmax_split.h assume the kernel's tiles");
 
 // How the blocks of a chunk agree: every block leaves {min, tag} and {max, tag} in a slot of its own, two
 // 8-byte words each of which says by its tag that it belongs to this launch, and thread t of every block
@@ -169,9 +145,7 @@ Split split_chunks(int count, int64_t chunk_bytes, bool aligned, int sms) {
 // maxima by atomics with an arrival counter took 4 us more with 296 blocks.
 // With 148 blocks that is 22 thousand waiting threads on 19 lines of L2 (4.6 us): above kDirect blocks the first
 // block collects, and the others wait for its answer (2.3 us; 16 blocks among themselves: 1.5 us).
-constexpr int kSlotBytes = 16;
 constexpr int kDirect = 24;
-inline size_t slot_bytes(int count, int per_chunk) { return (size_t)count * (per_chunk + 1) * kSlotBytes; }
 
 __device__ __forceinline__ void leave_minmax(unsigned long long* slot, float mn, float mx, uint32_t tag) {
   const unsigned long long hi = (unsigned long long)tag << 32;
@@ -217,23 +191,7 @@ __device__ __forceinline__ bool agree(unsigned long long* mine, int part, int pe
   return all;
 }
 
-// Smaller chunks belong to a cluster instead, whose blocks agree through each other's shared memory: nothing of the launch has
-// to be resident as a whole, it may start while its predecessor ends, and it needs no slots.  (Cooperative launches follow each
-// other in steps of 2 us.)  Up to 8 chunks have up to 16 blocks each; more chunks have 8, as clusters of 16 do not find room on all
-// SMs at once.  The last slice sizes are those beyond which the launch of all SMs is as fast or faster.  us, cooperative / cluster:
-// fp32, one chunk of 128 KB 6.2/4.3, 1 MB 6.2/4.4, 1.6 MB 8.2/6.1, 2.1 MB 8.2/6.8, 3.2 MB 8.2/9.0; 8 chunks of 0.4 MB 8.2/5.2, of 1.3 MB
-// 8.2/7.5, of 2 MB 10.3/9.0; 16 chunks of 0.4 MB 8.2/8.5 by 16 and 5.8 by 8 blocks, of 1.3 MB 10.3/10.7 by 8; unaligned fp16,
-// 3 chunks of 0.7 MB 9.4/7.8, of 1.4 MB 9.5/10.2.
-constexpr int64_t kClusterSlice = 32 << 10;  // aimed at
-// Blocks of the cluster that handles a chunk of this size; 1: a block alone, 0: no cluster.
-int cluster_blocks(int64_t chunk_bytes, int count, bool aligned) {
-  const int most = count <= 8 ? 16 : 8;
-  if (chunk_bytes <= kTileBytes) return 1;
-  if (chunk_bytes > most * (!aligned ? kTileBytes : count <= 8 ? 2 * kTileBytes : kTileBytes + kTileBytes / 2)) return 0;
-  int n = 2;
-  while (n < most && n * kClusterSlice < chunk_bytes) n *= 2;
-  return n;
-}
+// Smaller chunks belong to a cluster instead (cluster_blocks()).
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // The blocks of a cluster, each with its (mn, mx) in every thread, exchange them: afterwards the chunk's are those over the block's
@@ -632,6 +590,48 @@ uint32_t next_tag() {
   return t;
 }
 
+// The largest cluster that the stream's context can run: 16 blocks on the whole GPU, 8 in a green context of any size, fewer under other
+// limits.  Asked once per stream, by an id that no other stream of the process gets.
+int largest_cluster(cudaStream_t s) {
+  static std::mutex mu;
+  static std::map<unsigned long long, int> known;
+  static thread_local unsigned long long last_id = 0;
+  static thread_local int last = -1;
+  unsigned long long id = 0;
+  const bool has_id = cudaStreamGetId(s, &id) == cudaSuccess;
+  if (has_id && last >= 0 && id == last_id) return last;
+  if (!has_id) cudaGetLastError();
+  std::lock_guard<std::mutex> g(mu);
+  int largest = -1;
+  if (auto it = known.find(id); has_id && it != known.end()) largest = it->second;
+  if (largest < 0) {
+    auto* kernel = compress_kernel<float, true, true>;
+    BAGUA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    for (largest = 16; largest > 1; largest /= 2) {
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = (unsigned)largest;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)largest);
+      cfg.blockDim = dim3(kThreads);
+      cfg.stream = s;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      int fit = 0;
+      if (cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) == cudaSuccess && fit > 0) break;
+      cudaGetLastError();
+    }
+    if (known.size() >= 256) known.clear();
+    if (has_id) known[id] = largest;
+  }
+  if (has_id) {
+    last_id = id;
+    last = largest;
+  }
+  return largest;
+}
+
 template <typename T>
 void compress_t(const void* in, int64_t num_real, int64_t chunk, int n_chunks, uint8_t* out, size_t out_bytes,
                 int target, void* scratch, size_t scratch_bytes, cudaStream_t s) {
@@ -639,7 +639,8 @@ void compress_t(const void* in, int64_t num_real, int64_t chunk, int n_chunks, u
   const int first = target >= 0 ? target : 0;
   const int count = target >= 0 ? 1 : n_chunks;
   const bool aligned = ((uintptr_t)in % 16 == 0) && ((uintptr_t)out % 16 == 0) && (chunk % 16 == 0) && (off % 16 == 0);
-  const int blocks = cluster_blocks(chunk * (int64_t)sizeof(T), count, aligned);
+  const int largest = chunk * (int64_t)sizeof(T) > kTileBytes ? largest_cluster(s) : 0;
+  const int blocks = cluster_blocks(chunk * (int64_t)sizeof(T), count, aligned, largest);
   if (blocks == 1) {
     launch_overlapped(aligned ? compress_kernel<T, true, false> : compress_kernel<T, false, false>, dim3(count), dim3(kThreads), s,
                       (const T*)in, num_real, chunk, first, count, 1, count, 1, out, off, (unsigned long long*)nullptr, 0u);
@@ -783,12 +784,8 @@ void decompress_t(const uint8_t* in, size_t in_bytes, int64_t chunk, int n_chunk
 
 }  // namespace
 
-size_t compress_scratch_bytes(int n_chunks, int64_t bytes) {
-  // a call for one chunk of the buffer may give that chunk more blocks than a call for all of them
-  size_t most = 0;
-  for (int count : {n_chunks, 1})
-    if (!cluster_blocks(bytes, count, false)) most = std::max(most, slot_bytes(count, split_chunks(count, bytes, false, sm_count()).per_chunk));
-  return most;
+size_t compress_scratch_bytes(int n_chunks, int64_t bytes, cudaStream_t s) {
+  return bytes <= kTileBytes ? 0 : scratch_bytes(n_chunks, bytes, sm_count(), largest_cluster(s));
 }
 
 void compress_minmax_u8(const void* in, DType dt, int64_t num_real, int64_t chunk, int n_chunks, uint8_t* out,

@@ -78,7 +78,7 @@ std::shared_ptr<RawTensor> compress(const RawTensor& t, const std::string& metho
   std::shared_ptr<PoolBlock> scratch;
   size_t scratch_bytes = 0;
   if (t.device_id() >= 0) {
-    scratch_bytes = kernels::compress_scratch_bytes(n_chunks, chunk, t.dtype());
+    scratch_bytes = kernels::compress_scratch_bytes(n_chunks, chunk, t.dtype(), t.ctx(stream));
     if (scratch_bytes) scratch = MemoryPool::for_device(t.device_id()).pull_cleared(scratch_bytes, stream);
   }
   kernels::compress_minmax_u8(t.data_ptr(), t.dtype(), t.num_elements(), chunk, n_chunks, (uint8_t*)out->data_ptr(),

@@ -1,6 +1,10 @@
 """Properties of the MinMaxUInt8 compressor (host implementation = the oracle the GPU
 kernels are compared against).  Reference numerics:
 bagua-core-internal/kernels/bagua_kernels.cu:10,411-432,465-467."""
+import os
+import shutil
+import subprocess
+
 import numpy as np
 import pytest
 import torch
@@ -106,3 +110,15 @@ def test_rejects_bad_arguments():
         bc.BaguaTensorPy(x, "x").compress("TopK", 1, -1)
     with pytest.raises(RuntimeError):
         bc.BaguaTensorPy(torch.zeros(4, dtype=torch.int64), "i").compress("MinMaxUInt8", 1, -1)
+
+
+def test_a_compress_call_gets_no_larger_cluster_than_its_context_can_run(tmp_path):
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("needs g++")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    exe = str(tmp_path / "minmax_split")
+    subprocess.run([gxx, "-std=c++17", "-O1", "-I", os.path.join(root, "bagua_core_b200", "csrc"),
+                    os.path.join(root, "tests", "cpp", "minmax_split.cc"), "-o", exe], check=True)
+    run = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert run.returncode == 0 and " 0 failures" in run.stdout, run.stdout + run.stderr
