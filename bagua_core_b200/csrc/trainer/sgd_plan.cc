@@ -1,5 +1,6 @@
 #include "sgd_plan.h"
 
+#include <c10/cuda/CUDAGuard.h>
 #include <cuda_runtime.h>
 
 #include <cstring>
@@ -69,10 +70,12 @@ void SgdPlan::zero_grad(uint64_t stream) {
     for (; k < segs_.size() && grad_buffer_[k] == buffer && segs_[k].g == from + n; ++k) n += segs_[k].n;
     if (n) fill.push_back({from, n});
   }
-  if (device_ >= 0)
+  if (device_ >= 0) {
+    const c10::cuda::CUDAGuard on((c10::DeviceIndex)device_);  // memory can be set from any device, a kernel not
     kernels::cuda::fill_zero(fill.data(), (int)fill.size(), (cudaStream_t)stream);
-  else
+  } else {
     for (const auto& f : fill) std::memset(f.p, 0, (size_t)f.n * sizeof(float));
+  }
 }
 
 }  // namespace trainer

@@ -160,3 +160,19 @@ def test_zero_grad_clears_every_bucket_and_nothing_else(sizes):
     opt.step()
     for i, p in enumerate(m.parameters()):
         assert (p == i).all() and not p.grad.any()
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs a second GPU")
+def test_zero_grad_works_on_the_device_of_its_buckets():
+    import bagua_core_b200 as bb
+
+    plan, grads = bb._C.SgdPlan(), []
+    for _ in range(3):
+        p, g, m = (torch.ones(5000, device="cuda:1") for _ in range(3))
+        plan.add(p, g, m, None, 0)
+        grads.append(g)
+    torch.cuda.synchronize(1)
+    with torch.cuda.device(0):
+        plan.zero_grad(torch.cuda.current_stream(1).cuda_stream)
+    torch.cuda.synchronize(1)
+    assert not any(g.any() for g in grads)
