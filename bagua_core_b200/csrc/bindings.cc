@@ -686,6 +686,47 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       },
       py::arg("tensors"), py::arg("flat"), py::arg("gather"), py::arg("stream"),
       "Flatten (gather) or unflatten a list of tensors into / out of `flat` (packed back to back) with one kernel.");
+  m.def(
+      "k_multi_copy_joined",
+      [](std::vector<std::pair<std::vector<at::Tensor>, at::Tensor>> buckets, bool gather, uint64_t stream) {
+        std::vector<kernels::MultiCopySeg> segs;
+        std::vector<kernels::MultiCopyItem> items;
+        std::vector<size_t> first;
+        for (auto& [tensors, flat] : buckets) {
+          unsigned long long off = 0;
+          first.push_back(segs.size());
+          for (auto& t : tensors) {
+            BAGUA_CHECK(t.is_cuda() && t.is_contiguous() && t.device() == flat.device(), Tensor,
+                        "multi_copy: tensors must be contiguous and on the flat buffer's GPU");
+            if (t.nbytes()) segs.push_back(kernels::MultiCopySeg{t.data_ptr(), off, (unsigned long long)t.nbytes()});
+            off += t.nbytes();
+          }
+          BAGUA_CHECK(flat.is_contiguous() && (unsigned long long)flat.nbytes() >= off, Tensor, "multi_copy: a flat buffer is too small");
+          items.push_back({nullptr, (int)(segs.size() - first.back()), flat.data_ptr(), (size_t)off});
+        }
+        if (segs.empty()) return;
+        at::Tensor table = at::empty({(int64_t)(segs.size() * sizeof(kernels::MultiCopySeg))}, buckets[0].second.options().dtype(at::kByte));
+        BAGUA_CUDA_CHECK(cudaMemcpyAsync(table.data_ptr(), segs.data(), segs.size() * sizeof(kernels::MultiCopySeg),
+                                         cudaMemcpyHostToDevice, (cudaStream_t)stream));
+        for (size_t k = 0; k < items.size(); ++k) items[k].segs = (const kernels::MultiCopySeg*)table.data_ptr() + first[k];
+        kernels::cuda::multi_copy_joined(items.data(), (int)items.size(), gather, (cudaStream_t)stream);
+        BAGUA_CUDA_CHECK(cudaStreamSynchronize((cudaStream_t)stream));  // `table` and `segs` die with this call
+      },
+      py::arg("buckets"), py::arg("gather"), py::arg("stream"), "k_multi_copy for several (tensors, flat) in one launch.");
+  m.def(
+      "k_quantise_twice",
+      [](std::vector<at::Tensor> tensors, uint64_t stream) {
+        std::vector<std::unique_ptr<PoolRawTensor>> raws;
+        std::vector<RawTensor*> ts;
+        for (auto& t : tensors) {
+          BAGUA_CHECK(t.is_cuda() && t.is_contiguous(), Tensor, "quantise_twice works on contiguous CUDA tensors");
+          raws.push_back(std::make_unique<PoolRawTensor>(t.data_ptr(), nullptr, t.numel(), t.numel(), dtype_from_torch(t.scalar_type()),
+                                                         (int)t.device().index()));
+          ts.push_back(raws.back().get());
+        }
+        tensor_ops::quantise_twice(ts, "MinMaxUInt8", stream);
+      },
+      py::arg("tensors"), py::arg("stream"), "Every tensor compressed and decompressed twice as one chunk, in place, in one launch for 16 of them.");
   m.def("k_divide_inplace", [](at::Tensor x, float d, uint64_t stream) {
     kernels::divide_inplace(x.data_ptr(), dtype_from_torch(x.scalar_type()), x.numel(), d, ctx_of(x, stream));
   });

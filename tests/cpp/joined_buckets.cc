@@ -5,6 +5,7 @@
 //   failing   a bucket that cannot be prepared fails alone
 //   watchdog  a launch that does not return is reported under the names of all its buckets
 //   locks     backends that hold the same buckets in opposite orders do not wait for each other
+//   most      a launch has 16 buckets at most, none of them twice
 //   staging   buckets that are staged together take one block from the pool, whichever of them meet
 //   overlap   buckets that share memory, or whose tensors have moved to where they do, get what they get one after the other
 #include <cuda_runtime.h>
@@ -349,8 +350,31 @@ void staging() {
     }
 }
 
+void most() {
+  std::vector<float> x(21 * 16), y(16);
+  auto op = make_centralized_low_precision_op(one_rank(1), true, "MinMaxUInt8");
+  {
+    CommBackend backend(100, 0);
+    std::vector<BucketPtr> buckets;
+    for (int k = 0; k < 21; ++k) buckets.push_back(make_bucket("b" + std::to_string(k), {{x.data() + 16 * k, 16}}, op));
+    backend.register_ordered_buckets(buckets);
+    burst(backend, buckets);
+    EXPECT(backend.wait_pending_comm_ops() == 21, "21 buckets");
+    EXPECT(quantise_launches == (std::vector<int>{1, 16, 4}), "not 16 at a time");
+    for (float v : x) EXPECT(v == 1, "%g", v);
+  }
+  CommBackend backend(100, 0);
+  const BucketPtr one = make_bucket("one", {{y.data(), 16}}, op);
+  backend.register_ordered_buckets({one});
+  quantise_launches.clear();
+  burst(backend, {one, one, one});
+  EXPECT(backend.wait_pending_comm_ops() == 3, "three times");
+  EXPECT(quantise_launches == (std::vector<int>{1, 1, 1}), "joined with itself");
+  for (float v : y) EXPECT(v == 7, "%g", v);
+}
+
 const std::map<std::string, void (*)()> kCases = {
-    {"failing", failing}, {"locks", locks}, {"overlap", overlap}, {"staging", staging}, {"watchdog", watchdog}};
+    {"failing", failing}, {"locks", locks}, {"most", most}, {"overlap", overlap}, {"staging", staging}, {"watchdog", watchdog}};
 }  // namespace
 
 int main(int argc, char** argv) {

@@ -53,3 +53,7 @@ def test_a_bucket_that_cannot_be_prepared_fails_alone(program):
 
 def test_the_watchdog_names_all_buckets_of_a_launch(program):
     _run(program, "watchdog")
+
+
+def test_a_launch_has_sixteen_buckets_at_most_and_none_twice(program):
+    _run(program, "most")

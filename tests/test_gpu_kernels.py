@@ -527,3 +527,91 @@ def test_buckets_that_are_handed_over_together_get_what_they_get_alone(sizes, dt
     backend.close()
     for ts, w in zip(parts, want):
         assert torch.equal(torch.cat(ts), w)
+
+
+def _twice(t):
+    import bagua_core as bc
+
+    t = t.clone()
+    for _ in range(2 if t.numel() else 0):
+        c = bc.BaguaTensorPy(t, "w").compress("MinMaxUInt8", 1, -1)
+        bc.BaguaTensorPy(t, "w").decompress_from("MinMaxUInt8", 1, c)
+    return t
+
+
+# nothing, one value, one block, blocks by size, more blocks wanted than there are (their shares), several launches
+@pytest.mark.parametrize("sizes", [[0], [1], [16385], [3, 0], [2621440, 17], [16384, 16385, 1, 200003], [1 << 20] * 5,
+                                   [4 << 20, 1, 9 << 20, 40000, 3 << 20], [(1 << 18) + k for k in range(16)], [1 << 20, 5] * 8, [70001, 0, 3] * 11])
+@pytest.mark.parametrize("dt", DTYPES)
+@pytest.mark.parametrize("offset", [0, 1])
+def test_buffers_that_are_quantised_in_one_launch_get_what_each_gets_alone(sizes, dt, offset):
+    import bagua_core_b200 as bb
+
+    bases = [_rand(n + offset + 1, dt, i) * (i + 1) for i, n in enumerate(sizes)]
+    parts = [b[offset:offset + n] for b, n in zip(bases, sizes)]
+    want = [_twice(p) for p in parts]
+    edges = [(b[:offset].clone(), b[offset + n:].clone()) for b, n in zip(bases, sizes)]
+    torch.cuda.synchronize()
+    bb._C.k_quantise_twice(parts, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    for b, p, w, (front, back) in zip(bases, parts, want, edges):
+        assert torch.equal(p, w) and torch.equal(b[:offset], front) and torch.equal(b[offset + p.numel():], back)
+
+
+@pytest.mark.parametrize("count", [1, 2, 4, 5, 16])
+@pytest.mark.parametrize("seed", range(3))
+def test_buckets_that_are_copied_in_one_launch(count, seed):
+    """Some without tensors, tiles that end with a bucket, tensors at any address."""
+    import bagua_core_b200 as bb
+
+    g = torch.Generator().manual_seed(100 * count + seed)
+    pool = torch.randint(0, 256, (8 << 20,), dtype=torch.uint8, generator=g).cuda()
+    at, buckets = seed, []
+    for k in range(count):
+        sizes = [] if k % 5 == 3 else torch.randint(1, 60000, (int(torch.randint(1, 9, (1,), generator=g)),), generator=g).tolist()
+        if k % 4 == 1:
+            sizes.append(16384 * 4 - sum(sizes) % 16384)
+        ts = []
+        for n in sizes:
+            ts.append(pool[at:at + n])
+            at += n + int(torch.randint(0, 19, (1,), generator=g))
+        buckets.append((ts, torch.zeros(sum(sizes) + 33, dtype=torch.uint8, device="cuda")))
+    assert at <= pool.numel()
+    st = torch.cuda.current_stream().cuda_stream
+    bb._C.k_multi_copy_joined(buckets, True, st)
+    for ts, flat in buckets:
+        n = sum(t.numel() for t in ts)
+        assert torch.equal(flat[:n], torch.cat(ts) if ts else flat[:0]) and not flat[n:].any()
+    before = pool.clone()
+    for ts, _ in buckets:
+        for t in ts:
+            t.zero_()
+    bb._C.k_multi_copy_joined(buckets, False, st)
+    assert torch.equal(pool, before)
+
+
+def test_compression_in_a_context_of_few_sms():
+    """Green contexts run no clusters of 16 blocks."""
+    green = pytest.importorskip("torch.cuda.green_contexts")
+    import bagua_core as bc
+
+    xs = [_rand(n, torch.float32, n) for n in (1000, 100000, 262144, 524288)]
+
+    def round_trips():
+        outs = []
+        for x in xs:
+            out = torch.empty_like(x)
+            bc.BaguaTensorPy(out, "o").decompress_from("MinMaxUInt8", 1, bc.BaguaTensorPy(x, "x").compress("MinMaxUInt8", 1, -1))
+            outs.append(out)
+        torch.cuda.synchronize()
+        return outs
+
+    want = round_trips()
+    context = green.GreenContext.create(16, 0)
+    context.set_context()
+    try:
+        got = round_trips()
+    finally:
+        context.pop_context()
+    for a, b in zip(want, got):
+        assert torch.equal(a, b)
