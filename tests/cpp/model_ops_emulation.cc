@@ -90,6 +90,78 @@ int check_bias_relu(int64_t rows, int C, int blocks, std::mt19937& rng) {
   return bad;
 }
 
+// What training runs on a GPU: the forward leaves a bit per value and the backward reads those instead of the activation.
+int check_bias_relu_signs(int64_t rows, int C, int blocks, std::mt19937& rng) {
+  const int cgroups = C / 8;
+  const int64_t nvec = rows * cgroups;
+  Buf z((size_t)nvec), bias((size_t)cgroups), want;
+  fill(z, rng, false);
+  fill(bias, rng, false);
+  raw(z)[0] = 0x8000;  // -0 + -0 is not positive
+  raw(bias)[0] = 0x8000;
+  want = z;
+  bias_relu_inplace_bf16_host(raw(want), raw(bias), rows, C);
+  std::vector<uint8_t> signs((size_t)nvec, 0xa5);
+  launch(blocks, kThreads, [&] {
+    bias_relu_body<true>(reinterpret_cast<uint4*>(z.data()), reinterpret_cast<const __nv_bfloat16*>(raw(bias)), nvec, cgroups, signs.data());
+  });
+  int bad = 0;
+  for (int64_t i = 0; i < nvec * 8; ++i) {
+    // (zeros of either sign are equal)
+    bad += raw(z)[i] != raw(want)[i] && ((raw(z)[i] | raw(want)[i]) & 0x7fffu) != 0;
+    bad += (signs[(size_t)(i / 8)] >> (i % 8) & 1) != ((raw(want)[i] & 0x7fffu) != 0 && raw(want)[i] < 0x8000u);
+  }
+  Buf dy((size_t)nvec), dz((size_t)nvec), dz_want((size_t)nvec);
+  fill(dy, rng, false);
+  std::vector<float> db_want((size_t)C), db((size_t)C, -1.f), partial((size_t)blocks * (size_t)C, -1.f);
+  bias_relu_backward_bf16_host(raw(dy), raw(want), raw(dz_want), db_want.data(), rows, C);
+  std::vector<std::vector<float>> sacc((size_t)blocks, std::vector<float>((size_t)kThreads * 8));
+  launch(blocks, kThreads, [&] {
+    bias_relu_backward_body<true>(reinterpret_cast<const uint4*>(dy.data()), nullptr, reinterpret_cast<uint4*>(dz.data()), partial.data(), rows,
+                                  cgroups, sacc[hostemu::t_block_idx.x].data(), signs.data());
+  });
+  launch((C + 127) / 128, 128, [&] { bias_grad_finish_body(partial.data(), db.data(), blocks, C); });
+  bad += std::memcmp(dz.data(), dz_want.data(), (size_t)nvec * 16) != 0;
+  for (int c = 0; c < C; ++c)
+    if (std::fabs(db[(size_t)c] - db_want[(size_t)c]) > 1e-3f * (1.f + std::fabs(db_want[(size_t)c]))) ++bad;
+  return bad;
+}
+
+int check_bias_relu_pool_codes(int64_t N, int64_t H, int64_t W, int C, int blocks, std::mt19937& rng) {
+  const int cgroups = C / 8;
+  const int64_t nin = N * H * W * cgroups, nout = N * (H / 2) * (W / 2) * cgroups;
+  Buf z((size_t)nin), p((size_t)nout), bias((size_t)cgroups), y_want, p_want((size_t)nout);
+  fill(z, rng, false);
+  fill(bias, rng, false);
+  y_want = z;
+  bias_relu_pool_bf16_host(raw(y_want), raw(p_want), raw(bias), N, H, W, C);
+  const Buf z_before = z;
+  std::vector<uint32_t> codes((size_t)nout, 0xa5a5a5a5u);
+  launch(blocks, kThreads, [&] {
+    bias_relu_pool_only_body<true>(reinterpret_cast<const uint4*>(z.data()), reinterpret_cast<uint4*>(p.data()),
+                                   reinterpret_cast<const __nv_bfloat16*>(raw(bias)), N * (H / 2) * (W / 2), W / 2, W, cgroups, codes.data());
+  });
+  int bad = std::memcmp(z.data(), z_before.data(), (size_t)nin * 16) != 0;
+  for (int64_t i = 0; i < nout * 8; ++i) bad += raw(p)[i] != raw(p_want)[i] && ((raw(p)[i] | raw(p_want)[i]) & 0x7fffu) != 0;
+
+  Buf dp((size_t)nout), dz((size_t)nin), dz_want((size_t)nin);
+  fill(dp, rng, false);
+  for (auto& v : dz)
+    for (auto& h : v.h) h = 0x7fc0;  // every element must be overwritten
+  std::vector<float> db_want((size_t)C), db((size_t)C, -1.f), partial((size_t)blocks * (size_t)C, -1.f);
+  bias_relu_pool_backward_bf16_host(raw(dp), raw(y_want), raw(dz_want), db_want.data(), N, H, W, C);
+  std::vector<std::vector<float>> sacc((size_t)blocks, std::vector<float>((size_t)kThreads * 8));
+  launch(blocks, kThreads, [&] {
+    bias_relu_pool_backward_codes_body(reinterpret_cast<const uint4*>(dp.data()), codes.data(), reinterpret_cast<uint4*>(dz.data()),
+                                       partial.data(), N * (H / 2) * (W / 2), W / 2, W, cgroups, sacc[hostemu::t_block_idx.x].data());
+  });
+  launch((C + 127) / 128, 128, [&] { bias_grad_finish_body(partial.data(), db.data(), blocks, C); });
+  bad += std::memcmp(dz.data(), dz_want.data(), (size_t)nin * 16) != 0;
+  for (int c = 0; c < C; ++c)
+    if (std::fabs(db[(size_t)c] - db_want[(size_t)c]) > 1e-3f * (1.f + std::fabs(db_want[(size_t)c]))) ++bad;
+  return bad;
+}
+
 int check_maxpool(int64_t N, int64_t H, int64_t W, int C, int blocks, std::mt19937& rng) {
   const int cgroups = C / 8;
   const int64_t nin = N * H * W * cgroups, nout = N * (H / 2) * (W / 2) * cgroups;
@@ -190,6 +262,17 @@ int main() {
     failures += bad != 0;
     ++cases;
   }
+  for (const auto& c : br)
+    if (const int bad = check_bias_relu_signs(c.rows, c.C, c.blocks, rng)) {
+      std::fprintf(stderr, "bias+ReLU with signs [%lld, %d] on %d blocks: %d mismatches\n", (long long)c.rows, c.C, c.blocks, bad);
+      ++failures;
+    }
+  for (const auto& c : bp)
+    if (const int bad = check_bias_relu_pool_codes(c.N, c.H, c.W, c.C, c.blocks, rng)) {
+      std::fprintf(stderr, "bias+ReLU+pool with codes [%lld, %lld, %lld, %d] on %d blocks: %d mismatches\n", (long long)c.N, (long long)c.H,
+                   (long long)c.W, c.C, c.blocks, bad);
+      ++failures;
+    }
   // index arithmetic on both sides of the 32-bit limit, against plain 64-bit division
   {
     const int64_t big = (int64_t)1 << 32;
