@@ -305,7 +305,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
     if (s_failed)  // no copy may be in flight when the block leaves
-      for (int k = max(0, issued - kStages); k < issued; ++k) barrier_wait(shared_address(&s_full[k % kStages]), (uint32_t)(k / kStages) & 1);
+      for (int k = max(0, issued - kStages); k < issued; ++k)
+        barrier_wait(shared_address(&s_full[k % kStages]), (uint32_t)(k / kStages) & 1);
   } else if (warp == 1) {
     // products: the whole warp walks along, so that the descriptions stay in uniform registers, and one lane issues
     int stage = 0;
@@ -320,8 +321,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t a = stages + stage * p.stage_bytes(), b = a + p.a_planes * p.a_plane;
-      const uint32_t a0 = operand_low(a + p.product[0].a_start, p.product[0].a_step), b0 = operand_low(b + p.product[0].b_start, p.product[0].b_step);
-      const uint32_t a1 = operand_low(a + p.product[1].a_start, p.product[1].a_step), b1 = operand_low(b + p.product[1].b_start, p.product[1].b_step);
+      const uint32_t a0 = operand_low(a + p.product[0].a_start, p.product[0].a_step);
+      const uint32_t b0 = operand_low(b + p.product[0].b_start, p.product[0].b_step);
+      const uint32_t a1 = operand_low(a + p.product[1].a_start, p.product[1].a_step);
+      const uint32_t b1 = operand_low(b + p.product[1].b_start, p.product[1].b_step);
       if (issues) {
 #pragma unroll 2
         for (int k = 0; k < p.steps; ++k) {
@@ -374,7 +377,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 // A thread of the block's first dimension takes four input channels of one (output channel, tap); the second dimension takes
 // the splits in turn, and its sums are added in order.
 __global__ void __launch_bounds__(kFoldThreads)
-    conv_wgrad_fold_kernel(const float4* __restrict__ partial, const Plan p, int Co, int Ci, __nv_bfloat16* __restrict__ dw, int64_t stride_co, int64_t stride_r, int64_t stride_s, int64_t stride_ci) {
+    conv_wgrad_fold_kernel(const float4* __restrict__ partial, const Plan p, int Co, int Ci, __nv_bfloat16* __restrict__ dw,
+                           int64_t stride_co, int64_t stride_r, int64_t stride_s, int64_t stride_ci) {
   __shared__ float4 s_sum[kFoldThreads];
   const int per_tap = Ci / 4;
   const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);  // [co][tap][ci / 4]
@@ -541,8 +545,8 @@ void conv_wgrad(const void* dz, const void* x, void* dw, const int64_t (&strides
   while (sharers < kFoldThreads / kFoldX && sharers * 4 <= p.splits && quads * sharers < (int64_t)sm_count() * 1024) sharers *= 2;
   const int across = kFoldThreads / sharers;
   const dim3 grid((unsigned)((quads + across - 1) / across)), block(across, sharers);
-  launch_overlapped(conv_wgrad_fold_kernel, grid, block, stream, (const float4*)scratch, p, (int)Co, (int)Ci, (__nv_bfloat16*)dw, strides[0],
-                    strides[1], strides[2], strides[3]);
+  launch_overlapped(conv_wgrad_fold_kernel, grid, block, stream, (const float4*)scratch, p, (int)Co, (int)Ci, (__nv_bfloat16*)dw,
+                    strides[0], strides[1], strides[2], strides[3]);
 }
 
 }  // namespace model_ops

@@ -20,7 +20,6 @@ namespace cuda {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kSMs = 148;
 
 template <typename T>
 struct VecTraits;
@@ -191,27 +190,25 @@ struct CastTable {
 __global__ void __launch_bounds__(kThreads) cast_bf16_kernel(const __grid_constant__ CastTable table) {
   wait_for_predecessor();
   int k = 0;
-  for (int64_t tile = blockIdx.x; tile < table.first_tile[table.n]; tile += gridDim.x) {
-    while (tile >= table.first_tile[k + 1]) ++k;
-    const CastSegment& a = table.seg[k];
-    const int64_t base = (tile - table.first_tile[k]) * kCastTile;
-    auto* dst = reinterpret_cast<__nv_bfloat16*>(a.dst);
-    const bool vec = ((reinterpret_cast<uintptr_t>(a.src) & 15u) | (reinterpret_cast<uintptr_t>(a.dst) & 7u)) == 0;
-    if (vec && base + kCastTile <= a.n) {
-      float4 v[kCastVecs];
+  while ((int64_t)blockIdx.x >= table.first_tile[k + 1]) ++k;
+  const CastSegment& a = table.seg[k];
+  const int64_t base = ((int64_t)blockIdx.x - table.first_tile[k]) * kCastTile;
+  auto* dst = reinterpret_cast<__nv_bfloat16*>(a.dst);
+  const bool vec = ((reinterpret_cast<uintptr_t>(a.src) & 15u) | (reinterpret_cast<uintptr_t>(a.dst) & 7u)) == 0;
+  if (vec && base + kCastTile <= a.n) {
+    float4 v[kCastVecs];
 #pragma unroll
-      for (int u = 0; u < kCastVecs; ++u) v[u] = reinterpret_cast<const float4*>(a.src + base)[u * kThreads + threadIdx.x];
+    for (int u = 0; u < kCastVecs; ++u) v[u] = reinterpret_cast<const float4*>(a.src + base)[u * kThreads + threadIdx.x];
 #pragma unroll
-      for (int u = 0; u < kCastVecs; ++u) {
-        uint2 h;
-        *reinterpret_cast<__nv_bfloat162*>(&h.x) = __floats2bfloat162_rn(v[u].x, v[u].y);
-        *reinterpret_cast<__nv_bfloat162*>(&h.y) = __floats2bfloat162_rn(v[u].z, v[u].w);
-        reinterpret_cast<uint2*>(dst + base)[u * kThreads + threadIdx.x] = h;
-      }
-    } else {
-      const int64_t end = base + kCastTile < a.n ? base + kCastTile : a.n;
-      for (int64_t i = base + threadIdx.x; i < end; i += kThreads) dst[i] = __float2bfloat16_rn(a.src[i]);
+    for (int u = 0; u < kCastVecs; ++u) {
+      uint2 h;
+      *reinterpret_cast<__nv_bfloat162*>(&h.x) = __floats2bfloat162_rn(v[u].x, v[u].y);
+      *reinterpret_cast<__nv_bfloat162*>(&h.y) = __floats2bfloat162_rn(v[u].z, v[u].w);
+      reinterpret_cast<uint2*>(dst + base)[u * kThreads + threadIdx.x] = h;
     }
+  } else {
+    const int64_t end = base + kCastTile < a.n ? base + kCastTile : a.n;
+    for (int64_t i = base + threadIdx.x; i < end; i += kThreads) dst[i] = __float2bfloat16_rn(a.src[i]);
   }
 }
 
@@ -275,10 +272,10 @@ __device__ __forceinline__ void sgd_update(const SgdSegment& a, float& pv, float
 
 // SGD steps of several flat buffers in one launch, each with its own hyperparameters: a stream of 20 bytes per
 // parameter (22 with the bf16 copy), bound by memory.  One launch per buffer left the chip to drain and fill again
-// between buffers of a few MB (10 buckets of 10 MB with bf16 copies: 108 us, now 97; 86 at the copy bandwidth).
+// between buffers of a few MB (10 buckets of 10 MB with bf16 copies: 108 us, 97 in one launch).
 // Buffers are cut into tiles of kSgdTile elements, a block each; the table travels with the launch.  (Blocks that stay and take the tiles
-// in turn are slower, see grid_for(): 138 M elements 485 us, 397 with a block per tile, 403 with tiles of two vectors per thread; 25.6 M with bf16
-// copies 102.6, 84.7, 88.2.)
+// in turn are slower, see grid_for(): 138 M elements 485 us, 397 with a block per tile, 403 with tiles of two vectors per thread; those 10
+// buckets of 25.6 M 102.6, 84.7, 88.2; 86 at the rate of a copy.)
 constexpr int kSgdVecs = 1;
 constexpr int kSgdTile = kThreads * 4 * kSgdVecs;
 constexpr int kSgdSegments = 40;
@@ -291,45 +288,43 @@ struct SgdTable {
 __global__ void __launch_bounds__(kThreads) sgd_kernel(const __grid_constant__ SgdTable table) {
   wait_for_predecessor();
   int k = 0;
-  for (int64_t tile = blockIdx.x; tile < table.first_tile[table.n]; tile += gridDim.x) {
-    while (tile >= table.first_tile[k + 1]) ++k;
-    const SgdSegment& a = table.seg[k];
-    const int64_t base = (tile - table.first_tile[k]) * kSgdTile;
-    const bool has_m = a.momentum != 0.f, read_m = has_m && !a.first;
-    if (a.vec && base + kSgdTile <= a.n) {
-      float4 pv[kSgdVecs], gv[kSgdVecs], bv[kSgdVecs];
+  while ((int64_t)blockIdx.x >= table.first_tile[k + 1]) ++k;
+  const SgdSegment& a = table.seg[k];
+  const int64_t base = ((int64_t)blockIdx.x - table.first_tile[k]) * kSgdTile;
+  const bool has_m = a.momentum != 0.f, read_m = has_m && !a.first;
+  if (a.vec && base + kSgdTile <= a.n) {
+    float4 pv[kSgdVecs], gv[kSgdVecs], bv[kSgdVecs];
 #pragma unroll
-      for (int u = 0; u < kSgdVecs; ++u) {
-        const int64_t i = base / 4 + u * kThreads + threadIdx.x;
-        pv[u] = reinterpret_cast<const float4*>(a.p)[i];
-        gv[u] = reinterpret_cast<const float4*>(a.g)[i];
-        bv[u] = read_m ? reinterpret_cast<const float4*>(a.m)[i] : make_float4(0, 0, 0, 0);
-      }
+    for (int u = 0; u < kSgdVecs; ++u) {
+      const int64_t i = base / 4 + u * kThreads + threadIdx.x;
+      pv[u] = reinterpret_cast<const float4*>(a.p)[i];
+      gv[u] = reinterpret_cast<const float4*>(a.g)[i];
+      bv[u] = read_m ? reinterpret_cast<const float4*>(a.m)[i] : make_float4(0, 0, 0, 0);
+    }
 #pragma unroll
-      for (int u = 0; u < kSgdVecs; ++u) {
-        const int64_t i = base / 4 + u * kThreads + threadIdx.x;
-        sgd_update(a, pv[u].x, gv[u].x, bv[u].x);
-        sgd_update(a, pv[u].y, gv[u].y, bv[u].y);
-        sgd_update(a, pv[u].z, gv[u].z, bv[u].z);
-        sgd_update(a, pv[u].w, gv[u].w, bv[u].w);
-        reinterpret_cast<float4*>(a.p)[i] = pv[u];
-        if (has_m) reinterpret_cast<float4*>(a.m)[i] = bv[u];
-        if (a.shadow) {
-          uint2 h;
-          *reinterpret_cast<__nv_bfloat162*>(&h.x) = __floats2bfloat162_rn(pv[u].x, pv[u].y);
-          *reinterpret_cast<__nv_bfloat162*>(&h.y) = __floats2bfloat162_rn(pv[u].z, pv[u].w);
-          reinterpret_cast<uint2*>(a.shadow)[i] = h;
-        }
+    for (int u = 0; u < kSgdVecs; ++u) {
+      const int64_t i = base / 4 + u * kThreads + threadIdx.x;
+      sgd_update(a, pv[u].x, gv[u].x, bv[u].x);
+      sgd_update(a, pv[u].y, gv[u].y, bv[u].y);
+      sgd_update(a, pv[u].z, gv[u].z, bv[u].z);
+      sgd_update(a, pv[u].w, gv[u].w, bv[u].w);
+      reinterpret_cast<float4*>(a.p)[i] = pv[u];
+      if (has_m) reinterpret_cast<float4*>(a.m)[i] = bv[u];
+      if (a.shadow) {
+        uint2 h;
+        *reinterpret_cast<__nv_bfloat162*>(&h.x) = __floats2bfloat162_rn(pv[u].x, pv[u].y);
+        *reinterpret_cast<__nv_bfloat162*>(&h.y) = __floats2bfloat162_rn(pv[u].z, pv[u].w);
+        reinterpret_cast<uint2*>(a.shadow)[i] = h;
       }
-    } else {
-      const int64_t end = base + kSgdTile < a.n ? base + kSgdTile : a.n;
-      for (int64_t i = base + threadIdx.x; i < end; i += kThreads) {
-        float pv = a.p[i], bv = read_m ? a.m[i] : 0.f;
-        sgd_update(a, pv, a.g[i], bv);
-        a.p[i] = pv;
-        if (has_m) a.m[i] = bv;
-        if (a.shadow) reinterpret_cast<__nv_bfloat16*>(a.shadow)[i] = __float2bfloat16_rn(pv);
-      }
+    }
+  } else {
+    const int64_t end = base + kSgdTile < a.n ? base + kSgdTile : a.n;
+    for (int64_t i = base + threadIdx.x; i < end; i += kThreads) {
+      float pv = a.p[i], bv = read_m ? a.m[i] : 0.f;
+      sgd_update(a, pv, a.g[i], bv);
+      a.p[i] = pv;
+      if (has_m) a.m[i] = bv;
+      if (a.shadow) reinterpret_cast<__nv_bfloat16*>(a.shadow)[i] = __float2bfloat16_rn(pv);
     }
   }
 }

@@ -776,9 +776,11 @@ void decompress_t(const uint8_t* in, size_t in_bytes, int64_t chunk, int n_chunk
   const int64_t words = chunk / VE, cap = std::max<int64_t>(1, (int64_t)sm_count() * 8 / n_chunks);
   const int64_t want = std::max<int64_t>(1, (words + kDqThreads * 2 - 1) / (kDqThreads * 2)), each = kDqThreads * kDqMany;
   const dim3 grid((unsigned)std::min(want, std::max(cap, (words + each - 1) / each)), (unsigned)n_chunks);
-  auto* kernel = words > cap * each                     ? (aligned ? dequantise_kernel<T, true, kDqMany, true> : dequantise_kernel<T, false, kDqMany, true>)
-                 : words > cap * kDqThreads * kDqFew ? (aligned ? dequantise_kernel<T, true, kDqMany, false> : dequantise_kernel<T, false, kDqMany, false>)
-                                                        : (aligned ? dequantise_kernel<T, true, kDqFew, false> : dequantise_kernel<T, false, kDqFew, false>);
+  auto* kernel = aligned ? dequantise_kernel<T, true, kDqFew, false> : dequantise_kernel<T, false, kDqFew, false>;
+  if (words > cap * each)
+    kernel = aligned ? dequantise_kernel<T, true, kDqMany, true> : dequantise_kernel<T, false, kDqMany, true>;
+  else if (words > cap * kDqThreads * kDqFew)
+    kernel = aligned ? dequantise_kernel<T, true, kDqMany, false> : dequantise_kernel<T, false, kDqMany, false>;
   launch_overlapped(kernel, grid, dim3(kDqThreads), s, in, off, chunk, (T*)out);
 }
 

@@ -83,6 +83,7 @@ void bias_relu_pool_bf16(void* y, void* p, const void* bias, int64_t N, int64_t 
 // which position of its window every pooled value came from (model_ops_bodies.cuh).
 void bias_relu_pool_only_bf16(const void* z, void* p, const void* bias, int64_t N, int64_t H, int64_t W, int C,
                               cudaStream_t stream, void* codes = nullptr);
+// Without codes; blocks train through the codes, this is what they are compared with.
 // dp: [N, H/2, W/2, C]; y as written by the in-place forward and bias null, or y = z and its bias;
 // dz: [N, H, W, C] (every element written); db: [C] fp32; scratch of
 // bias_relu_backward_scratch_bytes(N*(H/2)*(W/2), C) bytes.

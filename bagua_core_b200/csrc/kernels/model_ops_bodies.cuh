@@ -98,6 +98,11 @@ __device__ __forceinline__ uint32_t spread_bits(uint32_t bits, int k) {
   return ((0u - (b & 1u)) & 0x0000ffffu) | ((0u - ((b >> 1) & 1u)) & 0xffff0000u);
 }
 
+// Of eight values those whose bit is set.
+__device__ __forceinline__ uint4 keep_bits(const uint4& v, uint32_t bits) {
+  return make_uint4(v.x & spread_bits(bits, 0), v.y & spread_bits(bits, 1), v.z & spread_bits(bits, 2), v.w & spread_bits(bits, 3));
+}
+
 // ---- forward ----------------------------------------------------------------------
 __device__ __forceinline__ uint4 bias_relu_vec(const uint4& x, const float* b) {
   float f[8];
@@ -170,7 +175,7 @@ __device__ __forceinline__ void bias_relu_backward_body(const uint4* dy, const u
   int64_t row = (int64_t)blockIdx.x * rows_per_iter + ro;
   if constexpr (kSigns) {
     auto one = [&](const uint4& g, uint32_t bits) {
-      const uint4 r = make_uint4(g.x & spread_bits(bits, 0), g.y & spread_bits(bits, 1), g.z & spread_bits(bits, 2), g.w & spread_bits(bits, 3));
+      const uint4 r = keep_bits(g, bits);
       float f[8];
       unpack8(r, f);
 #pragma unroll
@@ -476,6 +481,7 @@ __device__ __forceinline__ uint32_t route_to_first_max(uint32_t& y0, uint32_t& y
 // zero elsewhere; db[c] = column sums of dz.  Thread (ro, cg) visits pooled pixels ro, ro + R, ...
 // and always the same 8 channels, like the un-pooled backward.  kFromZ: `y` holds the convolution's
 // output z, and the activation max(z + bias, 0), rounded as the forward rounds it, is made again here.
+// (Blocks train through bias_relu_pool_backward_codes_body; these two forms are what it is compared with.)
 template <bool kFromZ = false>
 __device__ __forceinline__ void bias_relu_pool_backward_body(const uint4* __restrict__ dp, const uint4* __restrict__ y,
                                                              uint4* __restrict__ dz, float* __restrict__ partial,
@@ -582,8 +588,7 @@ __device__ __forceinline__ void bias_relu_pool_backward_codes_body(const uint4* 
     uint4 sum = make_uint4(0, 0, 0, 0);
 #pragma unroll
     for (int at = 0; at < 4; ++at) {
-      const uint32_t bits = code >> (8 * at);
-      const uint4 r = make_uint4(g.x & spread_bits(bits, 0), g.y & spread_bits(bits, 1), g.z & spread_bits(bits, 2), g.w & spread_bits(bits, 3));
+      const uint4 r = keep_bits(g, code >> (8 * at));
       dz[q.x00 + (at & 1 ? q.dw : 0) + (at & 2 ? q.dh : 0)] = r;
       sum = make_uint4(sum.x | r.x, sum.y | r.y, sum.z | r.z, sum.w | r.w);  // a channel goes to one position at most
     }

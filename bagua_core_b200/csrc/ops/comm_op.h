@@ -32,8 +32,8 @@ class CommOp {
  public:
   virtual ~CommOp() = default;
   virtual void execute_background_communication(const BucketPtr& bucket) = 0;
-  // Whether the op's part on `bucket`, lying like that, is one that several buckets can do in one launch, and if so with `other`, the op of another
-  // bucket, too.  Such buckets are executed together, by one of their ops; the results are those of one after the other.  Those that
+  // Whether the op's part on `bucket`, lying like that, is one that several buckets can do in one launch, and if so with `other`, the
+  // op of another bucket, too.  Such buckets are executed together, by one of their ops; the results are those of one after the other.  Those that
   // are staged are staged in one buffer of `staging_bytes`, which is the same from call to call.  The result says why those that could
   // not be prepared were left out (empty: done); what fails all of them is thrown.
   virtual bool joins(const BaguaBucket& /*bucket*/, const BucketLayout& /*layout*/) const { return false; }

@@ -94,7 +94,8 @@ struct OpFrame {
 
 // Buckets of a communicator of one rank on a GPU: nothing travels, each bucket's part is local, and several that are ready at once are
 // gathered, worked on and scattered in one launch each.  Not where somebody looks at them one by one, nor buckets that keep the GPU busy
-// for longer than they wait for it anyway (VGG-16's bf16 buckets, one of them of 205 MB, quantised: 185 us alone, 192 all joined, 180-183 with this limit).
+// for longer than they wait for it anyway (VGG-16's bf16 buckets, one of them of 205 MB, quantised: 185 us alone, 192 all joined,
+// 180-183 with a limit of kJoinedBytes).
 bool joins_over_one_rank(const Communicator& comm, const BaguaBucket& bucket, const BucketLayout& layout) {
   return bucket.device_id() >= 0 && layout.bytes <= kJoinedBytes &&
          comm.kind() == Communicator::Kind::Single && comm.internode() && comm.internode()->nranks() == 1 &&

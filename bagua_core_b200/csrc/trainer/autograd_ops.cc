@@ -517,7 +517,8 @@ struct ConvNode : public AccumulatingNode {
            model_ops::first_conv_backward_supported(a.size(0), a.size(2), a.size(3), a.size(1), xs.size(1));
   }
   bool first_layer(const at::Tensor& xs, const at::Tensor& dy, const at::Tensor& a) {
-    return !task_should_compute_output(0) && task_should_compute_output(1) && (uintptr_t)dy.data_ptr() % 16 == 0 && first_layer_shape(xs, a);
+    return !task_should_compute_output(0) && task_should_compute_output(1) && (uintptr_t)dy.data_ptr() % 16 == 0 &&
+           first_layer_shape(xs, a);
   }
   void first_layer_backward(const at::Tensor& xs, const at::Tensor& dy, const at::Tensor& a, variable_list& out) {
     const int C = (int)a.size(1), Ci = (int)xs.size(1);
