@@ -491,9 +491,10 @@ struct ConvNode : public AccumulatingNode {
   }
 
   // The weight gradient of a 3 x 3 convolution of many channels, where this package's kernel is the faster one.  bf16 parameters
-  // only: where they are fp32 (autocast) their gradients keep the bits of the library's.  Of this kernel's 0.1-0.3 % are rounded the
-  // other way, which as such is nothing; but VGG-16 at batch 32, which would take 4185 us a step instead of 4521, is chaotic: the few
-  // weights whose bf16 copies differ after one such step move the second step's gradients by 5 to 15 % (relative norm).
+  // only: where they are fp32 (autocast) their gradients keep the bits of the library's.  This kernel's are the more exact ones (0.05-0.2 %
+  // are not the exact sum's rounding, 0.35-1.4 % of the library's), but VGG-16 at batch 32, which would take 4185 us a step instead of 4521,
+  // is chaotic: gradients 1e-4 apart (relative norm) in one step are 10 % apart in the next, as far as another choice of the
+  // library's algorithms moves them (profiles/vgg16_weight_gradient_rounding.md).
   bool own_weight_gradient(const at::Tensor& xs, const at::Tensor& dz) const {
     return dz.is_cuda() && is_plain3x3() && weight.scalar_type() == at::kBFloat16 && xs.scalar_type() == at::kBFloat16 &&
            dz.scalar_type() == at::kBFloat16 && xs.is_contiguous(at::MemoryFormat::ChannelsLast) &&
