@@ -593,8 +593,9 @@ uint32_t next_tag() {
 // The largest cluster that the stream's context can run: 16 blocks on the whole GPU, 8 in a green context of any size, fewer under other
 // limits.  Asked once per stream, by an id that no other stream of the process gets.
 int largest_cluster(cudaStream_t s) {
-  static std::mutex mu;
-  static std::map<unsigned long long, int> known;
+  // (never given back: engine threads may outlive static objects)
+  static std::mutex& mu = *new std::mutex;
+  static std::map<unsigned long long, int>& known = *new std::map<unsigned long long, int>;
   static thread_local unsigned long long last_id = 0;
   static thread_local int last = -1;
   unsigned long long id = 0;
