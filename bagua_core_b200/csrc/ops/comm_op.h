@@ -28,19 +28,21 @@ struct EngineConfig {
 // Buckets that are executed together have at most this many bytes each, and as many in all of those that are staged.
 constexpr int64_t kJoinedBytes = 32 << 20;
 
+using JoinedFailures = std::vector<std::pair<size_t, std::string>>;
+
 class CommOp {
  public:
   virtual ~CommOp() = default;
   virtual void execute_background_communication(const BucketPtr& bucket) = 0;
   // Whether the op's part on `bucket`, lying like that, is one that several buckets can do in one launch, and if so with `other`, the
   // op of another bucket, too.  Such buckets are executed together, by one of their ops; the results are those of one after the other.  Those that
-  // are staged are staged in one buffer of `staging_bytes`, which is the same from call to call.  The result says why those that could
-  // not be prepared were left out (empty: done); what fails all of them is thrown.
+  // are staged are staged in one buffer of `staging_bytes`, which is the same from call to call.  The result names those that could
+  // not be prepared and were left out, by place, and why; what fails all of them is thrown.
   virtual bool joins(const BaguaBucket& /*bucket*/, const BucketLayout& /*layout*/) const { return false; }
   virtual bool joins_with(const CommOp& /*other*/) const { return false; }
-  virtual std::vector<std::string> execute_joined(const std::vector<BucketPtr>& buckets, int64_t /*staging_bytes*/) {
+  virtual JoinedFailures execute_joined(const std::vector<BucketPtr>& buckets, int64_t /*staging_bytes*/) {
     for (const BucketPtr& b : buckets) execute_background_communication(b);
-    return std::vector<std::string>(buckets.size());
+    return {};
   }
   virtual std::string describe() const = 0;
   // State worth checkpointing (e.g. the gossip step counter); empty for stateless ops.

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cstdio>
 #include <cstdlib>
 #include <deque>
@@ -108,22 +109,25 @@ void copy_joined(std::vector<kernels::MultiCopyItem>& items, bool gather, uint64
                                      (cudaStream_t)stream);
 }
 // Held together the locks of several buckets are taken by address: two backends may hold the same buckets in different orders.
-std::vector<std::unique_lock<std::mutex>> lock_all(const std::vector<BucketPtr>& buckets) {
-  std::vector<std::unique_lock<std::mutex>> locks;
-  for (const BucketPtr& b : buckets) locks.emplace_back(b->exec_mutex(), std::defer_lock);
-  std::vector<std::unique_lock<std::mutex>*> order;
-  for (auto& l : locks) order.push_back(&l);
-  std::sort(order.begin(), order.end(), [](auto* a, auto* b) { return std::less<std::mutex*>()(a->mutex(), b->mutex()); });
-  for (auto* l : order) l->lock();
-  return locks;
+void lock_all(const std::vector<BucketPtr>& buckets, std::array<std::unique_lock<std::mutex>, kernels::kMaxJoined>& locks) {
+  std::array<std::unique_lock<std::mutex>*, kernels::kMaxJoined> order;
+  const auto end = order.begin() + buckets.size();
+  for (size_t k = 0; k < buckets.size(); ++k) {
+    locks[k] = std::unique_lock<std::mutex>(buckets[k]->exec_mutex(), std::defer_lock);
+    order[k] = &locks[k];
+  }
+  std::sort(order.begin(), end, [](auto* a, auto* b) { return std::less<std::mutex*>()(a->mutex(), b->mutex()); });
+  for (auto it = order.begin(); it != end; ++it) (*it)->lock();
 }
 // All staging buffers of the batch are wanted until its scatter is launched; they are parts of one block, which every batch of these
 // buckets pulls in the same size: what the pool holds does not depend on which buckets happened to meet.  A bucket that cannot be
 // prepared fails alone.
-std::vector<std::string> run_joined(Communicator& comm, const std::vector<BucketPtr>& buckets, int64_t staging_bytes,
-                                    const std::function<void(std::vector<RawTensor*>&)>& work) {
-  std::vector<std::string> errors(buckets.size());
-  auto locks = lock_all(buckets);
+JoinedFailures run_joined(Communicator& comm, const std::vector<BucketPtr>& buckets, int64_t staging_bytes,
+                          const std::function<void(std::vector<RawTensor*>&)>& work) {
+  BAGUA_CHECK(buckets.size() <= (size_t)kernels::kMaxJoined, Bucket, "too many buckets for one launch");
+  JoinedFailures failed;
+  std::array<std::unique_lock<std::mutex>, kernels::kMaxJoined> locks;
+  lock_all(buckets, locks);
   JoinedStaging staging(staging_bytes, buckets[0]->device_id(), comm.stream());
   std::vector<kernels::MultiCopyItem> scatter;
   std::deque<OpFrame> frames;
@@ -133,15 +137,15 @@ std::vector<std::string> run_joined(Communicator& comm, const std::vector<Bucket
       frames.emplace_back(std::move(locks[k]), buckets[k], comm, false, false, &staging);
       raws.push_back(frames.back().ct.raw.get());
     } catch (const std::exception& e) {
-      errors[k] = e.what();
+      failed.emplace_back(k, e.what());
     }
   }
-  if (frames.empty()) return errors;
+  if (frames.empty()) return failed;
   copy_joined(staging.gather, true, comm.stream());
   work(raws);
   for (OpFrame& f : frames) f.ct.finish(false, &scatter);
   copy_joined(scatter, false, comm.stream());
-  return errors;
+  return failed;
 }
 bool occupies_for_probe() {
   static const bool on = std::getenv("BAGUA_B200_PROBE_OCCUPY") != nullptr;
@@ -214,7 +218,7 @@ class CentralizedFullPrecisionSynchronous : public CommOp {
     auto* o = dynamic_cast<const CentralizedFullPrecisionSynchronous*>(&other);
     return o && o->comm_->internode() == comm_->internode();
   }
-  std::vector<std::string> execute_joined(const std::vector<BucketPtr>& buckets, int64_t staging_bytes) override {
+  JoinedFailures execute_joined(const std::vector<BucketPtr>& buckets, int64_t staging_bytes) override {
     return run_joined(*comm_, buckets, staging_bytes, [](std::vector<RawTensor*>&) {});
   }
 
@@ -274,7 +278,7 @@ class CentralizedLowPrecisionSynchronous : public CommOp {
     auto* o = dynamic_cast<const CentralizedLowPrecisionSynchronous*>(&other);
     return o && o->comm_->internode() == comm_->internode() && o->method_ == method_;
   }
-  std::vector<std::string> execute_joined(const std::vector<BucketPtr>& buckets, int64_t staging_bytes) override {
+  JoinedFailures execute_joined(const std::vector<BucketPtr>& buckets, int64_t staging_bytes) override {
     return run_joined(*comm_, buckets, staging_bytes,
                [&](std::vector<RawTensor*>& ts) { tensor_ops::quantise_twice(ts, method_, comm_->stream()); });
   }

@@ -99,27 +99,26 @@ void CommBackend::execute(const std::vector<std::shared_ptr<ScheduledCommOp>>& b
     }
   }
   const ScheduledCommOp& op = *batch[0];
-  std::vector<BucketPtr> buckets;
-  for (auto& item : batch) buckets.push_back(item->bucket);
+  const std::vector<BucketPtr>& buckets = current_.buckets;  // which only this thread writes
   {
     std::lock_guard<std::mutex> g(current_.mu);
-    current_.buckets = buckets;
+    for (auto& item : batch) current_.buckets.push_back(item->bucket);
     current_.since = std::chrono::steady_clock::now();
     current_.reported = false;
   }
   const uint64_t t0 = Telemetry::instance().now();
-  std::vector<std::string> errors(batch.size());
+  std::string err;
+  JoinedFailures failed;
   // Optional NVTX range per bucket or joined batch (BAGUA_B200_NVTX=1) so that profiler timelines line up
   // with bucket names; a no-op when no tool is attached.
   static const bool nvtx = env_long("BAGUA_B200_NVTX", 0) != 0;
   if (nvtx) nvtxRangePushA(batch.size() > 1 ? names_of(buckets).c_str() : op.bucket->name().c_str());
   try {
     if (joined) {
-      errors = op.ops[0]->execute_joined(buckets, op.staging_bytes);
-      EngineStats::global().ops_executed += (uint64_t)std::count(errors.begin(), errors.end(), "");
-      for (size_t k = 0; k < batch.size(); ++k)
-        if (!errors[k].empty())
-          BAGUA_LOG(Error, "communication op on bucket `" << batch[k]->bucket->name() << "` failed: " << errors[k]);
+      failed = op.ops[0]->execute_joined(buckets, op.staging_bytes);
+      EngineStats::global().ops_executed += batch.size() - failed.size();
+      for (auto& [k, why] : failed)
+        BAGUA_LOG(Error, "communication op on bucket `" << buckets[k]->name() << "` failed: " << why);
     } else {
       for (auto& o : op.ops) {
         o->execute_background_communication(op.bucket);
@@ -127,8 +126,8 @@ void CommBackend::execute(const std::vector<std::shared_ptr<ScheduledCommOp>>& b
       }
     }
   } catch (const std::exception& e) {
-    errors.assign(batch.size(), e.what());
-    BAGUA_LOG(Error, "communication op on " << names_of(buckets) << " failed: " << e.what());
+    err = e.what();
+    BAGUA_LOG(Error, "communication op on " << names_of(buckets) << " failed: " << err);
   }
   if (nvtx) nvtxRangePop();
   for (auto& item : batch) Telemetry::instance().record("bucket_executed", item->bucket->name(), t0);
@@ -137,10 +136,13 @@ void CommBackend::execute(const std::vector<std::shared_ptr<ScheduledCommOp>>& b
     current_.buckets.clear();
   }
   for (size_t k = 0; k < batch.size(); ++k) {
-    if (errors[k].empty())
+    const std::string* why = err.empty() ? nullptr : &err;
+    for (auto& f : failed)
+      if (f.first == k) why = &f.second;
+    if (!why)
       batch[k]->event.finish();
     else
-      batch[k]->event.fail(errors[k]);
+      batch[k]->event.fail(*why);
     BAGUA_LOG(Debug, "comm op executed: " << batch[k]->name);
   }
 }

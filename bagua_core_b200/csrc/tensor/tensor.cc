@@ -266,24 +266,26 @@ CommunicationTensor BaguaBucket::get_communication_tensor(uint64_t stream, bool 
                                                           JoinedStaging* joined) {
   CommunicationTensor ct;
   ct.stream = stream;
+  // one pass: a bucket may have hundreds of tensors, and their owners' threads are at work on them
+  const size_t es = dtype_bytes(dtype_);
+  int64_t total = 0;
+  bool adjacent = true;
+  const uint64_t first = tensors_[0]->data_ptr();
   for (auto& t : tensors_) {
     uint64_t ev = t->take_ready_event();
     if (ev != 0 && device_ >= 0)
       BAGUA_CUDA_CHECK(cudaStreamWaitEvent((cudaStream_t)stream, (cudaEvent_t)ev, 0));
+    adjacent = adjacent && t->data_ptr() == first + (uint64_t)total * es;
+    total += t->num_elements_allocated();
   }
-  const int64_t total = total_allocated();
-  if (!force_copy && contiguous()) {
-    int64_t real = 0;
-    for (auto& t : tensors_) real += t->num_elements_allocated();
-    ct.raw = std::make_shared<PoolRawTensor>((void*)(uintptr_t)tensors_[0]->data_ptr(), nullptr, real, total, dtype_,
-                                             device_);
+  if (!force_copy && adjacent) {
+    ct.raw = std::make_shared<PoolRawTensor>((void*)(uintptr_t)first, nullptr, total, total, dtype_, device_);
     ct.need_copy_back = false;
     return ct;
   }
   // Staged: one launch gathers every tensor into a pool buffer (the reference issues one copy
   // per tensor, datatypes/mod.rs:1012-1023).
   auto buf = joined ? joined->take(dtype_, total) : PoolRawTensor::allocate(device_, dtype_, total, stream);
-  const size_t es = dtype_bytes(dtype_);
   unsigned long long off = 0;
   kernels::Ctx c{device_, (cudaStream_t)stream};
   ct.segments.reserve(tensors_.size());
