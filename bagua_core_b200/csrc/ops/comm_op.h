@@ -35,9 +35,9 @@ class CommOp {
   virtual ~CommOp() = default;
   virtual void execute_background_communication(const BucketPtr& bucket) = 0;
   // Whether the op's part on `bucket`, lying like that, is one that several buckets can do in one launch, and if so with `other`, the
-  // op of another bucket, too.  Such buckets are executed together, by one of their ops; the results are those of one after the other.  Those that
-  // are staged are staged in one buffer of `staging_bytes`, which is the same from call to call.  The result names those that could
-  // not be prepared and were left out, by place, and why; what fails all of them is thrown.
+  // op of another bucket, too.  Such buckets are executed together, by one of their ops; the results are those of one after the
+  // other.  Those that are staged are staged in one buffer of `staging_bytes`, which is the same from call to call.  The result
+  // names those that could not be prepared and were left out, by place, and why; what fails all of them is thrown.
   virtual bool joins(const BaguaBucket& /*bucket*/, const BucketLayout& /*layout*/) const { return false; }
   virtual bool joins_with(const CommOp& /*other*/) const { return false; }
   virtual JoinedFailures execute_joined(const std::vector<BucketPtr>& buckets, int64_t /*staging_bytes*/) {
