@@ -39,6 +39,7 @@ class CommOp {
   // other.  Those that are staged are staged in one buffer of `staging_bytes`, which is the same from call to call.  The result
   // names those that could not be prepared and were left out, by place, and why; what fails all of them is thrown.
   virtual bool joins(const BaguaBucket& /*bucket*/, const BucketLayout& /*layout*/) const { return false; }
+  virtual int joined_base_us() const { return 0; }  // what a batch takes on the GPU besides its bytes
   virtual bool joins_with(const CommOp& /*other*/) const { return false; }
   virtual JoinedFailures execute_joined(const std::vector<BucketPtr>& buckets, int64_t /*staging_bytes*/) {
     for (const BucketPtr& b : buckets) execute_background_communication(b);

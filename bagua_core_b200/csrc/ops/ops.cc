@@ -214,6 +214,7 @@ class CentralizedFullPrecisionSynchronous : public CommOp {
   bool joins(const BaguaBucket& bucket, const BucketLayout& layout) const override {
     return joins_over_one_rank(*comm_, bucket, layout) && !occupies_for_probe() && !layout.contiguous;
   }
+  int joined_base_us() const override { return 6; }
   bool joins_with(const CommOp& other) const override {
     auto* o = dynamic_cast<const CentralizedFullPrecisionSynchronous*>(&other);
     return o && o->comm_->internode() == comm_->internode();
@@ -274,6 +275,7 @@ class CentralizedLowPrecisionSynchronous : public CommOp {
     return o.str();
   }
   bool joins(const BaguaBucket& bucket, const BucketLayout& layout) const override { return joins_over_one_rank(*comm_, bucket, layout); }
+  int joined_base_us() const override { return 8; }
   bool joins_with(const CommOp& other) const override {
     auto* o = dynamic_cast<const CentralizedLowPrecisionSynchronous*>(&other);
     return o && o->comm_->internode() == comm_->internode() && o->method_ == method_;

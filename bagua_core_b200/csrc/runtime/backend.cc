@@ -51,7 +51,8 @@ void CommBackend::worker_loop() {
     if (!joinable) continue;
     int64_t bytes = 0;
     for (auto& item : batch) bytes += item->layout->bytes;
-    busy_until_ = std::max(busy_until_, std::chrono::steady_clock::now()) + std::chrono::microseconds(kJoinBaseUs + bytes / kJoinBytesPerUs);
+    busy_until_ = std::max(busy_until_, std::chrono::steady_clock::now()) +
+                  std::chrono::microseconds(batch[0]->ops[0]->joined_base_us() + bytes / kJoinBytesPerUs);
   }
 }
 

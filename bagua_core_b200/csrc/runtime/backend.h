@@ -84,14 +84,16 @@ class CommBackend {
   Channel<EventChannel> not_waited_;
   // Buckets that become ready faster than the GPU takes them one by one are handed over together: one that finds the GPU busy with
   // earlier ones for longer than a launch takes to reach it (kJoinAheadUs) waits for more, unless somebody waits for the buckets.  How
-  // long the GPU is busy is reckoned: 8 us for what is joined and 4 us for every 10 MB (quantised twice: 12.3 us for one bucket of 10 MB,
-  // 16.4 for two, 24.5 for four).  Bursts over one rank, us, alone / together: 13 fp32 buckets of 8 MB quantised 164 / 125, 7 staged bf16
+  // long the GPU is busy is reckoned: 8 us for what is quantised, 6 for what is copied, and 4 us for every 10 MB (quantised twice: 12.3 us
+  // for one bucket of 10 MB, 16.4 for two, 24.5 for four).  Bursts over one rank, us, alone / together: 13 fp32 buckets of 8 MB quantised 164 / 125, 7 staged bf16
   // ones of 7 MB quantised 186 / 124, 7 staged fp16 ones copied 102 / 89, 3 staged fp32 ones of 8 MB, which come too slowly, 54-66 both.
-  // Ahead by 12 us: 126, 141, 98; waiting until the GPU is done: 13 buckets 122, but 3 quantised ones 50 / 55.
+  // Ahead by 12 us: 126, 141, 98; waiting until the GPU is done: 13 buckets 122, but 3 quantised ones 50 / 55.  Ahead by 8 us and with 8 us
+  // for copies too, as it was while the worker took longer to hand over, / as here: 13 buckets 127 / 121, 7 staged bf16 ones 134 / 115, 22
+  // staged fp16 ones of 2 MB 249 / 243, 3 staged fp32 ones of 8 MB 46 / 47; with 8 us for copies 52.
   // A joined launch waits for the youngest of its buckets' gradients.  Training steps over one rank, quantised, us, alone / together, in
   // two runs each: VGG-16 at batch 32 4609-4642 / 4585-4613, at batch 8 with buckets of 5 MB 2508-2543 / 2488-2490, MLPs of 6 layers
   // of width 4096 1584-1594 / 1582-1590, of 2048 870-880 / 830-881: buckets that come 40 us apart are not joined.
-  static constexpr int64_t kJoinBaseUs = 8, kJoinBytesPerUs = 2500000, kJoinAheadUs = 8, kJoinMostUs = 40;
+  static constexpr int64_t kJoinBytesPerUs = 2500000, kJoinAheadUs = 6, kJoinMostUs = 40;
   std::shared_ptr<ScheduledCommOp> next_;                // worker only
   std::chrono::steady_clock::time_point busy_until_{};   // worker only: the GPU, as reckoned
   std::atomic<int> waiters_{0};                                 // threads in wait_pending_comm_ops()
